@@ -202,6 +202,26 @@ int mb200_moe_grouped_ffn(const void* xs, const void* const* w13_host, const voi
                           int64_t hidden, int64_t n_experts, int64_t top_k, const mb200_moe_comm* comm, void* workspace,
                           size_t workspace_bytes, void* stream);
 
+/* ---------------------------------------------------------------------------------------------
+ * Linears and mixtures of layered decoders (no counterpart in the reference; the formulas of `epi` are those of
+ * mbh_linear, include/mistral_b200_hybrid.h, 0 .. 7 without the decays).  bf16 in, fp32 accumulation, the step that follows the
+ * Linear in its epilogue.
+ * mb200_layer_linear: T >= 128 rows, N % 128 == 0, K % 64 == 0.  out: bf16 results; out32: the fp32 residual stream or fp32 results.
+ *     rowscale [T, rs_pitch] fp32 or NULL: hidden unit c of row t is scaled by rowscale[t, c / rs_group].  n_act columns through SiLU.
+ * mb200_layer_moe: y32 [T, width] fp32 (+= when add) sum over the token's choices idx [T, top] < n_experts of
+ *     wsel * (act W2_e^T), act = step(hn W13_e^T); w13 [E * 2 ff, width] (gate/up rows interleaved; RELU2: [E * ff, width]),
+ *     w2 [width, E * ff].  The weight multiplies the hidden units (GLU: the expert's input).  width % 128 == 0, ff % 64 == 0,
+ *     T <= 65535.  Buffers (device, uninitialised): slot [T * top] int32, plan [plan_words] int32, xs [rows_cap, width] bf16,
+ *     row_w [rows_cap] fp32, act [rows_cap, ff] bf16, rows32 [rows_cap, width] fp32.
+ */
+#define MB200_LAYER_MOE_MAX_EXPERTS 48
+int mb200_layer_linear(const void* x, const void* w, const void* bias, void* out, float* out32, int64_t T, int64_t N, int64_t K, int epi, int64_t n_act,
+                       float limit, float alpha, const float* rowscale, int64_t rs_pitch, int64_t rs_group, void* stream);
+int mb200_layer_moe_sizes(int64_t T, int64_t n_experts, int64_t top, int64_t* rows_cap, int64_t* plan_words);
+int mb200_layer_moe(const void* hn, const void* w13, const void* w2, const int32_t* idx, const float* wsel, int64_t T, int64_t dim, int64_t ff, int64_t n_experts,
+                    int64_t top, int epi, float limit, float alpha, int32_t* slot, int32_t* plan, void* xs, float* row_w, void* act, float* rows32, float* y32,
+                    int add, void* stream);
+
 /* Buffers that other ranks (one process per GPU) can write: plain cudaMalloc + CUDA IPC.  alloc zero-fills and synchronises;
  * export writes the 64-byte IPC handle to pass to the other processes (e.g. torch.distributed.all_gather_object); open maps a
  * peer's buffer into this process (peer access over NVLink is enabled lazily).  These are the only entry points that allocate. */

@@ -46,6 +46,11 @@ _SIGNATURES = {
                                 c_void_p, c_void_p, c_void_p]),
     "mb200_moe_grouped_ffn": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64,
                                       c_int64, c_int64, c_int64, c_int64, c_void_p, c_void_p, c_size_t, c_void_p]),
+    "mb200_layer_linear": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int, c_int64, c_float, c_float, c_void_p,
+                                   c_int64, c_int64, c_void_p]),
+    "mb200_layer_moe_sizes": (c_int, [c_int64, c_int64, c_int64, ctypes.POINTER(c_int64), ctypes.POINTER(c_int64)]),
+    "mb200_layer_moe": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64, c_int64, c_int, c_float, c_float,
+                                c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p]),
     "mb200_comm_alloc": (c_int, [c_size_t, ctypes.POINTER(c_void_p)]),
     "mb200_comm_free": (c_int, [c_void_p]),
     "mb200_comm_export": (c_int, [c_void_p, c_void_p]),
@@ -266,6 +271,35 @@ def moe_grouped_ffn(b, w13_host, w2_host, residual: Optional[torch.Tensor], out:
                                        _ptr(b.slot), _ptr(residual), _ptr(b.g), b.yw_ptr, _ptr(out), T, dim, hidden, E, k,
                                        ctypes.cast(ctypes.pointer(comm), c_void_p) if comm is not None else None, ws.ptr, ws.nbytes, _stream()),
            "mb200_moe_grouped_ffn")
+
+
+def layer_linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: Optional[torch.Tensor], out32: Optional[torch.Tensor], epi: int,
+                 n_act: int = 0, limit: float = 0.0, alpha: float = 0.0, rowscale: Optional[torch.Tensor] = None, group: int = 1) -> None:
+    """A layered decoder's Linear over T >= 128 rows with the step that follows it in the GEMM's epilogue (include/mistral_b200.h)."""
+    T, K = x.shape
+    _check(lib().mb200_layer_linear(_ptr(x), _ptr(w), _ptr(bias), _ptr(out), _ptr(out32), T, w.shape[0], K, epi, n_act, limit, alpha, _ptr(rowscale),
+                                    rowscale.shape[1] if rowscale is not None else 0, group, _stream()), "mb200_layer_linear")
+
+
+LAYER_MOE_MAX_EXPERTS = 48
+LAYER_MOE_MAX_TOKENS = 8192  # tokens per call of layer_moe: bounds the row buffers
+
+
+def layer_moe(hn: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, idx: torch.Tensor, wsel: torch.Tensor, E: int, ff: int, epi: int, limit: float,
+              alpha: float, y32: torch.Tensor, add: bool) -> None:
+    """y32 (+)= the weighted sum of each token's chosen experts, computing the chosen (token, expert) rows only (include/mistral_b200.h)."""
+    top = idx.shape[1]
+    for r0 in range(0, hn.shape[0], LAYER_MOE_MAX_TOKENS):
+        h, sel, wts, y = (t[r0: r0 + LAYER_MOE_MAX_TOKENS] for t in (hn, idx, wsel, y32))
+        T, D = h.shape
+        rc, pw = c_int64(0), c_int64(0)
+        _check(lib().mb200_layer_moe_sizes(T, E, top, ctypes.byref(rc), ctypes.byref(pw)), "mb200_layer_moe_sizes")
+        rows = rc.value
+        new = lambda n, dt: torch.empty(n, dtype=dt, device=h.device)  # noqa: E731
+        slot, plan, row_w = new(T * top, torch.int32), new(pw.value, torch.int32), new(rows, torch.float32)
+        xs, act, rows32 = new(rows * D, h.dtype), new(rows * ff, h.dtype), new(rows * D, torch.float32)
+        _check(lib().mb200_layer_moe(_ptr(h), _ptr(w13), _ptr(w2), _ptr(sel), _ptr(wts), T, D, ff, E, top, epi, limit, alpha, _ptr(slot), _ptr(plan), _ptr(xs),
+                                     _ptr(row_w), _ptr(act), _ptr(rows32), _ptr(y), int(add), _stream()), "mb200_layer_moe")
 
 
 def comm_alloc(nbytes: int) -> int:

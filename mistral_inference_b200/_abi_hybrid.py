@@ -14,7 +14,7 @@ from . import _abi, build
 from ._abi import Mb200Error
 
 ABI_VERSION = 6
-EPI_STORE, EPI_RESIDUAL, EPI_GLU, EPI_F32, EPI_RESIDUAL_SCALED = 0, 1, 2, 3, 5
+EPI_STORE, EPI_RESIDUAL, EPI_GLU, EPI_F32, EPI_SWIGLU, EPI_RESIDUAL_SCALED, EPI_RELU2, EPI_GEGLU = 0, 1, 2, 3, 4, 5, 6, 7
 _DT = {torch.bfloat16: 0, torch.float32: 1}
 _lib: Optional[ctypes.CDLL] = None
 
@@ -139,21 +139,17 @@ def rmsnorm_pair(x32: torch.Tensor, w: torch.Tensor, w2: torch.Tensor, eps: floa
     return y, y2
 
 
-_ws: dict = {}
-
-
-def _workspace(device: torch.device) -> "_abi.Workspace":
-    if device not in _ws:
-        _ws[device] = _abi.Workspace(_abi.workspace_bytes(1, 64, 1, 1, 128, 64, 0, 1), device)
-    return _ws[device]
-
-
 def _prompt_gemm_ok(x: torch.Tensor, M: int, N: int, K: int) -> bool:
-    """Large bf16 Linears of prompts go to the main library's persistent tcgen05 GEMM when it is built and the shape fits its
-    tiles (K % 64 == 0, N % 128 == 0, at least one 128-row tile); everything else runs on this library's own kernels.  A checkout
-    that has only libmb200_hybrid.so never builds the main library for this."""
+    """Large bf16 Linears of prompts go to the main library's persistent tcgen05 GEMM (`_abi.layer_linear`: the step after the Linear is its
+    epilogue) when it is built and the shape fits its tiles (K % 64 == 0, N % 128 == 0, at least one 128-row tile); everything else runs on
+    this library's own kernels.  A checkout that has only libmb200_hybrid.so never builds the main library for this."""
     return (x.dtype == torch.bfloat16 and M >= 128 and K % 64 == 0 and N % 128 == 0 and os.environ.get("MB200_HYBRID_GEMM", "1") != "0"
             and _abi.library_path().exists())
+
+
+def _aligned(*tensors: Optional[torch.Tensor]) -> bool:
+    """16-byte aligned starts: what the tensor-core GEMM's copies and vector accesses need."""
+    return all(t is None or t.data_ptr() % 16 == 0 for t in tensors)
 
 
 def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, *, epi: int = EPI_STORE, n_act: int = 0,
@@ -172,13 +168,11 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None
         out32 = torch.empty(M, N, dtype=torch.float32, device=x.device)
     else:
         out = torch.empty(M, N // 2 if epi == EPI_GLU else N, dtype=x.dtype, device=x.device)
-    if _prompt_gemm_ok(x, M, N, K):
-        # the framework's tcgen05 GEMM (bf16 out), then this library's epilogue over its result
-        y = torch.empty(M, N, dtype=x.dtype, device=x.device)
-        _abi.linear_residual(x.contiguous(), w, None, y, _workspace(x.device))
-        _check(lib().mbh_linear_epilogue(_ptr(y), _ptr(bias), _ptr(out), _ptr(out32), M, N, epi, n_act, limit, alpha, dt_of(x.dtype), _stream()),
-               "mbh_linear_epilogue")
-        return out if out is not None else out32
+    if _prompt_gemm_ok(x, M, N, K) and _aligned(w, bias, out32) and epi in (EPI_STORE, EPI_RESIDUAL, EPI_RESIDUAL_SCALED, EPI_F32, EPI_GLU):
+        xc = x.contiguous()
+        if _aligned(xc):
+            _abi.layer_linear(xc, w, bias, out, out32, epi, n_act, limit, alpha)
+            return out if out is not None else out32
     xp, ldx = _rows(x)
     _check(lib().mbh_linear(xp, ldx, _ptr(w), _ptr(bias), _ptr(out), _ptr(out32), M, N, K, epi, n_act, limit, alpha, dt_of(x.dtype), _stream()),
            "mbh_linear")
@@ -264,11 +258,8 @@ def linear_swiglu(x: torch.Tensor, w: torch.Tensor, rowscale: Optional[torch.Ten
         assert rowscale.dtype == torch.float32 and rowscale.shape[0] == M and group > 0 and (N // 2 + group - 1) // group <= rowscale.shape[1]
         pitch = rowscale.shape[1]
     out = torch.empty(M, N // 2, dtype=x.dtype, device=x.device)
-    if _prompt_gemm_ok(x, M, N, K):
-        y = torch.empty(M, N, dtype=x.dtype, device=x.device)
-        _abi.linear_residual(x, w, None, y, _workspace(x.device))
-        _check(lib().mbh_swiglu_epilogue(_ptr(y), _ptr(out), M, N, _ptr(rowscale), pitch, group, int(gelu), dt_of(x.dtype), _stream()),
-               "mbh_swiglu_epilogue")
+    if _prompt_gemm_ok(x, M, N, K) and _aligned(x, w):
+        _abi.layer_linear(x, w, None, out, None, EPI_GEGLU if gelu else EPI_SWIGLU, rowscale=rowscale, group=max(group, 1))
         return out
     _check(lib().mbh_linear_swiglu(_ptr(x), _ptr(w), _ptr(out), M, N, K, _ptr(rowscale), pitch, group, int(gelu), dt_of(x.dtype), _stream()),
            "mbh_linear_swiglu")
@@ -308,6 +299,24 @@ def moe_sparse(h: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, idx: torch.
     y32 = torch.empty(T, D, dtype=torch.float32, device=h.device) if add_to is None else add_to
     _check(lib().mbh_moe_sparse(_ptr(h), _ptr(w13), _ptr(w2), _ptr(idx), _ptr(wsel), _ptr(act), _ptr(y32), T, D, ff, E, top, int(glu), limit, alpha,
                                 int(add_to is not None), dt_of(h.dtype), _stream()), "mbh_moe_sparse")
+    return y32
+
+
+def moe_grouped_ok(h: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, E: int, ff: int) -> bool:
+    """Prompts of a mixture whose sizes fit the main library's grouped GEMMs (bf16, width % 128 == 0, ff % 64 == 0, the first Linear's rows
+    per expert a multiple of 128) compute the chosen (token, expert) rows only; other sizes run every expert on every token."""
+    units = w13.shape[0] // E
+    return (h.dtype == torch.bfloat16 and h.shape[1] % 128 == 0 and ff % 64 == 0 and units % 128 == 0 and E <= _abi.LAYER_MOE_MAX_EXPERTS and _aligned(h, w13, w2)
+            and os.environ.get("MB200_HYBRID_GEMM", "1") != "0" and _abi.library_path().exists())
+
+
+def moe_grouped(h: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, idx: torch.Tensor, wsel: torch.Tensor, E: int, ff: int, epi: int,
+                limit: float = 0.0, alpha: float = 0.0, add_to: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """fp32 [T, width]: the weighted sum of each token's chosen experts (indices >= E: none); added to add_to (fp32) when given.  epi: the
+    unit between the two Linears (EPI_SWIGLU, EPI_GLU with the weight on the expert's input, EPI_GEGLU, EPI_RELU2)."""
+    assert idx.dtype == torch.int32 and wsel.dtype == torch.float32 and idx.shape == wsel.shape
+    y32 = torch.empty(h.shape, dtype=torch.float32, device=h.device) if add_to is None else add_to
+    _abi.layer_moe(h, w13, w2, idx, wsel, E, ff, epi, limit, alpha, y32, add_to is not None)
     return y32
 
 
@@ -564,10 +573,8 @@ def linear_glu(x: torch.Tensor, w: torch.Tensor, limit: float, alpha: float, row
         assert rowscale.dtype == torch.float32 and rowscale.shape[0] == M and group > 0 and (N // 2 + group - 1) // group <= rowscale.shape[1]
         pitch = rowscale.shape[1]
     out = torch.empty(M, N // 2, dtype=x.dtype, device=x.device)
-    if _prompt_gemm_ok(x, M, N, K):
-        y = torch.empty(M, N, dtype=x.dtype, device=x.device)
-        _abi.linear_residual(x, w, None, y, _workspace(x.device))
-        _check(lib().mbh_glu_epilogue(_ptr(y), _ptr(out), M, N, limit, alpha, _ptr(rowscale), pitch, group, dt_of(x.dtype), _stream()), "mbh_glu_epilogue")
+    if _prompt_gemm_ok(x, M, N, K) and _aligned(x, w):
+        _abi.layer_linear(x, w, None, out, None, EPI_GLU, limit=limit, alpha=alpha, rowscale=rowscale, group=max(group, 1))
         return out
     _check(lib().mbh_linear_glu(_ptr(x), _ptr(w), _ptr(out), M, N, K, limit, alpha, _ptr(rowscale), pitch, group, dt_of(x.dtype), _stream()), "mbh_linear_glu")
     return out
@@ -648,10 +655,8 @@ def linear_relu2(x: torch.Tensor, w: torch.Tensor, rowscale: Optional[torch.Tens
         assert rowscale.dtype == torch.float32 and rowscale.shape[0] == M and group > 0 and (N + group - 1) // group <= rowscale.shape[1]
         pitch = rowscale.shape[1]
     out = torch.empty(M, N, dtype=x.dtype, device=x.device)
-    if _prompt_gemm_ok(x, M, N, K):
-        y = torch.empty(M, N, dtype=x.dtype, device=x.device)
-        _abi.linear_residual(x, w, None, y, _workspace(x.device))
-        _check(lib().mbh_relu2_epilogue(_ptr(y), _ptr(out), M, N, _ptr(rowscale), pitch, group, dt_of(x.dtype), _stream()), "mbh_relu2_epilogue")
+    if _prompt_gemm_ok(x, M, N, K) and _aligned(x, w):
+        _abi.layer_linear(x, w, None, out, None, EPI_RELU2, rowscale=rowscale, group=max(group, 1))
         return out
     _check(lib().mbh_linear_relu2(_ptr(x), _ptr(w), _ptr(out), M, N, K, _ptr(rowscale), pitch, group, dt_of(x.dtype), _stream()), "mbh_linear_relu2")
     return out

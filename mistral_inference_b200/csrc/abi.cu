@@ -416,6 +416,87 @@ int mb200_moe_grouped_ffn(const void* xs, const void* const* w13_host, const voi
   return MB200_OK;
 }
 
+// ---- Linears and mixtures of layered decoders ----------------------------------------------------------------------------------
+static int layer_epilogue(EpiParams& e, const void* bias, void* out, float* out32, int64_t N, int epi, int64_t n_act, float limit, float alpha) {
+  MB_CHECK_ARG(epi >= LAYER_STORE && epi <= LAYER_GEGLU, "layer_linear: step %d", epi);
+  const bool gated = epi == LAYER_GLU || epi == LAYER_SWIGLU || epi == LAYER_GEGLU;
+  const bool f32 = epi == LAYER_RESIDUAL || epi == LAYER_F32 || epi == LAYER_RESIDUAL_SCALED;
+  MB_CHECK_ARG(f32 ? out32 != nullptr : out != nullptr, "layer_linear: output missing");
+  MB_CHECK_ARG(((uintptr_t)bias | (uintptr_t)out | (uintptr_t)out32) % 16 == 0, "layer_linear: bias and outputs must be 16-byte aligned");
+  e.layer = epi;
+  e.n_act = (int)n_act;
+  e.limit = limit;
+  e.alpha = alpha;
+  e.bias = bias;
+  e.out = out;
+  e.out_f32 = out32;
+  e.ld_out = gated ? N / 2 : N;
+  return MB200_OK;
+}
+
+int mb200_layer_linear(const void* x, const void* w, const void* bias, void* out, float* out32, int64_t T, int64_t N, int64_t K, int epi, int64_t n_act,
+                       float limit, float alpha, const float* rowscale, int64_t rs_pitch, int64_t rs_group, void* stream) {
+  MB_CHECK_ARG(x && w, "layer_linear: null pointer");
+  MB_CHECK_ARG(T >= TG_BM && N % 128 == 0 && K % TG_BK == 0, "layer_linear: T=%lld N=%lld K=%lld (T >= 128, N %% 128, K %% 64)", (long long)T, (long long)N,
+               (long long)K);
+  MB_CHECK_ARG(rowscale == nullptr || (rs_pitch >= 1 && rs_group >= 1), "layer_linear: row scale pitch %lld group %lld", (long long)rs_pitch, (long long)rs_group);
+  EpiParams e;
+  int rc = layer_epilogue(e, bias, out, out32, N, epi, n_act, limit, alpha);
+  if (rc) return rc;
+  e.rowscale = rowscale;
+  e.rs_pitch = (int)rs_pitch;
+  e.rs_group = (int)rs_group;
+  GemmParams g;
+  g.a = x;
+  g.w = w;
+  g.T = (int)T;
+  g.N = (int)N;
+  g.K = (int)K;
+  g.epi = e;
+  return launch_gemm_tcgen05_prompt<EPI_LAYER>(g, (cudaStream_t)stream);
+}
+
+int mb200_layer_moe_sizes(int64_t T, int64_t n_experts, int64_t top, int64_t* rows_cap, int64_t* plan_words) {
+  MB_CHECK_ARG(T >= 1 && n_experts >= 1 && top >= 1, "layer_moe_sizes: bad arguments");
+  if (rows_cap) *rows_cap = moe_row_cap(T * top, n_experts, TG_BM);
+  if (plan_words) *plan_words = moe_plan_words(T * top, n_experts, TG_BM);
+  return MB200_OK;
+}
+
+int mb200_layer_moe(const void* hn, const void* w13, const void* w2, const int32_t* idx, const float* wsel, int64_t T, int64_t dim, int64_t ff, int64_t n_experts,
+                    int64_t top, int epi, float limit, float alpha, int32_t* slot, int32_t* plan, void* xs, float* row_w, void* act, float* rows32, float* y32,
+                    int add, void* stream) {
+  MB_CHECK_ARG(hn && w13 && w2 && idx && wsel && slot && plan && xs && row_w && act && rows32 && y32, "layer_moe: null pointer");
+  MB_CHECK_ARG(epi == LAYER_GLU || epi == LAYER_SWIGLU || epi == LAYER_GEGLU || epi == LAYER_RELU2, "layer_moe: step %d", epi);
+  const int64_t units = epi == LAYER_RELU2 ? ff : 2 * ff;  // weight rows of an expert's first Linear
+  MB_CHECK_ARG(T >= 1 && top >= 1 && n_experts >= 1 && n_experts <= MB200_LAYER_MOE_MAX_EXPERTS && dim % 128 == 0 && ff % 64 == 0 && units % 128 == 0 && T <= 65535,
+               "layer_moe: T=%lld width=%lld ff=%lld E=%lld top=%lld", (long long)T, (long long)dim, (long long)ff, (long long)n_experts, (long long)top);
+  cudaStream_t st = (cudaStream_t)stream;
+  const int64_t pairs = T * top, cap = moe_tile_cap(pairs, n_experts, TG_BM), rows_cap = cap * TG_BM;
+  const size_t plan_smem = ((size_t)n_experts * MP_THREADS + 2 * n_experts + 1) * sizeof(int32_t);
+  MB_CHECK_CUDA(cudaFuncSetAttribute(moe_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan_smem));
+  moe_plan_kernel<<<1, MP_THREADS, plan_smem, st>>>(idx, (int)pairs, (int)n_experts, TG_BM, 0, 1, (int)cap, slot, plan);
+  MB_CHECK_LAUNCH("moe_plan_kernel");
+  layer_moe_gather_kernel<<<(unsigned)ceil_div(pairs, 8), 256, 0, st>>>((const uint4*)hn, wsel, slot, (int)pairs, (int)top, (int)(dim / 8), (uint4*)xs, row_w);
+  MB_CHECK_LAUNCH("layer_moe_gather_kernel");
+  EpiParams e1, e2;
+  int rc = layer_epilogue(e1, nullptr, act, nullptr, units, epi, 0, limit, alpha);
+  if (rc) return rc;
+  e1.rowscale = row_w;  // one weight per row
+  e1.rs_pitch = 1;
+  e1.rs_group = (int)units;
+  rc = launch_grouped_packed(xs, rows_cap, dim, units, w13, n_experts * units, dim, units, 0, pairs, n_experts, plan, e1, st);
+  if (rc) return rc;
+  rc = layer_epilogue(e2, nullptr, nullptr, rows32, dim, LAYER_F32, 0, 0.f, 0.f);
+  if (rc) return rc;
+  rc = launch_grouped_packed(act, rows_cap, ff, dim, w2, dim, n_experts * ff, 0, ff, pairs, n_experts, plan, e2, st);
+  if (rc) return rc;
+  layer_moe_combine_kernel<<<dim3((unsigned)ceil_div(dim / 4, 256), (unsigned)T), 256, 0, st>>>((const float4*)rows32, slot, (float4*)y32, (int)T, (int)top,
+                                                                                            (int)(dim / 4), add);
+  MB_CHECK_LAUNCH("layer_moe_combine_kernel");
+  return MB200_OK;
+}
+
 // ---- NVLink peer buffers for the expert-parallel exchange: plain CUDA IPC on cudaMalloc'ed memory ------------------------------
 int mb200_comm_alloc(size_t bytes, void** ptr_out) {
   MB_CHECK_ARG(ptr_out && bytes > 0, "comm_alloc: bad arguments");

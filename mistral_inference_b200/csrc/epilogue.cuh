@@ -14,7 +14,11 @@ enum EpiMode : int {
   EPI_SWIGLU = 3,    // g[t, n/2] = bf16( bf16(silu(bf16(acc0))) * bf16(acc1) )   (transformer_layers.py:106)
   EPI_QKV_ROPE = 4,  // split into q/k/v, rotate q,k pairs, optional ring scatter  (transformer_layers.py:66-70, cache.py:91-92)
   EPI_MOE_SCALE = 5, // yw[row, n] = bf16( w[row] * bf16(acc) ), stored on every rank of an expert-parallel group  (moe.py:31)
+  EPI_LAYER = 6,     // the Linears of layered decoders: bias, then the step named by EpiParams::layer (LayerEpi)
 };
+
+// What follows a layered decoder's Linear (numbers shared with csrc/hybrid/hybrid_linear.cuh, which states the formulas).
+enum LayerEpi : int { LAYER_STORE = 0, LAYER_RESIDUAL = 1, LAYER_GLU = 2, LAYER_F32 = 3, LAYER_SWIGLU = 4, LAYER_RESIDUAL_SCALED = 5, LAYER_RELU2 = 6, LAYER_GEGLU = 7 };
 
 constexpr int kMaxPeers = 8;
 
@@ -38,6 +42,12 @@ struct EpiParams {
   const void* row_w = nullptr;  // bf16 [rows]
   void* peer_out[kMaxPeers] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   int n_peers = 0;
+  // EPI_LAYER
+  int layer = 0, n_act = 0;              // LayerEpi; columns below n_act go through SiLU (LAYER_STORE)
+  float limit = 0.f, alpha = 0.f;
+  const void* bias = nullptr;            // bf16 [N] or null
+  const float* rowscale = nullptr;       // fp32 [T, rs_pitch] or null: hidden unit c of row t is scaled by rowscale[t, c / rs_group]
+  int rs_pitch = 0, rs_group = 1;
 };
 
 template <int MODE>
@@ -123,9 +133,183 @@ __device__ __forceinline__ void epi_prefetch128(const EpiParams& p, int t, int n
   }
 }
 
+// EPI_LAYER.  The step is chosen at run time (uniform over the launch): one kernel per tile shape serves every layered decoder.  The
+// choice is made once per 32 columns, never inside a loop over them: with the branches inside, the chains of exponential and
+// reciprocal ran one after the other and a tile's epilogue took longer than its MMAs (gate/up of 4096 x 28672 x 4096: 1015 us against
+// 642 us for the plain store).  The Linear's sum (+ bias) is rounded to bf16 once before the step, except for fp32 results.
+//
+// sigmoid(x) with one ex2.approx and one rcp.approx: the argument's product with log2(e) is carried in two parts, so the relative error
+// stays at a few 2^-23 for every x (expf and a rounded division give the same).  A NaN argument gives a number: callers multiply by x.
+__device__ __forceinline__ float layer_sigmoid(float x) {
+  const float z = fminf(fmaxf(x, -120.f), 120.f);
+  const float hi = z * -1.4426950408889634f, lo = fmaf(z, -1.4426950408889634f, -hi);
+  float e, r;
+  asm("ex2.approx.f32 %0, %1;" : "=f"(e) : "f"(hi));
+  e = fmaf(e, lo * 0.6931471805599453f, e);
+  if (hi > 127.f) e = INFINITY;  // (infinity times a zero or negative lo must not turn into something else)
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(1.f + e));
+  return r;
+}
+__device__ __forceinline__ float layer_gelu(float z) { return 0.5f * z * (1.f + tanhf(0.7978845608028654f * fmaf(0.044715f * z * z, z, z))); }
+
+__device__ __forceinline__ bool layer_step_is_f32(int step) { return step == LAYER_F32 || step == LAYER_RESIDUAL || step == LAYER_RESIDUAL_SCALED; }
+
+__device__ __forceinline__ void layer_sums(const EpiParams& p, int n, const uint32_t (&v)[32], float (&x)[32]) {
+#pragma unroll
+  for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(v[j]);
+  if (p.bias != nullptr) {
+    const uint4* b4 = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.bias) + n);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const uint4 b = __ldg(b4 + q);
+      const uint32_t u[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        x[8 * q + 2 * j] += bf16lo(u[j]);
+        x[8 * q + 2 * j + 1] += bf16hi(u[j]);
+      }
+    }
+  }
+}
+
+// fp32 results and the fp32 residual stream, for the 32 rows t0 .. of one warp (all lanes call; rows from `rows` on are not stored).  A
+// thread owns a row of the accumulator, but 16-byte accesses of 32 different rows are half a sector each: the 32 x 32 block goes
+// through 4 KB of shared memory (the warp's own; 16-byte units XORed with the row: no bank conflicts) and out as whole 128-byte lines.
+__device__ __forceinline__ void epi_layer32_f32(const EpiParams& p, int t0, int rows, int n, const uint32_t (&v)[32], float4* stg) {
+  const int lane = (int)(threadIdx.x & 31), step = p.layer;
+  float4* const base = reinterpret_cast<float4*>(p.out_f32 + (int64_t)t0 * p.ld_out + n) + (lane & 7);
+  const int64_t pitch = p.ld_out / 4;
+  float4 r[8];
+  if (step != LAYER_F32) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int row = 4 * i + (lane >> 3);
+      if (row < rows) r[i] = base[row * pitch];
+    }
+  }
+  float x[32];
+  layer_sums(p, n, v, x);
+  if (step == LAYER_F32) {
+    if (p.limit > 0.f) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) x[j] = p.limit * tanhf(x[j] / p.limit);
+    }
+    const float f = p.alpha != 0.f ? p.alpha : 1.f;
+#pragma unroll
+    for (int j = 0; j < 32; ++j) x[j] *= f;
+  } else {
+#pragma unroll
+    for (int j = 0; j < 32; ++j) x[j] = round_bf16(x[j]);
+  }
+  __syncwarp();
+#pragma unroll
+  for (int q = 0; q < 8; ++q) stg[lane * 8 + (q ^ (lane & 7))] = make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
+  __syncwarp();
+  const float f = step == LAYER_RESIDUAL_SCALED ? p.alpha : 1.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int row = 4 * i + (lane >> 3);
+    float4 o = stg[row * 8 + ((lane & 7) ^ (row & 7))];
+    if (row < rows) {
+      if (step != LAYER_F32) o = make_float4(r[i].x + f * o.x, r[i].y + f * o.y, r[i].z + f * o.z, r[i].w + f * o.w);
+      base[row * pitch] = o;
+    }
+  }
+}
+
+// the bf16 results: row t, columns n .. n + 31 of the accumulator
+__device__ __forceinline__ void epi_layer32_bf16(const EpiParams& p, int t, int n, const uint32_t (&v)[32]) {
+  const int step = p.layer;
+  float x[32];
+  layer_sums(p, n, v, x);
+#pragma unroll
+  for (int j = 0; j < 32; ++j) x[j] = round_bf16(x[j]);
+  if (step == LAYER_STORE || step == LAYER_RELU2) {
+    if (step == LAYER_STORE) {
+      if (n + 32 <= p.n_act) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) x[j] *= layer_sigmoid(x[j]);
+      } else if (n < p.n_act) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+          if (n + j < p.n_act) x[j] *= layer_sigmoid(x[j]);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        const float y = fmaxf(x[j], 0.f);
+        x[j] = y * y;
+      }
+      if (p.rowscale != nullptr) {
+        const float* rs = p.rowscale + (int64_t)t * p.rs_pitch;
+        const int g = n / p.rs_group;
+        if ((n + 31) / p.rs_group == g) {
+          const float f = rs[g];
+#pragma unroll
+          for (int j = 0; j < 32; ++j) x[j] = f == 0.f ? 0.f : x[j] * f;
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) x[j] *= rs[(n + j) / p.rs_group];
+        }
+      }
+    }
+    uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out) + (int64_t)t * p.ld_out + n);
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      dst[q] = make_uint4(pack2_rn(x[8 * q], x[8 * q + 1]), pack2_rn(x[8 * q + 2], x[8 * q + 3]), pack2_rn(x[8 * q + 4], x[8 * q + 5]),
+                          pack2_rn(x[8 * q + 6], x[8 * q + 7]));
+    return;
+  }
+  // gated units: 16 (gate, up) pairs -> 16 outputs
+  const int c = n >> 1;
+  uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out) + (int64_t)t * p.ld_out + c);
+  float s0 = 1.f;
+  float s[16];
+  bool one = true;  // one scale for the 16 outputs
+  if (p.rowscale != nullptr) {
+    const float* row = p.rowscale + (int64_t)t * p.rs_pitch;
+    const int g = c / p.rs_group;
+    one = (c + 15) / p.rs_group == g;
+    if (one) {
+      s0 = row[g];
+      if (s0 == 0.f) {  // an expert that the token did not choose: nothing of it counts, not even an infinity
+        dst[0] = dst[1] = make_uint4(0, 0, 0, 0);
+        return;
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) s[j] = row[(c + j) / p.rs_group];
+    }
+  }
+  if (one) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) s[j] = s0;
+  }
+  if (step == LAYER_GLU) {  // the scale multiplies the expert's INPUT: gate and up, before the clamps
+    const float limit = p.limit, alpha = p.alpha;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const float g = fminf(x[2 * j] * s[j], limit), u = fminf(fmaxf(x[2 * j + 1] * s[j], -limit), limit);
+      x[j] = g * layer_sigmoid(alpha * g) * (u + 1.f);
+    }
+  } else if (step == LAYER_SWIGLU) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) x[j] = x[2 * j] * layer_sigmoid(x[2 * j]) * x[2 * j + 1] * s[j];
+  } else {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) x[j] = layer_gelu(x[2 * j]) * x[2 * j + 1] * s[j];
+  }
+#pragma unroll
+  for (int q = 0; q < 2; ++q)
+    dst[q] = make_uint4(pack2_rn(x[8 * q], x[8 * q + 1]), pack2_rn(x[8 * q + 2], x[8 * q + 3]), pack2_rn(x[8 * q + 4], x[8 * q + 5]),
+                        pack2_rn(x[8 * q + 6], x[8 * q + 7]));
+}
+
 template <int MODE>
 __device__ __forceinline__ void epi_chunk32(const EpiParams& p, int t, int n, const uint32_t (&v)[32]) {
-  if constexpr (MODE == EPI_STORE || MODE == EPI_RESIDUAL) {
+  if constexpr (MODE == EPI_LAYER) {
+    epi_layer32_bf16(p, t, n, v);  // (fp32 results: epi_layer32_f32, by whole warps)
+  } else if constexpr (MODE == EPI_STORE || MODE == EPI_RESIDUAL) {
     uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out) + (int64_t)t * p.ld_out + n);
     uint32_t o[16];
     if constexpr (MODE == EPI_RESIDUAL) {

@@ -64,6 +64,7 @@ struct TgCfg {
   static constexpr int kStages = (TA < 128 || BN < 128) ? (kShortRingStages < 3 ? 3 : (kShortRingStages > kMaxStages ? kMaxStages : kShortRingStages))
                                                         : (BN == 128 ? 6 : 4);
   static constexpr int kSmem = kStages * kStageBytes + kSlack + 1024 /*align*/ + 512 /*barriers*/;
+  static constexpr int kSmemLayer = kSmem + 4 * 4096;  // EPI_LAYER: 4 KB per epilogue warp to turn fp32 blocks (epi_layer32_f32)
   static constexpr int kTmemCols = 2 * BN <= 32 ? 32 : (2 * BN <= 64 ? 64 : (2 * BN <= 128 ? 128 : (2 * BN <= 256 ? 256 : 512)));  // 2 accumulators
   // Instruction descriptor (cute::UMMA::InstrDescriptor): D = F32, A = B = BF16, both K-major, N >> 3 at bit 17, M >> 4 at bit 24
   static constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TG_BM >> 4) << 24);
@@ -72,6 +73,9 @@ struct TgCfg {
 struct TcGemmParams {
   int T, N, K;
   EpiParams epi;
+  // grouped, experts packed in ONE matrix (layered decoders): expert e's weights start w_n * e rows and w_k * e columns into the single
+  // tensor map; w_n = w_k = 0: a tensor map per expert
+  int w_n = 0, w_k = 0;
 };
 
 // ---- PTX wrappers ---------------------------------------------------------------------------------
@@ -274,7 +278,10 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
         int mu, nt;
         tile_mn(tile, mu, nt);
         const int m0 = GROUPED ? grouped_m0(mu, store_unused) : (mu * CL + rank) * TG_BM, n0 = nt * TG_BN;
-        const CUtensorMap* wmap = GROUPED ? map_w_base + tile_expert[mu] : map_w_base;
+        const int expert = GROUPED ? tile_expert[mu] : 0;
+        const bool packed = GROUPED && (p.w_n | p.w_k) != 0;
+        const CUtensorMap* wmap = map_w_base + (packed ? 0 : expert);
+        const int wr = n0 + (packed ? expert * p.w_n : 0), wc = packed ? expert * p.w_k : 0;
         for (int kb = 0; kb < num_k; ++kb, ++it) {
           const uint32_t s = it % TG_STAGES, par = (it / TG_STAGES) & 1;
           mbar_wait(&empty[s], par ^ 1, 11, it);
@@ -282,10 +289,10 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
           uint8_t* sa = smem + s * TG_STAGE_BYTES;
           tma_load_2d(sa, &map_a, &full[s], kb * TG_BK, m0);
           if (CL > 1)
-            tma_load_2d_multicast(sa + TG_A_BYTES + rank * (TG_B_BYTES / CL), wmap, &full[s], kb * TG_BK, n0 + rank * (TG_BN / CL),
+            tma_load_2d_multicast(sa + TG_A_BYTES + rank * (TG_B_BYTES / CL), wmap, &full[s], wc + kb * TG_BK, wr + rank * (TG_BN / CL),
                                   (uint16_t)((1u << CL) - 1));
           else
-            tma_load_2d(sa + TG_A_BYTES, wmap, &full[s], kb * TG_BK, n0);
+            tma_load_2d(sa + TG_A_BYTES, wmap, &full[s], wc + kb * TG_BK, wr);
         }
       }
     }
@@ -333,7 +340,25 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
       const uint32_t trow = tmem_base + ((uint32_t)lane_base << 16) + acc * TG_BN;
       uint32_t va[32], vb[32];
       tmem_ld_32x32b_x32_nowait(trow, va);
-      if constexpr (TG_BN == 32) {
+      if constexpr (MODE == EPI_LAYER) {
+        const bool f32 = layer_step_is_f32(p.epi.layer);
+        const int rows = store ? max(0, min(32, p.T - m0 - lane_base)) : 0;
+        float4* stg = reinterpret_cast<float4*>(reinterpret_cast<uint8_t*>(full) + 512) + (warp & 3) * 256;
+        auto chunk = [&](int n, const uint32_t (&v)[32]) {
+          if (f32)
+            epi_layer32_f32(p.epi, m0 + lane_base, rows, n, v, stg);
+          else if (t < p.T)
+            epi_layer32_bf16(p.epi, t, n, v);
+        };
+#pragma unroll 1
+        for (int c = 0; c < TG_BN / 32; ++c) {
+          tmem_wait_ld();
+#pragma unroll
+          for (int j = 0; j < 32; ++j) vb[j] = va[j];
+          if (c + 1 < TG_BN / 32) tmem_ld_32x32b_x32_nowait(trow + (c + 1) * 32, va);
+          chunk(n0 + c * 32, vb);
+        }
+      } else if constexpr (TG_BN == 32) {
         tmem_wait_ld();
         if (t < p.T) epi_chunk32<MODE>(p.epi, t, n0, va);
       } else {
@@ -428,6 +453,7 @@ inline int tcgen05_forced_bn() {
 template <int MODE, int BN>
 int launch_gemm_tcgen05_bn(const GemmParams& g, bool pair, int sms, cudaStream_t stream) {
   using Cfg = TgCfg<BN>;
+  constexpr int kSmem = MODE == EPI_LAYER ? Cfg::kSmemLayer : Cfg::kSmem;
   CUtensorMap map_a, map_w;
   int rc = make_tensor_map_2d(&map_a, g.a, g.T, g.K, TG_BM);
   if (rc) return rc;
@@ -440,11 +466,11 @@ int launch_gemm_tcgen05_bn(const GemmParams& g, bool pair, int sms, cudaStream_t
   p.epi = g.epi;
   if (pair) {
     const int supers = ceil_div(ceil_div(g.T, TG_BM), 2) * (g.N / BN), pairs = sms / 2;
-    MB_CHECK_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<MODE, 2, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
+    MB_CHECK_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<MODE, 2, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2u * (unsigned)(supers < pairs ? supers : pairs));
     cfg.blockDim = dim3(TG_THREADS);
-    cfg.dynamicSmemBytes = Cfg::kSmem;
+    cfg.dynamicSmemBytes = kSmem;
     cfg.stream = stream;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -458,8 +484,8 @@ int launch_gemm_tcgen05_bn(const GemmParams& g, bool pair, int sms, cudaStream_t
     return MB200_OK;
   }
   const int tiles = ceil_div(g.T, TG_BM) * (g.N / BN);
-  MB_CHECK_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<MODE, 1, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
-  gemm_tcgen05_kernel<MODE, 1, BN><<<tiles < sms ? tiles : sms, TG_THREADS, Cfg::kSmem, stream>>>(map_a, map_w, p);
+  MB_CHECK_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<MODE, 1, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+  gemm_tcgen05_kernel<MODE, 1, BN><<<tiles < sms ? tiles : sms, TG_THREADS, kSmem, stream>>>(map_a, map_w, p);
   MB_CHECK_LAUNCH("gemm_tcgen05_kernel");
   return MB200_OK;
 }
@@ -518,15 +544,13 @@ int launch_gemm_tcgen05_small_ta(const GemmParams& g, int sms, cudaStream_t stre
   }
 }
 
+// T >= TG_BM
 template <int MODE>
-int launch_gemm_tcgen05(const GemmParams& g, cudaStream_t stream) {
+int launch_gemm_tcgen05_prompt(const GemmParams& g, cudaStream_t stream) {
   const bool pair = tcgen05_cluster_enabled() && g.T >= 4 * TG_BM;
   int dev = 0, sms = 0;
   MB_CHECK_CUDA(cudaGetDevice(&dev));
   MB_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  if (g.T <= 32) return launch_gemm_tcgen05_small_ta<MODE, 32>(g, sms, stream);
-  if (g.T <= 64) return launch_gemm_tcgen05_small_ta<MODE, 64>(g, sms, stream);
-  if (g.T < TG_BM) return launch_gemm_tcgen05_small_ta<MODE, 128>(g, sms, stream);
   // 128-wide tiles only when 256-wide ones cannot fill the machine once (small T or N).  Measured at T = 4096: narrowing the
   // N = 4096 GEMMs (512 tiles = 3.46 rounds -> 1024 tiles = 6.9 rounds) makes them SLOWER (wo+w2 237 -> 343 us on average):
   // per flop the narrow tile pulls 1.5x the bytes out of L2, and that, not tile quantisation, is the binding limit there.
@@ -542,6 +566,17 @@ int launch_gemm_tcgen05(const GemmParams& g, cudaStream_t stream) {
   if (bn == 192) return launch_gemm_tcgen05_bn<MODE, 192>(g, pair, sms, stream);
   const bool narrow = bn == 128;
   return narrow ? launch_gemm_tcgen05_bn<MODE, 128>(g, pair, sms, stream) : launch_gemm_tcgen05_bn<MODE, 256>(g, pair, sms, stream);
+}
+
+template <int MODE>
+int launch_gemm_tcgen05(const GemmParams& g, cudaStream_t stream) {
+  if (g.T >= TG_BM) return launch_gemm_tcgen05_prompt<MODE>(g, stream);
+  int dev = 0, sms = 0;
+  MB_CHECK_CUDA(cudaGetDevice(&dev));
+  MB_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  if (g.T <= 32) return launch_gemm_tcgen05_small_ta<MODE, 32>(g, sms, stream);
+  if (g.T <= 64) return launch_gemm_tcgen05_small_ta<MODE, 64>(g, sms, stream);
+  return launch_gemm_tcgen05_small_ta<MODE, 128>(g, sms, stream);
 }
 
 }  // namespace mb200

@@ -514,8 +514,9 @@ class LatentAttention(nn.Module):
 class MoeFeedForward(nn.Module):
     """Mixture of gated experts with an fp32 softmax router (args.MoeFfArgs).  Packed weights: w13 [E * 2 * ff, width], expert after
     expert with gate and up rows interleaved; w2 [width, E * ff], expert e's down projection in columns e*ff ..; identity experts have
-    no weights.  Few tokens (decode) stream the chosen experts only; prompts run all experts as two Linears, the first one's
-    epilogue scaling every expert's hidden units by the token's routing weight (0 when not chosen)."""
+    no weights.  Few tokens (decode) stream the chosen experts only; bf16 prompts of suitable sizes compute the chosen (token, expert) rows as
+    grouped GEMMs; other prompts run all experts as two Linears, the first one's epilogue scaling every expert's hidden units by the token's
+    routing weight (0 when not chosen)."""
 
     def __init__(self, width: int, a: MoeFfArgs):
         super().__init__()
@@ -532,8 +533,10 @@ class MoeFeedForward(nn.Module):
         if hn.shape[0] <= self.sparse_max_tokens:
             y32 = _h.moe_sparse(hn, self.w13, self.w2, idx, wsel, a.experts, a.ff)
         else:
-            act = _h.linear_swiglu(hn, self.w13, rowscale=dense, group=a.ff)
-            y32 = _h.linear(act, self.w2, epi=_h.EPI_F32)
+            if _h.moe_grouped_ok(hn, self.w13, self.w2, a.experts, a.ff):
+                y32 = _h.moe_grouped(hn, self.w13, self.w2, idx, wsel, a.experts, a.ff, _h.EPI_SWIGLU)
+            else:
+                y32 = _h.linear(_h.linear_swiglu(hn, self.w13, rowscale=dense, group=a.ff), self.w2, epi=_h.EPI_F32)
             if a.identity:
                 _h.rows_axpy(y32, hn, dense, a.experts)
         if post is None:
@@ -845,6 +848,8 @@ class ScaledInputMoe(nn.Module):
         dense, idx, wsel = _h.moe_route(hn, self.router, None, 1, 1, a.top, score=1)
         if hn.shape[0] <= self.sparse_max_tokens:
             _h.moe_sparse(hn, self.w13, self.w2, idx, wsel, a.experts, a.ff, glu=True, limit=a.limit, alpha=a.alpha, add_to=x32)
+        elif _h.moe_grouped_ok(hn, self.w13, self.w2, a.experts, a.ff):
+            _h.moe_grouped(hn, self.w13, self.w2, idx, wsel, a.experts, a.ff, _h.EPI_GLU, a.limit, a.alpha, add_to=x32)
         else:
             act = _h.linear_glu(hn, self.w13, a.limit, a.alpha, rowscale=dense, group=a.ff)
             _h.linear(act, self.w2, epi=_h.EPI_RESIDUAL, residual=x32)
@@ -1105,6 +1110,8 @@ class Relu2Moe(nn.Module):
         dense, idx, wsel = _h.moe_route(hn, self.router, None, 1, 1, a.top, score=0, scale=a.router_scale)
         if hn.shape[0] <= self.sparse_max_tokens:
             y32 = _h.moe_sparse(hn, self.w_up, self.w2, idx, wsel, a.experts, a.ff, glu=2)
+        elif _h.moe_grouped_ok(hn, self.w_up, self.w2, a.experts, a.ff):
+            y32 = _h.moe_grouped(hn, self.w_up, self.w2, idx, wsel, a.experts, a.ff, _h.EPI_RELU2)
         else:
             y32 = _h.linear(_h.linear_relu2(hn, self.w_up, rowscale=dense, group=a.ff), self.w2, epi=_h.EPI_F32)
         if self.shared is not None:
@@ -1290,6 +1297,8 @@ class GroupedMoe(nn.Module):
                                                group_two=True, renorm=True, w_gate=self.shared_gate)
         if hn.shape[0] <= self.sparse_max_tokens:
             _h.moe_sparse(hn, self.w13, self.w2, idx, wsel, a.experts, a.ff, add_to=x32)
+        elif _h.moe_grouped_ok(hn, self.w13, self.w2, a.experts, a.ff):
+            _h.moe_grouped(hn, self.w13, self.w2, idx, wsel, a.experts, a.ff, _h.EPI_SWIGLU, add_to=x32)
         else:
             _h.linear(_h.linear_swiglu(hn, self.w13, rowscale=dense, group=a.ff), self.w2, epi=_h.EPI_RESIDUAL, residual=x32)
         if self.shared is not None:
@@ -1340,6 +1349,8 @@ class ChosenSoftmaxMoe(nn.Module):
         dense, idx, wsel = _h.moe_route(hn, self.router, None, 1, 1, a.top, score=2, w_bias=self.router_bias, always=self.always)
         if hn.shape[0] <= self.sparse_max_tokens:
             y32 = _h.moe_sparse(hn, self.w13, self.w2, idx, wsel, self.total, a.ff, add_to=x32 if post is None else None)
+        elif _h.moe_grouped_ok(hn, self.w13, self.w2, self.total, a.ff):
+            y32 = _h.moe_grouped(hn, self.w13, self.w2, idx, wsel, self.total, a.ff, _h.EPI_SWIGLU, add_to=x32 if post is None else None)
         elif post is None:
             y32 = _h.linear(_h.linear_swiglu(hn, self.w13, rowscale=dense, group=a.ff), self.w2, epi=_h.EPI_RESIDUAL, residual=x32)
         else:
