@@ -67,6 +67,11 @@ int mbh_attn_bias(const void* q, const void* cache_k, const void* cache_v, const
 int mbh_lightning_scan(const void* qkvg, void* state, const void* decay, const void* q_start, const void* seqpos, const void* slots, void* o32,
                        int64_t B, int64_t H, int64_t d, int64_t e, int dt, void* stream);
 
+/* The same over prompts in chunks of tokens, on tensor cores: bf16 storage, d 32, 64 or 128, e a multiple of 32, qkvg 16-byte aligned.
+ * State, decayed values and decayed scores enter the products as three bf16 parts each: fp32 throughout. */
+int mbh_lightning_prompt(const void* qkvg, void* state, const void* decay, const void* q_start, const void* seqpos, const void* slots, void* o32,
+                         int64_t B, int64_t H, int64_t d, int64_t e, void* stream);
+
 /* y[t, :] = rms_norm(o32[t, :N]; eps) * w * sigmoid(g[t * g_pitch + g_off + :N]). */
 int mbh_gated_headnorm(const void* o32, const void* w, const void* g, int64_t g_pitch, int64_t g_off, void* y, int64_t T, int64_t N, float eps,
                        int dt, void* stream);

@@ -30,6 +30,7 @@ _SIGNATURES = {
     "mbh_attn_prep": (c_int, [P, P, P, P, P, P, P, P, P, P, c_int, I, I, I, I, I, F, F, I, c_int, P]),
     "mbh_attn_bias": (c_int, [P, P, P, P, I, P, P, P, P, I, I, I, I, I, I, I, F, I, I, P, c_int, P]),
     "mbh_lightning_scan": (c_int, [P, P, P, P, P, P, P, I, I, I, I, c_int, P]),
+    "mbh_lightning_prompt": (c_int, [P, P, P, P, P, P, P, I, I, I, I, P]),
     "mbh_gated_headnorm": (c_int, [P, P, P, I, I, P, I, I, F, c_int, P]),
     "mbh_embed_add": (c_int, [P, P, F, P, I, I, c_int, P]),
     "mbh_layernorm": (c_int, [P, P, P, P, P, I, I, F, c_int, P]),
@@ -212,8 +213,16 @@ def attn_splits(T: int, H: int, W: int, n_sm: int = 148) -> int:
     return int(max(1, min((2 * n_sm + T * H - 1) // (T * H), (W + 511) // 512, 32)))
 
 
-def lightning_scan(qkvg, state, decay, q_start, seqpos, slots, o32, B: int, H: int, d: int, e: int) -> None:
+LIGHTNING_CHUNK_MIN = 12  # prompts (portions) at least this long run in chunks on tensor cores where the sizes allow
+
+
+def lightning_scan(qkvg, state, decay, q_start, seqpos, slots, o32, B: int, H: int, d: int, e: int, longest: int = 1) -> None:
+    """longest: tokens of the longest sequence of this call (a long one in bf16 runs in chunks; the token-by-token scan otherwise)."""
     assert state.dtype == torch.float32 and decay.dtype == torch.float32 and o32.dtype == torch.float32
+    if longest >= LIGHTNING_CHUNK_MIN and qkvg.dtype == torch.bfloat16 and d in (32, 64, 128) and e % 32 == 0 and _aligned(qkvg):
+        _check(lib().mbh_lightning_prompt(_ptr(qkvg), _ptr(state), _ptr(decay), _ptr(q_start), _ptr(seqpos), _ptr(slots), _ptr(o32), B, H, d, e, _stream()),
+               "mbh_lightning_prompt")
+        return
     _check(lib().mbh_lightning_scan(_ptr(qkvg), _ptr(state), _ptr(decay), _ptr(q_start), _ptr(seqpos), _ptr(slots), _ptr(o32), B, H, d, e,
                                     dt_of(qkvg.dtype), _stream()), "mbh_lightning_scan")
 

@@ -1,6 +1,7 @@
 // C ABI of libmb200_hybrid.so: the kernels of layered decoders (per-layer mixer kinds, fp32 residual stream, bf16 or fp32
 // storage).  Declarations: include/mistral_b200_hybrid.h.  `dt` selects the storage type of activations and weights:
 // 0 = bf16, 1 = fp32.  Every call returns 0 or a CUDA error code; mbh_last_error() gives the text.
+#include "hybrid_lightning.cuh"
 #include "hybrid_linear.cuh"
 #include "hybrid_mixers.cuh"
 #include "hybrid_attn_flash.cuh"
@@ -299,6 +300,18 @@ int mbh_lightning_scan(const void* qkvg, void* state, const void* decay, const v
     cudaError_t err = cudaSuccess;
     DISPATCH(dt, err = launch_lightning<ST>(a, (cudaStream_t)stream));
     return err ? fail(err, "mbh_lightning_scan") : 0;
+}
+
+int mbh_lightning_prompt(const void* qkvg, void* state, const void* decay, const void* q_start, const void* seqpos, const void* slots, void* o32,
+                         int64_t B, int64_t H, int64_t d, int64_t e, void* stream) {
+    if (B == 0) return 0;
+    if ((d != 32 && d != 64 && d != 128) || e <= 0 || e % LC_E) return bad("mbh_lightning_prompt: key size 32, 64 or 128, value size a multiple of 32");
+    if (reinterpret_cast<uintptr_t>(qkvg) % 16 || reinterpret_cast<uintptr_t>(o32) % 8) return bad("mbh_lightning_prompt: unaligned pointers");
+    LightningArgs a{qkvg, (float*)state, (const float*)decay, (const int*)q_start, (const int*)seqpos, (const int*)slots, (float*)o32,
+                    (int)B, (int)H, (int)d, (int)e};
+    cudaStream_t st = (cudaStream_t)stream;
+    const cudaError_t err = d == 128 ? run_lightning_chunk<128>(a, st) : d == 64 ? run_lightning_chunk<64>(a, st) : run_lightning_chunk<32>(a, st);
+    return err ? fail(err, "mbh_lightning_prompt") : 0;
 }
 
 int mbh_gated_headnorm(const void* o32, const void* w, const void* g, int64_t g_pitch, int64_t g_off, void* y, int64_t T, int64_t N, float eps,

@@ -355,7 +355,8 @@ class LightningMixer(nn.Module):
         T = hn.shape[0]
         qkvg = _h.linear(hn, self.wqkvg, n_act=2 * self.nqk + self.nv)
         o32 = torch.empty(T, self.nv, dtype=torch.float32, device=hn.device)
-        _h.lightning_scan(qkvg, view.state, self.decay, md.q_start, md.seqpos, md.slots, o32, len(md.seqlens), a.heads, a.dim, a.vdim)
+        _h.lightning_scan(qkvg, view.state, self.decay, md.q_start, md.seqpos, md.slots, o32, len(md.seqlens), a.heads, a.dim, a.vdim,
+                          longest=md.max_seqlen)
         y = _h.gated_headnorm(o32, self.norm, qkvg, qkvg.shape[1], 2 * self.nqk + self.nv, self.eps)
         project_out(y, self.wo, x32, post)
 

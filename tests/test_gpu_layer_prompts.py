@@ -54,3 +54,61 @@ def test_chosen_expert_rows(kind, T, width, ff, E, top, idle, monkeypatch):
     acc = base.clone()
     h.moe_grouped(hn, w13, w2, idx.to(DEV), wts, E, ff, epi, 1.5, 1.7, add_to=acc)
     assert torch.equal(acc, base + got), "blocks of tokens and the sum into a stream change nothing"
+
+
+def _scan64(q, k, v, decay, state, lens):
+    """o [T, H, e] and the final states of sum_j decay^(i-j) (q_i . k_j) v_j in float64, token by token."""
+    o, t = torch.empty(*v.shape, dtype=torch.float64, device=v.device), 0
+    for b, n in enumerate(lens):
+        for _ in range(n):
+            state[b] = decay[:, None, None] * state[b] + k[t][:, :, None] * v[t][:, None, :]
+            o[t] = (state[b] * q[t][:, :, None]).sum(1)
+            t += 1
+    return o, state
+
+
+@pytest.mark.parametrize("H,d,e", [(3, 128, 128), (2, 64, 96), (5, 32, 32)])
+@pytest.mark.parametrize("lens", [[64], [65, 1, 12], [200, 63], [16, 128, 129]])
+def test_lightning_chunks(H, d, e, lens):
+    """Chunk edges, ragged batches, rows in another order than the batch, states carried on: the chunked kernel against float64 and against the
+    token-by-token scan, which it must not be less exact than (products of fp32 numbers in three bf16 parts: 2^-21 on either side)."""
+    from mistral_inference_b200 import _abi_hybrid as h
+
+    g = torch.Generator().manual_seed(sum(lens) + d)
+    T, B = sum(lens), len(lens)
+    x = torch.randn(T, 2 * H * d + 2 * H * e, generator=g).bfloat16().to(DEV)
+    decay = torch.linspace(0.3, 1.0, H).to(DEV)
+    slots = torch.arange(B).flip(0).int().to(DEV)
+    start = torch.randn(B, H, d, e, generator=g).to(DEV)
+    seqpos = torch.tensor([0 if b == 0 else 7 for b in range(B)], dtype=torch.int32, device=DEV)
+    q_start = torch.tensor([0] + lens).cumsum(0).int().to(DEV)
+    q, k = (x[:, i * H * d:(i + 1) * H * d].double().view(T, H, d) for i in (0, 1))
+    v = x[:, 2 * H * d: 2 * H * d + H * e].double().view(T, H, e)
+    first = start.double()[slots.long()].clone()
+    first[0] = 0  # nothing before: whatever the row held does not count
+    ref, last = _scan64(q, k, v, decay.double(), first, lens)
+    got = []
+    for longest in (max(lens), 1):
+        state, o = start.clone(), torch.empty(T, H * e, dtype=torch.float32, device=DEV)
+        h.lightning_scan(x, state, decay, q_start, seqpos, slots, o, B, H, d, e, longest=max(longest, 12) if longest > 1 else 1)
+        got.append((rel(o, ref.flatten(1)), rel(state[slots.long()], last)))
+    assert got[0][0] < max(2 ** -21, 1.2 * got[1][0]) and got[0][1] < max(2 ** -21, 1.2 * got[1][1]), got
+
+
+def test_lightning_infinity_reaches_no_earlier_token():
+    from mistral_inference_b200 import _abi_hybrid as h
+
+    T, H, d, e = 150, 2, 64, 64
+    g = torch.Generator().manual_seed(3)
+    x = torch.randn(T, 2 * H * d + 2 * H * e, generator=g).bfloat16().to(DEV)
+    x[100, 2 * H * d + 5] = float("inf")  # head 0, column 5 of the values
+    decay, one = torch.full((H,), 0.9, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    q_start = torch.tensor([0, T], dtype=torch.int32, device=DEV)
+    outs = []
+    for longest in (T, 1):
+        state, o = torch.zeros(1, H, d, e, device=DEV), torch.empty(T, H * e, dtype=torch.float32, device=DEV)
+        h.lightning_scan(x, state, decay, q_start, one, one, o, 1, H, d, e, longest=longest)
+        outs.append((o, state))
+    for a, b in zip(*outs):
+        assert torch.equal(torch.isfinite(a), torch.isfinite(b)) and torch.equal(torch.isnan(a), torch.isnan(b))
+        assert rel(a[torch.isfinite(b)], b[torch.isfinite(b)].double()) < 1e-6
