@@ -213,7 +213,15 @@ int mb200_moe_grouped_ffn(const void* xs, const void* const* w13_host, const voi
  *     w2 [width, E * ff].  The weight multiplies the hidden units (GLU: the expert's input).  width % 128 == 0, ff % 64 == 0,
  *     T <= 65535.  Buffers (device, uninitialised): slot [T * top] int32, plan [plan_words] int32, xs [rows_cap, width] bf16,
  *     row_w [rows_cap] fp32, act [rows_cap, ff] bf16, rows32 [rows_cap, width] fp32.
+ * mb200_layer_attention: causal softmax attention of prompts (bf16, head size 128, H / KV query heads to a key/value head), every key and
+ *     value already in the ring: cache_k/v [blocks, W, KV, 128], sequence b in block slots[b], position p in row p (p < W).  Query i of
+ *     sequence b is at position seqpos[b] + i.  bias [n_tab, H] fp32 or NULL is added to the scaled scores by distance (larger distances take
+ *     the last row); n_tab at most mb200_layer_attention_max_table().  out [T, H * 128] bf16.
  */
+int mb200_layer_attention_max_table(void);
+int mb200_layer_attention(const void* q, const void* cache_k, const void* cache_v, const float* bias, int64_t n_tab, const int32_t* q_start, const int32_t* seqpos,
+                          const int32_t* slots, void* out, int64_t T, int64_t B, int64_t blocks, int64_t max_seqlen, int64_t W, int64_t n_heads,
+                          int64_t n_kv_heads, float scale, void* stream);
 #define MB200_LAYER_MOE_MAX_EXPERTS 48
 int mb200_layer_linear(const void* x, const void* w, const void* bias, void* out, float* out32, int64_t T, int64_t N, int64_t K, int epi, int64_t n_act,
                        float limit, float alpha, const float* rowscale, int64_t rs_pitch, int64_t rs_group, void* stream);

@@ -48,6 +48,9 @@ _SIGNATURES = {
                                       c_int64, c_int64, c_int64, c_int64, c_void_p, c_void_p, c_size_t, c_void_p]),
     "mb200_layer_linear": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int, c_int64, c_float, c_float, c_void_p,
                                    c_int64, c_int64, c_void_p]),
+    "mb200_layer_attention_max_table": (c_int, []),
+    "mb200_layer_attention": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64,
+                                      c_int64, c_int64, c_int64, c_float, c_void_p]),
     "mb200_layer_moe_sizes": (c_int, [c_int64, c_int64, c_int64, ctypes.POINTER(c_int64), ctypes.POINTER(c_int64)]),
     "mb200_layer_moe": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64, c_int64, c_int, c_float, c_float,
                                 c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p]),
@@ -279,6 +282,13 @@ def layer_linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor],
     T, K = x.shape
     _check(lib().mb200_layer_linear(_ptr(x), _ptr(w), _ptr(bias), _ptr(out), _ptr(out32), T, w.shape[0], K, epi, n_act, limit, alpha, _ptr(rowscale),
                                     rowscale.shape[1] if rowscale is not None else 0, group, _stream()), "mb200_layer_linear")
+
+
+def layer_attention(q, cache_k, cache_v, bias, q_start, seqpos, slots, out, B: int, max_seqlen: int, H: int, KV: int, scale: float) -> None:
+    """Prompt attention over a ring that holds every key, head size 128 (include/mistral_b200.h)."""
+    _check(lib().mb200_layer_attention(_ptr(q), _ptr(cache_k), _ptr(cache_v), _ptr(bias), bias.shape[0] if bias is not None else 0, _ptr(q_start), _ptr(seqpos),
+                                       _ptr(slots), _ptr(out), q.shape[0], B, cache_k.shape[0], max_seqlen, cache_k.shape[1], H, KV, scale, _stream()),
+           "mb200_layer_attention")
 
 
 LAYER_MOE_MAX_EXPERTS = 48

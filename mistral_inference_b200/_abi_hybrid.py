@@ -198,9 +198,18 @@ def attn_prep(qkv, qnorm, knorm, positions, cache_rows, q_out, cache_k, cache_v,
                                _stream()), "mbh_attn_prep")
 
 
+ATTN_TCGEN05_MIN = 48  # prompts (portions) at least this long fill enough of the tcgen05 kernel's 128-query tiles
+
+
 def attn_bias(q, cache_k, cache_v, bias_tab, positions, q_start, slots, out, B: int, W: int, H: int, G: int, d: int, e: int, scale: float,
-              n_tiles: int = 0, splits: int = 1) -> None:
-    """n_tiles = sum over sequences of ceil(len / 64) selects the tensor-core prompt kernel (bf16); 0 the exact fp32 one."""
+              n_tiles: int = 0, splits: int = 1, seqpos=None, longest: int = 0) -> None:
+    """n_tiles = sum over sequences of ceil(len / 64) selects a tensor-core prompt kernel (bf16); 0 the exact fp32 one.  With seqpos (tokens
+    before this call, per sequence) and the longest sequence's length, heads of 128 take the main library's tcgen05 kernel where it is built."""
+    if (n_tiles and seqpos is not None and longest >= ATTN_TCGEN05_MIN and d == e == 128 and q.dtype == torch.bfloat16 and scale > 0 and _aligned(q, cache_k, cache_v, out)
+            and cache_k.shape[1] == W and os.environ.get("MB200_HYBRID_GEMM", "1") != "0" and _abi.library_path().exists()
+            and (bias_tab is None or bias_tab.shape[0] <= _abi.lib().mb200_layer_attention_max_table())):
+        _abi.layer_attention(q, cache_k, cache_v, bias_tab, q_start, seqpos, slots, out, B, longest, H, G, scale)
+        return
     assert bias_tab is None or (bias_tab.dtype == torch.float32 and bias_tab.shape[1] == H)
     scratch = torch.empty(q.shape[0] * H * splits * (2 + e), dtype=torch.float32, device=q.device) if splits > 1 and n_tiles == 0 else None
     _check(lib().mbh_attn_bias(_ptr(q), _ptr(cache_k), _ptr(cache_v), _ptr(bias_tab), bias_tab.shape[0] if bias_tab is not None else 0, _ptr(positions), _ptr(q_start), _ptr(slots),

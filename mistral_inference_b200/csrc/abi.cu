@@ -6,7 +6,7 @@
 #include "attn_decode.cuh"
 #include "attn_decode_tma.cuh"
 #include "attn_prefill.cuh"
-#include "attn_prefill_tcgen05.cuh"
+#include "attn_prompt_tcgen05.cuh"
 #include "decode_megakernel.cuh"
 #include "elementwise.cuh"
 #include "gemm_mma.cuh"
@@ -20,6 +20,9 @@ namespace mb200 {
 thread_local char g_err[512] = "";
 static unsigned long long* g_mk_prof = nullptr;
 static unsigned long long* g_mk_prof_bar = nullptr;  // debug: decode megakernel phase timeline buffer (device)
+
+// the shortest longest sequence of a call from which prompt attention takes the tcgen05 kernel (128 queries a tile)
+constexpr int64_t MB200_ATTN_FIRST_MIN = 128, MB200_ATTN_PORTION_MIN = 48;
 
 constexpr size_t kWsHeader = 64 * 1024;  // persistent, zero-initialised by the caller once: self-resetting counters
 inline size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
@@ -218,8 +221,23 @@ int mb200_attn_prefill(const void* q, const void* k_new, const void* v_new, cons
   MB_CHECK_ARG(head_dim == kHeadDim, "attn_prefill: head_dim=%lld unsupported (128 only)", (long long)head_dim);
   MB_CHECK_ARG(n_heads % n_kv_heads == 0, "attn_prefill: H %% KV != 0");
   if (T == 0) return MB200_OK;
-  if (causal == 2 && tcgen05_attn_eligible(T, max_seqlen))  // first prefill: every key comes from the chunk -> tcgen05 / TMEM / TMA kernel
-    return launch_attn_prefill_tcgen05(q, k_new, v_new, q_start, out, T, B, max_seqlen, W, n_heads, n_kv_heads, (cudaStream_t)stream);
+  // Long enough prompts (first ones and portions): the tcgen05 kernel, 128 queries a tile.  Short ones keep the mma.sync kernel (64 queries a
+  // tile, twice the CTAs).
+  if (causal && tcgen05_attn_enabled() && max_seqlen >= (causal == 2 ? MB200_ATTN_FIRST_MIN : MB200_ATTN_PORTION_MIN)) {
+    FaParams f;
+    f.q_start = q_start;
+    f.seqpos = causal == 2 ? nullptr : seqpos;
+    f.slots = nullptr;
+    f.bias = nullptr;
+    f.n_tab = 0;
+    f.out = (bf16*)out;
+    f.B = (int)B;
+    f.W = f.window = (int)W;
+    f.H = (int)n_heads;
+    f.KV = (int)n_kv_heads;
+    f.scale_log2 = 0.08838834764831845f * 1.4426950408889634f;
+    return launch_attn_prompt_tcgen05(f, q, k_new, v_new, causal == 2 ? nullptr : cache_k, causal == 2 ? nullptr : cache_v, B, T, max_seqlen, (cudaStream_t)stream);
+  }
   AttnPrefillParams p;
   p.q = (const bf16*)q;
   p.k_new = (const bf16*)k_new;
@@ -417,6 +435,32 @@ int mb200_moe_grouped_ffn(const void* xs, const void* const* w13_host, const voi
 }
 
 // ---- Linears and mixtures of layered decoders ----------------------------------------------------------------------------------
+int mb200_layer_attention_max_table(void) { return FA_MAX_TAB; }
+
+int mb200_layer_attention(const void* q, const void* cache_k, const void* cache_v, const float* bias, int64_t n_tab, const int32_t* q_start, const int32_t* seqpos,
+                          const int32_t* slots, void* out, int64_t T, int64_t B, int64_t blocks, int64_t max_seqlen, int64_t W, int64_t n_heads,
+                          int64_t n_kv_heads, float scale, void* stream) {
+  MB_CHECK_ARG(q && cache_k && cache_v && q_start && seqpos && slots && out, "layer_attention: null pointer");
+  MB_CHECK_ARG(T >= 0 && B >= 1 && B <= 65535 && blocks >= 1 && W >= 1 && n_kv_heads >= 1 && n_heads % n_kv_heads == 0 && scale > 0.f,
+               "layer_attention: T=%lld B=%lld W=%lld H=%lld KV=%lld", (long long)T, (long long)B, (long long)W, (long long)n_heads, (long long)n_kv_heads);
+  MB_CHECK_ARG(bias == nullptr || (n_tab >= 1 && n_tab <= FA_MAX_TAB), "layer_attention: a table of %lld distances (at most %d)", (long long)n_tab, FA_MAX_TAB);
+  if (T == 0) return MB200_OK;
+  FaParams f;
+  f.q_start = q_start;
+  f.seqpos = seqpos;
+  f.slots = slots;
+  f.bias = bias;
+  f.n_tab = bias != nullptr ? (int)n_tab : 0;
+  f.out = (bf16*)out;
+  f.B = (int)B;
+  f.W = (int)W;
+  f.window = (int)W;  // the ring holds the whole sequence
+  f.H = (int)n_heads;
+  f.KV = (int)n_kv_heads;
+  f.scale_log2 = scale * 1.4426950408889634f;
+  return launch_attn_prompt_tcgen05(f, q, nullptr, nullptr, cache_k, cache_v, blocks, T, max_seqlen, (cudaStream_t)stream);
+}
+
 static int layer_epilogue(EpiParams& e, const void* bias, void* out, float* out32, int64_t N, int epi, int64_t n_act, float limit, float alpha) {
   MB_CHECK_ARG(epi >= LAYER_STORE && epi <= LAYER_GEGLU, "layer_linear: step %d", epi);
   const bool gated = epi == LAYER_GLU || epi == LAYER_SWIGLU || epi == LAYER_GEGLU;

@@ -330,7 +330,7 @@ class BiasedAttention(nn.Module):
         _h.attn_bias(q, view.cache_k, view.cache_v, self.bias_table(), md.positions, md.q_start, md.slots, out, len(md.seqlens), md.window,
                      a.heads, a.kv_heads, a.dim, a.vdim, a.scale,
                      n_tiles=sum((n + 63) // 64 for n in md.seqlens) if md.max_seqlen >= FLASH_MIN_QUERIES else 0,
-                     splits=_h.attn_splits(T, a.heads, md.window))
+                     splits=_h.attn_splits(T, a.heads, md.window), seqpos=md.seqpos, longest=md.max_seqlen)
         project_out(out, self.wo, x32, post)
 
 

@@ -112,3 +112,73 @@ def test_lightning_infinity_reaches_no_earlier_token():
     for a, b in zip(*outs):
         assert torch.equal(torch.isfinite(a), torch.isfinite(b)) and torch.equal(torch.isnan(a), torch.isnan(b))
         assert rel(a[torch.isfinite(b)], b[torch.isfinite(b)].double()) < 1e-6
+
+
+def _attend64(q, k, v, qpos, kpos, scale, window, bias):
+    H, G = q.shape[1], k.shape[1]
+    dist = qpos[:, None] - kpos[None]
+    out = []
+    for head in range(H):
+        s = q[:, head] @ k[:, head // (H // G)].T * scale
+        if bias is not None:
+            s = s + bias[dist.clamp(0, len(bias) - 1), head]
+        s = s.masked_fill((dist < 0) | (dist >= window), float("-inf"))
+        out.append(torch.softmax(s, -1) @ v[:, head // (H // G)])
+    return torch.stack(out, 1).flatten(1)
+
+
+@pytest.mark.parametrize("H,KV", [(4, 2), (3, 1), (2, 2), (8, 1)])
+@pytest.mark.parametrize("lens,past,W", [([128], [0], 128), ([129, 60], [5, 0], 300), ([300], [1], 301), ([70, 257, 1], [400, 128, 3], 512), ([200, 48], [777, 90], 256),
+                                         ([64], [1000], 70)])
+def test_prompt_attention_over_ring_and_own_rows(H, KV, lens, past, W):
+    """Portions of prompts on the tcgen05 kernel: rings that wrap, runs around the 128-key tile, windows, rows nothing has written (NaN here),
+    one and two heads per CTA; P is rounded to bf16 (2^-9 relative)."""
+    from mistral_inference_b200 import _abi
+
+    g = torch.Generator().manual_seed(sum(lens) + W)
+    B, T, hd = len(lens), sum(lens), 128
+    rnd = lambda *s: torch.randn(*s, generator=g).bfloat16().to(DEV)  # noqa: E731
+    q, k, v = rnd(T, H, hd), rnd(T, KV, hd), rnd(T, KV, hd)
+    ring_k, ring_v = (torch.full((B, W, KV, hd), float("nan"), dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    q_start = torch.tensor([0] + lens).cumsum(0).int().to(DEV)
+    out, ref = torch.empty(T, H * hd, dtype=torch.bfloat16, device=DEV), []
+    for b, (n, m) in enumerate(zip(lens, past)):
+        have = min(m, W)
+        old = torch.arange(m - have, m, device=DEV)
+        ok, ov = rnd(have, KV, hd), rnd(have, KV, hd)
+        ring_k[b, old % W], ring_v[b, old % W] = ok, ov
+        a, z = int(q_start[b]), int(q_start[b + 1])
+        pos = torch.arange(m, m + n, device=DEV)
+        ref.append(_attend64(q[a:z].double(), torch.cat((ok, k[a:z])).double(), torch.cat((ov, v[a:z])).double(), pos, torch.cat((old, pos)), hd ** -0.5, W, None))
+    _abi.attn_prefill(q, k, v, ring_k, ring_v, q_start, torch.tensor(past, dtype=torch.int32, device=DEV), out, B, max(lens), W, H, KV, hd, causal=True,
+                      first_prefill=max(past) == 0)
+    assert rel(out, torch.cat(ref)) < 2 ** -8
+
+
+@pytest.mark.parametrize("n_tab", [0, 1, 40, 500])
+@pytest.mark.parametrize("lens,past", [([64], [0]), ([130, 33], [0, 0]), ([250, 1], [300, 5]), ([128, 128], [128, 1])])
+def test_prompt_attention_with_a_bias_over_the_ring(n_tab, lens, past):
+    """Every key in the ring (row blocks in another order than the batch, unwritten rows NaN), a bias table shorter and longer than the distances."""
+    from mistral_inference_b200 import _abi_hybrid as h
+
+    g = torch.Generator().manual_seed(sum(lens) + n_tab)
+    B, T, H, KV, hd = len(lens), sum(lens), 4, 2, 128
+    W = max(m + n for m, n in zip(past, lens)) + 3
+    rnd = lambda *s: torch.randn(*s, generator=g).bfloat16().to(DEV)  # noqa: E731
+    q = rnd(T, H * hd)
+    ring_k, ring_v = (torch.full((B + 1, W, KV, hd), float("nan"), dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    bias = torch.randn(n_tab, H, generator=g).to(DEV) * 2 if n_tab else None
+    slots = torch.arange(B).flip(0).add(1).int().to(DEV)
+    q_start = torch.tensor([0] + lens).cumsum(0).int().to(DEV)
+    seqpos, positions, ref = torch.tensor(past, dtype=torch.int32, device=DEV), [], []
+    for b, (n, m) in enumerate(zip(lens, past)):
+        kk, vv = rnd(m + n, KV, hd), rnd(m + n, KV, hd)
+        ring_k[slots[b].item(), : m + n], ring_v[slots[b].item(), : m + n] = kk, vv
+        pos = torch.arange(m, m + n, device=DEV)
+        positions.append(pos.int())
+        a, z = int(q_start[b]), int(q_start[b + 1])
+        ref.append(_attend64(q[a:z].view(n, H, hd).double(), kk.double(), vv.double(), pos, torch.arange(m + n, device=DEV), 0.1, W, bias.double() if n_tab else None))
+    out = torch.empty(T, H * hd, dtype=torch.bfloat16, device=DEV)
+    tiles = sum((n + 63) // 64 for n in lens)
+    h.attn_bias(q, ring_k, ring_v, bias, torch.cat(positions), q_start, slots, out, B, W, H, KV, hd, hd, 0.1, n_tiles=tiles, seqpos=seqpos, longest=max(lens))
+    assert rel(out, torch.cat(ref)) < 2 ** -8
