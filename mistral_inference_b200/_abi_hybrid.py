@@ -198,7 +198,7 @@ def attn_prep(qkv, qnorm, knorm, positions, cache_rows, q_out, cache_k, cache_v,
                                _stream()), "mbh_attn_prep")
 
 
-ATTN_TCGEN05_MIN = 48  # prompts (portions) at least this long fill enough of the tcgen05 kernel's 128-query tiles
+ATTN_TCGEN05_MIN = 16  # prompts (portions) at least this long take the tcgen05 kernel (128-query tiles) where the sizes allow
 
 
 def attn_bias(q, cache_k, cache_v, bias_tab, positions, q_start, slots, out, B: int, W: int, H: int, G: int, d: int, e: int, scale: float,

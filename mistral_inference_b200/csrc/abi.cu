@@ -21,8 +21,9 @@ thread_local char g_err[512] = "";
 static unsigned long long* g_mk_prof = nullptr;
 static unsigned long long* g_mk_prof_bar = nullptr;  // debug: decode megakernel phase timeline buffer (device)
 
-// the shortest longest sequence of a call from which prompt attention takes the tcgen05 kernel (128 queries a tile)
-constexpr int64_t MB200_ATTN_FIRST_MIN = 128, MB200_ATTN_PORTION_MIN = 48;
+// The longest sequence of a call from which prompt attention takes the tcgen05 kernel (128 queries a tile).  Portions: 8 x 20 queries over 420
+// keys 27 -> 20 us, 1 x 20 over 3020 keys 117 -> 77 us.  First prompts below 128 tokens are as long as the launch either way.
+constexpr int64_t MB200_ATTN_FIRST_MIN = 128, MB200_ATTN_PORTION_MIN = 16;
 
 constexpr size_t kWsHeader = 64 * 1024;  // persistent, zero-initialised by the caller once: self-resetting counters
 inline size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }

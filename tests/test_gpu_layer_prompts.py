@@ -182,3 +182,32 @@ def test_prompt_attention_with_a_bias_over_the_ring(n_tab, lens, past):
     tiles = sum((n + 63) // 64 for n in lens)
     h.attn_bias(q, ring_k, ring_v, bias, torch.cat(positions), q_start, slots, out, B, W, H, KV, hd, hd, 0.1, n_tiles=tiles, seqpos=seqpos, longest=max(lens))
     assert rel(out, torch.cat(ref)) < 2 ** -8
+
+
+@pytest.mark.parametrize("M,N,K", [(9, 130, 64), (127, 96, 100), (128, 128, 7), (129, 257, 300), (33, 2048, 2048), (300, 640, 8192), (17, 6, 1029)])
+def test_fp32_linear_in_parts(M, N, K):
+    """fp32 Linears of prompts on the tensor cores: tile edges, k parts over clusters, rows that are no multiple of 16 bytes.  The part products
+    that are left out are below 2^-21 of a product each; the sum is no further from float64 than a chain of FMAs is."""
+    from mistral_inference_b200 import _abi_hybrid as h
+
+    g = torch.Generator().manual_seed(M + N + K)
+    x, w, b = torch.randn(M, K, generator=g).to(DEV), torch.randn(N, K, generator=g).to(DEV), torch.randn(N, generator=g).to(DEV)
+    ref = x.double() @ w.double().T + b.double()
+    got = h.linear(x, w, b, epi=h.EPI_F32)
+    chain = torch.zeros(M, N, device=DEV)
+    for k in range(K):  # one rounded multiply-add per column, as an FMA chain takes them
+        chain = torch.addcmul(chain, x[:, k:k + 1], w[:, k][None])
+    assert rel(got, ref) < max(2 ** -22, 1.1 * rel(chain + b, ref))
+    base = torch.randn(M, N, generator=g).to(DEV)
+    assert rel(h.linear(x, w, None, epi=h.EPI_RESIDUAL, residual=base.clone()), base.double() + x.double() @ w.double().T) < 2 ** -21
+    big, tiny = h.linear(x * 1e30, w * 1e-30, epi=h.EPI_F32), h.linear(x * 2.0 ** -60, w * 2.0 ** 60, epi=h.EPI_F32)
+    assert rel(big, (x * 1e30).double() @ (w * 1e-30).double().T) < 2 ** -21 and rel(tiny, x.double() @ w.double().T) < 2 ** -21
+
+
+def test_fp32_linear_infinities():
+    from mistral_inference_b200 import _abi_hybrid as h
+
+    x, w = torch.ones(40, 256, device=DEV), torch.ones(300, 256, device=DEV)
+    x[3, 7], x[4, 9], w[130, 8], w[131, 7] = float("inf"), float("nan"), float("-inf"), 0.0
+    got, ref = h.linear(x, w, epi=h.EPI_F32), x.double() @ w.double().T
+    assert torch.equal(torch.isnan(got), torch.isnan(ref)) and torch.equal(torch.nan_to_num(got).double(), torch.nan_to_num(ref.float()).double())
