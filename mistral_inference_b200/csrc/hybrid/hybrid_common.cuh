@@ -2,7 +2,7 @@
 //
 // Every kernel of this library is a template over the storage type of activations and weights (bf16 or fp32) and does
 // its arithmetic in fp32.  The residual stream, softmax, norms and recurrent state are fp32 in both modes; in fp32 mode
-// nothing is rounded below 32 bits (plain FMA, no TF32).
+// nothing is rounded below 32 bits (FMAs, or tensor-core products of three bf16 parts that add up to the fp32 number; no TF32).
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -11,6 +11,8 @@
 namespace mbh {
 
 using bf16 = __nv_bfloat16;
+
+__device__ __forceinline__ bool not_finite(float x) { return (__float_as_uint(x) & 0x7f800000u) == 0x7f800000u; }
 
 template <typename T> __device__ __forceinline__ float to_f(T v);
 template <> __device__ __forceinline__ float to_f<float>(float v) { return v; }

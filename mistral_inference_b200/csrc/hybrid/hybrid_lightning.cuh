@@ -45,7 +45,6 @@ __device__ __forceinline__ void split3_pack(float x, float y, uint32_t& hi, uint
     split3(y, yh, ym, yl);
     hi = pack_bf16(xh, yh); mid = pack_bf16(xm, ym); lo = pack_bf16(xl, yl);
 }
-__device__ __forceinline__ bool not_finite(float x) { return (__float_as_uint(x) & 0x7f800000u) == 0x7f800000u; }
 
 template <int D>
 __global__ void __launch_bounds__(LC_THREADS) lightning_chunk_kernel(LightningArgs a) {

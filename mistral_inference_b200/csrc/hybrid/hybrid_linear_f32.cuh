@@ -11,16 +11,16 @@
 // 3 x ~250 tokens, width 2048, two layers.
 //
 // CTA = 128 x 128 outputs, or one of `splits` parts of their k range (a cluster; the parts are added through distributed shared memory in
-// rank order, so a small problem fills the chip and the result is the same every time).  9 warps: eight load fp32 from global memory
+// rank order, so a small problem fills the chip and the result is the same every time).  17 warps: sixteen load fp32 from global memory
 // (one k-block ahead, in registers), split, write the six part tiles (128B-swizzled, K-major) of a stage and add the block before to
-// their registers; one thread of the ninth issues the MMAs.  Two stages: the MMAs of a block run under the splitting of the next.
+// their registers; one thread of the last issues the MMAs (with eight workers the loads' latency was in the open: 3530 us of Linears against 1870).  Two stages: the MMAs of a block run under the splitting of the next.
 // An infinity or a NaN in the operands of a tile: its outputs are computed again with FMAs (inf x 0 parts would give NaN).
 #pragma once
 #include "hybrid_linear.cuh"
 
 namespace mbh {
 
-constexpr int FT_BM = 128, FT_BN = 128, FT_BK = 64, FT_THREADS = 288, FT_TILE = 128 * 64 * 2;  // a part tile: 128 rows of 128 bytes
+constexpr int FT_BM = 128, FT_BN = 128, FT_BK = 64, FT_WARPS = 16 /* workers */, FT_THREADS = 32 * (FT_WARPS + 1), FT_TILE = 128 * 64 * 2;  // a part tile: 128 rows of 128 bytes
 constexpr int FT_STAGE = 6 * FT_TILE, FT_SMEM = 2 * FT_STAGE + 1024, FT_LD = FT_BN + 4;
 static_assert(FT_BM * FT_LD * 4 <= 2 * FT_STAGE, "the sums of a tile fit in the stages");
 
@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) linear_f32_parts(LinearArgs a, 
     unsigned char* const sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(ft_raw) + 1023) & ~(uintptr_t)1023);
     __shared__ uint64_t full[2], done[2];
     __shared__ uint32_t tmem_slot;
-    __shared__ int flags;  // 1: an operand that is not finite; 2: a wait that ended without its event
+    __shared__ int flags;  // 1: a sum that is not finite; 2: a wait that ended without its event
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // row tiles fastest: the CTAs that share a tile of W run together
     const int tiles_m = (a.M + FT_BM - 1) / FT_BM, tile = blockIdx.x / splits, rank = blockIdx.x % splits;
@@ -89,11 +89,11 @@ __global__ void __launch_bounds__(FT_THREADS, 1) linear_f32_parts(LinearArgs a, 
     const int nkb = (a.K + FT_BK - 1) / FT_BK, kb0 = (int)((long long)nkb * rank / splits), kb1 = (int)((long long)nkb * (rank + 1) / splits);
 
     if (tid == 0) {
-        for (int i = 0; i < 2; ++i) { ft_bar_init(&full[i], 8); ft_bar_init(&done[i], 1); }
+        for (int i = 0; i < 2; ++i) { ft_bar_init(&full[i], FT_WARPS); ft_bar_init(&done[i], 1); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         flags = 0;
     }
-    if (warp == 8) {
+    if (warp == FT_WARPS) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(ft_smem(&tmem_slot)), "r"(256u) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -107,16 +107,18 @@ __global__ void __launch_bounds__(FT_THREADS, 1) linear_f32_parts(LinearArgs a, 
     __syncthreads();
     ft_fence_after();
     const uint32_t tmem = tmem_slot;
-    float acc[64];
-    if (warp < 8) {
-        // float4 i of this thread: row (i * 16 + tid / 16), columns 4 (tid % 16) .. of the k-block
+    constexpr int NF = FT_BM * FT_BK / 4 / (32 * FT_WARPS), RS = FT_BM / NF, NC = FT_BN / (FT_WARPS / 4);  // float4s and row step of a worker, its columns of the sums
+    float acc[NC];
+    int strange = 0;  // a sum that is not finite
+    if (warp < FT_WARPS) {
+        // float4 i of this thread: row (i * RS + tid / 16), columns 4 (tid % 16) .. of the k-block
         const int r0 = tid >> 4, c4 = (tid & 15) * 4;
-        float4 px[8], pw[8];
+        float4 px[NF], pw[NF];
         auto fetch = [&](int kb) {
             const int k = kb * FT_BK + c4;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int r = r0 + 16 * i;
+            for (int i = 0; i < NF; ++i) {
+                const int r = r0 + RS * i;
                 px[i] = pw[i] = make_float4(0.f, 0.f, 0.f, 0.f);
                 const float *xp = X + (size_t)r * a.x_pitch() + k, *wp = W + (size_t)r * a.K + k;
                 if (VEC) {
@@ -135,7 +137,6 @@ __global__ void __launch_bounds__(FT_THREADS, 1) linear_f32_parts(LinearArgs a, 
                 }
             }
         };
-        uint32_t odd = 0;  // 1 once an operand with all exponent bits set has been seen
         auto put = [&](unsigned char* tile, int r, const float4& v) {
             const float* f = reinterpret_cast<const float*>(&v);
             uint32_t part[3][2];
@@ -143,7 +144,6 @@ __global__ void __launch_bounds__(FT_THREADS, 1) linear_f32_parts(LinearArgs a, 
             for (int e = 0; e < 2; ++e) {
                 const float x = f[2 * e], y = f[2 * e + 1];
                 const uint32_t ux = __float_as_uint(x), uy = __float_as_uint(y);
-                odd |= ((ux & 0x7f800000u) == 0x7f800000u) | ((uy & 0x7f800000u) == 0x7f800000u);
                 const float rx = x - __uint_as_float(ux & 0xffff0000u), ry = y - __uint_as_float(uy & 0xffff0000u);
                 const uint32_t mx = __float_as_uint(rx), my = __float_as_uint(ry);
                 const uint32_t lx = __float_as_uint(rx - __uint_as_float(mx & 0xffff0000u)), ly = __float_as_uint(ry - __uint_as_float(my & 0xffff0000u));
@@ -156,8 +156,8 @@ __global__ void __launch_bounds__(FT_THREADS, 1) linear_f32_parts(LinearArgs a, 
             for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(at + q * FT_TILE) = make_uint2(part[q][0], part[q][1]);
         };
 #pragma unroll
-        for (int j = 0; j < 64; ++j) acc[j] = 0.f;
-        const uint32_t mine = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (warp >> 2) * 64;
+        for (int j = 0; j < NC; ++j) acc[j] = 0.f;
+        const uint32_t mine = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (warp >> 2) * NC;
         bool alive = true;
         auto promote = [&](int it) {
             if (alive && !ft_bar_wait(&done[it & 1], (it >> 1) & 1)) { alive = false; atomicOr(&flags, 2); }
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) linear_f32_parts(LinearArgs a, 
             ft_fence_after();
             float v[32];
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
+            for (int c = 0; c < NC / 32; ++c) {
                 ft_ld32(mine + (it & 1) * 128 + c * 32, v);
 #pragma unroll
                 for (int j = 0; j < 32; ++j) acc[c * 32 + j] += v[j];
@@ -178,8 +178,8 @@ __global__ void __launch_bounds__(FT_THREADS, 1) linear_f32_parts(LinearArgs a, 
         for (int it = 0; it < kb1 - kb0; ++it) {
             unsigned char* st = sm + (it & 1) * FT_STAGE;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int r = r0 + 16 * i;
+            for (int i = 0; i < NF; ++i) {
+                const int r = r0 + RS * i;
                 if (r < rows) put(st, r, px[i]);
                 if (r < cols) put(st + 3 * FT_TILE, r, pw[i]);
             }
@@ -190,7 +190,10 @@ __global__ void __launch_bounds__(FT_THREADS, 1) linear_f32_parts(LinearArgs a, 
             if (it > 0) promote(it - 1);
         }
         if (kb0 < kb1) promote(kb1 - kb0 - 1);
-        if (odd) atomicOr(&flags, 1);
+        // an operand that is not finite makes a part that is NaN (inf - inf), so every sum it enters is NaN: found here, once
+#pragma unroll
+        for (int j = 0; j < NC; ++j) strange |= not_finite(acc[j]);
+        if (strange) atomicOr(&flags, 1);
     } else if (lane == 0) {
         bool alive = true;
         for (int it = 0; it < kb1 - kb0; ++it) {
@@ -211,12 +214,12 @@ __global__ void __launch_bounds__(FT_THREADS, 1) linear_f32_parts(LinearArgs a, 
     __syncthreads();  // every MMA has completed (the last promote waited for it): the stages are free
     ft_fence_after();
     float(*sum)[FT_LD] = reinterpret_cast<float(*)[FT_LD]>(sm);
-    if (warp < 8) {
-        const int r = (warp & 3) * 32 + lane, c = (warp >> 2) * 64;
+    if (warp < FT_WARPS) {
+        const int r = (warp & 3) * 32 + lane, c = (warp >> 2) * NC;
 #pragma unroll
-        for (int j = 0; j < 64; j += 4) *reinterpret_cast<float4*>(&sum[r][c + j]) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
+        for (int j = 0; j < NC; j += 4) *reinterpret_cast<float4*>(&sum[r][c + j]) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
     }
-    if (warp == 8) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u));
+    if (warp == FT_WARPS) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u));
     int mark = 0;
     if (splits > 1) {
         ft_cluster_sync();
