@@ -30,6 +30,7 @@ _SIGNATURES = {
     "mbh_attn_prep": (c_int, [P, P, P, P, P, P, P, P, P, P, c_int, I, I, I, I, I, F, F, I, c_int, P]),
     "mbh_attn_bias": (c_int, [P, P, P, P, I, P, P, P, P, I, I, I, I, I, I, I, F, I, I, P, c_int, P]),
     "mbh_lightning_scan": (c_int, [P, P, P, P, P, P, P, I, I, I, I, c_int, P]),
+    "mbh_attn_bias_decode": (c_int, [P, P, P, P, I, P, P, P, I, I, I, I, I, I, F, I, P, P]),
     "mbh_lightning_prompt": (c_int, [P, P, P, P, P, P, P, I, I, I, I, P]),
     "mbh_gated_headnorm": (c_int, [P, P, P, I, I, P, I, I, F, c_int, P]),
     "mbh_embed_add": (c_int, [P, P, F, P, I, I, c_int, P]),
@@ -515,6 +516,22 @@ def attn_decode(q, cache_k, cache_v, positions, slots, out, B: int, W: int, H: i
     _check(lib().mbh_attn_decode(_ptr(q), _ptr(cache_k), _ptr(cache_v), _ptr(positions), _ptr(slots), _ptr(out), B, W, H, G, d, e, scale, splits, _ptr(scratch), window,
                                  int(chunked), softcap, _ptr(sink), gp, g_pitch, int(gate_entry), maps, _ptr(lam), out_scale, norm_eps, dt_of(q.dtype), _stream()),
            "mbh_attn_decode")
+
+
+BIAS_DECODE_SIZES = {(32, 32), (64, 64), (64, 128), (128, 64), (128, 128)}  # (key, value) sizes of the decode kernel with a bias
+
+
+def attn_bias_decode_ok(q: torch.Tensor, cache_k: torch.Tensor, cache_v: torch.Tensor, H: int, G: int, d: int, e: int) -> bool:
+    return (q.dtype == torch.bfloat16 and H % G == 0 and H // G <= DECODE_MAX_GROUP and (d, e) in BIAS_DECODE_SIZES and _aligned(q, cache_k, cache_v)
+            and os.environ.get("MB200_ATTN_DECODE", "1") != "0")
+
+
+def attn_bias_decode(q, cache_k, cache_v, bias_tab, positions, slots, out, B: int, W: int, H: int, G: int, d: int, e: int, scale: float) -> None:
+    """`attn_bias` for one token per sequence on tensor cores (attn_bias_decode_ok says when)."""
+    splits = attn_decode_splits(B, G, W)
+    scratch = torch.empty(B * H * splits * (2 + e), dtype=torch.float32, device=q.device)
+    _check(lib().mbh_attn_bias_decode(_ptr(q), _ptr(cache_k), _ptr(cache_v), _ptr(bias_tab), bias_tab.shape[0], _ptr(positions), _ptr(slots), _ptr(out), B, W, H, G, d, e,
+                                      scale, splits, _ptr(scratch), _stream()), "mbh_attn_bias_decode")
 
 
 def window_decode_plan(T: int, H: int, W: int):

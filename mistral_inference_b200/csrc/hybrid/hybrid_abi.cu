@@ -291,6 +291,26 @@ int mbh_attn_decode(const void* q, const void* ring_k, const void* ring_v, const
     return err ? fail(err, "mbh_attn_decode") : 0;
 }
 
+int mbh_attn_bias_decode(const void* q, const void* ring_k, const void* ring_v, const void* bias_tab, int64_t n_tab, const void* positions, const void* slots, void* out,
+                         int64_t B, int64_t W, int64_t H, int64_t G, int64_t d, int64_t e, float scale, int64_t splits, void* scratch, void* stream) {
+    if (B == 0) return 0;
+    if (H % G) return bad("mbh_attn_bias_decode: heads must be a multiple of kv heads");
+    if (!bias_tab || n_tab < 1) return bad("mbh_attn_bias_decode: a bias table");
+    if (splits < 1 || splits > AT_MAX_SPLITS || !scratch) return bad("mbh_attn_bias_decode: 1 to 64 splits, with scratch");
+    AttnArgs a{};
+    a.q = q; a.cache_k = ring_k; a.cache_v = ring_v; a.bias_tab = (const float*)bias_tab; a.n_tab = (int)n_tab; a.positions = (const int*)positions;
+    a.slots = (const int*)slots; a.out = out;
+    a.T = (int)B; a.B = (int)B; a.W = (int)W; a.H = (int)H; a.G = (int)G; a.d = (int)d; a.e = (int)e; a.scale = scale; a.splits = (int)splits; a.scratch = (float*)scratch;
+    a.maps = 1;
+    cudaStream_t st = (cudaStream_t)stream;
+    cudaError_t err = cudaSuccess;
+    if (!launch_attn_decode(a, st, err)) return bad("mbh_attn_bias_decode: head sizes without a kernel");
+    if (err) return fail(err, "mbh_attn_bias_decode");
+    run_attn_merge<__nv_bfloat16>(a, st);
+    err = cudaGetLastError();
+    return err ? fail(err, "mbh_attn_bias_decode") : 0;
+}
+
 int mbh_lightning_scan(const void* qkvg, void* state, const void* decay, const void* q_start, const void* seqpos, const void* slots, void* o32,
                        int64_t B, int64_t H, int64_t d, int64_t e, int dt, void* stream) {
     if (B == 0) return 0;

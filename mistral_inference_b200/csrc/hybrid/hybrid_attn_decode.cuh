@@ -5,8 +5,11 @@
 // pieces arriving by cp.async in a private ring of DA_STAGES buffers -- warps never wait for one another before the end, when they are merged
 // through shared memory.  The splits' partial results have the layout of attn_bias_kernel's and go through the same merge kernels (sinks,
 // differences of two maps, gates).  With MAPS 2 both maps of a head are computed here: their keys are one row, their values are shared.
+// BIAS: AttnArgs::bias_tab is added to the scores by distance, and the weights stay 32 bits wide -- they multiply the values as three bf16 parts
+// (hybrid_lightning.cuh), as exact as the fp32 kernel of hybrid_mixers.cuh that these layers ran on, which reads a ring row once per query head:
+// 116 us for 8 sequences of ~1800 tokens, 16 / 4 heads, against 16 us here and 4 us of merging.
 #pragma once
-#include "hybrid_attn_flash.cuh"
+#include "hybrid_lightning.cuh"
 
 namespace mbh {
 
@@ -18,8 +21,10 @@ template <int D, int E, int MAPS> constexpr size_t attn_decode_smem() {
     return stages > merge ? stages : merge;
 }
 
-template <int D, int E, int MAPS>
+template <int D, int E, int MAPS, bool BIAS = false>
 __global__ void __launch_bounds__(DA_WARPS * 32) attn_decode_mma_kernel(AttnArgs a) {
+    static_assert(!BIAS || MAPS == 1, "a bias with two maps is not built");
+    constexpr int PARTS = BIAS ? 3 : 1;
     constexpr int KP = MAPS * D + 8, VP = E + 8, STAGE = DA_KEYS * (KP + VP);
     constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
     extern __shared__ __align__(16) unsigned char da_smem[];
@@ -85,7 +90,17 @@ __global__ void __launch_bounds__(DA_WARPS * 32) attn_decode_mma_kernel(AttnArgs
         __syncwarp();
         const bf16* ks = mine + stage * STAGE;
         const bf16* vs = ks + DA_KEYS * KP;
-        uint32_t pa[MAPS][4];
+        uint32_t pa[MAPS * PARTS][4];
+        float bias[2][4];  // in log2 units, requested before the products
+        if constexpr (BIAS) {
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const int row = gid + (c >> 1) * 8, dist = min(max(pos - (c0 + nt * 8 + tig * 2 + (c & 1)), 0), a.n_tab - 1);
+                    bias[nt][c] = row < R ? __ldg(a.bias_tab + (size_t)dist * a.H + g * R + row) * LOG2E : 0.f;
+                }
+        }
 #pragma unroll
         for (int m = 0; m < MAPS; ++m) {
             float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
@@ -105,7 +120,9 @@ __global__ void __launch_bounds__(DA_WARPS * 32) attn_decode_mma_kernel(AttnArgs
                     const bool ok = c0 + nt * 8 + tig * 2 + c <= pos;
                     float x0 = s[nt][c], x1 = s[nt][2 + c];
                     if (capped) { x0 = softcap_fast(x0, a.softcap, capf); x1 = softcap_fast(x1, a.softcap, capf); }
-                    s[nt][c] = ok ? x0 * unit : -INFINITY; s[nt][2 + c] = ok ? x1 * unit : -INFINITY;
+                    x0 = BIAS ? fmaf(x0, unit, bias[nt][c]) : x0 * unit;
+                    x1 = BIAS ? fmaf(x1, unit, bias[nt][2 + c]) : x1 * unit;
+                    s[nt][c] = ok ? x0 : -INFINITY; s[nt][2 + c] = ok ? x1 : -INFINITY;
                     t0 = fmaxf(t0, s[nt][c]); t1 = fmaxf(t1, s[nt][2 + c]);
                 }
             // key c0 is visible, so the new maxima are finite
@@ -123,8 +140,13 @@ __global__ void __launch_bounds__(DA_WARPS * 32) attn_decode_mma_kernel(AttnArgs
             l[m][0] = l[m][0] * f0 + q0; l[m][1] = l[m][1] * f1 + q1;
 #pragma unroll
             for (int ne = 0; ne < E / 8; ++ne) { o[m][ne][0] *= f0; o[m][ne][1] *= f0; o[m][ne][2] *= f1; o[m][ne][3] *= f1; }
-            pa[m][0] = pack_bf16(s[0][0], s[0][1]); pa[m][1] = pack_bf16(s[0][2], s[0][3]);
-            pa[m][2] = pack_bf16(s[1][0], s[1][1]); pa[m][3] = pack_bf16(s[1][2], s[1][3]);
+            if constexpr (BIAS) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) split3_pack(s[u >> 1][(u & 1) * 2], s[u >> 1][(u & 1) * 2 + 1], pa[0][u], pa[1][u], pa[2][u]);
+            } else {
+                pa[m][0] = pack_bf16(s[0][0], s[0][1]); pa[m][1] = pack_bf16(s[0][2], s[0][3]);
+                pa[m][2] = pack_bf16(s[1][0], s[1][1]); pa[m][3] = pack_bf16(s[1][2], s[1][3]);
+            }
         }
         const bf16* vp = vs + (((lane >> 3) & 1) * 8 + (lane & 7)) * VP + (lane >> 4) * 8;
 #pragma unroll
@@ -132,10 +154,12 @@ __global__ void __launch_bounds__(DA_WARPS * 32) attn_decode_mma_kernel(AttnArgs
             uint32_t vf[4];
             ldmatrix4_trans(vf, vp + np * 16);
 #pragma unroll
-            for (int m = 0; m < MAPS; ++m) {
-                mma_bf16(o[m][2 * np], pa[m], vf[0], vf[1]);
-                mma_bf16(o[m][2 * np + 1], pa[m], vf[2], vf[3]);
-            }
+            for (int m = 0; m < MAPS; ++m)
+#pragma unroll
+                for (int q = PARTS - 1; q >= 0; --q) {  // the smallest part first
+                    mma_bf16(o[m][2 * np], pa[m * PARTS + q], vf[0], vf[1]);
+                    mma_bf16(o[m][2 * np + 1], pa[m * PARTS + q], vf[2], vf[3]);
+                }
         }
         __syncwarp();  // the buffer is used up
         stage = (stage + 1) % DA_STAGES;
@@ -181,19 +205,25 @@ __global__ void __launch_bounds__(DA_WARPS * 32) attn_decode_mma_kernel(AttnArgs
     }
 }
 
-template <int D, int E, int MAPS> inline cudaError_t run_attn_decode(const AttnArgs& a, cudaStream_t st) {
+template <int D, int E, int MAPS, bool BIAS = false> inline cudaError_t run_attn_decode(const AttnArgs& a, cudaStream_t st) {
     constexpr size_t smem = attn_decode_smem<D, E, MAPS>();
     if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(attn_decode_mma_kernel<D, E, MAPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t e = cudaFuncSetAttribute(attn_decode_mma_kernel<D, E, MAPS, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e) return e;
     }
-    attn_decode_mma_kernel<D, E, MAPS><<<dim3((unsigned)(a.B * a.G), (unsigned)a.splits), DA_WARPS * 32, smem, st>>>(a);
+    attn_decode_mma_kernel<D, E, MAPS, BIAS><<<dim3((unsigned)(a.B * a.G), (unsigned)a.splits), DA_WARPS * 32, smem, st>>>(a);
     return cudaGetLastError();
 }
 
 // true when a (D, E, maps) instantiation exists; launches it (partial results only)
 inline bool launch_attn_decode(const AttnArgs& a, cudaStream_t st, cudaError_t& err) {
     if (a.H / a.G > DA_MAX_GROUP) return false;
+    if (a.bias_tab) {
+#define MBH_DAB(DD, EE) if (a.d == DD && a.e == EE && a.maps == 1) { err = run_attn_decode<DD, EE, 1, true>(a, st); return true; }
+        MBH_DAB(32, 32) MBH_DAB(64, 64) MBH_DAB(64, 128) MBH_DAB(128, 64) MBH_DAB(128, 128)
+#undef MBH_DAB
+        return false;
+    }
 #define MBH_DA(DD, EE, MM) if (a.d == DD && a.e == EE && a.maps == MM) { err = run_attn_decode<DD, EE, MM>(a, st); return true; }
     MBH_DA(32, 32, 1) MBH_DA(64, 32, 1) MBH_DA(64, 64, 1) MBH_DA(64, 128, 1) MBH_DA(128, 64, 1) MBH_DA(128, 128, 1) MBH_DA(96, 64, 1) MBH_DA(96, 96, 1)
     MBH_DA(32, 32, 2) MBH_DA(32, 64, 2) MBH_DA(48, 96, 2) MBH_DA(64, 64, 2) MBH_DA(64, 128, 2) MBH_DA(96, 96, 2) MBH_DA(128, 128, 2)

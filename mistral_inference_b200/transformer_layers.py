@@ -327,10 +327,13 @@ class BiasedAttention(nn.Module):
         _h.attn_prep(qkv, self.q_norm, self.k_norm, md.positions, md.cache_rows, q, view.cache_k, view.cache_v, ctx.get("v_first"), self.vmix, mode,
                      a.heads, a.kv_heads, a.dim, a.vdim, self.eps, a.temp_coef, a.temp_every)
         out = torch.empty(T, a.heads * a.vdim, dtype=hn.dtype, device=hn.device)
-        _h.attn_bias(q, view.cache_k, view.cache_v, self.bias_table(), md.positions, md.q_start, md.slots, out, len(md.seqlens), md.window,
-                     a.heads, a.kv_heads, a.dim, a.vdim, a.scale,
-                     n_tiles=sum((n + 63) // 64 for n in md.seqlens) if md.max_seqlen >= FLASH_MIN_QUERIES else 0,
-                     splits=_h.attn_splits(T, a.heads, md.window), seqpos=md.seqpos, longest=md.max_seqlen)
+        if not md.prefill and _h.attn_bias_decode_ok(q, view.cache_k, view.cache_v, a.heads, a.kv_heads, a.dim, a.vdim):
+            _h.attn_bias_decode(q, view.cache_k, view.cache_v, self.bias_table(), md.positions, md.slots, out, T, md.window, a.heads, a.kv_heads, a.dim, a.vdim, a.scale)
+        else:
+            _h.attn_bias(q, view.cache_k, view.cache_v, self.bias_table(), md.positions, md.q_start, md.slots, out, len(md.seqlens), md.window,
+                         a.heads, a.kv_heads, a.dim, a.vdim, a.scale,
+                         n_tiles=sum((n + 63) // 64 for n in md.seqlens) if md.max_seqlen >= FLASH_MIN_QUERIES else 0,
+                         splits=_h.attn_splits(T, a.heads, md.window), seqpos=md.seqpos, longest=md.max_seqlen)
         project_out(out, self.wo, x32, post)
 
 

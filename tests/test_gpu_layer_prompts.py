@@ -211,3 +211,29 @@ def test_fp32_linear_infinities():
     x[3, 7], x[4, 9], w[130, 8], w[131, 7] = float("inf"), float("nan"), float("-inf"), 0.0
     got, ref = h.linear(x, w, epi=h.EPI_F32), x.double() @ w.double().T
     assert torch.equal(torch.isnan(got), torch.isnan(ref)) and torch.equal(torch.nan_to_num(got).double(), torch.nan_to_num(ref.float()).double())
+
+
+@pytest.mark.parametrize("H,G,d,e", [(16, 4, 128, 128), (3, 1, 64, 128), (16, 1, 32, 32), (2, 2, 128, 64)])
+@pytest.mark.parametrize("pos", [[0], [15, 16, 63], [64, 500, 1, 2047]])
+@pytest.mark.parametrize("n_tab", [1, 30, 1200])
+def test_decode_attention_with_a_bias(H, G, d, e, pos, n_tab):
+    """One token per sequence: against float64, and no further from it than the exact fp32 kernel (the output's bf16 rounding apart, 2^-9); rows
+    nothing has written are NaN."""
+    from mistral_inference_b200 import _abi_hybrid as h
+
+    g = torch.Generator().manual_seed(H + d + len(pos))
+    B, W = len(pos), max(pos) + 2
+    q = torch.randn(B, H * d, generator=g).bfloat16().to(DEV)
+    ring_k, ring_v = (torch.full((B, W, G, n), float("nan"), dtype=torch.bfloat16, device=DEV) for n in (d, e))
+    bias = torch.randn(n_tab, H, generator=g).to(DEV) * 2
+    slots, ref = torch.arange(B).flip(0).int().to(DEV), []
+    for b, p in enumerate(pos):
+        kk, vv = (torch.randn(p + 1, G, n, generator=g).bfloat16().to(DEV) for n in (d, e))
+        ring_k[B - 1 - b, : p + 1], ring_v[B - 1 - b, : p + 1] = kk, vv
+        ref.append(_attend64(q[b].view(1, H, d).double(), kk.double(), vv.double(), torch.tensor([p], device=DEV), torch.arange(p + 1, device=DEV), 0.2, W, bias.double()))
+    ref, positions = torch.cat(ref), torch.tensor(pos, dtype=torch.int32, device=DEV)
+    got, exact = (torch.empty(B, H * e, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    assert h.attn_bias_decode_ok(q, ring_k, ring_v, H, G, d, e)
+    h.attn_bias_decode(q, ring_k, ring_v, bias, positions, slots, got, B, W, H, G, d, e, 0.2)
+    h.attn_bias(q, ring_k, ring_v, bias, positions, torch.arange(B + 1, dtype=torch.int32, device=DEV), slots, exact, B, W, H, G, d, e, 0.2, splits=h.attn_splits(B, H, W))
+    assert rel(got, ref) < 2 ** -9 and rel(got, ref) < 1.1 * rel(exact, ref) + 2 ** -16
