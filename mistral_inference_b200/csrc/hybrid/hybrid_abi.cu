@@ -1,6 +1,8 @@
 // C ABI of libmb200_hybrid.so: the kernels of layered decoders (per-layer mixer kinds, fp32 residual stream, bf16 or fp32
 // storage).  Declarations: include/mistral_b200_hybrid.h.  `dt` selects the storage type of activations and weights:
 // 0 = bf16, 1 = fp32.  Every call returns 0 or a CUDA error code; mbh_last_error() gives the text.
+#include <algorithm>
+
 #include "hybrid_lightning.cuh"
 #include "hybrid_linear.cuh"
 #include "hybrid_mixers.cuh"
@@ -35,10 +37,9 @@ template <typename T>
 static cudaError_t launch_lightning(const LightningArgs& a, cudaStream_t st) {
     const int threads = LS_THREADS;
     dim3 grid(a.B * a.H, (a.e + threads - 1) / threads);
-    if (a.d <= 32) lightning_scan_kernel<T, 32><<<grid, threads, 0, st>>>(a);
-    else if (a.d <= 64) lightning_scan_kernel<T, 64><<<grid, threads, 0, st>>>(a);
-    else lightning_scan_kernel<T, 128><<<grid, threads, 0, st>>>(a);
-    return cudaGetLastError();
+    if (a.d <= 32) return launch_pdl(lightning_scan_kernel<T, 32>, grid, dim3(threads), 0, st, a);
+    if (a.d <= 64) return launch_pdl(lightning_scan_kernel<T, 64>, grid, dim3(threads), 0, st, a);
+    return launch_pdl(lightning_scan_kernel<T, 128>, grid, dim3(threads), 0, st, a);
 }
 
 
@@ -88,10 +89,10 @@ template <typename T> static void run_mlstm_gates(const MlstmGateArgs& a, int64_
     mlstm_qab_kernel<T><<<dim3((unsigned)T_, jb), 256, 0, st>>>(a);
 }
 template <typename T> static void run_embed(const void* tokens, const void* table, float scale, void* x32, int64_t T_, int64_t D, cudaStream_t st) {
-    embed_scale_kernel<T><<<(unsigned)T_, 128, 0, st>>>((const int64_t*)tokens, (const T*)table, scale, (float*)x32, (int)D);
+    launch_pdl(embed_scale_kernel<T, false>, dim3((unsigned)T_), dim3(256), 0, st, (const int64_t*)tokens, (const T*)table, scale, (float*)x32, (int)D);
 }
 template <typename T> static void run_embed_add(const void* tokens, const void* table, float scale, void* x32, int64_t T_, int64_t D, cudaStream_t st) {
-    embed_scale_kernel<T, true><<<(unsigned)T_, 128, 0, st>>>((const int64_t*)tokens, (const T*)table, scale, (float*)x32, (int)D);
+    launch_pdl(embed_scale_kernel<T, true>, dim3((unsigned)T_), dim3(256), 0, st, (const int64_t*)tokens, (const T*)table, scale, (float*)x32, (int)D);
 }
 template <typename T> static void run_layernorm(const void* x32, const void* w, const void* b, void* y, void* acc32, int64_t T_, int64_t D, float eps,
                                                 cudaStream_t st) {
@@ -112,7 +113,7 @@ template <typename T> static void run_moe_sparse(const MoeSparseArgs& a, int64_t
 }
 template <typename T> static void run_rmsnorm(const void* x32, const void* w, const void* w2, void* y, void* y2, int64_t T_, int64_t D, float eps, float offset,
                                               cudaStream_t st) {
-    rmsnorm_f32_kernel<T><<<(unsigned)T_, D >= 1024 ? 256 : 128, 0, st>>>((const float*)x32, (const T*)w, (const T*)w2, (T*)y, (T*)y2, (int)D, eps, offset);
+    launch_pdl(rmsnorm_f32_kernel<T>, dim3((unsigned)T_), dim3(D >= 1024 ? 256 : 128), 0, st, (const float*)x32, (const T*)w, (const T*)w2, (T*)y, (T*)y2, (int)D, eps, offset);
 }
 template <typename T> static void run_epilogue(const LinearArgs& a, const void* y, cudaStream_t st) {
     if constexpr (sizeof(T) == 2) {
@@ -121,13 +122,17 @@ template <typename T> static void run_epilogue(const LinearArgs& a, const void* 
     const size_t pairs = (size_t)a.M * (a.N >> 1);
     linear_epilogue_kernel<T><<<(unsigned)((pairs + 255) / 256), 256, 0, st>>>(a, (const T*)y);
 }
-template <typename T> static void run_prep(const AttnPrepArgs& a, int64_t T_, cudaStream_t st) { attn_prep_kernel<T><<<(unsigned)T_, 128, 0, st>>>(a); }
+template <typename T> static void run_prep(const AttnPrepArgs& a, int64_t T_, cudaStream_t st) {
+    // few tokens (decode): a warp per head, so that no head waits for another; many: four warps walk the heads, tokens fill the chip
+    const int warps = T_ >= 1024 ? 4 : (int)std::min<int64_t>(32, std::max(4, a.H + a.G));
+    launch_pdl(attn_prep_kernel<T>, dim3((unsigned)T_), dim3(32 * warps), 0, st, a);
+}
 // the partial results in a.scratch -> a.out
 template <typename T> static void run_attn_merge(const AttnArgs& a, cudaStream_t st) {
     if (a.maps > 1) attn_diff_merge_kernel<T><<<(unsigned)(a.T * a.H), AD_THREADS, 0, st>>>(a);
     else
-        attn_merge_kernel<T><<<dim3((unsigned)(a.T * a.H), (unsigned)((a.e + 127) / 128)), 128, 0, st>>>(a.scratch, (T*)a.out, a.splits, a.e, a.sigmoid, a.sink, a.H, a.gate,
-                                                                                                    a.gate_pitch, a.gate_entry);
+        launch_pdl(attn_merge_kernel<T>, dim3((unsigned)(a.T * a.H), (unsigned)((a.e + 127) / 128)), dim3(128), 0, st, (const float*)a.scratch, (T*)a.out, a.splits, a.e, a.sigmoid, a.sink,
+                   a.H, a.gate, a.gate_pitch, a.gate_entry);
 }
 template <typename T> static void run_attn(const AttnArgs& a, size_t smem, cudaStream_t st) {
     attn_bias_kernel<T><<<dim3((unsigned)(a.T * a.H * a.maps), (unsigned)a.splits), AT_WARPS * 32, smem, st>>>(a);
@@ -135,7 +140,7 @@ template <typename T> static void run_attn(const AttnArgs& a, size_t smem, cudaS
 }
 template <typename T> static void run_headnorm(const void* o32, const void* w, const void* g, int64_t g_pitch, int64_t g_off, void* y, int64_t T_,
                                                int64_t N, float eps, cudaStream_t st) {
-    gated_headnorm_kernel<T><<<(unsigned)T_, 128, 0, st>>>((const float*)o32, (const T*)w, (const T*)g, (int)g_pitch, (int)g_off, (T*)y, (int)N, eps);
+    launch_pdl(gated_headnorm_kernel<T>, dim3((unsigned)T_), dim3(N > 1024 ? 256 : 128), 0, st, (const float*)o32, (const T*)w, (const T*)g, (int)g_pitch, (int)g_off, (T*)y, (int)N, eps);
 }
 
 template <typename T, int HPW> static cudaError_t run_latent_decode(const LatentDecodeArgs& a, void* out, const float* sink, size_t smem, cudaStream_t st) {

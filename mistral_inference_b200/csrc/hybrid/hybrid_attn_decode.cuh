@@ -28,6 +28,8 @@ __global__ void __launch_bounds__(DA_WARPS * 32) attn_decode_mma_kernel(AttnArgs
     constexpr int KP = MAPS * D + 8, VP = E + 8, STAGE = DA_KEYS * (KP + VP);
     constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
     extern __shared__ __align__(16) unsigned char da_smem[];
+    pdl_trigger();
+    pdl_wait();
     const int b = blockIdx.x / a.G, g = blockIdx.x % a.G, R = a.H / a.G, split = blockIdx.y;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
     bf16* const mine = reinterpret_cast<bf16*>(da_smem) + warp * DA_STAGES * STAGE;
@@ -211,8 +213,7 @@ template <int D, int E, int MAPS, bool BIAS = false> inline cudaError_t run_attn
         const cudaError_t e = cudaFuncSetAttribute(attn_decode_mma_kernel<D, E, MAPS, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e) return e;
     }
-    attn_decode_mma_kernel<D, E, MAPS, BIAS><<<dim3((unsigned)(a.B * a.G), (unsigned)a.splits), DA_WARPS * 32, smem, st>>>(a);
-    return cudaGetLastError();
+    return launch_pdl(attn_decode_mma_kernel<D, E, MAPS, BIAS>, dim3((unsigned)(a.B * a.G), (unsigned)a.splits), dim3(DA_WARPS * 32), smem, st, a);
 }
 
 // true when a (D, E, maps) instantiation exists; launches it (partial results only)

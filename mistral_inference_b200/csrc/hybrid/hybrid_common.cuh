@@ -99,4 +99,25 @@ __device__ __forceinline__ float softplus_exact(float x) { return fmaxf(x, 0.f) 
 // cap * tanh(x / cap) through one exponential: tanh(y) = 1 - 2 / (1 + e^(2y)), off by about 1e-7 * cap
 __device__ __forceinline__ float softcap_fast(float x, float cap, float two_over_cap) { return cap - __fdividef(2.f * cap, 1.f + __expf(x * two_over_cap)); }
 
+// Programmatic dependent launch: a kernel launched through launch_pdl may start while its predecessor in the stream still runs; up to pdl_wait() it
+// touches nothing that an earlier kernel writes (weights only).  pdl_wait() returns when the predecessor has completed and its writes are
+// visible.  Both are no-ops in a kernel launched the ordinary way.  A decode step is some 80 short kernels: their launches and first loads
+// otherwise stand in the open.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
+
 }  // namespace mbh

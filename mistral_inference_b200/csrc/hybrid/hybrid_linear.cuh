@@ -20,7 +20,7 @@
 // Linear); accumulation is fp32 in both modes.
 //
 // Kernels: `linear_tiled_mma` (bf16) and `linear_f32_parts` (fp32, hybrid_linear_f32.cuh) for prompts, any shape; `linear_skinny` (M <= 8 rows, FMA,
-// one warp per pair of weight rows) and `linear_skinny_mma` (bf16, 3..8 rows, tensor cores) for decode: every weight byte is read
+// one warp per pair of weight rows) and `linear_skinny_mma` (bf16, up to 16 rows, tensor cores) for decode: every weight byte is read
 // once with 16-byte loads; `linear_decay_mma` for decays from a low rank; `linear_epilogue8_kernel` (bf16, eight columns per thread) and
 // `linear_epilogue_kernel` apply the epilogues to the output of another GEMM (the main library's
 // tcgen05 GEMM takes the large aligned bf16 Linears of prompts, see _abi_hybrid.linear).
@@ -337,42 +337,75 @@ __global__ void __launch_bounds__(SK_WARPS * 32) linear_skinny(LinearArgs a) {
         }
 }
 
-// ------------------------------------------------------------------------------------------------ skinny on tensor cores (bf16, 3..8 rows)
-// y^T = W x^T: the 16 weight rows of a CTA are the M side of m16n8k16 tiles, the (up to 8) tokens the N side, so a decode batch
+// ------------------------------------------------------------------------------------------------ skinny on tensor cores (bf16, 1..16 rows)
+// y^T = W x^T: the 16 weight rows of a CTA are the M side of m16n8k16 tiles, the (up to 8 NT) tokens the N side, so a decode batch
 // costs one tensor-core instruction per 16 x 16 weights instead of 8 FMAs per weight.  The CTA's warps split K; every lane
-// loads 16 contiguous bytes of two weight rows and of one token's activations per step -- the k order inside a step is
+// loads 16 contiguous bytes of two weight rows and of a token's activations per step -- the k order inside a step is
 // permuted identically for both operands, which a dot product does not notice.  Needs K % 8 == 0 and 16-byte aligned rows.
-constexpr int SKM_WARPS = 8;
+// Bound by memory latency more than by bandwidth (a CTA has 8 to 32 steps of 8 KB): the weights of the first SKM_AHEAD steps -- all of them up to
+// K = 2048 -- are requested before the wait for the predecessor's output, later ones as their registers come free.
+constexpr int SKM_WARPS = 8, SKM_AHEAD = 8, SKM_MAX_M = 16;
 
-__global__ void __launch_bounds__(SKM_WARPS * 32) linear_skinny_mma(LinearArgs a) {
-    __shared__ float part[SKM_WARPS][16][9];
+__device__ __forceinline__ uint4 load_weights(const bf16* p) {  // read once: not kept in L1
+    uint4 r;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
+    return r;
+}
+
+template <int NT>
+__global__ void __launch_bounds__(SKM_WARPS * 32, 2) linear_skinny_mma(LinearArgs a) {
+    __shared__ float part[SKM_WARPS][16][8 * NT + 1];
     const bf16* X = static_cast<const bf16*>(a.x);
     const bf16* W = static_cast<const bf16*>(a.w);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
-    const int n0 = blockIdx.x * 16;
-    const bf16* wa = W + (size_t)min(n0 + gid, a.N - 1) * a.K;
-    const bf16* wb = W + (size_t)min(n0 + gid + 8, a.N - 1) * a.K;
-    const bool xrow = gid < a.M;
-    const bf16* xr = X + (size_t)(xrow ? gid : 0) * a.x_pitch();
-    float c[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4  // four steps of loads in flight per warp: the kernel waits on global memory, not on the tensor pipe
-    for (int kb = warp * 32; kb < a.K; kb += SKM_WARPS * 32) {
-        const int k = kb + tig * 8;
-        uint4 va = make_uint4(0, 0, 0, 0), vb = va, vx = va;
-        if (k < a.K) {
-            va = *reinterpret_cast<const uint4*>(wa + k);
-            vb = *reinterpret_cast<const uint4*>(wb + k);
-            if (xrow) vx = *reinterpret_cast<const uint4*>(xr + k);
-        }
-        const uint32_t a0[4] = {va.x, vb.x, va.y, vb.y}, a1[4] = {va.z, vb.z, va.w, vb.w};
-        mma_bf16(c, a0, vx.x, vx.y);
-        mma_bf16(c, a1, vx.z, vx.w);
+    const int n0 = blockIdx.x * 16, k0 = warp * 32 + tig * 8;
+    constexpr int STEP = SKM_WARPS * 32;
+    const bf16* wa = W + (size_t)min(n0 + gid, a.N - 1) * a.K + k0;
+    const bf16* wb = W + (size_t)min(n0 + gid + 8, a.N - 1) * a.K + k0;
+    uint4 va[SKM_AHEAD], vb[SKM_AHEAD];
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int u = 0; u < SKM_AHEAD; ++u) {
+        const bool ok = k0 + u * STEP < a.K;
+        va[u] = ok ? load_weights(wa + u * STEP) : zero;
+        vb[u] = ok ? load_weights(wb + u * STEP) : zero;
     }
-    part[warp][gid][tig * 2] = c[0]; part[warp][gid][tig * 2 + 1] = c[1];
-    part[warp][gid + 8][tig * 2] = c[2]; part[warp][gid + 8][tig * 2 + 1] = c[3];
+    pdl_trigger();
+    pdl_wait();
+    float c[NT][4];
+    const bf16* xr[NT];
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+        c[t][0] = c[t][1] = c[t][2] = c[t][3] = 0.f;
+        xr[t] = X + (size_t)min(t * 8 + gid, a.M - 1) * a.x_pitch() + k0;  // rows past the end repeat the last one: their sums go nowhere
+    }
+    const int steps = (a.K + STEP - 1) / STEP;
+    for (int i = 0; i < steps; i += SKM_AHEAD) {
+#pragma unroll
+        for (int u = 0; u < SKM_AHEAD; ++u) {
+            const int k = (i + u) * STEP;
+            uint4 vx[NT];
+#pragma unroll
+            for (int t = 0; t < NT; ++t) vx[t] = k0 + k < a.K ? *reinterpret_cast<const uint4*>(xr[t] + k) : zero;
+            const uint32_t a0[4] = {va[u].x, vb[u].x, va[u].y, vb[u].y}, a1[4] = {va[u].z, vb[u].z, va[u].w, vb[u].w};
+#pragma unroll
+            for (int t = 0; t < NT; ++t) {
+                mma_bf16(c[t], a0, vx[t].x, vx[t].y);
+                mma_bf16(c[t], a1, vx[t].z, vx[t].w);
+            }
+            const bool more = k0 + k + SKM_AHEAD * STEP < a.K;
+            va[u] = more ? load_weights(wa + k + SKM_AHEAD * STEP) : zero;
+            vb[u] = more ? load_weights(wb + k + SKM_AHEAD * STEP) : zero;
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+        part[warp][gid][t * 8 + tig * 2] = c[t][0]; part[warp][gid][t * 8 + tig * 2 + 1] = c[t][1];
+        part[warp][gid + 8][t * 8 + tig * 2] = c[t][2]; part[warp][gid + 8][t * 8 + tig * 2 + 1] = c[t][3];
+    }
     __syncthreads();
-    if (threadIdx.x < 64) {
-        const int m = threadIdx.x & 7, r = (threadIdx.x >> 3) * 2, n = n0 + r;
+    if (threadIdx.x < 64 * NT) {
+        const int m = threadIdx.x % (8 * NT), r = threadIdx.x / (8 * NT) * 2, n = n0 + r;
         if (m < a.M && n < a.N) {
             float s0 = 0.f, s1 = 0.f;
 #pragma unroll
@@ -487,9 +520,9 @@ template <typename T>
 inline cudaError_t launch_linear(const LinearArgs& a, cudaStream_t st) {
     if (a.M <= 0 || a.N <= 0) return cudaSuccess;
     if constexpr (sizeof(T) == 2) {
-        if (a.M > 2 && a.M <= 8 && a.K % 8 == 0 && a.x_pitch() % 8 == 0 && (reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.w)) % 16 == 0) {
-            linear_skinny_mma<<<(a.N + 15) / 16, SKM_WARPS * 32, 0, st>>>(a);
-            return cudaGetLastError();
+        if (a.M <= SKM_MAX_M && a.K % 8 == 0 && a.x_pitch() % 8 == 0 && (reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.w)) % 16 == 0) {
+            const dim3 grid((a.N + 15) / 16);
+            return a.M <= 8 ? launch_pdl(linear_skinny_mma<1>, grid, dim3(SKM_WARPS * 32), 0, st, a) : launch_pdl(linear_skinny_mma<2>, grid, dim3(SKM_WARPS * 32), 0, st, a);
         }
     }
     if (a.M <= SK_MAX_M) {

@@ -22,8 +22,24 @@ namespace mbh {
 // ------------------------------------------------------------------------------------------------ embedding, norm
 template <typename T, bool ADD = false>
 __global__ void embed_scale_kernel(const int64_t* __restrict__ tok, const T* __restrict__ E, float scale, float* __restrict__ x, int D) {
+    pdl_trigger();
+    pdl_wait();
     const T* row = E + (size_t)tok[blockIdx.x] * D;
     float* o = x + (size_t)blockIdx.x * D;
+    if (D % 4 == 0 && (reinterpret_cast<uintptr_t>(E) | reinterpret_cast<uintptr_t>(x)) % 16 == 0) {  // four columns per thread and step
+#pragma unroll 4
+        for (int i = threadIdx.x * 4; i < D; i += blockDim.x * 4) {
+            float v[4];
+            load4(row + i, v);
+            float4 u = make_float4(v[0] * scale, v[1] * scale, v[2] * scale, v[3] * scale);
+            if (ADD) {
+                const float4 old = *reinterpret_cast<const float4*>(o + i);
+                u = make_float4(old.x + u.x, old.y + u.y, old.z + u.z, old.w + u.w);
+            }
+            *reinterpret_cast<float4*>(o + i) = u;
+        }
+        return;
+    }
     for (int i = threadIdx.x; i < D; i += blockDim.x) {
         const float v = to_f(row[i]) * scale;
         o[i] = ADD ? o[i] + v : v;
@@ -58,6 +74,8 @@ template <typename T>
 __global__ void rmsnorm_f32_kernel(const float* __restrict__ x, const T* __restrict__ w, const T* __restrict__ w2, T* __restrict__ y, T* __restrict__ y2, int D,
                                    float eps, float offset) {
     __shared__ float red[32];
+    pdl_trigger();
+    pdl_wait();
     const float* r = x + (size_t)blockIdx.x * D;
     T* o = y + (size_t)blockIdx.x * D;
     T* o2 = y2 ? y2 + (size_t)blockIdx.x * D : nullptr;
@@ -129,6 +147,8 @@ struct AttnPrepArgs {
 
 template <typename T>
 __global__ void attn_prep_kernel(AttnPrepArgs a) {
+    pdl_trigger();
+    pdl_wait();
     const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const int Nq = a.H * a.d, Nk = a.G * a.d, Nv = a.G * a.e;
     const T* row = static_cast<const T*>(a.qkv) + (size_t)t * (Nq + Nk + Nv);
@@ -136,22 +156,35 @@ __global__ void attn_prep_kernel(AttnPrepArgs a) {
     const int crow = a.cache_rows ? a.cache_rows[t] : -1;
     float temp = 1.f;
     if (a.temp_every > 0) temp = 1.f + a.temp_coef * logf((float)((pos + 1) / a.temp_every + 1));
+    constexpr int KEEP = 4;  // entries of a head per lane that stay in registers between the two passes
     for (int h = warp; h < a.H + a.G; h += nw) {
         const bool is_q = h < a.H;
         const T* src = row + (is_q ? h * a.d : Nq + (h - a.H) * a.d);
         const T* nwgt = static_cast<const T*>(is_q ? a.qnorm : a.knorm);
-        float ss = 0.f;
-        for (int i = lane; i < a.d; i += 32) { float v = to_f(src[i]); ss = fmaf(v, v, ss); }
+        float ss = 0.f, keep[KEEP], wk[KEEP];
+#pragma unroll
+        for (int k = 0; k < KEEP; ++k) {
+            const int i = lane + 32 * k;
+            keep[k] = i < a.d ? to_f(src[i]) : 0.f;
+            wk[k] = i < a.d && nwgt ? to_f(nwgt[i]) : 1.f;
+        }
+#pragma unroll
+        for (int k = 0; k < KEEP; ++k) ss = fmaf(keep[k], keep[k], ss);
+        for (int i = lane + 32 * KEEP; i < a.d; i += 32) { float v = to_f(src[i]); ss = fmaf(v, v, ss); }
         ss = warp_sum(ss);
         const float inv = nwgt ? 1.f / sqrtf(ss / (float)a.d + a.eps) : 1.f;
         T* dst;
         if (is_q) dst = static_cast<T*>(a.q_out) + (size_t)t * Nq + h * a.d;
         else { if (crow < 0) continue; dst = static_cast<T*>(a.cache_k) + (size_t)crow * Nk + (h - a.H) * a.d; }
-        for (int i = lane; i < a.d; i += 32) {
-            float v = to_f(src[i]) * inv * (nwgt ? to_f(nwgt[i]) : 1.f);
+        auto emit = [&](int i, float x, float w) {
+            float v = x * inv * w;
             if (is_q) v = rnd<T>(v) * temp;
             dst[i] = from_f<T>(v);
-        }
+        };
+#pragma unroll
+        for (int k = 0; k < KEEP; ++k)
+            if (lane + 32 * k < a.d) emit(lane + 32 * k, keep[k], wk[k]);
+        for (int i = lane + 32 * KEEP; i < a.d; i += 32) emit(i, to_f(src[i]), nwgt ? to_f(nwgt[i]) : 1.f);
     }
     const T* vsrc = row + Nq + Nk;
     T* vf = static_cast<T*>(a.v_first) + (size_t)t * Nv;
@@ -412,6 +445,8 @@ __global__ void attn_merge_kernel(const float* __restrict__ scratch, T* __restri
                                   int H = 1, const void* gate = nullptr, int gate_pitch = 0, int gate_entry = 0) {
     __shared__ float f[AT_MAX_SPLITS];
     __shared__ float red[32];
+    pdl_trigger();
+    pdl_wait();
     const float* part = scratch + (size_t)blockIdx.x * splits * (2 + e);
     float M = -INFINITY;
     for (int s = threadIdx.x & 31; s < splits; s += 32) M = fmaxf(M, part[(size_t)s * (2 + e)]);
@@ -514,6 +549,8 @@ constexpr int LS_TB = 16, LS_THREADS = 128;
 template <typename T, int DMAX>
 __global__ void __launch_bounds__(LS_THREADS) lightning_scan_kernel(LightningArgs a) {
     constexpr int R = 2 * LS_TB * DMAX / LS_THREADS;  // staged values per thread and tile
+    pdl_trigger();
+    pdl_wait();
     __shared__ __align__(16) float ks[LS_TB][DMAX], qs[LS_TB][DMAX];
     const int b = blockIdx.x / a.H, h = blockIdx.x % a.H;
     const int c = blockIdx.y * LS_THREADS + threadIdx.x;
@@ -581,14 +618,43 @@ template <typename T>
 __global__ void gated_headnorm_kernel(const float* __restrict__ o, const T* __restrict__ w, const T* __restrict__ g, int g_pitch, int g_off,
                                       T* __restrict__ y, int N, float eps) {
     __shared__ float red[32];
+    pdl_trigger();
+    pdl_wait();
     const float* r = o + (size_t)blockIdx.x * N;
     const T* gr = g + (size_t)blockIdx.x * g_pitch + g_off;
+    T* out = y + (size_t)blockIdx.x * N;
     float ss = 0.f;
+    constexpr int KEEP = 4;  // steps of four columns per thread, all loads of a row in flight at once
+    if (N % 4 == 0 && N <= KEEP * 4 * (int)blockDim.x && g_pitch % 4 == 0 && g_off % 4 == 0 &&
+        ((reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(y)) % 16 == 0)) {
+        float v[KEEP][4], gv[KEEP][4], wv[KEEP][4];
+#pragma unroll
+        for (int k = 0; k < KEEP; ++k) {
+            const int i = (k * blockDim.x + threadIdx.x) * 4;
+            if (i < N) { load4(r + i, v[k]); load4(gr + i, gv[k]); load4(w + i, wv[k]); }
+            else v[k][0] = v[k][1] = v[k][2] = v[k][3] = 0.f;
+        }
+#pragma unroll
+        for (int k = 0; k < KEEP; ++k)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) ss = fmaf(v[k][u], v[k][u], ss);
+        ss = block_sum(ss, red);
+        const float inv = 1.f / sqrtf(ss / (float)N + eps);
+#pragma unroll
+        for (int k = 0; k < KEEP; ++k) {
+            const int i = (k * blockDim.x + threadIdx.x) * 4;
+            if (i >= N) break;
+            float u[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) u[c] = v[k][c] * inv * wv[k][c] * sigmoid_exact(gv[k][c]);
+            store4<T>(out + i, u);
+        }
+        return;
+    }
     for (int i = threadIdx.x; i < N; i += blockDim.x) ss = fmaf(r[i], r[i], ss);
     ss = block_sum(ss, red);
     const float inv = 1.f / sqrtf(ss / (float)N + eps);
-    for (int i = threadIdx.x; i < N; i += blockDim.x)
-        y[(size_t)blockIdx.x * N + i] = from_f<T>(r[i] * inv * to_f(w[i]) * sigmoid_exact(to_f(gr[i])));
+    for (int i = threadIdx.x; i < N; i += blockDim.x) out[i] = from_f<T>(r[i] * inv * to_f(w[i]) * sigmoid_exact(to_f(gr[i])));
 }
 
 }  // namespace mbh
