@@ -131,6 +131,17 @@ int mb200_lm_head(const void* x, const void* norm_w, const void* w_out, float* l
                   int64_t vocab, float eps, void* workspace, size_t workspace_bytes, void* stream);
 
 /* ---------------------------------------------------------------------------------------------
+ * Scoring: final RMSNorm + lm head + log-softmax + gather in one pass, the logits never written (generate.py:97-118).  T >= 128, dim % 64 == 0,
+ * vocab % 128 == 0.
+ *   out [T] fp32: log_softmax(logits[t])[target[t]] where target[t] >= 0 (others untouched)
+ *   keep_row [T] int32: row of kept_logits [., vocab] fp32 that takes row t's logits, or -1
+ *   partial [T * vocab / 64 * 2], target_logit [T]: fp32 scratch
+ */
+int mb200_lm_head_logprobs(const void* x, const void* norm_w, const void* w_out, const int64_t* target_dev, const int32_t* keep_row_dev, float* kept_logits,
+                           float* out_dev, float* partial, float* target_logit, int64_t T, int64_t dim, int64_t vocab, float eps, void* workspace,
+                           size_t workspace_bytes, void* stream);
+
+/* ---------------------------------------------------------------------------------------------
  * Device-side step state of the batched decode loop.  Replaces BufferCache.get_input_metadata for one-token steps
  * (cache.py:197-263: positions, cache_positions, the padded-keys mask's kv_seqlen) and update_seqlens
  * (cache.py:191-192) with one tiny kernel, so a CUDA graph of the decode step replays without host writes.

@@ -37,6 +37,8 @@ _SIGNATURES = {
                                  c_void_p]),
     "mb200_lm_head": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_float, c_void_p, c_size_t,
                               c_void_p]),
+    "mb200_lm_head_logprobs": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64,
+                                       c_float, c_void_p, c_size_t, c_void_p]),
     "mb200_decode_meta": (c_int, [c_void_p, c_void_p, c_int64, c_void_p, c_int64, c_void_p]),
     "mb200_argmax_rows": (c_int, [c_void_p, c_void_p, c_int64, c_int64, c_void_p]),
     "mb200_logprob_gather": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_void_p]),
@@ -222,6 +224,21 @@ def lm_head(x, norm_w, w_out, logits, eps, ws: Workspace) -> None:
     T, dim = x.shape
     _check(lib().mb200_lm_head(_ptr(x), _ptr(norm_w), _ptr(w_out), _ptr(logits), T, dim, w_out.shape[0], eps, ws.ptr, ws.nbytes,
                                _stream()), "mb200_lm_head")
+
+
+def lm_head_logprobs_ok(T: int, dim: int, vocab: int) -> bool:
+    return T >= 128 and dim % 64 == 0 and vocab % 128 == 0 and os.environ.get("MB200_GEMM", "")[:1] != "m"
+
+
+def lm_head_logprobs(x, norm_w, w_out, target, keep_row, kept_logits, out, eps, ws: Workspace) -> None:
+    """out[t] = log_softmax(head(norm(x)))[t, target[t]] where target[t] >= 0; rows with keep_row[t] >= 0 leave their logits in kept_logits."""
+    T, dim = x.shape
+    V = w_out.shape[0]
+    assert target.dtype == torch.long and keep_row.dtype == torch.int32 and kept_logits.dtype == torch.float32 and kept_logits.shape[1] == V and out.dtype == torch.float32
+    partial = torch.empty(T * (V // 64) * 2, dtype=torch.float32, device=x.device)
+    target_logit = torch.empty(T, dtype=torch.float32, device=x.device)
+    _check(lib().mb200_lm_head_logprobs(_ptr(x), _ptr(norm_w), _ptr(w_out), _ptr(target), _ptr(keep_row), _ptr(kept_logits), _ptr(out), _ptr(partial),
+                                        _ptr(target_logit), T, dim, V, eps, ws.ptr, ws.nbytes, _stream()), "mb200_lm_head_logprobs")
 
 
 def argmax_rows(logits: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:

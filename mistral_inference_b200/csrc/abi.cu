@@ -292,6 +292,37 @@ int mb200_lm_head(const void* x, const void* norm_w, const void* w_out, float* l
   return run_linear<EPI_F32>(x, norm_w, w_out, e, T, vocab, dim, eps, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
+int mb200_lm_head_logprobs(const void* x, const void* norm_w, const void* w_out, const int64_t* target_dev, const int32_t* keep_row_dev, float* kept_logits,
+                           float* out_dev, float* partial, float* target_logit, int64_t T, int64_t dim, int64_t vocab, float eps, void* workspace,
+                           size_t workspace_bytes, void* stream) {
+  MB_CHECK_ARG(x && norm_w && w_out && target_dev && keep_row_dev && kept_logits && out_dev && partial && target_logit, "lm_head_logprobs: null pointer");
+  MB_CHECK_ARG(T >= TG_BM && vocab % 128 == 0 && dim % TG_BK == 0, "lm_head_logprobs: T=%lld dim=%lld vocab=%lld (T >= 128, dim %% 64, vocab %% 128)",
+               (long long)T, (long long)dim, (long long)vocab);
+  cudaStream_t st = (cudaStream_t)stream;
+  const size_t need = kWsHeader + SK_PARTIAL_BYTES + align256((size_t)T * dim * 2);
+  if (workspace == nullptr || workspace_bytes < need) return fail(MB200_E_WORKSPACE, "lm_head_logprobs: workspace %zu < %zu", workspace_bytes, need);
+  void* normed = (uint8_t*)workspace + kWsHeader + SK_PARTIAL_BYTES;
+  int rc = run_rmsnorm(x, norm_w, normed, T, dim, eps, st);
+  if (rc) return rc;
+  GemmParams g;
+  g.a = normed;
+  g.w = w_out;
+  g.T = (int)T;
+  g.N = (int)vocab;
+  g.K = (int)dim;
+  g.epi.out_f32 = kept_logits;
+  g.epi.ld_out = vocab;
+  g.epi.target = (const long long*)target_dev;
+  g.epi.keep_row = keep_row_dev;
+  g.epi.partial = (float2*)partial;
+  g.epi.target_logit = target_logit;
+  rc = launch_gemm_tcgen05_prompt<EPI_LOGPROB>(g, st);
+  if (rc) return rc;
+  logprob_combine_kernel<<<(unsigned)ceil_div(T, 8), 256, 0, st>>>((const float2*)partial, target_logit, (const long long*)target_dev, out_dev, (int)T, (int)(vocab / 64));
+  MB_CHECK_LAUNCH("logprob_combine_kernel");
+  return MB200_OK;
+}
+
 int mb200_argmax_rows(const float* logits, int64_t* out_dev, int64_t T, int64_t vocab, void* stream) {
   MB_CHECK_ARG(logits && out_dev && T >= 0 && vocab >= 1, "argmax_rows: bad arguments");
   if (T == 0) return MB200_OK;

@@ -15,6 +15,8 @@ enum EpiMode : int {
   EPI_QKV_ROPE = 4,  // split into q/k/v, rotate q,k pairs, optional ring scatter  (transformer_layers.py:66-70, cache.py:91-92)
   EPI_MOE_SCALE = 5, // yw[row, n] = bf16( w[row] * bf16(acc) ), stored on every rank of an expert-parallel group  (moe.py:31)
   EPI_LAYER = 6,     // the Linears of layered decoders: bias, then the step named by EpiParams::layer (LayerEpi)
+  EPI_LOGPROB = 7,   // scoring: the logits bf16(acc) of 64 columns -> (maximum, sum of exp(. - maximum)), the target's logit, whole rows of
+                     // logits only where asked for                              (generate.py:97-118)
 };
 
 // What follows a layered decoder's Linear (numbers shared with csrc/hybrid/hybrid_linear.cuh, which states the formulas).
@@ -42,6 +44,11 @@ struct EpiParams {
   const void* row_w = nullptr;  // bf16 [rows]
   void* peer_out[kMaxPeers] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   int n_peers = 0;
+  // EPI_LOGPROB
+  const long long* target = nullptr;     // [T]: rows with a negative target need no partial sums
+  const int32_t* keep_row = nullptr;     // [T]: row of out_f32 that takes this row's logits, or -1
+  float2* partial = nullptr;             // [T, N / 64]
+  float* target_logit = nullptr;         // [T]
   // EPI_LAYER
   int layer = 0, n_act = 0;              // LayerEpi; columns below n_act go through SiLU (LAYER_STORE)
   float limit = 0.f, alpha = 0.f;
@@ -130,6 +137,39 @@ __device__ __forceinline__ void epi_prefetch128(const EpiParams& p, int t, int n
       for (int i = 0; i < 4; ++i) prefetch_l1(cs + 128 * i);
     }
     if (n0 >= p.q_dim && p.cache_rows != nullptr) prefetch_l1(p.cache_rows + t);
+  }
+}
+
+// EPI_LOGPROB, columns n .. n + 31 of row t.  m, s: running maximum and sum of this row's current 64 columns.
+__device__ __forceinline__ void epi_logprob32(const EpiParams& p, int t, int n, const uint32_t (&v)[32], long long tgt, int keep, float& m, float& s) {
+  float y[32];
+#pragma unroll
+  for (int j = 0; j < 32; ++j) y[j] = round_bf16(__uint_as_float(v[j]));
+  if (keep >= 0) {
+    float4* dst = reinterpret_cast<float4*>(p.out_f32 + (int64_t)keep * p.ld_out + n);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) dst[q] = make_float4(y[4 * q], y[4 * q + 1], y[4 * q + 2], y[4 * q + 3]);
+  }
+  if (tgt < 0) return;
+  float mx = y[0];
+#pragma unroll
+  for (int j = 1; j < 32; ++j) mx = fmaxf(mx, y[j]);
+  mx = fmaxf(m, mx);
+  if (mx != -INFINITY) {
+    float a0 = 0.f, a1 = 0.f;
+#pragma unroll
+    for (int j = 0; j < 32; j += 2) {
+      a0 += expf(y[j] - mx);
+      a1 += expf(y[j + 1] - mx);
+    }
+    s = s * expf(m - mx) + (a0 + a1);
+    m = mx;
+  }
+  if (tgt >= n && tgt < n + 32) {
+    float x = 0.f;
+#pragma unroll
+    for (int j = 0; j < 32; ++j) x = n + j == (int)tgt ? y[j] : x;
+    p.target_logit[t] = x;
   }
 }
 

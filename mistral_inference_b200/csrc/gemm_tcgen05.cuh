@@ -340,7 +340,25 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
       const uint32_t trow = tmem_base + ((uint32_t)lane_base << 16) + acc * TG_BN;
       uint32_t va[32], vb[32];
       tmem_ld_32x32b_x32_nowait(trow, va);
-      if constexpr (MODE == EPI_LAYER) {
+      if constexpr (MODE == EPI_LOGPROB) {
+        const bool live = t < p.T;
+        const long long tgt = live ? p.epi.target[t] : -1;
+        const int keep = live ? p.epi.keep_row[t] : -1;
+        float m = -INFINITY, sum = 0.f;
+#pragma unroll 1
+        for (int c = 0; c < TG_BN / 32; ++c) {
+          tmem_wait_ld();
+#pragma unroll
+          for (int j = 0; j < 32; ++j) vb[j] = va[j];
+          if (c + 1 < TG_BN / 32) tmem_ld_32x32b_x32_nowait(trow + (c + 1) * 32, va);
+          if (live) epi_logprob32(p.epi, t, n0 + c * 32, vb, tgt, keep, m, sum);
+          if (c & 1) {
+            if (tgt >= 0) p.epi.partial[(int64_t)t * (p.N / 64) + (n0 + c * 32) / 64] = make_float2(m, sum);
+            m = -INFINITY;
+            sum = 0.f;
+          }
+        }
+      } else if constexpr (MODE == EPI_LAYER) {
         const bool f32 = layer_step_is_f32(p.epi.layer);
         const int rows = store ? max(0, min(32, p.T - m0 - lane_base)) : 0;
         float4* stg = reinterpret_cast<float4*>(reinterpret_cast<uint8_t*>(full) + 512) + (warp & 3) * 256;

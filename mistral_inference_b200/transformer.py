@@ -4,6 +4,7 @@
 on-disk contract (params.json + consolidated.safetensors | consolidated.00.pth, reference state-dict keys);
 the layer loop calls the fused libmb200 kernels.  bf16 on CUDA only; there is no PyTorch/CPU fallback.
 """
+import itertools
 import json
 import logging
 import math
@@ -16,11 +17,12 @@ from torch import nn
 
 from . import _abi
 from .args import TransformerArgs
-from .cache import BufferCache, CacheInputMetadata
+from .cache import BufferCache, CacheInputMetadata, upload
 from .rope import precompute_freqs_cis
 from .transformer_layers import RMSNorm, TransformerBlock
 
 ROPE_TABLE_LEN = 128_000  # transformer.py:116
+SCORE_BLOCK_TOKENS = 4096  # rows of the lm head per scoring call: bounds the partial sums (67 MB at a vocabulary of 131072)
 _NVTX = os.environ.get("MB200_NVTX", "0") == "1"
 
 
@@ -164,7 +166,7 @@ class Transformer(nn.Module):
             input_metadata = cache.get_input_metadata(seqlens)
             positions = input_metadata[0].positions
         else:
-            positions = torch.cat([torch.arange(0, s, dtype=torch.int32) for s in seqlens]).to(self.device)
+            positions = upload(torch.cat([torch.arange(0, s, dtype=torch.int32) for s in seqlens]), self.device)
 
         if self.pipeline_rank == 0:
             assert self.tok_embeddings is not None
@@ -228,7 +230,7 @@ class Transformer(nn.Module):
                 input_metadata = cache.get_input_metadata(seqlens)
             positions = input_metadata[0].positions
         else:
-            positions = torch.cat([torch.arange(0, s, dtype=torch.int32) for s in seqlens]).to(self.device)
+            positions = upload(torch.cat([torch.arange(0, s, dtype=torch.int32) for s in seqlens]), self.device)
         assert self.tok_embeddings is not None
         h = self.tok_embeddings(input_ids)
         rope = self.rope_table
@@ -403,30 +405,51 @@ class Transformer(nn.Module):
                          targets: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
         """One prompt chunk for generate(): returns (lp [T] fp32 with lp[t] = log_softmax(logits[t])[targets[t]] where
         targets[t] >= 0, logits [B, V] fp32 of each sequence's last token).  Replaces forward + log_softmax over [T, V] +
-        per-token gathers (generate.py:97-118): the lm head runs over blocks of rows, each followed by the fused
-        log-softmax + gather kernel, so the full [T, V] logits never exist."""
+        per-token gathers (generate.py:97-118).  From 128 tokens on the lm head's epilogue reduces the logits where they are computed
+        (blocks of up to SCORE_BLOCK_TOKENS rows) and keeps the rows of the sequences' last tokens; the [T, V] logits never exist.
+        Fewer tokens: the logits of all rows, then the fused log-softmax + gather kernel."""
         self._last_static_logits = 0
         T, V = input_ids.shape[0], self.vocab_size
-        last_idx = torch.tensor(seqlens, device=input_ids.device).cumsum(0) - 1
+        ends = list(itertools.accumulate(seqlens))
         lp = torch.zeros(T, dtype=torch.float32, device=input_ids.device)
         if self.num_pipeline_ranks > 1:  # reference-compatible pipeline mode: logits arrive by broadcast (transformer.py:236-237)
             logits = self.forward(input_ids, seqlens, cache).float().contiguous()
             _abi.logprob_gather(logits, targets, out=lp)
-            return lp, logits.index_select(0, last_idx)
+            return lp, logits.index_select(0, torch.tensor([e - 1 for e in ends], device=input_ids.device))
         self._check_runnable()
         h = self._hidden_no_norm(input_ids, seqlens, cache)
         if cache is not None:
             cache.update_seqlens(seqlens)
         assert self.norm is not None and self.output_weight is not None
-        rows = max(128, (256 << 20) // (4 * V))
         ws = self.workspace(max(T, 1))
+        if not _abi.lm_head_logprobs_ok(T, self.args.dim, V):
+            return self._logprobs_of_written_logits(h, targets, ends, lp, ws)
+        keep = torch.full((T,), -1, dtype=torch.int32)
+        keep[torch.tensor(ends) - 1] = torch.arange(len(ends), dtype=torch.int32)
+        keep = upload(keep, h.device)
+        last_logits = torch.empty(len(ends), V, dtype=torch.float32, device=h.device)
+        n = -(-T // SCORE_BLOCK_TOKENS)
+        step = -(-T // (256 * n)) * 256 if n > 1 else T  # equal blocks of whole pairs of row tiles, none below 128 rows
+        bounds = list(range(0, T, step)) + [T]
+        if n > 1 and bounds[-1] - bounds[-2] < 128:
+            del bounds[-2]
+        for r0, r1 in zip(bounds, bounds[1:]):
+            _abi.lm_head_logprobs(h[r0:r1], self.norm.weight, self.output_weight, targets[r0:r1], keep[r0:r1], last_logits, lp[r0:r1], self.args.norm_eps, ws)
+        return lp, last_logits
+
+    def _logprobs_of_written_logits(self, h: torch.Tensor, targets: torch.Tensor, ends: List[int], lp: torch.Tensor, ws: "_abi.Workspace"
+                                    ) -> Tuple[torch.Tensor, torch.Tensor]:
+        T, V = h.shape[0], self.vocab_size
+        rows = max(128, (256 << 20) // (4 * V))
         block = torch.empty(min(rows, T), V, dtype=torch.float32, device=h.device)
+        last_logits = torch.empty(len(ends), V, dtype=torch.float32, device=h.device)
         for r0 in range(0, T, rows):
             r1 = min(T, r0 + rows)
             _abi.lm_head(h[r0:r1], self.norm.weight, self.output_weight, block[: r1 - r0], self.args.norm_eps, ws)
             _abi.logprob_gather(block[: r1 - r0], targets[r0:r1], out=lp[r0:r1])
-        last_logits = torch.empty(len(seqlens), V, dtype=torch.float32, device=h.device)
-        _abi.lm_head(h.index_select(0, last_idx), self.norm.weight, self.output_weight, last_logits, self.args.norm_eps, ws)
+            for b, e in enumerate(ends):
+                if r0 < e <= r1:
+                    last_logits[b].copy_(block[e - 1 - r0])
         return lp, last_logits
 
     # ------------------------------------------------------------------ weights

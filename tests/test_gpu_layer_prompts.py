@@ -237,3 +237,30 @@ def test_decode_attention_with_a_bias(H, G, d, e, pos, n_tab):
     h.attn_bias_decode(q, ring_k, ring_v, bias, positions, slots, got, B, W, H, G, d, e, 0.2)
     h.attn_bias(q, ring_k, ring_v, bias, positions, torch.arange(B + 1, dtype=torch.int32, device=DEV), slots, exact, B, W, H, G, d, e, 0.2, splits=h.attn_splits(B, H, W))
     assert rel(got, ref) < 2 ** -9 and rel(got, ref) < 1.1 * rel(exact, ref) + 2 ** -16
+
+
+@pytest.mark.parametrize("lens", [[128], [70, 59, 1], [300, 1, 212], [513, 700]])
+def test_scoring_without_written_logits(lens, monkeypatch):
+    """Log-probabilities reduced in the lm head's epilogue against the pass over written logits: tile edges, rows without a target, blocks of rows,
+    targets at both ends of the vocabulary.  The logits are the same bf16 numbers and only sums of exponentials are taken in another order; at 128
+    rows the written logits come from the split-k kernel, whose other order of sums may flip a rounding: one bf16 step of the largest."""
+    import mistral_inference_b200 as mi
+    from mistral_inference_b200 import _abi, transformer
+
+    args = mi.TransformerArgs(dim=256, n_layers=1, head_dim=128, hidden_dim=512, n_heads=4, n_kv_heads=2, norm_eps=1e-5, vocab_size=640, max_batch_size=4)
+    m = transformer.Transformer.empty(args, DEV, torch.bfloat16)
+    g = torch.Generator(device=DEV).manual_seed(5)
+    for p in m.parameters():
+        p.normal_(0, 0.2, generator=g) if p.dim() > 1 else p.fill_(1.0)
+    T = sum(lens)
+    ids, targets = torch.randint(0, 640, (T,), device=DEV, generator=g), torch.randint(0, 640, (T,), device=DEV, generator=g)
+    targets[0], targets[1], targets[T - 1], targets[T // 2] = 0, 639, -1, -1
+    got, last = m.forward_logprobs(ids, lens, None, targets)
+    monkeypatch.setattr(transformer, "SCORE_BLOCK_TOKENS", 300)
+    got2, last2 = m.forward_logprobs(ids, lens, None, targets)
+    monkeypatch.setattr(_abi, "lm_head_logprobs_ok", lambda *a: False)
+    ref, ref_last = m.forward_logprobs(ids, lens, None, targets)
+    step = ref_last.abs().max().item() * 2 ** -7 if T == 128 else 0.0
+    assert (last - ref_last).abs().max() <= step and (last2 - ref_last).abs().max() <= step and (got[targets < 0] == 0).all()
+    for a in (got, got2):
+        assert (a - ref).abs().max() <= 1e-5 * ref.abs().max() + 2 * step
