@@ -219,6 +219,8 @@ int mb200_moe_grouped_ffn(const void* xs, const void* const* w13_host, const voi
  * Linear in its epilogue.
  * mb200_layer_linear: T >= 128 rows, N % 128 == 0, K % 64 == 0.  out: bf16 results; out32: the fp32 residual stream or fp32 results.
  *     rowscale [T, rs_pitch] fp32 or NULL: hidden unit c of row t is scaled by rowscale[t, c / rs_group].  n_act columns through SiLU.
+ *     scratch: mb200_layer_linear_scratch(T, N, K) bytes (uninitialised, this call's own), or NULL (also when that is 0): without it the last
+ *     tiles are not cut.
  * mb200_layer_moe: y32 [T, width] fp32 (+= when add) sum over the token's choices idx [T, top] < n_experts of
  *     wsel * (act W2_e^T), act = step(hn W13_e^T); w13 [E * 2 ff, width] (gate/up rows interleaved; RELU2: [E * ff, width]),
  *     w2 [width, E * ff].  The weight multiplies the hidden units (GLU: the expert's input).  width % 128 == 0, ff % 64 == 0,
@@ -235,7 +237,8 @@ int mb200_layer_attention(const void* q, const void* cache_k, const void* cache_
                           int64_t n_kv_heads, float scale, void* stream);
 #define MB200_LAYER_MOE_MAX_EXPERTS 48
 int mb200_layer_linear(const void* x, const void* w, const void* bias, void* out, float* out32, int64_t T, int64_t N, int64_t K, int epi, int64_t n_act,
-                       float limit, float alpha, const float* rowscale, int64_t rs_pitch, int64_t rs_group, void* stream);
+                       float limit, float alpha, const float* rowscale, int64_t rs_pitch, int64_t rs_group, void* scratch, void* stream);
+size_t mb200_layer_linear_scratch(int64_t T, int64_t N, int64_t K);
 int mb200_layer_moe_sizes(int64_t T, int64_t n_experts, int64_t top, int64_t* rows_cap, int64_t* plan_words);
 int mb200_layer_moe(const void* hn, const void* w13, const void* w2, const int32_t* idx, const float* wsel, int64_t T, int64_t dim, int64_t ff, int64_t n_experts,
                     int64_t top, int epi, float limit, float alpha, int32_t* slot, int32_t* plan, void* xs, float* row_w, void* act, float* rows32, float* y32,

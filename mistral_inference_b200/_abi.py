@@ -49,7 +49,8 @@ _SIGNATURES = {
     "mb200_moe_grouped_ffn": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64,
                                       c_int64, c_int64, c_int64, c_int64, c_void_p, c_void_p, c_size_t, c_void_p]),
     "mb200_layer_linear": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int, c_int64, c_float, c_float, c_void_p,
-                                   c_int64, c_int64, c_void_p]),
+                                   c_int64, c_int64, c_void_p, c_void_p]),
+    "mb200_layer_linear_scratch": (c_size_t, [c_int64, c_int64, c_int64]),
     "mb200_layer_attention_max_table": (c_int, []),
     "mb200_layer_attention": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64,
                                       c_int64, c_int64, c_int64, c_float, c_void_p]),
@@ -297,8 +298,10 @@ def layer_linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor],
                  n_act: int = 0, limit: float = 0.0, alpha: float = 0.0, rowscale: Optional[torch.Tensor] = None, group: int = 1) -> None:
     """A layered decoder's Linear over T >= 128 rows with the step that follows it in the GEMM's epilogue (include/mistral_b200.h)."""
     T, K = x.shape
+    need = lib().mb200_layer_linear_scratch(T, w.shape[0], K)
+    scratch = torch.empty(need, dtype=torch.uint8, device=x.device) if need else None
     _check(lib().mb200_layer_linear(_ptr(x), _ptr(w), _ptr(bias), _ptr(out), _ptr(out32), T, w.shape[0], K, epi, n_act, limit, alpha, _ptr(rowscale),
-                                    rowscale.shape[1] if rowscale is not None else 0, group, _stream()), "mb200_layer_linear")
+                                    rowscale.shape[1] if rowscale is not None else 0, group, _ptr(scratch), _stream()), "mb200_layer_linear")
 
 
 def layer_attention(q, cache_k, cache_v, bias, q_start, seqpos, slots, out, B: int, max_seqlen: int, H: int, KV: int, scale: float) -> None:

@@ -67,7 +67,11 @@ static int run_linear(const void* x, const void* norm_w, const void* w, const Ep
   g.K = (int)K;
   g.epi = epi;
   if (streamk_eligible(T, N, K)) return launch_streamk<MODE>(g, workspace, workspace_bytes, kWsHeader, st);  // decode-sized batches: HBM-bound
-  if (tcgen05_gemm_eligible(T, N, K)) return launch_gemm_tcgen05<MODE>(g, st);
+  if (tcgen05_gemm_eligible(T, N, K)) {
+    static_assert(TG_CUT_BYTES <= SK_PARTIAL_BYTES && 2 * TG_MAX_CUTS <= SK_MAX_CTAS, "cut tiles use the stream-K kernel's part of the workspace");
+    const bool room = workspace != nullptr && workspace_bytes >= kWsHeader + SK_PARTIAL_BYTES;
+    return launch_gemm_tcgen05<MODE>(g, st, room ? (uint8_t*)workspace + kWsHeader : nullptr, room ? (unsigned*)((uint8_t*)workspace + SK_FLAGS_OFFSET) : nullptr);
+  }
   return launch_gemm_mma<MODE>(g, st);
 }
 }  // namespace mb200
@@ -316,7 +320,7 @@ int mb200_lm_head_logprobs(const void* x, const void* norm_w, const void* w_out,
   g.epi.keep_row = keep_row_dev;
   g.epi.partial = (float2*)partial;
   g.epi.target_logit = target_logit;
-  rc = launch_gemm_tcgen05_prompt<EPI_LOGPROB>(g, st);
+  rc = launch_gemm_tcgen05_prompt<EPI_LOGPROB>(g, st, (uint8_t*)workspace + kWsHeader, (unsigned*)((uint8_t*)workspace + SK_FLAGS_OFFSET));
   if (rc) return rc;
   logprob_combine_kernel<<<(unsigned)ceil_div(T, 8), 256, 0, st>>>((const float2*)partial, target_logit, (const long long*)target_dev, out_dev, (int)T, (int)(vocab / 64));
   MB_CHECK_LAUNCH("logprob_combine_kernel");
@@ -511,7 +515,7 @@ static int layer_epilogue(EpiParams& e, const void* bias, void* out, float* out3
 }
 
 int mb200_layer_linear(const void* x, const void* w, const void* bias, void* out, float* out32, int64_t T, int64_t N, int64_t K, int epi, int64_t n_act,
-                       float limit, float alpha, const float* rowscale, int64_t rs_pitch, int64_t rs_group, void* stream) {
+                       float limit, float alpha, const float* rowscale, int64_t rs_pitch, int64_t rs_group, void* scratch, void* stream) {
   MB_CHECK_ARG(x && w, "layer_linear: null pointer");
   MB_CHECK_ARG(T >= TG_BM && N % 128 == 0 && K % TG_BK == 0, "layer_linear: T=%lld N=%lld K=%lld (T >= 128, N %% 128, K %% 64)", (long long)T, (long long)N,
                (long long)K);
@@ -529,7 +533,24 @@ int mb200_layer_linear(const void* x, const void* w, const void* bias, void* out
   g.N = (int)N;
   g.K = (int)K;
   g.epi = e;
-  return launch_gemm_tcgen05_prompt<EPI_LAYER>(g, (cudaStream_t)stream);
+  unsigned* flags = nullptr;
+  if (scratch != nullptr) {
+    flags = reinterpret_cast<unsigned*>((uint8_t*)scratch + TG_CUT_BYTES);
+    MB_CHECK_CUDA(cudaMemsetAsync(flags, 0, 2 * TG_MAX_CUTS * sizeof(unsigned), (cudaStream_t)stream));
+  }
+  return launch_gemm_tcgen05_prompt<EPI_LAYER>(g, (cudaStream_t)stream, scratch, flags);
+}
+
+size_t mb200_layer_linear_scratch(int64_t T, int64_t N, int64_t K) {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+  if (T < 4 * TG_BM || N % 256 != 0 || sms < 2) return 0;
+  TcGemmParams p;
+  p.T = (int)T;
+  p.N = (int)N;
+  p.K = (int)K;
+  plan_pairs(p, sms / 2, &p, nullptr);  // (any non-null scratch: would the launch cut tiles?)
+  return p.cut_pairs > 0 ? TG_CUT_BYTES + 2 * TG_MAX_CUTS * sizeof(unsigned) : 0;
 }
 
 int mb200_layer_moe_sizes(int64_t T, int64_t n_experts, int64_t top, int64_t* rows_cap, int64_t* plan_words) {

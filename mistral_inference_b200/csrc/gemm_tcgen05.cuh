@@ -76,7 +76,14 @@ struct TcGemmParams {
   // grouped, experts packed in ONE matrix (layered decoders): expert e's weights start w_n * e rows and w_k * e columns into the single
   // tensor map; w_n = w_k = 0: a tensor map per expert
   int w_n = 0, w_k = 0;
+  // cluster pairs of 256-wide tiles, dense (plan_pairs): work items are the odd last row of tiles (two column tiles an item), whole tile pairs, and
+  // at the end the last `cut_pairs` pairs, each cut into `cut` parts along k.  cut_pairs < 0: every pair whole, an odd row as pairs too
+  int cut_pairs = -1, cut = 1;
+  float* partials = nullptr;   // [(cut - 1) * cut_pairs][2 CTAs][256 / 4][128 rows] float4: what the parts but the first leave for it
+  unsigned* flags = nullptr;   // [(cut - 1) * cut_pairs * 2], zero between launches
 };
+constexpr int TG_MAX_CUTS = 40;  // (cut - 1) * cut_pairs at most: 256 KB each
+constexpr size_t TG_CUT_BYTES = (size_t)TG_MAX_CUTS * 2 * TG_BM * 256 * sizeof(float);
 
 // ---- PTX wrappers ---------------------------------------------------------------------------------
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1) {
@@ -162,9 +169,9 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
 // GROUPED = true (mixture of experts, csrc/moe.cuh): the A rows are the (token, expert) pairs sorted by expert, every expert's
 // segment padded to a multiple of TA rows; m tile i covers rows plan.tile_row0[i] .. + TA of expert plan.tile_expert[i], whose
 // weight matrix has its own tensor map (map_w[expert]).  The number of m tiles is DEVICE data (no host sync after routing).
-constexpr int MOE_PLAN_HEADER = 64;  // int32 words: [0] m tiles of this rank, [1] padded rows in total, [2] tile capacity, [6] tile pairs, [8..] segment starts
+constexpr int MOE_PLAN_HEADER = 64;  // int32 words: [0] m tiles of this rank, [1] padded rows in total, [2] tile capacity, [6] tile pairs and single tiles, [7] how many of these are pairs (they come first), [8..] segment starts
 // after the header: tile_expert[cap], tile_row0[cap], pair_expert[cap], pair_info[cap] (cap = plan[2]).  A PAIR is two vertically
-// adjacent m tiles of ONE expert (or a single last tile: bit 30 of pair_info clear), the unit of the 2-CTA cluster variant.
+// adjacent m tiles of ONE expert (bit 30 of pair_info), a single tile the last one of an odd number: the units of the 2-CTA cluster variant.
 constexpr int MOE_PAIR_SECOND = 1 << 30;
 constexpr int MOE_MAX_EXPERTS = 16;  // tensor maps travel as kernel parameters (128 B each)
 struct MoeWeightMaps {
@@ -192,8 +199,17 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
   const int cta = (int)blockIdx.x / CL, n_cta = (int)gridDim.x / CL;  // cluster index / clusters in the grid
   // a cluster walks "super tiles" of CL vertically adjacent tiles; rows past T read as zeros (TMA) and are never stored
   // grouped: m units are the plan's tiles (single CTA) or tile pairs (cluster of two)
-  const int num_m = GROUPED ? (CL > 1 ? plan[6] : plan[0]) : ((p.T + TG_BM - 1) / TG_BM + CL - 1) / CL;
-  const int num_n = p.N / TG_BN, num_tiles = num_m * num_n, num_k = p.K / TG_BK;
+  // SINGLE tiles (pairs of 256-wide tiles only): where a row of tiles has no neighbour below, the two CTAs take the SAME rows and two
+  // neighbouring column tiles instead of a pair whose second tile is recomputed or empty.
+  constexpr bool kSingles = CL == 2 && BN == 256;
+  constexpr bool kCuts = kSingles && !GROUPED;
+  const int m_tiles = (p.T + TG_BM - 1) / TG_BM, num_n = p.N / TG_BN, num_k = p.K / TG_BK;
+  const bool planned = kCuts && p.cut_pairs >= 0;
+  const int num_m = GROUPED ? (kSingles ? plan[7] : (CL > 1 ? plan[6] : plan[0])) : (planned ? m_tiles / 2 : (m_tiles + CL - 1) / CL);
+  const int half_n = (num_n + 1) / 2;
+  const int lone_rows = GROUPED ? (kSingles ? plan[6] - plan[7] : 0) : (planned ? m_tiles & 1 : 0);
+  const int lone = lone_rows * half_n, whole = num_m * num_n - (planned ? p.cut_pairs : 0);
+  const int num_tiles = lone + whole + (planned ? p.cut * p.cut_pairs : 0);
   const int32_t* tile_expert = GROUPED ? plan + MOE_PLAN_HEADER + (CL > 1 ? 2 * plan[2] : 0) : nullptr;
   const int32_t* tile_row0 = GROUPED ? tile_expert + plan[2] : nullptr;
   // Tile order.  The persistent CTAs take tiles t = cta, cta + n_cta, ...: at any moment ~n_cta consecutive tile ids are in flight,
@@ -234,16 +250,41 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
     mu = mblk * kGM + q % gm;
     nt = nb * kGN + q / gm;
   };
-  // first row of this CTA's m tile of unit `u` (cluster rank 1 takes the pair's second tile; a missing second tile is recomputed
-  // from the first one's rows and not stored)
-  auto grouped_m0 = [&](int u, bool& store) {
-    const int info = tile_row0[u];
-    store = true;
-    if (CL == 1) return info;
-    const int row0 = info & (MOE_PAIR_SECOND - 1);
-    if (rank == 0) return row0;
-    store = (info & MOE_PAIR_SECOND) != 0;
-    return store ? row0 + TG_BM : row0;
+  struct Item {
+    int mu, m0, n0, kb0, kb1;
+    bool store, lone;  // lone: a single tile, W is not shared with the other CTA
+    int part, slot;    // part of a cut pair (0: the owner, which adds the others' sums), -1: not cut
+  };
+  auto item_of = [&](int tile) {
+    Item it;
+    it.kb0 = 0, it.kb1 = num_k, it.store = true, it.lone = false, it.part = -1, it.slot = 0, it.mu = 0;
+    if (kSingles && tile < lone) {
+      const int row = tile % lone_rows, nt = 2 * (tile / lone_rows) + rank;
+      it.lone = true;
+      it.store = nt < num_n;
+      it.n0 = min(nt, num_n - 1) * TG_BN;
+      it.mu = GROUPED ? num_m + row : 0;
+      it.m0 = GROUPED ? tile_row0[it.mu] & (MOE_PAIR_SECOND - 1) : (m_tiles - 1) * TG_BM;
+      return it;
+    }
+    int t = tile - lone, nt;
+    if (kCuts && t >= whole) {
+      const int s = t - whole;
+      it.part = s / p.cut_pairs;
+      it.slot = s % p.cut_pairs;
+      it.kb0 = num_k * it.part / p.cut;
+      it.kb1 = num_k * (it.part + 1) / p.cut;
+      t = whole + it.slot;
+    }
+    tile_mn(t, it.mu, nt);
+    it.n0 = nt * TG_BN;
+    if (GROUPED) {
+      const int info = tile_row0[it.mu];
+      it.m0 = CL == 1 ? info : (info & (MOE_PAIR_SECOND - 1)) + rank * TG_BM;  // (CL == 2: the plan's first units have both tiles)
+    } else {
+      it.m0 = (it.mu * CL + rank) * TG_BM;
+    }
+    return it;
   };
   const CUtensorMap& map_w = *map_w_base;
 
@@ -274,21 +315,22 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
     if (lane == 0) {
       uint32_t it = 0;
       for (int tile = cta; tile < num_tiles; tile += n_cta) {
-        bool store_unused;
-        int mu, nt;
-        tile_mn(tile, mu, nt);
-        const int m0 = GROUPED ? grouped_m0(mu, store_unused) : (mu * CL + rank) * TG_BM, n0 = nt * TG_BN;
-        const int expert = GROUPED ? tile_expert[mu] : 0;
+        const Item w = item_of(tile);
+        const int m0 = w.m0, n0 = w.n0;
+        const int expert = GROUPED ? tile_expert[w.mu] : 0;
         const bool packed = GROUPED && (p.w_n | p.w_k) != 0;
         const CUtensorMap* wmap = map_w_base + (packed ? 0 : expert);
         const int wr = n0 + (packed ? expert * p.w_n : 0), wc = packed ? expert * p.w_k : 0;
-        for (int kb = 0; kb < num_k; ++kb, ++it) {
+        for (int kb = w.kb0; kb < w.kb1; ++kb, ++it) {
           const uint32_t s = it % TG_STAGES, par = (it / TG_STAGES) & 1;
           mbar_wait(&empty[s], par ^ 1, 11, it);
           mbar_arrive_expect_tx(&full[s], TG_STAGE_BYTES);  // A + both halves of W (the peer's half may land first: tx-count goes negative)
           uint8_t* sa = smem + s * TG_STAGE_BYTES;
           tma_load_2d(sa, &map_a, &full[s], kb * TG_BK, m0);
-          if (CL > 1)
+          if (kSingles && w.lone) {  // the boxes are half tiles
+            tma_load_2d(sa + TG_A_BYTES, wmap, &full[s], wc + kb * TG_BK, wr);
+            tma_load_2d(sa + TG_A_BYTES + TG_B_BYTES / 2, wmap, &full[s], wc + kb * TG_BK, wr + TG_BN / 2);
+          } else if (CL > 1)
             tma_load_2d_multicast(sa + TG_A_BYTES + rank * (TG_B_BYTES / CL), wmap, &full[s], wc + kb * TG_BK, wr + rank * (TG_BN / CL),
                                   (uint16_t)((1u << CL) - 1));
           else
@@ -305,7 +347,12 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
         mbar_wait(&tmem_empty[acc], acc_par ^ 1, 12, acc_it);  // the epilogue has drained this accumulator buffer
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * TG_BN;
-        for (int kb = 0; kb < num_k; ++kb, ++it) {
+        int kb0 = 0, kb1 = num_k;
+        if (kCuts) {
+          const Item w = item_of(tile);
+          kb0 = w.kb0, kb1 = w.kb1;
+        }
+        for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const uint32_t s = it % TG_STAGES, par = (it / TG_STAGES) & 1;
           mbar_wait(&full[s], par, 13, it);
           tc_fence_after();
@@ -313,7 +360,7 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
           const uint64_t adesc = umma_desc_sw128(a_addr), bdesc = umma_desc_sw128(a_addr + TG_A_BYTES);
 #pragma unroll
           for (int k = 0; k < TG_BK / 16; ++k)  // +32 bytes (= 2 in 16-byte units) per K = 16 step inside the 128-byte swizzled row
-            umma_bf16(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), kUmmaIdesc, (kb | k) ? 1u : 0u);
+            umma_bf16(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), kUmmaIdesc, (kb > kb0 || k) ? 1u : 0u);
           if (CL > 1)  // frees the stage in both CTAs (each producer writes into both) when these MMAs have read it
             umma_commit_multicast(&empty[s], (uint16_t)((1u << CL) - 1));
           else
@@ -327,10 +374,9 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
     const int lane_base = (warp & 3) * 32;
     uint32_t acc_it = 0;
     for (int tile = cta; tile < num_tiles; tile += n_cta, ++acc_it) {
-      bool store = true;
-      int mu, nt;
-      tile_mn(tile, mu, nt);
-      const int m0 = GROUPED ? grouped_m0(mu, store) : (mu * CL + rank) * TG_BM, n0 = nt * TG_BN;
+      const Item w = item_of(tile);
+      const int m0 = w.m0, n0 = w.n0;
+      const bool store = w.store;
       const uint32_t acc = acc_it & 1, acc_par = (acc_it >> 1) & 1;
       mbar_wait(&tmem_full[acc], acc_par, 14, acc_it);
       tc_fence_after();
@@ -339,6 +385,60 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
       // two register buffers: the TMEM load of chunk c+1 is in flight while chunk c goes through the epilogue
       const uint32_t trow = tmem_base + ((uint32_t)lane_base << 16) + acc * TG_BN;
       uint32_t va[32], vb[32];
+      const int row = lane_base + lane;
+      if constexpr (kCuts) {
+        if (w.part > 0) {
+          // a later part of a cut pair: its fp32 sums go to the owner, column quads of 128 rows side by side
+          const int at = ((w.part - 1) * p.cut_pairs + w.slot) * 2 + rank;
+          float4* dst = reinterpret_cast<float4*>(p.partials) + (size_t)at * (TG_BN / 4) * TG_BM + row;
+#pragma unroll 1
+          for (int c = 0; c < TG_BN / 32; ++c) {
+            tmem_ld_32x32b_x32(trow + c * 32, va);
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+              dst[(c * 8 + q) * TG_BM] = make_float4(__uint_as_float(va[4 * q]), __uint_as_float(va[4 * q + 1]), __uint_as_float(va[4 * q + 2]), __uint_as_float(va[4 * q + 3]));
+          }
+          __threadfence();
+          asm volatile("bar.sync 2, 128;" ::: "memory");
+          if (threadIdx.x == 64) st_release_u32(p.flags + at, 1u);
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&tmem_empty[acc]);
+          continue;
+        }
+        if (w.part == 0) {  // the owner: the other parts run at the same time on other clusters (the launch's last items, all resident)
+          const int other = (int)threadIdx.x - 64;
+          if (other < p.cut - 1) {
+            const unsigned* f = p.flags + (other * p.cut_pairs + w.slot) * 2 + rank;
+            unsigned spins = 0;
+            while (ld_acquire_u32(f) == 0u) {
+              if (++spins == MB200_WATCHDOG_SPINS) {
+                printf("[mb200 watchdog] cluster %d waits for part %d of pair %d\n", cta, other + 1, w.slot);
+                __trap();
+              }
+            }
+          }
+          asm volatile("bar.sync 2, 128;" ::: "memory");
+        }
+      }
+      // the other parts' sums of columns 32 c .. + 31, in the order of k
+      auto plus = [&](int c, uint32_t (&v)[32]) {
+        if constexpr (kCuts) {
+          if (w.part == 0) {
+            for (int o = 0; o < p.cut - 1; ++o) {
+              const float4* src = reinterpret_cast<const float4*>(p.partials) + (size_t)((o * p.cut_pairs + w.slot) * 2 + rank) * (TG_BN / 4) * TG_BM + row;
+#pragma unroll
+              for (int q = 0; q < 8; ++q) {
+                const float4 x = __ldcg(src + (c * 8 + q) * TG_BM);
+                v[4 * q] = __float_as_uint(__uint_as_float(v[4 * q]) + x.x);
+                v[4 * q + 1] = __float_as_uint(__uint_as_float(v[4 * q + 1]) + x.y);
+                v[4 * q + 2] = __float_as_uint(__uint_as_float(v[4 * q + 2]) + x.z);
+                v[4 * q + 3] = __float_as_uint(__uint_as_float(v[4 * q + 3]) + x.w);
+              }
+            }
+          }
+        }
+      };
       tmem_ld_32x32b_x32_nowait(trow, va);
       if constexpr (MODE == EPI_LOGPROB) {
         const bool live = t < p.T;
@@ -351,6 +451,7 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
 #pragma unroll
           for (int j = 0; j < 32; ++j) vb[j] = va[j];
           if (c + 1 < TG_BN / 32) tmem_ld_32x32b_x32_nowait(trow + (c + 1) * 32, va);
+          plus(c, vb);
           if (live) epi_logprob32(p.epi, t, n0 + c * 32, vb, tgt, keep, m, sum);
           if (c & 1) {
             if (tgt >= 0) p.epi.partial[(int64_t)t * (p.N / 64) + (n0 + c * 32) / 64] = make_float2(m, sum);
@@ -374,6 +475,7 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
 #pragma unroll
           for (int j = 0; j < 32; ++j) vb[j] = va[j];
           if (c + 1 < TG_BN / 32) tmem_ld_32x32b_x32_nowait(trow + (c + 1) * 32, va);
+          plus(c, vb);
           chunk(n0 + c * 32, vb);
         }
       } else if constexpr (TG_BN == 32) {
@@ -384,10 +486,18 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
         for (int c = 0; c < TG_BN / 32; c += 2) {
           tmem_wait_ld();
           tmem_ld_32x32b_x32_nowait(trow + (c + 1) * 32, vb);
+          plus(c, va);
           if (t < p.T) epi_chunk32<MODE>(p.epi, t, n0 + c * 32, va);
           tmem_wait_ld();
           if (c + 2 < TG_BN / 32) tmem_ld_32x32b_x32_nowait(trow + (c + 2) * 32, va);
+          plus(c + 1, vb);
           if (t < p.T) epi_chunk32<MODE>(p.epi, t, n0 + (c + 1) * 32, vb);
+        }
+      }
+      if constexpr (kCuts) {
+        if (w.part == 0) {  // everybody has read: ready for the next launch
+          asm volatile("bar.sync 2, 128;" ::: "memory");
+          if ((int)threadIdx.x - 64 < p.cut - 1) p.flags[(((int)threadIdx.x - 64) * p.cut_pairs + w.slot) * 2 + rank] = 0u;
         }
       }
       tc_fence_before();
@@ -468,8 +578,28 @@ inline int tcgen05_forced_bn() {
   return e != nullptr ? atoi(e) : 0;
 }
 
+// How a dense launch of cluster pairs (256 x 256 outputs an item, `units` pairs on the chip) ends.  Items run in rounds of `units`; when the
+// last round is at most half full, its pairs are cut along k into as many parts as fill it (at most four, eight k-blocks each): the parts' fp32
+// sums meet in the first part's epilogue, in the order of k.  The odd last row of tiles comes first, two column tiles an item.
+// T = 4096, 7B shapes: wo + w2 498 -> 486 us (3.46 rounds, the last half full); T = 1102 (9 row tiles): wo 48 -> 29 us, w2 151 -> 100 us.
+inline void plan_pairs(TcGemmParams& p, int units, void* scratch, unsigned* flags) {
+  const int m_tiles = (p.T + TG_BM - 1) / TG_BM, num_n = p.N / 256, pairs = m_tiles / 2 * num_n, lone = (m_tiles & 1) * ((num_n + 1) / 2);
+  const int rest = (pairs + lone) % units;
+  p.cut_pairs = 0;
+  p.cut = 1;
+  if (scratch == nullptr || rest == 0 || rest > pairs) return;
+  int cut = units / rest;
+  if (cut > 4) cut = 4;
+  while (cut > 1 && ((cut - 1) * rest > TG_MAX_CUTS || p.K / TG_BK < 8 * cut)) --cut;
+  if (cut < 2) return;
+  p.cut = cut;
+  p.cut_pairs = rest;
+  p.partials = reinterpret_cast<float*>(scratch);
+  p.flags = flags;
+}
+
 template <int MODE, int BN>
-int launch_gemm_tcgen05_bn(const GemmParams& g, bool pair, int sms, cudaStream_t stream) {
+int launch_gemm_tcgen05_bn(const GemmParams& g, bool pair, int sms, cudaStream_t stream, void* scratch, unsigned* flags) {
   using Cfg = TgCfg<BN>;
   constexpr int kSmem = MODE == EPI_LAYER ? Cfg::kSmemLayer : Cfg::kSmem;
   CUtensorMap map_a, map_w;
@@ -483,7 +613,10 @@ int launch_gemm_tcgen05_bn(const GemmParams& g, bool pair, int sms, cudaStream_t
   p.K = g.K;
   p.epi = g.epi;
   if (pair) {
-    const int supers = ceil_div(ceil_div(g.T, TG_BM), 2) * (g.N / BN), pairs = sms / 2;
+    const int pairs = sms / 2;
+    int supers = ceil_div(ceil_div(g.T, TG_BM), 2) * (g.N / BN);
+    if (BN == 256) plan_pairs(p, pairs, scratch, flags);
+    if (p.cut_pairs > 0) supers = pairs;  // the last round is full
     MB_CHECK_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<MODE, 2, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2u * (unsigned)(supers < pairs ? supers : pairs));
@@ -562,9 +695,9 @@ int launch_gemm_tcgen05_small_ta(const GemmParams& g, int sms, cudaStream_t stre
   }
 }
 
-// T >= TG_BM
+// T >= TG_BM.  scratch: TG_CUT_BYTES for the sums of cut tiles, flags: 2 * TG_MAX_CUTS words, zero (or neither)
 template <int MODE>
-int launch_gemm_tcgen05_prompt(const GemmParams& g, cudaStream_t stream) {
+int launch_gemm_tcgen05_prompt(const GemmParams& g, cudaStream_t stream, void* scratch = nullptr, unsigned* flags = nullptr) {
   const bool pair = tcgen05_cluster_enabled() && g.T >= 4 * TG_BM;
   int dev = 0, sms = 0;
   MB_CHECK_CUDA(cudaGetDevice(&dev));
@@ -580,15 +713,18 @@ int launch_gemm_tcgen05_prompt(const GemmParams& g, cudaStream_t stream) {
   // 192-wide tiles (N = 6144: 5.19 rounds of 256 -> 6.92 rounds at 3/4 of the cost) were measured too: qkv+RoPE at T = 4096
   // 156 -> 169 us, slower for the same reason.  They stay available for N that is a multiple of 192 only and for the tests.
   const int forced = tcgen05_forced_bn();
-  if ((forced == 128 || forced == 192 || forced == 256) && g.N % forced == 0) bn = forced;
-  if (bn == 192) return launch_gemm_tcgen05_bn<MODE, 192>(g, pair, sms, stream);
+  if ((forced == 128 || forced == 192 || forced == 256) && g.N % forced == 0) {
+    bn = forced;
+    scratch = nullptr;  // a pinned width is a plain schedule: every output's sum runs over k in one go, whatever the tile
+  }
+  if (bn == 192) return launch_gemm_tcgen05_bn<MODE, 192>(g, pair, sms, stream, nullptr, nullptr);
   const bool narrow = bn == 128;
-  return narrow ? launch_gemm_tcgen05_bn<MODE, 128>(g, pair, sms, stream) : launch_gemm_tcgen05_bn<MODE, 256>(g, pair, sms, stream);
+  return narrow ? launch_gemm_tcgen05_bn<MODE, 128>(g, pair, sms, stream, nullptr, nullptr) : launch_gemm_tcgen05_bn<MODE, 256>(g, pair, sms, stream, scratch, flags);
 }
 
 template <int MODE>
-int launch_gemm_tcgen05(const GemmParams& g, cudaStream_t stream) {
-  if (g.T >= TG_BM) return launch_gemm_tcgen05_prompt<MODE>(g, stream);
+int launch_gemm_tcgen05(const GemmParams& g, cudaStream_t stream, void* scratch, unsigned* flags) {
+  if (g.T >= TG_BM) return launch_gemm_tcgen05_prompt<MODE>(g, stream, scratch, flags);
   int dev = 0, sms = 0;
   MB_CHECK_CUDA(cudaGetDevice(&dev));
   MB_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));

@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(MP_THREADS) moe_plan_kernel(const int32_t* __r
       plan[3] = pairs;
       plan[4] += touched;
       plan[5] += 1;
-      plan[6] = 0;  // decode-sized calls never take the cluster variant
+      plan[6] = plan[7] = 0;  // calls this small never take the cluster variant
     }
     __syncthreads();
     for (int i = tid; i < pairs; i += MP_THREADS) slot[i] = sel[i] < E ? slot[i] + seg[sel[i]] : -1;
@@ -197,12 +197,21 @@ __global__ void __launch_bounds__(MP_THREADS) moe_plan_kernel(const int32_t* __r
           plan[MOE_PLAN_HEADER + n] = e;
           plan[MOE_PLAN_HEADER + tile_cap + n] = rows + m * tile_rows;
         }
-        for (int m = 0; m < m_tiles && np < tile_cap; m += 2, ++np) {  // pairs of vertically adjacent tiles for the 2-CTA cluster GEMM
+        for (int m = 0; m + 1 < m_tiles && np < tile_cap; m += 2, ++np) {  // pairs of vertically adjacent tiles for the 2-CTA cluster GEMM
           plan[MOE_PLAN_HEADER + 2 * tile_cap + np] = e;
-          plan[MOE_PLAN_HEADER + 3 * tile_cap + np] = (rows + m * tile_rows) | (m + 1 < m_tiles ? MOE_PAIR_SECOND : 0);
+          plan[MOE_PLAN_HEADER + 3 * tile_cap + np] = (rows + m * tile_rows) | MOE_PAIR_SECOND;
         }
       }
       rows += m_tiles * tile_rows;
+    }
+    plan[7] = np;
+    for (int e = 0; e < E; ++e) {  // then the last tiles of the experts that have an odd number of them
+      const int m_tiles = (total[e] + tile_rows - 1) / tile_rows;
+      if ((m_tiles & 1) && e % shard_world == shard_rank && np < tile_cap) {
+        plan[MOE_PLAN_HEADER + 2 * tile_cap + np] = e;
+        plan[MOE_PLAN_HEADER + 3 * tile_cap + np] = seg[e] + (m_tiles - 1) * tile_rows;
+        ++np;
+      }
     }
     plan[6] = np;
     seg[E] = rows;
@@ -562,7 +571,7 @@ inline int launch_grouped_packed(const void* a, int64_t rows_cap, int64_t K, int
   int dev = 0, sms = 0;
   MB_CHECK_CUDA(cudaGetDevice(&dev));
   MB_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  if (N % 256 == 0 && pairs >= 384 * E)
+  if (N % 256 == 0 && pairs >= 384 * E && pairs > 512)  // (the plan of up to 512 rows lists no pairs)
     return launch_grouped_packed_bn<256, 2>(a, rows_cap, K, N, w, w_rows, w_cols, w_n, w_k, plan, epi, sms, stream);
   return launch_grouped_packed_bn<128, 1>(a, rows_cap, K, N, w, w_rows, w_cols, w_n, w_k, plan, epi, sms, stream);
 }

@@ -21,7 +21,7 @@ def _unit(kind, z, w, limit, alpha):
 
 
 @pytest.mark.parametrize("kind", ["silu", "gelu", "glu", "relu2"])
-@pytest.mark.parametrize("T,width,ff,E,top,idle", [(1, 128, 64, 1, 1, 0), (17, 128, 64, 5, 2, 2), (129, 384, 192, 3, 3, 0), (300, 256, 128, 48, 6, 5), (1100, 128, 128, 2, 2, 1)])
+@pytest.mark.parametrize("T,width,ff,E,top,idle", [(1, 128, 64, 1, 1, 0), (17, 128, 64, 5, 2, 2), (129, 384, 192, 3, 3, 0), (300, 256, 128, 48, 6, 5), (1100, 128, 128, 2, 2, 1), (450, 256, 128, 1, 1, 0), (2100, 256, 128, 2, 1, 0)])
 def test_chosen_expert_rows(kind, T, width, ff, E, top, idle, monkeypatch):
     """The grouped form of a mixture: experts nobody chose, choices that name no expert (>= E), segments around the 128-row tile, pairs of tiles
     (the last shape: from 384 rows per expert on), more tokens than one call takes.  The hidden units' three bf16 roundings (gate, up, result;
