@@ -217,10 +217,10 @@ int mb200_moe_grouped_ffn(const void* xs, const void* const* w13_host, const voi
  * Linears and mixtures of layered decoders (no counterpart in the reference; the formulas of `epi` are those of
  * mbh_linear, include/mistral_b200_hybrid.h, 0 .. 7 without the decays).  bf16 in, fp32 accumulation, the step that follows the
  * Linear in its epilogue.
- * mb200_layer_linear: T >= 128 rows, N % 128 == 0, K % 64 == 0.  out: bf16 results; out32: the fp32 residual stream or fp32 results.
+ * mb200_layer_linear: N % 128 == 0, K % 64 == 0.  out: bf16 results; out32: the fp32 residual stream or fp32 results.
  *     rowscale [T, rs_pitch] fp32 or NULL: hidden unit c of row t is scaled by rowscale[t, c / rs_group].  n_act columns through SiLU.
  *     scratch: mb200_layer_linear_scratch(T, N, K) bytes (uninitialised, this call's own), or NULL (also when that is 0): without it the last
- *     tiles are not cut.
+ *     tiles are not cut; fewer than 128 rows need it.
  * mb200_layer_moe: y32 [T, width] fp32 (+= when add) sum over the token's choices idx [T, top] < n_experts of
  *     wsel * (act W2_e^T), act = step(hn W13_e^T); w13 [E * 2 ff, width] (gate/up rows interleaved; RELU2: [E * ff, width]),
  *     w2 [width, E * ff].  The weight multiplies the hidden units (GLU: the expert's input).  width % 128 == 0, ff % 64 == 0,

@@ -296,7 +296,7 @@ def moe_grouped_ffn(b, w13_host, w2_host, residual: Optional[torch.Tensor], out:
 
 def layer_linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: Optional[torch.Tensor], out32: Optional[torch.Tensor], epi: int,
                  n_act: int = 0, limit: float = 0.0, alpha: float = 0.0, rowscale: Optional[torch.Tensor] = None, group: int = 1) -> None:
-    """A layered decoder's Linear over T >= 128 rows with the step that follows it in the GEMM's epilogue (include/mistral_b200.h)."""
+    """A layered decoder's Linear with the step that follows it in the GEMM's epilogue (include/mistral_b200.h)."""
     T, K = x.shape
     need = lib().mb200_layer_linear_scratch(T, w.shape[0], K)
     scratch = torch.empty(need, dtype=torch.uint8, device=x.device) if need else None

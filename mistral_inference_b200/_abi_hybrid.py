@@ -141,11 +141,15 @@ def rmsnorm_pair(x32: torch.Tensor, w: torch.Tensor, w2: torch.Tensor, eps: floa
     return y, y2
 
 
+PROMPT_GEMM_MIN_ROWS = 17  # fewer rows: this library's own kernel, which streams the weights past up to 16 tokens
+
+
 def _prompt_gemm_ok(x: torch.Tensor, M: int, N: int, K: int) -> bool:
-    """Large bf16 Linears of prompts go to the main library's persistent tcgen05 GEMM (`_abi.layer_linear`: the step after the Linear is its
-    epilogue) when it is built and the shape fits its tiles (K % 64 == 0, N % 128 == 0, at least one 128-row tile); everything else runs on
-    this library's own kernels.  A checkout that has only libmb200_hybrid.so never builds the main library for this."""
-    return (x.dtype == torch.bfloat16 and M >= 128 and K % 64 == 0 and N % 128 == 0 and os.environ.get("MB200_HYBRID_GEMM", "1") != "0"
+    """Large bf16 Linears of prompts go to the main library's tcgen05 GEMMs (`_abi.layer_linear`: the step after the Linear is the
+    epilogue; below 128 rows the stream-K kernel, above the persistent one) when it is built and the shape fits their tiles (K % 64 == 0,
+    N % 128 == 0); everything else runs on this library's own kernels.  A checkout that has only libmb200_hybrid.so never builds the main
+    library for this."""
+    return (x.dtype == torch.bfloat16 and M >= PROMPT_GEMM_MIN_ROWS and K % 64 == 0 and N % 128 == 0 and os.environ.get("MB200_HYBRID_GEMM", "1") != "0"
             and _abi.library_path().exists())
 
 

@@ -26,6 +26,9 @@ static unsigned long long* g_mk_prof_bar = nullptr;  // debug: decode megakernel
 constexpr int64_t MB200_ATTN_FIRST_MIN = 128, MB200_ATTN_PORTION_MIN = 16;
 
 constexpr size_t kWsHeader = 64 * 1024;  // persistent, zero-initialised by the caller once: self-resetting counters
+// behind the header: partial sums of the stream-K kernel or of the prompt GEMM's cut tiles (both with their flags in the header)
+constexpr size_t kWsPartial = TG_CUT_BYTES > SK_PARTIAL_BYTES ? TG_CUT_BYTES : SK_PARTIAL_BYTES;
+static_assert(2 * TG_MAX_CUTS <= SK_MAX_CTAS, "the flags of cut tiles use those of the stream-K kernel");
 inline size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
 static int run_rmsnorm(const void* x, const void* w, void* out, int64_t T, int64_t dim, float eps, cudaStream_t st) {
@@ -52,9 +55,9 @@ static int run_linear(const void* x, const void* norm_w, const void* w, const Ep
   }
   const void* a = x;
   if (norm_w) {
-    const size_t need = kWsHeader + SK_PARTIAL_BYTES + align256((size_t)T * K * 2);
+    const size_t need = kWsHeader + kWsPartial + align256((size_t)T * K * 2);
     if (workspace == nullptr || workspace_bytes < need) return fail(MB200_E_WORKSPACE, "linear: workspace %zu < %zu", workspace_bytes, need);
-    void* normed = (uint8_t*)workspace + kWsHeader + SK_PARTIAL_BYTES;  // after the stream-K partial slots
+    void* normed = (uint8_t*)workspace + kWsHeader + kWsPartial;  // after the stream-K partial slots
     int rc = run_rmsnorm(x, norm_w, normed, T, K, eps, st);
     if (rc) return rc;
     a = normed;
@@ -68,8 +71,7 @@ static int run_linear(const void* x, const void* norm_w, const void* w, const Ep
   g.epi = epi;
   if (streamk_eligible(T, N, K)) return launch_streamk<MODE>(g, workspace, workspace_bytes, kWsHeader, st);  // decode-sized batches: HBM-bound
   if (tcgen05_gemm_eligible(T, N, K)) {
-    static_assert(TG_CUT_BYTES <= SK_PARTIAL_BYTES && 2 * TG_MAX_CUTS <= SK_MAX_CTAS, "cut tiles use the stream-K kernel's part of the workspace");
-    const bool room = workspace != nullptr && workspace_bytes >= kWsHeader + SK_PARTIAL_BYTES;
+    const bool room = workspace != nullptr && workspace_bytes >= kWsHeader + kWsPartial;
     return launch_gemm_tcgen05<MODE>(g, st, room ? (uint8_t*)workspace + kWsHeader : nullptr, room ? (unsigned*)((uint8_t*)workspace + SK_FLAGS_OFFSET) : nullptr);
   }
   return launch_gemm_mma<MODE>(g, st);
@@ -98,7 +100,7 @@ size_t mb200_workspace_bytes(int64_t T, int64_t dim, int64_t n_heads, int64_t n_
   const int64_t widest = dim > hidden ? dim : hidden;
   const int64_t rep = n_kv_heads > 0 ? n_heads / n_kv_heads : 1;
   size_t s = kWsHeader;
-  s += SK_PARTIAL_BYTES;                                                  // stream-K partial accumulators (decode-sized GEMMs)
+  s += kWsPartial;                                                        // partial accumulators of split tiles
   s += align256((size_t)T * widest * 2);                                  // normed activations
   s += attn_decode_workspace(max_batch, n_kv_heads, 64, rep);             // split-KV partials (n_splits <= 64)
   // decode_step scratch (residual ping-pong, h, q, attn, g) lives in the same region as the normed activations
@@ -303,9 +305,9 @@ int mb200_lm_head_logprobs(const void* x, const void* norm_w, const void* w_out,
   MB_CHECK_ARG(T >= TG_BM && vocab % 128 == 0 && dim % TG_BK == 0, "lm_head_logprobs: T=%lld dim=%lld vocab=%lld (T >= 128, dim %% 64, vocab %% 128)",
                (long long)T, (long long)dim, (long long)vocab);
   cudaStream_t st = (cudaStream_t)stream;
-  const size_t need = kWsHeader + SK_PARTIAL_BYTES + align256((size_t)T * dim * 2);
+  const size_t need = kWsHeader + kWsPartial + align256((size_t)T * dim * 2);
   if (workspace == nullptr || workspace_bytes < need) return fail(MB200_E_WORKSPACE, "lm_head_logprobs: workspace %zu < %zu", workspace_bytes, need);
-  void* normed = (uint8_t*)workspace + kWsHeader + SK_PARTIAL_BYTES;
+  void* normed = (uint8_t*)workspace + kWsHeader + kWsPartial;
   int rc = run_rmsnorm(x, norm_w, normed, T, dim, eps, st);
   if (rc) return rc;
   GemmParams g;
@@ -517,7 +519,7 @@ static int layer_epilogue(EpiParams& e, const void* bias, void* out, float* out3
 int mb200_layer_linear(const void* x, const void* w, const void* bias, void* out, float* out32, int64_t T, int64_t N, int64_t K, int epi, int64_t n_act,
                        float limit, float alpha, const float* rowscale, int64_t rs_pitch, int64_t rs_group, void* scratch, void* stream) {
   MB_CHECK_ARG(x && w, "layer_linear: null pointer");
-  MB_CHECK_ARG(T >= TG_BM && N % 128 == 0 && K % TG_BK == 0, "layer_linear: T=%lld N=%lld K=%lld (T >= 128, N %% 128, K %% 64)", (long long)T, (long long)N,
+  MB_CHECK_ARG(T >= 1 && N % 128 == 0 && K % TG_BK == 0, "layer_linear: T=%lld N=%lld K=%lld (N %% 128, K %% 64)", (long long)T, (long long)N,
                (long long)K);
   MB_CHECK_ARG(rowscale == nullptr || (rs_pitch >= 1 && rs_group >= 1), "layer_linear: row scale pitch %lld group %lld", (long long)rs_pitch, (long long)rs_group);
   EpiParams e;
@@ -534,6 +536,11 @@ int mb200_layer_linear(const void* x, const void* w, const void* bias, void* out
   g.K = (int)K;
   g.epi = e;
   unsigned* flags = nullptr;
+  if (T < TG_BM) {  // few rows: the weight-streaming stream-K kernel, its flags in front of its partial sums
+    MB_CHECK_ARG(scratch != nullptr, "layer_linear: fewer than 128 rows need scratch");
+    MB_CHECK_CUDA(cudaMemsetAsync((uint8_t*)scratch + SK_FLAGS_OFFSET, 0, SK_MAX_CTAS * sizeof(unsigned), (cudaStream_t)stream));
+    return launch_streamk<EPI_LAYER>(g, scratch, kWsHeader + SK_PARTIAL_BYTES, kWsHeader, (cudaStream_t)stream);
+  }
   if (scratch != nullptr) {
     flags = reinterpret_cast<unsigned*>((uint8_t*)scratch + TG_CUT_BYTES);
     MB_CHECK_CUDA(cudaMemsetAsync(flags, 0, 2 * TG_MAX_CUTS * sizeof(unsigned), (cudaStream_t)stream));
@@ -542,9 +549,10 @@ int mb200_layer_linear(const void* x, const void* w, const void* bias, void* out
 }
 
 size_t mb200_layer_linear_scratch(int64_t T, int64_t N, int64_t K) {
+  if (T < TG_BM) return kWsHeader + SK_PARTIAL_BYTES;
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-  if (T < 4 * TG_BM || N % 256 != 0 || sms < 2) return 0;
+  if (T <= TG_BM || N % 256 != 0 || sms < 2 || (T < 4 * TG_BM && !pairs_fill(T, N, K, sms / 2, true))) return 0;
   TcGemmParams p;
   p.T = (int)T;
   p.N = (int)N;

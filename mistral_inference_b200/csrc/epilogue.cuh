@@ -257,6 +257,30 @@ __device__ __forceinline__ void epi_layer32_f32(const EpiParams& p, int t0, int 
   }
 }
 
+// the same for one row by one thread (the few rows of the stream-K kernel)
+__device__ __forceinline__ void epi_layer32_f32_row(const EpiParams& p, int t, int n, const uint32_t (&v)[32]) {
+  float x[32];
+  layer_sums(p, n, v, x);
+  float4* dst = reinterpret_cast<float4*>(p.out_f32 + (int64_t)t * p.ld_out + n);
+  if (p.layer == LAYER_F32) {
+    if (p.limit > 0.f) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) x[j] = p.limit * tanhf(x[j] / p.limit);
+    }
+    const float f = p.alpha != 0.f ? p.alpha : 1.f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) dst[q] = make_float4(x[4 * q] * f, x[4 * q + 1] * f, x[4 * q + 2] * f, x[4 * q + 3] * f);
+    return;
+  }
+  const float f = p.layer == LAYER_RESIDUAL_SCALED ? p.alpha : 1.f;
+  float4 r[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) r[q] = dst[q];
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+    dst[q] = make_float4(r[q].x + f * round_bf16(x[4 * q]), r[q].y + f * round_bf16(x[4 * q + 1]), r[q].z + f * round_bf16(x[4 * q + 2]), r[q].w + f * round_bf16(x[4 * q + 3]));
+}
+
 // the bf16 results: row t, columns n .. n + 31 of the accumulator
 __device__ __forceinline__ void epi_layer32_bf16(const EpiParams& p, int t, int n, const uint32_t (&v)[32]) {
   const int step = p.layer;
@@ -348,7 +372,10 @@ __device__ __forceinline__ void epi_layer32_bf16(const EpiParams& p, int t, int 
 template <int MODE>
 __device__ __forceinline__ void epi_chunk32(const EpiParams& p, int t, int n, const uint32_t (&v)[32]) {
   if constexpr (MODE == EPI_LAYER) {
-    epi_layer32_bf16(p, t, n, v);  // (fp32 results: epi_layer32_f32, by whole warps)
+    if (layer_step_is_f32(p.layer))
+      epi_layer32_f32_row(p, t, n, v);  // few rows; many: epi_layer32_f32, by whole warps
+    else
+      epi_layer32_bf16(p, t, n, v);
   } else if constexpr (MODE == EPI_STORE || MODE == EPI_RESIDUAL) {
     uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out) + (int64_t)t * p.ld_out + n);
     uint32_t o[16];

@@ -82,7 +82,7 @@ struct TcGemmParams {
   float* partials = nullptr;   // [(cut - 1) * cut_pairs][2 CTAs][256 / 4][128 rows] float4: what the parts but the first leave for it
   unsigned* flags = nullptr;   // [(cut - 1) * cut_pairs * 2], zero between launches
 };
-constexpr int TG_MAX_CUTS = 40;  // (cut - 1) * cut_pairs at most: 256 KB each
+constexpr int TG_MAX_CUTS = 56;  // (cut - 1) * cut_pairs at most: 256 KB each
 constexpr size_t TG_CUT_BYTES = (size_t)TG_MAX_CUTS * 2 * TG_BM * 256 * sizeof(float);
 
 // ---- PTX wrappers ---------------------------------------------------------------------------------
@@ -149,6 +149,15 @@ __device__ __forceinline__ void tmem_ld_32x32b_x32_nowait(uint32_t taddr, uint32
       : "r"(taddr));
 }
 
+__device__ __forceinline__ void tmem_st_32x32b_x32(uint32_t taddr, const uint32_t (&v)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, "
+      "%21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
+      "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]),
+      "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]),
+      "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
+      : "memory");
+}
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_ld_32x32b_x32(uint32_t taddr, uint32_t (&v)[32]) {
   tmem_ld_32x32b_x32_nowait(taddr, v);
@@ -193,6 +202,7 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
   uint64_t* tmem_full = empty + TG_STAGES;  // [2]
   uint64_t* tmem_empty = tmem_full + 2;     // [2]
   uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
+  uint64_t* cut_full = tmem_empty + 3;  // copies of another part's sums (kCuts)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = CL > 1 ? (int)cluster_ctarank() : 0;
@@ -297,6 +307,7 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
       mbar_init(&tmem_full[i], 1);
       mbar_init(&tmem_empty[i], 4);  // one arrive per epilogue warp
     }
+    mbar_init(cut_full, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
     if (!GROUPED) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
@@ -386,6 +397,17 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
       const uint32_t trow = tmem_base + ((uint32_t)lane_base << 16) + acc * TG_BN;
       uint32_t va[32], vb[32];
       const int row = lane_base + lane;
+      auto add_part = [&](int c, uint32_t (&v)[32]) {  // columns 32 c .. + 31 of the part that lies in the ring: quads of 128 rows side by side
+        const float4* src = reinterpret_cast<const float4*>(smem) + row;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const float4 x = src[(c * 8 + q) * TG_BM];
+          v[4 * q] = __float_as_uint(__uint_as_float(v[4 * q]) + x.x);
+          v[4 * q + 1] = __float_as_uint(__uint_as_float(v[4 * q + 1]) + x.y);
+          v[4 * q + 2] = __float_as_uint(__uint_as_float(v[4 * q + 2]) + x.z);
+          v[4 * q + 3] = __float_as_uint(__uint_as_float(v[4 * q + 3]) + x.w);
+        }
+      };
       if constexpr (kCuts) {
         if (w.part > 0) {
           // a later part of a cut pair: its fp32 sums go to the owner, column quads of 128 rows side by side
@@ -398,6 +420,7 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
             for (int q = 0; q < 8; ++q)
               dst[(c * 8 + q) * TG_BM] = make_float4(__uint_as_float(va[4 * q]), __uint_as_float(va[4 * q + 1]), __uint_as_float(va[4 * q + 2]), __uint_as_float(va[4 * q + 3]));
           }
+          asm volatile("fence.proxy.async;" ::: "memory");
           __threadfence();
           asm volatile("bar.sync 2, 128;" ::: "memory");
           if (threadIdx.x == 64) st_release_u32(p.flags + at, 1u);
@@ -406,37 +429,49 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
           if (lane == 0) mbar_arrive(&tmem_empty[acc]);
           continue;
         }
-        if (w.part == 0) {  // the owner: the other parts run at the same time on other clusters (the launch's last items, all resident)
-          const int other = (int)threadIdx.x - 64;
-          if (other < p.cut - 1) {
-            const unsigned* f = p.flags + (other * p.cut_pairs + w.slot) * 2 + rank;
-            unsigned spins = 0;
-            while (ld_acquire_u32(f) == 0u) {
-              if (++spins == MB200_WATCHDOG_SPINS) {
-                printf("[mb200 watchdog] cluster %d waits for part %d of pair %d\n", cta, other + 1, w.slot);
-                __trap();
+        if (w.part == 0) {
+          // The owner: the other parts run at the same time on other clusters (the launch's last items).  This CTA's ring is free (its last MMA has
+          // completed): each part's 128 KB come in by bulk copies and are added in the order of k -- all but the last into the accumulator,
+          // the last in the epilogue below.  (Loaded 128 bytes per thread and column chunk instead, a launch paid ~12 us of L2 latency here.)
+          for (int o = 0; o < p.cut - 1; ++o) {
+            if (threadIdx.x == 64) {
+              const int at = (o * p.cut_pairs + w.slot) * 2 + rank;
+              unsigned spins = 0;
+              while (ld_acquire_u32(p.flags + at) == 0u) {
+                if (++spins == MB200_WATCHDOG_SPINS) {
+                  printf("[mb200 watchdog] cluster %d waits for part %d of pair %d\n", cta, o + 1, w.slot);
+                  __trap();
+                }
               }
+              p.flags[at] = 0u;  // ready for the next launch
+              asm volatile("fence.proxy.async;" ::: "memory");  // written with ordinary stores, read by the copy engine
+              constexpr uint32_t kBytes = TG_BM * TG_BN * 4, kCopy = 32768;
+              mbar_arrive_expect_tx(cut_full, kBytes);
+              const uint8_t* src = reinterpret_cast<const uint8_t*>(p.partials) + (size_t)at * kBytes;
+#pragma unroll
+              for (uint32_t i = 0; i < kBytes; i += kCopy)
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(smem + i)), "l"(src + i), "r"(kCopy),
+                             "r"(smem_u32(cut_full))
+                             : "memory");
+            }
+            __syncwarp();
+            mbar_wait(cut_full, o & 1, 15, o);
+            if (o + 1 < p.cut - 1) {
+#pragma unroll 1
+              for (int c = 0; c < TG_BN / 32; ++c) {
+                tmem_ld_32x32b_x32(trow + c * 32, va);
+                add_part(c, va);
+                tmem_st_32x32b_x32(trow + c * 32, va);
+              }
+              asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+              asm volatile("bar.sync 2, 128;" ::: "memory");  // everybody has read: the next part may come
             }
           }
-          asm volatile("bar.sync 2, 128;" ::: "memory");
         }
       }
-      // the other parts' sums of columns 32 c .. + 31, in the order of k
       auto plus = [&](int c, uint32_t (&v)[32]) {
         if constexpr (kCuts) {
-          if (w.part == 0) {
-            for (int o = 0; o < p.cut - 1; ++o) {
-              const float4* src = reinterpret_cast<const float4*>(p.partials) + (size_t)((o * p.cut_pairs + w.slot) * 2 + rank) * (TG_BN / 4) * TG_BM + row;
-#pragma unroll
-              for (int q = 0; q < 8; ++q) {
-                const float4 x = __ldcg(src + (c * 8 + q) * TG_BM);
-                v[4 * q] = __float_as_uint(__uint_as_float(v[4 * q]) + x.x);
-                v[4 * q + 1] = __float_as_uint(__uint_as_float(v[4 * q + 1]) + x.y);
-                v[4 * q + 2] = __float_as_uint(__uint_as_float(v[4 * q + 2]) + x.z);
-                v[4 * q + 3] = __float_as_uint(__uint_as_float(v[4 * q + 3]) + x.w);
-              }
-            }
-          }
+          if (w.part == 0) add_part(c, v);
         }
       };
       tmem_ld_32x32b_x32_nowait(trow, va);
@@ -492,12 +527,6 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
           if (c + 2 < TG_BN / 32) tmem_ld_32x32b_x32_nowait(trow + (c + 2) * 32, va);
           plus(c + 1, vb);
           if (t < p.T) epi_chunk32<MODE>(p.epi, t, n0 + (c + 1) * 32, vb);
-        }
-      }
-      if constexpr (kCuts) {
-        if (w.part == 0) {  // everybody has read: ready for the next launch
-          asm volatile("bar.sync 2, 128;" ::: "memory");
-          if ((int)threadIdx.x - 64 < p.cut - 1) p.flags[(((int)threadIdx.x - 64) * p.cut_pairs + w.slot) * 2 + rank] = 0u;
         }
       }
       tc_fence_before();
@@ -596,6 +625,18 @@ inline void plan_pairs(TcGemmParams& p, int units, void* scratch, unsigned* flag
   p.cut_pairs = rest;
   p.partials = reinterpret_cast<float*>(scratch);
   p.flags = flags;
+}
+
+// Whether pairs of 256-wide tiles (and, for k of at least 8192, the parts they would be cut into) fill half of the chip's `units` pairs
+inline bool pairs_fill(int64_t T, int64_t N, int64_t K, int units, bool cuts) {
+  if (T <= TG_BM || N % 256 != 0 || K % TG_BK != 0) return false;
+  TcGemmParams p;
+  p.T = (int)T;
+  p.N = (int)N;
+  p.K = (int)K;
+  plan_pairs(p, units, cuts && K >= 8192 ? &p : nullptr, nullptr);  // (any scratch: how would it be cut?)
+  const int m_tiles = (p.T + TG_BM - 1) / TG_BM, num_n = p.N / 256, items = m_tiles / 2 * num_n + (m_tiles & 1) * ((num_n + 1) / 2) + (p.cut - 1) * p.cut_pairs;
+  return 2 * items >= units;
 }
 
 template <int MODE, int BN>
@@ -698,7 +739,7 @@ int launch_gemm_tcgen05_small_ta(const GemmParams& g, int sms, cudaStream_t stre
 // T >= TG_BM.  scratch: TG_CUT_BYTES for the sums of cut tiles, flags: 2 * TG_MAX_CUTS words, zero (or neither)
 template <int MODE>
 int launch_gemm_tcgen05_prompt(const GemmParams& g, cudaStream_t stream, void* scratch = nullptr, unsigned* flags = nullptr) {
-  const bool pair = tcgen05_cluster_enabled() && g.T >= 4 * TG_BM;
+  bool pair = tcgen05_cluster_enabled() && g.T >= 4 * TG_BM;
   int dev = 0, sms = 0;
   MB_CHECK_CUDA(cudaGetDevice(&dev));
   MB_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -713,6 +754,13 @@ int launch_gemm_tcgen05_prompt(const GemmParams& g, cudaStream_t stream, void* s
   // 192-wide tiles (N = 6144: 5.19 rounds of 256 -> 6.92 rounds at 3/4 of the cost) were measured too: qkv+RoPE at T = 4096
   // 156 -> 169 us, slower for the same reason.  They stay available for N that is a multiple of 192 only and for the tests.
   const int forced = tcgen05_forced_bn();
+  // Too few 256-wide tiles to fill the chip: pairs of them all the same when they, or their parts along a long k, fill half of it -- a pair reads
+  // a weight once for 256 rows and half as much of L2 per flop.  Measured (128-wide tiles, then pairs): 4096 x 14336 at T = 171 69, 45 us, at 700
+  // 141 | 91; 6144 x 4096 at 400 44 | 33, at 171 (24 pairs) 24 | 26; 2048 x 8192 at 400 41 | 31; 2048 x 2048 at 700 (24 pairs) 15 | 20.
+  if (bn == 128 && forced == 0 && tcgen05_cluster_enabled() && pairs_fill(g.T, g.N, g.K, sms / 2, scratch != nullptr)) {
+    pair = true;
+    bn = 256;
+  }
   if ((forced == 128 || forced == 192 || forced == 256) && g.N % forced == 0) {
     bn = forced;
     scratch = nullptr;  // a pinned width is a plain schedule: every output's sum runs over k in one go, whatever the tile

@@ -264,3 +264,24 @@ def test_scoring_without_written_logits(lens, monkeypatch):
     assert (last - ref_last).abs().max() <= step and (last2 - ref_last).abs().max() <= step and (got[targets < 0] == 0).all()
     for a in (got, got2):
         assert (a - ref).abs().max() <= 1e-5 * ref.abs().max() + 2 * step
+
+
+@pytest.mark.parametrize("T", [17, 32, 33, 64, 65, 127, 128, 171, 600])
+@pytest.mark.parametrize("N,K", [(256, 128), (4096, 8192)])
+def test_prompt_linear_steps_by_rows(T, N, K):
+    """The steps behind a prompt's Linear at every change of kernel over the rows (stream-K boxes, single tiles, pairs cut along k): bf16 results
+    within a rounding (2^-8) of float64, fp32 ones within 2^-8 of the sum's scale for the rounded sum that is added."""
+    from mistral_inference_b200 import _abi_hybrid as h
+
+    g = torch.Generator(device=DEV).manual_seed(T + N)
+    x, w = torch.randn(T, K, device=DEV, generator=g).bfloat16(), (torch.randn(N, K, device=DEV, generator=g) / K ** 0.5).bfloat16()
+    b, base, rs = torch.randn(N, device=DEV, generator=g).bfloat16(), torch.randn(T, N, device=DEV, generator=g), torch.rand(T, 2, device=DEV, generator=g)
+    z = x.double() @ w.double().T
+    zb = z + b.double()
+    assert h._prompt_gemm_ok(x, T, N, K)
+    assert rel(h.linear(x, w, b, n_act=N // 2), torch.cat((torch.nn.functional.silu(zb[:, : N // 2]), zb[:, N // 2:]), 1)) < 2 ** -8
+    assert rel(h.linear(x, w, b, epi=h.EPI_F32, alpha=0.5), 0.5 * zb) < 1e-5
+    assert rel(h.linear(x, w, epi=h.EPI_RESIDUAL, residual=base.clone()) - base, z) < 2 ** -8
+    gate, up, s = z[:, 0::2], z[:, 1::2], rs.double().repeat_interleave(N // 4, 1)
+    assert rel(h.linear_swiglu(x, w, rs, N // 4), torch.nn.functional.silu(gate) * up * s) < 2 ** -7
+    assert rel(h.linear(x, w, epi=h.EPI_GLU, limit=1.5, alpha=1.7), gate.clamp(max=1.5) * torch.sigmoid(1.7 * gate.clamp(max=1.5)) * (up.clamp(-1.5, 1.5) + 1)) < 2 ** -7
