@@ -42,25 +42,29 @@ template <int MODE>
 static int run_linear(const void* x, const void* norm_w, const void* w, const EpiParams& epi, int64_t T, int64_t N, int64_t K, float eps,
                       void* workspace, size_t workspace_bytes, cudaStream_t st) {
   MB_CHECK_ARG(T >= 1, "linear: T=%lld", (long long)T);
-  if (T <= MB200_SKINNY_MAX_T) {
-    SkinnyParams p;
-    p.x = x;
-    p.norm_w = norm_w;
-    p.w = w;
-    p.N = (int)N;
-    p.K = (int)K;
-    p.eps = eps;
-    p.epi = epi;
+  const size_t need = kWsHeader + kWsPartial + align256((size_t)T * K * 2);
+  const bool room = workspace != nullptr && workspace_bytes >= need;
+  SkinnyParams p;
+  p.x = x;
+  p.norm_w = norm_w;
+  p.w = w;
+  p.N = (int)N;
+  p.K = (int)K;
+  p.eps = eps;
+  p.epi = epi;
+  if ((T <= MB200_SKINNY_MAX_T && !skinny_mma_better(T, K, norm_w != nullptr)) || (T <= MB200_SKINNY_MAX_T && norm_w && !room))
     return norm_w ? launch_skinny<MODE, true>(p, (int)T, st) : launch_skinny<MODE, false>(p, (int)T, st);
-  }
   const void* a = x;
   if (norm_w) {
-    const size_t need = kWsHeader + kWsPartial + align256((size_t)T * K * 2);
-    if (workspace == nullptr || workspace_bytes < need) return fail(MB200_E_WORKSPACE, "linear: workspace %zu < %zu", workspace_bytes, need);
-    void* normed = (uint8_t*)workspace + kWsHeader + kWsPartial;  // after the stream-K partial slots
+    if (!room) return fail(MB200_E_WORKSPACE, "linear: workspace %zu < %zu", workspace_bytes, need);
+    void* normed = (uint8_t*)workspace + kWsHeader + kWsPartial;  // after the partial sums
     int rc = run_rmsnorm(x, norm_w, normed, T, K, eps, st);
     if (rc) return rc;
     a = normed;
+  }
+  if (T <= MB200_SKINNY_MAX_T) {
+    p.x = a;
+    return launch_skinny_mma<MODE>(p, (int)T, st);
   }
   GemmParams g;
   g.a = a;
@@ -71,8 +75,8 @@ static int run_linear(const void* x, const void* norm_w, const void* w, const Ep
   g.epi = epi;
   if (streamk_eligible(T, N, K)) return launch_streamk<MODE>(g, workspace, workspace_bytes, kWsHeader, st);  // decode-sized batches: HBM-bound
   if (tcgen05_gemm_eligible(T, N, K)) {
-    const bool room = workspace != nullptr && workspace_bytes >= kWsHeader + kWsPartial;
-    return launch_gemm_tcgen05<MODE>(g, st, room ? (uint8_t*)workspace + kWsHeader : nullptr, room ? (unsigned*)((uint8_t*)workspace + SK_FLAGS_OFFSET) : nullptr);
+    const bool cuts = workspace != nullptr && workspace_bytes >= kWsHeader + kWsPartial;
+    return launch_gemm_tcgen05<MODE>(g, st, cuts ? (uint8_t*)workspace + kWsHeader : nullptr, cuts ? (unsigned*)((uint8_t*)workspace + SK_FLAGS_OFFSET) : nullptr);
   }
   return launch_gemm_mma<MODE>(g, st);
 }

@@ -285,3 +285,28 @@ def test_prompt_linear_steps_by_rows(T, N, K):
     gate, up, s = z[:, 0::2], z[:, 1::2], rs.double().repeat_interleave(N // 4, 1)
     assert rel(h.linear_swiglu(x, w, rs, N // 4), torch.nn.functional.silu(gate) * up * s) < 2 ** -7
     assert rel(h.linear(x, w, epi=h.EPI_GLU, limit=1.5, alpha=1.7), gate.clamp(max=1.5) * torch.sigmoid(1.7 * gate.clamp(max=1.5)) * (up.clamp(-1.5, 1.5) + 1)) < 2 ** -7
+
+
+@pytest.mark.parametrize("T", [2, 3, 4])
+@pytest.mark.parametrize("N,K", [(8, 256), (18, 8), (130, 2056), (512, 4096), (48, 4104), (1024, 5120), (64, 14336)])
+def test_linear_of_a_few_tokens(T, N, K):
+    """Either side of the step from FMAs to tensor cores (k above 4096, or four tokens with a norm): rows past the last full 16, k past the last full 256 and the
+    norm in front.  A Linear's output is bf16 (logits too, held as fp32): within its rounding, 2^-8, of float64, beside 2 K * 2^-24 of the sum
+    of the products' sizes (the sum in fp32, and once more where that moves it over a rounding's edge)."""
+    from mistral_inference_b200 import _abi
+
+    g = torch.Generator(device=DEV).manual_seed(T * N + K)
+    x, w = torch.randn(T, K, device=DEV, generator=g).bfloat16(), (torch.randn(N, K, device=DEV, generator=g) / K ** 0.5).bfloat16()
+    nw = torch.rand(K, device=DEV, generator=g).bfloat16()
+    ws = _abi.Workspace(_abi.workspace_bytes(8, K, 1, 1, 128, 256, N, 8), DEV)
+    logits = torch.full((T, N), float("nan"), device=DEV)
+    _abi.lm_head(x, nw, w, logits, 1e-5, ws)
+    n = _abi.rmsnorm(x, nw, 1e-5).double()
+    ref = n @ w.double().T
+    assert ((logits - ref).abs() <= 2 ** -8 * ref.abs() + 2 * K * 2 ** -24 * (n.abs() @ w.double().abs().T)).all()
+    res, out = torch.randn(T, N, device=DEV, generator=g).bfloat16(), torch.empty(T, N, dtype=torch.bfloat16, device=DEV)
+    _abi.linear_residual(x, w, None, out, ws)
+    assert rel(out, x.double() @ w.double().T) < 2 ** -8
+    ref = x.double() @ w.double().T + res.double()
+    _abi.linear_residual(x, w, res, res, ws)  # in place
+    assert rel(res, ref) < 2 ** -7  # the product's rounding and the sum's, 2^-8 of each size
