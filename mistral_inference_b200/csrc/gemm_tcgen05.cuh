@@ -2,10 +2,12 @@
 //
 // Roofline: tensor pipe (2*T*N*K flops).  Persistent, warp-specialised kernel, one CTA per SM:
 //   warp 0   TMA producer: cp.async.bulk.tensor (128B-swizzled [128 x 64] A tile + [BN x 64] W tile per stage) -> 4- or 6-stage
-//            ring.  For T >= 512 the CTAs run as clusters of two on vertically adjacent tiles and each fetches half of the
-//            shared W tile, multicast into both shared memories (2/3 of the L2 -> SM traffic of the single-CTA kernel)
-//   warp 1   MMA issuer: one elected thread issues tcgen05.mma (M = 128, N = BN, K = 16 x 4 per stage); tcgen05.commit
-//            releases the shared-memory stage (in both CTAs of a pair) and, after the last k-block, publishes the accumulator
+//            ring.  For T >= 512 the CTAs run as clusters of two on vertically adjacent tiles: one MMA of 256 rows spans both SMs
+//            (cta_group::2), each CTA fetches its own 128 rows of A and HALF of the W tile (2/3 of the L2 -> SM traffic of the
+//            single-CTA kernel, a ring of six or seven stages)
+//   warp 1   MMA issuer: one elected thread issues tcgen05.mma (M = 128, N = BN, K = 16 x 4 per stage; a pair: M = 256, issued by
+//            its first CTA for both); tcgen05.commit releases the shared-memory stage (in both CTAs of a pair) and, after the last
+//            k-block, publishes the accumulator
 //   warps 2-5 epilogue: one thread per output row reads the fp32 accumulator out of TMEM 32 columns at a time (two TMEM
 //            buffers, so the MMAs of the next tile overlap this one's epilogue; two register buffers, so the next tcgen05.ld
 //            overlaps this chunk's arithmetic) and runs the row-chunk epilogues of epilogue.cuh (bf16 rounding, then RoPE +
@@ -38,10 +40,11 @@ constexpr int TG_A_BYTES = TG_BM * TG_BK * 2;
 // memory -- accumulator row i depends on A row i only, and rows >= T are never stored.  The stage shrinks to (TA + BN) * 128
 // bytes, so the ring gets deep enough (16-20 stages) to keep a whole SM's share of HBM bandwidth in flight: those launches are
 // weight-streaming GEMMs, bound by HBM, with BN chosen by the launcher to give every SM at most one (equal) tile per round.
-template <int BN, int TA = 128>
+// CL = 2: a pair of CTAs (see tc_gemm_body); a CTA's stage holds half of the W tile.  EXTRA: shared memory an epilogue needs beside the ring.
+template <int BN, int TA = 128, int CL = 1, int EXTRA = 0>
 struct TgCfg {
   static constexpr int kABytes = TA * TG_BK * 2;
-  static constexpr int kBBytes = BN * TG_BK * 2;
+  static constexpr int kBBytes = BN / CL * TG_BK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
   // The MMA always reads M = 128 rows (16 KB) from a stage's A base; with a short A box that runs on into the stage's W tile
   // (harmless: accumulator row i depends on A row i only) and, in the LAST stage, past it when the stage is smaller than 16 KB.
@@ -55,20 +58,21 @@ struct TgCfg {
 #else
   static constexpr int kSlack = TA < 128 ? TG_A_BYTES : 0;
 #endif
-  static constexpr int kMaxStages = (227 * 1024 - 1024 - 512 - kSlack) / kStageBytes;
+  static constexpr int kMaxStages = (227 * 1024 - 1024 - 512 - kSlack - EXTRA) / kStageBytes;
   // decode-sized variants: a ring of ~100 KB (80 KB of weights in flight per CTA, above the ~45-65 KB bandwidth-delay product of
   // one SM's HBM share) instead of the whole 227 KB: measured faster in a chain of dependent launches (scripts/bench_linear.py:
   // qkv 24.0 -> 21.3 us, down 39.5 -> 36.8 us; only the 1.3 GB lm head loses 5 %) -- a successor's CTA, which starts when the
   // predecessor's CTA on its SM exits, has its first ring filled sooner, and other decode kernels' CTAs fit beside it.
   static constexpr int kShortRingStages = (100 * 1024) / kStageBytes;
-  static constexpr int kStages = (TA < 128 || BN < 128) ? (kShortRingStages < 3 ? 3 : (kShortRingStages > kMaxStages ? kMaxStages : kShortRingStages))
+  static constexpr int kStages = CL == 2 ? (kMaxStages > 8 ? 8 : kMaxStages) : (TA < 128 || BN < 128) ? (kShortRingStages < 3 ? 3 : (kShortRingStages > kMaxStages ? kMaxStages : kShortRingStages))
                                                         : (BN == 128 ? 6 : 4);
-  static constexpr int kSmem = kStages * kStageBytes + kSlack + 1024 /*align*/ + 512 /*barriers*/;
-  static constexpr int kSmemLayer = kSmem + 4 * 4096;  // EPI_LAYER: 4 KB per epilogue warp to turn fp32 blocks (epi_layer32_f32)
+  static constexpr int kSmem = kStages * kStageBytes + kSlack + 1024 /*align*/ + 512 /*barriers*/ + EXTRA;
   static constexpr int kTmemCols = 2 * BN <= 32 ? 32 : (2 * BN <= 64 ? 64 : (2 * BN <= 128 ? 128 : (2 * BN <= 256 ? 256 : 512)));  // 2 accumulators
   // Instruction descriptor (cute::UMMA::InstrDescriptor): D = F32, A = B = BF16, both K-major, N >> 3 at bit 17, M >> 4 at bit 24
-  static constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TG_BM >> 4) << 24);
+  static constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(CL * TG_BM >> 4) << 24);
 };
+template <int MODE>
+constexpr int kEpiSmem = MODE == EPI_LAYER ? 4 * 4096 : 0;  // 4 KB per epilogue warp to turn fp32 blocks (epi_layer32_f32)
 
 struct TcGemmParams {
   int T, N, K;
@@ -76,9 +80,9 @@ struct TcGemmParams {
   // grouped, experts packed in ONE matrix (layered decoders): expert e's weights start w_n * e rows and w_k * e columns into the single
   // tensor map; w_n = w_k = 0: a tensor map per expert
   int w_n = 0, w_k = 0;
-  // cluster pairs of 256-wide tiles, dense (plan_pairs): work items are the odd last row of tiles (two column tiles an item), whole tile pairs, and
-  // at the end the last `cut_pairs` pairs, each cut into `cut` parts along k.  cut_pairs < 0: every pair whole, an odd row as pairs too
-  int cut_pairs = -1, cut = 1;
+  // pairs of 256-wide tiles, dense (plan_pairs): work items are whole tile pairs and at the end the last `cut_pairs` pairs, each cut into `cut`
+  // parts along k
+  int cut_pairs = 0, cut = 1;
   float* partials = nullptr;   // [(cut - 1) * cut_pairs][2 CTAs][256 / 4][128 rows] float4: what the parts but the first leave for it
   unsigned* flags = nullptr;   // [(cut - 1) * cut_pairs * 2], zero between launches
 };
@@ -91,13 +95,12 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
                "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
                : "memory");
 }
-// Same, delivered to the same shared-memory offset (and signalled on the same barrier offset) of every CTA in cta_mask.
-__device__ __forceinline__ void tma_load_2d_multicast(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, uint16_t cta_mask) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.multicast::cluster [%0], [%1, {%3, %4}], [%2], %5;" ::"r"(
-          smem_u32(smem_dst)),
-      "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "h"(cta_mask)
-      : "memory");
+// Same for a pair of CTAs that share MMAs: the tile goes to this CTA's shared memory, its bytes count on `bar`, a shared::cluster address that
+// may lie in the other CTA of the pair.
+__device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
+  asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(smem_dst)),
+               "l"(map), "r"(bar), "r"(c0), "r"(c1)
+               : "memory");
 }
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
@@ -108,12 +111,30 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void tmem_alloc(uint32_t* smem_result, uint32_t ncols) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_result)), "r"(ncols) : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+// shared::cluster address of `p`'s offset in the cluster's first CTA
+__device__ __forceinline__ uint32_t cluster_first(const void* p) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(0u));
+  return r;
 }
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) { asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory"); }
+// CL: CTAs that share MMAs (1 or 2).  Every tcgen05 instruction of a kernel names the same cta_group; a pair allocates in both CTAs.
+template <int CL = 1>
+__device__ __forceinline__ void tmem_alloc(uint32_t* smem_result, uint32_t ncols) {
+  if constexpr (CL == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_result)), "r"(ncols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  } else {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_result)), "r"(ncols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+}
+template <int CL = 1>
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+  if constexpr (CL == 1)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+  else
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -128,14 +149,24 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint6
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// the same by a pair of CTAs (issued by the first): its A and B tiles are the rows of both CTAs' shared memories at these offsets, D its rows' halves
+__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
+      "}\n" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 // arrive on an mbarrier once every previously issued tcgen05.mma of this thread has completed
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-// the same arrival on the barrier at this offset in every CTA of cta_mask
-__device__ __forceinline__ void umma_commit_multicast(uint64_t* bar, uint16_t cta_mask) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
-               "h"(cta_mask)
+// the same for the MMAs of a pair, on the barrier at this offset in both CTAs
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)), "h"((uint16_t)3)
                : "memory");
 }
 __device__ __forceinline__ void tmem_ld_32x32b_x32_nowait(uint32_t taddr, uint32_t (&v)[32]) {
@@ -170,17 +201,23 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
   return (uint64_t)((smem_addr & 0x3ffff) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
 
-// CL = 2: thread-block clusters of two CTAs that work on vertically adjacent tiles (same W columns, consecutive 128-row blocks).
-// Each CTA fetches HALF of the shared [256 x 64] W tile and TMA-multicasts it into both shared memories, so the L2 -> SM traffic
-// per CTA and k-block drops from 48 KB to 32 KB (at T = 4096 the single-CTA kernel pulls ~20 TB/s out of L2).  A stage may be
-// refilled only when BOTH CTAs' MMAs have read it: the empty barriers count two commits, each multicast to the pair.
+// CL = 2: clusters of two CTAs that share MMAs (cta_group::2) on vertically adjacent tiles (same W columns, consecutive 128-row blocks).  A CTA
+// holds its 128 rows of A and half of the [256 x 64] W tile, the MMA reads both shared memories: 32 KB per CTA and k-block out of L2 where the
+// single-CTA kernel takes 48 KB (at T = 4096 it pulls ~20 TB/s), and a stage of 32 KB leaves room for a ring of seven.  Both CTAs' copies
+// count on the first CTA's full[] barrier; its MMA thread issues for both and its commits free the stage, and publish the accumulator, in both;
+// both CTAs' epilogues release an accumulator on the first CTA's tmem_empty[].  No copy is multicast: each tile is read by the CTA that holds it.
+// A last row of tiles without a neighbour below is a pair whose second tile lies past the end of A: zeros, read from nowhere, never stored.  (The
+// pair's MMA of 128 rows, 64 in each CTA, takes as long as that of 256: with it on such rows, scoring 1102 tokens was 2186 us against 2006.)
+// Measured against single-CTA MMAs whose W tile each CTA copied into both, ring of four: 4096-token prompt 1728 -> 1707 us a layer, 1102 tokens
+// through a 131072-wide head 2064 -> 2006, 4096 tokens through two layers of width 4096 3995 -> 3854; eight experts of ~512 rows, half of them with
+// a fifth tile, 1679 -> 1736 (there the two CTAs of a lone row took two column tiles).
 //
 // GROUPED = true (mixture of experts, csrc/moe.cuh): the A rows are the (token, expert) pairs sorted by expert, every expert's
 // segment padded to a multiple of TA rows; m tile i covers rows plan.tile_row0[i] .. + TA of expert plan.tile_expert[i], whose
 // weight matrix has its own tensor map (map_w[expert]).  The number of m tiles is DEVICE data (no host sync after routing).
-constexpr int MOE_PLAN_HEADER = 64;  // int32 words: [0] m tiles of this rank, [1] padded rows in total, [2] tile capacity, [6] tile pairs and single tiles, [7] how many of these are pairs (they come first), [8..] segment starts
+constexpr int MOE_PLAN_HEADER = 64;  // int32 words: [0] m tiles of this rank, [1] padded rows in total, [2] tile capacity, [6] tile pairs, [8..] segment starts
 // after the header: tile_expert[cap], tile_row0[cap], pair_expert[cap], pair_info[cap] (cap = plan[2]).  A PAIR is two vertically
-// adjacent m tiles of ONE expert (bit 30 of pair_info), a single tile the last one of an odd number: the units of the 2-CTA cluster variant.
+// adjacent m tiles of ONE expert (or a single last tile: bit 30 of pair_info clear), the unit of the 2-CTA cluster variant.
 constexpr int MOE_PAIR_SECOND = 1 << 30;
 constexpr int MOE_MAX_EXPERTS = 16;  // tensor maps travel as kernel parameters (128 B each)
 struct MoeWeightMaps {
@@ -190,8 +227,8 @@ struct MoeWeightMaps {
 template <int MODE, int CL, int BN, int TA, bool GROUPED>
 __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUtensorMap* map_w_base, const TcGemmParams& p, const int32_t* plan) {
   static_assert(TA == 128 || CL == 1, "small-batch variant is single-CTA");
-  using Cfg = TgCfg<BN, TA>;
-  constexpr int TG_STAGES = Cfg::kStages, TG_B_BYTES = Cfg::kBBytes, TG_STAGE_BYTES = Cfg::kStageBytes, TG_TMEM_COLS = Cfg::kTmemCols;
+  using Cfg = TgCfg<BN, TA, CL, kEpiSmem<MODE>>;
+  constexpr int TG_STAGES = Cfg::kStages, TG_STAGE_BYTES = Cfg::kStageBytes, TG_TMEM_COLS = Cfg::kTmemCols;
   constexpr int TG_A_BYTES = Cfg::kABytes;  // shadows the 128-row constant
   constexpr int TG_BN = BN;
   constexpr uint32_t kUmmaIdesc = Cfg::kIdesc;
@@ -209,17 +246,11 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
   const int cta = (int)blockIdx.x / CL, n_cta = (int)gridDim.x / CL;  // cluster index / clusters in the grid
   // a cluster walks "super tiles" of CL vertically adjacent tiles; rows past T read as zeros (TMA) and are never stored
   // grouped: m units are the plan's tiles (single CTA) or tile pairs (cluster of two)
-  // SINGLE tiles (pairs of 256-wide tiles only): where a row of tiles has no neighbour below, the two CTAs take the SAME rows and two
-  // neighbouring column tiles instead of a pair whose second tile is recomputed or empty.
-  constexpr bool kSingles = CL == 2 && BN == 256;
-  constexpr bool kCuts = kSingles && !GROUPED;
-  const int m_tiles = (p.T + TG_BM - 1) / TG_BM, num_n = p.N / TG_BN, num_k = p.K / TG_BK;
-  const bool planned = kCuts && p.cut_pairs >= 0;
-  const int num_m = GROUPED ? (kSingles ? plan[7] : (CL > 1 ? plan[6] : plan[0])) : (planned ? m_tiles / 2 : (m_tiles + CL - 1) / CL);
-  const int half_n = (num_n + 1) / 2;
-  const int lone_rows = GROUPED ? (kSingles ? plan[6] - plan[7] : 0) : (planned ? m_tiles & 1 : 0);
-  const int lone = lone_rows * half_n, whole = num_m * num_n - (planned ? p.cut_pairs : 0);
-  const int num_tiles = lone + whole + (planned ? p.cut * p.cut_pairs : 0);
+  constexpr bool kCuts = CL == 2 && BN == 256 && !GROUPED;
+  static_assert(!kCuts || TG_STAGES * TG_STAGE_BYTES >= TG_BM * BN * 4, "another part's sums fit in the ring");
+  const int num_n = p.N / TG_BN, num_k = p.K / TG_BK;
+  const int num_m = GROUPED ? (CL > 1 ? plan[6] : plan[0]) : ((p.T + TG_BM - 1) / TG_BM + CL - 1) / CL;
+  const int whole = num_m * num_n - (kCuts ? p.cut_pairs : 0), num_tiles = whole + (kCuts ? p.cut * p.cut_pairs : 0);
   const int32_t* tile_expert = GROUPED ? plan + MOE_PLAN_HEADER + (CL > 1 ? 2 * plan[2] : 0) : nullptr;
   const int32_t* tile_row0 = GROUPED ? tile_expert + plan[2] : nullptr;
   // Tile order.  The persistent CTAs take tiles t = cta, cta + n_cta, ...: at any moment ~n_cta consecutive tile ids are in flight,
@@ -262,22 +293,12 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
   };
   struct Item {
     int mu, m0, n0, kb0, kb1;
-    bool store, lone;  // lone: a single tile, W is not shared with the other CTA
-    int part, slot;    // part of a cut pair (0: the owner, which adds the others' sums), -1: not cut
+    int part, slot;  // part of a cut pair (0: the owner, which adds the others' sums), -1: not cut
   };
   auto item_of = [&](int tile) {
     Item it;
-    it.kb0 = 0, it.kb1 = num_k, it.store = true, it.lone = false, it.part = -1, it.slot = 0, it.mu = 0;
-    if (kSingles && tile < lone) {
-      const int row = tile % lone_rows, nt = 2 * (tile / lone_rows) + rank;
-      it.lone = true;
-      it.store = nt < num_n;
-      it.n0 = min(nt, num_n - 1) * TG_BN;
-      it.mu = GROUPED ? num_m + row : 0;
-      it.m0 = GROUPED ? tile_row0[it.mu] & (MOE_PAIR_SECOND - 1) : (m_tiles - 1) * TG_BM;
-      return it;
-    }
-    int t = tile - lone, nt;
+    it.kb0 = 0, it.kb1 = num_k, it.part = -1, it.slot = 0;
+    int t = tile, nt;
     if (kCuts && t >= whole) {
       const int s = t - whole;
       it.part = s / p.cut_pairs;
@@ -290,7 +311,8 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
     it.n0 = nt * TG_BN;
     if (GROUPED) {
       const int info = tile_row0[it.mu];
-      it.m0 = CL == 1 ? info : (info & (MOE_PAIR_SECOND - 1)) + rank * TG_BM;  // (CL == 2: the plan's first units have both tiles)
+      it.m0 = info & (MOE_PAIR_SECOND - 1);
+      if (CL > 1 && rank == 1) it.m0 = (info & MOE_PAIR_SECOND) != 0 ? it.m0 + TG_BM : p.T;  // p.T: past the last row
     } else {
       it.m0 = (it.mu * CL + rank) * TG_BM;
     }
@@ -301,21 +323,21 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
   if (threadIdx.x == 0) {
     for (int i = 0; i < TG_STAGES; ++i) {
       mbar_init(&full[i], 1);
-      mbar_init(&empty[i], CL);
+      mbar_init(&empty[i], 1);
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&tmem_full[i], 1);
-      mbar_init(&tmem_empty[i], 4);  // one arrive per epilogue warp
+      mbar_init(&tmem_empty[i], 4 * CL);  // one arrive per epilogue warp
     }
     mbar_init(cut_full, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
     if (!GROUPED) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
   }
-  if (warp == 1) tmem_alloc(tmem_base_slot, TG_TMEM_COLS);
+  if (warp == 1) tmem_alloc<CL>(tmem_base_slot, TG_TMEM_COLS);
   tc_fence_before();
   if (CL > 1)
-    cluster_sync_all();  // the peer's barriers must be initialised before any multicast copy or commit reaches them
+    cluster_sync_all();  // the peer's barriers must be initialised before any copy or commit reaches them
   else
     __syncthreads();
   tc_fence_after();
@@ -335,23 +357,24 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
         for (int kb = w.kb0; kb < w.kb1; ++kb, ++it) {
           const uint32_t s = it % TG_STAGES, par = (it / TG_STAGES) & 1;
           mbar_wait(&empty[s], par ^ 1, 11, it);
-          mbar_arrive_expect_tx(&full[s], TG_STAGE_BYTES);  // A + both halves of W (the peer's half may land first: tx-count goes negative)
           uint8_t* sa = smem + s * TG_STAGE_BYTES;
-          tma_load_2d(sa, &map_a, &full[s], kb * TG_BK, m0);
-          if (kSingles && w.lone) {  // the boxes are half tiles
+          if (CL > 1) {
+            // the pair's four tiles count on the first CTA's barrier (the other CTA's may land before it is armed: the count goes negative)
+            if (rank == 0) mbar_arrive_expect_tx(&full[s], CL * TG_STAGE_BYTES);
+            const uint32_t bar = cluster_first(&full[s]);
+            tma_load_2d_pair(sa, &map_a, bar, kb * TG_BK, m0);
+            tma_load_2d_pair(sa + TG_A_BYTES, wmap, bar, wc + kb * TG_BK, wr + rank * (TG_BN / CL));
+          } else {
+            mbar_arrive_expect_tx(&full[s], TG_STAGE_BYTES);
+            tma_load_2d(sa, &map_a, &full[s], kb * TG_BK, m0);
             tma_load_2d(sa + TG_A_BYTES, wmap, &full[s], wc + kb * TG_BK, wr);
-            tma_load_2d(sa + TG_A_BYTES + TG_B_BYTES / 2, wmap, &full[s], wc + kb * TG_BK, wr + TG_BN / 2);
-          } else if (CL > 1)
-            tma_load_2d_multicast(sa + TG_A_BYTES + rank * (TG_B_BYTES / CL), wmap, &full[s], wc + kb * TG_BK, wr + rank * (TG_BN / CL),
-                                  (uint16_t)((1u << CL) - 1));
-          else
-            tma_load_2d(sa + TG_A_BYTES, wmap, &full[s], wc + kb * TG_BK, wr);
+          }
         }
       }
     }
   } else if (warp == 1) {
-    // ================= MMA issuer (one thread) =================
-    if (lane == 0) {
+    // ================= MMA issuer (one thread, for both CTAs of a pair) =================
+    if (lane == 0 && rank == 0) {
       uint32_t it = 0, acc_it = 0;
       for (int tile = cta; tile < num_tiles; tile += n_cta, ++acc_it) {
         const uint32_t acc = acc_it & 1, acc_par = (acc_it >> 1) & 1;
@@ -371,28 +394,39 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
           const uint64_t adesc = umma_desc_sw128(a_addr), bdesc = umma_desc_sw128(a_addr + TG_A_BYTES);
 #pragma unroll
           for (int k = 0; k < TG_BK / 16; ++k)  // +32 bytes (= 2 in 16-byte units) per K = 16 step inside the 128-byte swizzled row
-            umma_bf16(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), kUmmaIdesc, (kb > kb0 || k) ? 1u : 0u);
-          if (CL > 1)  // frees the stage in both CTAs (each producer writes into both) when these MMAs have read it
-            umma_commit_multicast(&empty[s], (uint16_t)((1u << CL) - 1));
+            if constexpr (CL > 1)
+              umma_bf16_pair(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), kUmmaIdesc, (kb > kb0 || k) ? 1u : 0u);
+            else
+              umma_bf16(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), kUmmaIdesc, (kb > kb0 || k) ? 1u : 0u);
+          if (CL > 1)  // frees the stage in both CTAs when these MMAs have read it
+            umma_commit_pair(&empty[s]);
           else
             umma_commit(&empty[s]);
         }
-        umma_commit(&tmem_full[acc]);  // accumulator complete
+        if (CL > 1)
+          umma_commit_pair(&tmem_full[acc]);  // accumulator complete, in both CTAs
+        else
+          umma_commit(&tmem_full[acc]);
       }
     }
   } else {
     // ================= epilogue warps 2..5: TMEM lanes 32*(warp%4) .. +31 =================
     const int lane_base = (warp & 3) * 32;
+    auto release = [&](uint32_t acc) {  // the MMA thread may overwrite this accumulator buffer
+      if (CL > 1)
+        mbar_arrive_cluster(cluster_first(&tmem_empty[acc]));
+      else
+        mbar_arrive(&tmem_empty[acc]);
+    };
     uint32_t acc_it = 0;
     for (int tile = cta; tile < num_tiles; tile += n_cta, ++acc_it) {
       const Item w = item_of(tile);
       const int m0 = w.m0, n0 = w.n0;
-      const bool store = w.store;
       const uint32_t acc = acc_it & 1, acc_par = (acc_it >> 1) & 1;
       mbar_wait(&tmem_full[acc], acc_par, 14, acc_it);
       tc_fence_after();
       // accumulator rows >= TA were computed from whatever follows the short A box in shared memory: never stored
-      const int t = (store && (TA == 128 || lane_base + lane < TA)) ? m0 + lane_base + lane : 0x7fffffff;
+      const int t = (TA == 128 || lane_base + lane < TA) ? m0 + lane_base + lane : 0x7fffffff;
       // two register buffers: the TMEM load of chunk c+1 is in flight while chunk c goes through the epilogue
       const uint32_t trow = tmem_base + ((uint32_t)lane_base << 16) + acc * TG_BN;
       uint32_t va[32], vb[32];
@@ -426,7 +460,7 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
           if (threadIdx.x == 64) st_release_u32(p.flags + at, 1u);
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&tmem_empty[acc]);
+          if (lane == 0) release(acc);
           continue;
         }
         if (w.part == 0) {
@@ -496,7 +530,7 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
         }
       } else if constexpr (MODE == EPI_LAYER) {
         const bool f32 = layer_step_is_f32(p.epi.layer);
-        const int rows = store ? max(0, min(32, p.T - m0 - lane_base)) : 0;
+        const int rows = max(0, min(32, p.T - m0 - lane_base));
         float4* stg = reinterpret_cast<float4*>(reinterpret_cast<uint8_t*>(full) + 512) + (warp & 3) * 256;
         auto chunk = [&](int n, const uint32_t (&v)[32]) {
           if (f32)
@@ -531,15 +565,15 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&tmem_empty[acc]);
+      if (lane == 0) release(acc);
     }
   }
   tc_fence_before();
   if (CL > 1)
-    cluster_sync_all();  // the peer's last commits still arrive on this CTA's barriers
+    cluster_sync_all();  // the peer's last commits and arrivals still reach this CTA's barriers, its MMAs this CTA's memory
   else
     __syncthreads();
-  if (warp == 1) tmem_dealloc(tmem_base, TG_TMEM_COLS);
+  if (warp == 1) tmem_dealloc<CL>(tmem_base, TG_TMEM_COLS);
 }
 
 template <int MODE, int CL, int BN, int TA = 128>
@@ -607,16 +641,14 @@ inline int tcgen05_forced_bn() {
   return e != nullptr ? atoi(e) : 0;
 }
 
-// How a dense launch of cluster pairs (256 x 256 outputs an item, `units` pairs on the chip) ends.  Items run in rounds of `units`; when the
-// last round is at most half full, its pairs are cut along k into as many parts as fill it (at most four, eight k-blocks each): the parts' fp32
-// sums meet in the first part's epilogue, in the order of k.  The odd last row of tiles comes first, two column tiles an item.
-// T = 4096, 7B shapes: wo + w2 498 -> 486 us (3.46 rounds, the last half full); T = 1102 (9 row tiles): wo 48 -> 29 us, w2 151 -> 100 us.
+// How a dense launch of pairs (256 x 256 outputs an item, `units` pairs on the chip) ends.  Items run in rounds of `units`; when the last round is
+// at most half full, its pairs are cut along k into as many parts as fill it (at most four, eight k-blocks each): the parts' fp32 sums meet in the
+// first part's epilogue, in the order of k.
 inline void plan_pairs(TcGemmParams& p, int units, void* scratch, unsigned* flags) {
-  const int m_tiles = (p.T + TG_BM - 1) / TG_BM, num_n = p.N / 256, pairs = m_tiles / 2 * num_n, lone = (m_tiles & 1) * ((num_n + 1) / 2);
-  const int rest = (pairs + lone) % units;
+  const int rest = (p.T + 2 * TG_BM - 1) / (2 * TG_BM) * (p.N / 256) % units;
   p.cut_pairs = 0;
   p.cut = 1;
-  if (scratch == nullptr || rest == 0 || rest > pairs) return;
+  if (scratch == nullptr || rest == 0) return;
   int cut = units / rest;
   if (cut > 4) cut = 4;
   while (cut > 1 && ((cut - 1) * rest > TG_MAX_CUTS || p.K / TG_BK < 8 * cut)) --cut;
@@ -635,14 +667,12 @@ inline bool pairs_fill(int64_t T, int64_t N, int64_t K, int units, bool cuts) {
   p.N = (int)N;
   p.K = (int)K;
   plan_pairs(p, units, cuts && K >= 8192 ? &p : nullptr, nullptr);  // (any scratch: how would it be cut?)
-  const int m_tiles = (p.T + TG_BM - 1) / TG_BM, num_n = p.N / 256, items = m_tiles / 2 * num_n + (m_tiles & 1) * ((num_n + 1) / 2) + (p.cut - 1) * p.cut_pairs;
-  return 2 * items >= units;
+  return 2 * ((p.T + 2 * TG_BM - 1) / (2 * TG_BM) * (p.N / 256) + (p.cut - 1) * p.cut_pairs) >= units;
 }
 
 template <int MODE, int BN>
 int launch_gemm_tcgen05_bn(const GemmParams& g, bool pair, int sms, cudaStream_t stream, void* scratch, unsigned* flags) {
-  using Cfg = TgCfg<BN>;
-  constexpr int kSmem = MODE == EPI_LAYER ? Cfg::kSmemLayer : Cfg::kSmem;
+  constexpr int kSmem = TgCfg<BN, 128, 1, kEpiSmem<MODE>>::kSmem, kSmemPair = TgCfg<BN, 128, 2, kEpiSmem<MODE>>::kSmem;
   CUtensorMap map_a, map_w;
   int rc = make_tensor_map_2d(&map_a, g.a, g.T, g.K, TG_BM);
   if (rc) return rc;
@@ -658,11 +688,11 @@ int launch_gemm_tcgen05_bn(const GemmParams& g, bool pair, int sms, cudaStream_t
     int supers = ceil_div(ceil_div(g.T, TG_BM), 2) * (g.N / BN);
     if (BN == 256) plan_pairs(p, pairs, scratch, flags);
     if (p.cut_pairs > 0) supers = pairs;  // the last round is full
-    MB_CHECK_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<MODE, 2, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+    MB_CHECK_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<MODE, 2, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemPair));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2u * (unsigned)(supers < pairs ? supers : pairs));
     cfg.blockDim = dim3(TG_THREADS);
-    cfg.dynamicSmemBytes = kSmem;
+    cfg.dynamicSmemBytes = kSmemPair;
     cfg.stream = stream;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;

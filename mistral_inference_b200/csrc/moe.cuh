@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(MP_THREADS) moe_plan_kernel(const int32_t* __r
       plan[3] = pairs;
       plan[4] += touched;
       plan[5] += 1;
-      plan[6] = plan[7] = 0;  // calls this small never take the cluster variant
+      plan[6] = 0;  // calls this small never take the cluster variant
     }
     __syncthreads();
     for (int i = tid; i < pairs; i += MP_THREADS) slot[i] = sel[i] < E ? slot[i] + seg[sel[i]] : -1;
@@ -197,21 +197,12 @@ __global__ void __launch_bounds__(MP_THREADS) moe_plan_kernel(const int32_t* __r
           plan[MOE_PLAN_HEADER + n] = e;
           plan[MOE_PLAN_HEADER + tile_cap + n] = rows + m * tile_rows;
         }
-        for (int m = 0; m + 1 < m_tiles && np < tile_cap; m += 2, ++np) {  // pairs of vertically adjacent tiles for the 2-CTA cluster GEMM
+        for (int m = 0; m < m_tiles && np < tile_cap; m += 2, ++np) {  // pairs of vertically adjacent tiles for the 2-CTA cluster GEMM
           plan[MOE_PLAN_HEADER + 2 * tile_cap + np] = e;
-          plan[MOE_PLAN_HEADER + 3 * tile_cap + np] = (rows + m * tile_rows) | MOE_PAIR_SECOND;
+          plan[MOE_PLAN_HEADER + 3 * tile_cap + np] = (rows + m * tile_rows) | (m + 1 < m_tiles ? MOE_PAIR_SECOND : 0);
         }
       }
       rows += m_tiles * tile_rows;
-    }
-    plan[7] = np;
-    for (int e = 0; e < E; ++e) {  // then the last tiles of the experts that have an odd number of them
-      const int m_tiles = (total[e] + tile_rows - 1) / tile_rows;
-      if ((m_tiles & 1) && e % shard_world == shard_rank && np < tile_cap) {
-        plan[MOE_PLAN_HEADER + 2 * tile_cap + np] = e;
-        plan[MOE_PLAN_HEADER + 3 * tile_cap + np] = seg[e] + (m_tiles - 1) * tile_rows;
-        ++np;
-      }
     }
     plan[6] = np;
     seg[E] = rows;
@@ -353,7 +344,7 @@ inline int64_t moe_row_cap(int64_t pairs, int64_t E, int tile_rows) { return moe
 template <int MODE, int BN, int TA, int CL = 1>
 int launch_grouped_bn(const void* a, int64_t rows_cap, int64_t K, int64_t N, const void* const* w_host, int E, const int32_t* plan, const EpiParams& epi,
                       int sms, cudaStream_t stream) {
-  using Cfg = TgCfg<BN, TA>;
+  using Cfg = TgCfg<BN, TA, CL, kEpiSmem<MODE>>;
   CUtensorMap map_a;
   MoeWeightMaps maps;
   int rc = make_tensor_map_2d(&map_a, a, rows_cap, K, TA);
@@ -364,7 +355,7 @@ int launch_grouped_bn(const void* a, int64_t rows_cap, int64_t K, int64_t N, con
       maps.m[e] = map_a;
       continue;
     }
-    rc = make_tensor_map_2d(&maps.m[e], w, N, K, BN / CL);  // cluster pairs: each CTA fetches half of the W tile and multicasts it
+    rc = make_tensor_map_2d(&maps.m[e], w, N, K, BN / CL);  // pairs: each CTA holds half of the W tile
     if (rc) return rc;
   }
   TcGemmParams p;
@@ -441,7 +432,7 @@ int launch_grouped(const void* a, int64_t rows_cap, int64_t K, int64_t N, const 
     return launch_grouped_streamk<MODE, 64>(a, rows_cap, K, N, w_host, E, plan, epi, workspace, workspace_bytes, header, sms, stream);
   }
   if (tile_rows == 128) {
-    // enough rows per expert for vertically adjacent tile pairs: the 2-CTA cluster kernel (W tile multicast, 2/3 of the L2 -> SM traffic)
+    // enough rows per expert for vertically adjacent tile pairs: the 2-CTA kernel (W tile shared, 2/3 of the L2 -> SM traffic)
     if (N % 256 == 0 && tcgen05_cluster_enabled() && rows_cap >= (int64_t)E * 512)
       return launch_grouped_bn<MODE, 256, 128, 2>(a, rows_cap, K, N, w_host, E, plan, epi, sms, stream);
     if (N % 256 == 0) return launch_grouped_bn<MODE, 256, 128>(a, rows_cap, K, N, w_host, E, plan, epi, sms, stream);
@@ -531,7 +522,7 @@ __global__ void __launch_bounds__(256) layer_moe_combine_kernel(const float4* __
 template <int BN, int CL>
 int launch_grouped_packed_bn(const void* a, int64_t rows_cap, int64_t K, int64_t N, const void* w, int64_t w_rows, int64_t w_cols, int64_t w_n, int64_t w_k,
                              const int32_t* plan, const EpiParams& epi, int sms, cudaStream_t stream) {
-  using Cfg = TgCfg<BN, 128>;
+  using Cfg = TgCfg<BN, 128, CL, kEpiSmem<EPI_LAYER>>;
   CUtensorMap map_a;
   MoeWeightMaps maps;
   int rc = make_tensor_map_2d(&map_a, a, rows_cap, K, 128);
@@ -546,11 +537,11 @@ int launch_grouped_packed_bn(const void* a, int64_t rows_cap, int64_t K, int64_t
   p.epi = epi;
   p.w_n = (int)w_n;
   p.w_k = (int)w_k;
-  MB_CHECK_CUDA(cudaFuncSetAttribute(gemm_tcgen05_grouped_kernel<EPI_LAYER, CL, BN, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemLayer));
+  MB_CHECK_CUDA(cudaFuncSetAttribute(gemm_tcgen05_grouped_kernel<EPI_LAYER, CL, BN, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(sms / CL * CL));
   cfg.blockDim = dim3(TG_THREADS);
-  cfg.dynamicSmemBytes = Cfg::kSmemLayer;
+  cfg.dynamicSmemBytes = Cfg::kSmem;
   cfg.stream = stream;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -571,7 +562,7 @@ inline int launch_grouped_packed(const void* a, int64_t rows_cap, int64_t K, int
   int dev = 0, sms = 0;
   MB_CHECK_CUDA(cudaGetDevice(&dev));
   MB_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  if (N % 256 == 0 && pairs >= 384 * E && pairs > 512)  // (the plan of up to 512 rows lists no pairs)
+  if (N % 256 == 0 && tcgen05_cluster_enabled() && pairs >= 384 * E && pairs > 512)  // (the plan of up to 512 rows lists no pairs)
     return launch_grouped_packed_bn<256, 2>(a, rows_cap, K, N, w, w_rows, w_cols, w_n, w_k, plan, epi, sms, stream);
   return launch_grouped_packed_bn<128, 1>(a, rows_cap, K, N, w, w_rows, w_cols, w_n, w_k, plan, epi, sms, stream);
 }

@@ -140,7 +140,7 @@ def test_gemm_against_cuda_core_gemm(ws):
 
 @pytest.mark.parametrize("bn", ["128", "192", "256"])
 def test_gemm_cluster_pair_matches_single_cta(ws, bn, monkeypatch):
-    """T >= 512 runs the 2-CTA cluster kernel (W tile multicast to the pair); 128-row slices of the same input run the
+    """T >= 512 runs the 2-CTA kernel (one MMA of 256 rows over both); 128-row slices of the same input run the
     single-CTA kernel.  Rows are independent and accumulate in the same k order, so the two must agree bit for bit --
     through the residual and the SiLU*mul epilogues, with a ragged last tile and an odd number of row tiles, for both tile
     widths (the launcher picks the width per shape; MB200_GEMM_BN pins it here)."""
