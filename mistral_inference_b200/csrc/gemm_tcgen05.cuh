@@ -25,6 +25,7 @@
 #include "decode_megakernel.cuh"  // mbarrier helpers with the watchdog
 #include "epilogue.cuh"
 #include "gemm_mma.cuh"
+#include "split_schedule.cuh"
 
 namespace mb200 {
 
@@ -86,6 +87,7 @@ struct TcGemmParams {
   float* partials = nullptr;   // [(cut - 1) * cut_pairs][2 CTAs][256 / 4][128 rows] float4: what the parts but the first leave for it
   unsigned* flags = nullptr;   // [(cut - 1) * cut_pairs * 2], zero between launches
 };
+constexpr unsigned CUT_GIVEN_UP = 2u;  // a flag: 0, 1 (the part is there), or this
 constexpr int TG_MAX_CUTS = 56;  // (cut - 1) * cut_pairs at most: 256 KB each
 constexpr size_t TG_CUT_BYTES = (size_t)TG_MAX_CUTS * 2 * TG_BM * 256 * sizeof(float);
 
@@ -240,6 +242,7 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
   uint64_t* tmem_empty = tmem_full + 2;     // [2]
   uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
   uint64_t* cut_full = tmem_empty + 3;  // copies of another part's sums (kCuts)
+  volatile uint32_t* cut_lost = tmem_base_slot + 1;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = CL > 1 ? (int)cluster_ctarank() : 0;
@@ -300,9 +303,9 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
     it.kb0 = 0, it.kb1 = num_k, it.part = -1, it.slot = 0;
     int t = tile, nt;
     if (kCuts && t >= whole) {
-      const int s = t - whole;
-      it.part = s / p.cut_pairs;
-      it.slot = s % p.cut_pairs;
+      const CutItem c = cut_item(t - whole, p.cut, p.cut_pairs);
+      it.part = c.part;
+      it.slot = c.slot;
       it.kb0 = num_k * it.part / p.cut;
       it.kb1 = num_k * (it.part + 1) / p.cut;
       t = whole + it.slot;
@@ -330,6 +333,7 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
       mbar_init(&tmem_empty[i], 4 * CL);  // one arrive per epilogue warp
     }
     mbar_init(cut_full, 1);
+    *cut_lost = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
     if (!GROUPED) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
@@ -431,11 +435,13 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
       const uint32_t trow = tmem_base + ((uint32_t)lane_base << 16) + acc * TG_BN;
       uint32_t va[32], vb[32];
       const int row = lane_base + lane;
+      bool lost = false;  // a part of this pair never came
       auto add_part = [&](int c, uint32_t (&v)[32]) {  // columns 32 c .. + 31 of the part that lies in the ring: quads of 128 rows side by side
         const float4* src = reinterpret_cast<const float4*>(smem) + row;
+        const float none = __uint_as_float(0x7fffffffu);
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-          const float4 x = src[(c * 8 + q) * TG_BM];
+          const float4 x = lost ? make_float4(none, none, none, none) : src[(c * 8 + q) * TG_BM];
           v[4 * q] = __float_as_uint(__uint_as_float(v[4 * q]) + x.x);
           v[4 * q + 1] = __float_as_uint(__uint_as_float(v[4 * q + 1]) + x.y);
           v[4 * q + 2] = __float_as_uint(__uint_as_float(v[4 * q + 2]) + x.z);
@@ -457,38 +463,50 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
           asm volatile("fence.proxy.async;" ::: "memory");
           __threadfence();
           asm volatile("bar.sync 2, 128;" ::: "memory");
-          if (threadIdx.x == 64) st_release_u32(p.flags + at, 1u);
+          if (threadIdx.x == 64) {
+            __threadfence();
+            if (atomicExch(p.flags + at, 1u) == CUT_GIVEN_UP) atomicExch(p.flags + at, 0u);
+          }
           tc_fence_before();
           __syncwarp();
           if (lane == 0) release(acc);
           continue;
         }
         if (w.part == 0) {
-          // The owner: the other parts run at the same time on other clusters (the launch's last items).  This CTA's ring is free (its last MMA has
-          // completed): each part's 128 KB come in by bulk copies and are added in the order of k -- all but the last into the accumulator,
-          // the last in the epilogue below.  (Loaded 128 bytes per thread and column chunk instead, a launch paid ~12 us of L2 latency here.)
+          // The owner: the other parts lie on lower clusters (cut_item).  This CTA's ring is free (its last MMA has completed): each part's 128 KB
+          // come in by bulk copies and are added in the order of k -- all but the last into the accumulator, the last in the epilogue below.
+          // (Loaded 128 bytes per thread and column chunk instead, a launch paid ~12 us of L2 latency here.)
           for (int o = 0; o < p.cut - 1; ++o) {
             if (threadIdx.x == 64) {
               const int at = (o * p.cut_pairs + w.slot) * 2 + rank;
-              unsigned spins = 0;
-              while (ld_acquire_u32(p.flags + at) == 0u) {
-                if (++spins == MB200_WATCHDOG_SPINS) {
-                  printf("[mb200 watchdog] cluster %d waits for part %d of pair %d\n", cta, o + 1, w.slot);
-                  __trap();
+              unsigned spins = 0, there = 0u;
+              while ((there = ld_acquire_u32(p.flags + at)) == 0u && ++spins < MB200_WATCHDOG_SPINS) {
+              }
+              if (there == 0u) {  // gives up: the flag says so to a part that comes after all and puts it back; the pair's results are NaN
+                there = atomicCAS(p.flags + at, 0u, CUT_GIVEN_UP);
+                __threadfence();
+              }
+              if (there == 0u) {
+                printf("[mb200 watchdog] cluster %d: part %d of pair %d never came\n", cta, o + 1, w.slot);
+                *cut_lost = 1u;
+              } else {
+                p.flags[at] = 0u;  // ready for the next launch
+                if (!lost) {
+                  asm volatile("fence.proxy.async;" ::: "memory");  // written with ordinary stores, read by the copy engine
+                  constexpr uint32_t kBytes = TG_BM * TG_BN * 4, kCopy = 32768;
+                  mbar_arrive_expect_tx(cut_full, kBytes);
+                  const uint8_t* src = reinterpret_cast<const uint8_t*>(p.partials) + (size_t)at * kBytes;
+#pragma unroll
+                  for (uint32_t i = 0; i < kBytes; i += kCopy)
+                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(smem + i)), "l"(src + i),
+                                 "r"(kCopy), "r"(smem_u32(cut_full))
+                                 : "memory");
                 }
               }
-              p.flags[at] = 0u;  // ready for the next launch
-              asm volatile("fence.proxy.async;" ::: "memory");  // written with ordinary stores, read by the copy engine
-              constexpr uint32_t kBytes = TG_BM * TG_BN * 4, kCopy = 32768;
-              mbar_arrive_expect_tx(cut_full, kBytes);
-              const uint8_t* src = reinterpret_cast<const uint8_t*>(p.partials) + (size_t)at * kBytes;
-#pragma unroll
-              for (uint32_t i = 0; i < kBytes; i += kCopy)
-                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(smem + i)), "l"(src + i), "r"(kCopy),
-                             "r"(smem_u32(cut_full))
-                             : "memory");
             }
-            __syncwarp();
+            asm volatile("bar.sync 2, 128;" ::: "memory");
+            lost = *cut_lost != 0u;
+            if (lost) continue;  // the other parts' flags still go back to zero
             mbar_wait(cut_full, o & 1, 15, o);
             if (o + 1 < p.cut - 1) {
 #pragma unroll 1
@@ -641,20 +659,15 @@ inline int tcgen05_forced_bn() {
   return e != nullptr ? atoi(e) : 0;
 }
 
-// How a dense launch of pairs (256 x 256 outputs an item, `units` pairs on the chip) ends.  Items run in rounds of `units`; when the last round is
-// at most half full, its pairs are cut along k into as many parts as fill it (at most four, eight k-blocks each): the parts' fp32 sums meet in the
-// first part's epilogue, in the order of k.
+// How a dense launch of pairs (256 x 256 outputs an item, `units` pairs on the chip) ends: cut_plan.  The parts' fp32 sums meet in the first part's
+// epilogue, in the order of k.
 inline void plan_pairs(TcGemmParams& p, int units, void* scratch, unsigned* flags) {
-  const int rest = (p.T + 2 * TG_BM - 1) / (2 * TG_BM) * (p.N / 256) % units;
   p.cut_pairs = 0;
   p.cut = 1;
-  if (scratch == nullptr || rest == 0) return;
-  int cut = units / rest;
-  if (cut > 4) cut = 4;
-  while (cut > 1 && ((cut - 1) * rest > TG_MAX_CUTS || p.K / TG_BK < 8 * cut)) --cut;
-  if (cut < 2) return;
-  p.cut = cut;
-  p.cut_pairs = rest;
+  if (scratch == nullptr) return;
+  const CutPlan c = cut_plan((long long)ceil_div(p.T, 2 * TG_BM) * (p.N / 256), p.K / TG_BK, units, TG_MAX_CUTS);
+  p.cut_pairs = c.cut_pairs;
+  p.cut = c.cut;
   p.partials = reinterpret_cast<float*>(scratch);
   p.flags = flags;
 }
@@ -667,7 +680,7 @@ inline bool pairs_fill(int64_t T, int64_t N, int64_t K, int units, bool cuts) {
   p.N = (int)N;
   p.K = (int)K;
   plan_pairs(p, units, cuts && K >= 8192 ? &p : nullptr, nullptr);  // (any scratch: how would it be cut?)
-  return 2 * ((p.T + 2 * TG_BM - 1) / (2 * TG_BM) * (p.N / 256) + (p.cut - 1) * p.cut_pairs) >= units;
+  return 2 * (ceil_div(T, 2 * TG_BM) * (p.N / 256) + (p.cut - 1) * p.cut_pairs) >= units;
 }
 
 template <int MODE, int BN>
