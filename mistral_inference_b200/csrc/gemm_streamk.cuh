@@ -6,9 +6,9 @@
 //     ~40 % and [32 x 64] ~26 %: per stage the one-thread TMA producer and the one-thread MMA issuer each spend a few hundred
 //     cycles, so a stage must carry >= 16 KB.  Tiles are therefore always 128 wide;
 //   * N / 128 tiles do not divide over 148 SMs (wo of Nemo: 40 tiles; gate/up: 224 = 1.5 rounds), so the work is cut stream-K
-//     style instead: the (tile, k-block) units of the whole problem are one sequence, and CTA c takes the c-th contiguous 1/G of
+//   * N / 128 tiles do not divide over 148 SMs: the (tile, k-block) units of the whole problem are one sequence, and CTA c takes the c-th contiguous 1/G of
 //     it -- every SM streams the same number of bytes (+- one 16 KB stage) in one pass, whatever N and K are.
-// A CTA's range covers the tail of one tile, some whole tiles and the head of another (or, when tiles are longer than ranges,
+// CTAs are counted from the launch's last block (split_schedule.cuh).  A CTA's range covers the tail of one tile, some whole tiles and the head of another (or, when tiles are longer than ranges,
 // a piece from the middle of one).  Partial tiles are reduced deterministically: a contributor that does not hold the tile's
 // first k-block writes its fp32 accumulator to its own slot of the workspace and raises its flag -- always as the FIRST segment
 // of its range; the owner of the first k-block -- always as the LAST segment of its range -- waits for the flags, sums the slots
@@ -70,7 +70,7 @@ __device__ __forceinline__ void sk_gemm_body(const CUtensorMap& map_a, const CUt
   uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int G = (int)gridDim.x, cta = (int)blockIdx.x;
+  const int G = (int)gridDim.x, cta = streamk_range((int)blockIdx.x, (int)gridDim.x);  // an owner waits for blocks that started before it
   if (GROUPED) pdl_wait();  // the routing plan (m tiles) is the preceding kernels' output
   const int num_m = GROUPED ? plan[0] : 1, num_n = p.N / SK_BN, num_k = p.K / TG_BK;
   const int32_t* tile_expert = GROUPED ? plan + MOE_PLAN_HEADER : nullptr;

@@ -43,4 +43,8 @@ MB_HD CutItem cut_item(int s, int cut, int cut_pairs) {
   return i;
 }
 
+// gemm_streamk.cuh cuts its units into one contiguous range a block; the range that holds a tile's first k-block waits for the ranges behind it.  Block
+// b takes the b-th range from the end.
+MB_HD int streamk_range(int block, int grid) { return grid - 1 - block; }
+
 }  // namespace mb200

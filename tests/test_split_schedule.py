@@ -7,6 +7,8 @@ from pathlib import Path
 
 import pytest
 
+from tests.test_streamk_protocol import SHAPES, SK_BN, TG_BK, owner_last, segments
+
 CSRC = Path(__file__).resolve().parents[1] / "mistral_inference_b200" / "csrc"
 SOURCE = """
 #include "split_schedule.cuh"
@@ -18,6 +20,7 @@ extern "C" void item(int s, int cut, int cut_pairs, int* out) {
   const mb200::CutItem i = mb200::cut_item(s, cut, cut_pairs);
   out[0] = i.part; out[1] = i.slot;
 }
+extern "C" int range(int block, int grid) { return mb200::streamk_range(block, grid); }
 """
 
 
@@ -34,7 +37,7 @@ def lib(tmp_path_factory):
         f(*a, out)
         return tuple(out)
 
-    return type("Lib", (), dict(plan=staticmethod(lambda *a: call(handle.plan, *a)), item=staticmethod(lambda *a: call(handle.item, *a))))
+    return type("Lib", (), dict(plan=staticmethod(lambda *a: call(handle.plan, *a)), item=staticmethod(lambda *a: call(handle.item, *a)), range=staticmethod(handle.range)))
 
 
 def run_blocks(steps, resident, r):
@@ -77,3 +80,25 @@ def test_owners_of_cut_pairs_wait_for_earlier_clusters_only(lib, units):
         for resident in (1, 2, units // 2, units):
             run_blocks(steps, max(resident, 1), r)
     assert seen >= ({2, 3, 4} if units > 5 else {2})
+
+
+@pytest.mark.parametrize("G", [148, 37, 3])
+def test_streamk_owners_wait_for_earlier_blocks_only(lib, G):
+    """The ranges and roles are those of test_streamk_protocol; here their blocks start one after the other."""
+    r = random.Random(G)
+    for N, K in SHAPES[::4]:
+        num_k = K // TG_BK
+        total = N // SK_BN * num_k
+        grid = min(G, total)
+        steps = []
+        for block in range(grid):
+            c, mine = lib.range(block, grid), []
+            for tile, kb0, kb1 in segments(total, num_k, grid, c):
+                if kb0 != 0:
+                    mine.append(("post", c))
+                elif kb1 != num_k:
+                    mine += [("wait", o) for o in range(c + 1, owner_last(total, num_k, grid, c, tile) + 1)]
+            steps.append(mine)
+        assert sorted(lib.range(b, grid) for b in range(grid)) == list(range(grid))
+        for resident in (1, grid // 2 + 1, grid):
+            run_blocks(steps, resident, r)
