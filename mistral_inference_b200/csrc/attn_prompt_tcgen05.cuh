@@ -14,8 +14,10 @@
 //             maximum and sum stay in the thread.  O is rescaled only when a maximum grew by more than 2^8 (P stays far inside bf16's range)
 // TMEM columns: S_0 / P_0 at 0, S_1 / P_1 at 128, O_0 at 256, O_1 at 384.
 //
-// Key tiles are laid from the END of a run backwards: rows before the run are older tokens or, below row 0, zeros of the copy engine.  A
-// tile laid forwards would read ring rows that nothing has written yet, and 0 x NaN is not 0.
+// Key tiles are laid from the END of a run backwards: rows before the run are older tokens, another sequence's rows (own rows) or, below row 0,
+// zeros of the copy engine.  A tile laid forwards would read ring rows that nothing has written yet.  The mask makes the weights of rows before the
+// run 0, but 0 x NaN is not 0: on a run's first tile (three at most per CTA) the softmax warps of head 0 overwrite those rows of V with zeros, so
+// that a sequence's infinities stay its own and tokens before a tile's window do not count at all.
 //
 // One head per CTA, two S buffers, two threads per row (before): 191 us a layer at T = 4096, 32 / 8 heads; portions of prompts and the
 // layered decoders went through mma.sync kernels: 520 us for 3 x ~650 queries over ~2900 keys, 1997 us for 4096 queries with a bias.
@@ -336,6 +338,16 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
                      : "memory");
       }
       l_run += (l4[0] + l4[1]) + (l4[2] + l4[3]);
+      if (pos0 < run_lo && u == 0) {  // (a row's 128 bytes of each box keep their place under the swizzle)
+        const int it = 2 * t + 1, s = it % FA_SLOTS, bytes = (run_lo - pos0) * 128;
+        mbar_wait(&kv_full[s], (it / FA_SLOTS) & 1, 29, t);
+        uint8_t* const v = sKV + s * FA_TILE_BYTES;
+        for (int i = r * 16; i < bytes; i += FA_BM * 16) {
+          *reinterpret_cast<uint4*>(v + i) = make_uint4(0, 0, 0, 0);
+          *reinterpret_cast<uint4*>(v + FA_TILE_BYTES / 2 + i) = make_uint4(0, 0, 0, 0);
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      }
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();

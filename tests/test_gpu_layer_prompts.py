@@ -155,6 +155,39 @@ def test_prompt_attention_over_ring_and_own_rows(H, KV, lens, past, W):
     assert rel(out, torch.cat(ref)) < 2 ** -8
 
 
+@pytest.mark.parametrize("H,KV", [(4, 2), (3, 1)])
+@pytest.mark.parametrize("lens,past,W,bad", [([100, 60, 20], [9, 7, 30], 200, 0), ([100, 60, 130], [0, 0, 0], 300, 1), ([129, 255], [0, 0], 64, 0), ([40], [500], 64, None),
+                                             ([140, 33], [77, 300], 128, None)])
+def test_prompt_attention_keeps_bad_values_where_they_are(H, KV, lens, past, W, bad):
+    """NaN and infinity in one sequence's own keys and values (`bad`), or in ring rows that have left every query's window (None), reach no other
+    token: the others' outputs are the bits that finite values there give."""
+    from mistral_inference_b200 import _abi
+
+    g = torch.Generator().manual_seed(sum(lens) + W)
+    B, T, hd = len(lens), sum(lens), 128
+    rnd = lambda *s: torch.randn(*s, generator=g).bfloat16().to(DEV)  # noqa: E731
+    q, k, v, ring_k, ring_v = rnd(T, H, hd), rnd(T, KV, hd), rnd(T, KV, hd), rnd(B, W, KV, hd), rnd(B, W, KV, hd)
+    q_start = torch.tensor([0] + lens).cumsum(0).int().to(DEV)
+    outs = []
+    for spoil in (False, True):
+        k1, v1, rk, rv = k.clone(), v.clone(), ring_k.clone(), ring_v.clone()
+        if spoil and bad is not None:
+            a, z = int(q_start[bad]), int(q_start[bad + 1])
+            v1[a:z], k1[a:z:2] = float("nan"), float("inf")
+        elif spoil:
+            for b, m in enumerate(past):
+                if m >= W:  # position m - W: the oldest row; the first query, m, sees m - W + 1 and later ones
+                    rk[b, (m - W) % W], rv[b, (m - W) % W] = float("inf"), float("nan")
+        out = torch.empty(T, H * hd, dtype=torch.bfloat16, device=DEV)
+        _abi.attn_prefill(q, k1, v1, rk, rv, q_start, torch.tensor(past, dtype=torch.int32, device=DEV), out, B, max(lens), W, H, KV, hd, causal=True,
+                          first_prefill=max(past) == 0)
+        outs.append(out)
+    for b in range(B):
+        if b != bad:
+            a, z = int(q_start[b]), int(q_start[b + 1])
+            assert torch.isfinite(outs[1][a:z]).all() and torch.equal(outs[0][a:z], outs[1][a:z]), b
+
+
 @pytest.mark.parametrize("n_tab", [0, 1, 40, 500])
 @pytest.mark.parametrize("lens,past", [([64], [0]), ([130, 33], [0, 0]), ([250, 1], [300, 5]), ([128, 128], [128, 1])])
 def test_prompt_attention_with_a_bias_over_the_ring(n_tab, lens, past):
