@@ -164,6 +164,10 @@ __device__ __forceinline__ void epi_logprob32(const EpiParams& p, int t, int n, 
     }
     s = s * expf(m - mx) + (a0 + a1);
     m = mx;
+  } else {  // nothing but -infinity adds nothing; a NaN, which fmaxf passes over, counts
+#pragma unroll
+    for (int j = 0; j < 32; ++j)
+      if (y[j] != y[j]) s = y[j];
   }
   if (tgt >= n && tgt < n + 32) {
     float x = 0.f;

@@ -299,6 +299,29 @@ def test_scoring_without_written_logits(lens, monkeypatch):
         assert (a - ref).abs().max() <= 1e-5 * ref.abs().max() + 2 * step
 
 
+@pytest.mark.parametrize("T", [128, 200, 700])
+@pytest.mark.parametrize("cols", [(64, 96), (96, 128), (0, 64), (639, 640), (5, 6), (0, 640)])
+@pytest.mark.parametrize("value", ["nan", "-inf"])
+def test_scoring_counts_logits_that_are_no_numbers(T, cols, value):
+    """Whole groups of NaN logits make the row's log-probability NaN, groups of -infinity add nothing, as in the pass over written logits."""
+    from mistral_inference_b200 import _abi
+
+    g = torch.Generator(device=DEV).manual_seed(T)
+    D, V = 128, 640
+    x, w = torch.rand(T, D, device=DEV, generator=g).bfloat16() + 0.5, (torch.randn(V, D, device=DEV, generator=g) / 8).bfloat16()
+    w[cols[0]:cols[1]] = float(value)  # x is positive: the logits are NaN or -infinity
+    nw, targets = torch.ones(D, device=DEV, dtype=torch.bfloat16), torch.randint(0, V, (T,), device=DEV, generator=g)
+    ws = _abi.Workspace(_abi.workspace_bytes(T, D, 1, 1, 128, 256, V, 1), DEV)
+    logits, ref, got = torch.empty(T, V, device=DEV), torch.zeros(T, device=DEV), torch.zeros(T, device=DEV)
+    _abi.lm_head(x, nw, w, logits, 1e-5, ws)
+    _abi.logprob_gather(logits, targets, out=ref)
+    _abi.lm_head_logprobs(x, nw, w, targets, torch.full((T,), -1, dtype=torch.int32, device=DEV), torch.empty(1, V, device=DEV), got, 1e-5, ws)
+    assert (torch.isnan(ref).all() if value == "nan" or cols == (0, V) else torch.isfinite(ref[(targets < cols[0]) | (targets >= cols[1])]).all())
+    assert torch.equal(torch.isnan(got), torch.isnan(ref)) and torch.equal(torch.isinf(got), torch.isinf(ref))
+    ok, step = torch.isfinite(ref), logits[torch.isfinite(logits)].abs().max().item() * 2 ** -7 if torch.isfinite(logits).any() else 0.0
+    assert (got - ref)[ok].abs().max() <= 1e-5 * 10 + (2 * step if T == 128 else 0.0) if ok.any() else True
+
+
 @pytest.mark.parametrize("T", [17, 32, 33, 64, 65, 127, 128, 171, 600])
 @pytest.mark.parametrize("N,K", [(256, 128), (4096, 8192)])
 def test_prompt_linear_steps_by_rows(T, N, K):
