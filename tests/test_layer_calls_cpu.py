@@ -1,0 +1,46 @@
+"""What the Python entry points of the prompt kernels refuse before anything is launched."""
+import pytest
+import torch
+
+from mistral_inference_b200 import _abi, _abi_hybrid as h
+
+
+@pytest.mark.parametrize("table", [torch.zeros(9, 4, dtype=torch.bfloat16), torch.zeros(4, 9), torch.zeros(36)])
+@pytest.mark.parametrize("longest", [1, 200])
+def test_bias_tables_of_another_layout_are_refused(table, longest, monkeypatch):
+    monkeypatch.setattr(_abi, "layer_attention", lambda *a: pytest.fail("launched"))
+    q, ring = torch.zeros(200, 4 * 128, dtype=torch.bfloat16), torch.zeros(1, 300, 2, 128, dtype=torch.bfloat16)
+    i = torch.zeros(2, dtype=torch.int32)
+    with pytest.raises(AssertionError, match="bias table"):
+        h.attn_bias(q, ring, ring, table, i, i, i, q, 1, 300, 4, 2, 128, 128, 0.1, n_tiles=4, seqpos=i, longest=longest)
+    with pytest.raises(AssertionError, match="bias table"):
+        h.attn_bias_decode(q[:1], ring, ring, table, i, i, q, 1, 300, 4, 2, 128, 128, 0.1)
+
+
+@pytest.mark.parametrize("what", ["idx", "rows", "w13", "w2", "add"])
+def test_mixtures_of_other_shapes_are_refused(what, monkeypatch):
+    monkeypatch.setattr(_abi, "layer_moe", lambda *a: pytest.fail("launched"))
+    T, D, E, ff, bf = 40, 256, 3, 128, torch.bfloat16
+    x, w13, w2, add = torch.zeros(T, D, dtype=bf), torch.zeros(E * 2 * ff, D, dtype=bf), torch.zeros(D, E * ff, dtype=bf), torch.zeros(T, D)
+    idx, wsel = torch.zeros(T, 2, dtype=torch.int32), torch.zeros(T, 2)
+    if what == "idx":
+        idx = idx.long()
+    elif what == "rows":
+        idx, wsel = idx[1:], wsel[1:]
+    elif what == "w13":
+        w13 = w13[:, : D // 2]
+    elif what == "w2":
+        w2 = w2[:, ff:]
+    else:
+        add = add.to(bf)
+    with pytest.raises(AssertionError, match="choices|experts' weights|add_to"):
+        h.moe_grouped(x, w13, w2, idx, wsel, E, ff, h.EPI_SWIGLU, add_to=add)
+
+
+@pytest.mark.parametrize("what", ["target", "keep", "out"])
+def test_scoring_takes_one_target_a_token(what):
+    T, V, bf = 130, 128, torch.bfloat16
+    target, keep, out = torch.zeros(T, dtype=torch.long), torch.zeros(T, dtype=torch.int32), torch.zeros(T)
+    target, keep, out = (t[1:] if what == n else t for t, n in ((target, "target"), (keep, "keep"), (out, "out")))
+    with pytest.raises(AssertionError, match="targets and kept rows|results"):
+        _abi.lm_head_logprobs(torch.zeros(T, 64, dtype=bf), torch.ones(64, dtype=bf), torch.zeros(V, 64, dtype=bf), target, keep, torch.zeros(1, V), out, 1e-5, None)
