@@ -235,7 +235,8 @@ def lm_head_logprobs(x, norm_w, w_out, target, keep_row, kept_logits, out, eps, 
     """out[t] = log_softmax(head(norm(x)))[t, target[t]] where target[t] >= 0; rows with keep_row[t] >= 0 leave their logits in kept_logits."""
     T, dim = x.shape
     V = w_out.shape[0]
-    assert target.dtype == torch.long and keep_row.dtype == torch.int32 and kept_logits.dtype == torch.float32 and kept_logits.shape[1] == V and out.dtype == torch.float32
+    assert target.dtype == torch.long and target.shape == (T,) and keep_row.dtype == torch.int32 and keep_row.shape == (T,), "targets and kept rows: one a token"
+    assert kept_logits.dtype == torch.float32 and kept_logits.shape[1] == V and out.dtype == torch.float32 and out.shape == (T,), "results"
     partial = torch.empty(T * (V // 64) * 2, dtype=torch.float32, device=x.device)
     target_logit = torch.empty(T, dtype=torch.float32, device=x.device)
     _check(lib().mb200_lm_head_logprobs(_ptr(x), _ptr(norm_w), _ptr(w_out), _ptr(target), _ptr(keep_row), _ptr(kept_logits), _ptr(out), _ptr(partial),

@@ -206,16 +206,20 @@ def attn_prep(qkv, qnorm, knorm, positions, cache_rows, q_out, cache_k, cache_v,
 ATTN_TCGEN05_MIN = 16  # prompts (portions) at least this long take the tcgen05 kernel (128-query tiles) where the sizes allow
 
 
+def _check_bias_table(bias_tab: Optional[torch.Tensor], H: int) -> None:
+    assert bias_tab is None or (bias_tab.dtype == torch.float32 and bias_tab.dim() == 2 and bias_tab.shape[1] == H), "bias table: fp32 [distances, heads]"
+
+
 def attn_bias(q, cache_k, cache_v, bias_tab, positions, q_start, slots, out, B: int, W: int, H: int, G: int, d: int, e: int, scale: float,
               n_tiles: int = 0, splits: int = 1, seqpos=None, longest: int = 0) -> None:
     """n_tiles = sum over sequences of ceil(len / 64) selects a tensor-core prompt kernel (bf16); 0 the exact fp32 one.  With seqpos (tokens
     before this call, per sequence) and the longest sequence's length, heads of 128 take the main library's tcgen05 kernel where it is built."""
+    _check_bias_table(bias_tab, H)
     if (n_tiles and seqpos is not None and longest >= ATTN_TCGEN05_MIN and d == e == 128 and q.dtype == torch.bfloat16 and scale > 0 and _aligned(q, cache_k, cache_v, out)
             and cache_k.shape[1] == W and os.environ.get("MB200_HYBRID_GEMM", "1") != "0" and _abi.library_path().exists()
             and (bias_tab is None or bias_tab.shape[0] <= _abi.lib().mb200_layer_attention_max_table())):
         _abi.layer_attention(q, cache_k, cache_v, bias_tab, q_start, seqpos, slots, out, B, longest, H, G, scale)
         return
-    assert bias_tab is None or (bias_tab.dtype == torch.float32 and bias_tab.shape[1] == H)
     scratch = torch.empty(q.shape[0] * H * splits * (2 + e), dtype=torch.float32, device=q.device) if splits > 1 and n_tiles == 0 else None
     _check(lib().mbh_attn_bias(_ptr(q), _ptr(cache_k), _ptr(cache_v), _ptr(bias_tab), bias_tab.shape[0] if bias_tab is not None else 0, _ptr(positions), _ptr(q_start), _ptr(slots),
                                _ptr(out), q.shape[0], B, W, H, G, d, e, scale, n_tiles, splits, _ptr(scratch), dt_of(q.dtype), _stream()), "mbh_attn_bias")
@@ -337,7 +341,11 @@ def moe_grouped(h: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, idx: torch
                 limit: float = 0.0, alpha: float = 0.0, add_to: Optional[torch.Tensor] = None) -> torch.Tensor:
     """fp32 [T, width]: the weighted sum of each token's chosen experts (indices >= E: none); added to add_to (fp32) when given.  epi: the
     unit between the two Linears (EPI_SWIGLU, EPI_GLU with the weight on the expert's input, EPI_GEGLU, EPI_RELU2)."""
-    assert idx.dtype == torch.int32 and wsel.dtype == torch.float32 and idx.shape == wsel.shape
+    T, D = h.shape
+    units = w13.shape[0] // E
+    assert idx.dtype == torch.int32 and wsel.dtype == torch.float32 and idx.shape == wsel.shape and idx.shape[0] == T, "choices: int32 and fp32 [tokens, top]"
+    assert w13.dtype == w2.dtype == h.dtype and w13.shape == (units * E, D) and w2.shape == (D, E * ff) and units == (ff if epi == EPI_RELU2 else 2 * ff), "experts' weights"
+    assert add_to is None or (add_to.dtype == torch.float32 and add_to.shape == (T, D)), "add_to: fp32 [tokens, width]"
     y32 = torch.empty(h.shape, dtype=torch.float32, device=h.device) if add_to is None else add_to
     _abi.layer_moe(h, w13, w2, idx, wsel, E, ff, epi, limit, alpha, y32, add_to is not None)
     return y32
@@ -532,6 +540,7 @@ def attn_bias_decode_ok(q: torch.Tensor, cache_k: torch.Tensor, cache_v: torch.T
 
 def attn_bias_decode(q, cache_k, cache_v, bias_tab, positions, slots, out, B: int, W: int, H: int, G: int, d: int, e: int, scale: float) -> None:
     """`attn_bias` for one token per sequence on tensor cores (attn_bias_decode_ok says when)."""
+    _check_bias_table(bias_tab, H)
     splits = attn_decode_splits(B, G, W)
     scratch = torch.empty(B * H * splits * (2 + e), dtype=torch.float32, device=q.device)
     _check(lib().mbh_attn_bias_decode(_ptr(q), _ptr(cache_k), _ptr(cache_v), _ptr(bias_tab), bias_tab.shape[0], _ptr(positions), _ptr(slots), _ptr(out), B, W, H, G, d, e,
