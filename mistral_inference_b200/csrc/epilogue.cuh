@@ -4,6 +4,7 @@
 // and the packed gate/up weight puts w1[i], w3[i] on rows 2i, 2i+1.
 #pragma once
 #include "common.cuh"
+#include "sigmoid.cuh"
 
 namespace mb200 {
 
@@ -181,18 +182,19 @@ __device__ __forceinline__ void epi_logprob32(const EpiParams& p, int t, int n, 
 // choice is made once per 32 columns, never inside a loop over them: with the branches inside, the chains of exponential and
 // reciprocal ran one after the other and a tile's epilogue took longer than its MMAs (gate/up of 4096 x 28672 x 4096: 1015 us against
 // 642 us for the plain store).  The Linear's sum (+ bias) is rounded to bf16 once before the step, except for fp32 results.
-//
-// sigmoid(x) with one ex2.approx and one rcp.approx: the argument's product with log2(e) is carried in two parts, so the relative error
-// stays at a few 2^-23 for every x (expf and a rounded division give the same).  A NaN argument gives a number: callers multiply by x.
 __device__ __forceinline__ float layer_sigmoid(float x) {
-  const float z = fminf(fmaxf(x, -120.f), 120.f);
-  const float hi = z * -1.4426950408889634f, lo = fmaf(z, -1.4426950408889634f, -hi);
-  float e, r;
-  asm("ex2.approx.f32 %0, %1;" : "=f"(e) : "f"(hi));
-  e = fmaf(e, lo * 0.6931471805599453f, e);
-  if (hi > 127.f) e = INFINITY;  // (infinity times a zero or negative lo must not turn into something else)
-  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(1.f + e));
-  return r;
+  return sigmoid_by(
+      x,
+      [](float v) {
+        float r;
+        asm("ex2.approx.f32 %0, %1;" : "=f"(r) : "f"(v));
+        return r;
+      },
+      [](float v) {
+        float r;
+        asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(v));
+        return r;
+      });
 }
 __device__ __forceinline__ float layer_gelu(float z) { return 0.5f * z * (1.f + tanhf(0.7978845608028654f * fmaf(0.044715f * z * z, z, z))); }
 
