@@ -2,7 +2,8 @@
 //
 // Every kernel of this library is a template over the storage type of activations and weights (bf16 or fp32) and does
 // its arithmetic in fp32.  The residual stream, softmax, norms and recurrent state are fp32 in both modes; in fp32 mode
-// nothing is rounded below 32 bits (FMAs, or tensor-core products of three bf16 parts that add up to the fp32 number; no TF32).
+// nothing is rounded below 32 bits (FMAs, or tensor-core products of three bf16 parts that add up to the fp32 number, less than 2^-26 of a
+// product left out; no TF32).
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>

@@ -19,7 +19,7 @@
 // In bf16 mode the Linear's own output is rounded to bf16 before the epilogue's arithmetic (the rounding point of a bf16
 // Linear); accumulation is fp32 in both modes.
 //
-// Kernels: `linear_tiled_mma` (bf16) and `linear_f32_parts` (fp32, hybrid_linear_f32.cuh) for prompts, any shape; `linear_skinny` (M <= 8 rows, FMA,
+// Kernels: `linear_tiled_mma` (bf16), `linear_f32_parts` (fp32, hybrid_linear_f32.cuh) and `linear_tiled_fma` (fp32, K < 16) for prompts, any shape; `linear_skinny` (M <= 8 rows, FMA,
 // one warp per pair of weight rows) and `linear_skinny_mma` (bf16, up to 16 rows, tensor cores) for decode: every weight byte is read
 // once with 16-byte loads; `linear_decay_mma` for decays from a low rank; `linear_epilogue8_kernel` (bf16, eight columns per thread) and
 // `linear_epilogue_kernel` apply the epilogues to the output of another GEMM (the main library's
@@ -106,6 +106,51 @@ __device__ __forceinline__ void epilogue_pair(const LinearArgs& a, int m, int n,
         o[0] = v0;
         if (has1) o[1] = v1;
         break; }
+    }
+}
+
+// ------------------------------------------------------------------------------------------------ tiled, FMA (fp32, short rows)
+constexpr int LT_BM = 64, LT_BN = 64, LT_BK = 16, LT_THREADS = 256;
+
+__global__ void __launch_bounds__(LT_THREADS) linear_tiled_fma(LinearArgs a) {
+    __shared__ float As[LT_BK][LT_BM + 4];
+    __shared__ float Ws[LT_BK][LT_BN + 4];
+    const float* X = static_cast<const float*>(a.x);
+    const float* W = static_cast<const float*>(a.w);
+    const int m0 = blockIdx.y * LT_BM, n0 = blockIdx.x * LT_BN;
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    float acc[4][4] = {};
+    const int lr = tid >> 2, lc = (tid & 3) * 4;  // loader: row lr of the tile, 4 consecutive k
+    for (int k0 = 0; k0 < a.K; k0 += LT_BK) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            int k = k0 + lc + i;
+            int m = m0 + lr, n = n0 + lr;
+            As[lc + i][lr] = (m < a.M && k < a.K) ? X[(size_t)m * a.x_pitch() + k] : 0.f;
+            Ws[lc + i][lr] = (n < a.N && k < a.K) ? W[(size_t)n * a.K + k] : 0.f;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < LT_BK; ++k) {
+            float av[4], wv[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) { av[i] = As[k][ty * 4 + i]; wv[i] = Ws[k][tx * 4 + i]; }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], wv[j], acc[i][j]);
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        int m = m0 + ty * 4 + i;
+        if (m >= a.M) continue;
+#pragma unroll
+        for (int j = 0; j < 4; j += 2) {
+            int n = n0 + tx * 4 + j;
+            if (n < a.N) epilogue_pair<float>(a, m, n, acc[i][j], acc[i][j + 1], n + 1 < a.N);
+        }
     }
 }
 
@@ -534,6 +579,8 @@ inline cudaError_t launch_linear(const LinearArgs& a, cudaStream_t st) {
     } else if constexpr (sizeof(T) == 2) {
         dim3 grid((a.N + MM_BN - 1) / MM_BN, (a.M + MM_BM - 1) / MM_BM);
         linear_tiled_mma<<<grid, MM_THREADS, 0, st>>>(a);
+    } else if (a.K < FT_MIN_K) {
+        linear_tiled_fma<<<dim3((a.N + LT_BN - 1) / LT_BN, (a.M + LT_BM - 1) / LT_BM), LT_THREADS, 0, st>>>(a);
     } else {
         return launch_linear_f32_parts(a, st);
     }

@@ -1,10 +1,16 @@
 // fp32 Linears of prompts on the tensor cores (tcgen05): y = x W^T with every fp32 operand as three bf16 parts.
 //
-// An fp32 number is hi + mid + lo exactly (8 significant bits each, truncated), and x w = sum of nine part products, of which the six
-// largest are formed: hi hi, hi mid, mid hi, hi lo, lo hi, mid mid; the other three are below 2^-21 of x w.  Products of bf16 numbers are
-// exact in the tensor core; what it loses is in its running sum, so (a) the small products of a k-block are summed first and the four
-// hi hi instructions last, and (b) the accumulator starts anew for every 64 columns of k and is added to fp32 registers with ordinary
-// rounded additions.  Measured against float64 (2048 .. 8192 columns) the error is below that of the FMA chain it replaces.
+// An fp32 number is hi + mid / 2^8 + lo / 2^16 exactly: hi the nearest bf16, mid the nearest to 2^8 times what is left, lo 2^8 times the rest of that (at
+// most 8 significant bits; the powers of two keep the parts of small numbers above bf16's smallest, down to 2^-126; of fp32's subnormal numbers hi has fewer bits, and a
+// product of one is right to 2^-20).  x w is the sum of nine part
+// products, of which the six largest are formed; the other three are below 2^-26 of x w, of either sign.  Products of bf16 numbers are exact in
+// the tensor core; what it loses is in its running sum, so (a) the small products of a k-block are summed first, at their own scale -- the
+// accumulator is divided by 2^8 where the next larger ones start -- and the four hi hi instructions last, and (b) the accumulator starts anew for
+// every 64 columns of k and is added to fp32 registers with ordinary rounded additions.
+// Error against float64 in units of 2^-24 (2-norm; operands normal, then in 1 .. 2), here and by a chain of FMAs: K = 8 0.78 / 0.92, 0.96 / 0.79;
+// 16 0.81 / 1.28, 1.00 / 1.04; 64 1.3 / 2.4, 1.0 / 2.0; 2048 1.7 / 13.5, 1.2 / 11.4 (the same with operands of 2^-118).  Below FT_MIN_K columns the chain is the
+// more exact one for operands of one sign and keeps the job (linear_tiled_fma).  With truncated parts and without the scales, as this began: 1.6 at any K,
+// 7.8 for x = w = 1 + 2^-7 - 2^-23 and 300 at 2^-118.
 //
 // What bounds it: shared memory.  128 x 128 x 16 instructions read 8 KB per 64 cycles, all that the SM has, and the parts are written through
 // it too: about 0.6 of the tensor rate, a sixth of which counts.  The 64 x 64 FMA tiles it replaces (24 TFLOP/s of 74): 8870 us of Linears for
@@ -14,13 +20,14 @@
 // rank order, so a small problem fills the chip and the result is the same every time).  17 warps: sixteen load fp32 from global memory
 // (one k-block ahead, in registers), split, write the six part tiles (128B-swizzled, K-major) of a stage and add the block before to
 // their registers; one thread of the last issues the MMAs (with eight workers the loads' latency was in the open: 3530 us of Linears against 1870).  Two stages: the MMAs of a block run under the splitting of the next.
-// An infinity or a NaN in the operands of a tile: its outputs are computed again with FMAs (inf x 0 parts would give NaN).
+// An infinity or a NaN in the operands of a tile, or a number from 2^120 on (256 x is formed): its outputs are computed again with FMAs (ft_fma_rows).
 #pragma once
 #include "hybrid_linear.cuh"
 
 namespace mbh {
 
 constexpr int FT_BM = 128, FT_BN = 128, FT_BK = 64, FT_WARPS = 16 /* workers */, FT_THREADS = 32 * (FT_WARPS + 1), FT_TILE = 128 * 64 * 2;  // a part tile: 128 rows of 128 bytes
+constexpr int FT_MIN_K = 16;
 constexpr int FT_STAGE = 6 * FT_TILE, FT_SMEM = 2 * FT_STAGE + 1024, FT_LD = FT_BN + 4;
 static_assert(FT_BM * FT_LD * 4 <= 2 * FT_STAGE, "the sums of a tile fit in the stages");
 
@@ -41,24 +48,50 @@ __device__ __forceinline__ uint64_t ft_desc(uint32_t addr) {
     return (uint64_t)((addr & 0x3ffff) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
 constexpr uint32_t FT_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(FT_BN >> 3) << 17) | ((uint32_t)(FT_BM >> 4) << 24);  // bf16 x bf16 -> fp32
+// D = A B (accumulate 0) or A B + D / 2^DOWN
+template <int DOWN>
 __device__ __forceinline__ void ft_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t accumulate) {
-    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d), "l"(a), "l"(b), "r"(FT_IDESC), "r"(accumulate) : "memory");
+    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p, %5;\n}\n" ::"r"(d), "l"(a), "l"(b), "r"(FT_IDESC), "r"(accumulate),
+                 "n"(DOWN)
+                 : "memory");
 }
 __device__ __forceinline__ void ft_commit(uint64_t* b) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(ft_smem(b)) : "memory");
 }
 __device__ __forceinline__ void ft_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void ft_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void ft_ld32(uint32_t addr, float (&v)[32]) {
+__device__ __forceinline__ void ft_ld16(uint32_t addr, float (&v)[16]) {
     uint32_t* u = reinterpret_cast<uint32_t*>(v);
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, "
-        "%27, %28, %29, %30, %31}, [%32];"
-        : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]), "=r"(u[8]), "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]),
-          "=r"(u[13]), "=r"(u[14]), "=r"(u[15]), "=r"(u[16]), "=r"(u[17]), "=r"(u[18]), "=r"(u[19]), "=r"(u[20]), "=r"(u[21]), "=r"(u[22]), "=r"(u[23]), "=r"(u[24]),
-          "=r"(u[25]), "=r"(u[26]), "=r"(u[27]), "=r"(u[28]), "=r"(u[29]), "=r"(u[30]), "=r"(u[31])
-        : "r"(addr));
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]), "=r"(u[8]), "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]),
+                   "=r"(u[13]), "=r"(u[14]), "=r"(u[15])
+                 : "r"(addr));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+// two numbers to the nearest bf16, and back
+__device__ __forceinline__ uint32_t ft_pack(float x, float y) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(y), "f"(x));
+    return r;
+}
+// pairs of fp32 numbers in a 64-bit register
+__device__ __forceinline__ uint64_t ft_two(float x, float y) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ float ft_first(uint64_t v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float ft_second(uint64_t v) { return __uint_as_float((uint32_t)(v >> 32)); }
+__device__ __forceinline__ uint64_t ft_unpack(uint32_t u) { return ft_two(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u)); }
+__device__ __forceinline__ uint64_t ft_mul2(uint64_t v, float f) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(v), "l"(ft_two(f, f)));
+    return r;
+}
+__device__ __forceinline__ uint64_t ft_fma2(uint64_t v, float f, uint64_t add) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(v), "l"(ft_two(f, f)), "l"(add));
+    return r;
 }
 __device__ __forceinline__ float ft_ld_cluster(uint32_t addr, uint32_t rank) {
     uint32_t remote;
@@ -70,6 +103,59 @@ __device__ __forceinline__ float ft_ld_cluster(uint32_t addr, uint32_t rank) {
 __device__ __forceinline__ void ft_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// `share` rows of a tile from row `first` on (a multiple of 16, at most 128) with FMAs in the order of k, through shared memory (the stages: the parts are not needed
+// any more).  A thread takes four columns of every 16th row.  About the time the whole tile takes with FMAs, once per tile that holds an infinity or a NaN.
+template <bool VEC>
+__device__ __noinline__ void ft_fma_rows(const LinearArgs& a, const float* X, const float* W, float* sm, int m0, int n0, int first, int share, int rows, int cols) {
+    constexpr int KB = 64, XP = KB + 4, WP = FT_BN + 4;
+    float *xs = sm, *ws = sm + FT_BM * XP;  // [share][XP], [KB][WP]
+    static_assert((FT_BM * XP + KB * WP) * 4 <= 2 * FT_STAGE, "both blocks fit in the stages");
+    const int tid = threadIdx.x, c4 = (tid & 31) * 4, r0 = tid >> 5, nr = share / 16;
+    float acc[8][4];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+    for (int k0 = 0; k0 < a.K; k0 += KB) {
+        __syncthreads();
+        for (int i = tid; i < (share + FT_BN) * (KB / 4); i += FT_THREADS) {
+            const int r = i / (KB / 4), kc = (i % (KB / 4)) * 4, k = k0 + kc, n = r - share;
+            const bool is_x = r < share, ok = is_x ? first + r < rows : n < cols;
+            const float* src = is_x ? X + (size_t)(first + r) * a.x_pitch() + k : W + (size_t)n * a.K + k;
+            float v[4];
+            if (VEC) {
+                const float4 u = ok && k < a.K ? *reinterpret_cast<const float4*>(src) : make_float4(0.f, 0.f, 0.f, 0.f);
+                v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w;
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) v[e] = ok && k + e < a.K ? src[e] : 0.f;
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) (is_x ? xs[r * XP + kc + e] : ws[(kc + e) * WP + n]) = v[e];
+        }
+        __syncthreads();
+        if (tid < 512)
+#pragma unroll 4
+            for (int k = 0; k < KB; ++k) {
+                const float4 w = *reinterpret_cast<const float4*>(ws + k * WP + c4);
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    if (i < nr) {
+                        const float x = xs[(r0 + 16 * i) * XP + k];
+                        acc[i][0] = fmaf(x, w.x, acc[i][0]); acc[i][1] = fmaf(x, w.y, acc[i][1]);
+                        acc[i][2] = fmaf(x, w.z, acc[i][2]); acc[i][3] = fmaf(x, w.w, acc[i][3]);
+                    }
+            }
+    }
+    if (tid >= 512) return;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int r = first + r0 + 16 * i;
+        if (i >= nr || r >= rows) continue;
+#pragma unroll
+        for (int j = 0; j < 4; j += 2)
+            if (c4 + j < cols) epilogue_pair<float>(a, m0 + r, n0 + c4 + j, acc[i][j], acc[i][j + 1], n0 + c4 + j + 1 < a.N);
+    }
 }
 
 template <bool VEC>
@@ -142,14 +228,15 @@ __global__ void __launch_bounds__(FT_THREADS, 1) linear_f32_parts(LinearArgs a, 
             uint32_t part[3][2];
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-                const float x = f[2 * e], y = f[2 * e + 1];
-                const uint32_t ux = __float_as_uint(x), uy = __float_as_uint(y);
-                const float rx = x - __uint_as_float(ux & 0xffff0000u), ry = y - __uint_as_float(uy & 0xffff0000u);
-                const uint32_t mx = __float_as_uint(rx), my = __float_as_uint(ry);
-                const uint32_t lx = __float_as_uint(rx - __uint_as_float(mx & 0xffff0000u)), ly = __float_as_uint(ry - __uint_as_float(my & 0xffff0000u));
-                part[0][e] = __byte_perm(ux, uy, 0x7632);
-                part[1][e] = __byte_perm(mx, my, 0x7632);
-                part[2][e] = __byte_perm(lx, ly, 0x7632);  // at most 8 significant bits are left: exact
+                // every subtraction is exact; 256 x first, so that both steps of a part are one instruction for two numbers
+                const uint64_t v8 = ft_mul2(ft_two(f[2 * e], f[2 * e + 1]), 256.f);
+                const uint32_t h = ft_pack(f[2 * e], f[2 * e + 1]);
+                const uint64_t r1 = ft_fma2(ft_unpack(h), -256.f, v8);
+                const uint32_t m = ft_pack(ft_first(r1), ft_second(r1));
+                const uint64_t r2 = ft_fma2(ft_unpack(m), -256.f, ft_mul2(r1, 256.f));
+                part[0][e] = h;
+                part[1][e] = m;
+                part[2][e] = __byte_perm(__float_as_uint(ft_first(r2)), __float_as_uint(ft_second(r2)), 0x7632);  // at most 8 significant bits are left: exact
             }
             unsigned char* at = tile + r * 128 + (((c4 * 2) ^ ((r & 7) << 4)) & 0x7f);  // 16-byte units XORed with the row
 #pragma unroll
@@ -163,12 +250,12 @@ __global__ void __launch_bounds__(FT_THREADS, 1) linear_f32_parts(LinearArgs a, 
             if (alive && !ft_bar_wait(&done[it & 1], (it >> 1) & 1)) { alive = false; atomicOr(&flags, 2); }
             __syncwarp();
             ft_fence_after();
-            float v[32];
+            float v[16];  // (32 at once spill beside the operands in flight)
 #pragma unroll
-            for (int c = 0; c < NC / 32; ++c) {
-                ft_ld32(mine + (it & 1) * 128 + c * 32, v);
+            for (int c = 0; c < NC / 16; ++c) {
+                ft_ld16(mine + (it & 1) * 128 + c * 16, v);
 #pragma unroll
-                for (int j = 0; j < 32; ++j) acc[c * 32 + j] += v[j];
+                for (int j = 0; j < 16; ++j) acc[c * 16 + j] += v[j];
             }
             ft_fence_before();
         };
@@ -205,8 +292,11 @@ __global__ void __launch_bounds__(FT_THREADS, 1) linear_f32_parts(LinearArgs a, 
 #pragma unroll
             for (int p = 0; p < 6; ++p)
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    ft_mma(d, ft_desc(base + PX[p] * FT_TILE) + (uint64_t)(2 * k), ft_desc(base + (3 + PW[p]) * FT_TILE) + (uint64_t)(2 * k), (p | k) ? 1u : 0u);
+                for (int k = 0; k < 4; ++k) {
+                    const uint64_t xd = ft_desc(base + PX[p] * FT_TILE) + (uint64_t)(2 * k), wd = ft_desc(base + (3 + PW[p]) * FT_TILE) + (uint64_t)(2 * k);
+                    if (k == 0 && (p == 3 || p == 5)) ft_mma<8>(d, xd, wd, 1u);  // the scale of the parts changes: 2^16, 2^8, 1
+                    else ft_mma<0>(d, xd, wd, (p | k) ? 1u : 0u);
+                }
             ft_commit(&done[it & 1]);
         }
     }
@@ -230,22 +320,23 @@ __global__ void __launch_bounds__(FT_THREADS, 1) linear_f32_parts(LinearArgs a, 
     }
     // this CTA's share of the tile's rows: sums over the ranks in order, then the step that follows the Linear, a pair of columns per thread
     const int share = FT_BM / splits, first = rank * share;
-    for (int i = tid; i < share * (FT_BN / 2); i += FT_THREADS) {
-        const int r = first + i / (FT_BN / 2), c = (i % (FT_BN / 2)) * 2;
-        if (r >= rows || c >= cols) continue;
-        float v0 = 0.f, v1 = 0.f;
-        if (mark & 2) {
-            v0 = v1 = __int_as_float(0x7fffffff);
-        } else if (mark & 1) {
-            const float *x = X + (size_t)r * a.x_pitch(), *w0 = W + (size_t)c * a.K, *w1 = W + (size_t)min(c + 1, cols - 1) * a.K;
-            for (int k = 0; k < a.K; ++k) { v0 = fmaf(x[k], w0[k], v0); v1 = fmaf(x[k], w1[k], v1); }
-        } else if (splits > 1) {
-            for (int s = 0; s < splits; ++s) { v0 += ft_ld_cluster(ft_smem(&sum[r][c]), s); v1 += ft_ld_cluster(ft_smem(&sum[r][c + 1]), s); }
-        } else {
-            const float2 v = *reinterpret_cast<const float2*>(&sum[r][c]);
-            v0 = v.x; v1 = v.y;
+    if (mark == 1) {
+        ft_fma_rows<VEC>(a, X, W, reinterpret_cast<float*>(sm), m0, n0, first, share, rows, cols);
+    } else {
+        for (int i = tid; i < share * (FT_BN / 2); i += FT_THREADS) {
+            const int r = first + i / (FT_BN / 2), c = (i % (FT_BN / 2)) * 2;
+            if (r >= rows || c >= cols) continue;
+            float v0 = 0.f, v1 = 0.f;
+            if (mark & 2) {
+                v0 = v1 = __int_as_float(0x7fffffff);
+            } else if (splits > 1) {
+                for (int s = 0; s < splits; ++s) { v0 += ft_ld_cluster(ft_smem(&sum[r][c]), s); v1 += ft_ld_cluster(ft_smem(&sum[r][c + 1]), s); }
+            } else {
+                const float2 v = *reinterpret_cast<const float2*>(&sum[r][c]);
+                v0 = v.x; v1 = v.y;
+            }
+            epilogue_pair<float>(a, m0 + r, n0 + c, v0, v1, n0 + c + 1 < a.N);
         }
-        epilogue_pair<float>(a, m0 + r, n0 + c, v0, v1, n0 + c + 1 < a.N);
     }
     if (splits > 1) ft_cluster_sync();  // nobody leaves while its sums are being read
 }

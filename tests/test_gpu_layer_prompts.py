@@ -237,6 +237,49 @@ def test_fp32_linear_in_parts(M, N, K):
     assert rel(big, (x * 1e30).double() @ (w * 1e-30).double().T) < 2 ** -21 and rel(tiny, x.double() @ w.double().T) < 2 ** -21
 
 
+def _operands(kind, *shape, g):
+    if kind == "normal":
+        return torch.randn(*shape, generator=g)
+    if kind == "positive":
+        return 1 + torch.rand(*shape, generator=g)
+    if kind == "low bits":  # what truncated parts leave out has one sign
+        return torch.full(shape, 1 + 2.0 ** -7 - 2.0 ** -23)
+    return torch.randn(*shape, generator=g) * 2.0 ** {"tiny": -118, "huge": 115, "least": -122}[kind]
+
+
+@pytest.mark.parametrize("K", [1, 3, 8, 15, 16, 17, 64, 100, 2048])
+@pytest.mark.parametrize("kx,kw", [("normal", "normal"), ("positive", "positive"), ("low bits", "low bits"), ("tiny", "normal"), ("tiny", "huge"), ("normal", "tiny"), ("huge", "tiny"),
+                                   ("least", "huge")])
+def test_fp32_linear_is_no_less_exact_than_fmas(kx, kw, K):
+    """Either side of the step from FMAs to parts, operands of one sign, with all low bits set, and from both ends of fp32's range: no further from
+    float64 than a chain of FMAs is, beside the one step in which the tensor core cuts its sum off, at most 2^-23 of it, and below 16 columns not even that."""
+    from mistral_inference_b200 import _abi_hybrid as h
+
+    g = torch.Generator().manual_seed(K)
+    x, w = _operands(kx, 40, K, g=g).to(DEV), _operands(kw, 200, K, g=g).to(DEV)
+    ref, chain = x.double() @ w.double().T, torch.zeros(40, 200, device=DEV)
+    for k in range(K):
+        chain = torch.addcmul(chain, x[:, k:k + 1], w[:, k][None])
+    assert rel(h.linear(x, w, epi=h.EPI_F32), ref) <= max(2.0 ** -23 if K >= 16 else 0.0, 1.02 * rel(chain, ref))
+
+
+@pytest.mark.parametrize("M,N,K", [(40, 300, 256), (130, 200, 2048), (128, 128, 1029), (260, 1000, 640)])
+def test_fp32_linear_with_infinities_is_a_chain_of_fmas(M, N, K):
+    """A tile that holds an infinity or a NaN: exactly the FMA chain's results in all its rows, whatever part of the chip it was spread over."""
+    from mistral_inference_b200 import _abi_hybrid as h
+
+    g = torch.Generator().manual_seed(M)
+    x, w = torch.randn(M, K, generator=g).to(DEV), torch.randn(N, K, generator=g).to(DEV)
+    x[3, 7], x[M - 1, K - 1], w[N - 1, 8] = float("inf"), float("nan"), float("-inf")
+    chain = torch.zeros(M, N, device=DEV)
+    for k in range(K):
+        chain = torch.addcmul(chain, x[:, k:k + 1], w[:, k][None])
+    got = h.linear(x, w, epi=h.EPI_F32)
+    assert torch.equal(torch.isnan(got), torch.isnan(chain)) and torch.equal(torch.isinf(got), torch.isinf(chain))
+    m0, n0 = (M - 1) // 128 * 128, (N - 1) // 128 * 128
+    assert torch.equal(torch.nan_to_num(got[:128]), torch.nan_to_num(chain[:128])) and torch.equal(torch.nan_to_num(got[m0:, n0:]), torch.nan_to_num(chain[m0:, n0:]))
+
+
 def test_fp32_linear_infinities():
     from mistral_inference_b200 import _abi_hybrid as h
 
