@@ -24,12 +24,10 @@ SlidingWindow = Union[None, int, List[Optional[int]]]
 
 
 def upload(host: torch.Tensor, device: torch.device) -> torch.Tensor:
-    """A small host tensor on `device` without making the host wait for the stream: a copy from pageable memory ends in a stream
-    synchronisation (~100 us of idle GPU per prompt call, as nothing can be queued behind it).  torch's pinned-memory pool hands a
-    block out again only once the copies that read it have run."""
-    if device.type != "cuda":
-        return host.to(device)
-    return host.pin_memory().to(device, non_blocking=True)
+    """A small host tensor on `device` without making the host wait for the stream: the call takes a copy of pageable memory for itself before it
+    returns, and the stream is free to be busy (8 to 17 us whether it is or not; `.to(device)` waits for it, ~100 us of idle GPU per prompt
+    call, as nothing can be queued meanwhile; a detour through pinned memory costs 12 to 25 us, and an allocation of it on the first call of a size)."""
+    return host.to(device, non_blocking=True)
 
 
 def get_cache_sizes(n_layers: int, max_seq_len: int, sliding_window: SlidingWindow) -> List[int]:
