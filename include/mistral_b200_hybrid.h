@@ -13,7 +13,7 @@
 extern "C" {
 #endif
 
-#define MBH_ABI_VERSION 6
+#define MBH_ABI_VERSION 7
 
 int mbh_abi_version(void);
 const char* mbh_last_error(void);
@@ -39,10 +39,6 @@ int mbh_linear(const void* x, int64_t ldx, const void* w, const void* bias, void
 /* Decays of a gated recurrence: out32[M, N] = exp(-exp(a_log[n / group]) * softplus(x W^T + bias)), fp32 from the sum on; a_log [N / group]. */
 int mbh_linear_decay(const void* x, int64_t ldx, const void* w, const void* bias, const void* a_log, int64_t group, void* out32, int64_t M, int64_t N, int64_t K,
                      int dt, void* stream);
-
-/* The epilogues of mbh_linear alone, applied to y[M, N] (storage type, N even) that another GEMM produced. */
-int mbh_linear_epilogue(const void* y, const void* bias, void* out, void* out32, int64_t M, int64_t N, int epi, int64_t n_act, float limit, float alpha,
-                        int dt, void* stream);
 
 /* Splits qkv[T, H*d + G*d + G*e]; RMS-norms every q and k head over d with the shared weights qnorm / knorm [d] (null: no
  * norm); multiplies q at position p by 1 + temp_coef * ln(floor((p + 1) / temp_every) + 1) (temp_every = 0: no temperature);
@@ -84,11 +80,9 @@ int mbh_embed_add(const void* tokens, const void* table, float scale, void* x32,
 int mbh_layernorm(const void* x32, const void* w, const void* b, void* y, void* acc32, int64_t T, int64_t D, float eps, int dt, void* stream);
 
 /* Linear with interleaved gate/up rows (as epilogue 2 of mbh_linear) and out[M, N/2] = act(gate) * up * rowscale[m, c / rs_group];
- * act 0: SiLU, 1: the tanh form of gelu; rowscale: fp32 [M, rs_pitch] or null (no scaling).  mbh_swiglu_epilogue applies the same to y[M, N] of another GEMM. */
+ * act 0: SiLU, 1: the tanh form of gelu; rowscale: fp32 [M, rs_pitch] or null (no scaling). */
 int mbh_linear_swiglu(const void* x, const void* w, void* out, int64_t M, int64_t N, int64_t K, const void* rowscale, int64_t rs_pitch,
                       int64_t rs_group, int act, int dt, void* stream);
-int mbh_swiglu_epilogue(const void* y, void* out, int64_t M, int64_t N, const void* rowscale, int64_t rs_pitch, int64_t rs_group, int act, int dt,
-                        void* stream);
 
 /* Latent attention, input side.  y [T, pitch] holds the query latent (q_rank entries from column 0; q_rank 0: none) and, from column kv_off,
  * [key/value latent (kv_rank) | shared rotated key part (rot_dim)].  cq [T, q_rank] = rms_norm(query latent) * qnorm; the token's row
@@ -185,11 +179,9 @@ int mbh_attn_decode(const void* q, const void* ring_k, const void* ring_v, const
                     const void* gate, int64_t gate_pitch, int gate_entry, int64_t maps, const void* lambda, float out_scale, float norm_eps, int dt, void* stream);
 
 /* Linear with interleaved gate/up rows and the clamped gated unit of mbh_linear's epilogue 2; gate and up of column c are multiplied by
- * rowscale[m, c / rs_group] (fp32 [M, rs_pitch]; null: 1) BEFORE the clamps.  mbh_glu_epilogue applies the same to y[M, N] of another GEMM. */
+ * rowscale[m, c / rs_group] (fp32 [M, rs_pitch]; null: 1) BEFORE the clamps. */
 int mbh_linear_glu(const void* x, const void* w, void* out, int64_t M, int64_t N, int64_t K, float limit, float alpha, const void* rowscale,
                    int64_t rs_pitch, int64_t rs_group, int dt, void* stream);
-int mbh_glu_epilogue(const void* y, void* out, int64_t M, int64_t N, float limit, float alpha, const void* rowscale, int64_t rs_pitch, int64_t rs_group,
-                     int dt, void* stream);
 
 /* x32[t, :] = table[tokens[t], :] * scale + pos_table[positions[t], :] (learned positions; positions int32 [T]). */
 int mbh_embed_pos(const void* tokens, const void* positions, const void* table, const void* pos_table, float scale, void* x32, int64_t T, int64_t D,
@@ -266,12 +258,9 @@ int mbh_gla_qab(const void* qk, int64_t pitch, const void* z32, void* qab, int64
 int mbh_whole_norm_prep(const void* qkv, const void* qnorm, const void* knorm, const void* cache_rows, void* q_out, void* k_out, void* v_out,
                         void* ring_k, void* ring_v, int64_t T, int64_t Nq, int64_t Nk, int64_t Nv, float eps, int dt, void* stream);
 
-/* out[M, N] = max(x W^T, 0)^2 * rowscale[m, n / rs_group] (rowscale fp32 [M, rs_pitch] or null); mbh_relu2_epilogue applies the same to
- * y[M, N] (N even) of another GEMM. */
+/* out[M, N] = max(x W^T, 0)^2 * rowscale[m, n / rs_group] (rowscale fp32 [M, rs_pitch] or null). */
 int mbh_linear_relu2(const void* x, const void* w, void* out, int64_t M, int64_t N, int64_t K, const void* rowscale, int64_t rs_pitch,
                      int64_t rs_group, int dt, void* stream);
-int mbh_relu2_epilogue(const void* y, void* out, int64_t M, int64_t N, const void* rowscale, int64_t rs_pitch, int64_t rs_group, int dt,
-                       void* stream);
 
 /* Gated delta rule, S <- diag(g) S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q per head.  y [T, y_pitch] = q (G*d) | k (G*d) | v (H*e) | beta
  * logits (H) | decay latent (ra) | gate latent (rg) | ...; head h uses q / k head h / (H / G).  q, k and v first pass a causal convolution over

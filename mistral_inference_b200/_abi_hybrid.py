@@ -13,7 +13,7 @@ import torch
 from . import _abi, build
 from ._abi import Mb200Error
 
-ABI_VERSION = 6
+ABI_VERSION = 7
 EPI_STORE, EPI_RESIDUAL, EPI_GLU, EPI_F32, EPI_SWIGLU, EPI_RESIDUAL_SCALED, EPI_RELU2, EPI_GEGLU = 0, 1, 2, 3, 4, 5, 6, 7
 _DT = {torch.bfloat16: 0, torch.float32: 1}
 _lib: Optional[ctypes.CDLL] = None
@@ -26,7 +26,6 @@ _SIGNATURES = {
     "mbh_rmsnorm": (c_int, [P, P, P, P, P, I, I, F, F, c_int, P]),
     "mbh_linear_decay": (c_int, [P, I, P, P, P, I, P, I, I, I, c_int, P]),
     "mbh_linear": (c_int, [P, I, P, P, P, P, I, I, I, c_int, I, F, F, c_int, P]),
-    "mbh_linear_epilogue": (c_int, [P, P, P, P, I, I, c_int, I, F, F, c_int, P]),
     "mbh_attn_prep": (c_int, [P, P, P, P, P, P, P, P, P, P, c_int, I, I, I, I, I, F, F, I, c_int, P]),
     "mbh_attn_bias": (c_int, [P, P, P, P, I, P, P, P, P, I, I, I, I, I, I, I, F, I, I, P, c_int, P]),
     "mbh_lightning_scan": (c_int, [P, P, P, P, P, P, P, I, I, I, I, c_int, P]),
@@ -36,7 +35,6 @@ _SIGNATURES = {
     "mbh_embed_add": (c_int, [P, P, F, P, I, I, c_int, P]),
     "mbh_layernorm": (c_int, [P, P, P, P, P, I, I, F, c_int, P]),
     "mbh_linear_swiglu": (c_int, [P, P, P, I, I, I, P, I, I, c_int, c_int, P]),
-    "mbh_swiglu_epilogue": (c_int, [P, P, I, I, P, I, I, c_int, c_int, P]),
     "mbh_latent_prep": (c_int, [P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, c_int, F, F, P, c_int, P]),
     "mbh_latent_absorb": (c_int, [P, I, P, P, P, P, I, I, I, I, I, c_int, I, F, c_int, P]),
     "mbh_latent_expand": (c_int, [P, P, P, I, I, I, I, I, c_int, P]),
@@ -49,7 +47,6 @@ _SIGNATURES = {
     "mbh_attn_window": (c_int, [P, P, P, P, I, P, P, P, P, I, I, I, I, I, I, I, F, I, I, P, I, c_int, P, P, P, I, c_int, F, P, P, I, c_int, I, P, F, F, c_int, P]),
     "mbh_attn_decode": (c_int, [P, P, P, P, P, P, I, I, I, I, I, I, F, I, P, I, c_int, F, P, P, I, c_int, I, P, F, F, c_int, P]),
     "mbh_linear_glu": (c_int, [P, P, P, I, I, I, F, F, P, I, I, c_int, P]),
-    "mbh_glu_epilogue": (c_int, [P, P, I, I, F, F, P, I, I, c_int, P]),
     "mbh_embed_pos": (c_int, [P, P, P, P, F, P, I, I, c_int, P]),
     "mbh_rot_prep": (c_int, [P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, c_int, F, c_int, F, c_int, P]),
     "mbh_kv_scatter": (c_int, [P, P, P, P, P, I, I, I, c_int, P]),
@@ -64,7 +61,6 @@ _SIGNATURES = {
     "mbh_gla_qab": (c_int, [P, I, P, P, I, I, F, F, c_int, P]),
     "mbh_whole_norm_prep": (c_int, [P, P, P, P, P, P, P, P, P, I, I, I, I, F, c_int, P]),
     "mbh_linear_relu2": (c_int, [P, P, P, I, I, I, P, I, I, c_int, P]),
-    "mbh_relu2_epilogue": (c_int, [P, P, I, I, P, I, I, c_int, P]),
     "mbh_delta_prep": (c_int, [P, I, P, I, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, c_int, P]),
     "mbh_delta_scan": (c_int, [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, P]),
     "mbh_delta_step": (c_int, [P, I, I, I, P, I, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, F, c_int, P]),

@@ -115,13 +115,6 @@ template <typename T> static void run_rmsnorm(const void* x32, const void* w, co
                                               cudaStream_t st) {
     launch_pdl(rmsnorm_f32_kernel<T>, dim3((unsigned)T_), dim3(D >= 1024 ? 256 : 128), 0, st, (const float*)x32, (const T*)w, (const T*)w2, (T*)y, (T*)y2, (int)D, eps, offset);
 }
-template <typename T> static void run_epilogue(const LinearArgs& a, const void* y, cudaStream_t st) {
-    if constexpr (sizeof(T) == 2) {
-        if (launch_epilogue8(a, (const bf16*)y, st)) return;
-    }
-    const size_t pairs = (size_t)a.M * (a.N >> 1);
-    linear_epilogue_kernel<T><<<(unsigned)((pairs + 255) / 256), 256, 0, st>>>(a, (const T*)y);
-}
 template <typename T> static void run_prep(const AttnPrepArgs& a, int64_t T_, cudaStream_t st) {
     // few tokens (decode): a warp per head, so that no head waits for another; many: four warps walk the heads, tokens fill the chip
     const int warps = T_ >= 1024 ? 4 : (int)std::min<int64_t>(32, std::max(4, a.H + a.G));
@@ -204,17 +197,6 @@ int mbh_linear_decay(const void* x, int64_t ldx, const void* w, const void* bias
     if (dt == 0 && launch_linear_decay_mma(a, (cudaStream_t)stream, e)) return e ? fail(e, "mbh_linear_decay") : 0;
     DISPATCH(dt, e = launch_linear<ST>(a, (cudaStream_t)stream));
     return e ? fail(e, "mbh_linear_decay") : 0;
-}
-
-int mbh_linear_epilogue(const void* y, const void* bias, void* out, void* out32, int64_t M, int64_t N, int epi, int64_t n_act, float limit, float alpha,
-                        int dt, void* stream) {
-    if (((epi < 0 || epi > 3) && epi != EPI_RESIDUAL_SCALED) || (N & 1)) return bad("mbh_linear_epilogue: unknown epilogue or odd N");
-    if (M == 0) return 0;
-    LinearArgs a{nullptr, nullptr, bias, out, (float*)out32, (int)M, (int)N, 0, epi, (int)n_act, limit, alpha};
-    cudaStream_t st = (cudaStream_t)stream;
-    DISPATCH(dt, run_epilogue<ST>(a, y, st));
-    cudaError_t e = cudaGetLastError();
-    return e ? fail(e, "mbh_linear_epilogue") : 0;
 }
 
 int mbh_attn_prep(const void* qkv, const void* qnorm, const void* knorm, const void* positions, const void* cache_rows, void* q_out, void* cache_k,
@@ -375,18 +357,6 @@ int mbh_linear_swiglu(const void* x, const void* w, void* out, int64_t M, int64_
     return e ? fail(e, "mbh_linear_swiglu") : 0;
 }
 
-int mbh_swiglu_epilogue(const void* y, void* out, int64_t M, int64_t N, const void* rowscale, int64_t rs_pitch, int64_t rs_group, int act, int dt,
-                        void* stream) {
-    if (N & 1) return bad("mbh_swiglu_epilogue: odd N");
-    if (rowscale && rs_group <= 0) return bad("mbh_swiglu_epilogue: rs_group must be positive");
-    if (M == 0) return 0;
-    LinearArgs a{nullptr, nullptr, nullptr, out, nullptr, (int)M, (int)N, 0, act ? EPI_GEGLU : EPI_SWIGLU, 0, 0.f, 0.f, (const float*)rowscale, (int)rs_pitch, (int)rs_group};
-    cudaStream_t st = (cudaStream_t)stream;
-    DISPATCH(dt, run_epilogue<ST>(a, y, st));
-    cudaError_t e = cudaGetLastError();
-    return e ? fail(e, "mbh_swiglu_epilogue") : 0;
-}
-
 int mbh_latent_prep(const void* y, const void* qnorm, const void* cnorm, const void* freq, const void* positions, const void* cache_rows, void* cq,
                     void* ring, int64_t T, int64_t pitch, int64_t q_rank, int64_t kv_off, int64_t kv_rank, int64_t rot_dim, int64_t rot_dims, int halves, float eps,
                     float mag, void* own, int dt, void* stream) {
@@ -521,18 +491,6 @@ int mbh_linear_glu(const void* x, const void* w, void* out, int64_t M, int64_t N
     cudaError_t e = cudaSuccess;
     DISPATCH(dt, e = launch_linear<ST>(a, (cudaStream_t)stream));
     return e ? fail(e, "mbh_linear_glu") : 0;
-}
-
-int mbh_glu_epilogue(const void* y, void* out, int64_t M, int64_t N, float limit, float alpha, const void* rowscale, int64_t rs_pitch, int64_t rs_group,
-                     int dt, void* stream) {
-    if (N & 1) return bad("mbh_glu_epilogue: odd N");
-    if (rowscale && rs_group <= 0) return bad("mbh_glu_epilogue: rs_group must be positive");
-    if (M == 0) return 0;
-    LinearArgs a{nullptr, nullptr, nullptr, out, nullptr, (int)M, (int)N, 0, EPI_GLU, 0, limit, alpha, (const float*)rowscale, (int)rs_pitch, (int)rs_group};
-    cudaStream_t st = (cudaStream_t)stream;
-    DISPATCH(dt, run_epilogue<ST>(a, y, st));
-    cudaError_t e = cudaGetLastError();
-    return e ? fail(e, "mbh_glu_epilogue") : 0;
 }
 
 int mbh_embed_pos(const void* tokens, const void* positions, const void* table, const void* pos_table, float scale, void* x32, int64_t T, int64_t D,
@@ -728,18 +686,6 @@ int mbh_linear_relu2(const void* x, const void* w, void* out, int64_t M, int64_t
     cudaError_t e = cudaSuccess;
     DISPATCH(dt, e = launch_linear<ST>(a, (cudaStream_t)stream));
     return e ? fail(e, "mbh_linear_relu2") : 0;
-}
-
-int mbh_relu2_epilogue(const void* y, void* out, int64_t M, int64_t N, const void* rowscale, int64_t rs_pitch, int64_t rs_group, int dt,
-                       void* stream) {
-    if (M == 0 || N == 0) return 0;
-    if (N & 1) return bad("mbh_relu2_epilogue: N must be even");
-    if (rowscale && rs_group <= 0) return bad("mbh_relu2_epilogue: rs_group must be positive");
-    LinearArgs a{nullptr, nullptr, nullptr, out, nullptr, (int)M, (int)N, 0, EPI_RELU2, 0, 0.f, 0.f, (const float*)rowscale, (int)rs_pitch, (int)rs_group};
-    cudaStream_t st = (cudaStream_t)stream;
-    DISPATCH(dt, run_epilogue<ST>(a, y, st));
-    cudaError_t e = cudaGetLastError();
-    return e ? fail(e, "mbh_relu2_epilogue") : 0;
 }
 
 }  // extern "C"
