@@ -409,3 +409,23 @@ def test_linear_of_a_few_tokens(T, N, K):
     ref = x.double() @ w.double().T + res.double()
     _abi.linear_residual(x, w, res, res, ws)  # in place
     assert rel(res, ref) < 2 ** -7  # the product's rounding and the sum's, 2^-8 of each size
+
+
+@pytest.mark.parametrize("T,N,K", [(500, 4096, 8192), (100, 4096, 4096)])
+def test_two_streams_of_linears_that_share_their_tiles(T, N, K):
+    """Pairs cut along k and split stream-K tiles on two streams at once (each call has its own scratch): the bits of one stream alone.  Owners wait
+    for blocks that started before them only, so neither launch needs the whole chip."""
+    from mistral_inference_b200 import _abi, _abi_hybrid as h
+
+    g = torch.Generator(device=DEV).manual_seed(T)
+    assert _abi.lib().mb200_layer_linear_scratch(T, N, K) > 0
+    x, w = torch.randn(T, K, device=DEV, generator=g).bfloat16(), (torch.randn(N, K, device=DEV, generator=g) / K ** 0.5).bfloat16()
+    ref = h.linear(x, w, epi=h.EPI_F32)
+    torch.cuda.synchronize()
+    streams, got = [torch.cuda.Stream() for _ in range(2)], []
+    for _ in range(10):
+        for s in streams:
+            with torch.cuda.stream(s):
+                got.append(h.linear(x, w, epi=h.EPI_F32))
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, ref) for o in got)
