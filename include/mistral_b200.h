@@ -3,7 +3,7 @@
  * transformer hot path (Attention block + FeedForward/MoE block + the norm / lm-head either side).
  *
  * The reference (mistralai/mistral-inference @ 2557e12) is pure Python and has NO FFI / plugin
- * boundary (SURVEY.md section 0.3, 8b); its hot path is a sequence of torch / xformers library calls.
+ * boundary; its hot path is a sequence of torch / xformers library calls.
  * Each entry point below replaces one group of those call sites and cites them.  The reference-side
  * binding is a ctypes stub; in this repo the caller is
  * mistral_inference_b200/_abi.py, which mirrors the reference's Python API on top.
@@ -17,7 +17,7 @@
  *   - returns 0 on success, a negative MB200_E_* code otherwise; mb200_last_error() gives the
  *     thread-local message.  Nothing throws across the boundary.
  *   - integer metadata (positions, rows, lengths) are int32 device arrays.
- *   - head_dim must be 128 (every config in BASELINE.json); dims must be multiples of 8 (16-byte rows).
+ *   - head_dim must be 128; dims must be multiples of 8 (16-byte rows).
  */
 #ifndef MISTRAL_B200_H_
 #define MISTRAL_B200_H_

@@ -57,7 +57,7 @@ class TransformerArgs:
         # same aliasing as args.py:58-59
         self.sliding_window = self.sliding_window if self.sliding_window is not None else self._sliding_window
         if self.vision_encoder is not None:
-            raise NotImplementedError("vision_encoder (Pixtral) is outside the accelerated hot path (SURVEY.md 2, row 10)")
+            raise NotImplementedError("vision_encoder (Pixtral) is outside the accelerated hot path")
         if isinstance(self.moe, dict):
             self.moe = MoeArgs.from_dict(self.moe)
         if isinstance(self.lora, dict):

@@ -1,6 +1,6 @@
 """Builds libmb200.so (the C-ABI CUDA library) in-tree with nvcc for sm_100a.
 
-In-tree so the built .so travels to the GPU box with the gpurun snapshot (a JIT cache would not).
+In-tree, so that a copy of the checkout carries its built libraries with it (a JIT cache would not).
 `python -m mistral_inference_b200.build [--force] [--verbose]`
 """
 import hashlib

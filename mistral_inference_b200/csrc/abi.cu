@@ -189,7 +189,7 @@ int mb200_attn_decode(const void* q, const void* cache_k, const void* cache_v, c
   p.H = (int)n_heads;
   p.KV = (int)n_kv_heads;
   p.S = (int)n_splits;
-  p.scale = 0.08838834764831845f;  // 128^-0.5 (xformers default scale; Attention.scale is unused, SURVEY E-3)
+  p.scale = 0.08838834764831845f;  // 128^-0.5 (xformers default scale; Attention.scale is unused)
   p.partial = nullptr;
   p.counters = nullptr;
   if (n_splits > 1) {

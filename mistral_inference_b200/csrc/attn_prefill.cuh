@@ -7,7 +7,7 @@
 // reference's interleave_kv / unrotate / repeat_kv copies (cache.py:94-117, transformer_layers.py:84) become
 // address arithmetic -- key at absolute position j of sequence b lives in ring row b*W + j % W if j < seqpos[b]
 // (already cached) and in the chunk buffer at token q_start[b] + j - seqpos[b] otherwise.
-// Mask (cache.py:240,243-248; SURVEY.md Appendix B): query at absolute position p sees keys in (p - W, p].
+// Mask (cache.py:240,243-248): query at absolute position p sees keys in (p - W, p].
 #pragma once
 #include "gemm_mma.cuh"
 

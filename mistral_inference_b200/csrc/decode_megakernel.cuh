@@ -12,7 +12,7 @@
 //   * 8 CONSUMER warps do the math out of shared memory (fp32 FMA on bf16 pairs; batch 1 is ~0.1 flop/byte, far
 //     below the CUDA-core roof, tensor cores would not help), with the same fused prologues/epilogues as the
 //     per-op kernels (RMSNorm, RoPE + ring scatter, SiLU*mul, residual adds) and the same rounding points as the
-//     reference.
+//     reference (oracle/restatement.py states them).
 //   * phases are separated by a self-resetting sense-reversing grid barrier (5 per layer).
 // Row pairs (2 rows = one RoPE pair / one gate-up pair) are dealt to CTAs as contiguous ranges:
 // CTA c owns pairs [c*P/G, (c+1)*P/G) of each matrix, so its slice of every weight matrix is one contiguous byte
@@ -40,7 +40,7 @@ constexpr int MK_PRODUCER_WARPS = MB200_MK_PRODUCERS;  // one issuing thread eac
 #define MB200_MK_WG 0
 #endif
 #if MB200_MK_WG
-// Experiment (round 2): producers in their own warpgroup so that setmaxnreg can move registers to the consumers (384 threads launch
+// Experiment: producers in their own warpgroup so that setmaxnreg can move registers to the consumers (384 threads launch
 // with 168 registers; the pool a CTA can re-acquire is only what it released: (168 - 120) x 128 = (192 - 168) x 256).
 constexpr int MK_THREADS = MK_CONSUMERS + 128;
 #else
@@ -280,7 +280,7 @@ __device__ __forceinline__ AttnSlice attn_slice(const MkParams& p, int W) {
 // function of (blockIdx, shapes, pos), so the producer simply walks it, blocking only on free ring slots.  Its per-stage
 // budget is ~350 cycles (5.5 stages/us per SM at the HBM share of one SM): keep these loops lean -- a generic "schedule
 // iterator" version (needed for a second, L2-prefetch cursor) cost 5 % end to end on its own.
-// Experiment on record: running cp.async.bulk.prefetch.L2 D stages ahead to use the L2 as a second-level ring
+// Experiment: running cp.async.bulk.prefetch.L2 D stages ahead to use the L2 as a second-level ring
 // made things WORSE on B200 (3.4 -> 4.3 ms/token at D = 16, 5.0 at D = 64): the prefetched lines do not survive until the copy.
 __device__ __forceinline__ void bulk_g2s_hint(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar, uint64_t policy) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(

@@ -54,7 +54,7 @@ __global__ void kv_ring_write_kernel(const uint4* __restrict__ k_new, const uint
   }
 }
 
-// Device-side step state of the batched decode loop (SURVEY.md N2; replaces cache.py:197-263 for one-token steps).  Reads the
+// Device-side step state of the batched decode loop (replaces cache.py:197-263 for one-token steps).  Reads the
 // per-sequence positions, writes the metadata block every layer's kernels read -- same layout as the host-built block of
 // mistral_inference_b200/cache.py::build_metadata_host for seqlens = [1] * B:
 //   positions[B] | q_start[B + 1] | seqpos[B] | per distinct window W: cache_rows[B], kv_len[B]

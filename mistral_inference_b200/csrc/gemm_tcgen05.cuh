@@ -52,7 +52,7 @@ struct TgCfg {
   // A full 16 KB of slack is more than the 20-24 KB stages of the stream-K kernel need, and it is what keeps its CTAs at 117.5 KB:
   // TWO of them do not fit an SM.  That is deliberate: with the exact slack (-DMB200_TIGHT_SLACK: 101.5 KB, the successor launch's
   // CTA sits beside the running one from its start) the Nemo-12B batch-32 step measured 7.48 ms against 6.85 ms on the same box
-  // (call 22) -- the early CTA's ring fill and polling take bandwidth and issue slots from the launch that is on the critical path.
+  // -- the early CTA's ring fill and polling take bandwidth and issue slots from the launch that is on the critical path.
   // As it is, a successor CTA starts when the predecessor's CTA on that SM exits, i.e. during the predecessor's reduction tail.
 #ifdef MB200_TIGHT_SLACK
   static constexpr int kSlack = (TA < 128 && kStageBytes < TG_A_BYTES) ? TG_A_BYTES - kStageBytes : 0;

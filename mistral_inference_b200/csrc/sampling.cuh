@@ -1,4 +1,4 @@
-// Device-side token selection and log-probabilities (SURVEY.md N1): the per-token tail of generate().
+// Device-side token selection and log-probabilities: the per-token tail of generate().
 //
 //   argmax_rows_kernel      greedy pick: torch.argmax(logits, -1) (generate.py:156), first index on ties
 //   logprob_gather_kernel   log_softmax(logits, -1)[t, target[t]] (generate.py:101-117,134-135) without materialising [T, V]

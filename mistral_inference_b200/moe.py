@@ -9,7 +9,7 @@ else -- prefill and batched decode -- goes through two C-ABI calls per layer wit
                          out = h + sum_j bf16(w_j * y_j) taken in ascending expert index, rounded to bf16 at every step exactly
                          like the reference's `results[idx] += w * expert(x)` loop (moe.py:28-31)
 
-Expert parallelism (SURVEY.md 8e): with `expert_shard = (g, G)` this rank owns the experts `e % G == g` and holds no weights of
+Expert parallelism: with `expert_shard = (g, G)` this rank owns the experts `e % G == g` and holds no weights of
 the others.  Every rank evaluates the router and the row plan redundantly (deterministic, identical on all ranks), runs the
 grouped GEMMs for its own experts, and the DOWN PROJECTION'S EPILOGUE stores each weighted output row into the row buffer of
 every rank over NVLink (peer memory mapped with CUDA IPC, `ExpertComm`): the exchange is an all-gather of rows fused into the

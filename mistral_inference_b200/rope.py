@@ -2,7 +2,7 @@
 
 The table is built on the CPU in fp32 exactly as the reference does (transformer.py:108-120 builds it on
 the default device, then moves it) and uploaded, so the kernels multiply by the very same cos/sin bits
-instead of calling sincosf on the device (SURVEY.md Appendix A-3).  The rotation itself
+instead of calling sincosf on the device.  The rotation itself
 (rope.py:13-23) is the epilogue of the fused QKV kernel (csrc/epilogue.cuh, EPI_QKV_ROPE).
 """
 import torch

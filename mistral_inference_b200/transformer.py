@@ -55,7 +55,7 @@ class Transformer(nn.Module):
                  expert_parallel: Optional[Tuple[int, int]] = None, expert_group: Any = None):
         """Same signature as the reference (transformer.py:34-40) plus `expert_parallel = (rank, world)`: MoE experts sharded
         `e % world == rank` over the ranks of `expert_group` (default process group), everything else replicated, one
-        all-reduce of [T, dim] per MoE layer (SURVEY.md 8e)."""
+        all-reduce of [T, dim] per MoE layer."""
         super().__init__()
         self.args = args
         self.expert_parallel = expert_parallel or (0, 1)
@@ -383,7 +383,7 @@ class Transformer(nn.Module):
         self._last_static_logits = st["logits"].data_ptr()
         return st["logits"]
 
-    # ------------------------------------------------------------------ generate() support (SURVEY.md N1 / N2)
+    # ------------------------------------------------------------------ generate() support
     def last_argmax_valid_for(self, logits: torch.Tensor) -> bool:
         """True when `last_argmax` is the decode kernel's own argmax of exactly this logits buffer."""
         return self.last_argmax is not None and logits.data_ptr() == self._last_static_logits

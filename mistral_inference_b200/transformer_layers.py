@@ -84,7 +84,7 @@ class Attention(nn.Module):
         out = torch.empty(T, self.q_dim, dtype=x.dtype, device=x.device)
         H, KV, hd = self.n_heads, self.n_kv_heads, self.head_dim
         if cache is None:
-            # cache-less forward: unmasked over the whole flattened batch (SURVEY.md Appendix E-2)
+            # cache-less forward: unmasked over the whole flattened batch
             _abi.attn_qkv(x, norm_w, self.wqkv, rope, positions, q, k, v, None, None, None, H, KV, hd, eps, ws)
             _abi.attn_prefill(q, k, v, None, None, None, None, out, 1, T, 0, H, KV, hd, causal=False)
             return out
@@ -163,7 +163,7 @@ class TransformerBlock(nn.Module):
         self.ffn_norm = RMSNorm(dim, eps=norm_eps)
         self.feed_forward: nn.Module
         if moe is not None:
-            g, G = expert_shard  # this rank allocates only the experts it owns (e % G == g): SURVEY.md 8(e)
+            g, G = expert_shard  # this rank allocates only the experts it owns (e % G == g)
             self.feed_forward = MoeLayer(experts={e: FeedForward(dim=dim, hidden_dim=hidden_dim, lora=lora) for e in range(moe.num_experts) if e % G == g},
                                          gate_weight=nn.Parameter(torch.empty(moe.num_experts, dim), requires_grad=False), moe_args=moe,
                                          expert_shard=expert_shard, expert_group=expert_group)

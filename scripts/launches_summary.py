@@ -1,11 +1,11 @@
 #!/usr/bin/env python
-"""gpurun_out/launches.csv (ncu --metrics gpu__time_duration.sum --csv) -> the per-kernel table kept in profiles/."""
+"""launches.csv (ncu --metrics gpu__time_duration.sum --csv) -> the per-kernel table kept in profiles/."""
 import collections
 import csv
 import re
 import sys
 
-path = sys.argv[1] if len(sys.argv) > 1 else "gpurun_out/launches.csv"
+path = sys.argv[1] if len(sys.argv) > 1 else "launches.csv"
 lines = [l for l in open(path) if not l.startswith("==")]
 agg, n = collections.OrderedDict(), 0
 for row in csv.DictReader(lines):

@@ -1,5 +1,5 @@
 """Debug: per-phase timeline of the decode megakernel (CTA 0), Mistral-7B shape at kv_len 4096.
-usage (GPU box): python scripts/mk_timeline.py [n_layers]"""
+usage: python scripts/mk_timeline.py [n_layers]"""
 import sys
 from pathlib import Path
 
