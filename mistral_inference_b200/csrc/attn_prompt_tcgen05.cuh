@@ -4,7 +4,8 @@
 // rows.  One kernel serves first prompts, portions of prompts over a partly filled ring, and the layered decoders' attention, whose keys
 // all lie in the ring.
 //
-// Roofline: tensor pipe and MUFU alike (a 128 x 128 tile is 1024 cycles of MMA for S and P V and 1024 of exp2).  CTA = (two query heads
+// Roofline: tensor pipe and MUFU alike (a 128 x 128 tile is 1024 cycles of MMA for S and P V and 1024 of exp2; 4096 tokens under
+// ncu: tensor pipe 44 % of the cycles).  CTA = (two query heads
 // of one key/value head, 128 queries, sequence): the two S tiles share every K and V tile, and while the softmax warps of one head work the
 // tensor cores work for the other.  10 warps:
 //   warp 0    TMA producer: both Q tiles once, then K, V, K, V, ... tiles of 128 keys (two 128B-swizzled [128 x 64] boxes) into a ring of 32 KB slots

@@ -13,7 +13,8 @@
 //
 // Nothing that was 32 bits wide loses any: q, k, v are bf16 as stored; the state, the decayed values a^(C-1-j) v_j and the decayed scores
 // a^(i-j) (q_i . k_j) are fp32 and enter the products as three bf16 parts each (8 + 8 + 8 significant bits: the parts add up to the
-// number exactly or to its last bit), accumulated in fp32; powers of the decay come from a table made in double precision.
+// number exactly or to its last bit; of numbers below 2^-110 what lies under bf16's smallest, 2^-133, is gone), accumulated in fp32; powers of the
+// decay come from a table made in double precision.
 // A chunk with an infinity or a NaN anywhere (or in the state) is walked token by token instead, so that a token's numbers reach no earlier one.
 #pragma once
 #include "hybrid_attn_flash.cuh"
