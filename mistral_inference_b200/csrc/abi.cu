@@ -10,6 +10,7 @@
 #include "decode_megakernel.cuh"
 #include "elementwise.cuh"
 #include "gemm_mma.cuh"
+#include "gemm_pair.cuh"
 #include "gemm_streamk.cuh"
 #include "gemm_tcgen05.cuh"
 #include "moe.cuh"
@@ -556,13 +557,9 @@ size_t mb200_layer_linear_scratch(int64_t T, int64_t N, int64_t K) {
   if (T < TG_BM) return kWsHeader + SK_PARTIAL_BYTES;
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-  if (T <= TG_BM || N % 256 != 0 || sms < 2 || (T < 4 * TG_BM && !pairs_fill(T, N, K, sms / 2, true))) return 0;
-  TcGemmParams p;
-  p.T = (int)T;
-  p.N = (int)N;
-  p.K = (int)K;
-  plan_pairs(p, sms / 2, &p, nullptr);  // (any non-null scratch: would the launch cut tiles?)
-  return p.cut_pairs > 0 ? TG_CUT_BYTES + 2 * TG_MAX_CUTS * sizeof(unsigned) : 0;
+  if (T <= TG_BM || sms < 2 || !pairs_fill(T, N, K, sms / 2, true)) return 0;
+  const long long tiles = (long long)pair_token_tiles(T) * ceil_div(N, GP_ROWS);
+  return cut_plan(tiles, (int)(K / TG_BK), sms / 2, TG_MAX_CUTS).cut_pairs > 0 ? TG_CUT_BYTES + 2 * TG_MAX_CUTS * sizeof(unsigned) : 0;
 }
 
 int mb200_layer_moe_sizes(int64_t T, int64_t n_experts, int64_t top, int64_t* rows_cap, int64_t* plan_words) {

@@ -263,6 +263,61 @@ __device__ __forceinline__ void epi_layer32_f32(const EpiParams& p, int t0, int 
   }
 }
 
+// the same for a warp whose lanes hold the columns: v[j] is row t0 + j of column n, an access is one 128-byte line.  First what is there already (_fetch, into
+// r), then the step, then _store.  (Row offsets are 32-bit products of the pitch: as 64-bit ones they cost the registers that the rows need.)
+__device__ __forceinline__ void epi_layer32_f32_lanes_fetch(const EpiParams& p, int t0, int rows, int n, uint32_t (&r)[32]) {
+  if (p.layer == LAYER_F32) return;
+  const float* base = p.out_f32 + (int64_t)t0 * p.ld_out + n;
+  const int ld = (int)p.ld_out;
+  if (rows >= 32) {
+#pragma unroll
+    for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(base[j * ld]);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 32; ++j)
+      if (j < rows) r[j] = __float_as_uint(base[j * ld]);
+  }
+}
+__device__ __forceinline__ void epi_layer32_f32_lanes(const EpiParams& p, int n, uint32_t (&v)[32], const uint32_t (&r)[32], bool valid) {
+  if (p.bias != nullptr) {
+    const float b = valid ? bf16_to_float(reinterpret_cast<const uint16_t*>(p.bias)[n]) : 0.f;
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + b);
+  }
+  if (p.layer == LAYER_F32) {
+    if (p.limit > 0.f) {
+#pragma unroll 1
+      for (int j = 0; j < 32; ++j) {  // (a soft cap: heads only; one copy of tanhf, the registers by a select)
+        float x = 0.f;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) x = i == j ? __uint_as_float(v[i]) : x;
+        x = p.limit * tanhf(x / p.limit);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] = i == j ? __float_as_uint(x) : v[i];
+      }
+    }
+    const float f = p.alpha != 0.f ? p.alpha : 1.f;
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * f);
+  } else {
+    const float f = p.layer == LAYER_RESIDUAL_SCALED ? p.alpha : 1.f;
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(r[j]) + f * round_bf16(__uint_as_float(v[j])));
+  }
+}
+__device__ __forceinline__ void epi_layer32_f32_lanes_store(const EpiParams& p, int t0, int rows, int n, const uint32_t (&v)[32]) {
+  float* const base = p.out_f32 + (int64_t)t0 * p.ld_out + n;
+  const int ld = (int)p.ld_out;
+  if (rows >= 32) {
+#pragma unroll
+    for (int j = 0; j < 32; ++j) base[j * ld] = __uint_as_float(v[j]);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 32; ++j)
+      if (j < rows) base[j * ld] = __uint_as_float(v[j]);
+  }
+}
+
 // the same for one row by one thread (the few rows of the stream-K kernel)
 __device__ __forceinline__ void epi_layer32_f32_row(const EpiParams& p, int t, int n, const uint32_t (&v)[32]) {
   float x[32];
@@ -473,6 +528,213 @@ __device__ __forceinline__ void epi_chunk32(const EpiParams& p, int t, int n, co
       for (int q = 0; q < 4; ++q) reinterpret_cast<uint4*>(ring)[q] = make_uint4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
     }
   }
+}
+
+// ---- feature-lane epilogues (gemm_pair.cuh) ------------------------------------------------------------------------------------
+// There a warp's accumulator block has the 32 features in its lanes and 32 tokens in each lane's registers.  Lanes 2i and 2i + 1 exchange halves, as bf16 pairs, and
+// then hold both features of pair i for 16 tokens each: what epi_pair takes.  A store instruction writes the 32 features of two tokens (2 x 64 bytes).
+// y0, y1: features n, n + 1 of tokens t0 + j, as packed pairs of tokens (2q, 2q + 1); tokens from `rows` on are not stored.
+__device__ __forceinline__ float bf16_of(const uint32_t (&y)[8], int j) { return j & 1 ? bf16hi(y[j >> 1]) : bf16lo(y[j >> 1]); }
+
+// words q of own[16] hold tokens 2q, 2q + 1 of this lane's feature
+__device__ __forceinline__ void exchange_pairs(const uint32_t (&own)[16], uint32_t (&y0)[8], uint32_t (&y1)[8]) {
+  const bool odd = threadIdx.x & 1;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const uint32_t other = __shfl_xor_sync(0xffffffffu, odd ? own[q] : own[8 + q], 1);
+    y0[q] = odd ? other : own[q];
+    y1[q] = odd ? own[8 + q] : other;
+  }
+}
+
+// What the step reads for these tokens, requested a block ahead: the residual's pairs, the positions, the rows' weights.
+template <int MODE>
+__device__ __forceinline__ void epi_pairs16_fetch(const EpiParams& p, int t0, int rows, int n, uint32_t (&r)[16]) {
+  if constexpr (MODE == EPI_RESIDUAL) {
+    const uint16_t* src = reinterpret_cast<const uint16_t*>(p.residual) + (int64_t)t0 * p.ld_out + n;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) r[j] = j < rows ? *reinterpret_cast<const uint32_t*>(src + j * (int)p.ld_out) : 0u;
+  } else if constexpr (MODE == EPI_MOE_SCALE) {
+    const uint16_t* src = reinterpret_cast<const uint16_t*>(p.row_w) + t0;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) r[j] = j < rows ? (uint32_t)src[j] << 16 : 0u;
+  } else if constexpr (MODE == EPI_QKV_ROPE) {
+    if (n < p.q_dim + p.kv_dim) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) r[j] = j < rows ? (uint32_t)p.positions[t0 + j] : 0u;
+    }
+  } else if constexpr (MODE == EPI_LAYER) {  // one scale per row (the mixtures)
+    if (p.rowscale != nullptr && p.rs_pitch == 1) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) r[j] = j < rows ? __float_as_uint(p.rowscale[t0 + j]) : 0u;
+    }
+  }
+}
+
+// Gated units: 16 tokens of unit c (in lane pair by lane pair).  Two lane pairs exchange halves, so that a store is 4 bytes, units c & ~1 and c | 1 of a token.
+__device__ __forceinline__ void store_units16(void* out, int ld, int t0, int rows, int c, const float (&x)[16]) {
+  const bool hi = threadIdx.x & 2;
+  uint16_t* dst = reinterpret_cast<uint16_t*>(out) + (int64_t)(t0 + (hi ? 8 : 0)) * ld + (c & ~1);
+  const int left = rows - (hi ? 8 : 0);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const uint32_t a = pack2_rn(x[2 * q], x[2 * q + 1]), b = pack2_rn(x[8 + 2 * q], x[9 + 2 * q]);
+    const uint32_t other = __shfl_xor_sync(0xffffffffu, hi ? a : b, 2);
+    const uint32_t u0 = hi ? other : a, u1 = hi ? b : other;  // tokens 2q, 2q + 1 (+ 8) of the two units
+    if (2 * q < left) *reinterpret_cast<uint32_t*>(dst + 2 * q * ld) = __byte_perm(u0, u1, 0x5410);
+    if (2 * q + 1 < left) *reinterpret_cast<uint32_t*>(dst + (2 * q + 1) * ld) = __byte_perm(u0, u1, 0x7632);
+  }
+}
+
+template <int MODE>
+__device__ __forceinline__ void epi_pairs16(const EpiParams& p, int t0, int rows, int n, const uint32_t (&y0)[8], const uint32_t (&y1)[8], const uint32_t (&r)[16]) {
+  if constexpr (MODE == EPI_STORE || MODE == EPI_RESIDUAL || MODE == EPI_MOE_SCALE) {
+    const int64_t off = (int64_t)t0 * p.ld_out + n;
+    uint32_t o[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const float a = bf16_of(y0, j), b = bf16_of(y1, j);
+      if constexpr (MODE == EPI_RESIDUAL)
+        o[j] = pack2_rn(a + bf16lo(r[j]), b + bf16hi(r[j]));
+      else if constexpr (MODE == EPI_MOE_SCALE)
+        o[j] = pack2_rn(__uint_as_float(r[j]) * a, __uint_as_float(r[j]) * b);
+      else
+        o[j] = __byte_perm(y0[j >> 1], y1[j >> 1], j & 1 ? 0x7632 : 0x5410);
+    }
+    uint16_t* dst = reinterpret_cast<uint16_t*>(p.out) + off;
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+      if (j < rows) *reinterpret_cast<uint32_t*>(dst + j * (int)p.ld_out) = o[j];
+    if constexpr (MODE == EPI_MOE_SCALE) {
+      for (int k = 0; k < p.n_peers; ++k) {  // the same rows on the other ranks (NVLink peer stores)
+        uint16_t* pd = reinterpret_cast<uint16_t*>(p.peer_out[k]) + off;
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          if (j < rows) *reinterpret_cast<uint32_t*>(pd + j * (int)p.ld_out) = o[j];
+      }
+    }
+  } else if constexpr (MODE == EPI_F32) {
+    float* dst = p.out_f32 + (int64_t)t0 * p.ld_out + n;
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+      if (j < rows) *reinterpret_cast<float2*>(dst + j * (int)p.ld_out) = make_float2(bf16_of(y0, j), bf16_of(y1, j));
+  } else if constexpr (MODE == EPI_SWIGLU) {
+    float x[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) x[j] = round_bf16(fast_silu(bf16_of(y0, j))) * bf16_of(y1, j);
+    store_units16(p.out, (int)p.ld_out, t0, rows, n >> 1, x);
+  } else if constexpr (MODE == EPI_QKV_ROPE) {
+    const bool rotate = n < p.q_dim + p.kv_dim, ring = n >= p.q_dim && p.cache_rows != nullptr;  // (the warp's 32 features lie in one head)
+    uint32_t o[16];
+    if (rotate) {
+      const float* tab = p.rope + (n & (kHeadDim - 1));
+      float2 cs[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) cs[j] = j < rows ? __ldg(reinterpret_cast<const float2*>(tab + (int64_t)(int)r[j] * kHeadDim)) : make_float2(0.f, 0.f);
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        float re, im;
+        ref_cmul(bf16_of(y0, j), bf16_of(y1, j), cs[j].x, cs[j].y, re, im);
+        o[j] = pack2_rn(re, im);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) o[j] = __byte_perm(y0[j >> 1], y1[j >> 1], j & 1 ? 0x7632 : 0x5410);
+    }
+    const bool is_q = n < p.q_dim;
+    const int width = is_q ? p.q_dim : p.kv_dim, c = is_q ? n : (rotate ? n - p.q_dim : n - p.q_dim - p.kv_dim);
+    uint16_t* dst = reinterpret_cast<uint16_t*>(is_q ? p.q_out : (rotate ? p.k_out : p.v_out)) + (int64_t)t0 * width + c;
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+      if (j < rows) *reinterpret_cast<uint32_t*>(dst + j * width) = o[j];
+    if (ring) {
+      uint16_t* cache = reinterpret_cast<uint16_t*>(rotate ? p.cache_k : p.cache_v) + c;
+      int row[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) row[j] = j < rows ? p.cache_rows[t0 + j] : -1;
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        if (row[j] >= 0) *reinterpret_cast<uint32_t*>(cache + (int64_t)row[j] * p.kv_dim) = o[j];
+    }
+  }
+}
+
+// EPI_LAYER's bf16 results (bias added and sums rounded before the exchange).  SCALED: the rows have scales; r: those of rs_pitch 1 (the mixtures), fetched ahead.
+template <bool SCALED>
+__device__ __forceinline__ void epi_layer_pairs16(const EpiParams& p, int t0, int rows, int n, const uint32_t (&y0)[8], const uint32_t (&y1)[8], const uint32_t (&r)[16]) {
+  const int step = p.layer;
+  if (step == LAYER_STORE || step == LAYER_RELU2) {
+    uint16_t* dst = reinterpret_cast<uint16_t*>(p.out) + (int64_t)t0 * p.ld_out + n;
+    uint32_t o[16];
+    if (step == LAYER_STORE) {
+      const bool act0 = n < p.n_act, act1 = n + 1 < p.n_act;
+      if (__any_sync(0xffffffffu, act0)) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          const float a = bf16_of(y0, j), b = bf16_of(y1, j);
+          o[j] = pack2_rn(act0 ? a * layer_sigmoid(a) : a, act1 ? b * layer_sigmoid(b) : b);
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) o[j] = __byte_perm(y0[j >> 1], y1[j >> 1], j & 1 ? 0x7632 : 0x5410);
+      }
+    } else {
+      const float* rs0 = nullptr;
+      const float* rs1 = nullptr;
+      if constexpr (SCALED) {
+        rs0 = p.rowscale + (int64_t)t0 * p.rs_pitch + n / p.rs_group;
+        rs1 = p.rowscale + (int64_t)t0 * p.rs_pitch + (n + 1) / p.rs_group;
+      }
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const float a = fmaxf(bf16_of(y0, j), 0.f), b = fmaxf(bf16_of(y1, j), 0.f);
+        float u = a * a, v = b * b;
+        if constexpr (SCALED) {
+          const float f0 = j < rows ? rs0[j * p.rs_pitch] : 0.f, f1 = rs1 == rs0 ? f0 : (j < rows ? rs1[j * p.rs_pitch] : 0.f);
+          u = f0 == 0.f ? 0.f : u * f0;
+          v = f1 == 0.f ? 0.f : v * f1;
+        }
+        o[j] = pack2_rn(u, v);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+      if (j < rows) *reinterpret_cast<uint32_t*>(dst + j * (int)p.ld_out) = o[j];
+    return;
+  }
+  float s[16], x[16];
+  if constexpr (SCALED) {
+    if (p.rs_pitch == 1) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) s[j] = __uint_as_float(r[j]);
+    } else {
+      const float* rs = p.rowscale + (int64_t)t0 * p.rs_pitch + (n >> 1) / p.rs_group;
+#pragma unroll
+      for (int j = 0; j < 16; ++j) s[j] = j < rows ? rs[j * p.rs_pitch] : 0.f;
+    }
+  }
+  if (step == LAYER_GLU) {  // the scale multiplies the expert's INPUT: gate and up, before the clamps
+    const float limit = p.limit, alpha = p.alpha;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      float g = bf16_of(y0, j), u = bf16_of(y1, j);
+      if constexpr (SCALED) g *= s[j], u *= s[j];
+      g = fminf(g, limit);
+      x[j] = g * layer_sigmoid(alpha * g) * (fminf(fmaxf(u, -limit), limit) + 1.f);
+    }
+  } else if (step == LAYER_SWIGLU) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) x[j] = bf16_of(y0, j) * layer_sigmoid(bf16_of(y0, j)) * bf16_of(y1, j);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) x[j] = layer_gelu(bf16_of(y0, j)) * bf16_of(y1, j);
+  }
+  if constexpr (SCALED) {
+    const bool glu = step == LAYER_GLU;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) x[j] = s[j] == 0.f ? 0.f : (glu ? x[j] : x[j] * s[j]);  // (an expert that the token did not choose: nothing of it counts, not even an infinity)
+  }
+  store_units16(p.out, (int)p.ld_out, t0, rows, n >> 1, x);
 }
 
 }  // namespace mb200

@@ -1,13 +1,10 @@
 // C[T, N] = A[T, K] * W[N, K]^T on the 5th-generation tensor cores: tcgen05.mma with TMEM accumulators, TMA-fed.
 //
-// Roofline: tensor pipe (2*T*N*K flops; active 90 % of the cycles at 4096 x 28672 x 4096 under ncu).  Persistent, warp-specialised kernel, one CTA per SM:
-//   warp 0   TMA producer: cp.async.bulk.tensor (128B-swizzled [128 x 64] A tile + [BN x 64] W tile per stage) -> 4- or 6-stage
-//            ring.  For T >= 512 the CTAs run as clusters of two on vertically adjacent tiles: one MMA of 256 rows spans both SMs
-//            (cta_group::2), each CTA fetches its own 128 rows of A and HALF of the W tile (2/3 of the L2 -> SM traffic of the
-//            single-CTA kernel, a ring of six or seven stages)
-//   warp 1   MMA issuer: one elected thread issues tcgen05.mma (M = 128, N = BN, K = 16 x 4 per stage; a pair: M = 256, issued by
-//            its first CTA for both); tcgen05.commit releases the shared-memory stage (in both CTAs of a pair) and, after the last
-//            k-block, publishes the accumulator
+// Here: the PTX wrappers, the tensor maps and the kernel for short prompts, whose tiles belong to one CTA each; from a few hundred rows on pairs of CTAs
+// share MMAs (gemm_pair.cuh).  Persistent, warp-specialised, one CTA per SM:
+//   warp 0   TMA producer: cp.async.bulk.tensor (128B-swizzled [128 x 64] A tile + [BN x 64] W tile per stage) -> 4- or 6-stage ring
+//   warp 1   MMA issuer: one elected thread issues tcgen05.mma (M = 128, N = BN, K = 16 x 4 per stage); tcgen05.commit releases the
+//            shared-memory stage and, after the last k-block, publishes the accumulator
 //   warps 2-5 epilogue: one thread per output row reads the fp32 accumulator out of TMEM 32 columns at a time (two TMEM
 //            buffers, so the MMAs of the next tile overlap this one's epilogue; two register buffers, so the next tcgen05.ld
 //            overlaps this chunk's arithmetic) and runs the row-chunk epilogues of epilogue.cuh (bf16 rounding, then RoPE +
@@ -41,11 +38,11 @@ constexpr int TG_A_BYTES = TG_BM * TG_BK * 2;
 // memory -- accumulator row i depends on A row i only, and rows >= T are never stored.  The stage shrinks to (TA + BN) * 128
 // bytes, so the ring gets deep enough (16-20 stages) to keep a whole SM's share of HBM bandwidth in flight: those launches are
 // weight-streaming GEMMs, bound by HBM, with BN chosen by the launcher to give every SM at most one (equal) tile per round.
-// CL = 2: a pair of CTAs (see tc_gemm_body); a CTA's stage holds half of the W tile.  EXTRA: shared memory an epilogue needs beside the ring.
-template <int BN, int TA = 128, int CL = 1, int EXTRA = 0>
+// EXTRA: shared memory an epilogue needs beside the ring.
+template <int BN, int TA = 128, int EXTRA = 0>
 struct TgCfg {
   static constexpr int kABytes = TA * TG_BK * 2;
-  static constexpr int kBBytes = BN / CL * TG_BK * 2;
+  static constexpr int kBBytes = BN * TG_BK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
   // The MMA always reads M = 128 rows (16 KB) from a stage's A base; with a short A box that runs on into the stage's W tile
   // (harmless: accumulator row i depends on A row i only) and, in the LAST stage, past it when the stage is smaller than 16 KB.
@@ -65,12 +62,12 @@ struct TgCfg {
   // qkv 24.0 -> 21.3 us, down 39.5 -> 36.8 us; only the 1.3 GB lm head loses 5 %) -- a successor's CTA, which starts when the
   // predecessor's CTA on its SM exits, has its first ring filled sooner, and other decode kernels' CTAs fit beside it.
   static constexpr int kShortRingStages = (100 * 1024) / kStageBytes;
-  static constexpr int kStages = CL == 2 ? (kMaxStages > 8 ? 8 : kMaxStages) : (TA < 128 || BN < 128) ? (kShortRingStages < 3 ? 3 : (kShortRingStages > kMaxStages ? kMaxStages : kShortRingStages))
+  static constexpr int kStages = (TA < 128 || BN < 128) ? (kShortRingStages < 3 ? 3 : (kShortRingStages > kMaxStages ? kMaxStages : kShortRingStages))
                                                         : (BN == 128 ? 6 : 4);
   static constexpr int kSmem = kStages * kStageBytes + kSlack + 1024 /*align*/ + 512 /*barriers*/ + EXTRA;
   static constexpr int kTmemCols = 2 * BN <= 32 ? 32 : (2 * BN <= 64 ? 64 : (2 * BN <= 128 ? 128 : (2 * BN <= 256 ? 256 : 512)));  // 2 accumulators
   // Instruction descriptor (cute::UMMA::InstrDescriptor): D = F32, A = B = BF16, both K-major, N >> 3 at bit 17, M >> 4 at bit 24
-  static constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(CL * TG_BM >> 4) << 24);
+  static constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TG_BM >> 4) << 24);
 };
 template <int MODE>
 constexpr int kEpiSmem = MODE == EPI_LAYER ? 4 * 4096 : 0;  // 4 KB per epilogue warp to turn fp32 blocks (epi_layer32_f32)
@@ -81,15 +78,7 @@ struct TcGemmParams {
   // grouped, experts packed in ONE matrix (layered decoders): expert e's weights start w_n * e rows and w_k * e columns into the single
   // tensor map; w_n = w_k = 0: a tensor map per expert
   int w_n = 0, w_k = 0;
-  // pairs of 256-wide tiles, dense (plan_pairs): work items are whole tile pairs and at the end the last `cut_pairs` pairs, each cut into `cut`
-  // parts along k
-  int cut_pairs = 0, cut = 1;
-  float* partials = nullptr;   // [(cut - 1) * cut_pairs][2 CTAs][256 / 4][128 rows] float4: what the parts but the first leave for it
-  unsigned* flags = nullptr;   // [(cut - 1) * cut_pairs * 2], zero between launches
 };
-constexpr unsigned CUT_GIVEN_UP = 2u;  // a flag: 0, 1 (the part is there), or this
-constexpr int TG_MAX_CUTS = 56;  // (cut - 1) * cut_pairs at most: 256 KB each
-constexpr size_t TG_CUT_BYTES = (size_t)TG_MAX_CUTS * 2 * TG_BM * 256 * sizeof(float);
 
 // ---- PTX wrappers ---------------------------------------------------------------------------------
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1) {
@@ -102,6 +91,12 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
 __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
   asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(smem_dst)),
                "l"(map), "r"(bar), "r"(c0), "r"(c1)
+               : "memory");
+}
+// `bytes` from global memory to this CTA's shared memory, both 16-byte aligned
+__device__ __forceinline__ void bulk_load(void* smem_dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(smem_dst)), "l"(src), "r"(bytes),
+               "r"(smem_u32(bar))
                : "memory");
 }
 __device__ __forceinline__ uint32_t cluster_ctarank() {
@@ -203,33 +198,59 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
   return (uint64_t)((smem_addr & 0x3ffff) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
 
-// CL = 2: clusters of two CTAs that share MMAs (cta_group::2) on vertically adjacent tiles (same W columns, consecutive 128-row blocks).  A CTA
-// holds its 128 rows of A and half of the [256 x 64] W tile, the MMA reads both shared memories: 32 KB per CTA and k-block out of L2 where the
-// single-CTA kernel takes 48 KB (at T = 4096 it pulls ~20 TB/s), and a stage of 32 KB leaves room for a ring of seven.  Both CTAs' copies
-// count on the first CTA's full[] barrier; its MMA thread issues for both and its commits free the stage, and publish the accumulator, in both;
-// both CTAs' epilogues release an accumulator on the first CTA's tmem_empty[].  No copy is multicast: each tile is read by the CTA that holds it.
-// A last row of tiles without a neighbour below is a pair whose second tile lies past the end of A: zeros, read from nowhere, never stored.  (The
-// pair's MMA of 128 rows, 64 in each CTA, takes as long as that of 256: with it on such rows, scoring 1102 tokens was 2186 us against 2006.)
-// Measured against single-CTA MMAs whose W tile each CTA copied into both, ring of four: 4096-token prompt 1728 -> 1707 us a layer, 1102 tokens
-// through a 131072-wide head 2064 -> 2006, 4096 tokens through two layers of width 4096 3995 -> 3854; eight experts of ~512 rows, half of them with
-// a fifth tile, 1679 -> 1736 (there the two CTAs of a lone row took two column tiles).
-//
+// Tile order.  The persistent CTAs (pairs) take tiles t = cta, cta + n_cta, ...: at any moment ~n_cta consecutive tile ids are in flight,
+// in lock step through K.  With few m units (T <= 4096: the whole A matrix fits the 126 MB L2) the walk is m-fastest: the CTAs
+// that share a W tile run together.  With many (a 32 x 1024-token prefill: A = 335 MB; a Mixtral prefill: 277 MB of gathered rows)
+// m-fastest makes every CTA stream its own A tile from DRAM once per n tile -- measured with ncu: 32.7 GB of DRAM reads for a
+// grouped gate/up GEMM whose operands total 2.2 GB, 4.9 TB/s, DRAM-bound at 1.15 PFLOP/s.  There the in-flight set is shaped as a
+// GM x GN block instead (GM m units share each W tile, GN n tiles share each A tile): DRAM traffic per tile drops ~4x.
+template <int kGM, int kGN>
+__device__ __forceinline__ void tile_mn(int tile, int num_m, int num_n, int& mu, int& nt) {
+  if (num_m <= 16) {
+    mu = tile % num_m;
+    nt = tile / num_m;
+    return;
+  }
+  const int per_row = kGN * num_m, rows_full = num_n / kGN;  // an "n-block row": all m units x kGN n tiles
+  int nb, r, gn;
+  if (tile < rows_full * per_row) {
+    nb = tile / per_row;
+    r = tile % per_row;
+    gn = kGN;
+  } else {
+    nb = rows_full;
+    r = tile - rows_full * per_row;
+    gn = num_n - rows_full * kGN;
+  }
+  const int blk = kGM * gn, mb_full = num_m / kGM;
+  int mblk, q, gm;
+  if (r < mb_full * blk) {
+    mblk = r / blk;
+    q = r % blk;
+    gm = kGM;
+  } else {
+    mblk = mb_full;
+    q = r - mb_full * blk;
+    gm = num_m - mb_full * kGM;
+  }
+  mu = mblk * kGM + q % gm;
+  nt = nb * kGN + q / gm;
+}
+
 // GROUPED = true (mixture of experts, csrc/moe.cuh): the A rows are the (token, expert) pairs sorted by expert, every expert's
 // segment padded to a multiple of TA rows; m tile i covers rows plan.tile_row0[i] .. + TA of expert plan.tile_expert[i], whose
 // weight matrix has its own tensor map (map_w[expert]).  The number of m tiles is DEVICE data (no host sync after routing).
-constexpr int MOE_PLAN_HEADER = 64;  // int32 words: [0] m tiles of this rank, [1] padded rows in total, [2] tile capacity, [6] tile pairs, [8..] segment starts
-// after the header: tile_expert[cap], tile_row0[cap], pair_expert[cap], pair_info[cap] (cap = plan[2]).  A PAIR is two vertically
-// adjacent m tiles of ONE expert (or a single last tile: bit 30 of pair_info clear), the unit of the 2-CTA cluster variant.
-constexpr int MOE_PAIR_SECOND = 1 << 30;
+constexpr int MOE_PLAN_HEADER = 64;  // int32 words: [0] m tiles of this rank, [1] padded rows in total, [2] tile capacity, [6] token tiles of pairs of CTAs, [8..] segment starts
+// after the header: tile_expert[cap], tile_row0[cap], pair_expert[cap], pair_info[cap] (cap = plan[2]).  The last two list the token tiles of
+// gemm_pair.cuh: info = first row (a multiple of 32) | width / 32.
 constexpr int MOE_MAX_EXPERTS = 16;  // tensor maps travel as kernel parameters (128 B each)
 struct MoeWeightMaps {
   CUtensorMap m[MOE_MAX_EXPERTS];
 };
 
-template <int MODE, int CL, int BN, int TA, bool GROUPED>
+template <int MODE, int BN, int TA, bool GROUPED>
 __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUtensorMap* map_w_base, const TcGemmParams& p, const int32_t* plan) {
-  static_assert(TA == 128 || CL == 1, "small-batch variant is single-CTA");
-  using Cfg = TgCfg<BN, TA, CL, kEpiSmem<MODE>>;
+  using Cfg = TgCfg<BN, TA, kEpiSmem<MODE>>;
   constexpr int TG_STAGES = Cfg::kStages, TG_STAGE_BYTES = Cfg::kStageBytes, TG_TMEM_COLS = Cfg::kTmemCols;
   constexpr int TG_A_BYTES = Cfg::kABytes;  // shadows the 128-row constant
   constexpr int TG_BN = BN;
@@ -241,86 +262,15 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
   uint64_t* tmem_full = empty + TG_STAGES;  // [2]
   uint64_t* tmem_empty = tmem_full + 2;     // [2]
   uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
-  uint64_t* cut_full = tmem_empty + 3;  // copies of another part's sums (kCuts)
-  volatile uint32_t* cut_lost = tmem_base_slot + 1;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rank = CL > 1 ? (int)cluster_ctarank() : 0;
-  const int cta = (int)blockIdx.x / CL, n_cta = (int)gridDim.x / CL;  // cluster index / clusters in the grid
-  // a cluster walks "super tiles" of CL vertically adjacent tiles; rows past T read as zeros (TMA) and are never stored
-  // grouped: m units are the plan's tiles (single CTA) or tile pairs (cluster of two)
-  constexpr bool kCuts = CL == 2 && BN == 256 && !GROUPED;
-  static_assert(!kCuts || TG_STAGES * TG_STAGE_BYTES >= TG_BM * BN * 4, "another part's sums fit in the ring");
+  const int cta = (int)blockIdx.x, n_cta = (int)gridDim.x;
   const int num_n = p.N / TG_BN, num_k = p.K / TG_BK;
-  const int num_m = GROUPED ? (CL > 1 ? plan[6] : plan[0]) : ((p.T + TG_BM - 1) / TG_BM + CL - 1) / CL;
-  const int whole = num_m * num_n - (kCuts ? p.cut_pairs : 0), num_tiles = whole + (kCuts ? p.cut * p.cut_pairs : 0);
-  const int32_t* tile_expert = GROUPED ? plan + MOE_PLAN_HEADER + (CL > 1 ? 2 * plan[2] : 0) : nullptr;
+  const int num_m = GROUPED ? plan[0] : (p.T + TG_BM - 1) / TG_BM;  // rows past T read as zeros (TMA) and are never stored
+  const int num_tiles = num_m * num_n;
+  const int32_t* tile_expert = GROUPED ? plan + MOE_PLAN_HEADER : nullptr;
   const int32_t* tile_row0 = GROUPED ? tile_expert + plan[2] : nullptr;
-  // Tile order.  The persistent CTAs take tiles t = cta, cta + n_cta, ...: at any moment ~n_cta consecutive tile ids are in flight,
-  // in lock step through K.  With few m units (T <= 4096: the whole A matrix fits the 126 MB L2) the walk is m-fastest: the CTAs
-  // that share a W tile run together.  With many (a 32 x 1024-token prefill: A = 335 MB; a Mixtral prefill: 277 MB of gathered rows)
-  // m-fastest makes every CTA stream its own A tile from DRAM once per n tile -- measured with ncu: 32.7 GB of DRAM reads for a
-  // grouped gate/up GEMM whose operands total 2.2 GB, 4.9 TB/s, DRAM-bound at 1.15 PFLOP/s.  There the in-flight set is shaped as a
-  // GM x GN block instead (GM m units share each W tile, GN n tiles share each A tile): DRAM traffic per tile drops ~4x.
-  constexpr int kGM = CL > 1 ? 8 : 12, kGN = CL > 1 ? 9 : 12;
-  auto tile_mn = [&](int tile, int& mu, int& nt) {
-    if (num_m <= 16) {
-      mu = tile % num_m;
-      nt = tile / num_m;
-      return;
-    }
-    const int per_row = kGN * num_m, rows_full = num_n / kGN;  // an "n-block row": all m units x kGN n tiles
-    int nb, r, gn;
-    if (tile < rows_full * per_row) {
-      nb = tile / per_row;
-      r = tile % per_row;
-      gn = kGN;
-    } else {
-      nb = rows_full;
-      r = tile - rows_full * per_row;
-      gn = num_n - rows_full * kGN;
-    }
-    const int blk = kGM * gn, mb_full = num_m / kGM;
-    int mblk, q, gm;
-    if (r < mb_full * blk) {
-      mblk = r / blk;
-      q = r % blk;
-      gm = kGM;
-    } else {
-      mblk = mb_full;
-      q = r - mb_full * blk;
-      gm = num_m - mb_full * kGM;
-    }
-    mu = mblk * kGM + q % gm;
-    nt = nb * kGN + q / gm;
-  };
-  struct Item {
-    int mu, m0, n0, kb0, kb1;
-    int part, slot;  // part of a cut pair (0: the owner, which adds the others' sums), -1: not cut
-  };
-  auto item_of = [&](int tile) {
-    Item it;
-    it.kb0 = 0, it.kb1 = num_k, it.part = -1, it.slot = 0;
-    int t = tile, nt;
-    if (kCuts && t >= whole) {
-      const CutItem c = cut_item(t - whole, p.cut, p.cut_pairs);
-      it.part = c.part;
-      it.slot = c.slot;
-      it.kb0 = num_k * it.part / p.cut;
-      it.kb1 = num_k * (it.part + 1) / p.cut;
-      t = whole + it.slot;
-    }
-    tile_mn(t, it.mu, nt);
-    it.n0 = nt * TG_BN;
-    if (GROUPED) {
-      const int info = tile_row0[it.mu];
-      it.m0 = info & (MOE_PAIR_SECOND - 1);
-      if (CL > 1 && rank == 1) it.m0 = (info & MOE_PAIR_SECOND) != 0 ? it.m0 + TG_BM : p.T;  // p.T: past the last row
-    } else {
-      it.m0 = (it.mu * CL + rank) * TG_BM;
-    }
-    return it;
-  };
+  auto m0_of = [&](int mu) { return GROUPED ? tile_row0[mu] : mu * TG_BM; };
   const CUtensorMap& map_w = *map_w_base;
 
   if (threadIdx.x == 0) {
@@ -330,20 +280,15 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&tmem_full[i], 1);
-      mbar_init(&tmem_empty[i], 4 * CL);  // one arrive per epilogue warp
+      mbar_init(&tmem_empty[i], 4);  // one arrive per epilogue warp
     }
-    mbar_init(cut_full, 1);
-    *cut_lost = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
     if (!GROUPED) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
   }
-  if (warp == 1) tmem_alloc<CL>(tmem_base_slot, TG_TMEM_COLS);
+  if (warp == 1) tmem_alloc(tmem_base_slot, TG_TMEM_COLS);
   tc_fence_before();
-  if (CL > 1)
-    cluster_sync_all();  // the peer's barriers must be initialised before any copy or commit reaches them
-  else
-    __syncthreads();
+  __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_base_slot;
 
@@ -352,45 +297,33 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
     if (lane == 0) {
       uint32_t it = 0;
       for (int tile = cta; tile < num_tiles; tile += n_cta) {
-        const Item w = item_of(tile);
-        const int m0 = w.m0, n0 = w.n0;
-        const int expert = GROUPED ? tile_expert[w.mu] : 0;
+        int mu, nt;
+        tile_mn<12, 12>(tile, num_m, num_n, mu, nt);
+        const int m0 = m0_of(mu), n0 = nt * TG_BN;
+        const int expert = GROUPED ? tile_expert[mu] : 0;
         const bool packed = GROUPED && (p.w_n | p.w_k) != 0;
         const CUtensorMap* wmap = map_w_base + (packed ? 0 : expert);
         const int wr = n0 + (packed ? expert * p.w_n : 0), wc = packed ? expert * p.w_k : 0;
-        for (int kb = w.kb0; kb < w.kb1; ++kb, ++it) {
+        for (int kb = 0; kb < num_k; ++kb, ++it) {
           const uint32_t s = it % TG_STAGES, par = (it / TG_STAGES) & 1;
           mbar_wait(&empty[s], par ^ 1, 11, it);
           uint8_t* sa = smem + s * TG_STAGE_BYTES;
-          if (CL > 1) {
-            // the pair's four tiles count on the first CTA's barrier (the other CTA's may land before it is armed: the count goes negative)
-            if (rank == 0) mbar_arrive_expect_tx(&full[s], CL * TG_STAGE_BYTES);
-            const uint32_t bar = cluster_first(&full[s]);
-            tma_load_2d_pair(sa, &map_a, bar, kb * TG_BK, m0);
-            tma_load_2d_pair(sa + TG_A_BYTES, wmap, bar, wc + kb * TG_BK, wr + rank * (TG_BN / CL));
-          } else {
-            mbar_arrive_expect_tx(&full[s], TG_STAGE_BYTES);
-            tma_load_2d(sa, &map_a, &full[s], kb * TG_BK, m0);
-            tma_load_2d(sa + TG_A_BYTES, wmap, &full[s], wc + kb * TG_BK, wr);
-          }
+          mbar_arrive_expect_tx(&full[s], TG_STAGE_BYTES);
+          tma_load_2d(sa, &map_a, &full[s], kb * TG_BK, m0);
+          tma_load_2d(sa + TG_A_BYTES, wmap, &full[s], wc + kb * TG_BK, wr);
         }
       }
     }
   } else if (warp == 1) {
-    // ================= MMA issuer (one thread, for both CTAs of a pair) =================
-    if (lane == 0 && rank == 0) {
+    // ================= MMA issuer (one thread) =================
+    if (lane == 0) {
       uint32_t it = 0, acc_it = 0;
       for (int tile = cta; tile < num_tiles; tile += n_cta, ++acc_it) {
         const uint32_t acc = acc_it & 1, acc_par = (acc_it >> 1) & 1;
         mbar_wait(&tmem_empty[acc], acc_par ^ 1, 12, acc_it);  // the epilogue has drained this accumulator buffer
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * TG_BN;
-        int kb0 = 0, kb1 = num_k;
-        if (kCuts) {
-          const Item w = item_of(tile);
-          kb0 = w.kb0, kb1 = w.kb1;
-        }
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
+        for (int kb = 0; kb < num_k; ++kb, ++it) {
           const uint32_t s = it % TG_STAGES, par = (it / TG_STAGES) & 1;
           mbar_wait(&full[s], par, 13, it);
           tc_fence_after();
@@ -398,34 +331,20 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
           const uint64_t adesc = umma_desc_sw128(a_addr), bdesc = umma_desc_sw128(a_addr + TG_A_BYTES);
 #pragma unroll
           for (int k = 0; k < TG_BK / 16; ++k)  // +32 bytes (= 2 in 16-byte units) per K = 16 step inside the 128-byte swizzled row
-            if constexpr (CL > 1)
-              umma_bf16_pair(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), kUmmaIdesc, (kb > kb0 || k) ? 1u : 0u);
-            else
-              umma_bf16(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), kUmmaIdesc, (kb > kb0 || k) ? 1u : 0u);
-          if (CL > 1)  // frees the stage in both CTAs when these MMAs have read it
-            umma_commit_pair(&empty[s]);
-          else
-            umma_commit(&empty[s]);
+            umma_bf16(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), kUmmaIdesc, (kb > 0 || k) ? 1u : 0u);
+          umma_commit(&empty[s]);
         }
-        if (CL > 1)
-          umma_commit_pair(&tmem_full[acc]);  // accumulator complete, in both CTAs
-        else
-          umma_commit(&tmem_full[acc]);
+        umma_commit(&tmem_full[acc]);
       }
     }
   } else {
     // ================= epilogue warps 2..5: TMEM lanes 32*(warp%4) .. +31 =================
     const int lane_base = (warp & 3) * 32;
-    auto release = [&](uint32_t acc) {  // the MMA thread may overwrite this accumulator buffer
-      if (CL > 1)
-        mbar_arrive_cluster(cluster_first(&tmem_empty[acc]));
-      else
-        mbar_arrive(&tmem_empty[acc]);
-    };
     uint32_t acc_it = 0;
     for (int tile = cta; tile < num_tiles; tile += n_cta, ++acc_it) {
-      const Item w = item_of(tile);
-      const int m0 = w.m0, n0 = w.n0;
+      int mu, nt;
+      tile_mn<12, 12>(tile, num_m, num_n, mu, nt);
+      const int m0 = m0_of(mu), n0 = nt * TG_BN;
       const uint32_t acc = acc_it & 1, acc_par = (acc_it >> 1) & 1;
       mbar_wait(&tmem_full[acc], acc_par, 14, acc_it);
       tc_fence_after();
@@ -434,98 +353,6 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
       // two register buffers: the TMEM load of chunk c+1 is in flight while chunk c goes through the epilogue
       const uint32_t trow = tmem_base + ((uint32_t)lane_base << 16) + acc * TG_BN;
       uint32_t va[32], vb[32];
-      const int row = lane_base + lane;
-      bool lost = false;  // a part of this pair never came
-      auto add_part = [&](int c, uint32_t (&v)[32]) {  // columns 32 c .. + 31 of the part that lies in the ring: quads of 128 rows side by side
-        const float4* src = reinterpret_cast<const float4*>(smem) + row;
-        const float none = __uint_as_float(0x7fffffffu);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const float4 x = lost ? make_float4(none, none, none, none) : src[(c * 8 + q) * TG_BM];
-          v[4 * q] = __float_as_uint(__uint_as_float(v[4 * q]) + x.x);
-          v[4 * q + 1] = __float_as_uint(__uint_as_float(v[4 * q + 1]) + x.y);
-          v[4 * q + 2] = __float_as_uint(__uint_as_float(v[4 * q + 2]) + x.z);
-          v[4 * q + 3] = __float_as_uint(__uint_as_float(v[4 * q + 3]) + x.w);
-        }
-      };
-      if constexpr (kCuts) {
-        if (w.part > 0) {
-          // a later part of a cut pair: its fp32 sums go to the owner, column quads of 128 rows side by side
-          const int at = ((w.part - 1) * p.cut_pairs + w.slot) * 2 + rank;
-          float4* dst = reinterpret_cast<float4*>(p.partials) + (size_t)at * (TG_BN / 4) * TG_BM + row;
-#pragma unroll 1
-          for (int c = 0; c < TG_BN / 32; ++c) {
-            tmem_ld_32x32b_x32(trow + c * 32, va);
-#pragma unroll
-            for (int q = 0; q < 8; ++q)
-              dst[(c * 8 + q) * TG_BM] = make_float4(__uint_as_float(va[4 * q]), __uint_as_float(va[4 * q + 1]), __uint_as_float(va[4 * q + 2]), __uint_as_float(va[4 * q + 3]));
-          }
-          asm volatile("fence.proxy.async;" ::: "memory");
-          __threadfence();
-          asm volatile("bar.sync 2, 128;" ::: "memory");
-          if (threadIdx.x == 64) {
-            __threadfence();
-            if (atomicExch(p.flags + at, 1u) == CUT_GIVEN_UP) atomicExch(p.flags + at, 0u);
-          }
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) release(acc);
-          continue;
-        }
-        if (w.part == 0) {
-          // The owner: the other parts lie on lower clusters (cut_item).  This CTA's ring is free (its last MMA has completed): each part's 128 KB
-          // come in by bulk copies and are added in the order of k -- all but the last into the accumulator, the last in the epilogue below.
-          // (Loaded 128 bytes per thread and column chunk instead, a launch paid ~12 us of L2 latency here.)
-          for (int o = 0; o < p.cut - 1; ++o) {
-            if (threadIdx.x == 64) {
-              const int at = (o * p.cut_pairs + w.slot) * 2 + rank;
-              unsigned spins = 0, there = 0u;
-              while ((there = ld_acquire_u32(p.flags + at)) == 0u && ++spins < MB200_WATCHDOG_SPINS) {
-              }
-              if (there == 0u) {  // gives up: the flag says so to a part that comes after all and puts it back; the pair's results are NaN
-                there = atomicCAS(p.flags + at, 0u, CUT_GIVEN_UP);
-                __threadfence();
-              }
-              if (there == 0u) {
-                printf("[mb200 watchdog] cluster %d: part %d of pair %d never came\n", cta, o + 1, w.slot);
-                *cut_lost = 1u;
-              } else {
-                p.flags[at] = 0u;  // ready for the next launch
-                if (!lost) {
-                  asm volatile("fence.proxy.async;" ::: "memory");  // written with ordinary stores, read by the copy engine
-                  constexpr uint32_t kBytes = TG_BM * TG_BN * 4, kCopy = 32768;
-                  mbar_arrive_expect_tx(cut_full, kBytes);
-                  const uint8_t* src = reinterpret_cast<const uint8_t*>(p.partials) + (size_t)at * kBytes;
-#pragma unroll
-                  for (uint32_t i = 0; i < kBytes; i += kCopy)
-                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(smem + i)), "l"(src + i),
-                                 "r"(kCopy), "r"(smem_u32(cut_full))
-                                 : "memory");
-                }
-              }
-            }
-            asm volatile("bar.sync 2, 128;" ::: "memory");
-            lost = *cut_lost != 0u;
-            if (lost) continue;  // the other parts' flags still go back to zero
-            mbar_wait(cut_full, o & 1, 15, o);
-            if (o + 1 < p.cut - 1) {
-#pragma unroll 1
-              for (int c = 0; c < TG_BN / 32; ++c) {
-                tmem_ld_32x32b_x32(trow + c * 32, va);
-                add_part(c, va);
-                tmem_st_32x32b_x32(trow + c * 32, va);
-              }
-              asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-              asm volatile("bar.sync 2, 128;" ::: "memory");  // everybody has read: the next part may come
-            }
-          }
-        }
-      }
-      auto plus = [&](int c, uint32_t (&v)[32]) {
-        if constexpr (kCuts) {
-          if (w.part == 0) add_part(c, v);
-        }
-      };
       tmem_ld_32x32b_x32_nowait(trow, va);
       if constexpr (MODE == EPI_LOGPROB) {
         const bool live = t < p.T;
@@ -538,7 +365,6 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
 #pragma unroll
           for (int j = 0; j < 32; ++j) vb[j] = va[j];
           if (c + 1 < TG_BN / 32) tmem_ld_32x32b_x32_nowait(trow + (c + 1) * 32, va);
-          plus(c, vb);
           if (live) epi_logprob32(p.epi, t, n0 + c * 32, vb, tgt, keep, m, sum);
           if (c & 1) {
             if (tgt >= 0) p.epi.partial[(int64_t)t * (p.N / 64) + (n0 + c * 32) / 64] = make_float2(m, sum);
@@ -562,7 +388,6 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
 #pragma unroll
           for (int j = 0; j < 32; ++j) vb[j] = va[j];
           if (c + 1 < TG_BN / 32) tmem_ld_32x32b_x32_nowait(trow + (c + 1) * 32, va);
-          plus(c, vb);
           chunk(n0 + c * 32, vb);
         }
       } else if constexpr (TG_BN == 32) {
@@ -573,38 +398,33 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
         for (int c = 0; c < TG_BN / 32; c += 2) {
           tmem_wait_ld();
           tmem_ld_32x32b_x32_nowait(trow + (c + 1) * 32, vb);
-          plus(c, va);
           if (t < p.T) epi_chunk32<MODE>(p.epi, t, n0 + c * 32, va);
           tmem_wait_ld();
           if (c + 2 < TG_BN / 32) tmem_ld_32x32b_x32_nowait(trow + (c + 2) * 32, va);
-          plus(c + 1, vb);
           if (t < p.T) epi_chunk32<MODE>(p.epi, t, n0 + (c + 1) * 32, vb);
         }
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) release(acc);
+      if (lane == 0) mbar_arrive(&tmem_empty[acc]);
     }
   }
   tc_fence_before();
-  if (CL > 1)
-    cluster_sync_all();  // the peer's last commits and arrivals still reach this CTA's barriers, its MMAs this CTA's memory
-  else
-    __syncthreads();
-  if (warp == 1) tmem_dealloc<CL>(tmem_base, TG_TMEM_COLS);
+  __syncthreads();
+  if (warp == 1) tmem_dealloc(tmem_base, TG_TMEM_COLS);
 }
 
-template <int MODE, int CL, int BN, int TA = 128>
+template <int MODE, int BN, int TA = 128>
 __global__ void __launch_bounds__(TG_THREADS, 1)
     gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const TcGemmParams p) {
-  tc_gemm_body<MODE, CL, BN, TA, false>(map_a, &map_w, p, nullptr);
+  tc_gemm_body<MODE, BN, TA, false>(map_a, &map_w, p, nullptr);
 }
 
-template <int MODE, int CL, int BN, int TA>
+template <int MODE, int BN, int TA>
 __global__ void __launch_bounds__(TG_THREADS, 1)
     gemm_tcgen05_grouped_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ MoeWeightMaps maps_w, const TcGemmParams p,
                                 const int32_t* __restrict__ plan) {
-  tc_gemm_body<MODE, CL, BN, TA, true>(map_a, maps_w.m, p, plan);
+  tc_gemm_body<MODE, BN, TA, true>(map_a, maps_w.m, p, plan);
 }
 
 // ---- host: tensor maps (driver API through the runtime's entry-point lookup, no libcuda link dependency) ----
@@ -659,68 +479,22 @@ inline int tcgen05_forced_bn() {
   return e != nullptr ? atoi(e) : 0;
 }
 
-// How a dense launch of pairs (256 x 256 outputs an item, `units` pairs on the chip) ends: cut_plan.  The parts' fp32 sums meet in the first part's
-// epilogue, in the order of k.
-inline void plan_pairs(TcGemmParams& p, int units, void* scratch, unsigned* flags) {
-  p.cut_pairs = 0;
-  p.cut = 1;
-  if (scratch == nullptr) return;
-  const CutPlan c = cut_plan((long long)ceil_div(p.T, 2 * TG_BM) * (p.N / 256), p.K / TG_BK, units, TG_MAX_CUTS);
-  p.cut_pairs = c.cut_pairs;
-  p.cut = c.cut;
-  p.partials = reinterpret_cast<float*>(scratch);
-  p.flags = flags;
-}
-
-// Whether pairs of 256-wide tiles (and, for k of at least 8192, the parts they would be cut into) fill half of the chip's `units` pairs
-inline bool pairs_fill(int64_t T, int64_t N, int64_t K, int units, bool cuts) {
-  if (T <= TG_BM || N % 256 != 0 || K % TG_BK != 0) return false;
-  TcGemmParams p;
-  p.T = (int)T;
-  p.N = (int)N;
-  p.K = (int)K;
-  plan_pairs(p, units, cuts && K >= 8192 ? &p : nullptr, nullptr);  // (any scratch: how would it be cut?)
-  return 2 * (ceil_div(T, 2 * TG_BM) * (p.N / 256) + (p.cut - 1) * p.cut_pairs) >= units;
-}
-
 template <int MODE, int BN>
-int launch_gemm_tcgen05_bn(const GemmParams& g, bool pair, int sms, cudaStream_t stream, void* scratch, unsigned* flags) {
-  constexpr int kSmem = TgCfg<BN, 128, 1, kEpiSmem<MODE>>::kSmem, kSmemPair = TgCfg<BN, 128, 2, kEpiSmem<MODE>>::kSmem;
+int launch_gemm_tcgen05_bn(const GemmParams& g, int sms, cudaStream_t stream) {
+  constexpr int kSmem = TgCfg<BN, 128, kEpiSmem<MODE>>::kSmem;
   CUtensorMap map_a, map_w;
   int rc = make_tensor_map_2d(&map_a, g.a, g.T, g.K, TG_BM);
   if (rc) return rc;
-  rc = make_tensor_map_2d(&map_w, g.w, g.N, g.K, pair ? BN / 2 : BN);
+  rc = make_tensor_map_2d(&map_w, g.w, g.N, g.K, BN);
   if (rc) return rc;
   TcGemmParams p;
   p.T = g.T;
   p.N = g.N;
   p.K = g.K;
   p.epi = g.epi;
-  if (pair) {
-    const int pairs = sms / 2;
-    int supers = ceil_div(ceil_div(g.T, TG_BM), 2) * (g.N / BN);
-    if (BN == 256) plan_pairs(p, pairs, scratch, flags);
-    if (p.cut_pairs > 0) supers = pairs;  // the last round is full
-    MB_CHECK_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<MODE, 2, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemPair));
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2u * (unsigned)(supers < pairs ? supers : pairs));
-    cfg.blockDim = dim3(TG_THREADS);
-    cfg.dynamicSmemBytes = kSmemPair;
-    cfg.stream = stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = 2;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    MB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<MODE, 2, BN>, map_a, map_w, p));
-    MB_CHECK_LAUNCH("gemm_tcgen05_kernel<cluster 2>");
-    return MB200_OK;
-  }
   const int tiles = ceil_div(g.T, TG_BM) * (g.N / BN);
-  MB_CHECK_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<MODE, 1, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
-  gemm_tcgen05_kernel<MODE, 1, BN><<<tiles < sms ? tiles : sms, TG_THREADS, kSmem, stream>>>(map_a, map_w, p);
+  MB_CHECK_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<MODE, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+  gemm_tcgen05_kernel<MODE, BN><<<tiles < sms ? tiles : sms, TG_THREADS, kSmem, stream>>>(map_a, map_w, p);
   MB_CHECK_LAUNCH("gemm_tcgen05_kernel");
   return MB200_OK;
 }
@@ -762,8 +536,8 @@ int launch_gemm_tcgen05_small_bn(const GemmParams& g, int sms, cudaStream_t stre
   p.K = g.K;
   p.epi = g.epi;
   const int tiles = g.N / BN;
-  MB_CHECK_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<MODE, 1, BN, TA>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
-  gemm_tcgen05_kernel<MODE, 1, BN, TA><<<tiles < sms ? tiles : sms, TG_THREADS, Cfg::kSmem, stream>>>(map_a, map_w, p);
+  MB_CHECK_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<MODE, BN, TA>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
+  gemm_tcgen05_kernel<MODE, BN, TA><<<tiles < sms ? tiles : sms, TG_THREADS, Cfg::kSmem, stream>>>(map_a, map_w, p);
   MB_CHECK_LAUNCH("gemm_tcgen05_kernel<small batch>");
   return MB200_OK;
 }
@@ -779,46 +553,8 @@ int launch_gemm_tcgen05_small_ta(const GemmParams& g, int sms, cudaStream_t stre
   }
 }
 
-// T >= TG_BM.  scratch: TG_CUT_BYTES for the sums of cut tiles, flags: 2 * TG_MAX_CUTS words, zero (or neither)
 template <int MODE>
-int launch_gemm_tcgen05_prompt(const GemmParams& g, cudaStream_t stream, void* scratch = nullptr, unsigned* flags = nullptr) {
-  bool pair = tcgen05_cluster_enabled() && g.T >= 4 * TG_BM;
-  int dev = 0, sms = 0;
-  MB_CHECK_CUDA(cudaGetDevice(&dev));
-  MB_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  // 128-wide tiles only when 256-wide ones cannot fill the machine once (small T or N).  Measured at T = 4096: narrowing the
-  // N = 4096 GEMMs (512 tiles = 3.46 rounds -> 1024 tiles = 6.9 rounds) makes them SLOWER (wo+w2 237 -> 343 us on average):
-  // per flop the narrow tile pulls 1.5x the bytes out of L2, and that, not tile quantisation, is the binding limit there.
-  const int units = pair ? sms / 2 : sms, m_units = pair ? ceil_div(ceil_div(g.T, TG_BM), 2) : ceil_div(g.T, TG_BM);
-  int bn = 256;
-  if (g.N % 256 != 0 || (int64_t)m_units * (g.N / 256) < units) {
-    bn = g.N % 128 == 0 ? 128 : 192;
-  }
-  // 192-wide tiles (N = 6144: 5.19 rounds of 256 -> 6.92 rounds at 3/4 of the cost) were measured too: qkv+RoPE at T = 4096
-  // 156 -> 169 us, slower for the same reason.  They stay available for N that is a multiple of 192 only and for the tests.
-  const int forced = tcgen05_forced_bn();
-  // Too few 256-wide tiles to fill the chip: pairs of them all the same when they, or their parts along a long k, fill half of it -- a pair reads
-  // a weight once for 256 rows and half as much of L2 per flop.  Measured (128-wide tiles, then pairs): 4096 x 14336 at T = 171 69, 45 us, at 700
-  // 141 | 91; 6144 x 4096 at 400 44 | 33, at 171 (24 pairs) 24 | 26; 2048 x 8192 at 400 41 | 31; 2048 x 2048 at 700 (24 pairs) 15 | 20.
-  if (bn == 128 && forced == 0 && tcgen05_cluster_enabled() && pairs_fill(g.T, g.N, g.K, sms / 2, scratch != nullptr)) {
-    pair = true;
-    bn = 256;
-  }
-  if ((forced == 128 || forced == 192 || forced == 256) && g.N % forced == 0) {
-    bn = forced;
-    scratch = nullptr;  // a pinned width is a plain schedule: every output's sum runs over k in one go, whatever the tile
-  }
-  if (bn == 192) return launch_gemm_tcgen05_bn<MODE, 192>(g, pair, sms, stream, nullptr, nullptr);
-  const bool narrow = bn == 128;
-  return narrow ? launch_gemm_tcgen05_bn<MODE, 128>(g, pair, sms, stream, nullptr, nullptr) : launch_gemm_tcgen05_bn<MODE, 256>(g, pair, sms, stream, scratch, flags);
-}
-
-template <int MODE>
-int launch_gemm_tcgen05(const GemmParams& g, cudaStream_t stream, void* scratch, unsigned* flags) {
-  if (g.T >= TG_BM) return launch_gemm_tcgen05_prompt<MODE>(g, stream, scratch, flags);
-  int dev = 0, sms = 0;
-  MB_CHECK_CUDA(cudaGetDevice(&dev));
-  MB_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+int launch_gemm_tcgen05_small(const GemmParams& g, int sms, cudaStream_t stream) {
   if (g.T <= 32) return launch_gemm_tcgen05_small_ta<MODE, 32>(g, sms, stream);
   if (g.T <= 64) return launch_gemm_tcgen05_small_ta<MODE, 64>(g, sms, stream);
   return launch_gemm_tcgen05_small_ta<MODE, 128>(g, sms, stream);

@@ -18,6 +18,7 @@
 //                       reference for any k and any number of ranks.
 // Roofline: tensor pipe for prefill (2 * rows * 3 * dim * hidden flop), HBM for decode (every touched expert's weights once).
 #pragma once
+#include "gemm_pair.cuh"
 #include "gemm_streamk.cuh"
 #include "gemm_tcgen05.cuh"
 
@@ -154,7 +155,7 @@ __global__ void __launch_bounds__(MP_THREADS) moe_plan_kernel(const int32_t* __r
       plan[3] = pairs;
       plan[4] += touched;
       plan[5] += 1;
-      plan[6] = 0;  // calls this small never take the cluster variant
+      plan[6] = 0;  // calls this small never run on pairs of CTAs
     }
     __syncthreads();
     for (int i = tid; i < pairs; i += MP_THREADS) slot[i] = sel[i] < E ? slot[i] + seg[sel[i]] : -1;
@@ -197,9 +198,11 @@ __global__ void __launch_bounds__(MP_THREADS) moe_plan_kernel(const int32_t* __r
           plan[MOE_PLAN_HEADER + n] = e;
           plan[MOE_PLAN_HEADER + tile_cap + n] = rows + m * tile_rows;
         }
-        for (int m = 0; m < m_tiles && np < tile_cap; m += 2, ++np) {  // pairs of vertically adjacent tiles for the 2-CTA cluster GEMM
+        const int units = (total[e] + 31) / 32, items = (units + 7) / 8;  // token tiles of pairs of CTAs: at most 256 wide, widths differ by at most 32
+        for (int m = 0; m < items && np < tile_cap; ++m, ++np) {
+          const int u0 = units * m / items, u1 = units * (m + 1) / items;
           plan[MOE_PLAN_HEADER + 2 * tile_cap + np] = e;
-          plan[MOE_PLAN_HEADER + 3 * tile_cap + np] = (rows + m * tile_rows) | (m + 1 < m_tiles ? MOE_PAIR_SECOND : 0);
+          plan[MOE_PLAN_HEADER + 3 * tile_cap + np] = (rows + 32 * u0) | (u1 - u0);
         }
       }
       rows += m_tiles * tile_rows;
@@ -341,49 +344,55 @@ inline int64_t moe_tile_cap(int64_t pairs, int64_t E, int tile_rows) { return (p
 inline int64_t moe_plan_words(int64_t pairs, int64_t E, int tile_rows) { return MOE_PLAN_HEADER + 4 * moe_tile_cap(pairs, E, tile_rows); }
 inline int64_t moe_row_cap(int64_t pairs, int64_t E, int tile_rows) { return moe_tile_cap(pairs, E, tile_rows) * tile_rows; }
 
-template <int MODE, int BN, int TA, int CL = 1>
+// tensor maps of the experts' weights, boxes of `rows` rows; another rank's experts (never referenced by this rank's tiles) get `map_a`
+inline int make_expert_maps(MoeWeightMaps* maps, const CUtensorMap& map_a, const void* const* w_host, int E, int64_t N, int64_t K, int rows) {
+  for (int e = 0; e < MOE_MAX_EXPERTS; ++e) {
+    if (e >= E || w_host[e] == nullptr) {
+      maps->m[e] = map_a;
+      continue;
+    }
+    const int rc = make_tensor_map_2d(&maps->m[e], w_host[e], N, K, rows);
+    if (rc) return rc;
+  }
+  return MB200_OK;
+}
+
+template <int MODE, int BN, int TA>
 int launch_grouped_bn(const void* a, int64_t rows_cap, int64_t K, int64_t N, const void* const* w_host, int E, const int32_t* plan, const EpiParams& epi,
                       int sms, cudaStream_t stream) {
-  using Cfg = TgCfg<BN, TA, CL, kEpiSmem<MODE>>;
+  using Cfg = TgCfg<BN, TA, kEpiSmem<MODE>>;
   CUtensorMap map_a;
   MoeWeightMaps maps;
   int rc = make_tensor_map_2d(&map_a, a, rows_cap, K, TA);
   if (rc) return rc;
-  for (int e = 0; e < MOE_MAX_EXPERTS; ++e) {
-    const void* w = e < E && w_host[e] != nullptr ? w_host[e] : nullptr;
-    if (w == nullptr) {  // an expert of another rank: never referenced by this rank's tiles
-      maps.m[e] = map_a;
-      continue;
-    }
-    rc = make_tensor_map_2d(&maps.m[e], w, N, K, BN / CL);  // pairs: each CTA holds half of the W tile
-    if (rc) return rc;
-  }
+  rc = make_expert_maps(&maps, map_a, w_host, E, N, K, BN);
+  if (rc) return rc;
   TcGemmParams p;
   p.T = (int)rows_cap;
   p.N = (int)N;
   p.K = (int)K;
   p.epi = epi;
-  MB_CHECK_CUDA(cudaFuncSetAttribute(gemm_tcgen05_grouped_kernel<MODE, CL, BN, TA>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
-  if (CL == 1) {
-    gemm_tcgen05_grouped_kernel<MODE, CL, BN, TA><<<sms, TG_THREADS, Cfg::kSmem, stream>>>(map_a, maps, p, plan);
-    MB_CHECK_LAUNCH("gemm_tcgen05_grouped_kernel");
-    return MB200_OK;
-  }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(2u * (unsigned)(sms / 2));
-  cfg.blockDim = dim3(TG_THREADS);
-  cfg.dynamicSmemBytes = Cfg::kSmem;
-  cfg.stream = stream;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = 2;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  MB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, gemm_tcgen05_grouped_kernel<MODE, CL, BN, TA>, map_a, maps, p, plan));
-  MB_CHECK_LAUNCH("gemm_tcgen05_grouped_kernel<cluster 2>");
+  MB_CHECK_CUDA(cudaFuncSetAttribute(gemm_tcgen05_grouped_kernel<MODE, BN, TA>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
+  gemm_tcgen05_grouped_kernel<MODE, BN, TA><<<sms, TG_THREADS, Cfg::kSmem, stream>>>(map_a, maps, p, plan);
+  MB_CHECK_LAUNCH("gemm_tcgen05_grouped_kernel");
   return MB200_OK;
+}
+
+// pairs of CTAs over the plan's token tiles (packed experts: w_n | w_k != 0, one map).  scratch, flags: as launch_gemm_pair
+template <int MODE>
+int launch_grouped_pair(const CUtensorMap& map_a, const MoeWeightMaps& maps, int64_t rows_cap, int64_t K, int64_t N, int64_t w_n, int64_t w_k, const int32_t* plan,
+                        const EpiParams& epi, int sms, cudaStream_t stream, void* scratch, unsigned* flags) {
+  PairParams p;
+  p.T = (int)rows_cap;
+  p.N = (int)N;
+  p.K = (int)K;
+  p.epi = epi;
+  p.w_n = (int)w_n;
+  p.w_k = (int)w_k;
+  p.units = sms / 2;
+  p.partials = reinterpret_cast<float*>(scratch);
+  p.flags = flags;
+  return launch_pairs(gemm_pair_grouped_kernel<MODE>, p.units, stream, map_a, maps, p, plan);
 }
 
 // tile width: prefill (128-row tiles) takes the widest tile that divides N; decode-sized calls (32-row tiles, HBM-bound) pick the
@@ -399,15 +408,8 @@ int launch_grouped_streamk(const void* a, int64_t rows_cap, int64_t K, int64_t N
   MoeWeightMaps maps;
   int rc = make_tensor_map_2d(&map_a, a, rows_cap, K, TA);
   if (rc) return rc;
-  for (int e = 0; e < MOE_MAX_EXPERTS; ++e) {
-    const void* w = e < E && w_host[e] != nullptr ? w_host[e] : nullptr;
-    if (w == nullptr) {
-      maps.m[e] = map_a;
-      continue;
-    }
-    rc = make_tensor_map_2d(&maps.m[e], w, N, K, SK_BN);
-    if (rc) return rc;
-  }
+  rc = make_expert_maps(&maps, map_a, w_host, E, N, K, SK_BN);
+  if (rc) return rc;
   SkParams p;
   p.T = (int)rows_cap;
   p.N = (int)N;
@@ -432,9 +434,17 @@ int launch_grouped(const void* a, int64_t rows_cap, int64_t K, int64_t N, const 
     return launch_grouped_streamk<MODE, 64>(a, rows_cap, K, N, w_host, E, plan, epi, workspace, workspace_bytes, header, sms, stream);
   }
   if (tile_rows == 128) {
-    // enough rows per expert for vertically adjacent tile pairs: the 2-CTA kernel (W tile shared, 2/3 of the L2 -> SM traffic)
-    if (N % 256 == 0 && tcgen05_cluster_enabled() && rows_cap >= (int64_t)E * 512)
-      return launch_grouped_bn<MODE, 256, 128, 2>(a, rows_cap, K, N, w_host, E, plan, epi, sms, stream);
+    if (N % 128 == 0 && tcgen05_cluster_enabled() && rows_cap >= (int64_t)E * 512) {
+      CUtensorMap map_a;
+      MoeWeightMaps maps;
+      int rc = make_tensor_map_2d(&map_a, a, rows_cap, K, TG_BM);
+      if (rc) return rc;
+      rc = make_expert_maps(&maps, map_a, w_host, E, N, K, TG_BM);
+      if (rc) return rc;
+      const bool room = workspace != nullptr && workspace_bytes >= header + TG_CUT_BYTES;
+      return launch_grouped_pair<MODE>(map_a, maps, rows_cap, K, N, 0, 0, plan, epi, sms, stream, room ? (uint8_t*)workspace + header : nullptr,
+                                       room ? reinterpret_cast<unsigned*>((uint8_t*)workspace + SK_FLAGS_OFFSET) : nullptr);
+    }
     if (N % 256 == 0) return launch_grouped_bn<MODE, 256, 128>(a, rows_cap, K, N, w_host, E, plan, epi, sms, stream);
     if (N % 128 == 0) return launch_grouped_bn<MODE, 128, 128>(a, rows_cap, K, N, w_host, E, plan, epi, sms, stream);
     if (N % 64 == 0) return launch_grouped_bn<MODE, 64, 128>(a, rows_cap, K, N, w_host, E, plan, epi, sms, stream);
@@ -518,18 +528,22 @@ __global__ void __launch_bounds__(256) layer_moe_combine_kernel(const float4* __
   *dst = acc;
 }
 
-// w: rows x cols, expert e at row e * w_n, column e * w_k
-template <int BN, int CL>
-int launch_grouped_packed_bn(const void* a, int64_t rows_cap, int64_t K, int64_t N, const void* w, int64_t w_rows, int64_t w_cols, int64_t w_n, int64_t w_k,
-                             const int32_t* plan, const EpiParams& epi, int sms, cudaStream_t stream) {
-  using Cfg = TgCfg<BN, 128, CL, kEpiSmem<EPI_LAYER>>;
+// w: rows x cols, expert e at row e * w_n, column e * w_k.  N % 128 == 0, K % 64 == 0.
+inline int launch_grouped_packed(const void* a, int64_t rows_cap, int64_t K, int64_t N, const void* w, int64_t w_rows, int64_t w_cols, int64_t w_n, int64_t w_k,
+                                 int64_t pairs, int64_t E, const int32_t* plan, const EpiParams& epi, cudaStream_t stream) {
+  int dev = 0, sms = 0;
+  MB_CHECK_CUDA(cudaGetDevice(&dev));
+  MB_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   CUtensorMap map_a;
   MoeWeightMaps maps;
-  int rc = make_tensor_map_2d(&map_a, a, rows_cap, K, 128);
+  int rc = make_tensor_map_2d(&map_a, a, rows_cap, K, TG_BM);
   if (rc) return rc;
-  rc = make_tensor_map_2d(&maps.m[0], w, w_rows, w_cols, BN / CL);
+  rc = make_tensor_map_2d(&maps.m[0], w, w_rows, w_cols, TG_BM);
   if (rc) return rc;
   for (int e = 1; e < MOE_MAX_EXPERTS; ++e) maps.m[e] = maps.m[0];
+  if (tcgen05_cluster_enabled() && pairs >= 384 * E && pairs > 512)  // (the plan of up to 512 rows lists no token tiles of pairs)
+    return launch_grouped_pair<EPI_LAYER>(map_a, maps, rows_cap, K, N, w_n, w_k, plan, epi, sms, stream, nullptr, nullptr);
+  using Cfg = TgCfg<128, 128, kEpiSmem<EPI_LAYER>>;
   TcGemmParams p;
   p.T = (int)rows_cap;
   p.N = (int)N;
@@ -537,34 +551,10 @@ int launch_grouped_packed_bn(const void* a, int64_t rows_cap, int64_t K, int64_t
   p.epi = epi;
   p.w_n = (int)w_n;
   p.w_k = (int)w_k;
-  MB_CHECK_CUDA(cudaFuncSetAttribute(gemm_tcgen05_grouped_kernel<EPI_LAYER, CL, BN, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(sms / CL * CL));
-  cfg.blockDim = dim3(TG_THREADS);
-  cfg.dynamicSmemBytes = Cfg::kSmem;
-  cfg.stream = stream;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = CL;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  MB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, gemm_tcgen05_grouped_kernel<EPI_LAYER, CL, BN, 128>, map_a, maps, p, plan));
+  MB_CHECK_CUDA(cudaFuncSetAttribute(gemm_tcgen05_grouped_kernel<EPI_LAYER, 128, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
+  gemm_tcgen05_grouped_kernel<EPI_LAYER, 128, 128><<<sms, TG_THREADS, Cfg::kSmem, stream>>>(map_a, maps, p, plan);
   MB_CHECK_LAUNCH("gemm_tcgen05_grouped_kernel<layer>");
   return MB200_OK;
-}
-
-// N % 128 == 0, K % 64 == 0.  Pairs of tiles in 2-CTA clusters from about three full tiles per expert on: with fewer, a pair's missing
-// second tile costs more than the shared W tile saves.
-inline int launch_grouped_packed(const void* a, int64_t rows_cap, int64_t K, int64_t N, const void* w, int64_t w_rows, int64_t w_cols, int64_t w_n, int64_t w_k,
-                                 int64_t pairs, int64_t E, const int32_t* plan, const EpiParams& epi, cudaStream_t stream) {
-  int dev = 0, sms = 0;
-  MB_CHECK_CUDA(cudaGetDevice(&dev));
-  MB_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  if (N % 256 == 0 && tcgen05_cluster_enabled() && pairs >= 384 * E && pairs > 512)  // (the plan of up to 512 rows lists no pairs)
-    return launch_grouped_packed_bn<256, 2>(a, rows_cap, K, N, w, w_rows, w_cols, w_n, w_k, plan, epi, sms, stream);
-  return launch_grouped_packed_bn<128, 1>(a, rows_cap, K, N, w, w_rows, w_cols, w_n, w_k, plan, epi, sms, stream);
 }
 
 }  // namespace mb200
