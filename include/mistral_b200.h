@@ -221,7 +221,8 @@ int mb200_moe_grouped_ffn(const void* xs, const void* const* w13_host, const voi
  *     rowscale [T, rs_pitch] fp32 or NULL: hidden unit c of row t is scaled by rowscale[t, c / rs_group].  n_act columns through SiLU.
  *     scratch: mb200_layer_linear_scratch(T, N, K) bytes (uninitialised, this call's own), or NULL (also when that is 0): without it the last
  *     tiles are not cut; fewer than 128 rows need it.
- * mb200_layer_moe: y32 [T, width] fp32 (+= when add) sum over the token's choices idx [T, top] < n_experts of
+ * mb200_layer_moe: y32 [T, width] fp32 (+= when add & 1) sum over the token's choices idx [T, top] < n_experts (with add & 2 a choice from n_experts on is
+ *     the token itself, wsel * hn) of
  *     wsel * (act W2_e^T), act = step(hn W13_e^T); w13 [E * 2 ff, width] (gate/up rows interleaved; RELU2: [E * ff, width]),
  *     w2 [width, E * ff].  The weight multiplies the hidden units (GLU: the expert's input).  width % 128 == 0, ff % 64 == 0,
  *     T <= 65535.  Buffers (device, uninitialised): slot [T * top] int32, plan [plan_words] int32, xs [rows_cap, width] bf16,

@@ -317,8 +317,9 @@ LAYER_MOE_MAX_TOKENS = 8192  # tokens per call of layer_moe: bounds the row buff
 
 
 def layer_moe(hn: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, idx: torch.Tensor, wsel: torch.Tensor, E: int, ff: int, epi: int, limit: float,
-              alpha: float, y32: torch.Tensor, add: bool) -> None:
-    """y32 (+)= the weighted sum of each token's chosen experts, computing the chosen (token, expert) rows only (include/mistral_b200.h)."""
+              alpha: float, y32: torch.Tensor, add: bool, identity: bool = False) -> None:
+    """y32 (+)= the weighted sum of each token's chosen experts, computing the chosen (token, expert) rows only (include/mistral_b200.h); identity: choices
+    from E on are the token itself."""
     top = idx.shape[1]
     for r0 in range(0, hn.shape[0], LAYER_MOE_MAX_TOKENS):
         h, sel, wts, y = (t[r0: r0 + LAYER_MOE_MAX_TOKENS] for t in (hn, idx, wsel, y32))
@@ -330,7 +331,7 @@ def layer_moe(hn: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, idx: torch.
         slot, plan, row_w = new(T * top, torch.int32), new(pw.value, torch.int32), new(rows, torch.float32)
         xs, act, rows32 = new(rows * D, h.dtype), new(rows * ff, h.dtype), new(rows * D, torch.float32)
         _check(lib().mb200_layer_moe(_ptr(h), _ptr(w13), _ptr(w2), _ptr(sel), _ptr(wts), T, D, ff, E, top, epi, limit, alpha, _ptr(slot), _ptr(plan), _ptr(xs),
-                                     _ptr(row_w), _ptr(act), _ptr(rows32), _ptr(y), int(add), _stream()), "mb200_layer_moe")
+                                     _ptr(row_w), _ptr(act), _ptr(rows32), _ptr(y), int(add) | 2 * int(identity), _stream()), "mb200_layer_moe")
 
 
 def comm_alloc(nbytes: int) -> int:

@@ -334,16 +334,16 @@ def moe_grouped_ok(h: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, E: int,
 
 
 def moe_grouped(h: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, idx: torch.Tensor, wsel: torch.Tensor, E: int, ff: int, epi: int,
-                limit: float = 0.0, alpha: float = 0.0, add_to: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """fp32 [T, width]: the weighted sum of each token's chosen experts (indices >= E: none); added to add_to (fp32) when given.  epi: the
-    unit between the two Linears (EPI_SWIGLU, EPI_GLU with the weight on the expert's input, EPI_GEGLU, EPI_RELU2)."""
+                limit: float = 0.0, alpha: float = 0.0, add_to: Optional[torch.Tensor] = None, identity: bool = False) -> torch.Tensor:
+    """fp32 [T, width]: the weighted sum of each token's chosen experts (indices >= E: none, or with `identity` the token itself); added to add_to (fp32) when
+    given.  epi: the unit between the two Linears (EPI_SWIGLU, EPI_GLU with the weight on the expert's input, EPI_GEGLU, EPI_RELU2)."""
     T, D = h.shape
     units = w13.shape[0] // E
     assert idx.dtype == torch.int32 and wsel.dtype == torch.float32 and idx.shape == wsel.shape and idx.shape[0] == T, "choices: int32 and fp32 [tokens, top]"
     assert w13.dtype == w2.dtype == h.dtype and w13.shape == (units * E, D) and w2.shape == (D, E * ff) and units == (ff if epi == EPI_RELU2 else 2 * ff), "experts' weights"
     assert add_to is None or (add_to.dtype == torch.float32 and add_to.shape == (T, D)), "add_to: fp32 [tokens, width]"
     y32 = torch.empty(h.shape, dtype=torch.float32, device=h.device) if add_to is None else add_to
-    _abi.layer_moe(h, w13, w2, idx, wsel, E, ff, epi, limit, alpha, y32, add_to is not None)
+    _abi.layer_moe(h, w13, w2, idx, wsel, E, ff, epi, limit, alpha, y32, add_to is not None, identity)
     return y32
 
 

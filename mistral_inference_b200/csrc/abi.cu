@@ -402,7 +402,7 @@ int mb200_moe_route(const void* hn, const void* gate_w, int64_t T, int64_t dim, 
   MB_CHECK_LAUNCH("moe_route_kernel");
   const int tile_rows = moe_tile_rows(T);
   const int64_t pairs = T * top_k, cap = moe_tile_cap(pairs, n_experts, tile_rows);
-  const size_t plan_smem = ((size_t)n_experts * MP_THREADS + 2 * n_experts + 1) * sizeof(int32_t);
+  const size_t plan_smem = moe_plan_smem(n_experts);
   MB_CHECK_CUDA(cudaFuncSetAttribute(moe_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan_smem));
   moe_plan_kernel<<<1, MP_THREADS, plan_smem, st>>>(sel, (int)pairs, (int)n_experts, tile_rows, (int)shard_rank, (int)shard_world, (int)cap, slot, plan);
   MB_CHECK_LAUNCH("moe_plan_kernel");
@@ -579,7 +579,7 @@ int mb200_layer_moe(const void* hn, const void* w13, const void* w2, const int32
                "layer_moe: T=%lld width=%lld ff=%lld E=%lld top=%lld", (long long)T, (long long)dim, (long long)ff, (long long)n_experts, (long long)top);
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t pairs = T * top, cap = moe_tile_cap(pairs, n_experts, TG_BM), rows_cap = cap * TG_BM;
-  const size_t plan_smem = ((size_t)n_experts * MP_THREADS + 2 * n_experts + 1) * sizeof(int32_t);
+  const size_t plan_smem = moe_plan_smem(n_experts);
   MB_CHECK_CUDA(cudaFuncSetAttribute(moe_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan_smem));
   moe_plan_kernel<<<1, MP_THREADS, plan_smem, st>>>(idx, (int)pairs, (int)n_experts, TG_BM, 0, 1, (int)cap, slot, plan);
   MB_CHECK_LAUNCH("moe_plan_kernel");
@@ -597,8 +597,8 @@ int mb200_layer_moe(const void* hn, const void* w13, const void* w2, const int32
   if (rc) return rc;
   rc = launch_grouped_packed(act, rows_cap, ff, dim, w2, dim, n_experts * ff, 0, ff, pairs, n_experts, plan, e2, st);
   if (rc) return rc;
-  layer_moe_combine_kernel<<<dim3((unsigned)ceil_div(dim / 4, 256), (unsigned)T), 256, 0, st>>>((const float4*)rows32, slot, (float4*)y32, (int)T, (int)top,
-                                                                                            (int)(dim / 4), add);
+  layer_moe_combine_kernel<<<dim3((unsigned)ceil_div(dim / 4, 256), (unsigned)T), 256, 0, st>>>((const float4*)rows32, slot, wsel, (const uint2*)hn, (float4*)y32, (int)top,
+                                                                                            (int)(dim / 4), add & 1, add & 2);
   MB_CHECK_LAUNCH("layer_moe_combine_kernel");
   return MB200_OK;
 }

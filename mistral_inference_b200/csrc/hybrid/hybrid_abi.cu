@@ -460,7 +460,7 @@ int mbh_moe_route(const void* h, const void* w_router, const void* correction, v
     MoeRouteArgs a{h, w_router, correction, (float*)dense, (int*)idx, (float*)wsel, (int)width, (int)n, (int)groups, (int)keep, (int)top, score, w_bias, scale,
                    group_two, renorm, w_gate, (float*)gate, (int)always};
     cudaStream_t st = (cudaStream_t)stream;
-    DISPATCH(dt, moe_route_kernel<ST><<<(unsigned)T, MOE_ROUTE_THREADS, smem, st>>>(a));
+    DISPATCH(dt, launch_moe_route<ST>(a, T, smem, st));
     cudaError_t e = cudaGetLastError();
     return e ? fail(e, "mbh_moe_route") : 0;
 }

@@ -67,28 +67,9 @@ __device__ __forceinline__ float warp_dot(const T* __restrict__ w, const T* __re
     return warp_sum(acc);
 }
 
-constexpr int MOE_ROUTE_THREADS = 256;
-
-// one CTA per token; shared memory: z[n] | choice[n] | gbest[groups] | kept[groups]
+// One token's choice, by a warp: z[n] holds the outputs (the bias added), ch[n], gb[groups] and kept[groups] are scratch in shared memory.
 template <typename T>
-__global__ void __launch_bounds__(MOE_ROUTE_THREADS) moe_route_kernel(MoeRouteArgs a) {
-    extern __shared__ float sm[];
-    float* z = sm;
-    float* ch = sm + a.n;
-    float* gb = sm + 2 * a.n;
-    float* kept = gb + a.groups;
-    const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    const T* h = static_cast<const T*>(a.h) + (size_t)t * a.width;
-    const T* W = static_cast<const T*>(a.w_router);
-    for (int e = warp; e < a.n + (a.w_gate ? 1 : 0); e += nw) {
-        const float acc = warp_dot<T>(e < a.n ? W + (size_t)e * a.width : static_cast<const T*>(a.w_gate), h, a.width, lane);
-        if (lane == 0) {
-            if (e < a.n) z[e] = acc + (a.w_bias ? to_f(static_cast<const T*>(a.w_bias)[e]) : 0.f);
-            else a.gate[t] = sigmoid_exact(acc);
-        }
-    }
-    __syncthreads();
-    if (warp != 0) return;
+__device__ __forceinline__ void moe_choose(const MoeRouteArgs& a, int t, float* z, float* ch, float* gb, float* kept, int lane) {
     const int dn = a.n + a.always, tk = a.top + a.always;
     for (int s = lane; s < a.always; s += 32) {
         a.dense[(size_t)t * dn + a.n + s] = 1.f;
@@ -188,6 +169,167 @@ __global__ void __launch_bounds__(MOE_ROUTE_THREADS) moe_route_kernel(MoeRouteAr
             a.dense[(size_t)t * dn + ei] = w;
         }
     }
+}
+
+// The same for up to 32 outputs, one in each lane (z; lanes from n on: anything): no shared memory, a maximum over the warp is one instruction.  The same sums in the
+// same order as above.
+__device__ __forceinline__ unsigned moe_key(float v) {  // grows with v, 0 for nothing (NaN); -0 counts as 0
+    const unsigned u = __float_as_uint(v + 0.f);
+    return v == v ? ((u & 0x80000000u) ? ~u : (u | 0x80000000u)) : 0u;
+}
+// the lane with the largest key above `none` (the lowest of several), or -1
+__device__ __forceinline__ int moe_best(unsigned key, unsigned none) {
+    const unsigned top = __reduce_max_sync(0xffffffffu, key);
+    return top > none ? __ffs(__ballot_sync(0xffffffffu, key == top)) - 1 : -1;
+}
+template <typename T>
+__device__ __forceinline__ void moe_choose_lanes(const MoeRouteArgs& a, int t, float z, int lane) {
+    const int dn = a.n + a.always, tk = a.top + a.always;
+    const bool here = lane < a.n;
+    const unsigned LOWEST = moe_key(-INFINITY);
+    int my_idx = 0;              // lane k: choice k
+    float my_w = 0.f, my_dense = 0.f;
+    if (a.score == 2) {
+        const float mx = warp_max(here ? z : -INFINITY);
+        float den = 0.f, c = here ? z : -INFINITY;
+        for (int k = 0; k < a.top; ++k) {
+            int ei = moe_best(moe_key(c), LOWEST);
+            const float v = ei < 0 ? -INFINITY : __shfl_sync(0xffffffffu, c, ei);
+            if (ei < 0) ei = 0;
+            den += expf(v - mx);
+            if (lane == k) my_idx = ei;
+            if (lane == ei) c = -INFINITY;
+        }
+        const float own = __shfl_sync(0xffffffffu, z, my_idx);
+        my_w = expf(own - mx) / den * a.scale;
+        for (int k = 0; k < a.top; ++k) {
+            const int ei = __shfl_sync(0xffffffffu, my_idx, k);
+            const float w = __shfl_sync(0xffffffffu, my_w, k);
+            if (lane == ei) my_dense = w;
+        }
+    } else {
+        float sum = 1.f;
+        if (a.score == 1) {
+            z = sigmoid_exact(z);
+        } else {
+            const float mx = warp_max(here ? z : -INFINITY);
+            z = here ? expf(z - mx) : 0.f;
+            sum = warp_sum(z);
+        }
+        const float s = z / sum;
+        float c = here ? s + (a.correction ? to_f(static_cast<const T*>(a.correction)[lane]) : 0.f) : -INFINITY;
+        if (a.groups > 1 && a.keep < a.groups) {
+            const int gs = a.n / a.groups;
+            float b = -INFINITY, b2 = -INFINITY;  // lane g: group g
+            for (int i = 0; i < gs; ++i) {
+                const float o = __shfl_sync(0xffffffffu, c, min(lane * gs + i, 31));
+                b2 = fmaxf(b2, fminf(b, o));
+                b = fmaxf(b, o);
+            }
+            unsigned key = lane < a.groups ? moe_key((a.group_two && gs > 1) ? b + b2 : b) | 1u : 0u, kept = 0u;
+            for (int k = 0; k < a.keep; ++k) {
+                const int g = moe_best(key, 0u);
+                if (g < 0) break;
+                kept |= 1u << g;
+                if (lane == g) key = 0u;
+            }
+            if (here && !((kept >> (lane / gs)) & 1u)) c = -INFINITY;
+        }
+        float total = 0.f;
+        for (int k = 0; k < a.top; ++k) {
+            const int ei = moe_best(moe_key(c), LOWEST);
+            const float w = ei < 0 ? 0.f : __shfl_sync(0xffffffffu, s, ei);  // fewer eligible outputs than `top` (a configuration error): output 0, weight 0
+            total += w;
+            if (lane == k) {
+                my_idx = max(ei, 0);
+                my_w = w * a.scale;
+            }
+            if (lane == ei) {
+                my_dense = w * a.scale;
+                c = -INFINITY;
+            }
+        }
+        if (a.renorm) {
+            const float den = total + 1e-20f, own = __shfl_sync(0xffffffffu, s, my_idx);
+            my_w = own / den * a.scale;
+            for (int k = 0; k < a.top; ++k) {
+                const int ei = __shfl_sync(0xffffffffu, my_idx, k);
+                const float w = __shfl_sync(0xffffffffu, my_w, k);
+                if (lane == ei) my_dense = w;
+            }
+        }
+    }
+    if (here) a.dense[(size_t)t * dn + lane] = my_dense;
+    if (lane < a.top) {
+        a.idx[(size_t)t * tk + lane] = my_idx;
+        a.wsel[(size_t)t * tk + lane] = my_w;
+    }
+    for (int i = lane; i < a.always; i += 32) {
+        a.dense[(size_t)t * dn + a.n + i] = 1.f;
+        a.idx[(size_t)t * tk + a.top + i] = a.n + i;
+        a.wsel[(size_t)t * tk + a.top + i] = 1.f;
+    }
+}
+
+constexpr int MOE_ROUTE_THREADS = 256;
+
+// A CTA per TOK tokens: its warps share the outputs, then TOK of them choose; shared memory per token: z[n] | choice[n] | gbest[groups] | kept[groups].  Four tokens a CTA
+// from MOE_ROUTE_MANY tokens on: a piece of a router row out of L2 serves four sums, and four warps of eight choose where one did (2500 tokens, width 2048, 20
+// outputs: 48 us with one token a CTA and a choice through shared memory, 33 with that choice in registers, 26 with four; 592 tokens 9 with one and 13 with four,
+// 801 15 and 13).  A sum runs in the order of warp_dot either way.
+template <typename T, int TOK>
+__global__ void __launch_bounds__(MOE_ROUTE_THREADS) moe_route_kernel(MoeRouteArgs a, int tokens) {
+    extern __shared__ float sm[];
+    constexpr int V = Vec<T>::N;
+    const int per = 2 * a.n + 2 * a.groups, t0 = blockIdx.x * TOK, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const T* h[TOK];
+#pragma unroll
+    for (int i = 0; i < TOK; ++i) h[i] = static_cast<const T*>(a.h) + (size_t)min(t0 + i, tokens - 1) * a.width;
+    const T* W = static_cast<const T*>(a.w_router);
+    for (int e = warp; e < a.n + (a.w_gate ? 1 : 0); e += nw) {
+        const T* w = e < a.n ? W + (size_t)e * a.width : static_cast<const T*>(a.w_gate);
+        float acc[TOK];
+        if constexpr (TOK == 1) {
+            acc[0] = warp_dot<T>(w, h[0], a.width, lane);
+        } else {
+#pragma unroll
+            for (int i = 0; i < TOK; ++i) acc[i] = 0.f;
+#pragma unroll 2
+            for (int k = lane * V; k < a.width; k += 32 * V) {
+                float wv[V], x[TOK][V];
+                Vec<T>::load(w + k, wv);
+#pragma unroll
+                for (int i = 0; i < TOK; ++i) Vec<T>::load(h[i] + k, x[i]);
+#pragma unroll
+                for (int i = 0; i < TOK; ++i)
+#pragma unroll
+                    for (int v = 0; v < V; ++v) acc[i] = fmaf(wv[v], x[i][v], acc[i]);
+            }
+#pragma unroll
+            for (int i = 0; i < TOK; ++i) acc[i] = warp_sum(acc[i]);
+        }
+        if (lane == 0) {
+#pragma unroll
+            for (int i = 0; i < TOK; ++i) {
+                if (e < a.n) sm[i * per + e] = acc[i] + (a.w_bias ? to_f(static_cast<const T*>(a.w_bias)[e]) : 0.f);
+                else if (t0 + i < tokens) a.gate[t0 + i] = sigmoid_exact(acc[i]);
+            }
+        }
+    }
+    __syncthreads();
+    if (warp >= TOK || t0 + warp >= tokens) return;
+    float* z = sm + warp * per;
+    if (a.n <= 32) moe_choose_lanes<T>(a, t0 + warp, lane < a.n ? z[lane] : 0.f, lane);
+    else moe_choose<T>(a, t0 + warp, z, z + a.n, z + 2 * a.n, z + 2 * a.n + a.groups, lane);
+}
+
+constexpr int64_t MOE_ROUTE_MANY = 700;
+template <typename T>
+inline void launch_moe_route(const MoeRouteArgs& a, int64_t tokens, size_t smem, cudaStream_t st) {
+    // (the sums of four tokens at a time need rows of whole 16-byte pieces)
+    const bool aligned = a.width % Vec<T>::N == 0 && (reinterpret_cast<uintptr_t>(a.h) | reinterpret_cast<uintptr_t>(a.w_router) | reinterpret_cast<uintptr_t>(a.w_gate)) % 16 == 0;
+    if (tokens >= MOE_ROUTE_MANY && aligned && 4 * smem <= 48 * 1024) moe_route_kernel<T, 4><<<(unsigned)((tokens + 3) / 4), MOE_ROUTE_THREADS, 4 * smem, st>>>(a, (int)tokens);
+    else moe_route_kernel<T, 1><<<(unsigned)tokens, MOE_ROUTE_THREADS, smem, st>>>(a, (int)tokens);
 }
 
 struct MoeSparseArgs {

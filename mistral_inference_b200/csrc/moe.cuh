@@ -117,12 +117,13 @@ __global__ void __launch_bounds__(256) moe_route_kernel(const bf16* __restrict__
 // ---- plan: one CTA ---------------------------------------------------------------------------------------------------------
 // plan layout (int32): [0] m tiles owned by this rank, [1] padded rows in total, [2] tile capacity, [3] pairs, [4]/[5] statistics, [8 + e] start of
 // expert e's segment (e = 0..E), then tile_expert[capacity], tile_row0[capacity] from word MOE_PLAN_HEADER.
-constexpr int MP_THREADS = 1024;
+constexpr int MP_THREADS = 1024, MP_ROW = MP_THREADS + MP_THREADS / 32;
+inline size_t moe_plan_smem(int64_t E) { return ((size_t)E * MP_ROW + 2 * E + 1) * sizeof(int32_t); }
 __global__ void __launch_bounds__(MP_THREADS) moe_plan_kernel(const int32_t* __restrict__ sel, int pairs, int E, int tile_rows, int shard_rank,
                                                               int shard_world, int tile_cap, int32_t* __restrict__ slot, int32_t* __restrict__ plan) {
-  extern __shared__ int32_t sm[];  // cnt[E][MP_THREADS], then seg[E + 1], total[E]
+  extern __shared__ int32_t sm[];  // cnt[E][MP_ROW], then seg[E + 1], total[E]
   int32_t* cnt = sm;
-  int32_t* seg = sm + E * MP_THREADS;
+  int32_t* seg = sm + E * MP_ROW;
   int32_t* total = seg + E + 1;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (pairs <= 512) {
@@ -161,16 +162,25 @@ __global__ void __launch_bounds__(MP_THREADS) moe_plan_kernel(const int32_t* __r
     for (int i = tid; i < pairs; i += MP_THREADS) slot[i] = sel[i] < E ? slot[i] + seg[sel[i]] : -1;
     return;
   }
-  const int per = (pairs + MP_THREADS - 1) / MP_THREADS;
+  // This thread counts `per` neighbouring pairs, eight loads in flight at a time.  Row e of cnt has thread t's count at t + t / 32: the scan below, whose lanes take 32
+  // neighbouring counts each, would otherwise have all of them in one bank.
+  const int per = (pairs + MP_THREADS - 1) / MP_THREADS, mine = tid + (tid >> 5);
   const int p0 = min(tid * per, pairs), p1 = min(p0 + per, pairs);
-  for (int e = 0; e < E; ++e) cnt[e * MP_THREADS + tid] = 0;
-  for (int i = p0; i < p1; ++i)
-    if (sel[i] < E) cnt[sel[i] * MP_THREADS + tid] += 1;
+  for (int e = 0; e < E; ++e) cnt[e * MP_ROW + mine] = 0;
+  for (int i0 = p0; i0 < p1; i0 += 8) {
+    int v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = i0 + i < p1 ? sel[i0 + i] : E;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (v[i] < E) cnt[v[i] * MP_ROW + mine] += 1;
+  }
   __syncthreads();
   // exclusive scan of every expert's 1024 counts: warp w takes experts w, w + 32, ...; lane l scans entries [32 l, 32 l + 32)
   for (int e = warp; e < E; e += MP_THREADS / 32) {
-    int32_t* c = cnt + e * MP_THREADS + lane * 32;
+    int32_t* c = cnt + e * MP_ROW + lane * 33;
     int run = 0;
+#pragma unroll 8
     for (int i = 0; i < 32; ++i) {
       const int v = c[i];
       c[i] = run;
@@ -183,46 +193,64 @@ __global__ void __launch_bounds__(MP_THREADS) moe_plan_kernel(const int32_t* __r
       if (lane >= o) incl += up;
     }
     const int base = incl - run;
+#pragma unroll 8
     for (int i = 0; i < 32; ++i) c[i] += base;
     if (lane == 31) total[e] = incl;
   }
   __syncthreads();
-  if (tid == 0) {
-    int rows = 0, n = 0, np = 0;
-    for (int e = 0; e < E; ++e) {
-      seg[e] = rows;
-      plan[8 + e] = rows;
-      const int m_tiles = (total[e] + tile_rows - 1) / tile_rows;
-      if (e % shard_world == shard_rank) {
-        for (int m = 0; m < m_tiles && n < tile_cap; ++m, ++n) {
-          plan[MOE_PLAN_HEADER + n] = e;
-          plan[MOE_PLAN_HEADER + tile_cap + n] = rows + m * tile_rows;
-        }
-        const int units = (total[e] + 31) / 32, items = (units + 7) / 8;  // token tiles of pairs of CTAs: at most 256 wide, widths differ by at most 32
-        for (int m = 0; m < items && np < tile_cap; ++m, ++np) {
-          const int u0 = units * m / items, u1 = units * (m + 1) / items;
-          plan[MOE_PLAN_HEADER + 2 * tile_cap + np] = e;
-          plan[MOE_PLAN_HEADER + 3 * tile_cap + np] = (rows + 32 * u0) | (u1 - u0);
-        }
+  if (warp == 0) {  // segment starts and the tile lists, an expert per lane
+    int rows = 0, n = 0, np = 0, touched = 0;
+    for (int e0 = 0; e0 < E; e0 += 32) {
+      const int e = e0 + lane;
+      const bool here = e < E, own = here && e % shard_world == shard_rank;
+      const int have = here ? total[e] : 0, m_tiles = (have + tile_rows - 1) / tile_rows;
+      const int units = (have + 31) / 32, items = (units + 7) / 8;  // token tiles of pairs of CTAs: at most 256 wide, widths differ by at most 32
+      int r = m_tiles * tile_rows, k = own ? m_tiles : 0, q = own ? items : 0;
+      const int r_own = r, k_own = k, q_own = q;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int ur = __shfl_up_sync(0xffffffffu, r, o), uk = __shfl_up_sync(0xffffffffu, k, o), uq = __shfl_up_sync(0xffffffffu, q, o);
+        if (lane >= o) r += ur, k += uk, q += uq;
       }
-      rows += m_tiles * tile_rows;
+      const int row0 = rows + r - r_own, n0 = n + k - k_own, np0 = np + q - q_own;
+      if (here) {
+        seg[e] = row0;
+        plan[8 + e] = row0;
+      }
+      for (int m = 0; m < k_own && n0 + m < tile_cap; ++m) {
+        plan[MOE_PLAN_HEADER + n0 + m] = e;
+        plan[MOE_PLAN_HEADER + tile_cap + n0 + m] = row0 + m * tile_rows;
+      }
+      for (int m = 0; m < q_own && np0 + m < tile_cap; ++m) {
+        const int u0 = units * m / items, u1 = units * (m + 1) / items;
+        plan[MOE_PLAN_HEADER + 2 * tile_cap + np0 + m] = e;
+        plan[MOE_PLAN_HEADER + 3 * tile_cap + np0 + m] = (row0 + 32 * u0) | (u1 - u0);
+      }
+      rows += __shfl_sync(0xffffffffu, r, 31);
+      n += __shfl_sync(0xffffffffu, k, 31);
+      np += __shfl_sync(0xffffffffu, q, 31);
+      touched += __popc(__ballot_sync(0xffffffffu, have > 0));
     }
-    plan[6] = np;
-    seg[E] = rows;
-    plan[8 + E] = rows;
-    plan[0] = n;
-    plan[1] = rows;
-    plan[2] = tile_cap;
-    plan[3] = pairs;
-    int touched = 0;
-    for (int e = 0; e < E; ++e) touched += total[e] > 0;
-    plan[4] += touched;  // statistics (never reset by the kernel): experts with at least one row, summed over calls ...
-    plan[5] += 1;        // ... and the number of calls: the measured "distinct experts per layer" of bench.py
+    if (lane == 0) {
+      plan[0] = min(n, tile_cap);
+      plan[1] = rows;
+      plan[2] = tile_cap;
+      plan[3] = pairs;
+      plan[4] += touched;  // statistics (never reset by the kernel): experts with at least one row, summed over calls ...
+      plan[5] += 1;        // ... and the number of calls: the measured "distinct experts per layer" of bench.py
+      plan[6] = min(np, tile_cap);
+      seg[E] = rows;
+      plan[8 + E] = rows;
+    }
   }
   __syncthreads();
-  for (int i = p0; i < p1; ++i) {  // this thread's column of cnt is its own: the next free place of each expert
-    const int e = sel[i];
-    slot[i] = e < E ? seg[e] + cnt[e * MP_THREADS + tid]++ : -1;
+  for (int i0 = p0; i0 < p1; i0 += 8) {  // this thread's column of cnt is its own: the next free place of each expert
+    int v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = i0 + i < p1 ? sel[i0 + i] : E;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (i0 + i < p1) slot[i0 + i] = v[i] < E ? seg[v[i]] + cnt[v[i] * MP_ROW + mine]++ : -1;
   }
 }
 
@@ -507,22 +535,34 @@ __global__ void __launch_bounds__(256) layer_moe_gather_kernel(const uint4* __re
   for (int c = lane; c < row_chunks; c += 32) dst[c] = src[c];
 }
 
-__global__ void __launch_bounds__(256) layer_moe_combine_kernel(const float4* __restrict__ rows, const int32_t* __restrict__ slot, float4* __restrict__ y,
-                                                                int T, int k, int row_quads, int add) {
+// identity: a choice without a row is an identity expert, the token itself (hn) times the choice's weight
+__global__ void __launch_bounds__(256) layer_moe_combine_kernel(const float4* __restrict__ rows, const int32_t* __restrict__ slot, const float* __restrict__ wsel,
+                                                                const uint2* __restrict__ hn, float4* __restrict__ y, int k, int row_quads, int add, int identity) {
   const int c = blockIdx.x * 256 + threadIdx.x, t = blockIdx.y;
   if (c >= row_quads) return;
   const int32_t* sl = slot + (int64_t)t * k;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-  for (int j = 0; j < k; ++j) {
-    const int s = sl[j];
-    if (s < 0) continue;
-    const float4 v = __ldcs(rows + (int64_t)s * row_quads + c);
-    acc.x += v.x, acc.y += v.y, acc.z += v.z, acc.w += v.w;
-  }
   float4* dst = y + (int64_t)t * row_quads + c;
+  float4 o = acc;
+  if (add) o = *dst;
+  float own = 0.f;  // the identity experts' weights
+  for (int j0 = 0; j0 < k; j0 += 8) {
+    float4 v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int s = j0 + j < k ? sl[j0 + j] : -1;
+      v[j] = s >= 0 ? __ldcs(rows + (int64_t)s * row_quads + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+      if (identity && s < 0 && j0 + j < k) own += wsel[(int64_t)t * k + j0 + j];
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc.x += v[j].x, acc.y += v[j].y, acc.z += v[j].z, acc.w += v[j].w;
+  }
+  if (own != 0.f) {
+    const uint2 h = hn[(int64_t)t * row_quads + c];
+    acc.x = fmaf(own, bf16lo(h.x), acc.x), acc.y = fmaf(own, bf16hi(h.x), acc.y);
+    acc.z = fmaf(own, bf16lo(h.y), acc.z), acc.w = fmaf(own, bf16hi(h.y), acc.w);
+  }
   if (add) {
-    const float4 o = *dst;
     acc.x += o.x, acc.y += o.y, acc.z += o.z, acc.w += o.w;
   }
   *dst = acc;

@@ -534,19 +534,21 @@ class MoeFeedForward(nn.Module):
     def run(self, hn: torch.Tensor, x32: torch.Tensor, post: Optional[Norm] = None) -> None:
         a = self.a
         dense, idx, wsel = _h.moe_route(hn, self.router, self.correction, a.groups, a.keep, a.top)
+        # without a norm behind them the experts' sum goes straight into the residual stream, where the kernels can write it
+        direct = post is None and x32.dtype == torch.float32 and x32.is_contiguous() and x32.data_ptr() % 16 == 0
+        into = x32 if direct else None
         if hn.shape[0] <= self.sparse_max_tokens:
-            y32 = _h.moe_sparse(hn, self.w13, self.w2, idx, wsel, a.experts, a.ff)
+            y32 = _h.moe_sparse(hn, self.w13, self.w2, idx, wsel, a.experts, a.ff, add_to=into)
+        elif _h.moe_grouped_ok(hn, self.w13, self.w2, a.experts, a.ff):
+            y32 = _h.moe_grouped(hn, self.w13, self.w2, idx, wsel, a.experts, a.ff, _h.EPI_SWIGLU, add_to=into, identity=a.identity > 0)
         else:
-            if _h.moe_grouped_ok(hn, self.w13, self.w2, a.experts, a.ff):
-                y32 = _h.moe_grouped(hn, self.w13, self.w2, idx, wsel, a.experts, a.ff, _h.EPI_SWIGLU)
-            else:
-                y32 = _h.linear(_h.linear_swiglu(hn, self.w13, rowscale=dense, group=a.ff), self.w2, epi=_h.EPI_F32)
+            y32 = _h.linear(_h.linear_swiglu(hn, self.w13, rowscale=dense, group=a.ff), self.w2, epi=_h.EPI_F32)
             if a.identity:
                 _h.rows_axpy(y32, hn, dense, a.experts)
-        if post is None:
-            x32.add_(y32)
-        else:
+        if post is not None:
             post(y32, add_to=x32)
+        elif y32 is not x32:
+            x32.add_(y32)
 
     def checkpoint_names(self) -> List[str]:
         return ["router", "correction"] + [f"e{e}.{n}" for e in range(self.a.experts) for n in ("gate", "up", "down")]

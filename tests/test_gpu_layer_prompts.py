@@ -56,6 +56,86 @@ def test_chosen_expert_rows(kind, T, width, ff, E, top, idle, monkeypatch):
     assert torch.equal(acc, base + got), "blocks of tokens and the sum into a stream change nothing"
 
 
+@pytest.mark.parametrize("E,identity,T", [(16, 4, 1030), (40, 8, 700), (3, 1, 129)])
+def test_identity_choices_of_grouped_experts(E, identity, T):
+    """Choices from E on are the token itself times the choice's weight, summed with the experts; without the flag they count nothing.  More than 32
+    experts: the plan's second round of lanes."""
+    from mistral_inference_b200 import _abi_hybrid as h
+
+    width, ff, top = 256, 128, min(4, E)
+    g = torch.Generator().manual_seed(E)
+    hn = torch.randn(T, width, generator=g).bfloat16().to(DEV)
+    w13 = (torch.randn(2 * E * ff, width, generator=g) / width ** 0.5).bfloat16().to(DEV)
+    w2 = (torch.randn(width, E * ff, generator=g) / ff ** 0.5).bfloat16().to(DEV)
+    idx = torch.stack([torch.randperm(E + identity, generator=g)[:top] for _ in range(T)]).int().to(DEV)
+    wts = torch.rand(T, top, generator=g).to(DEV) + 0.1
+    base = torch.randn(T, width, generator=g).to(DEV)
+    plain = h.moe_grouped(hn, w13, w2, idx, wts, E, ff, h.EPI_SWIGLU)
+    got = h.moe_grouped(hn, w13, w2, idx, wts, E, ff, h.EPI_SWIGLU, add_to=base.clone(), identity=True)
+    own = torch.where(idx >= E, wts, 0.0).double().sum(1, keepdim=True)
+    ref = base.double() + plain.double() + own * hn.double()
+    assert rel(got, ref) < 2e-7  # a handful of fp32 additions
+    ref = torch.zeros(T, width, dtype=torch.float64, device=DEV)
+    for e in range(E):
+        t, j = torch.nonzero(idx == e, as_tuple=True)
+        ref.index_add_(0, t, _unit("silu", hn[t].double() @ w13[2 * e * ff:2 * (e + 1) * ff].double().T, wts[t, j].double()[:, None], 0, 0) @ w2[:, e * ff:(e + 1) * ff].double().T)
+    assert rel(plain, ref) < 3 * 2 ** -9
+
+
+def _route64(x, w, corr, groups, keep, top, score, scale=1.0, renorm=False, group_two=False, w_bias=None):
+    """(weights [T, n], 0 where not chosen) in float64, and by how much the closest decision was made."""
+    z = x.double() @ w.double().T
+    if score == 2:
+        z = z + w_bias.double()
+        v, i = z.topk(top, 1)
+        return torch.zeros_like(z).scatter(1, i, torch.softmax(v, 1) * scale), i
+    s = torch.softmax(z, 1) if score == 0 else torch.sigmoid(z)
+    c = s + (corr.double() if corr is not None else 0)
+    if groups > 1 and keep < groups:
+        g = c.view(c.shape[0], groups, -1)
+        g = g.topk(2, 2).values.sum(2) if group_two else g.max(2).values
+        ok = torch.zeros_like(g, dtype=torch.bool).scatter(1, g.topk(keep, 1).indices, True)
+        c = c.masked_fill(~ok.repeat_interleave(c.shape[1] // groups, 1), -float("inf"))
+    i = c.topk(top, 1).indices
+    v = s.gather(1, i)
+    if renorm:
+        v = v / (v.sum(1, keepdim=True) + 1e-20)
+    return torch.zeros_like(z).scatter(1, i, v * scale), i
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n,groups,keep,top,kw", [(20, 4, 2, 4, dict(score=0)), (8, 1, 1, 2, dict(score=1, scale=2.5, renorm=True)), (33, 3, 2, 5, dict(score=1, group_two=True)),
+                                                  (32, 16, 3, 4, dict(score=1, group_two=True)), (16, 1, 1, 3, dict(score=2, always=1)), (7, 1, 1, 7, dict(score=0, gate=True))])
+def test_routers_of_prompts_and_of_few_tokens(n, groups, keep, top, kw, dt):
+    """From 700 tokens on a CTA routes four, below one: every sum in the same order, so the same bits; up to 32 outputs are chosen from in registers, more in shared
+    memory.  Against float64: fp32 sums of 328 products, the choices where they are not closer than that."""
+    from mistral_inference_b200 import _abi_hybrid as h
+
+    T, width = 1025, 328  # not a whole number of 256-element steps; the last CTA has one token
+    kw = dict(kw)
+    g = torch.Generator().manual_seed(n)
+    r = lambda *s: torch.randn(*s, generator=g).to(dt).to(DEV)  # noqa: E731
+    x, w, corr = r(T, width), r(n, width) / 8, r(n) / 10 if kw["score"] != 2 else None
+    if kw.pop("gate", False):
+        kw["w_gate"] = r(1, width) / 8
+    if kw["score"] == 2:
+        kw["w_bias"] = r(n)
+    whole = h.moe_route(x, w, corr, groups, keep, top, **kw)
+    parts = [h.moe_route(x[i:i + 205], w, corr, groups, keep, top, **kw) for i in range(0, T, 205)]
+    for a, b in zip(whole, zip(*parts)):
+        assert torch.equal(a, torch.cat(b))
+    always, gate = kw.pop("always", 0), kw.pop("w_gate", None)
+    ref, choice = _route64(x, w, corr, groups, keep, top, **kw)
+    dense, idx, wsel = whole[:3]
+    same = (idx[:, :top].long().sort(1).values == choice.sort(1).values).all(1)
+    assert same.float().mean() > 0.995, "choices differ only where two outputs are as good as equal"
+    assert rel(dense[same, :n], ref[same]) < 1e-5
+    assert torch.equal(dense[:, n:], torch.ones_like(dense[:, n:])) and (idx[:, top:] == n).all() and dense.shape[1] == n + always
+    assert torch.equal(dense.gather(1, idx.long()), wsel)
+    if gate is not None:
+        assert rel(whole[3], torch.sigmoid(x.double() @ gate.double().T)) < 1e-5
+
+
 def _scan64(q, k, v, decay, state, lens):
     """o [T, H, e] and the final states of sum_j decay^(i-j) (q_i . k_j) v_j in float64, token by token."""
     o, t = torch.empty(*v.shape, dtype=torch.float64, device=v.device), 0
