@@ -62,6 +62,9 @@ int mbh_attn_bias(const void* q, const void* cache_k, const void* cache_v, const
  * state fp32 [slots, H, d, e] is read (unless seqpos[b] == 0: starts at zero) and written back; o32 fp32 [T, H*e]. */
 int mbh_lightning_scan(const void* qkvg, void* state, const void* decay, const void* q_start, const void* seqpos, const void* slots, void* o32,
                        int64_t B, int64_t H, int64_t d, int64_t e, int dt, void* stream);
+/* The same result for prompts: the rows of the state dealt to four warps (mbh_lightning_scan keeps a decode step's one token). */
+int mbh_lightning_split(const void* qkvg, void* state, const void* decay, const void* q_start, const void* seqpos, const void* slots, void* o32,
+                        int64_t B, int64_t H, int64_t d, int64_t e, int dt, void* stream);
 
 /* The same over prompts in chunks of tokens, on tensor cores: bf16 storage, d 32, 64 or 128, e a multiple of 32, qkvg 16-byte aligned.
  * State, decayed values and decayed scores enter the products as three bf16 parts each: fp32 throughout. */

@@ -6,6 +6,7 @@
 #include "hybrid_lightning.cuh"
 #include "hybrid_linear.cuh"
 #include "hybrid_mixers.cuh"
+#include "hybrid_attn_f32.cuh"
 #include "hybrid_attn_flash.cuh"
 #include "hybrid_attn_decode.cuh"
 #include "hybrid_latent.cuh"
@@ -40,6 +41,13 @@ static cudaError_t launch_lightning(const LightningArgs& a, cudaStream_t st) {
     if (a.d <= 32) return launch_pdl(lightning_scan_kernel<T, 32>, grid, dim3(threads), 0, st, a);
     if (a.d <= 64) return launch_pdl(lightning_scan_kernel<T, 64>, grid, dim3(threads), 0, st, a);
     return launch_pdl(lightning_scan_kernel<T, 128>, grid, dim3(threads), 0, st, a);
+}
+template <typename T>
+static cudaError_t launch_lightning_split(const LightningArgs& a, cudaStream_t st) {
+    dim3 grid(a.B * a.H, (a.e + LS_COLS - 1) / LS_COLS);
+    if (a.d <= 32) return launch_pdl(lightning_split_kernel<T, 32>, grid, dim3(LS_THREADS), 0, st, a);
+    if (a.d <= 64) return launch_pdl(lightning_split_kernel<T, 64>, grid, dim3(LS_THREADS), 0, st, a);
+    return launch_pdl(lightning_split_kernel<T, 128>, grid, dim3(LS_THREADS), 0, st, a);
 }
 
 
@@ -247,6 +255,8 @@ int mbh_attn_window(const void* q, const void* cache_k, const void* cache_v, con
     if (dt == 0 && n_tiles > 0 && launch_attn_flash(a, (int)n_tiles, st, ferr)) {
         return ferr ? fail(ferr, "mbh_attn_bias (flash)") : 0;
     }
+    // in fp32: the same form with FMAs
+    if (dt == 1 && n_tiles > 0 && launch_attn_f32(a, n_tiles, st, ferr)) return ferr ? fail(ferr, "mbh_attn_bias (fp32)") : 0;
     if (maps == 2 && !scratch) return bad("mbh_attn_window: two maps need scratch outside the tensor-core prompt kernel");
     DISPATCH(dt, run_attn<ST>(a, smem, st));
     cudaError_t err = cudaGetLastError();
@@ -307,6 +317,17 @@ int mbh_lightning_scan(const void* qkvg, void* state, const void* decay, const v
     cudaError_t err = cudaSuccess;
     DISPATCH(dt, err = launch_lightning<ST>(a, (cudaStream_t)stream));
     return err ? fail(err, "mbh_lightning_scan") : 0;
+}
+
+int mbh_lightning_split(const void* qkvg, void* state, const void* decay, const void* q_start, const void* seqpos, const void* slots, void* o32,
+                        int64_t B, int64_t H, int64_t d, int64_t e, int dt, void* stream) {
+    if (B == 0) return 0;
+    if (d > 128) return bad("mbh_lightning_split: key size above 128");
+    LightningArgs a{qkvg, (float*)state, (const float*)decay, (const int*)q_start, (const int*)seqpos, (const int*)slots, (float*)o32,
+                    (int)B, (int)H, (int)d, (int)e};
+    cudaError_t err = cudaSuccess;
+    DISPATCH(dt, err = launch_lightning_split<ST>(a, (cudaStream_t)stream));
+    return err ? fail(err, "mbh_lightning_split") : 0;
 }
 
 int mbh_lightning_prompt(const void* qkvg, void* state, const void* decay, const void* q_start, const void* seqpos, const void* slots, void* o32,

@@ -613,6 +613,88 @@ __global__ void __launch_bounds__(LS_THREADS) lightning_scan_kernel(LightningArg
     }
 }
 
+constexpr int LS_PARTS = 4, LS_COLS = LS_THREADS / LS_PARTS;
+
+// The same for prompts: one CTA per (sequence, head, block of LS_COLS value columns), a lane per column; the state's DMAX rows are dealt to the four warps, DMAX / 4
+// registers a thread, whose shares of the outputs of LS_TB tokens meet in shared memory.  (With a column per thread a prompt of three sequences was 48 CTAs, 1300
+// cycles a token: 217 us for 301 tokens, 16 heads of 128; here 92.  A decode step's one token is mostly the state's way in and out: 5 us longer here, so it keeps the
+// kernel above.)  Keys and queries of LS_TB tokens at a time go through shared memory; the next LS_TB tokens are fetched into registers while the current ones
+// are consumed, so the scan does not wait for global memory.  Sequential in t, exact in fp32.
+template <typename T, int DMAX>
+__global__ void __launch_bounds__(LS_THREADS) lightning_split_kernel(LightningArgs a) {
+    constexpr int R = 2 * LS_TB * DMAX / LS_THREADS;  // staged values per thread and tile
+    constexpr int NS = DMAX / LS_PARTS;               // this thread's rows of the state
+    pdl_trigger();
+    pdl_wait();
+    __shared__ __align__(16) float ks[LS_TB][DMAX], qs[LS_TB][DMAX];
+    __shared__ float os[LS_PARTS][LS_TB][LS_COLS];
+    const int b = blockIdx.x / a.H, h = blockIdx.x % a.H, part = threadIdx.x / LS_COLS, col = threadIdx.x % LS_COLS;
+    const int c = blockIdx.y * LS_COLS + col;
+    const bool live = c < a.e;
+    const int t0 = a.q_start[b], t1 = a.q_start[b + 1];
+    const int stride = 2 * a.H * a.d + 2 * a.H * a.e;
+    const T* X = static_cast<const T*>(a.qkvg);
+    float* st = a.state + (((size_t)a.slots[b] * a.H + h) * a.d) * a.e;
+    const float dec = a.decay[h];
+    const T* vcol = X + 2 * a.H * a.d + h * a.e + (live ? c : 0);
+    float S[NS], pre[R], vnext[LS_TB];
+    const bool fresh = a.seqpos[b] == 0;
+    auto row = [&](int j) { return part * NS + j; };
+#pragma unroll
+    for (int j = 0; j < NS; ++j) S[j] = (live && !fresh && row(j) < a.d) ? st[(size_t)row(j) * a.e + c] : 0.f;
+
+    auto fetch = [&](int tb) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int idx = threadIdx.x + r * LS_THREADS;
+            const int tt = idx / (2 * DMAX), rem = idx % (2 * DMAX), which = rem / DMAX, i = rem % DMAX;
+            const bool ok = tb + tt < t1 && i < a.d;
+            pre[r] = ok ? to_f(X[(size_t)(tb + tt) * stride + (which ? a.H * a.d : 0) + h * a.d + i]) : 0.f;
+        }
+#pragma unroll
+        for (int tt = 0; tt < LS_TB; ++tt) vnext[tt] = tb + tt < t1 ? to_f(vcol[(size_t)(tb + tt) * stride]) : 0.f;
+    };
+    fetch(t0);
+    for (int tb = t0; tb < t1; tb += LS_TB) {
+        const int nt = min(LS_TB, t1 - tb);
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int idx = threadIdx.x + r * LS_THREADS;
+            const int tt = idx / (2 * DMAX), rem = idx % (2 * DMAX), which = rem / DMAX, i = rem % DMAX;
+            (which ? ks : qs)[tt][i] = pre[r];
+        }
+        float v[LS_TB];  // this column's values
+#pragma unroll
+        for (int tt = 0; tt < LS_TB; ++tt) v[tt] = vnext[tt];
+        __syncthreads();
+        if (tb + LS_TB < t1) fetch(tb + LS_TB);
+#pragma unroll
+        for (int tt = 0; tt < LS_TB; ++tt) {
+            if (tt >= nt) break;
+            float o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f;
+#pragma unroll
+            for (int j = 0; j < NS; j += 4) {
+                const float4 k4 = *reinterpret_cast<const float4*>(&ks[tt][row(j)]);
+                const float4 q4 = *reinterpret_cast<const float4*>(&qs[tt][row(j)]);
+                S[j] = fmaf(dec, S[j], k4.x * v[tt]);         o0 = fmaf(S[j], q4.x, o0);
+                S[j + 1] = fmaf(dec, S[j + 1], k4.y * v[tt]); o1 = fmaf(S[j + 1], q4.y, o1);
+                S[j + 2] = fmaf(dec, S[j + 2], k4.z * v[tt]); o2 = fmaf(S[j + 2], q4.z, o2);
+                S[j + 3] = fmaf(dec, S[j + 3], k4.w * v[tt]); o3 = fmaf(S[j + 3], q4.w, o3);
+            }
+            os[part][tt][col] = (o0 + o1) + (o2 + o3);
+        }
+        __syncthreads();
+        for (int tt = part; tt < nt; tt += LS_PARTS)
+            if (live) a.o[(size_t)(tb + tt) * a.H * a.e + h * a.e + c] = (os[0][tt][col] + os[1][tt][col]) + (os[2][tt][col] + os[3][tt][col]);
+    }
+    if (live) {
+#pragma unroll
+        for (int j = 0; j < NS; ++j)
+            if (row(j) < a.d) st[(size_t)row(j) * a.e + c] = S[j];
+    }
+}
+
 // y[t, :] = o[t, :] / sqrt(mean(o[t]^2) + eps) * w * sigmoid(g[t, :]); g lives at column `g_off` of rows of pitch `g_pitch`
 template <typename T>
 __global__ void gated_headnorm_kernel(const float* __restrict__ o, const T* __restrict__ w, const T* __restrict__ g, int g_pitch, int g_off,

@@ -136,6 +136,75 @@ def test_routers_of_prompts_and_of_few_tokens(n, groups, keep, top, kw, dt):
         assert rel(whole[3], torch.sigmoid(x.double() @ gate.double().T)) < 1e-5
 
 
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("form", ["plain", "bias", "window", "chunked", "cap_sink", "gate", "own"])
+@pytest.mark.parametrize("lens,past", [([33], [0]), ([1, 64, 31, 90], [5, 0, 40, 3]), ([32, 65], [130, 0])])
+def test_fp32_attention_of_prompts(d, form, lens, past):
+    """Tiles of 32 queries and 32 keys in fp32 against float64, and against the kernel of one CTA per token and head, than which they may not be less exact than by
+    fp32's own rounding.  A token's infinities in keys and values reach no query that does not see it."""
+    from mistral_inference_b200 import _abi_hybrid as h
+
+    H, G, W, B = 4, 2, 256, len(lens)
+    g = torch.Generator().manual_seed(sum(lens) + d)
+    r = lambda *s: torch.randn(*s, generator=g).to(DEV)  # noqa: E731
+    T = sum(lens)
+    q, ring_k, ring_v = r(T, H * d), r(B + 1, W, G, d), r(B + 1, W, G, d)
+    slots = torch.tensor([B - b for b in range(B)], dtype=torch.int32, device=DEV)
+    starts = [0]
+    for n in lens:
+        starts.append(starts[-1] + n)
+    positions = torch.tensor([p + i for n, p in zip(lens, past) for i in range(n)], dtype=torch.int32, device=DEV)
+    q_start, seqpos = (torch.tensor(v, dtype=torch.int32, device=DEV) for v in (starts, past))
+    scale, window, kw, bias = d ** -0.5, 0, {}, None
+    if form == "bias":
+        bias = r(20, H)
+    elif form == "window":
+        window = 37
+    elif form == "chunked":
+        window, kw = 48, dict(chunked=True)
+    elif form == "cap_sink":
+        kw = dict(softcap=2.0, sink=r(H))
+    elif form == "gate":
+        kw = dict(gate=r(T, H * d), gate_entry=True)
+    elif form == "own":
+        kw = dict(own_k=r(T, G * d), own_v=r(T, G * d), seqpos=seqpos)
+    ring_k[slots[0].long(), past[0] + lens[0] - 1] = float("inf")  # the first sequence's last token
+    ring_v[slots[0].long(), past[0] + lens[0] - 1] = float("nan")
+
+    def run(tiles):
+        out = torch.empty(T, H * d, device=DEV)
+        if form == "bias":
+            h.attn_bias(q, ring_k, ring_v, bias, positions, q_start, slots, out, B, W, H, G, d, d, scale, n_tiles=tiles)
+        else:
+            h.attn_window(q, ring_k, ring_v, positions, q_start, slots, out, B, W, H, G, d, d, scale, window, n_tiles=tiles, **kw)
+        return out
+
+    got, old = run(sum((n + 63) // 64 for n in lens)), run(0)
+    ref = torch.empty(T, H * d, dtype=torch.float64, device=DEV)
+    for b in range(B):
+        for i in range(lens[b]):
+            t, p = starts[b] + i, past[b] + i
+            lo = 0 if not window else (p - p % window if kw.get("chunked") else max(0, p - window + 1))
+            k, v = (c[slots[b].long(), lo:p + 1].double() for c in (ring_k, ring_v))
+            if form == "own":
+                m = past[b] - lo
+                k = torch.cat([k[:m], kw["own_k"][starts[b]:t + 1].view(-1, G, d).double()])
+                v = torch.cat([v[:m], kw["own_v"][starts[b]:t + 1].view(-1, G, d).double()])
+            s = torch.einsum("hd,khd->hk", q[t].view(H, d).double(), k.repeat_interleave(H // G, 1)) * scale
+            if form == "cap_sink":
+                s = torch.cat([2 * torch.tanh(s / 2), kw["sink"].double()[:, None]], 1)
+            if bias is not None:
+                s = s + bias.double()[(p - torch.arange(lo, p + 1, device=DEV)).clamp(max=19)].T
+            w = torch.softmax(s, 1)[:, :k.shape[0]]
+            o = torch.einsum("hk,khd->hd", w, v.repeat_interleave(H // G, 1)).flatten()
+            ref[t] = o * torch.sigmoid(kw["gate"][t].double()) if form == "gate" else o
+    fine = torch.ones(T, dtype=torch.bool, device=DEV)
+    fine[starts[1] - 1] = form == "own"  # (own rows: the ring's are not read)
+    assert torch.isfinite(got[fine]).all()
+    assert rel(got[fine], ref[fine]) < max(1.5 * rel(old[fine], ref[fine]), 3e-7)
+    assert not torch.isfinite(got[~fine]).any() or form == "cap_sink"
+
+
 def _scan64(q, k, v, decay, state, lens):
     """o [T, H, e] and the final states of sum_j decay^(i-j) (q_i . k_j) v_j in float64, token by token."""
     o, t = torch.empty(*v.shape, dtype=torch.float64, device=v.device), 0
@@ -145,6 +214,32 @@ def _scan64(q, k, v, decay, state, lens):
             o[t] = (state[b] * q[t][:, :, None]).sum(1)
             t += 1
     return o, state
+
+
+@pytest.mark.parametrize("H,d,e", [(2, 128, 96), (3, 64, 40), (1, 100, 33), (2, 32, 7)])
+@pytest.mark.parametrize("lens", [[8], [17, 1, 16], [33, 40]])
+def test_lightning_scan_of_prompts(H, d, e, lens):
+    """fp32 prompts: the state's rows in four warps, tiles of 16 tokens, value columns in blocks of 32, against float64 and the scan of a column per thread: the
+    same state bit for bit, outputs to the rounding of a sum of d products."""
+    from mistral_inference_b200 import _abi_hybrid as h
+
+    g = torch.Generator().manual_seed(d + e)
+    T, B = sum(lens), len(lens)
+    x = torch.randn(T, 2 * H * d + 2 * H * e, generator=g).to(DEV)
+    q, k, v = x[:, :H * d].view(T, H, d).double(), x[:, H * d:2 * H * d].view(T, H, d).double(), x[:, 2 * H * d:2 * H * d + H * e].reshape(T, H, e).double()
+    decay = torch.linspace(0.5, 0.99, H).to(DEV)
+    start = [0]
+    for n in lens:
+        start.append(start[-1] + n)
+    q_start, seqpos, slots = (torch.tensor(t, dtype=torch.int32, device=DEV) for t in (start, [i % 2 * 5 for i in range(B)], list(range(B))))
+    first = torch.randn(B, H, d, e, generator=g).to(DEV)
+    states, outs = [first.clone(), first.clone()], [torch.empty(T, H * e, device=DEV) for _ in range(2)]
+    h.lightning_scan(x, states[0], decay, q_start, seqpos, slots, outs[0], B, H, d, e, longest=max(8, max(lens)))
+    h.lightning_scan(x, states[1], decay, q_start, seqpos, slots, outs[1], B, H, d, e, longest=1)
+    want = first.double() * (seqpos > 0)[:, None, None, None]
+    o, want = _scan64(q, k, v, decay.double(), want, lens)
+    assert torch.equal(states[0], states[1]) and rel(states[0], want) < 1e-6
+    assert rel(outs[0], o.flatten(1)) < max(1.2 * rel(outs[1], o.flatten(1)), 2e-7)
 
 
 @pytest.mark.parametrize("H,d,e", [(3, 128, 128), (2, 64, 96), (5, 32, 32)])
