@@ -404,10 +404,10 @@ int mb200_moe_route(const void* hn, const void* gate_w, int64_t T, int64_t dim, 
   const int64_t pairs = T * top_k, cap = moe_tile_cap(pairs, n_experts, tile_rows);
   const size_t plan_smem = moe_plan_smem(n_experts);
   MB_CHECK_CUDA(cudaFuncSetAttribute(moe_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan_smem));
-  moe_plan_kernel<<<1, MP_THREADS, plan_smem, st>>>(sel, (int)pairs, (int)n_experts, tile_rows, (int)shard_rank, (int)shard_world, (int)cap, slot, plan);
+  MB_CHECK_CUDA(launch_pdl(moe_plan_kernel, dim3(1), dim3(MP_THREADS), plan_smem, st, sel, (int)pairs, (int)n_experts, tile_rows, (int)shard_rank, (int)shard_world, (int)cap, slot, plan));
   MB_CHECK_LAUNCH("moe_plan_kernel");
-  moe_gather_kernel<<<(unsigned)ceil_div(pairs, 8), 256, 0, st>>>((const uint4*)hn, sel, (const bf16*)wts, slot, (int)pairs, (int)top_k, (int)(dim / 8),
-                                                                  (int)shard_rank, (int)shard_world, (uint4*)xs, (bf16*)row_w);
+  MB_CHECK_CUDA(launch_pdl(moe_gather_kernel, dim3((unsigned)ceil_div(pairs, 8)), dim3(256), 0, st, (const uint4*)hn, sel, (const bf16*)wts, slot, (int)pairs, (int)top_k,
+                           (int)(dim / 8), (int)shard_rank, (int)shard_world, (uint4*)xs, (bf16*)row_w));
   MB_CHECK_LAUNCH("moe_gather_kernel");
   return MB200_OK;
 }
@@ -472,7 +472,7 @@ int mb200_moe_grouped_ffn(const void* xs, const void* const* w13_host, const voi
       c.peer_flags[r] = (unsigned*)comm->peer_flags[r];
     }
   }
-  moe_combine_kernel<<<(unsigned)T, 128, 0, st>>>(c);
+  MB_CHECK_CUDA(launch_pdl(moe_combine_kernel, dim3((unsigned)T), dim3(128), 0, st, c));
   MB_CHECK_LAUNCH("moe_combine_kernel");
   return MB200_OK;
 }
@@ -581,9 +581,10 @@ int mb200_layer_moe(const void* hn, const void* w13, const void* w2, const int32
   const int64_t pairs = T * top, cap = moe_tile_cap(pairs, n_experts, TG_BM), rows_cap = cap * TG_BM;
   const size_t plan_smem = moe_plan_smem(n_experts);
   MB_CHECK_CUDA(cudaFuncSetAttribute(moe_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan_smem));
-  moe_plan_kernel<<<1, MP_THREADS, plan_smem, st>>>(idx, (int)pairs, (int)n_experts, TG_BM, 0, 1, (int)cap, slot, plan);
+  MB_CHECK_CUDA(launch_pdl(moe_plan_kernel, dim3(1), dim3(MP_THREADS), plan_smem, st, idx, (int)pairs, (int)n_experts, TG_BM, 0, 1, (int)cap, slot, plan));
   MB_CHECK_LAUNCH("moe_plan_kernel");
-  layer_moe_gather_kernel<<<(unsigned)ceil_div(pairs, 8), 256, 0, st>>>((const uint4*)hn, wsel, slot, (int)pairs, (int)top, (int)(dim / 8), (uint4*)xs, row_w);
+  MB_CHECK_CUDA(launch_pdl(layer_moe_gather_kernel, dim3((unsigned)ceil_div(pairs, 8)), dim3(256), 0, st, (const uint4*)hn, wsel, slot, (int)pairs, (int)top, (int)(dim / 8),
+                           (uint4*)xs, row_w));
   MB_CHECK_LAUNCH("layer_moe_gather_kernel");
   EpiParams e1, e2;
   int rc = layer_epilogue(e1, nullptr, act, nullptr, units, epi, 0, limit, alpha);
@@ -597,8 +598,8 @@ int mb200_layer_moe(const void* hn, const void* w13, const void* w2, const int32
   if (rc) return rc;
   rc = launch_grouped_packed(act, rows_cap, ff, dim, w2, dim, n_experts * ff, 0, ff, pairs, n_experts, plan, e2, st);
   if (rc) return rc;
-  layer_moe_combine_kernel<<<dim3((unsigned)ceil_div(dim / 4, 256), (unsigned)T), 256, 0, st>>>((const float4*)rows32, slot, wsel, (const uint2*)hn, (float4*)y32, (int)top,
-                                                                                            (int)(dim / 4), add & 1, add & 2);
+  MB_CHECK_CUDA(launch_pdl(layer_moe_combine_kernel, dim3((unsigned)ceil_div(dim / 4, 256), (unsigned)T), dim3(256), 0, st, (const float4*)rows32, slot, wsel, (const uint2*)hn,
+                           (float4*)y32, (int)top, (int)(dim / 4), add & 1, add & 2));
   MB_CHECK_LAUNCH("layer_moe_combine_kernel");
   return MB200_OK;
 }

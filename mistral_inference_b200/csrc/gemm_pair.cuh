@@ -85,6 +85,7 @@ constexpr int GP_SMEM = 227 * 1024;
 template <int MODE, bool GROUPED>
 __device__ __forceinline__ void pair_gemm_body(const CUtensorMap& map_a, const CUtensorMap* map_w_base, const PairParams& p, const int32_t* plan) {
   extern __shared__ uint8_t smem_raw[];
+  if (GROUPED) pdl_wait();  // the plan
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);  // SW128 wants 1024-B tiles
   uint8_t* turn = smem + kPairRing<MODE>;
   uint64_t* full = reinterpret_cast<uint64_t*>(turn + kPairTurn<MODE>);
@@ -170,6 +171,8 @@ __device__ __forceinline__ void pair_gemm_body(const CUtensorMap& map_a, const C
   cluster_sync_all();  // the peer's barriers must be initialised before any copy or commit reaches them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_base_slot;
+  pdl_trigger();
+  if (!GROUPED) pdl_wait();  // barriers, tensor memory and the cluster's meeting are behind the predecessor's end
 
   if (warp == 0) {
     // ================= TMA producer =================
@@ -466,13 +469,15 @@ int launch_pairs(Kernel kernel, int clusters, cudaStream_t stream, const Args&..
   cfg.blockDim = dim3(GP_THREADS);
   cfg.dynamicSmemBytes = GP_SMEM;
   cfg.stream = stream;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = 2;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
   MB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
   MB_CHECK_LAUNCH("gemm_pair_kernel");
   return MB200_OK;

@@ -121,6 +121,8 @@ constexpr int MP_THREADS = 1024, MP_ROW = MP_THREADS + MP_THREADS / 32;
 inline size_t moe_plan_smem(int64_t E) { return ((size_t)E * MP_ROW + 2 * E + 1) * sizeof(int32_t); }
 __global__ void __launch_bounds__(MP_THREADS) moe_plan_kernel(const int32_t* __restrict__ sel, int pairs, int E, int tile_rows, int shard_rank,
                                                               int shard_world, int tile_cap, int32_t* __restrict__ slot, int32_t* __restrict__ plan) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ int32_t sm[];  // cnt[E][MP_ROW], then seg[E + 1], total[E]
   int32_t* cnt = sm;
   int32_t* seg = sm + E * MP_ROW;
@@ -258,6 +260,8 @@ __global__ void __launch_bounds__(MP_THREADS) moe_plan_kernel(const int32_t* __r
 __global__ void __launch_bounds__(256) moe_gather_kernel(const uint4* __restrict__ hn, const int32_t* __restrict__ sel, const bf16* __restrict__ wts,
                                                          const int32_t* __restrict__ slot, int pairs, int k, int row_chunks, int shard_rank,
                                                          int shard_world, uint4* __restrict__ xs, bf16* __restrict__ row_w) {
+  pdl_trigger();
+  pdl_wait();
   const int pair = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (pair >= pairs) return;
   if (sel[pair] % shard_world != shard_rank) return;  // another rank's expert
@@ -292,6 +296,8 @@ __device__ __forceinline__ void st_release_sys_u32(unsigned* p, unsigned v) {
 }
 
 __global__ void __launch_bounds__(128) moe_combine_kernel(const MoeCombineParams p) {
+  pdl_trigger();
+  pdl_wait();
   const int t = blockIdx.x;
   if (p.n_ranks > 1) {
     // This kernel starts after this rank's down projection has finished (stream order), i.e. after its peer stores were issued
@@ -524,6 +530,8 @@ int launch_grouped(const void* a, int64_t rows_cap, int64_t K, int64_t N, const 
 // 800 us before (all experts on all tokens), 291 us now, of which 150 us are the grouped GEMMs and 49 us the router.
 __global__ void __launch_bounds__(256) layer_moe_gather_kernel(const uint4* __restrict__ hn, const float* __restrict__ wsel, const int32_t* __restrict__ slot,
                                                                int pairs, int k, int row_chunks, uint4* __restrict__ xs, float* __restrict__ row_w) {
+  pdl_trigger();
+  pdl_wait();
   const int pair = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (pair >= pairs) return;
   const int s = slot[pair];
@@ -538,6 +546,8 @@ __global__ void __launch_bounds__(256) layer_moe_gather_kernel(const uint4* __re
 // identity: a choice without a row is an identity expert, the token itself (hn) times the choice's weight
 __global__ void __launch_bounds__(256) layer_moe_combine_kernel(const float4* __restrict__ rows, const int32_t* __restrict__ slot, const float* __restrict__ wsel,
                                                                 const uint2* __restrict__ hn, float4* __restrict__ y, int k, int row_quads, int add, int identity) {
+  pdl_trigger();
+  pdl_wait();
   const int c = blockIdx.x * 256 + threadIdx.x, t = blockIdx.y;
   if (c >= row_quads) return;
   const int32_t* sl = slot + (int64_t)t * k;
