@@ -114,7 +114,7 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())  # torch.cuda.current_stream().cuda_stream without its objects
 
 
 class Workspace:

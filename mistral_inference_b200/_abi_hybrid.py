@@ -103,7 +103,7 @@ def _rows(x: torch.Tensor):
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())  # torch.cuda.current_stream().cuda_stream without its objects
 
 
 def dt_of(dtype: torch.dtype) -> int:

@@ -225,38 +225,64 @@ class BufferCache:
         assert len(seqlens) == len(self._kv_seqlens_host), (
             f"Batch size is {len(self._kv_seqlens_host)}, got {len(seqlens)}, did you forget to reset cache?")
         assert len(seqlens) > 0, seqlens
-        seqpos = np.asarray(self._kv_seqlens_host, dtype=np.int64)
-        sl = np.asarray(seqlens, dtype=np.int64)
-        B, T = len(seqlens), int(sl.sum())
-        first_prefill = bool(seqpos[0] == 0)
-        subsequent_prefill = bool((sl > 1).any())
+        B, T = len(seqlens), int(sum(seqlens))
+        first_prefill = self._kv_seqlens_host[0] == 0
         if first_prefill:
-            assert (seqpos == 0).all(), seqpos.tolist()  # cache.py:239
+            assert not any(self._kv_seqlens_host), self._kv_seqlens_host  # cache.py:239
+        distinct = sorted(set(self.cache_sizes))
+        with_slots = self.layer_specs is not None  # kernels of layered models take the row block of each sequence
+        assert with_slots or self.rows == list(range(B)), "this model's kernels address sequence b at row block b"
+        total = T + (B + 1) + B + len(distinct) * (T + B) + (B if with_slots else 0)
+        host = np.empty(total, dtype=np.int32)
+        longest = int(max(seqlens))
+        layout = {"T": T, "B": B, "prefill": first_prefill or longest > 1, "first_prefill": first_prefill, "max_seqlen": longest, "windows": distinct}
+        (self._fill_tokens if B > 16 else self._fill_sequences)(host, [int(n) for n in seqlens], T, distinct)
+        if with_slots:
+            host[total - B:] = self.rows
+        layout["slots"] = with_slots
+        return host, layout
+
+    def _fill_sequences(self, host: np.ndarray, lens: List[int], T: int, windows: List[int]) -> None:
+        """The block of few sequences, one after the other: three small calls each, where _fill_tokens makes some thirty over all tokens (five sequences 17 us
+        instead of 28)."""
+        B, past, t = len(lens), self._kv_seqlens_host, 0
+        o = T + 2 * B + 1
+        host[T] = 0
+        for b, (n, p, slot) in enumerate(zip(lens, past, self.rows)):
+            seq = np.arange(p, p + n, dtype=np.int32)
+            host[t:t + n] = seq
+            for j, W in enumerate(windows):
+                at = o + j * (T + B)
+                if p + n <= W:
+                    np.add(seq, slot * W, out=host[at + t:at + t + n])
+                else:
+                    rows = seq % W
+                    rows += slot * W
+                    rows[:max(0, n - W)] = -1  # only the last W tokens of each chunk (cache.py:226)
+                    host[at + t:at + t + n] = rows
+                host[at + T + b] = min(p + min(n, W), W)
+            t += n
+            host[T + 1 + b] = t
+            host[T + B + 1 + b] = p
+
+    def _fill_tokens(self, host: np.ndarray, lens: List[int], T: int, windows: List[int]) -> None:
+        """The block of many sequences, over all their tokens at once."""
+        B = len(lens)
+        seqpos, sl, slot = (np.asarray(v, dtype=np.int64) for v in (self._kv_seqlens_host, lens, self.rows))
         q_start = np.zeros(B + 1, dtype=np.int64)
         np.cumsum(sl, out=q_start[1:])
         batch_idx = np.repeat(np.arange(B, dtype=np.int64), sl)
         local = np.arange(T, dtype=np.int64) - q_start[batch_idx]
         positions = seqpos[batch_idx] + local
-        distinct = sorted(set(self.cache_sizes))
-        slot = np.asarray(self.rows, dtype=np.int64)
-        with_slots = self.layer_specs is not None  # kernels of layered models take the row block of each sequence
-        assert with_slots or self.rows == list(range(B)), "this model's kernels address sequence b at row block b"
-        total = T + (B + 1) + B + len(distinct) * (T + B) + (B if with_slots else 0)
-        host = np.empty(total, dtype=np.int32)
-        layout = {"T": T, "B": B, "prefill": first_prefill or subsequent_prefill, "first_prefill": first_prefill, "max_seqlen": int(sl.max()), "windows": distinct}
         o = 0
         host[o:o + T] = positions; o += T
         host[o:o + B + 1] = q_start; o += B + 1
         host[o:o + B] = seqpos; o += B
-        for W in distinct:
+        for W in windows:
             cached = local >= (sl[batch_idx] - W)  # only the last W tokens of each chunk (cache.py:226)
             rows = np.where(cached, positions % W + slot[batch_idx] * W, -1)
             host[o:o + T] = rows; o += T
             host[o:o + B] = np.minimum(seqpos + np.minimum(sl, W), W); o += B
-        if with_slots:
-            host[o:o + B] = slot; o += B
-        layout["slots"] = with_slots
-        return host, layout
 
     def metadata_from_block(self, dev: torch.Tensor, layout: dict, seqlens: List[int]) -> List[CacheInputMetadata]:
         T, B = layout["T"], layout["B"]
