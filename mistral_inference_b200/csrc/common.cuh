@@ -96,6 +96,8 @@ inline int ceil_div(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
 // transitively, everything before it).  A kernel signals with pdl_trigger() that its dependents may be scheduled; the hardware
 // launches them only when EVERY CTA of this grid has triggered or exited, i.e. when this grid no longer needs SM resources.
 // Both are no-ops in a kernel launched the ordinary way.  MB200_PDL=0 launches everything the ordinary way.
+// What a predecessor writes is never a `const __restrict__` parameter of such a kernel: the qualifier promises that nobody writes it while the grid
+// lives, so its loads may take the read-only path and move above pdl_wait().  (Weights may be.)
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

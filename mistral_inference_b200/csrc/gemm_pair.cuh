@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
 }
 template <int MODE>
 __global__ void __launch_bounds__(GP_THREADS, 1)
-    gemm_pair_grouped_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ MoeWeightMaps maps_w, const PairParams p, const int32_t* __restrict__ plan) {
+    gemm_pair_grouped_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ MoeWeightMaps maps_w, const PairParams p, const int32_t* plan) {
   pair_gemm_body<MODE, true>(map_a, maps_w.m, p, plan);
 }
 

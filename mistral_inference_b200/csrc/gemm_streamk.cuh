@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(TG_THREADS, 2)  // <= 168 registers: the reduc
 template <int MODE, int TA>
 __global__ void __launch_bounds__(TG_THREADS, 2)
     gemm_streamk_grouped_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ MoeWeightMaps maps_w, const SkParams p,
-                                const int32_t* __restrict__ plan) {
+                                const int32_t* plan) {
   sk_gemm_body<MODE, TA, true>(map_a, maps_w.m, p, plan);
 }
 

@@ -104,6 +104,8 @@ __device__ __forceinline__ float softcap_fast(float x, float cap, float two_over
 // touches nothing that an earlier kernel writes (weights only).  pdl_wait() returns when the predecessor has completed and its writes are
 // visible.  Both are no-ops in a kernel launched the ordinary way.  A decode step is some 80 short kernels: their launches and first loads
 // otherwise stand in the open.
+// What a predecessor writes is never a `const __restrict__` parameter of such a kernel: the qualifier promises that nobody writes it while the grid
+// lives, so its loads may take the read-only path and move above pdl_wait().  (Weights may be.)
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <typename... KArgs, typename... Args>

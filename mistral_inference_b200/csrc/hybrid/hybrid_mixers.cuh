@@ -21,7 +21,7 @@ namespace mbh {
 
 // ------------------------------------------------------------------------------------------------ embedding, norm
 template <typename T, bool ADD = false>
-__global__ void embed_scale_kernel(const int64_t* __restrict__ tok, const T* __restrict__ E, float scale, float* __restrict__ x, int D) {
+__global__ void embed_scale_kernel(const int64_t* tok, const T* __restrict__ E, float scale, float* __restrict__ x, int D) {
     pdl_trigger();
     pdl_wait();
     const T* row = E + (size_t)tok[blockIdx.x] * D;
@@ -71,7 +71,7 @@ __global__ void layernorm_f32_kernel(const float* __restrict__ x, const T* __res
 // One fp32 row per CTA.  w2 / y2 (both or neither): a second norm of the same row with its own weight.  offset: what the stored weight counts
 // from (0: the weight itself, 1: a weight stored around zero)
 template <typename T>
-__global__ void rmsnorm_f32_kernel(const float* __restrict__ x, const T* __restrict__ w, const T* __restrict__ w2, T* __restrict__ y, T* __restrict__ y2, int D,
+__global__ void rmsnorm_f32_kernel(const float* x, const T* __restrict__ w, const T* __restrict__ w2, T* __restrict__ y, T* __restrict__ y2, int D,
                                    float eps, float offset) {
     __shared__ float red[32];
     pdl_trigger();
@@ -441,7 +441,7 @@ __global__ void __launch_bounds__(AT_WARPS * 32) attn_bias_kernel(AttnArgs a) {
 // loads in flight).  grid (token * head, blocks of blockDim columns)
 constexpr int AT_MAX_SPLITS = 64;
 template <typename T>
-__global__ void attn_merge_kernel(const float* __restrict__ scratch, T* __restrict__ out, int splits, int e, int sigmoid = 0, const float* __restrict__ sink = nullptr,
+__global__ void attn_merge_kernel(const float* scratch, T* __restrict__ out, int splits, int e, int sigmoid = 0, const float* __restrict__ sink = nullptr,
                                   int H = 1, const void* gate = nullptr, int gate_pitch = 0, int gate_entry = 0) {
     __shared__ float f[AT_MAX_SPLITS];
     __shared__ float red[32];
@@ -697,7 +697,7 @@ __global__ void __launch_bounds__(LS_THREADS) lightning_split_kernel(LightningAr
 
 // y[t, :] = o[t, :] / sqrt(mean(o[t]^2) + eps) * w * sigmoid(g[t, :]); g lives at column `g_off` of rows of pitch `g_pitch`
 template <typename T>
-__global__ void gated_headnorm_kernel(const float* __restrict__ o, const T* __restrict__ w, const T* __restrict__ g, int g_pitch, int g_off,
+__global__ void gated_headnorm_kernel(const float* o, const T* __restrict__ w, const T* g, int g_pitch, int g_off,
                                       T* __restrict__ y, int N, float eps) {
     __shared__ float red[32];
     pdl_trigger();

@@ -29,7 +29,7 @@ constexpr int MOE_MAX_TOPK = 8;
 // ---- router: one warp per token (WIDE = false: prefill) or one CTA per token with the 8 warps splitting the row (WIDE = true:
 // decode-sized batches, where a single warp walking 4096 dims x 8 experts is pure load latency: 36 us measured for 8 tokens) ------
 template <int E, bool WIDE>
-__global__ void __launch_bounds__(256) moe_route_kernel(const bf16* __restrict__ hn, const bf16* __restrict__ gate_w, int T, int dim, int k,
+__global__ void __launch_bounds__(256) moe_route_kernel(const bf16* hn, const bf16* __restrict__ gate_w, int T, int dim, int k,
                                                         int32_t* __restrict__ sel, bf16* __restrict__ wts) {
   pdl_trigger();
   pdl_wait();  // hn is the preceding RMSNorm's output
@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(256) moe_route_kernel(const bf16* __restrict__
 // expert e's segment (e = 0..E), then tile_expert[capacity], tile_row0[capacity] from word MOE_PLAN_HEADER.
 constexpr int MP_THREADS = 1024, MP_ROW = MP_THREADS + MP_THREADS / 32;
 inline size_t moe_plan_smem(int64_t E) { return ((size_t)E * MP_ROW + 2 * E + 1) * sizeof(int32_t); }
-__global__ void __launch_bounds__(MP_THREADS) moe_plan_kernel(const int32_t* __restrict__ sel, int pairs, int E, int tile_rows, int shard_rank,
+__global__ void __launch_bounds__(MP_THREADS) moe_plan_kernel(const int32_t* sel, int pairs, int E, int tile_rows, int shard_rank,
                                                               int shard_world, int tile_cap, int32_t* __restrict__ slot, int32_t* __restrict__ plan) {
   pdl_trigger();
   pdl_wait();
@@ -257,8 +257,7 @@ __global__ void __launch_bounds__(MP_THREADS) moe_plan_kernel(const int32_t* __r
 }
 
 // ---- gather: one warp per (token, expert) pair ------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) moe_gather_kernel(const uint4* __restrict__ hn, const int32_t* __restrict__ sel, const bf16* __restrict__ wts,
-                                                         const int32_t* __restrict__ slot, int pairs, int k, int row_chunks, int shard_rank,
+__global__ void __launch_bounds__(256) moe_gather_kernel(const uint4* hn, const int32_t* sel, const bf16* wts, const int32_t* slot, int pairs, int k, int row_chunks, int shard_rank,
                                                          int shard_world, uint4* __restrict__ xs, bf16* __restrict__ row_w) {
   pdl_trigger();
   pdl_wait();
@@ -528,7 +527,7 @@ int launch_grouped(const void* a, int64_t rows_cap, int64_t K, int64_t N, const 
 // The experts lie packed in one matrix each (w13 [E * units, width], w2 [width, E * ff]): one tensor map, offsets by expert.
 // Choices >= E (identity experts) get no row.  A mixture's prompt of 2500 tokens, 16 experts of 1408, top 4 of 20 outputs, width 2048:
 // 800 us before (all experts on all tokens), 291 us now, of which 150 us are the grouped GEMMs and 49 us the router.
-__global__ void __launch_bounds__(256) layer_moe_gather_kernel(const uint4* __restrict__ hn, const float* __restrict__ wsel, const int32_t* __restrict__ slot,
+__global__ void __launch_bounds__(256) layer_moe_gather_kernel(const uint4* hn, const float* wsel, const int32_t* slot,
                                                                int pairs, int k, int row_chunks, uint4* __restrict__ xs, float* __restrict__ row_w) {
   pdl_trigger();
   pdl_wait();
@@ -544,8 +543,7 @@ __global__ void __launch_bounds__(256) layer_moe_gather_kernel(const uint4* __re
 }
 
 // identity: a choice without a row is an identity expert, the token itself (hn) times the choice's weight
-__global__ void __launch_bounds__(256) layer_moe_combine_kernel(const float4* __restrict__ rows, const int32_t* __restrict__ slot, const float* __restrict__ wsel,
-                                                                const uint2* __restrict__ hn, float4* __restrict__ y, int k, int row_quads, int add, int identity) {
+__global__ void __launch_bounds__(256) layer_moe_combine_kernel(const float4* rows, const int32_t* slot, const float* wsel, const uint2* hn, float4* __restrict__ y, int k, int row_quads, int add, int identity) {
   pdl_trigger();
   pdl_wait();
   const int c = blockIdx.x * 256 + threadIdx.x, t = blockIdx.y;

@@ -15,3 +15,18 @@ def test_no_copy_is_multicast_to_a_cluster(path):
     copies = re.findall(r'"[^"\n]*cp\.async\.bulk[^"\n]*"', text)
     assert not [c for c in copies if "multicast" in c]
     assert path.name != "gemm_tcgen05.cuh" or len(copies) >= 3
+
+
+WEIGHTS = {"w", "w2", "E", "gate_w", "sink"}  # parameters that only loading a model writes
+
+
+@pytest.mark.parametrize("files", ["*.cu*", "hybrid/*.cu*"])
+def test_what_a_predecessor_writes_is_no_read_only_parameter(files):
+    """Kernels launched programmatically are resident while their predecessor still writes what they will read.  `const __restrict__` promises that nobody
+    does, and lets the compiler read it through the read-only path, or before the wait: only weights may be declared so."""
+    text = "\n".join(re.sub(r"//[^\n]*", "", p.read_text()) for p in sorted(CSRC.glob(files)))
+    params = dict(re.findall(r"__global__[^;{]*?\b(\w+)\(((?:[^(){}]|\([^()]*\))*)\)\s*\{", text))
+    launched = set(re.findall(r"\blaunch_(?:pdl|pairs)\(\s*(\w+)", text)) & set(params)
+    assert len(launched) >= 9, launched
+    read_only = {k: set(re.findall(r"const\s+[\w:]+\s*\*\s*__restrict__\s+(\w+)", params[k])) - WEIGHTS for k in launched}
+    assert not {k: v for k, v in read_only.items() if v}
