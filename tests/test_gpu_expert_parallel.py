@@ -1,13 +1,14 @@
-"""Expert-parallel MoE with the real kernels: each rank owns the experts e % world == rank of a small Mixtral-style
-model; the down projection's epilogue stores every weighted expert row into every rank's row buffer (CUDA-IPC peer memory), a
-flag handshake follows, and every rank combines all rows in the reference's order (csrc/moe.cuh).  Prefill + decode logits must
-equal the UNSHARDED model's bit for bit -- for top-2 and for top-3 routing (no reduction order is left open).
+"""Expert-parallel MoE with the real kernels: each rank owns the experts e % world == rank of a small Mixtral-style model; the down
+projection's epilogue stores every weighted expert row into every rank's row buffer (CUDA-IPC peer memory), a flag handshake follows, and
+every rank combines all rows in the reference's order (csrc/moe.cuh).  Prefill + decode logits must equal the UNSHARDED model's bit for
+bit -- for top-2 and for top-3 routing (no reduction order is left open).
 
 Two set-ups:
-  * two processes sharing cuda:0 (gloo for the handle exchange): one GPU is enough, peer stores go through IPC mappings of the
-    same device; the handshake spins across time slices, so it is slow but exercises the whole protocol;
-  * one process per GPU with NCCL (needs >= 2 GPUs: `gpurun --gpus 2`): peer stores cross NVLink.
+  * the ranks' calls one after the other on one GPU, in one process: "peer" buffers are other tensors, and the handshake's flags are set
+    beforehand, so no kernel waits for another (kernels that wait for one another are never separate launches on one GPU);
+  * one process per GPU with NCCL (needs >= 2 GPUs): peer stores cross NVLink.
 """
+import ctypes
 import os
 import socket
 import sys
@@ -27,16 +28,12 @@ def _free_port() -> int:
         return s.getsockname()[1]
 
 
-def _worker(rank: int, world: int, port: int, q, backend: str, top_k: int):
+def _worker(rank: int, world: int, port: int, q, top_k: int):
     try:
         sys.path.insert(0, str(REPO))
         os.environ.update(MASTER_ADDR="127.0.0.1", MASTER_PORT=str(port), RANK=str(rank), WORLD_SIZE=str(world))
-        dev = rank if backend == "nccl" else 0
-        torch.cuda.set_device(dev)
-        if backend == "nccl":
-            torch.distributed.init_process_group("nccl", rank=rank, world_size=world, device_id=torch.device("cuda", dev))
-        else:
-            torch.distributed.init_process_group("gloo", rank=rank, world_size=world)
+        torch.cuda.set_device(rank)
+        torch.distributed.init_process_group("nccl", rank=rank, world_size=world, device_id=torch.device("cuda", rank))
         import mistral_inference_b200 as mi
         import synth
         from mistral_inference_b200.cache import BufferCache
@@ -78,11 +75,11 @@ def _worker(rank: int, world: int, port: int, q, backend: str, top_k: int):
         raise
 
 
-def _run(backend: str, top_k: int):
+def _run(top_k: int):
     ctx = mp.get_context("spawn")
     q = ctx.Queue()
     port = _free_port()
-    procs = [ctx.Process(target=_worker, args=(r, 2, port, q, backend, top_k)) for r in range(2)]
+    procs = [ctx.Process(target=_worker, args=(r, 2, port, q, top_k)) for r in range(2)]
     for pr in procs:
         pr.start()
     res = sorted(q.get(timeout=400) for _ in range(2))
@@ -93,16 +90,51 @@ def _run(backend: str, top_k: int):
     assert all(pr.exitcode == 0 for pr in procs)
 
 
-@pytest.mark.parametrize("top_k", [2, 3])
-def test_expert_parallel_equals_unsharded_two_processes_one_gpu(top_k):
-    _run("gloo", top_k)
+@pytest.mark.parametrize("T,dim,hid,top,world", [(21, 256, 256, 2, 2), (2, 256, 256, 3, 2), (70, 256, 256, 3, 3), (300, 384, 512, 2, 4)])
+def test_ranks_one_after_the_other_equal_unsharded(T, dim, hid, top, world):
+    """Every rank's rows reach its own buffer and its peers'; what each of them combines is the unsharded layer's output, bit for bit."""
+    from mistral_inference_b200 import _abi
+    from mistral_inference_b200.moe import MoeBuffers
+
+    E, dev = 8, torch.device("cuda", 0)
+    g = torch.Generator(device=dev).manual_seed(T)
+    r = lambda *s: torch.randn(*s, generator=g, device=dev)  # noqa: E731
+    x, h, gate_w = r(T, dim).bfloat16(), r(T, dim).bfloat16(), (r(E, dim) / dim ** 0.5).bfloat16()
+    w13 = [(r(2 * hid, dim) / dim ** 0.5).bfloat16() for _ in range(E)]
+    w2 = [(r(dim, hid) / hid ** 0.5).bfloat16() for _ in range(E)]
+    ws = _abi.Workspace(_abi.workspace_bytes(max(T, 8), dim, 32, 8, 128, hid, 0, 4), dev)
+
+    def tables(rank, n):
+        return [(ctypes.c_void_p * E)(*[w[e].data_ptr() if e % n == rank else None for e in range(E)]) for w in (w13, w2)]
+
+    def buffers():
+        return MoeBuffers(T, dim, hid, E, top, dev, torch.bfloat16)
+
+    want, b = torch.empty_like(x), buffers()
+    _abi.moe_route(x, gate_w, E, top, 0, 1, b)
+    _abi.moe_grouped_ffn(b, *tables(0, 1), h, want, T, dim, hid, E, top, None, ws)
+
+    rank_b, flags = [buffers() for _ in range(world)], torch.zeros(world, 64, dtype=torch.int32, device=dev)
+    state, out = torch.zeros(world, 64, dtype=torch.int32, device=dev), [torch.empty_like(x) for _ in range(world)]
+    for rank in [*range(world), *range(world - 1)]:  # (the last rank finds all rows the first time, the others the second time)
+        s = _abi.MoeCommStruct()
+        s.n_ranks, s.my_rank = world, rank
+        for i, p in enumerate(p for p in range(world) if p != rank):
+            s.peer_yw[i], s.peer_flags[i] = rank_b[p].yw_ptr, flags[p].data_ptr()
+        s.my_flags, s.epoch, s.done_counter = flags[rank].data_ptr(), state[rank].data_ptr(), state[rank].data_ptr() + 32 * 4
+        flags.fill_(1 << 20)  # every peer "has told" this rank: nothing to wait for
+        _abi.moe_route(x, gate_w, E, top, rank, world, rank_b[rank])
+        _abi.moe_grouped_ffn(rank_b[rank], *tables(rank, world), h, out[rank], T, dim, hid, E, top, s, ws)
+    for rank in range(world):
+        assert torch.equal(out[rank], want), f"rank {rank}"
+    assert state[:, 0].tolist() == [2] * (world - 1) + [1] and not state[:, 32].any()
 
 
 @pytest.mark.parametrize("top_k", [2, 3])
 def test_expert_parallel_equals_unsharded_two_gpus_nccl(top_k):
     if torch.cuda.device_count() < 2:
-        pytest.skip("needs 2 GPUs (gpurun --gpus 2)")
-    _run("nccl", top_k)
+        pytest.skip("needs 2 GPUs")
+    _run(top_k)
 
 
 # ----------------------------------------------------------------------------- reference-compatible pipeline mode on GPUs
@@ -164,5 +196,5 @@ def _run_pp(backend: str):
 
 def test_pipeline_ranks_two_gpus_nccl():
     if torch.cuda.device_count() < 2:
-        pytest.skip("needs 2 GPUs (gpurun --gpus 2)")
+        pytest.skip("needs 2 GPUs")
     _run_pp("nccl")
