@@ -18,7 +18,7 @@
 //
 // A last round of tiles that is at most half full is cut along k (split_schedule.cuh); the parts' fp32 sums meet in the first part's epilogue, in the order of k.
 //
-// GROUPED: the mixtures' form, token tiles from the plan of moe.cuh (pair_expert, pair_info), weights by expert.
+// GROUPED: the mixtures' form, token tiles from the plan of moe.cuh (pair_expert, pair_info), weights by expert; nothing is cut.
 #pragma once
 #include <type_traits>
 
@@ -105,7 +105,7 @@ __device__ __forceinline__ void pair_gemm_body(const CUtensorMap& map_a, const C
   const uint32_t arriving = 2u * (uint32_t)(GP_W_BYTES + p.box * TG_BK * 2);  // bytes of a k-block, in both CTAs
   const int num_n = (p.N + GP_ROWS - 1) / GP_ROWS, num_k = p.K / TG_BK;
   const int num_m = GROUPED ? plan[6] : p.tok_tiles;
-  const CutPlan cuts = p.partials != nullptr ? cut_plan((long long)num_m * num_n, num_k, p.units, TG_MAX_CUTS) : CutPlan{0, 1};
+  const CutPlan cuts = !GROUPED && p.partials != nullptr ? cut_plan((long long)num_m * num_n, num_k, p.units, TG_MAX_CUTS) : CutPlan{0, 1};
   const int whole = num_m * num_n - cuts.cut_pairs, num_tiles = whole + cuts.cut * cuts.cut_pairs;
   const int32_t* item_expert = GROUPED ? plan + MOE_PLAN_HEADER + 2 * plan[2] : nullptr;
   const int32_t* item_info = GROUPED ? item_expert + plan[2] : nullptr;

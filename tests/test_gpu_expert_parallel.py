@@ -90,9 +90,10 @@ def _run(top_k: int):
     assert all(pr.exitcode == 0 for pr in procs)
 
 
-@pytest.mark.parametrize("T,dim,hid,top,world", [(21, 256, 256, 2, 2), (2, 256, 256, 3, 2), (70, 256, 256, 3, 3), (300, 384, 512, 2, 4)])
+@pytest.mark.parametrize("T,dim,hid,top,world", [(21, 256, 256, 2, 2), (2, 256, 256, 3, 2), (70, 256, 256, 3, 3), (300, 384, 512, 2, 4), (1700, 1280, 2048, 2, 2)])
 def test_ranks_one_after_the_other_equal_unsharded(T, dim, hid, top, world):
-    """Every rank's rows reach its own buffer and its peers'; what each of them combines is the unsharded layer's output, bit for bit."""
+    """Every rank's rows reach its own buffer and its peers'; what each of them combines is the unsharded layer's output, bit for bit.  (The last: pairs of
+    CTAs, whose last rounds of tiles differ between one rank and two.)"""
     from mistral_inference_b200 import _abi
     from mistral_inference_b200.moe import MoeBuffers
 
