@@ -110,10 +110,11 @@ __global__ void __launch_bounds__(F3_THREADS, 2) attn_f32_kernel(AttnArgs a) {
 #pragma unroll
             for (int o = 8; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
             mx = fmaxf(m[i], mx);
-            const float f = m[i] == -INFINITY ? 0.f : expf(m[i] - mx);
+            const float z = mx == -INFINITY ? 0.f : mx;  // keys of nothing but -infinity so far weigh 0 (-infinity less itself is no number)
+            const float f = m[i] == -INFINITY ? 0.f : expf(m[i] - z);
             float p[2], sum;
 #pragma unroll
-            for (int k = 0; k < 2; ++k) p[k] = sees[k] ? expf(s[i][k] - mx) : 0.f;
+            for (int k = 0; k < 2; ++k) p[k] = sees[k] ? expf(s[i][k] - z) : 0.f;
             sum = p[0] + p[1];
 #pragma unroll
             for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);

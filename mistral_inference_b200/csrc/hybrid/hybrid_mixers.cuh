@@ -366,9 +366,10 @@ __global__ void __launch_bounds__(AT_WARPS * 32) attn_bias_kernel(AttnArgs a) {
         }
         cmax = warp_max(cmax);
         const float m_new = a.sigmoid ? 0.f : fmaxf(m, cmax);
-        const float corr = a.sigmoid ? 1.f : (m == -INFINITY) ? 0.f : expf(m - m_new);
+        const float z = m_new == -INFINITY ? 0.f : m_new;  // keys of nothing but -infinity so far weigh 0 (-infinity less itself is no number)
+        const float corr = a.sigmoid ? 1.f : (m == -INFINITY) ? 0.f : expf(m - z);
         float psum = 0.f;
-        for (int jj = lane; jj < cn; jj += 32) { float p = a.sigmoid ? sigmoid_exact(sc[jj]) : expf(sc[jj] - m_new); sc[jj] = p; psum += p; }
+        for (int jj = lane; jj < cn; jj += 32) { float p = a.sigmoid ? sigmoid_exact(sc[jj]) : expf(sc[jj] - z); sc[jj] = p; psum += p; }
         psum = warp_sum(psum);
         l = l * corr + psum;
         m = m_new;

@@ -205,6 +205,56 @@ def test_fp32_attention_of_prompts(d, form, lens, past):
     assert not torch.isfinite(got[~fine]).any() or form == "cap_sink"
 
 
+@pytest.mark.parametrize("tiled", [True, False])
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("form", ["window", "chunked", "bias", "one_distance"])
+def test_fp32_attention_of_keys_at_minus_infinity(form, d, tiled):
+    """Keys that score -infinity weigh nothing, also where they are all that a query sees of a tile: behind a window's or a chunk's start, and under a bias of
+    -infinity for everything far.  A query that sees nothing else has no numbers."""
+    from mistral_inference_b200 import _abi_hybrid as h
+
+    H, G, W, lens, past = 4, 2, 512, [90, 40, 33], [0, 47, 300]
+    g = torch.Generator().manual_seed(d)
+    r = lambda *s: torch.randn(*s, generator=g).to(DEV)  # noqa: E731
+    T, B = sum(lens), len(lens)
+    q, ring_k, ring_v = r(T, H, d), r(B, W, G, d), r(B, W, G, d)
+    q[:, :, 0] = q[:, :, 0].abs() + 0.1
+    window, kw, bias = 0, {}, None
+    if form == "window":
+        window = 37
+        ring_k[0, 59, :, 0] = ring_k[0, 31, :, 0] = -float("inf")  # the first key that position 95, 67 see: the 32nd of the tiles that start at 28, 0
+        ring_k[2, 264:296, :, 0] = -float("inf")                 # a whole tile
+    elif form == "chunked":
+        window, kw = 48, dict(chunked=True)
+        ring_k[:, 48:64, :, 0] = -float("inf")
+    else:
+        bias = r(20, H)
+        bias[-1] = -float("inf")
+        if form == "one_distance":
+            bias[:] = -float("inf")
+            bias[3] = 0.5
+    starts = [0, 90, 130, 163]
+    dev = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    positions, slots = dev([p + i for n, p in zip(lens, past) for i in range(n)]), dev(range(B))
+    out, tiles, scale = torch.empty(T, H * d, device=DEV), sum((n + 63) // 64 for n in lens) if tiled else 0, d ** -0.5
+    if bias is not None:
+        h.attn_bias(q.flatten(1), ring_k, ring_v, bias, positions, dev(starts), slots, out, B, W, H, G, d, d, scale, n_tiles=tiles)
+    else:
+        h.attn_window(q.flatten(1), ring_k, ring_v, positions, dev(starts), slots, out, B, W, H, G, d, d, scale, window, n_tiles=tiles, **kw)
+    ref = torch.empty(T, H * d, dtype=torch.float64, device=DEV)
+    for t, p in enumerate(positions.tolist()):
+        b = sum(t >= s for s in starts) - 1
+        lo = 0 if not window else (p - p % window if kw else max(0, p - window + 1))
+        k, v = (c[b, lo:p + 1].double().repeat_interleave(H // G, 1) for c in (ring_k, ring_v))
+        s = torch.einsum("hd,khd->hk", q[t].double(), k) * scale
+        if bias is not None:
+            s = s + bias.double()[(p - torch.arange(lo, p + 1, device=DEV)).clamp(max=19)].T
+        ref[t] = torch.einsum("hk,khd->hd", torch.softmax(s, 1), v).flatten()
+    assert torch.equal(out.isnan(), ref.isnan())
+    fine = ~ref.isnan()
+    assert fine.float().mean() > 0.75 and rel(out[fine], ref[fine]) < 1e-6
+
+
 def _scan64(q, k, v, decay, state, lens):
     """o [T, H, e] and the final states of sum_j decay^(i-j) (q_i . k_j) v_j in float64, token by token."""
     o, t = torch.empty(*v.shape, dtype=torch.float64, device=v.device), 0
