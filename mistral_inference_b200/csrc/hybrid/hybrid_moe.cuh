@@ -226,7 +226,7 @@ __device__ __forceinline__ void moe_choose_lanes(const MoeRouteArgs& a, int t, f
                 b2 = fmaxf(b2, fminf(b, o));
                 b = fmaxf(b, o);
             }
-            unsigned key = lane < a.groups ? moe_key((a.group_two && gs > 1) ? b + b2 : b) | 1u : 0u, kept = 0u;
+            unsigned key = lane < a.groups ? max(moe_key((a.group_two && gs > 1) ? b + b2 : b), 1u) : 0u, kept = 0u;  // (every group may be chosen, one without a number last)
             for (int k = 0; k < a.keep; ++k) {
                 const int g = moe_best(key, 0u);
                 if (g < 0) break;

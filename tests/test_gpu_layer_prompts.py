@@ -136,6 +136,22 @@ def test_routers_of_prompts_and_of_few_tokens(n, groups, keep, top, kw, dt):
         assert rel(whole[3], torch.sigmoid(x.double() @ gate.double().T)) < 1e-5
 
 
+@pytest.mark.parametrize("n", [32, 36])
+@pytest.mark.parametrize("T", [3, 701])
+def test_groups_one_rounding_apart(n, T):
+    """The better of two groups is kept when their scores are neighbouring numbers, whichever comes first: up to 32 outputs (in registers) and more (in shared
+    memory)."""
+    from mistral_inference_b200 import _abi_hybrid as h
+
+    x, w = torch.randn(T, 64, device=DEV), torch.zeros(n, 64, device=DEV)  # every score is 1/2
+    for low in (0, 1, 6):
+        for lo, hi in ((1, 5), (5, 1), (0, 7)):
+            corr = torch.full((n,), -0.25, device=DEV)
+            corr[4 * lo + 1], corr[4 * hi + 2] = low * 2.0 ** -24, (low + 1) * 2.0 ** -24
+            _, idx, _ = h.moe_route(x, w, corr, n // 4, 1, 2, score=1)
+            assert (idx == torch.tensor([4 * hi + 2, 4 * hi], dtype=torch.int32, device=DEV)).all(), (low, lo, hi)
+
+
 @pytest.mark.parametrize("d", [64, 128])
 @pytest.mark.parametrize("form", ["plain", "bias", "window", "chunked", "cap_sink", "gate", "own"])
 @pytest.mark.parametrize("lens,past", [([33], [0]), ([1, 64, 31, 90], [5, 0, 40, 3]), ([32, 65], [130, 0])])
