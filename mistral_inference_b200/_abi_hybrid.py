@@ -207,11 +207,24 @@ def _check_bias_table(bias_tab: Optional[torch.Tensor], H: int) -> None:
     assert bias_tab is None or (bias_tab.dtype == torch.float32 and bias_tab.dim() == 2 and bias_tab.shape[1] == H), "bias table: fp32 [distances, heads]"
 
 
+F32_TILE_ROWS = F32_TILE_KEYS = 400
+
+
+def f32_rows_alone(rows: int, keys: int) -> bool:
+    """Whether fp32 prompt attention gives every row (token and head) a CTA of its own.  A tile of 32 queries shares its keys, but one CTA walks all of them: few
+    rows over many keys leave the chip idle.  Heads of 128, us (rows alone, tiles): 64 rows over 500 keys 50, 66, over 4000 346, 468; 256 over 2000 197, 236;
+    384 over 2000 234, 240; 512 over 2000 275, 241; 64 over 100 42, 18."""
+    return rows < F32_TILE_ROWS and keys > F32_TILE_KEYS
+
+
 def attn_bias(q, cache_k, cache_v, bias_tab, positions, q_start, slots, out, B: int, W: int, H: int, G: int, d: int, e: int, scale: float,
-              n_tiles: int = 0, splits: int = 1, seqpos=None, longest: int = 0) -> None:
-    """n_tiles = sum over sequences of ceil(len / 64) selects a tensor-core prompt kernel (bf16); 0 the exact fp32 one.  With seqpos (tokens
-    before this call, per sequence) and the longest sequence's length, heads of 128 take the main library's tcgen05 kernel where it is built."""
+              n_tiles: int = 0, splits: int = 1, seqpos=None, longest: int = 0, keys: int = 0) -> None:
+    """n_tiles = sum over sequences of ceil(len / 64) selects a prompt kernel (bf16: tensor cores; fp32: tiles of 32 queries, unless `f32_rows_alone`); 0 the one
+    that gives every token and head a CTA (`splits` of them, along the keys).  keys: how many a query sees at most (0: the ring).  With seqpos (tokens before
+    this call, per sequence) and the longest sequence's length, heads of 128 take the main library's tcgen05 kernel where it is built."""
     _check_bias_table(bias_tab, H)
+    if q.dtype == torch.float32 and f32_rows_alone(q.shape[0] * H, keys or W):
+        n_tiles = 0
     if (n_tiles and seqpos is not None and longest >= ATTN_TCGEN05_MIN and d == e == 128 and q.dtype == torch.bfloat16 and scale > 0 and _aligned(q, cache_k, cache_v, out)
             and cache_k.shape[1] == W and os.environ.get("MB200_HYBRID_GEMM", "1") != "0" and _abi.library_path().exists()
             and (bias_tab is None or bias_tab.shape[0] <= _abi.lib().mb200_layer_attention_max_table())):
@@ -477,14 +490,17 @@ def kv_scatter(k, v, cache_rows, ring_k, ring_v) -> None:
 def attn_window(q, cache_k, cache_v, positions, q_start, slots, out, B: int, W: int, H: int, G: int, d: int, e: int, scale: float, window: int,
                 own_k=None, own_v=None, seqpos=None, n_tiles: int = 0, splits: int = 1, chunk: int = 0, head_bias=None,
                 softcap: float = 0.0, sink=None, chunked: bool = False, gate=None, gate_entry: bool = False, lam=None, out_scale: float = 1.0,
-                norm_eps: float = 0.0) -> None:
+                norm_eps: float = 0.0, keys: int = 0) -> None:
     """`attn_bias` without a bias, with a sliding window (0: none) and, for prompts, this call's own keys and values beside the ring.
-    chunk: keys per warp and step of the exact kernel (0: 128), see `window_decode_plan`.  head_bias (fp32 [H]): sigmoid weights instead
+    chunk: keys per warp and step of the kernel of a CTA per row (0: 128), see `window_decode_plan`.  head_bias (fp32 [H]): sigmoid weights instead
     of the softmax, every visible key weighing sigmoid(score + head_bias[h]), not normalised.  softcap > 0: scores softcap * tanh(. / softcap); sink
     (fp32 [H]): one more term exp(sink[h]) in the softmax denominator.  chunked: `window` is the size of chunks.  gate: columns of a matrix
     [T, .] whose sigmoid multiplies the output, one per head or (gate_entry) one per entry.  lam (fp32 [1]): differential attention, q holds
     [T, H, 2, d] and keys [., G, 2, d]; out = unit_rms(a_1 - lam a_2; norm_eps) * out_scale per head."""
     maps = 1 if lam is None else 2
+    keys = keys or W + (q.shape[0] if own_k is not None else 0)
+    if q.dtype == torch.float32 and f32_rows_alone(q.shape[0] * H, min(keys, window + 32) if window else keys):
+        n_tiles = 0
     flash = n_tiles > 0 and q.dtype == torch.bfloat16 and (d, e) in DIFF_FLASH_SIZES
     scratch = (torch.empty(q.shape[0] * H * maps * splits * (2 + e), dtype=torch.float32, device=q.device)
                if (splits > 1 and n_tiles == 0) or (maps > 1 and not flash) else None)

@@ -264,8 +264,13 @@ def padded_rows(n: int) -> int:
 
 
 def query_tiles(md) -> int:
-    """The number of 64-query tiles of this call for the tensor-core prompt kernel, 0 for the exact one."""
+    """The number of 64-query tiles of this call for the prompt kernels (fp32: tiles of 32), 0 for the kernel that gives every token and head a CTA."""
     return sum((n + 63) // 64 for n in md.seqlens) if md.max_seqlen >= FLASH_MIN_QUERIES else 0
+
+
+def most_keys(md) -> int:
+    """How many keys a query of a first prompt sees at most; 0 where earlier tokens lie in the ring."""
+    return md.max_seqlen if md.first_prefill else 0
 
 
 def distance_buckets(rows: int, far: float) -> List[int]:
@@ -332,7 +337,7 @@ class BiasedAttention(nn.Module):
         else:
             _h.attn_bias(q, view.cache_k, view.cache_v, self.bias_table(), md.positions, md.q_start, md.slots, out, len(md.seqlens), md.window,
                          a.heads, a.kv_heads, a.dim, a.vdim, a.scale,
-                         n_tiles=sum((n + 63) // 64 for n in md.seqlens) if md.max_seqlen >= FLASH_MIN_QUERIES else 0,
+                         n_tiles=query_tiles(md), keys=most_keys(md),
                          splits=_h.attn_splits(T, a.heads, md.window), seqpos=md.seqpos, longest=md.max_seqlen)
         project_out(out, self.wo, x32, post)
 
@@ -658,7 +663,7 @@ class RotaryWindowAttention(nn.Module):
         else:
             splits, chunk = _h.window_decode_plan(T, a.heads * a.maps, W) if not md.prefill else (1, 0)
             _h.attn_window(q, view.cache_k, view.cache_v, md.positions, md.q_start, md.slots, out, B, W, a.heads, a.kv_heads, a.dim, a.vdim, a.scale, window,
-                           own_k=k, own_v=v, seqpos=md.seqpos if own else None, n_tiles=query_tiles(md) if md.prefill else 0, splits=splits, chunk=chunk, **kind)
+                           own_k=k, own_v=v, seqpos=md.seqpos if own else None, n_tiles=query_tiles(md) if md.prefill else 0, keys=most_keys(md), splits=splits, chunk=chunk, **kind)
         if own:
             _h.kv_scatter(k, v, md.cache_rows, view.cache_k, view.cache_v)
         project_out(out, self.wo, x32, post, scale, bias=self.bo)
@@ -1038,7 +1043,7 @@ class SigmoidWindowAttention(nn.Module):
             q, k, v = _h.whole_norm_prep(qkv, self.q_norm, self.k_norm, None, None, None, self.nq, self.nk, self.nv, self.eps, own=True)
             _h.attn_window(q, view.cache_k, view.cache_v, md.positions, md.q_start, md.slots, out, B, W, a.heads, a.kv_heads, a.dim, a.vdim, a.scale,
                            window, own_k=k, own_v=v, seqpos=md.seqpos, head_bias=self.head_bias(),
-                           n_tiles=sum((n + 63) // 64 for n in md.seqlens) if md.max_seqlen >= FLASH_MIN_QUERIES else 0)
+                           n_tiles=query_tiles(md), keys=most_keys(md))
             _h.kv_scatter(k, v, md.cache_rows, view.cache_k, view.cache_v)
         else:
             q, _, _ = _h.whole_norm_prep(qkv, self.q_norm, self.k_norm, md.cache_rows, view.cache_k, view.cache_v, self.nq, self.nk, self.nv, self.eps,

@@ -221,6 +221,30 @@ def test_fp32_attention_of_prompts(d, form, lens, past):
     assert not torch.isfinite(got[~fine]).any() or form == "cap_sink"
 
 
+@pytest.mark.parametrize("lens,past,H", [([16], [900], 4), ([24, 1], [500, 30], 8), ([17, 33], [600, 0], 8)])
+def test_fp32_attention_of_few_rows_over_many_keys(lens, past, H):
+    """Below 400 rows (tokens and heads) over more than 400 keys every row has a CTA of its own, from there on tiles of 32 queries: both against float64."""
+    from mistral_inference_b200 import _abi_hybrid as h
+
+    G, d, W, B = 2, 128, 1024, len(lens)
+    g = torch.Generator().manual_seed(H)
+    r = lambda *s: torch.randn(*s, generator=g).to(DEV)  # noqa: E731
+    T, bias = sum(lens), r(30, H)
+    q, ring_k, ring_v = r(T, H * d), r(B, W, G, d), r(B, W, G, d)
+    dev = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    starts = [sum(lens[:b]) for b in range(B + 1)]
+    positions = [p + i for n, p in zip(lens, past) for i in range(n)]
+    assert h.f32_rows_alone(T * H, W) == (T * H < 400)
+    for splits in (1, 2):
+        out = torch.empty(T, H * d, device=DEV)
+        h.attn_bias(q, ring_k, ring_v, bias, dev(positions), dev(starts), dev(range(B)), out, B, W, H, G, d, d, d ** -0.5, n_tiles=B, splits=splits)
+        for t, p in enumerate(positions):
+            b = sum(t >= s for s in starts) - 1
+            k, v = (c[b, :p + 1].double().repeat_interleave(H // G, 1) for c in (ring_k, ring_v))
+            s = torch.einsum("hd,khd->hk", q[t].view(H, d).double(), k) * d ** -0.5 + bias.double()[(p - torch.arange(p + 1, device=DEV)).clamp(max=29)].T
+            assert rel(out[t], torch.einsum("hk,khd->hd", torch.softmax(s, 1), v).flatten()) < 2e-6
+
+
 @pytest.mark.parametrize("tiled", [True, False])
 @pytest.mark.parametrize("d", [64, 128])
 @pytest.mark.parametrize("form", ["window", "chunked", "bias", "one_distance"])

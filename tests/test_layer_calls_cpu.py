@@ -44,3 +44,28 @@ def test_scoring_takes_one_target_a_token(what):
     target, keep, out = (t[1:] if what == n else t for t, n in ((target, "target"), (keep, "keep"), (out, "out")))
     with pytest.raises(AssertionError, match="targets and kept rows|results"):
         _abi.lm_head_logprobs(torch.zeros(T, 64, dtype=bf), torch.ones(64, dtype=bf), torch.zeros(V, 64, dtype=bf), target, keep, torch.zeros(1, V), out, 1e-5, None)
+
+
+@pytest.mark.parametrize("T,H,W,window,own,keys,dtype,tiled", [
+    (24, 16, 4096, 0, False, 0, torch.float32, False),      # 384 rows behind a long ring: a CTA each
+    (25, 16, 4096, 0, False, 0, torch.float32, True),
+    (24, 16, 4096, 0, False, 24, torch.float32, True),      # a first prompt: its own keys only
+    (24, 16, 400, 0, False, 0, torch.float32, True),        # a short ring
+    (24, 16, 380, 0, True, 0, torch.float32, False),        # ... and the call's own keys beside it
+    (24, 16, 4096, 368, True, 0, torch.float32, True),      # a window
+    (24, 16, 4096, 369, True, 0, torch.float32, False),
+    (24, 16, 4096, 0, False, 0, torch.bfloat16, True),
+])
+def test_fp32_prompts_of_few_rows_over_many_keys(T, H, W, window, own, keys, dtype, tiled, monkeypatch):
+    """Which kernel a prompt's attention takes, by the query tiles that reach the library (none: a CTA per token and head)."""
+    seen = []
+    record = lambda *a: seen.append(a[17]) or 0  # noqa: E731
+    monkeypatch.setattr(h, "lib", lambda: type("Lib", (), {"mbh_attn_bias": staticmethod(record), "mbh_attn_window": staticmethod(record)}))
+    monkeypatch.setattr(h, "_ptr", lambda t: None)
+    monkeypatch.setattr(h, "_stream", lambda: 0)
+    q, ring, i = torch.zeros(T, H * 64, dtype=dtype), torch.zeros(1, W, 1, 64, dtype=dtype), torch.zeros(2, dtype=torch.int32)
+    k = q[:, :64].contiguous() if own else None
+    h.attn_window(q, ring, ring, i, i, i, q, 1, W, H, 1, 64, 64, 0.1, window, own_k=k, own_v=k, seqpos=i, n_tiles=1, keys=keys)
+    if not own and not window:
+        h.attn_bias(q, ring, ring, None, i, i, i, q, 1, W, H, 1, 64, 64, 0.1, n_tiles=1, keys=keys)
+    assert all((n > 0) == tiled for n in seen) and seen
