@@ -242,7 +242,14 @@ def attn_splits(T: int, H: int, W: int, n_sm: int = 148) -> int:
 
 
 LIGHTNING_CHUNK_MIN = 12  # prompts (portions) at least this long run in chunks on tensor cores where the sizes allow
-LIGHTNING_SPLIT_MIN = 8   # others at least this long: the scan whose state is dealt to several warps (0.3 us a token instead of 0.7, 5 us more for the state itself)
+LIGHTNING_SPLIT_MIN = 8   # others at least this long: the scan whose state is dealt to several warps, where `scan_is_dealt`
+
+
+def scan_is_dealt(B: int, H: int, e: int, longest: int, dtype: torch.dtype) -> bool:
+    """Whether the token-by-token scan deals a state's rows to four warps: a third of the time a token, but four times the CTAs (one to 32 value columns), which
+    pays until they fill the chip.  16 heads of 128 and 100 tokens, us with a column a thread and dealt: fp32 65, 33 (1 sequence: 64 CTAs), 87, 76 (8: 512), 32 heads
+    97, 119 (8: 1024); bf16 68, 50 (64), 69, 52 (192), 95, 101 (512)."""
+    return longest >= LIGHTNING_SPLIT_MIN and B * H * ((e + 31) // 32) <= (512 if dtype == torch.float32 else 256)
 
 
 def lightning_scan(qkvg, state, decay, q_start, seqpos, slots, o32, B: int, H: int, d: int, e: int, longest: int = 1) -> None:
@@ -252,7 +259,7 @@ def lightning_scan(qkvg, state, decay, q_start, seqpos, slots, o32, B: int, H: i
         _check(lib().mbh_lightning_prompt(_ptr(qkvg), _ptr(state), _ptr(decay), _ptr(q_start), _ptr(seqpos), _ptr(slots), _ptr(o32), B, H, d, e, _stream()),
                "mbh_lightning_prompt")
         return
-    scan = lib().mbh_lightning_split if longest >= LIGHTNING_SPLIT_MIN else lib().mbh_lightning_scan
+    scan = lib().mbh_lightning_split if scan_is_dealt(B, H, e, longest, qkvg.dtype) else lib().mbh_lightning_scan
     _check(scan(_ptr(qkvg), _ptr(state), _ptr(decay), _ptr(q_start), _ptr(seqpos), _ptr(slots), _ptr(o32), B, H, d, e, dt_of(qkvg.dtype), _stream()), "mbh_lightning_scan")
 
 

@@ -69,3 +69,16 @@ def test_fp32_prompts_of_few_rows_over_many_keys(T, H, W, window, own, keys, dty
     if not own and not window:
         h.attn_bias(q, ring, ring, None, i, i, i, q, 1, W, H, 1, 64, 64, 0.1, n_tiles=1, keys=keys)
     assert all((n > 0) == tiled for n in seen) and seen
+
+
+@pytest.mark.parametrize("B,H,e,longest,dtype,dealt", [
+    (1, 16, 128, 8, torch.float32, True), (1, 16, 128, 7, torch.float32, False), (8, 16, 128, 300, torch.float32, True), (8, 16, 129, 300, torch.float32, False),
+    (4, 16, 128, 8, torch.bfloat16, True), (8, 16, 96, 100, torch.bfloat16, False), (3, 32, 128, 9, torch.bfloat16, False)])
+def test_scans_that_fill_the_chip_keep_a_column_a_thread(B, H, e, longest, dtype, dealt, monkeypatch):
+    seen = []
+    monkeypatch.setattr(h, "lib", lambda: type("Lib", (), {n: staticmethod(lambda *a, n=n: seen.append(n) or 0) for n in ("mbh_lightning_scan", "mbh_lightning_split")}))
+    monkeypatch.setattr(h, "_ptr", lambda t: None)
+    monkeypatch.setattr(h, "_stream", lambda: 0)
+    x, f = torch.zeros(2, 8, dtype=dtype), torch.zeros(2)
+    h.lightning_scan(x, f, f, f, f, f, f, B, H, 100, e, longest=longest)
+    assert seen == ["mbh_lightning_split" if dealt else "mbh_lightning_scan"]
