@@ -273,11 +273,11 @@ __device__ __forceinline__ void moe_choose_lanes(const MoeRouteArgs& a, int t, f
 
 constexpr int MOE_ROUTE_THREADS = 256;
 
-// A CTA per TOK tokens: its warps share the outputs, then TOK of them choose; shared memory per token: z[n] | choice[n] | gbest[groups] | kept[groups].  Four tokens a CTA
-// from MOE_ROUTE_MANY tokens on: a piece of a router row out of L2 serves four sums, and four warps of eight choose where one did (2500 tokens, width 2048, 20
-// outputs: 48 us with one token a CTA and a choice through shared memory, 33 with that choice in registers, 26 with four; 592 tokens 9 with one and 13 with four,
-// 801 15 and 13).  A sum runs in the order of warp_dot either way.
-template <typename T, int TOK>
+// A CTA per TOK tokens: its warps share the outputs, then TOK of them choose; shared memory per token: z[n] | choice[n] | gbest[groups] | kept[groups].  Bound by the
+// latency of rows out of L2.  Four tokens a CTA (launch_moe_route): a piece of a router row serves four sums, and four warps of eight choose where one did.
+// AHEAD: eight loads of a sum stand in flight by themselves; otherwise the compiler chooses (in fp32 fewer, for a fifth CTA on an SM).  A sum runs in the order of
+// warp_dot in all of them.
+template <typename T, int TOK, bool AHEAD = false>
 __global__ void __launch_bounds__(MOE_ROUTE_THREADS) moe_route_kernel(MoeRouteArgs a, int tokens) {
     extern __shared__ float sm[];
     constexpr int V = Vec<T>::N;
@@ -290,7 +290,28 @@ __global__ void __launch_bounds__(MOE_ROUTE_THREADS) moe_route_kernel(MoeRouteAr
         const T* w = e < a.n ? W + (size_t)e * a.width : static_cast<const T*>(a.w_gate);
         float acc[TOK];
         if constexpr (TOK == 1) {
-            acc[0] = warp_dot<T>(w, h[0], a.width, lane);
+            if constexpr (AHEAD) {
+                constexpr int U = 4, S = 32 * V;  // steps at a time
+                float sum = 0.f;
+                for (int k = lane * V; k < a.width; k += U * S) {
+                    float wv[U][V], x[U][V];
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        if (k + u * S >= a.width) break;
+                        Vec<T>::load(w + k + u * S, wv[u]);
+                        Vec<T>::load(h[0] + k + u * S, x[u]);
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        if (k + u * S >= a.width) break;
+#pragma unroll
+                        for (int v = 0; v < V; ++v) sum = fmaf(wv[u][v], x[u][v], sum);
+                    }
+                }
+                acc[0] = warp_sum(sum);
+            } else {
+                acc[0] = warp_dot<T>(w, h[0], a.width, lane);
+            }
         } else {
 #pragma unroll
             for (int i = 0; i < TOK; ++i) acc[i] = 0.f;
@@ -323,13 +344,29 @@ __global__ void __launch_bounds__(MOE_ROUTE_THREADS) moe_route_kernel(MoeRouteAr
     else moe_choose<T>(a, t0 + warp, z, z + a.n, z + 2 * a.n, z + 2 * a.n + a.groups, lane);
 }
 
-constexpr int64_t MOE_ROUTE_MANY = 700;
+// Which form, by the number of tokens (us; width x outputs):
+//   Four tokens a CTA when that still fills the chip.  bf16, one and four: 700 tokens 2048 x 20 14, 12.5; 4096 x 256 216, 205; rows of more than 8 KB later: 7168 x 256, 700 tokens
+//   356, 374, 1300 tokens 493, 487.  fp32 (AHEAD) and four: 800 tokens 2048 x 64 51, 44; 4096 x 64 85, 106, 1300 tokens 126, 109.
+//   fp32 below that: AHEAD has four CTAs on an SM, the other five, each slower: 100 tokens 2048 x 64 18.5, 31; 4096 x 256 92, 195.  From 593 to 740 tokens the fifth spares
+//   a second round: 700 tokens 2048 x 64 51, 35; 4096 x 256 299, 226.
 template <typename T>
 inline void launch_moe_route(const MoeRouteArgs& a, int64_t tokens, size_t smem, cudaStream_t st) {
-    // (the sums of four tokens at a time need rows of whole 16-byte pieces)
+    // (four sums at a time, and AHEAD, need rows of whole 16-byte pieces)
     const bool aligned = a.width % Vec<T>::N == 0 && (reinterpret_cast<uintptr_t>(a.h) | reinterpret_cast<uintptr_t>(a.w_router) | reinterpret_cast<uintptr_t>(a.w_gate)) % 16 == 0;
-    if (tokens >= MOE_ROUTE_MANY && aligned && 4 * smem <= 48 * 1024) moe_route_kernel<T, 4><<<(unsigned)((tokens + 3) / 4), MOE_ROUTE_THREADS, 4 * smem, st>>>(a, (int)tokens);
-    else moe_route_kernel<T, 1><<<(unsigned)tokens, MOE_ROUTE_THREADS, smem, st>>>(a, (int)tokens);
+    constexpr bool F32 = sizeof(T) == 4;
+    constexpr int64_t SMS = 148;
+    const int64_t many = a.width * (int64_t)sizeof(T) > 8192 ? 1200 : (F32 ? 5 * SMS + 1 : 700);
+    if (tokens >= many && aligned && 4 * smem <= 48 * 1024) {
+        moe_route_kernel<T, 4><<<(unsigned)((tokens + 3) / 4), MOE_ROUTE_THREADS, 4 * smem, st>>>(a, (int)tokens);
+        return;
+    }
+    if constexpr (F32) {
+        if (aligned && (tokens <= 4 * SMS || tokens > 5 * SMS)) {
+            moe_route_kernel<T, 1, true><<<(unsigned)tokens, MOE_ROUTE_THREADS, smem, st>>>(a, (int)tokens);
+            return;
+        }
+    }
+    moe_route_kernel<T, 1><<<(unsigned)tokens, MOE_ROUTE_THREADS, smem, st>>>(a, (int)tokens);
 }
 
 struct MoeSparseArgs {

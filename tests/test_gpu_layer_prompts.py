@@ -104,26 +104,29 @@ def _route64(x, w, corr, groups, keep, top, score, scale=1.0, renorm=False, grou
 
 
 @pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("width", [328, 42, 2052])  # no whole number of steps; no whole 16-byte pieces; fp32 rows of more than 8 KB
 @pytest.mark.parametrize("n,groups,keep,top,kw", [(20, 4, 2, 4, dict(score=0)), (8, 1, 1, 2, dict(score=1, scale=2.5, renorm=True)), (33, 3, 2, 5, dict(score=1, group_two=True)),
                                                   (32, 16, 3, 4, dict(score=1, group_two=True)), (16, 1, 1, 3, dict(score=2, always=1)), (7, 1, 1, 7, dict(score=0, gate=True))])
-def test_routers_of_prompts_and_of_few_tokens(n, groups, keep, top, kw, dt):
-    """From 700 tokens on a CTA routes four, below one: every sum in the same order, so the same bits; up to 32 outputs are chosen from in registers, more in shared
-    memory.  Against float64: fp32 sums of 328 products, the choices where they are not closer than that."""
+def test_routers_of_prompts_and_of_few_tokens(n, groups, keep, top, kw, dt, width):
+    """For many tokens a CTA routes four, below one, in fp32 with more loads in flight or with more CTAs (593 to 740 tokens): every sum in the same order, so the same
+    bits; up to 32 outputs are chosen from in registers, more in shared memory.  Against float64: fp32 sums of `width` products, the choices where they are not
+    closer than that."""
     from mistral_inference_b200 import _abi_hybrid as h
 
-    T, width = 1025, 328  # not a whole number of 256-element steps; the last CTA has one token
+    T = 1201  # the last CTA has one token
     kw = dict(kw)
     g = torch.Generator().manual_seed(n)
     r = lambda *s: torch.randn(*s, generator=g).to(dt).to(DEV)  # noqa: E731
-    x, w, corr = r(T, width), r(n, width) / 8, r(n) / 10 if kw["score"] != 2 else None
+    x, w, corr = r(T, width), r(n, width) * (5 / width) ** 0.5, r(n) / 10 if kw["score"] != 2 else None
     if kw.pop("gate", False):
         kw["w_gate"] = r(1, width) / 8
     if kw["score"] == 2:
         kw["w_bias"] = r(n)
     whole = h.moe_route(x, w, corr, groups, keep, top, **kw)
-    parts = [h.moe_route(x[i:i + 205], w, corr, groups, keep, top, **kw) for i in range(0, T, 205)]
-    for a, b in zip(whole, zip(*parts)):
-        assert torch.equal(a, torch.cat(b))
+    for step in (205, 640):
+        parts = [h.moe_route(x[i:i + step], w, corr, groups, keep, top, **kw) for i in range(0, T, step)]
+        for a, b in zip(whole, zip(*parts)):
+            assert torch.equal(a, torch.cat(b))
     always, gate = kw.pop("always", 0), kw.pop("w_gate", None)
     ref, choice = _route64(x, w, corr, groups, keep, top, **kw)
     dense, idx, wsel = whole[:3]
