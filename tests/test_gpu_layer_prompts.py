@@ -634,7 +634,7 @@ def test_scoring_counts_logits_that_are_no_numbers(T, cols, value):
 
 
 @pytest.mark.parametrize("T", [17, 32, 33, 64, 65, 127, 128, 171, 600])
-@pytest.mark.parametrize("N,K", [(256, 128), (4096, 8192)])
+@pytest.mark.parametrize("N,K", [(256, 128), (4096, 8192), (4224, 128)])  # the last: at 600 rows pairs, half a tile of weights at the end
 def test_prompt_linear_steps_by_rows(T, N, K):
     """The steps behind a prompt's Linear at every change of kernel over the rows (stream-K boxes, single tiles, pairs cut along k): bf16 results
     within a rounding (2^-8) of float64, fp32 ones within 2^-8 of the sum's scale for the rounded sum that is added."""
