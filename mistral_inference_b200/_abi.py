@@ -113,8 +113,11 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return t.data_ptr()
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)  # the current stream's handle without its Python objects, where torch has it
+
+
 def _stream() -> int:
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())  # torch.cuda.current_stream().cuda_stream without its objects
+    return _raw_stream(torch.cuda.current_device()) if _raw_stream is not None else torch.cuda.current_stream().cuda_stream
 
 
 class Workspace:

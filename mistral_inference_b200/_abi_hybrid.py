@@ -11,7 +11,7 @@ from typing import Optional
 import torch
 
 from . import _abi, build
-from ._abi import Mb200Error
+from ._abi import Mb200Error, _stream
 
 ABI_VERSION = 7
 EPI_STORE, EPI_RESIDUAL, EPI_GLU, EPI_F32, EPI_SWIGLU, EPI_RESIDUAL_SCALED, EPI_RELU2, EPI_GEGLU = 0, 1, 2, 3, 4, 5, 6, 7
@@ -100,10 +100,6 @@ def _rows(x: torch.Tensor):
     """(pointer, elements between rows) of a matrix whose rows are contiguous: columns of a wider one are taken as they are."""
     assert x.is_cuda and x.dim() == 2 and x.stride(1) == 1, "rows of contiguous elements"
     return x.data_ptr(), max(x.stride(0), x.shape[1])
-
-
-def _stream() -> int:
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())  # torch.cuda.current_stream().cuda_stream without its objects
 
 
 def dt_of(dtype: torch.dtype) -> int:

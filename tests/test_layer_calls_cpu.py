@@ -82,3 +82,10 @@ def test_scans_that_fill_the_chip_keep_a_column_a_thread(B, H, e, longest, dtype
     x, f = torch.zeros(2, 8, dtype=dtype), torch.zeros(2)
     h.lightning_scan(x, f, f, f, f, f, f, B, H, 100, e, longest=longest)
     assert seen == ["mbh_lightning_split" if dealt else "mbh_lightning_scan"]
+
+
+def test_the_stream_where_torch_has_no_raw_getter(monkeypatch):
+    """The handle by torch's public way, for both libraries."""
+    monkeypatch.setattr(_abi, "_raw_stream", None)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: type("Stream", (), {"cuda_stream": 77}))
+    assert _abi._stream() == 77 == h._stream()
