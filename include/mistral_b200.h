@@ -29,7 +29,7 @@
 extern "C" {
 #endif
 
-#define MB200_ABI_VERSION 1
+#define MB200_ABI_VERSION 2
 
 #define MB200_OK 0
 #define MB200_E_INVALID (-1)   /* bad argument / unsupported shape */

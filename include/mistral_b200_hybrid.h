@@ -13,7 +13,7 @@
 extern "C" {
 #endif
 
-#define MBH_ABI_VERSION 7
+#define MBH_ABI_VERSION 8
 
 int mbh_abi_version(void);
 const char* mbh_last_error(void);

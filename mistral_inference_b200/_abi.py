@@ -15,7 +15,7 @@ import torch
 _LIB_PATH = Path(os.environ.get("MB200_LIB_PATH") or Path(__file__).resolve().parent / "libmb200.so")  # override: A/B builds of experiments
 _lib: Optional[ctypes.CDLL] = None
 
-ABI_VERSION = 1
+ABI_VERSION = 2
 SKINNY_MAX_T = 4
 WORKSPACE_HEADER_BYTES = 64 * 1024
 

@@ -13,7 +13,7 @@ import torch
 from . import _abi, build
 from ._abi import Mb200Error, _stream
 
-ABI_VERSION = 7
+ABI_VERSION = 8
 EPI_STORE, EPI_RESIDUAL, EPI_GLU, EPI_F32, EPI_SWIGLU, EPI_RESIDUAL_SCALED, EPI_RELU2, EPI_GEGLU = 0, 1, 2, 3, 4, 5, 6, 7
 _DT = {torch.bfloat16: 0, torch.float32: 1}
 _lib: Optional[ctypes.CDLL] = None

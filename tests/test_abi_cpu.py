@@ -2,6 +2,7 @@
 declares (no compute without a GPU), and the host-side mirror of the reference API behaves like the reference."""
 import ctypes
 import re
+import zlib
 from pathlib import Path
 
 import numpy as np
@@ -10,7 +11,7 @@ import torch
 
 import mistral_inference_b200 as mi
 import synth
-from mistral_inference_b200 import _abi
+from mistral_inference_b200 import _abi, _abi_hybrid
 from mistral_inference_b200.build import build_library
 from mistral_inference_b200.cache import BufferCache
 from mistral_inference_b200.transformer import Transformer
@@ -37,6 +38,27 @@ def test_header_symbols_exported(built):
 def test_library_loads_and_reports_version(built):
     assert _abi.lib().mb200_abi_version() == _abi.ABI_VERSION
     assert _abi.workspace_bytes(16, 4096, 32, 8, 128, 14336, 32000, 1) > _abi.WORKSPACE_HEADER_BYTES
+
+
+# What the headers declare, and how arguments are read where their text says more (a bit field), at each ABI version.  A change takes a new version, so that a library built
+# before it is refused and not called with arguments that it reads otherwise.
+HEADERS = {("mistral_b200.h", 2): 710053877, ("mistral_b200_hybrid.h", 8): 2860741691}
+
+
+@pytest.mark.parametrize("header,version", HEADERS)
+def test_declarations_of_this_abi_version(header, version):
+    text = (REPO / "include" / header).read_text()
+    assert int(re.search(r"_ABI_VERSION (\d+)", text).group(1)) == version == (_abi if header == "mistral_b200.h" else _abi_hybrid).ABI_VERSION
+    bits = re.findall(r"\w+ & \d+", " ".join(text.split()))
+    code = re.sub(r"/\*.*?\*/|//[^\n]*", " ", text, flags=re.S)
+    assert zlib.crc32((" ".join(code.split()) + "|".join(bits)).encode()) == HEADERS[header, version], "raise the ABI version with this change"
+
+
+def test_a_library_of_another_version_is_refused(built, monkeypatch):
+    monkeypatch.setattr(_abi, "_lib", None)
+    monkeypatch.setattr(_abi, "ABI_VERSION", _abi.ABI_VERSION + 1)
+    with pytest.raises(_abi.Mb200Error, match="ABI"):
+        _abi.lib()
 
 
 def test_argument_errors_do_not_need_a_gpu(built):
