@@ -7,7 +7,8 @@
 // The WEIGHTS are the MMA's 256 rows and the TOKENS its columns, because the number of columns of an MMA is free (any multiple of 32 up to 256) and that of its rows is not:
 // T tokens are dealt to ceil(T / 256) tiles whose widths differ by at most 32, and at most 31 columns of all are padding.  With the tokens as rows the last tile ran
 // as 256 rows whatever it held (an MMA of 128 rows over a pair takes as long): 1102 tokens cost 1280 rows, now 1120 columns; eight experts of ~512 rows
-// each cost 640 or 768, now what they have, to the next 32.
+// each cost 640 or 768, now what they have, to the next 32.  Time does not follow the columns alone: a k-block of a tile w wide takes about 256 + w clocks, of which
+// the 256 are the weight rows' way out of shared memory.  Five tiles for 1102 tokens: 480 clocks a k-block each instead of 512, and scoring them gained 4 %.
 //
 // Accumulators therefore lie transposed in TMEM: lane = feature, column = token.  Epilogues work on pairs of features (exchange_pairs, epilogue.cuh); fp32 results
 // need not even that, a warp's 32 features of a token are one 128-byte line.  Shared memory stays out of it: the MMAs' operands and the copies take all of its
@@ -40,7 +41,7 @@ constexpr unsigned CUT_GIVEN_UP = 2u;  // a flag: 0, 1 (the part is there), or t
 constexpr int TG_MAX_CUTS = 56;        // (cut - 1) * cut_pairs at most: 256 KB each
 constexpr size_t TG_CUT_BYTES = (size_t)TG_MAX_CUTS * 2 * TG_BM * 256 * sizeof(float);
 
-// Tiles in the order of tile_mn<8, 9>, by steps
+// Tiles in the order of tile_mn (gemm_tcgen05.cuh) with blocks of 8 x 9, by steps
 struct TileWalk {
   int q, mb, nb, gm, gn;  // place in the block, the block's first token and weight tile, its extents (m fastest)
   __device__ __forceinline__ void block(int num_m, int num_n) {
@@ -512,7 +513,7 @@ int launch_gemm_pair(const GemmParams& g, int sms, cudaStream_t stream, void* sc
   if (rc) return rc;
   const long long tiles = (long long)p.tok_tiles * ceil_div(g.N, GP_ROWS);
   const bool cut = scratch != nullptr && cut_plan(tiles, g.K / TG_BK, p.units, TG_MAX_CUTS).cut_pairs > 0;
-  return launch_pairs(gemm_pair_kernel<MODE>, cut || tiles > p.units ? p.units : (int)tiles, stream, map_a, map_w, p);  // (a cut last round is full)
+  return launch_pairs(gemm_pair_kernel<MODE>, cut || tiles > p.units ? p.units : (int)tiles, stream, map_a, map_w, p);  // (cut: item s of the last round runs on cluster s, so all of them are there)
 }
 
 // T >= TG_BM

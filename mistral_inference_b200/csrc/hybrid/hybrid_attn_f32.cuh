@@ -4,7 +4,8 @@
 // 0.9 GFLOP.  Here 32 queries share the keys: tiles of 32 keys and values come by cp.async, two stages; 256 threads form the 32 x 32 scores (2 queries x 2 keys each:
 // 4 16-byte loads for 16 FMAs, a dot product is one chain over d as before), the running (maximum, sum) of a query lives in the 16 lanes that hold its scores, and the weights
 // go transposed through shared memory to the threads that own 4 queries x E / 32 columns of the output.  68 us.  What bounds it now: the loads out of shared
-// memory (about 1.5 cycles to each of FMA) and, for prompts this short, the few tiles in flight.
+// memory (about 1.5 cycles to each of FMA) and, for prompts this short, the few tiles in flight.  Few rows over many keys, whose tiles would be a handful of CTAs that
+// walk all keys in turn, stay with attn_bias_kernel (the caller's choice).
 //
 // Bias, soft cap, sinks, gates, windows, chunks and rings as in attn_bias_kernel.  A key that a query does not see enters nothing, whatever its numbers: on tiles that
 // some query's range cuts, products are taken by index and not by a weight of zero (0 x infinity).

@@ -10,9 +10,10 @@
 //                       every rank of an expert-parallel group, which is what lets ranks write each other's rows), and the list
 //                       of m tiles of the experts this rank owns.
 //   moe_gather_kernel   xs[slot] = hn[token], row_w[slot] = routing weight  (rows of local experts only)
-//   gemm_tcgen05_grouped_kernel x2 (gemm_tcgen05.cuh): g = silu(xs W1_e^T) * (xs W3_e^T);  yw = bf16(w * bf16(g W2_e^T)), the
-//                       second one storing every row on ALL ranks of the group (peer stores over NVLink) -- the exchange step of
-//                       expert parallelism is the epilogue of the down projection, an all-gather of rows with no reduction.
+//   grouped GEMM x2     g = silu(xs W1_e^T) * (xs W3_e^T);  yw = bf16(w * bf16(g W2_e^T)), the second one storing every row on ALL
+//                       ranks of the group (peer stores over NVLink) -- the exchange step of expert parallelism is the epilogue of
+//                       the down projection, an all-gather of rows with no reduction.  gemm_streamk.cuh for few tokens,
+//                       gemm_tcgen05.cuh, and from ~512 rows an expert gemm_pair.cuh.
 //   moe_combine_kernel  (expert parallel: signal the peers / wait for theirs) out[t] = bf16(h[t] + sum_j yw[slot(t, j)]) with the
 //                       sum taken in ascending expert index, each step rounded to bf16 like `results +=` -- bit-identical to the
 //                       reference for any k and any number of ranks.
@@ -115,8 +116,9 @@ __global__ void __launch_bounds__(256) moe_route_kernel(const bf16* hn, const bf
 }
 
 // ---- plan: one CTA ---------------------------------------------------------------------------------------------------------
-// plan layout (int32): [0] m tiles owned by this rank, [1] padded rows in total, [2] tile capacity, [3] pairs, [4]/[5] statistics, [8 + e] start of
-// expert e's segment (e = 0..E), then tile_expert[capacity], tile_row0[capacity] from word MOE_PLAN_HEADER.
+// plan layout (int32): [0] m tiles owned by this rank, [1] padded rows in total, [2] tile capacity, [3] (token, expert) pairs, [4]/[5] statistics, [6] token tiles for
+// pairs of CTAs, [8 + e] start of expert e's segment (e = 0..E), then from word MOE_PLAN_HEADER four lists of `capacity` words: tile_expert, tile_row0 (m tiles),
+// pair_expert, pair_info (token tiles: first row | width / 32).
 constexpr int MP_THREADS = 1024, MP_ROW = MP_THREADS + MP_THREADS / 32;
 inline size_t moe_plan_smem(int64_t E) { return ((size_t)E * MP_ROW + 2 * E + 1) * sizeof(int32_t); }
 __global__ void __launch_bounds__(MP_THREADS) moe_plan_kernel(const int32_t* sel, int pairs, int E, int tile_rows, int shard_rank,
@@ -467,6 +469,8 @@ int launch_grouped(const void* a, int64_t rows_cap, int64_t K, int64_t N, const 
     return launch_grouped_streamk<MODE, 64>(a, rows_cap, K, N, w_host, E, plan, epi, workspace, workspace_bytes, header, sms, stream);
   }
   if (tile_rows == 128) {
+    // From about 384 rows an expert.  The layer of eight experts of 4096 x 14336 with the GEMMs below and with pairs, us: 300 tokens (75 rows an expert) 529, 562, 600 691, 598,
+    // 1000 836, 775, 1300 970, 1004, 1536 1182, 1079, 2048 1496, 1411.  (The line dates from tiles of 128-row pairs, half of which such segments left empty.)
     if (N % 128 == 0 && tcgen05_cluster_enabled() && rows_cap >= (int64_t)E * 512) {
       CUtensorMap map_a;
       MoeWeightMaps maps;
@@ -523,8 +527,8 @@ int launch_grouped(const void* a, int64_t rows_cap, int64_t K, int64_t N, const 
 //   grouped GEMM       rows32 = act W2_e^T                       (fp32 rows: the sum over a token's experts is never below fp32)
 //   layer_moe_combine  y32[t] (+)= sum_j rows32[slot(t, j)]      in the order of the token's choices: no atomics, the same bits each time
 // The experts lie packed in one matrix each (w13 [E * units, width], w2 [width, E * ff]): one tensor map, offsets by expert.
-// Choices >= E (identity experts) get no row.  A mixture's prompt of 2500 tokens, 16 experts of 1408, top 4 of 20 outputs, width 2048:
-// 800 us before (all experts on all tokens), 291 us now, of which 150 us are the grouped GEMMs and 49 us the router.
+// Choices >= E (identity experts) get no row; the combine adds them as the token itself.  A mixture's prompt of 2500 tokens, 16 experts of 1408, top 4 of 20 outputs,
+// width 2048: 800 us before (all experts on all tokens), 248 us now, of which ~150 us are the grouped GEMMs, 24 the router and 12 the plan.
 __global__ void __launch_bounds__(256) layer_moe_gather_kernel(const uint4* hn, const float* wsel, const int32_t* slot,
                                                                int pairs, int k, int row_chunks, uint4* __restrict__ xs, float* __restrict__ row_w) {
   pdl_trigger();
@@ -587,7 +591,9 @@ inline int launch_grouped_packed(const void* a, int64_t rows_cap, int64_t K, int
   rc = make_tensor_map_2d(&maps.m[0], w, w_rows, w_cols, TG_BM);
   if (rc) return rc;
   for (int e = 1; e < MOE_MAX_EXPERTS; ++e) maps.m[e] = maps.m[0];
-  if (tcgen05_cluster_enabled() && pairs >= 384 * E && pairs > 512)  // (the plan of up to 512 rows lists no token tiles of pairs)
+  // As in launch_grouped.  16 experts of 1408, width 2048, with the GEMM below and with pairs, us: 400 tokens 108, 107, 800 146, 127, 1200 168, 148, 1800 225, 180; eight of
+  // 14336, width 4096: 600 tokens 855, 595, 1300 1356, 1075, 2500 2333, 1800.  (The plan of up to 512 rows lists no token tiles of pairs.)
+  if (tcgen05_cluster_enabled() && pairs >= 384 * E && pairs > 512)
     return launch_grouped_pair<EPI_LAYER>(map_a, maps, rows_cap, K, N, w_n, w_k, plan, epi, sms, stream);
   using Cfg = TgCfg<128, 128, kEpiSmem<EPI_LAYER>>;
   TcGemmParams p;

@@ -13,8 +13,8 @@
 
 namespace mb200 {
 
-// Pairs of 256 x 256 outputs (gemm_tcgen05.cuh) run in rounds of `units` clusters; when the last round is at most half full, its pairs are cut along k
-// into as many parts as fill it (at most four, eight k-blocks each, max_parts partial sums): cut_pairs pairs in `cut` parts.  No cut: 0, 1.
+// Tiles of pairs of CTAs (gemm_pair.cuh: 256 features x up to 256 tokens) run in rounds of `units` clusters; when the last round is at most half full, its tiles are cut along k
+// into as many parts as fit it (at most four, eight k-blocks each, max_parts partial sums): cut_pairs tiles in `cut` parts.  No cut: 0, 1.
 struct CutPlan {
   int cut_pairs, cut;
 };
@@ -31,7 +31,7 @@ MB_HD CutPlan cut_plan(long long pairs, int num_k, int units, int max_parts) {
   return c;
 }
 
-// Item s of the last round: which part of which cut pair.  The last parts come first and the owners (part 0, which holds the first k-blocks) last;
+// Item s of the last round: which part of which cut tile.  The last parts come first and the owners (part 0, which holds the first k-blocks) last;
 // a round is one item a cluster, so item s runs on cluster s of the launch.
 struct CutItem {
   int part, slot;
