@@ -532,7 +532,7 @@ __device__ __forceinline__ void epi_chunk32(const EpiParams& p, int t, int n, co
 
 // ---- feature-lane epilogues (gemm_pair.cuh) ------------------------------------------------------------------------------------
 // There a warp's accumulator block has the 32 features in its lanes and 32 tokens in each lane's registers.  Lanes 2i and 2i + 1 exchange halves, as bf16 pairs, and
-// then hold both features of pair i for 16 tokens each: what epi_pair takes.  A store instruction writes the 32 features of two tokens (2 x 64 bytes).
+// then hold both features of pair i for 16 tokens each: what epi_pair takes.  For a store four features of a token come together (exchange_rows8).
 // y0, y1: features n, n + 1 of tokens t0 + j, as packed pairs of tokens (2q, 2q + 1); tokens from `rows` on are not stored.
 __device__ __forceinline__ float bf16_of(const uint32_t (&y)[8], int j) { return j & 1 ? bf16hi(y[j >> 1]) : bf16lo(y[j >> 1]); }
 
@@ -571,6 +571,28 @@ __device__ __forceinline__ void epi_pairs16_fetch(const EpiParams& p, int t0, in
   }
 }
 
+// A lane has features n, n + 1 (o[j]) of 16 tokens; lanes whose numbers differ by 2 exchange halves, and v[q] are features n & ~3 .. | 3 of token rows8() + q: eight
+// stores of 8 bytes where sixteen of 4 held up the MMAs, whose operands come out of L2 while a tile's results go there.  4096 x 18944 x 2048 219.6 -> 217.1 us,
+// 4096 x 4096 x 2048 60.3 -> 59.2, 4096 x 9472 x 4096 205.3 -> 203.8.  (Four stores of 16 bytes, one more exchange: 216.6, 59.9, 203.8.  Gated units by 8
+// bytes instead of 4: 1024 x 16384 x 2048 58 -> 61 in a loop, so they keep 4.)
+__device__ __forceinline__ int rows8() { return threadIdx.x & 2 ? 8 : 0; }
+__device__ __forceinline__ void exchange_rows8(const uint32_t (&o)[16], uint2 (&v)[8]) {
+  const bool hi = threadIdx.x & 2;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const uint32_t own = hi ? o[8 + q] : o[q], other = __shfl_xor_sync(0xffffffffu, hi ? o[q] : o[8 + q], 2);
+    v[q] = hi ? make_uint2(other, own) : make_uint2(own, other);
+  }
+}
+// base: features n & ~3 of the first of the 16 tokens, `rows` of which are there
+__device__ __forceinline__ void store_rows8(uint16_t* base, int ld, int rows, const uint2 (&v)[8]) {
+  const int t = rows8();
+  uint16_t* dst = base + (int64_t)t * ld;
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+    if (t + q < rows) *reinterpret_cast<uint2*>(dst + q * ld) = v[q];
+}
+
 // Gated units: 16 tokens of unit c (in lane pair by lane pair).  Two lane pairs exchange halves, so that a store is 4 bytes, units c & ~1 and c | 1 of a token.
 __device__ __forceinline__ void store_units16(void* out, int ld, int t0, int rows, int c, const float (&x)[16]) {
   const bool hi = threadIdx.x & 2;
@@ -589,7 +611,7 @@ __device__ __forceinline__ void store_units16(void* out, int ld, int t0, int row
 template <int MODE>
 __device__ __forceinline__ void epi_pairs16(const EpiParams& p, int t0, int rows, int n, const uint32_t (&y0)[8], const uint32_t (&y1)[8], const uint32_t (&r)[16]) {
   if constexpr (MODE == EPI_STORE || MODE == EPI_RESIDUAL || MODE == EPI_MOE_SCALE) {
-    const int64_t off = (int64_t)t0 * p.ld_out + n;
+    const int64_t off = (int64_t)t0 * p.ld_out + (n & ~3);
     uint32_t o[16];
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
@@ -601,17 +623,11 @@ __device__ __forceinline__ void epi_pairs16(const EpiParams& p, int t0, int rows
       else
         o[j] = __byte_perm(y0[j >> 1], y1[j >> 1], j & 1 ? 0x7632 : 0x5410);
     }
-    uint16_t* dst = reinterpret_cast<uint16_t*>(p.out) + off;
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-      if (j < rows) *reinterpret_cast<uint32_t*>(dst + j * (int)p.ld_out) = o[j];
+    uint2 v[8];
+    exchange_rows8(o, v);
+    store_rows8(reinterpret_cast<uint16_t*>(p.out) + off, (int)p.ld_out, rows, v);
     if constexpr (MODE == EPI_MOE_SCALE) {
-      for (int k = 0; k < p.n_peers; ++k) {  // the same rows on the other ranks (NVLink peer stores)
-        uint16_t* pd = reinterpret_cast<uint16_t*>(p.peer_out[k]) + off;
-#pragma unroll
-        for (int j = 0; j < 16; ++j)
-          if (j < rows) *reinterpret_cast<uint32_t*>(pd + j * (int)p.ld_out) = o[j];
-      }
+      for (int k = 0; k < p.n_peers; ++k) store_rows8(reinterpret_cast<uint16_t*>(p.peer_out[k]) + off, (int)p.ld_out, rows, v);  // the same rows on the other ranks (NVLink peer stores)
     }
   } else if constexpr (MODE == EPI_F32) {
     float* dst = p.out_f32 + (int64_t)t0 * p.ld_out + n;
@@ -641,20 +657,20 @@ __device__ __forceinline__ void epi_pairs16(const EpiParams& p, int t0, int rows
 #pragma unroll
       for (int j = 0; j < 16; ++j) o[j] = __byte_perm(y0[j >> 1], y1[j >> 1], j & 1 ? 0x7632 : 0x5410);
     }
+    uint2 v[8];
+    exchange_rows8(o, v);
     const bool is_q = n < p.q_dim;
-    const int width = is_q ? p.q_dim : p.kv_dim, c = is_q ? n : (rotate ? n - p.q_dim : n - p.q_dim - p.kv_dim);
-    uint16_t* dst = reinterpret_cast<uint16_t*>(is_q ? p.q_out : (rotate ? p.k_out : p.v_out)) + (int64_t)t0 * width + c;
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-      if (j < rows) *reinterpret_cast<uint32_t*>(dst + j * width) = o[j];
+    const int width = is_q ? p.q_dim : p.kv_dim, c = (is_q ? n : (rotate ? n - p.q_dim : n - p.q_dim - p.kv_dim)) & ~3;
+    store_rows8(reinterpret_cast<uint16_t*>(is_q ? p.q_out : (rotate ? p.k_out : p.v_out)) + (int64_t)t0 * width + c, width, rows, v);
     if (ring) {
       uint16_t* cache = reinterpret_cast<uint16_t*>(rotate ? p.cache_k : p.cache_v) + c;
-      int row[16];
+      const int t = rows8();
+      int row[8];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) row[j] = j < rows ? p.cache_rows[t0 + j] : -1;
+      for (int q = 0; q < 8; ++q) row[q] = t + q < rows ? p.cache_rows[t0 + t + q] : -1;
 #pragma unroll
-      for (int j = 0; j < 16; ++j)
-        if (row[j] >= 0) *reinterpret_cast<uint32_t*>(cache + (int64_t)row[j] * p.kv_dim) = o[j];
+      for (int q = 0; q < 8; ++q)
+        if (row[q] >= 0) *reinterpret_cast<uint2*>(cache + (int64_t)row[q] * p.kv_dim) = v[q];
     }
   }
 }
@@ -664,7 +680,6 @@ template <bool SCALED>
 __device__ __forceinline__ void epi_layer_pairs16(const EpiParams& p, int t0, int rows, int n, const uint32_t (&y0)[8], const uint32_t (&y1)[8], const uint32_t (&r)[16]) {
   const int step = p.layer;
   if (step == LAYER_STORE || step == LAYER_RELU2) {
-    uint16_t* dst = reinterpret_cast<uint16_t*>(p.out) + (int64_t)t0 * p.ld_out + n;
     uint32_t o[16];
     if (step == LAYER_STORE) {
       const bool act0 = n < p.n_act, act1 = n + 1 < p.n_act;
@@ -697,9 +712,9 @@ __device__ __forceinline__ void epi_layer_pairs16(const EpiParams& p, int t0, in
         o[j] = pack2_rn(u, v);
       }
     }
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-      if (j < rows) *reinterpret_cast<uint32_t*>(dst + j * (int)p.ld_out) = o[j];
+    uint2 v[8];
+    exchange_rows8(o, v);
+    store_rows8(reinterpret_cast<uint16_t*>(p.out) + (int64_t)t0 * p.ld_out + (n & ~3), (int)p.ld_out, rows, v);
     return;
   }
   float s[16], x[16];
