@@ -113,11 +113,18 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return t.data_ptr()
 
 
-_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)  # the current stream's handle without its Python objects, where torch has it
+def _public_stream() -> int:
+    return torch.cuda.current_stream().cuda_stream
 
 
-def _stream() -> int:
-    return _raw_stream(torch.cuda.current_device()) if _raw_stream is not None else torch.cuda.current_stream().cuda_stream
+_raw_getter = getattr(torch._C, "_cuda_getCurrentRawStream", None)  # the same handle without a stream's Python objects, where torch has it
+
+
+def _raw_stream() -> int:
+    return _raw_getter(torch.cuda.current_device())
+
+
+_stream = _public_stream if _raw_getter is None else _raw_stream
 
 
 class Workspace:

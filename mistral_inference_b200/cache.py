@@ -237,19 +237,20 @@ class BufferCache:
         longest = int(max(seqlens))
         layout = {"T": T, "B": B, "prefill": first_prefill or longest > 1, "first_prefill": first_prefill, "max_seqlen": longest, "windows": distinct}
         lens = [int(n) for n in seqlens]
-        (self._fill_sequences if self._by_sequence(lens, T, distinct) else self._fill_tokens)(host, lens, T, distinct)
+        (self._fill_sequences if self._by_sequence(B, longest, T, distinct) else self._fill_tokens)(host, lens, T, distinct)
         if with_slots:
             host[total - B:] = self.rows
         layout["slots"] = with_slots
         return host, layout
 
-    def _by_sequence(self, lens: List[int], T: int, windows: List[int]) -> bool:
+    def _by_sequence(self, B: int, longest: int, T: int, windows: List[int]) -> bool:
         """Which way of filling the block costs less, from the calls that each makes (us, measured): sequence by sequence a few per sequence and window, more
         where a ring wraps; over all tokens some thirty in all and more per token.  One window, sequence by sequence and over all tokens: 5 x 35 tokens 14, 21;
         8 x 1 20, 18; 16 x 1 39, 19; 16 x 400 51, 93; 16 x 1 behind a ring that wraps 79, 19."""
-        longest = max(p + n for p, n in zip(self._kv_seqlens_host, lens))
-        rings = sum(3.7 if longest > W else 1.0 for W in windows)
-        return len(lens) * (1.5 + rings) <= 10 + 8 * len(windows) + T * (0.008 + 0.009 * len(windows))
+        end, rings = max(self._kv_seqlens_host) + longest, 1.5
+        for W in windows:
+            rings += 3.7 if end > W else 1.0
+        return B * rings <= 10 + 8 * len(windows) + T * (0.008 + 0.009 * len(windows))
 
     def _fill_sequences(self, host: np.ndarray, lens: List[int], T: int, windows: List[int]) -> None:
         """The block of few sequences, one after the other."""
