@@ -393,7 +393,7 @@ def run_ours(a, rank: int, world: int):
 
     cpu = cpu_baseline(a, p, bounded_seconds=20.0) if (world == 1 and not a.no_cpu_baseline) else None
     step_gbs = step_bytes / (ms_per_step * 1e-3) / 1e9
-    prefill_kernels = ("gemm_tcgen05_kernel (tcgen05.mma/TMEM/TMA, 2-CTA MMAs) + attn_prompt_tcgen05_kernel "
+    prefill_kernels = ("gemm_pair_kernel (tcgen05.mma/TMEM/TMA, 2-CTA MMAs) + attn_prompt_tcgen05_kernel "
                        "(tcgen05 flash attention, S/P/O in TMEM) + rmsnorm/kv_ring_write" + (" + grouped expert GEMMs" if p.get("moe") else ""))
     per_layer = 9 if p.get("moe") else 7
     return {

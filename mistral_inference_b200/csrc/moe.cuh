@@ -15,8 +15,9 @@
 //                       the down projection, an all-gather of rows with no reduction.  gemm_streamk.cuh for few tokens,
 //                       gemm_tcgen05.cuh, and from ~512 rows an expert gemm_pair.cuh.
 //   moe_combine_kernel  (expert parallel: signal the peers / wait for theirs) out[t] = bf16(h[t] + sum_j yw[slot(t, j)]) with the
-//                       sum taken in ascending expert index, each step rounded to bf16 like `results +=` -- bit-identical to the
-//                       reference for any k and any number of ranks.
+//                       sum taken in ascending expert index, each step rounded to bf16 like `results +=`: the reference's
+//                       order for any k and any number of ranks.  (The rows themselves are the same on any number of ranks but for
+//                       stream-K's, whose sums are cut by the tiles that a rank has.)
 // Roofline: tensor pipe for prefill (2 * rows * 3 * dim * hidden flop), HBM for decode (every touched expert's weights once).
 #pragma once
 #include "gemm_pair.cuh"

@@ -14,7 +14,8 @@ the others.  Every rank evaluates the router and the row plan redundantly (deter
 grouped GEMMs for its own experts, and the DOWN PROJECTION'S EPILOGUE stores each weighted output row into the row buffer of
 every rank over NVLink (peer memory mapped with CUDA IPC, `ExpertComm`): the exchange is an all-gather of rows fused into the
 GEMM, not a collective call after it.  After a flag handshake every rank combines all k rows of every token in the reference's
-order, so the result is bit-identical to the unsharded model for any k -- no reduction order is left to a library.
+order: no reduction order is left to a library.  Calls of more than 64 tokens give the unsharded model's bits for any k; up to 64 the stream-K GEMM cuts
+its sums by the tiles that a rank has, and a row may differ by a bf16 rounding.
 """
 import ctypes
 from typing import Dict, List, Optional, Tuple

@@ -1,7 +1,7 @@
 """Expert-parallel MoE with the real kernels: each rank owns the experts e % world == rank of a small Mixtral-style model; the down
 projection's epilogue stores every weighted expert row into every rank's row buffer (CUDA-IPC peer memory), a flag handshake follows, and
-every rank combines all rows in the reference's order (csrc/moe.cuh).  Prefill + decode logits must equal the UNSHARDED model's bit for
-bit -- for top-2 and for top-3 routing (no reduction order is left open).
+every rank combines all rows in the reference's order (csrc/moe.cuh).  Prompts must equal the UNSHARDED layer's bit for bit -- for top-2 and
+for top-3 routing (no reduction order is left open) -- and at these sizes, where stream-K's blocks have a k-block each, decode steps too.
 
 Two set-ups:
   * the ranks' calls one after the other on one GPU, in one process: "peer" buffers are other tensors, and the handshake's flags are set
