@@ -4,7 +4,9 @@
 
 namespace mb200 {
 
-// out = bf16( bf16( x * rsqrt(mean(x^2) + eps) ) * w ), one CTA per token (transformer_layers.py:115-120)
+// out = bf16( bf16( x * rsqrt(mean(x^2) + eps) ) * w ), one CTA per token (transformer_layers.py:115-120).  Latency-bound: a row's loads, the weight's among them, stand in
+// flight together and stay in registers for the second pass (up to 8 * 256 * RN_KEEP columns; read twice, a step of 7 layers of the 7B shape took 5 us more).
+constexpr int RN_KEEP = 3;
 __global__ void __launch_bounds__(256) rmsnorm_kernel(const uint4* x, const uint4* __restrict__ w, uint4* __restrict__ out,
                                                       int dim, float eps) {
   pdl_trigger();
@@ -13,9 +15,15 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const uint4* x, const uint
   const uint4* xr = x + (int64_t)blockIdx.x * kc;
   uint4* orow = out + (int64_t)blockIdx.x * kc;
   __shared__ float red[8];
+  uint4 xv[RN_KEEP], wv[RN_KEEP];
+#pragma unroll
+  for (int k = 0; k < RN_KEEP; ++k) {
+    const int c = threadIdx.x + 256 * k;
+    xv[k] = wv[k] = make_uint4(0u, 0u, 0u, 0u);
+    if (c < kc) xv[k] = xr[c], wv[k] = w[c];
+  }
   float ss = 0.f;
-  for (int c = threadIdx.x; c < kc; c += 256) {
-    const uint4 v = xr[c];
+  auto square = [&](const uint4& v) {
     const uint32_t u[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -23,7 +31,10 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const uint4* x, const uint
       ss = fmaf(a, a, ss);
       ss = fmaf(b, b, ss);
     }
-  }
+  };
+#pragma unroll
+  for (int k = 0; k < RN_KEEP; ++k) square(xv[k]);
+  for (int c = threadIdx.x + 256 * RN_KEEP; c < kc; c += 256) square(xr[c]);
   ss = warp_sum(ss);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
   __syncthreads();
@@ -31,15 +42,18 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const uint4* x, const uint
 #pragma unroll
   for (int i = 0; i < 8; ++i) tot += red[i];
   const float r = ref_rsqrt(tot / (float)dim + eps);
-  for (int c = threadIdx.x; c < kc; c += 256) {
-    const uint4 v = xr[c], g = w[c];
+  auto emit = [&](int c, const uint4& v, const uint4& g) {
     const uint32_t u[4] = {v.x, v.y, v.z, v.w}, gw[4] = {g.x, g.y, g.z, g.w};
     uint32_t o[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j)
       o[j] = pack_bf16x2(round_bf16(bf16lo(u[j]) * r) * bf16lo(gw[j]), round_bf16(bf16hi(u[j]) * r) * bf16hi(gw[j]));
     orow[c] = make_uint4(o[0], o[1], o[2], o[3]);
-  }
+  };
+#pragma unroll
+  for (int k = 0; k < RN_KEEP; ++k)
+    if (threadIdx.x + 256 * k < kc) emit(threadIdx.x + 256 * k, xv[k], wv[k]);
+  for (int c = threadIdx.x + 256 * RN_KEEP; c < kc; c += 256) emit(c, xr[c], w[c]);
 }
 
 // cache[rows[t]] = src[t] for rows[t] >= 0 (cache.py:91-92); one warp per (token, K|V) row of KV*hd bf16

@@ -41,7 +41,7 @@ def rope():
     return table, torch.view_as_real(table).contiguous().to(DEV)
 
 
-@pytest.mark.parametrize("T,dim", [(1, 256), (5, 4096), (33, 5120), (2, 6144)])
+@pytest.mark.parametrize("T,dim", [(1, 256), (5, 4096), (33, 5120), (2, 6144), (3, 6152), (2, 14336)])  # the last two: more columns than stay in registers
 def test_rmsnorm(T, dim):
     x, w = rnd(T, dim, seed=1, scale=2.0), (1 + 0.2 * rnd(dim, seed=2).float()).to(torch.bfloat16)
     got = _abi.rmsnorm(x.to(DEV), w.to(DEV), 1e-5)
