@@ -140,10 +140,10 @@ def test_gemm_against_cuda_core_gemm(ws):
 
 @pytest.mark.parametrize("bn", ["128", "192", "256"])
 def test_gemm_cluster_pair_matches_single_cta(ws, bn, monkeypatch):
-    """T >= 512 runs the 2-CTA kernel (one MMA of 256 rows over both); 128-row slices of the same input run the
-    single-CTA kernel.  Rows are independent and accumulate in the same k order, so the two must agree bit for bit --
-    through the residual and the SiLU*mul epilogues, with a ragged last tile and an odd number of row tiles, for both tile
-    widths (the launcher picks the width per shape; MB200_GEMM_BN pins it here)."""
+    """Pinned to 256, T >= 512 runs on pairs of CTAs (weights as the rows of shared MMAs); 128 and 192, and 128-row slices of the same input,
+    run the single-CTA kernel.  Tokens are independent and accumulate in the same k order, so all must agree bit for bit --
+    through the residual and the SiLU*mul epilogues, with a ragged last tile and an odd number of row tiles
+    (the launcher picks the kernel and width per shape; MB200_GEMM_BN pins it here)."""
     monkeypatch.setenv("MB200_GEMM_BN", bn)
     monkeypatch.setenv("MB200_STREAMK", "0")  # the 128-row slices below must take the single-CTA tcgen05 kernel, not the stream-K one
     T, dim, hid = 700, 1536, 1536  # N = 1536 / 3072: multiples of all three tile widths
@@ -181,8 +181,8 @@ def test_gemm_cluster_pair_matches_single_cta(ws, bn, monkeypatch):
 
 
 def test_qkv_rope_epilogue_same_bits_for_every_tile_width(ws, rope, monkeypatch):
-    """Fused QKV + RoPE + ring scatter at Mistral-7B width (N = 6144 = 24 x 256 = 32 x 192 = 48 x 128) through the 2-CTA
-    cluster kernel: the three tile widths must produce identical q / k / v and identical cache rows."""
+    """Fused QKV + RoPE + ring scatter at Mistral-7B width (N = 6144 = 24 x 256 = 32 x 192 = 48 x 128) on pairs of CTAs
+    (256) and on single ones (192, 128): identical q / k / v and identical cache rows."""
     T, dim, H, KV, hd = 640, 4096, 32, 8, 128
     x = rnd(T, dim, seed=40).to(DEV)
     nw = (1 + 0.2 * rnd(dim, seed=41).float()).to(torch.bfloat16).to(DEV)
