@@ -14,7 +14,7 @@ from . import _abi, build
 from ._abi import Mb200Error, _stream
 
 ABI_VERSION = 8
-EPI_STORE, EPI_RESIDUAL, EPI_GLU, EPI_F32, EPI_SWIGLU, EPI_RESIDUAL_SCALED, EPI_RELU2, EPI_GEGLU = 0, 1, 2, 3, 4, 5, 6, 7
+EPI_STORE, EPI_RESIDUAL, EPI_GLU, EPI_F32, EPI_SWIGLU, EPI_RESIDUAL_SCALED, EPI_RELU2, EPI_GEGLU, EPI_DECAY = 0, 1, 2, 3, 4, 5, 6, 7, 8
 _DT = {torch.bfloat16: 0, torch.float32: 1}
 _lib: Optional[ctypes.CDLL] = None
 
@@ -26,6 +26,8 @@ _SIGNATURES = {
     "mbh_rmsnorm": (c_int, [P, P, P, P, P, I, I, F, F, c_int, P]),
     "mbh_linear_decay": (c_int, [P, I, P, P, P, I, P, I, I, I, c_int, P]),
     "mbh_linear": (c_int, [P, I, P, P, P, P, I, I, I, c_int, I, F, F, c_int, P]),
+    "mbh_linear_scratch": (I, [I, I, I, c_int]),
+    "mbh_linear_any": (c_int, [P, I, P, P, P, P, I, I, I, c_int, I, F, F, P, I, I, P, P, I, c_int, P]),
     "mbh_attn_prep": (c_int, [P, P, P, P, P, P, P, P, P, P, c_int, I, I, I, I, I, F, F, I, c_int, P]),
     "mbh_attn_bias": (c_int, [P, P, P, P, I, P, P, P, P, I, I, I, I, I, I, I, F, I, I, P, c_int, P]),
     "mbh_lightning_scan": (c_int, [P, P, P, P, P, P, P, I, I, I, I, c_int, P]),
@@ -134,6 +136,7 @@ def rmsnorm_pair(x32: torch.Tensor, w: torch.Tensor, w2: torch.Tensor, eps: floa
     return y, y2
 
 
+SKINNY_MAX_ROWS = 8  # of fp32: more rows run on tensor cores
 PROMPT_GEMM_MIN_ROWS = 17  # fewer rows: this library's own kernel, which streams the weights past up to 16 tokens
 
 
@@ -149,6 +152,21 @@ def _prompt_gemm_ok(x: torch.Tensor, M: int, N: int, K: int) -> bool:
 def _aligned(*tensors: Optional[torch.Tensor]) -> bool:
     """16-byte aligned starts: what the tensor-core GEMM's copies and vector accesses need."""
     return all(t is None or t.data_ptr() % 16 == 0 for t in tensors)
+
+
+def _linear_f32(x, w, bias, out, out32, epi: int, n_act: int = 0, limit: float = 0.0, alpha: float = 0.0, rowscale=None, group: int = 0, a_log=None) -> bool:
+    """fp32 prompts: the call with room for the parts of x from the caching allocator.  False: a call that needs none."""
+    M, K, N = x.shape[0], x.shape[1], w.shape[0]
+    if x.dtype != torch.float32 or M <= SKINNY_MAX_ROWS:
+        return False
+    need = lib().mbh_linear_scratch(M, N, K, 1)
+    if not need:
+        return False
+    xp, ldx = _rows(x)
+    scratch = torch.empty(need, dtype=torch.uint8, device=x.device)
+    _check(lib().mbh_linear_any(xp, ldx, _ptr(w), _ptr(bias), _ptr(out), _ptr(out32), M, N, K, epi, n_act, limit, alpha, _ptr(rowscale), rowscale.shape[1] if rowscale is not None else 0,
+                                group, _ptr(a_log), _ptr(scratch), need, 1, _stream()), "mbh_linear_any")
+    return True
 
 
 def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, *, epi: int = EPI_STORE, n_act: int = 0,
@@ -172,6 +190,8 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None
         if _aligned(xc):
             _abi.layer_linear(xc, w, bias, out, out32, epi, n_act, limit, alpha)
             return out if out is not None else out32
+    if _linear_f32(x, w, bias, out, out32, epi, n_act, limit, alpha):
+        return out if out is not None else out32
     xp, ldx = _rows(x)
     _check(lib().mbh_linear(xp, ldx, _ptr(w), _ptr(bias), _ptr(out), _ptr(out32), M, N, K, epi, n_act, limit, alpha, dt_of(x.dtype), _stream()),
            "mbh_linear")
@@ -184,6 +204,8 @@ def linear_decay(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor],
     N = w.shape[0]
     assert w.shape[1] == K and x.dtype == w.dtype and a_log.dtype == w.dtype and a_log.numel() * group == N
     out = torch.empty(M, N, dtype=torch.float32, device=x.device)
+    if _linear_f32(x, w, bias, None, out, EPI_DECAY, group=group, a_log=a_log):
+        return out
     xp, ldx = _rows(x)
     _check(lib().mbh_linear_decay(xp, ldx, _ptr(w), _ptr(bias), _ptr(a_log), group, _ptr(out), M, N, K, dt_of(x.dtype), _stream()), "mbh_linear_decay")
     return out
@@ -301,6 +323,8 @@ def linear_swiglu(x: torch.Tensor, w: torch.Tensor, rowscale: Optional[torch.Ten
     out = torch.empty(M, N // 2, dtype=x.dtype, device=x.device)
     if _prompt_gemm_ok(x, M, N, K) and _aligned(x, w):
         _abi.layer_linear(x, w, None, out, None, EPI_GEGLU if gelu else EPI_SWIGLU, rowscale=rowscale, group=max(group, 1))
+        return out
+    if _linear_f32(x, w, None, out, None, EPI_GEGLU if gelu else EPI_SWIGLU, rowscale=rowscale, group=group):
         return out
     _check(lib().mbh_linear_swiglu(_ptr(x), _ptr(w), _ptr(out), M, N, K, _ptr(rowscale), pitch, group, int(gelu), dt_of(x.dtype), _stream()),
            "mbh_linear_swiglu")
@@ -641,6 +665,8 @@ def linear_glu(x: torch.Tensor, w: torch.Tensor, limit: float, alpha: float, row
     if _prompt_gemm_ok(x, M, N, K) and _aligned(x, w):
         _abi.layer_linear(x, w, None, out, None, EPI_GLU, limit=limit, alpha=alpha, rowscale=rowscale, group=max(group, 1))
         return out
+    if _linear_f32(x, w, None, out, None, EPI_GLU, limit=limit, alpha=alpha, rowscale=rowscale, group=group):
+        return out
     _check(lib().mbh_linear_glu(_ptr(x), _ptr(w), _ptr(out), M, N, K, limit, alpha, _ptr(rowscale), pitch, group, dt_of(x.dtype), _stream()), "mbh_linear_glu")
     return out
 
@@ -722,6 +748,8 @@ def linear_relu2(x: torch.Tensor, w: torch.Tensor, rowscale: Optional[torch.Tens
     out = torch.empty(M, N, dtype=x.dtype, device=x.device)
     if _prompt_gemm_ok(x, M, N, K) and _aligned(x, w):
         _abi.layer_linear(x, w, None, out, None, EPI_RELU2, rowscale=rowscale, group=max(group, 1))
+        return out
+    if _linear_f32(x, w, None, out, None, EPI_RELU2, rowscale=rowscale, group=group):
         return out
     _check(lib().mbh_linear_relu2(_ptr(x), _ptr(w), _ptr(out), M, N, K, _ptr(rowscale), pitch, group, dt_of(x.dtype), _stream()), "mbh_linear_relu2")
     return out

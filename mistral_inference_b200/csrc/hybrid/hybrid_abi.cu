@@ -16,6 +16,7 @@
 #include "hybrid_stream.cuh"
 #include "hybrid_error.h"
 #include "../../../include/mistral_b200_hybrid.h"
+#include "../../../include/mistral_b200_hybrid_linear.h"
 
 #include <stdio.h>
 
@@ -180,6 +181,25 @@ int mbh_rmsnorm(const void* x32, const void* w, const void* w2, void* y, void* y
     DISPATCH(dt, run_rmsnorm<ST>(x32, w, w2, y, y2, T, D, eps, offset, st));
     cudaError_t e = cudaGetLastError();
     return e ? fail(e, "mbh_rmsnorm") : 0;
+}
+
+int64_t mbh_linear_scratch(int64_t M, int64_t N, int64_t K, int dt) {
+    if (dt != 1 || M <= SK_MAX_M || N <= 0 || K < FT_MIN_K) return 0;
+    return f32_scratch_bytes((int)M, (int)N, (int)K, FT_TO_SLOTS);
+}
+
+int mbh_linear_any(const void* x, int64_t ldx, const void* w, const void* bias, void* out, void* out32, int64_t M, int64_t N, int64_t K, int epi, int64_t n_act, float limit,
+                   float alpha, const void* rowscale, int64_t rs_pitch, int64_t rs_group, const void* a_log, void* scratch, int64_t scratch_bytes, int dt, void* stream) {
+    if (ldx < K) return bad("mbh_linear_any: rows of x overlap");
+    if (epi < 0 || epi > EPI_DECAY) return bad("mbh_linear_any: unknown epilogue");
+    if ((epi == EPI_GLU || epi == EPI_SWIGLU || epi == EPI_GEGLU) && (N & 1)) return bad("mbh_linear_any: the gated epilogues need interleaved (even) rows");
+    if ((rowscale && rs_group <= 0) || (epi == EPI_DECAY && (!a_log || rs_group <= 0 || N % rs_group))) return bad("mbh_linear_any: groups of outputs");
+    LinearArgs a{x, w, bias, out, (float*)out32, (int)M, (int)N, (int)K, epi, (int)n_act, limit, alpha, (const float*)rowscale, (int)rs_pitch, (int)rs_group};
+    a.a_log = a_log;
+    a.ldx = (int)ldx;
+    cudaError_t e = cudaSuccess;
+    DISPATCH(dt, e = launch_linear<ST>(a, (cudaStream_t)stream, scratch, scratch_bytes));
+    return e ? fail(e, "mbh_linear_any") : 0;
 }
 
 int mbh_linear(const void* x, int64_t ldx, const void* w, const void* bias, void* out, void* out32, int64_t M, int64_t N, int64_t K, int epi, int64_t n_act,

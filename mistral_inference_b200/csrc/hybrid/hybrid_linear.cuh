@@ -19,7 +19,7 @@
 // In bf16 mode the Linear's own output is rounded to bf16 before the epilogue's arithmetic (the rounding point of a bf16
 // Linear); accumulation is fp32 in both modes.
 //
-// Kernels: `linear_tiled_mma` (bf16), `linear_f32_parts` (fp32, hybrid_linear_f32.cuh) and `linear_tiled_fma` (fp32, K < 16) for prompts, any shape; `linear_skinny` (M <= 8 rows, FMA,
+// Kernels: `linear_tiled_mma` (bf16), `linear_f32_pair` (fp32, hybrid_linear_f32.cuh) and `linear_tiled_fma` (fp32, K < 16) for prompts, any shape; `linear_skinny` (M <= 8 rows, FMA,
 // one warp per pair of weight rows) and `linear_skinny_mma` (bf16, up to 16 rows, tensor cores) for decode: every weight byte is read
 // once with 16-byte loads; `linear_decay_mma` for decays from a low rank.  The large aligned bf16 Linears of prompts go to the main
 // library's tcgen05 GEMMs, with these steps in their epilogue (see _abi_hybrid.linear).
@@ -465,8 +465,9 @@ __global__ void __launch_bounds__(SKM_WARPS * 32, 2) linear_skinny_mma(LinearArg
 
 namespace mbh {
 
+// scratch: fp32 prompts; of mbh_linear_scratch bytes, or null: the call takes its own from the device's pool, in the order of the stream
 template <typename T>
-inline cudaError_t launch_linear(const LinearArgs& a, cudaStream_t st) {
+inline cudaError_t launch_linear(const LinearArgs& a, cudaStream_t st, void* scratch = nullptr, int64_t scratch_bytes = 0) {
     if (a.M <= 0 || a.N <= 0) return cudaSuccess;
     if constexpr (sizeof(T) == 2) {
         if (a.M <= SKM_MAX_M && a.K % 8 == 0 && a.x_pitch() % 8 == 0 && (reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.w)) % 16 == 0) {
@@ -483,10 +484,10 @@ inline cudaError_t launch_linear(const LinearArgs& a, cudaStream_t st) {
     } else if constexpr (sizeof(T) == 2) {
         dim3 grid((a.N + MM_BN - 1) / MM_BN, (a.M + MM_BM - 1) / MM_BM);
         linear_tiled_mma<<<grid, MM_THREADS, 0, st>>>(a);
-    } else if (a.K < FT_MIN_K) {
-        linear_tiled_fma<<<dim3((a.N + LT_BN - 1) / LT_BN, (a.M + LT_BM - 1) / LT_BM), LT_THREADS, 0, st>>>(a);
     } else {
-        return launch_linear_f32_parts(a, st);
+        cudaError_t e = cudaSuccess;
+        if (a.K >= FT_MIN_K && launch_linear_f32_pair(a, scratch, scratch_bytes, st, e)) return e;
+        linear_tiled_fma<<<dim3((a.N + LT_BN - 1) / LT_BN, (a.M + LT_BM - 1) / LT_BM), LT_THREADS, 0, st>>>(a);
     }
     return cudaGetLastError();
 }

@@ -12,61 +12,92 @@
 // more exact one for operands of one sign and keeps the job (linear_tiled_fma).  With truncated parts and without the scales, as this began: 1.6 at any K,
 // 7.8 for x = w = 1 + 2^-7 - 2^-23 and 300 at 2^-118.
 //
-// What bounds it: the sixteen warps that load, split, store and add.  750 x 16384 x 2048 under ncu: tensor pipe 38 % of the cycles, shared memory 41 %, both with
-// room.  The 64 x 64 FMA tiles it replaces (24 TFLOP/s of 74): 8870 us of Linears for 3 x ~250 tokens, width 2048, two layers; about 1820 here.
+// What bounds it: the MMAs, about 24 x (64 + w / 4) clocks a k-block of 64 for w tokens, and the power cap: 804 x 16384 x 2048 runs at 1.34 to 1.44 PFLOP/s of part products (225 us
+// stored, 236 with the gated unit, where tiles of 128 x 128 with both operands split in every CTA took 480); few tokens by the way of a k-block through two stages
+// (20 x 16384 x 2048: 51 us, 68 before, and 20 of them memory).
+// A pair of CTAs (cta_group::2) has 256 features x up to 224 tokens: the weights are the MMA's rows, because its columns can be any multiple of 16 and its
+// rows cannot.  x is split ahead, once, by a kernel of its own (f32_parts_kernel: 10 bytes an element) and comes in by TMA; W is split where it is used, each CTA its
+// own 128 rows, since its parts written out would cost 10 bytes an element of a matrix that is several times as large.
 //
-// CTA = 128 x 128 outputs, or one of `splits` parts of their k range (a cluster; the parts are added through distributed shared memory in
-// rank order, so a small problem fills the chip and the result is the same every time).  17 warps: sixteen load fp32 from global memory
-// (one k-block ahead, in registers), split, write the six part tiles (128B-swizzled, K-major) of a stage and add the block before to
-// their registers; one thread of the last issues the MMAs (with eight workers the loads' latency was in the open: 3530 us of Linears against 1870).  Two stages: the MMAs of a block run under the splitting of the next.
+// Warps: 0-7 load fp32 weights from global memory (one k-block ahead, in registers), split them and write the three part tiles (128B-swizzled, K-major) of a stage; 8-15 add
+// the sums of each k-block to their registers; 16 TMA (parts of x); 17 issues the MMAs for both CTAs.  Splitting and adding are warps of their own because each is a
+// chain of latencies of 1500 to 2500 clocks a k-block (a round trip to tensor memory alone is 300), and one warp that did both took 4000 of them for MMAs of 2800.
+// Two stages, two accumulators.  Clusters are persistent; a last round that is not full is cut along k, and f32_combine_kernel adds the parts in the order of k, so nobody waits for another
+// cluster and the result is the same every time.
+//
 // An infinity or a NaN in the operands of a tile, or a number from 2^120 on (256 x is formed): its outputs are computed again with FMAs (ft_fma_rows).
 #pragma once
+#include <cuda.h>
+
 #include "hybrid_linear.cuh"
 
 namespace mbh {
 
-constexpr int FT_BM = 128, FT_BN = 128, FT_BK = 64, FT_WARPS = 16 /* workers */, FT_THREADS = 32 * (FT_WARPS + 1), FT_TILE = 128 * 64 * 2;  // a part tile: 128 rows of 128 bytes
-constexpr int FT_MIN_K = 16;
-constexpr int FT_STAGE = 6 * FT_TILE, FT_SMEM = 2 * FT_STAGE + 1024, FT_LD = FT_BN + 4;
-static_assert(FT_BM * FT_LD * 4 <= 2 * FT_STAGE, "the sums of a tile fit in the stages");
+constexpr int FT_MIN_K = 16;  // shorter rows: linear_tiled_fma
+constexpr int FT_BN = 128, FT_BK = 64;  // features of a CTA (a pair: 256), columns of a k-block
+constexpr int FT_MAX_W = 224, FT_CHUNKS = FT_MAX_W / 32;  // tokens of a tile at most; blocks of 16 of them a warp adds up
+constexpr int FT_SPLIT_WARPS = 8, FT_SUM_WARPS = 8, FT_THREADS = 32 * (FT_SPLIT_WARPS + FT_SUM_WARPS + 4);
+// Registers a thread: 20 warps are launched with 96 each; the sums get 152 of them, the splitting warps 72 and the last four 32 (2 x 152 + 2 x 72 + 32 = 5 x 96).
+constexpr int FT_REGS = 96, FT_SPLIT_REGS = 72, FT_SUM_REGS = 152, FT_REST_REGS = 32;
+static_assert(2 * FT_SPLIT_REGS + 2 * FT_SUM_REGS + FT_REST_REGS <= 5 * FT_REGS, "a split of more than was launched with waits forever");
+constexpr int FT_TILE = FT_BN * FT_BK * 2, FT_STAGE = 3 * FT_TILE + 3 * (FT_MAX_W / 2) * FT_BK * 2;  // a part of W: 128 rows of 128 bytes; a stage: three of W, three of half the tile's tokens
+constexpr int FT_SMEM = 2 * FT_STAGE + 1024;
+constexpr int FT_REDO_WORDS = 512;  // a bit per tile of a cluster
+constexpr int FT_MAX_TOKENS = 4096;  // of a launch: the slots of a longer prompt would take as much memory as its result
 
 __device__ __forceinline__ uint32_t ft_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void ft_bar_init(uint64_t* b, uint32_t count) { asm volatile("mbarrier.init.shared.b64 [%0], %1;" ::"r"(ft_smem(b)), "r"(count) : "memory"); }
-__device__ __forceinline__ void ft_bar_arrive(uint64_t* b) { asm volatile("mbarrier.arrive.shared.b64 _, [%0];" ::"r"(ft_smem(b)) : "memory"); }
+__device__ __forceinline__ void ft_bar_arrive(uint32_t b) { asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(b) : "memory"); }  // b: ft_first_cta
+__device__ __forceinline__ void ft_bar_expect(uint64_t* b, uint32_t bytes) { asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" ::"r"(ft_smem(b)), "r"(bytes) : "memory"); }
 // Waits a bounded time.  false: gave up (the caller marks the CTA dead and goes on to the end without waiting again).
 __device__ __forceinline__ bool ft_bar_wait(uint64_t* b, uint32_t parity) {
     for (int i = 0; i < (1 << 22); ++i) {
         uint32_t ok;
-        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(ok) : "r"(ft_smem(b)), "r"(parity) : "memory");
+        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(ok) : "r"(ft_smem(b)), "r"(parity) : "memory");
         if (ok) return true;
     }
     return false;
 }
-// K-major, 128B-swizzled tile of 128-byte rows: 8-row groups 1024 B apart, version 1, layout SWIZZLE_128B
-__device__ __forceinline__ uint64_t ft_desc(uint32_t addr) {
-    return (uint64_t)((addr & 0x3ffff) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+// K-major, 128B-swizzled tile of 128-byte rows: 8-row groups 1024 B apart, version 1, layout SWIZZLE_128B.  The upper word of a descriptor is this, the lower the tile's address
+// in units of 16 bytes (and 1 << 16).
+constexpr uint32_t FT_DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t ft_desc_lo(uint32_t addr) { return ((addr & 0x3ffff) >> 4) | (1u << 16); }
+constexpr uint32_t FT_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(2 * FT_BN >> 4) << 24);  // bf16 x bf16 -> fp32, 256 rows; + the width / 8 at bit 17
+// D = A B (ACC false), A B + D / 2^DOWN, by the pair.  a, b: lower words of the descriptors (one addition each: the thread that issues is what bounds narrow tiles)
+template <bool ACC, int DOWN>
+__device__ __forceinline__ void ft_mma(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc) {
+    if constexpr (DOWN > 0)
+        asm volatile("{\n.reg .pred p;\n.reg .b64 da, db;\nmov.b64 da, {%1, %4};\nmov.b64 db, {%2, %4};\nsetp.ne.b32 p, 1, 0;\n"
+                     "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %3, p, %5;\n}\n" ::"r"(d), "r"(a), "r"(b), "r"(idesc), "n"(FT_DESC_HI), "n"(DOWN)
+                     : "memory");
+    else
+        asm volatile("{\n.reg .pred p;\n.reg .b64 da, db;\nmov.b64 da, {%1, %4};\nmov.b64 db, {%2, %4};\nsetp.ne.b32 p, %5, 0;\n"
+                     "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %3, p;\n}\n" ::"r"(d), "r"(a), "r"(b), "r"(idesc), "n"(FT_DESC_HI), "n"(ACC ? 1 : 0)
+                     : "memory");
 }
-constexpr uint32_t FT_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(FT_BN >> 3) << 17) | ((uint32_t)(FT_BM >> 4) << 24);  // bf16 x bf16 -> fp32
-// D = A B (accumulate 0) or A B + D / 2^DOWN
-template <int DOWN>
-__device__ __forceinline__ void ft_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t accumulate) {
-    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p, %5;\n}\n" ::"r"(d), "l"(a), "l"(b), "r"(FT_IDESC), "r"(accumulate),
-                 "n"(DOWN)
-                 : "memory");
+__device__ __forceinline__ bool ft_elect() {
+    uint32_t one;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
+    return one != 0u;
 }
+// on the barrier at this offset in both CTAs, once the MMAs issued so far have completed
 __device__ __forceinline__ void ft_commit(uint64_t* b) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(ft_smem(b)) : "memory");
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(ft_smem(b)), "h"((uint16_t)3) : "memory");
 }
 __device__ __forceinline__ void ft_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void ft_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void ft_ld16(uint32_t addr, float (&v)[16]) {
+__device__ __forceinline__ void ft_ld16(uint32_t addr, float (&v)[16]) {  // (ft_wait_ld before the numbers are used)
     uint32_t* u = reinterpret_cast<uint32_t*>(v);
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
                  : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]), "=r"(u[8]), "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]),
                    "=r"(u[13]), "=r"(u[14]), "=r"(u[15])
                  : "r"(addr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
+template <int R>
+__device__ __forceinline__ void ft_more_regs() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R)); }
+template <int R>
+__device__ __forceinline__ void ft_fewer_regs() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R)); }
+__device__ __forceinline__ void ft_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 // two numbers to the nearest bf16, and back
 __device__ __forceinline__ uint32_t ft_pack(float x, float y) {
     uint32_t r;
@@ -92,26 +123,43 @@ __device__ __forceinline__ uint64_t ft_fma2(uint64_t v, float f, uint64_t add) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(v), "l"(ft_two(f, f)), "l"(add));
     return r;
 }
-__device__ __forceinline__ float ft_ld_cluster(uint32_t addr, uint32_t rank) {
-    uint32_t remote;
-    float v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
-    return v;
+// four numbers as three times four bf16 parts; every subtraction is exact; 256 x first, so that both steps of a part are one instruction for two numbers
+__device__ __forceinline__ void ft_split4(const float4& v, uint2 (&part)[3]) {
+    const float f[4] = {v.x, v.y, v.z, v.w};
+    uint32_t p[3][2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const uint64_t v8 = ft_mul2(ft_two(f[2 * e], f[2 * e + 1]), 256.f);
+        const uint32_t h = ft_pack(f[2 * e], f[2 * e + 1]);
+        const uint64_t r1 = ft_fma2(ft_unpack(h), -256.f, v8);
+        const uint32_t m = ft_pack(ft_first(r1), ft_second(r1));
+        const uint64_t r2 = ft_fma2(ft_unpack(m), -256.f, ft_mul2(r1, 256.f));
+        p[0][e] = h;
+        p[1][e] = m;
+        p[2][e] = __byte_perm(__float_as_uint(ft_first(r2)), __float_as_uint(ft_second(r2)), 0x7632);  // at most 8 significant bits are left: exact
+    }
+#pragma unroll
+    for (int q = 0; q < 3; ++q) part[q] = make_uint2(p[q][0], p[q][1]);
+}
+// shared::cluster address of `p`'s offset in the cluster's first CTA
+__device__ __forceinline__ uint32_t ft_first_cta(const void* p) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(ft_smem(p)), "r"(0u));
+    return r;
 }
 __device__ __forceinline__ void ft_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// `share` rows of a tile from row `first` on (a multiple of 16, at most 128) with FMAs in the order of k, through shared memory (the stages: the parts are not needed
-// any more).  A thread takes four columns of every 16th row.  About the time the whole tile takes with FMAs, once per tile that holds an infinity or a NaN.
+// Up to 128 rows of x times a CTA's features with FMAs in the order of k, through shared memory (the stages: the parts are not needed any more).  A thread takes four
+// columns of every 16th row.  About the time the whole tile takes with FMAs, once per tile that holds an infinity or a NaN.
 template <bool VEC>
-__device__ __noinline__ void ft_fma_rows(const LinearArgs& a, const float* X, const float* W, float* sm, int m0, int n0, int first, int share, int rows, int cols) {
-    constexpr int KB = 64, XP = KB + 4, WP = FT_BN + 4;
-    float *xs = sm, *ws = sm + FT_BM * XP;  // [share][XP], [KB][WP]
-    static_assert((FT_BM * XP + KB * WP) * 4 <= 2 * FT_STAGE, "both blocks fit in the stages");
-    const int tid = threadIdx.x, c4 = (tid & 31) * 4, r0 = tid >> 5, nr = share / 16;
+__device__ __noinline__ void ft_fma_rows(const LinearArgs& a, const float* X, const float* W, float* sm, int m0, int n0, int rows, int cols) {
+    constexpr int KB = 64, XP = KB + 4, WP = FT_BN + 4, share = 128;
+    float *xs = sm, *ws = sm + share * XP;  // [share][XP], [KB][WP]
+    static_assert((share * XP + KB * WP) * 4 <= 2 * FT_STAGE, "both blocks fit in the stages");
+    const int tid = threadIdx.x, c4 = (tid & 31) * 4, r0 = tid >> 5, nr = (rows + 15) / 16;
     float acc[8][4];
 #pragma unroll
     for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
@@ -119,8 +167,8 @@ __device__ __noinline__ void ft_fma_rows(const LinearArgs& a, const float* X, co
         __syncthreads();
         for (int i = tid; i < (share + FT_BN) * (KB / 4); i += FT_THREADS) {
             const int r = i / (KB / 4), kc = (i % (KB / 4)) * 4, k = k0 + kc, n = r - share;
-            const bool is_x = r < share, ok = is_x ? first + r < rows : n < cols;
-            const float* src = is_x ? X + (size_t)(first + r) * a.x_pitch() + k : W + (size_t)n * a.K + k;
+            const bool is_x = r < share, ok = is_x ? r < rows : n < cols;
+            const float* src = is_x ? X + (size_t)r * a.x_pitch() + k : W + (size_t)n * a.K + k;
             float v[4];
             if (VEC) {
                 const float4 u = ok && k < a.K ? *reinterpret_cast<const float4*>(src) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -149,7 +197,7 @@ __device__ __noinline__ void ft_fma_rows(const LinearArgs& a, const float* X, co
     if (tid >= 512) return;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        const int r = first + r0 + 16 * i;
+        const int r = r0 + 16 * i;
         if (i >= nr || r >= rows) continue;
 #pragma unroll
         for (int j = 0; j < 4; j += 2)
@@ -157,211 +205,507 @@ __device__ __noinline__ void ft_fma_rows(const LinearArgs& a, const float* X, co
     }
 }
 
+// x [M, K] fp32 -> three bf16 part matrices [3][M][kp], kp = K rounded up to 8 (the columns past K are zero).  Bound by memory: 10 bytes an element.
+constexpr int FP_THREADS = 256;
 template <bool VEC>
-__global__ void __launch_bounds__(FT_THREADS, 1) linear_f32_parts(LinearArgs a, int splits) {
-    extern __shared__ __align__(1024) unsigned char ft_raw[];
-    unsigned char* const sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(ft_raw) + 1023) & ~(uintptr_t)1023);
-    __shared__ uint64_t full[2], done[2];
-    __shared__ uint32_t tmem_slot;
-    __shared__ int flags;  // 1: a sum that is not finite; 2: a wait that ended without its event
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // row tiles fastest: the CTAs that share a tile of W run together
-    const int tiles_m = (a.M + FT_BM - 1) / FT_BM, tile = blockIdx.x / splits, rank = blockIdx.x % splits;
-    const int n0 = tile / tiles_m * FT_BN, m0 = tile % tiles_m * FT_BM;
-    const float* X = static_cast<const float*>(a.x) + (size_t)m0 * a.x_pitch();
-    const float* W = static_cast<const float*>(a.w) + (size_t)n0 * a.K;
-    const int rows = min(FT_BM, a.M - m0), cols = min(FT_BN, a.N - n0);
-    const int nkb = (a.K + FT_BK - 1) / FT_BK, kb0 = (int)((long long)nkb * rank / splits), kb1 = (int)((long long)nkb * (rank + 1) / splits);
-
-    if (tid == 0) {
-        for (int i = 0; i < 2; ++i) { ft_bar_init(&full[i], FT_WARPS); ft_bar_init(&done[i], 1); }
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        flags = 0;
-    }
-    if (warp == FT_WARPS) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(ft_smem(&tmem_slot)), "r"(256u) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    // rows of x and W past the end stay zero in both stages
-    for (int i = tid; i < 2 * FT_STAGE / 16; i += FT_THREADS) {
-        const int r = (i % (FT_TILE / 16)) / 8, part = (i / (FT_TILE / 16)) % 6;
-        if (r >= (part < 3 ? rows : cols)) reinterpret_cast<uint4*>(sm)[i] = make_uint4(0, 0, 0, 0);
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    ft_fence_before();
-    __syncthreads();
-    ft_fence_after();
-    const uint32_t tmem = tmem_slot;
-    constexpr int NF = FT_BM * FT_BK / 4 / (32 * FT_WARPS), RS = FT_BM / NF, NC = FT_BN / (FT_WARPS / 4);  // float4s and row step of a worker, its columns of the sums
-    float acc[NC];
-    int strange = 0;  // a sum that is not finite
-    if (warp < FT_WARPS) {
-        // float4 i of this thread: row (i * RS + tid / 16), columns 4 (tid % 16) .. of the k-block
-        const int r0 = tid >> 4, c4 = (tid & 15) * 4;
-        float4 px[NF], pw[NF];
-        auto fetch = [&](int kb) {
-            const int k = kb * FT_BK + c4;
+__global__ void __launch_bounds__(FP_THREADS) f32_parts_kernel(const float* x, int ldx, int M, int K, int kp, bf16* parts, unsigned* counters, int n_counters) {
+    pdl_trigger();
+    pdl_wait();
+    if (blockIdx.x == 0)
+        for (int i = threadIdx.x; i < n_counters; i += FP_THREADS) counters[i] = 0u;
+    const int64_t per_row = kp / 8, total = (int64_t)M * per_row;
+    for (int64_t i = (int64_t)blockIdx.x * FP_THREADS + threadIdx.x; i < total; i += (int64_t)gridDim.x * FP_THREADS) {
+        const int m = (int)(i / per_row), k = (int)(i % per_row) * 8;
+        const float* src = x + (size_t)m * ldx + k;
+        float v[8];
+        if (VEC && k + 8 <= K) {
+            load4(src, v);
+            load4(src + 4, v + 4);
+        } else {
 #pragma unroll
-            for (int i = 0; i < NF; ++i) {
-                const int r = r0 + RS * i;
-                px[i] = pw[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-                const float *xp = X + (size_t)r * a.x_pitch() + k, *wp = W + (size_t)r * a.K + k;
-                if (VEC) {
-                    if (k < a.K) {
-                        if (r < rows) px[i] = *reinterpret_cast<const float4*>(xp);
-                        if (r < cols) pw[i] = __ldg(reinterpret_cast<const float4*>(wp));
-                    }
-                } else {
-                    float *x = reinterpret_cast<float*>(&px[i]), *w = reinterpret_cast<float*>(&pw[i]);
-#pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                        if (k + e < a.K) {
-                            if (r < rows) x[e] = xp[e];
-                            if (r < cols) w[e] = wp[e];
-                        }
-                }
-            }
-        };
-        auto put = [&](unsigned char* tile, int r, const float4& v) {
-            const float* f = reinterpret_cast<const float*>(&v);
-            uint32_t part[3][2];
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                // every subtraction is exact; 256 x first, so that both steps of a part are one instruction for two numbers
-                const uint64_t v8 = ft_mul2(ft_two(f[2 * e], f[2 * e + 1]), 256.f);
-                const uint32_t h = ft_pack(f[2 * e], f[2 * e + 1]);
-                const uint64_t r1 = ft_fma2(ft_unpack(h), -256.f, v8);
-                const uint32_t m = ft_pack(ft_first(r1), ft_second(r1));
-                const uint64_t r2 = ft_fma2(ft_unpack(m), -256.f, ft_mul2(r1, 256.f));
-                part[0][e] = h;
-                part[1][e] = m;
-                part[2][e] = __byte_perm(__float_as_uint(ft_first(r2)), __float_as_uint(ft_second(r2)), 0x7632);  // at most 8 significant bits are left: exact
-            }
-            unsigned char* at = tile + r * 128 + (((c4 * 2) ^ ((r & 7) << 4)) & 0x7f);  // 16-byte units XORed with the row
-#pragma unroll
-            for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(at + q * FT_TILE) = make_uint2(part[q][0], part[q][1]);
-        };
-#pragma unroll
-        for (int j = 0; j < NC; ++j) acc[j] = 0.f;
-        const uint32_t mine = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (warp >> 2) * NC;
-        bool alive = true;
-        auto promote = [&](int it) {
-            if (alive && !ft_bar_wait(&done[it & 1], (it >> 1) & 1)) { alive = false; atomicOr(&flags, 2); }
-            __syncwarp();
-            ft_fence_after();
-            float v[16];  // (32 at once spill beside the operands in flight)
-#pragma unroll
-            for (int c = 0; c < NC / 16; ++c) {
-                ft_ld16(mine + (it & 1) * 128 + c * 16, v);
-#pragma unroll
-                for (int j = 0; j < 16; ++j) acc[c * 16 + j] += v[j];
-            }
-            ft_fence_before();
-        };
-        if (kb0 < kb1) fetch(kb0);
-        // Block it may overwrite stage it & 1 and accumulator it & 1 once block it - 2 has been added up: promote() of it - 2 waited for its
-        // MMAs, and every warp arrives on full[] after that.
-        for (int it = 0; it < kb1 - kb0; ++it) {
-            unsigned char* st = sm + (it & 1) * FT_STAGE;
-#pragma unroll
-            for (int i = 0; i < NF; ++i) {
-                const int r = r0 + RS * i;
-                if (r < rows) put(st, r, px[i]);
-                if (r < cols) put(st + 3 * FT_TILE, r, pw[i]);
-            }
-            if (kb0 + it + 1 < kb1) fetch(kb0 + it + 1);
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) ft_bar_arrive(&full[it & 1]);
-            if (it > 0) promote(it - 1);
+            for (int e = 0; e < 8; ++e) v[e] = k + e < K ? src[e] : 0.f;
         }
-        if (kb0 < kb1) promote(kb1 - kb0 - 1);
-        // an operand that is not finite makes a part that is NaN (inf - inf), so every sum it enters is NaN: found here, once
+        uint2 lo[3], hi[3];
+        ft_split4(make_float4(v[0], v[1], v[2], v[3]), lo);
+        ft_split4(make_float4(v[4], v[5], v[6], v[7]), hi);
 #pragma unroll
-        for (int j = 0; j < NC; ++j) strange |= not_finite(acc[j]);
-        if (strange) atomicOr(&flags, 1);
-    } else if (lane == 0) {
-        bool alive = true;
-        for (int it = 0; it < kb1 - kb0; ++it) {
-            if (alive && !ft_bar_wait(&full[it & 1], (it >> 1) & 1)) { alive = false; atomicOr(&flags, 2); }
-            ft_fence_after();
-            const uint32_t base = ft_smem(sm + (it & 1) * FT_STAGE), d = tmem + (it & 1) * 128;
-            // (x part, W part), the small products first: 0 hi, 1 mid, 2 lo
-            constexpr int PX[6] = {1, 0, 2, 0, 1, 0}, PW[6] = {1, 2, 0, 1, 0, 0};
-#pragma unroll
-            for (int p = 0; p < 6; ++p)
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const uint64_t xd = ft_desc(base + PX[p] * FT_TILE) + (uint64_t)(2 * k), wd = ft_desc(base + (3 + PW[p]) * FT_TILE) + (uint64_t)(2 * k);
-                    if (k == 0 && (p == 3 || p == 5)) ft_mma<8>(d, xd, wd, 1u);  // the scale of the parts changes: 2^16, 2^8, 1
-                    else ft_mma<0>(d, xd, wd, (p | k) ? 1u : 0u);
-                }
-            ft_commit(&done[it & 1]);
-        }
+        for (int q = 0; q < 3; ++q) *reinterpret_cast<uint4*>(parts + ((size_t)q * M + m) * kp + k) = make_uint4(lo[q].x, lo[q].y, hi[q].x, hi[q].y);
     }
-    ft_fence_before();
-    __syncthreads();  // every MMA has completed (the last promote waited for it): the stages are free
-    ft_fence_after();
-    float(*sum)[FT_LD] = reinterpret_cast<float(*)[FT_LD]>(sm);
-    if (warp < FT_WARPS) {
-        const int r = (warp & 3) * 32 + lane, c = (warp >> 2) * NC;
-#pragma unroll
-        for (int j = 0; j < NC; j += 4) *reinterpret_cast<float4*>(&sum[r][c + j]) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
-    }
-    if (warp == FT_WARPS) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u));
-    int mark = 0;
-    if (splits > 1) {
-        ft_cluster_sync();
-        for (int s = 0; s < splits; ++s) mark |= __float_as_int(ft_ld_cluster(ft_smem(&flags), s));
-    } else {
-        __syncthreads();
-        mark = flags;
-    }
-    // this CTA's share of the tile's rows: sums over the ranks in order, then the step that follows the Linear, a pair of columns per thread
-    const int share = FT_BM / splits, first = rank * share;
-    if (mark == 1) {
-        ft_fma_rows<VEC>(a, X, W, reinterpret_cast<float*>(sm), m0, n0, first, share, rows, cols);
-    } else {
-        for (int i = tid; i < share * (FT_BN / 2); i += FT_THREADS) {
-            const int r = first + i / (FT_BN / 2), c = (i % (FT_BN / 2)) * 2;
-            if (r >= rows || c >= cols) continue;
-            float v0 = 0.f, v1 = 0.f;
-            if (mark & 2) {
-                v0 = v1 = __int_as_float(0x7fffffff);
-            } else if (splits > 1) {
-                for (int s = 0; s < splits; ++s) { v0 += ft_ld_cluster(ft_smem(&sum[r][c]), s); v1 += ft_ld_cluster(ft_smem(&sum[r][c + 1]), s); }
-            } else {
-                const float2 v = *reinterpret_cast<const float2*>(&sum[r][c]);
-                v0 = v.x; v1 = v.y;
-            }
-            epilogue_pair<float>(a, m0 + r, n0 + c, v0, v1, n0 + c + 1 < a.N);
-        }
-    }
-    if (splits > 1) ft_cluster_sync();  // nobody leaves while its sums are being read
 }
 
-inline cudaError_t launch_linear_f32_parts(const LinearArgs& a, cudaStream_t st) {
-    const int tiles_n = (a.N + FT_BN - 1) / FT_BN, tiles_m = (a.M + FT_BM - 1) / FT_BM, nkb = (a.K + FT_BK - 1) / FT_BK;
-    // split k until the CTAs fill the chip (148 SMs, one CTA each), at least four k-blocks a part
-    int splits = 1;
-    while (splits < 8 && (long long)tiles_n * tiles_m * splits * 2 <= 160 && nkb >= 8 * splits) splits *= 2;
-    const bool vec = a.K % 4 == 0 && a.x_pitch() % 4 == 0 && (reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.w)) % 16 == 0;
-    auto kernel = vec ? linear_f32_parts<true> : linear_f32_parts<false>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FT_SMEM);
+// How a Linear is dealt: tiles of 256 features x w tokens, token tiles fastest; items [0, whole) are tiles, the others parts of the tiles of the last round.
+struct F32Plan {
+    int w, tok_tiles, clusters, whole, cut, items;
+};
+inline F32Plan f32_plan(int M, int N, int K, int units) {
+    const int nkb = (K + FT_BK - 1) / FT_BK, n_tiles = (N + 2 * FT_BN - 1) / (2 * FT_BN), least = (M + FT_MAX_W - 1) / FT_MAX_W;
+    F32Plan best = {};
+    double best_cost = 0;
+    // A round costs 256 + w clocks a k-block and product.  More and narrower token tiles than needed pay where they fill a round better.
+    for (int tt = least; tt <= least + 5; ++tt) {
+        F32Plan p;
+        p.tok_tiles = tt;
+        p.w = ((M + tt - 1) / tt + 15) / 16 * 16;
+        if (tt > least && (p.w < 128 || (long long)(tt - 1) * p.w >= M)) break;  // (narrow tiles cost little less; a tile without tokens)
+        const long long tiles = (long long)tt * n_tiles;
+        const int rest = (int)(tiles % units);
+        int cut = rest ? units / rest : 1;
+        if (cut > 8) cut = 8;
+        while (cut > 1 && nkb < 2 * cut) --cut;
+        p.cut = cut;
+        p.whole = (int)(cut > 1 ? tiles - rest : tiles);
+        p.items = (int)(p.whole + (tiles - p.whole) * cut);
+        p.clusters = p.items < units ? p.items : units;
+        const double rounds = (double)(tiles / units) + (rest ? 1.0 / cut : 0.0), cost = rounds * (256 + p.w) * (1 + (rest ? 0.03 * cut : 0.0));
+        if (tt == least || cost < best_cost) best = p, best_cost = cost;
+    }
+    return best;
+}
+
+// A tile's sums go where the Linear's result goes, straight from the registers, if nothing but a bias follows; else, and for parts of cut tiles, to a slot of
+// [w tokens][128 features], and f32_combine_kernel takes them from there.  (With the residual add from the registers, whose loads stand in the open, 804 x 16384 x 2048 took 314 us
+// instead of 236.)
+enum { FT_TO_SLOTS = 0, FT_TO_OUT = 1 };
+inline int f32_step_of(const LinearArgs& a) {
+    return (a.epi == EPI_STORE && a.n_act <= 0) || (a.epi == EPI_F32 && a.limit <= 0.f && a.alpha == 0.f) ? FT_TO_OUT : FT_TO_SLOTS;
+}
+struct F32Args {
+    LinearArgs a;
+    F32Plan p;
+    int slot0;           // the first item that has slots (0, or p.whole)
+    float* slots;        // [items - slot0][2 CTAs][w][128]
+    unsigned* counters;  // [2 * tiles from slot0 on], zero: parts that are there, 2^16 for each that holds a number that is not finite
+};
+
+// The step after the Linear for the tiles whose sums (or parts of them, added in the order of k) lie in slots: four features of two tokens a thread.  Bound by memory.  A launch of its
+// own spreads the parts of cut tiles over the chip (added by the cluster that arrives last, 804 x 2048 x 2048 took 70 us instead of 49), and keeps the steps' code away from the registers of
+// the kernel before (with it inside, unrolled over a thread's tokens, 804 x 16384 x 2048 took 507 us).
+constexpr int FC_THREADS = 256, FC_TOKENS = 16;
+__global__ void __launch_bounds__(FC_THREADS) f32_combine_kernel(const __grid_constant__ F32Args args) {
+    pdl_trigger();
+    pdl_wait();
+    const LinearArgs& a = args.a;
+    const F32Plan& p = args.p;
+    const int blocks = (p.w + FC_TOKENS - 1) / FC_TOKENS, half = blockIdx.x / blocks, rank = half & 1, nth = half >> 1, tile = args.slot0 + nth;
+    if (args.counters[half] >> 16) return;  // computed again
+    const int parts = tile < p.whole ? 1 : p.cut, item = tile < p.whole ? tile : p.whole + (tile - p.whole) * p.cut;
+    const int t0 = tile % p.tok_tiles * p.w, n = (tile / p.tok_tiles * 2 + rank) * FT_BN + (threadIdx.x & 31) * 4, t = blockIdx.x % blocks * FC_TOKENS + (threadIdx.x >> 5);
+    if (n >= a.N) return;
+    const size_t slot = (size_t)p.w * FT_BN;
+    const float* src = args.slots + ((size_t)(item - args.slot0) * 2 + rank) * slot + (threadIdx.x & 31) * 4;
+    constexpr int U = FC_TOKENS * 32 / FC_THREADS;
+    float4 v[U];
+    const int end = min(p.w, a.M - t0);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+        if (t + u * (FC_THREADS / 32) < end) v[u] = __ldcg(reinterpret_cast<const float4*>(src + (size_t)(t + u * (FC_THREADS / 32)) * FT_BN));
+#pragma unroll 2
+    for (int s = 1; s < parts; ++s)
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (t + u * (FC_THREADS / 32) < end) {
+                const float4 x = __ldcg(reinterpret_cast<const float4*>(src + 2 * s * slot + (size_t)(t + u * (FC_THREADS / 32)) * FT_BN));
+                v[u].x += x.x, v[u].y += x.y, v[u].z += x.z, v[u].w += x.w;
+            }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int m = t0 + t + u * (FC_THREADS / 32);
+        if (t + u * (FC_THREADS / 32) >= end) continue;
+        epilogue_pair<float>(a, m, n, v[u].x, v[u].y, n + 1 < a.N);
+        if (n + 2 < a.N) epilogue_pair<float>(a, m, n + 2, v[u].z, v[u].w, n + 3 < a.N);
+    }
+}
+
+template <bool VEC>
+__global__ void __launch_bounds__(FT_THREADS, 1) linear_f32_pair(const __grid_constant__ CUtensorMap parts, const __grid_constant__ F32Args args) {
+    extern __shared__ __align__(1024) unsigned char ft_raw[];
+    unsigned char* const sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(ft_raw) + 1023) & ~(uintptr_t)1023);
+    __shared__ uint64_t full[2], done[2], taken[2];  // a stage is there; its MMAs have completed; their sums have been added (full and taken: the first CTA's)
+    __shared__ uint32_t tmem_slot;
+    __shared__ unsigned redo[FT_REDO_WORDS];
+    const LinearArgs& a = args.a;
+    const F32Plan& p = args.p;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int rank = blockIdx.x & 1, cluster = blockIdx.x >> 1;
+    const int nkb = (a.K + FT_BK - 1) / FT_BK;
+    const float* const W = static_cast<const float*>(a.w);
+    struct Item { int t0, n0, kb0, kb1, part; };  // first token, this CTA's first feature, k-blocks, part of a cut tile (-1: whole)
+    auto item_of = [&](int i) {
+        Item it;
+        int tile = i;
+        it.part = -1, it.kb0 = 0, it.kb1 = nkb;
+        if (i >= p.whole) {
+            tile = p.whole + (i - p.whole) / p.cut;
+            it.part = (i - p.whole) % p.cut;
+            it.kb0 = (int)((long long)nkb * it.part / p.cut);
+            it.kb1 = (int)((long long)nkb * (it.part + 1) / p.cut);
+        }
+        it.t0 = tile % p.tok_tiles * p.w;
+        it.n0 = (tile / p.tok_tiles * 2 + rank) * FT_BN;
+        return it;
+    };
+
+    if (tid == 0) {
+        for (int i = 0; i < 2; ++i) { ft_bar_init(&full[i], 2 * FT_SPLIT_WARPS + 1); ft_bar_init(&done[i], 1); ft_bar_init(&taken[i], 2 * FT_SUM_WARPS); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&parts) : "memory");
+    }
+    for (int i = tid; i < FT_REDO_WORDS; i += FT_THREADS) redo[i] = 0u;
+    if (warp == FT_SPLIT_WARPS + FT_SUM_WARPS + 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(ft_smem(&tmem_slot)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    ft_fence_before();
+    ft_cluster_sync();  // the other CTA's barriers are there before any copy or commit reaches them
+    ft_fence_after();
+    const uint32_t tmem = tmem_slot;
+    pdl_trigger();
+    if (warp < FT_SPLIT_WARPS) {
+        ft_fewer_regs<FT_SPLIT_REGS>();
+        constexpr int NF = FT_BN * FT_BK / 4 / (32 * FT_SPLIT_WARPS), RS = FT_BN / NF;  // float4s of a thread a k-block, and their row step
+        static_assert(RS % 8 == 0, "a thread's rows lie at the same place of the swizzle");
+        // float4 i of this thread: row (i * RS + tid / 16), columns 4 (tid % 16) .. of the k-block; the next block's are in flight while this one is split
+        const int r0 = tid >> 4, c4 = (tid & 15) * 4;
+        const size_t step = (size_t)RS * a.K;
+        float4 v[NF];
+        int item = cluster, kb = 0, cols = 0;
+        Item c = {};
+        const float* src = nullptr;
+        auto start = [&]() {  // the rows of `item`
+            if (item >= p.items) return;
+            c = item_of(item);
+            kb = c.kb0;
+            cols = a.N - c.n0 - r0;
+            src = W + (size_t)(c.n0 + r0) * a.K + c4;
+#pragma unroll
+            for (int i = 0; i < NF; ++i) v[i] = make_float4(0.f, 0.f, 0.f, 0.f);  // rows past N stay zero
+        };
+        auto fetch = [&]() {
+            const int k = kb * FT_BK;
+#pragma unroll
+            for (int i = 0; i < NF; ++i) {
+                if (VEC) {
+                    if (RS * i < cols) v[i] = __ldg(reinterpret_cast<const float4*>(src + i * step + k));
+                } else {
+                    float* w = reinterpret_cast<float*>(&v[i]);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) w[e] = RS * i < cols && k + c4 + e < a.K ? src[i * step + k + e] : 0.f;
+                }
+            }
+        };
+        auto fetch_vec_tail = [&]() {  // a block that runs past K, by whole float4s
+            const bool in = kb * FT_BK + c4 < a.K;
+#pragma unroll
+            for (int i = 0; i < NF; ++i) {
+                v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (in && RS * i < cols) v[i] = __ldg(reinterpret_cast<const float4*>(src + i * step + kb * FT_BK));
+            }
+        };
+        auto next = [&]() {
+            if (item >= p.items) return;
+            if (VEC && (kb + 1) * FT_BK > a.K) fetch_vec_tail();
+            else fetch();
+            if (++kb == c.kb1) item += p.clusters, kb = -1;
+        };
+        start();
+        next();
+        const uint32_t full_at[2] = {ft_first_cta(&full[0]), ft_first_cta(&full[1])};
+        unsigned char* const at = sm + r0 * 128 + (((c4 * 2) ^ ((r0 & 7) << 4)) & 0x7f);  // 16-byte units XORed with the row
+        int total = 0;
+        for (int i = cluster; i < p.items; i += p.clusters) {
+            const Item t = item_of(i);
+            total += t.kb1 - t.kb0;
+        }
+        bool alive = true;
+        for (int it = 0; it < total; ++it) {
+            if (it >= 2 && alive && !ft_bar_wait(&done[it & 1], ((it >> 1) - 1) & 1)) alive = false;
+            unsigned char* st = at + (it & 1) * FT_STAGE;
+#pragma unroll
+            for (int i = 0; i < NF; ++i) {
+                uint2 part[3];
+                ft_split4(v[i], part);
+#pragma unroll
+                for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(st + q * FT_TILE + i * RS * 128) = part[q];
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) ft_bar_arrive(full_at[it & 1]);
+            if (kb < 0) start();
+            next();  // (behind the arrival, which would wait for the loads)
+        }
+        __syncwarp();
+        ft_more_regs<FT_REGS>();
+    } else if (warp < FT_SPLIT_WARPS + FT_SUM_WARPS) {
+        ft_more_regs<FT_SUM_REGS>();
+        pdl_wait();
+        // this warp's sums: features 32 (warp % 4) .., tokens in blocks of 16, every second block
+        constexpr int THREADS = 32 * FT_SUM_WARPS;
+        const int etid = tid - 32 * FT_SPLIT_WARPS, g = (warp - FT_SPLIT_WARPS) >> 2, row = (warp & 3) * 32 + lane, n_ch = p.w / 16;
+        const uint32_t mine = tmem + ((uint32_t)((warp & 3) * 32) << 16) + g * 16;
+        const uint32_t taken_at[2] = {ft_first_cta(&taken[0]), ft_first_cta(&taken[1])};
+        float acc[FT_CHUNKS][16];
+        bool alive = true;
+        int it = 0, ord = 0;
+        for (int i = cluster; i < p.items; i += p.clusters, ++ord) {
+            const Item c = item_of(i);
+#pragma unroll
+            for (int q = 0; q < FT_CHUNKS; ++q)
+#pragma unroll
+                for (int j = 0; j < 16; ++j) acc[q][j] = 0.f;
+            for (int kb = c.kb0; kb < c.kb1; ++kb, ++it) {
+                if (alive && !ft_bar_wait(&done[it & 1], (it >> 1) & 1)) alive = false;
+                __syncwarp();
+                ft_fence_after();
+                const uint32_t from = mine + (it & 1) * 256;
+                // two blocks a round trip (300 clocks each)
+#pragma unroll
+                for (int q = 0; q < FT_CHUNKS; q += 2) {
+                    if (g + 2 * q >= n_ch) break;
+                    float u[16], v[16];
+                    const bool two = q + 1 < FT_CHUNKS && g + 2 * q + 2 < n_ch;
+                    ft_ld16(from + q * 32, u);
+                    if (two) ft_ld16(from + q * 32 + 32, v);
+                    ft_wait_ld();
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) acc[q][j] += u[j];
+                    if (q + 1 < FT_CHUNKS && two)
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) acc[q + 1 < FT_CHUNKS ? q + 1 : q][j] += v[j];
+                }
+                ft_fence_before();
+                __syncwarp();
+                if (lane == 0) ft_bar_arrive(taken_at[it & 1]);
+            }
+            // The tile's sums.  An operand that is not finite makes a part that is NaN (inf - inf), so every sum it enters is NaN: found here, once.
+            int strange = 0;
+#pragma unroll
+            for (int q = 0; q < FT_CHUNKS; ++q)
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    strange |= not_finite(acc[q][j]);
+                    if (!alive) acc[q][j] = __int_as_float(0x7fffffff);
+                }
+            if (!alive) strange = 0;
+            asm volatile("{\n.reg .pred p, q;\nsetp.ne.b32 p, %0, 0;\nbarrier.cta.red.or.pred q, 1, %1, p;\nselp.b32 %0, 1, 0, q;\n}\n" : "+r"(strange) : "n"(THREADS) : "memory");
+            const bool slotted = i >= args.slot0;
+            if (strange && (!slotted || c.part < 0)) {  // computed again at the end
+                if (etid == 0) {
+                    redo[ord >> 5] |= 1u << (ord & 31);
+                    if (slotted) args.counters[2 * (i - args.slot0) + rank] = 0x10001u;
+                }
+                continue;
+            }
+            if (slotted) {
+                float* const slot = args.slots + ((size_t)(i - args.slot0) * 2 + rank) * p.w * FT_BN + row;
+#pragma unroll
+                for (int q = 0; q < FT_CHUNKS; ++q)
+                    if (g + 2 * q < n_ch)
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) slot[((g + 2 * q) * 16 + j) * FT_BN] = acc[q][j];
+                if (c.part >= 0 && etid == 0) {  // of a cut tile with a number that is not finite the last part to arrive computes the tile again
+                    const unsigned before = atomicAdd(args.counters + 2 * (p.whole - args.slot0 + (i - p.whole) / p.cut) + rank, strange ? 0x10001u : 1u);
+                    if ((before & 0xffffu) + 1u == (unsigned)p.cut && (strange || before >> 16)) redo[ord >> 5] |= 1u << (ord & 31);
+                }
+                continue;
+            }
+            const int n = c.n0 + row;
+            const float bias = a.bias && n < a.N ? static_cast<const float*>(a.bias)[n] : 0.f;
+            float* const to = (a.epi == EPI_STORE ? static_cast<float*>(a.out) : a.out32) + n;
+#pragma unroll
+            for (int q = 0; q < FT_CHUNKS; ++q) {
+                const int t = c.t0 + (g + 2 * q) * 16;
+                if (g + 2 * q >= n_ch || n >= a.N) continue;
+#pragma unroll
+                for (int j = 0; j < 16; ++j)
+                    if (t + j < a.M) to[(size_t)(t + j) * a.N] = acc[q][j] + bias;
+            }
+        }
+        __syncwarp();
+        ft_fewer_regs<FT_REGS>();
+    } else {
+        ft_fewer_regs<FT_REST_REGS>();
+        if (warp == FT_SPLIT_WARPS + FT_SUM_WARPS && lane == 0) {
+            pdl_wait();
+            const int half = p.w / 2;
+            bool alive = true;
+            int it = 0;
+            for (int i = cluster; i < p.items; i += p.clusters) {
+                const Item c = item_of(i);
+                for (int kb = c.kb0; kb < c.kb1; ++kb, ++it) {
+                    if (it >= 2 && alive && !ft_bar_wait(&done[it & 1], ((it >> 1) - 1) & 1)) alive = false;
+                    if (!alive) continue;
+                    // the pair's copies count on the first CTA's barrier (the other CTA's may land before it is armed)
+                    if (rank == 0) ft_bar_expect(&full[it & 1], 2u * 3u * (uint32_t)half * 128u);
+                    asm volatile("cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(
+                                     ft_smem(sm + (it & 1) * FT_STAGE + 3 * FT_TILE)),
+                                 "l"(&parts), "r"(ft_first_cta(&full[it & 1])), "r"(kb * FT_BK), "r"(c.t0 + rank * half), "r"(0)
+                                 : "memory");
+                }
+            }
+        }
+        if (warp == FT_SPLIT_WARPS + FT_SUM_WARPS + 1 && rank == 0) {
+            // (the whole warp walks, one thread of it issues: so the operands are uniform.  In a thread's own registers the 24 instructions of a k-block took longer to
+            // issue than to run)
+            bool alive = true;
+            int it = 0;
+            const uint32_t idesc = FT_IDESC | (uint32_t)(p.w >> 3) << 17, x_part = (uint32_t)(p.w / 2) * 128u >> 4, first = ft_desc_lo(ft_smem(sm));
+            for (int i = cluster; i < p.items; i += p.clusters) {
+                const Item c = item_of(i);
+                for (int kb = c.kb0; kb < c.kb1; ++kb, ++it) {
+                    if (it >= 2 && alive && !ft_bar_wait(&taken[it & 1], ((it >> 1) - 1) & 1)) alive = false;
+                    if (alive && !ft_bar_wait(&full[it & 1], (it >> 1) & 1)) alive = false;
+                    if (!__all_sync(0xffffffffu, alive)) { alive = false; continue; }
+                    ft_fence_after();
+                    const uint32_t w0 = first + (it & 1) * (FT_STAGE >> 4), w1 = w0 + (FT_TILE >> 4), w2 = w1 + (FT_TILE >> 4), d = tmem + (it & 1) * 256;
+                    const uint32_t x0 = w2 + (FT_TILE >> 4), x1 = x0 + x_part, x2 = x1 + x_part;  // parts: 0 hi, 1 mid, 2 lo
+                    if (ft_elect()) {
+                        // the small products first; the scale of the parts changes twice: 2^16, 2^8, 1
+                        ft_mma<false, 0>(d, w1, x1, idesc);
+#pragma unroll
+                        for (int k = 2; k < 8; k += 2) ft_mma<true, 0>(d, w1 + k, x1 + k, idesc);
+#pragma unroll
+                        for (int k = 0; k < 8; k += 2) ft_mma<true, 0>(d, w2 + k, x0 + k, idesc);
+#pragma unroll
+                        for (int k = 0; k < 8; k += 2) ft_mma<true, 0>(d, w0 + k, x2 + k, idesc);
+                        ft_mma<true, 8>(d, w1, x0, idesc);
+#pragma unroll
+                        for (int k = 2; k < 8; k += 2) ft_mma<true, 0>(d, w1 + k, x0 + k, idesc);
+#pragma unroll
+                        for (int k = 0; k < 8; k += 2) ft_mma<true, 0>(d, w0 + k, x1 + k, idesc);
+                        ft_mma<true, 8>(d, w0, x0, idesc);
+#pragma unroll
+                        for (int k = 2; k < 8; k += 2) ft_mma<true, 0>(d, w0 + k, x0 + k, idesc);
+                        ft_commit(&done[it & 1]);
+                    }
+                    __syncwarp();
+                }
+            }
+        }
+        __syncwarp();
+        ft_more_regs<FT_REGS>();
+    }
+    ft_fence_before();
+    ft_cluster_sync();  // every MMA has completed, nothing reaches the other CTA any more: the stages are free
+    ft_fence_after();
+    if (warp == FT_SPLIT_WARPS + FT_SUM_WARPS + 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
+    for (int i = cluster, ord = 0; i < p.items; i += p.clusters, ++ord) {
+        if (!(redo[ord >> 5] >> (ord & 31) & 1u)) continue;
+        const Item c = item_of(i);
+        const int end = min(a.M, c.t0 + p.w);
+        for (int m = c.t0; m < end; m += 128)
+            ft_fma_rows<VEC>(a, static_cast<const float*>(a.x) + (size_t)m * a.x_pitch(), W + (size_t)c.n0 * a.K, reinterpret_cast<float*>(sm), m, c.n0, min(128, end - m),
+                             min(FT_BN, a.N - c.n0));
+    }
+}
+
+typedef CUresult (*FtEncode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                             CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+inline FtEncode ft_encode() {  // the driver's entry point through the runtime: no link against libcuda
+    static const FtEncode fn = [] {
+        void* ptr = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        return cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &found) == cudaSuccess && found == cudaDriverEntryPointSuccess ? reinterpret_cast<FtEncode>(ptr) : nullptr;
+    }();
+    return fn;
+}
+inline int ft_units() {  // pairs of SMs
+    int dev = 0, sms = 0;
+    return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms >= 2 ? sms / 2 : 1;
+}
+
+// scratch: counters, slots, the parts of x
+struct F32Scratch {
+    int64_t counters, slots, parts, bytes;
+    int kp;
+};
+inline F32Scratch f32_scratch(int M, int K, const F32Plan& p, int step) {
+    F32Scratch s;
+    const int64_t items = step == FT_TO_SLOTS ? p.items : p.items - p.whole;
+    s.kp = (K + 7) / 8 * 8;
+    s.counters = 2 * (step == FT_TO_SLOTS ? p.whole + (p.items - p.whole) / p.cut : (p.items - p.whole) / p.cut);
+    s.slots = (s.counters * 4 + 1023) / 1024 * 1024;
+    s.parts = s.slots + items * 2 * p.w * FT_BN * 4;
+    s.bytes = s.parts + 3 * (int64_t)M * s.kp * 2;
+    return s;
+}
+// of a Linear of M rows, whatever its step: launches of at most FT_MAX_TOKENS
+inline int64_t f32_scratch_bytes(int M, int N, int K, int step) {
+    const int m = M < FT_MAX_TOKENS ? M : FT_MAX_TOKENS, rest = M > m ? M % m : 0;
+    const int64_t bytes = f32_scratch(m, K, f32_plan(m, N, K, ft_units()), step).bytes, more = rest ? f32_scratch(rest, K, f32_plan(rest, N, K, ft_units()), step).bytes : 0;
+    return bytes > more ? bytes : more;
+}
+
+inline cudaError_t launch_f32_tokens(const LinearArgs& a, const F32Plan& p, int step, void* scratch, bool& taken, cudaStream_t st) {
+    const F32Scratch s = f32_scratch(a.M, a.K, p, step);
+    const F32Args args{a, p, step == FT_TO_SLOTS ? 0 : p.whole, reinterpret_cast<float*>(static_cast<char*>(scratch) + s.slots), static_cast<unsigned*>(scratch)};
+    bf16* const parts = reinterpret_cast<bf16*>(static_cast<char*>(scratch) + s.parts);
+    CUtensorMap map;
+    const cuuint64_t dims[3] = {(cuuint64_t)s.kp, (cuuint64_t)a.M, 3}, strides[2] = {(cuuint64_t)s.kp * 2, (cuuint64_t)a.M * s.kp * 2};
+    const cuuint32_t box[3] = {FT_BK, (cuuint32_t)p.w / 2, 3}, unit[3] = {1, 1, 1};
+    taken = ft_encode()(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, parts, dims, strides, box, unit, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    if (!taken) return cudaSuccess;
+    const auto aligned = [](const void* q) { return reinterpret_cast<uintptr_t>(q) % 16 == 0; };
+    const bool x_vec = a.x_pitch() % 4 == 0 && aligned(a.x), vec = x_vec && a.K % 4 == 0 && aligned(a.w);
+    const int64_t blocks = ((int64_t)a.M * (s.kp / 8) + FP_THREADS - 1) / FP_THREADS;
+    cudaError_t e = launch_pdl(x_vec ? f32_parts_kernel<true> : f32_parts_kernel<false>, dim3((unsigned)(blocks < 4096 ? blocks : 4096)), dim3(FP_THREADS), 0, st, static_cast<const float*>(a.x),
+                               a.x_pitch(), a.M, a.K, s.kp, parts, args.counters, (int)s.counters);
+    if (e) return e;
+    auto kernel = vec ? linear_f32_pair<true> : linear_f32_pair<false>;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FT_SMEM);
     if (e) return e;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)tiles_n * (unsigned)tiles_m * (unsigned)splits);
+    cfg.gridDim = dim3(2u * (unsigned)p.clusters);
     cfg.blockDim = dim3(FT_THREADS);
     cfg.dynamicSmemBytes = FT_SMEM;
     cfg.stream = st;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)splits;
+    at[0].val.clusterDim.x = 2;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, kernel, a, splits);
+    cfg.numAttrs = 2;
+    e = cudaLaunchKernelEx(&cfg, kernel, map, args);
+    if (!e && s.counters) e = launch_pdl(f32_combine_kernel, dim3((unsigned)s.counters * (unsigned)((p.w + FC_TOKENS - 1) / FC_TOKENS)), dim3(FC_THREADS), 0, st, args);
     return e ? e : cudaGetLastError();
+}
+
+// false: not for this kernel (no memory, more tiles a cluster than `redo` has bits): linear_tiled_fma takes it
+inline bool launch_linear_f32_pair(const LinearArgs& a, void* scratch, int64_t scratch_bytes, cudaStream_t st, cudaError_t& e) {
+    const int step = f32_step_of(a);
+    const int64_t need = f32_scratch_bytes(a.M, a.N, a.K, step);
+    {
+        const F32Plan p = f32_plan(a.M < FT_MAX_TOKENS ? a.M : FT_MAX_TOKENS, a.N, a.K, ft_units());
+        if (p.items / p.clusters >= 32 * FT_REDO_WORDS || !ft_encode()) return false;
+    }
+    if (!scratch || scratch_bytes < need || reinterpret_cast<uintptr_t>(scratch) % 16) {
+        void* own = nullptr;
+        if (cudaMallocAsync(&own, (size_t)need, st) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        const bool taken = launch_linear_f32_pair(a, own, need, st, e);
+        const cudaError_t f = cudaFreeAsync(own, st);
+        if (!e) e = f;
+        return taken;
+    }
+    for (int m = 0; m < a.M; m += FT_MAX_TOKENS) {  // (rows of everything that a row of x makes)
+        LinearArgs b = a;
+        b.M = a.M - m < FT_MAX_TOKENS ? a.M - m : FT_MAX_TOKENS;
+        b.ldx = a.x_pitch();
+        const bool half = a.epi == EPI_GLU || a.epi == EPI_SWIGLU || a.epi == EPI_GEGLU;
+        b.x = static_cast<const float*>(a.x) + (size_t)m * a.x_pitch();
+        if (a.out) b.out = static_cast<float*>(a.out) + (size_t)m * (half ? a.N / 2 : a.N);
+        if (a.out32) b.out32 = a.out32 + (size_t)m * a.N;
+        if (a.rowscale) b.rowscale = a.rowscale + (size_t)m * a.rs_pitch;
+        bool taken = false;
+        e = launch_f32_tokens(b, f32_plan(b.M, b.N, b.K, ft_units()), step, scratch, taken, st);
+        if (!taken) return false;  // (of the first rows: the map's sizes are the same for the others)
+        if (e) return true;
+    }
+    return true;
 }
 
 }  // namespace mbh

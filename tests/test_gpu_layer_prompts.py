@@ -697,3 +697,57 @@ def test_two_streams_of_linears_that_share_their_tiles(T, N, K):
                 got.append(h.linear(x, w, epi=h.EPI_F32))
     torch.cuda.synchronize()
     assert all(torch.equal(o, ref) for o in got)
+
+
+def _f32_step(h, kind, x, w, b, rs, base):
+    """(result, the same in float64) of one step after an fp32 Linear"""
+    N = w.shape[0]
+    y, F = x.double() @ w.double().T, torch.nn.functional
+    if kind == "store":
+        return h.linear(x, w, b, n_act=N // 2), torch.cat((F.silu((y + b.double())[:, : N // 2]), (y + b.double())[:, N // 2:]), 1)
+    if kind == "plain":
+        return h.linear(x, w, b), y + b.double()
+    if kind == "scaled add":
+        return h.linear(x, w, b, epi=h.EPI_RESIDUAL_SCALED, residual=base.clone(), alpha=0.3), base.double() + 0.3 * (y + b.double())
+    if kind == "logits":
+        return h.linear(x, w, None, epi=h.EPI_F32, limit=5.0, alpha=2.0), 2 * 5 * torch.tanh(y / 5)
+    if kind == "relu2":
+        return h.linear_relu2(x, w, rs, 8), y.clamp(min=0) ** 2 * rs.double().repeat_interleave(8, 1)[:, :N]
+    if kind == "decay":
+        a_log = torch.linspace(-1, 1, N // 2, device=DEV)
+        return h.linear_decay(x, w, b, a_log, 2), torch.exp(-torch.exp(a_log.double().repeat_interleave(2)) * F.softplus(y + b.double()))
+    g, u, r = y[:, 0::2], y[:, 1::2], rs.double().repeat_interleave(8, 1)[:, : N // 2]
+    if kind == "glu":
+        g, u = (g * r).clamp(max=2.0), (u * r).clamp(-2.0, 2.0)
+        return h.linear_glu(x, w, 2.0, 1.7, rs, 8), g * torch.sigmoid(1.7 * g) * (u + 1)
+    return h.linear_swiglu(x, w, rs, 8, gelu=kind == "geglu"), (F.gelu(g, approximate="tanh") if kind == "geglu" else F.silu(g)) * u * r
+
+
+@pytest.mark.parametrize("kind", ["store", "plain", "scaled add", "logits", "relu2", "decay", "glu", "swiglu", "geglu"])
+@pytest.mark.parametrize("M,N,K,pad", [(9, 256, 16, 0), (16, 258, 64, 4), (17, 130, 1030, 1), (224, 512, 72, 0), (225, 300, 132, 2), (449, 20480, 192, 0), (130, 2048, 1024, 0)])
+def test_fp32_linear_by_pairs(M, N, K, pad, kind):
+    """Token tiles of 16 to 224 and one more, weight tiles that end inside either CTA of a pair, k-blocks that end inside a float4 and rows of no whole float4s, tiles cut into parts, several
+    rounds, and every step behind: fp32 numbers, so 2^-24 of a result's scale, twice for a step's own rounding, and what the tensor core cuts off a sum (2^-23)."""
+    from mistral_inference_b200 import _abi_hybrid as h
+
+    g = torch.Generator().manual_seed(M + N + K)
+    rnd = lambda *s: torch.randn(*s, generator=g).to(DEV)  # noqa: E731
+    x, w, b, base = rnd(M, K + pad)[:, :K], rnd(N, K) / K ** 0.5, rnd(N), rnd(M, N)
+    if kind not in ("store", "plain", "scaled add", "logits"):
+        x = x.contiguous()
+    got, ref = _f32_step(h, kind, x, w, b, torch.rand(M, (N + 7) // 8, generator=g).to(DEV), base)
+    again, _ = _f32_step(h, kind, x, w, b, torch.rand(M, (N + 7) // 8, generator=torch.Generator().manual_seed(1)).to(DEV), base) if kind in ("plain", "store") else (got, None)
+    assert got.dtype == torch.float32 and rel(got, ref) < 2 ** -21 and torch.equal(got, again)
+
+
+def test_fp32_linear_of_more_rows_than_a_launch_takes():
+    """Rows in portions, each with what belongs to them; and the call that brings no memory of its own computes the same bits."""
+    from mistral_inference_b200 import _abi_hybrid as h
+
+    g = torch.Generator().manual_seed(1)
+    M, N, K = 2 * 4096 + 5, 40, 32
+    x, w, rs = torch.randn(M, K, generator=g).to(DEV), torch.randn(N, K, generator=g).to(DEV), torch.rand(M, 5, generator=g).to(DEV)
+    got, out = h.linear_relu2(x, w, rs, 8), torch.empty(M, N, device=DEV)
+    assert rel(got, (x.double() @ w.double().T).clamp(min=0) ** 2 * rs.double().repeat_interleave(8, 1)) < 2 ** -21
+    assert h.lib().mbh_linear_relu2(x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, rs.data_ptr(), 5, 8, 1, torch.cuda.current_stream().cuda_stream) == 0
+    assert torch.equal(out, got)
