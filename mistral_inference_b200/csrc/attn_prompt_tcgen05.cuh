@@ -207,8 +207,8 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
       }
     }
   } else if (warp == 1) {
-    // ================= MMA issuer =================
-    if (lane == 0) {
+    // ================= MMA issuer (one thread, elected by the warp) =================
+    {
       mbar_wait(q_full, 0, 22, 0);
       auto issue_s = [&](int u, int t) {  // S_u = Q_u K_t^T: 8 k-steps of 16 dims; dims 0..63 / 64..127 in two boxes 16 KB apart
         const int it = 2 * t, s = it % FA_SLOTS;
@@ -216,14 +216,17 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
           mbar_wait(&kv_full[s], (it / FA_SLOTS) & 1, 23, t);
           tc_fence_after();
         }
-        const uint32_t q_addr = smem_u32(sQ + u * FA_TILE_BYTES), k_addr = smem_u32(sKV + s * FA_TILE_BYTES);
+        const uint32_t q_desc = umma_desc_lo(smem_u32(sQ + u * FA_TILE_BYTES)), k_desc = umma_desc_lo(smem_u32(sKV + s * FA_TILE_BYTES));
+        if (elect_one()) {
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
-          const uint32_t off = (ks >> 2) * (FA_TILE_BYTES / 2) + (ks & 3) * 32;
-          umma_bf16(tmem + u * 128, umma_desc_sw128(q_addr + off), umma_desc_sw128(k_addr + off), kIdescQK, ks ? 1u : 0u);
+          for (int ks = 0; ks < 8; ++ks) {
+            const uint32_t off = ((ks >> 2) * (FA_TILE_BYTES / 2) + (ks & 3) * 32) >> 4;
+            umma_bf16(tmem + u * 128, q_desc + off, k_desc + off, kIdescQK, ks ? 1u : 0u);
+          }
+          umma_commit(&s_full[u]);
+          if (u == NU - 1) umma_commit(&kv_empty[s]);
         }
-        umma_commit(&s_full[u]);
-        if (u == NU - 1) umma_commit(&kv_empty[s]);
+        __syncwarp();
       };
 #pragma unroll
       for (int u = 0; u < NU; ++u) issue_s(u, 0);
@@ -235,12 +238,15 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
           mbar_wait(&p_full[u], t & 1, 24, t);  // the softmax warps have written P (and rescaled O)
           if (u == 0) mbar_wait(&kv_full[s], (it / FA_SLOTS) & 1, 25, t);
           tc_fence_after();
+          if (elect_one()) {
 #pragma unroll
-          for (int ks = 0; ks < 8; ++ks)  // 16 keys per step: P columns 8*ks (bf16 pairs), V rows 16*ks (128 B each)
-            umma_bf16_ts(tmem + FA_COL_O + u * 128, tmem + u * 128 + ks * 8, umma_desc_sw128_mn(v_addr + ks * 2048, FA_TILE_BYTES / 2), kIdescPV,
-                         (t | ks) ? 1u : 0u);
-          umma_commit(&pv_done[u]);
-          if (u == NU - 1) umma_commit(&kv_empty[s]);
+            for (int ks = 0; ks < 8; ++ks)  // 16 keys per step: P columns 8*ks (bf16 pairs), V rows 16*ks (128 B each)
+              umma_bf16_ts(tmem + FA_COL_O + u * 128, tmem + u * 128 + ks * 8, umma_desc_sw128_mn(v_addr + ks * 2048, FA_TILE_BYTES / 2), kIdescPV,
+                           (t | ks) ? 1u : 0u);
+            umma_commit(&pv_done[u]);
+            if (u == NU - 1) umma_commit(&kv_empty[s]);
+          }
+          __syncwarp();
           if (t + 1 < n_tiles) issue_s(u, t + 1);
         }
       }

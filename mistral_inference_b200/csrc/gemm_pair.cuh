@@ -7,8 +7,8 @@
 // The WEIGHTS are the MMA's 256 rows and the TOKENS its columns, because the number of columns of an MMA is free (any multiple of 32 up to 256) and that of its rows is not:
 // T tokens are dealt to ceil(T / 256) tiles whose widths differ by at most 32, and at most 31 columns of all are padding.  With the tokens as rows the last tile ran
 // as 256 rows whatever it held (an MMA of 128 rows over a pair takes as long): 1102 tokens cost 1280 rows, now 1120 columns; eight experts of ~512 rows
-// each cost 640 or 768, now what they have, to the next 32.  Time does not follow the columns alone: a k-block of a tile w wide takes about 256 + w clocks, of which
-// the 256 are the weight rows' way out of shared memory.  Five tiles for 1102 tokens: 480 clocks a k-block each instead of 512, and scoring them gained 4 %.
+// each cost 640 or 768, now what they have, to the next 32.  A k-block of a tile w wide takes 2 w clocks
+// and little more.  (256 + w, while one diverged lane issued the MMAs and the copies: see umma_bf16.)
 //
 // Accumulators therefore lie transposed in TMEM: lane = feature, column = token.  Epilogues work on pairs of features (exchange_pairs, epilogue.cuh); fp32 results
 // need not even that, a warp's 32 features of a token are one 128-byte line.  Shared memory stays out of it: the MMAs' operands and the copies take all of its
@@ -19,7 +19,11 @@
 //
 // A last round of tiles that is at most half full is cut along k (split_schedule.cuh); the parts' fp32 sums meet in the first part's epilogue, in the order of k.
 //
-// GROUPED: the mixtures' form, token tiles from the plan of moe.cuh (pair_expert, pair_info), weights by expert; nothing is cut.
+// GROUPED: the mixtures' form, token tiles from the plan of moe.cuh (pair_expert, pair_info), weights by expert; nothing is cut.  Token tiles there are 32 to 256 wide, and a tile's time
+// follows its width: clusters that take every n_cta-th tile drift apart by rounds, and the two or three that share an expert's weight tile no longer meet in L2 (2048 tokens, eight
+// experts of 4096 x 14336: 5.4 GB read from memory, 3.9 with the draw).  So a cluster takes the next tile that nobody has: the first CTA's producer draws it from a counter shortly before
+// it needs it and hands it to the warps of both CTAs (tile_full, tile_empty): 1545 us without, 1470 with.  Short tiles are dealt, their hand-over costs more (16 experts of 2048 x 1408,
+// 2500 tokens: 232 us dealt, 244 drawn); the line (GP_DRAW_MIN_K) lies between K = 2048 and 4096.
 #pragma once
 #include <type_traits>
 
@@ -30,7 +34,9 @@ namespace mb200 {
 constexpr int GP_ROWS = 256;                         // features a tile
 constexpr int GP_EPI_WARPS = 8, GP_THREADS = 64 + 32 * GP_EPI_WARPS;
 constexpr int GP_W_BYTES = TG_BM * TG_BK * 2;        // a CTA's half of the weight tile, per stage
-constexpr int GP_MAX_STAGES = 7, GP_SHAPES = 16, GP_INFO = 32;
+constexpr int GP_MAX_STAGES = 7, GP_SHAPES = 16, GP_INFO = 32, GP_DRAWN = 4;
+constexpr int GP_DRAW_MIN_K = 3072;
+constexpr int GP_DRAW_AHEAD = 24, GP_HAND_AHEAD = 14;  // k-blocks before a tile's last: the draw's way to memory and back, and the hand-over's to the other CTA, lie under copies
 static_assert(GP_SHAPES > GP_MAX_STAGES + 1, "see shape_s");
 template <int MODE>
 constexpr int kPairTurn = MODE == EPI_LOGPROB ? GP_EPI_WARPS * 2048 : 0;
@@ -75,6 +81,7 @@ struct PairParams {
   int units = 0;              // clusters on the chip
   float* partials = nullptr;  // [TG_MAX_CUTS][2 CTAs][256 / 4][128] float4: what the parts but the first leave for it; null: nothing is cut
   unsigned* flags = nullptr;  // [TG_MAX_CUTS * 2], zero between launches
+  unsigned* draw = nullptr;   // grouped: tiles drawn, zero between launches; null: tiles are dealt
 };
 
 // (a ring of a fixed number of fixed slots: with both in registers the loop that issues the MMAs took 4 % longer)
@@ -82,6 +89,41 @@ constexpr int GP_STAGE_BYTES = 2 * GP_W_BYTES;
 template <int MODE>
 constexpr int kPairStages = kPairRing<MODE> / GP_STAGE_BYTES;
 constexpr int GP_SMEM = 227 * 1024;
+
+// Waits for what the other CTA of the pair has written.
+__device__ __forceinline__ void mbar_wait_cluster(uint64_t* bar, uint32_t parity) {
+  uint32_t ok = 0, spins = 0;
+  do {
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    if (!ok && ++spins == MB200_WATCHDOG_SPINS) {
+      printf("[mb200 watchdog] block %d thread %d: no tile was handed out\n", (int)blockIdx.x, (int)threadIdx.x);
+      __trap();
+    }
+  } while (!ok);
+}
+// a tile's number into both CTAs' shared memories, and word of it on their barriers
+__device__ __forceinline__ void hand_tile(uint32_t* at, uint64_t* bar, uint32_t tile) {
+#pragma unroll
+  for (uint32_t r = 0; r < 2; ++r)
+    asm volatile(
+        "{\n"
+        ".reg .b32 a, b;\n"
+        "mapa.shared::cluster.u32 a, %0, %3;\n"
+        "mapa.shared::cluster.u32 b, %1, %3;\n"
+        "st.shared::cluster.u32 [a], %2;\n"
+        "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [b];\n"
+        "}\n" ::"r"(smem_u32(at)),
+        "r"(smem_u32(bar)), "r"(tile), "r"(r)
+        : "memory");
+}
 
 template <int MODE, bool GROUPED>
 __device__ __forceinline__ void pair_gemm_body(const CUtensorMap& map_a, const CUtensorMap* map_w_base, const PairParams& p, const int32_t* plan) {
@@ -96,8 +138,11 @@ __device__ __forceinline__ void pair_gemm_body(const CUtensorMap& map_a, const C
   uint64_t* cut_full = tmem_empty + 2;          // copies of another part's sums
   uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(cut_full + 1);
   volatile uint32_t* cut_lost = tmem_base_slot + 1;
-  volatile uint32_t* shape_s = tmem_base_slot + 2;  // [GP_SHAPES] (width / 32) << 24 | k-blocks
-  int32_t* info_s = reinterpret_cast<int32_t*>(tmem_base_slot + 2 + GP_SHAPES);  // [GP_INFO] grouped: the plan's first token tiles
+  uint64_t* tile_full = cut_full + 2;              // [GP_DRAWN] grouped: a drawn tile is there (each CTA's own)
+  uint64_t* tile_empty = tile_full + GP_DRAWN;     // [GP_DRAWN] everybody has read it (the first CTA's)
+  uint32_t* drawn_s = reinterpret_cast<uint32_t*>(tile_empty + GP_DRAWN);  // [GP_DRAWN]
+  volatile uint32_t* shape_s = drawn_s + GP_DRAWN;  // [GP_SHAPES] (width / 32) << 24 | k-blocks
+  int32_t* info_s = reinterpret_cast<int32_t*>(drawn_s + GP_DRAWN + GP_SHAPES);  // [GP_INFO] grouped: the plan's first token tiles
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = (int)cluster_ctarank();
@@ -150,6 +195,16 @@ __device__ __forceinline__ void pair_gemm_body(const CUtensorMap& map_a, const C
     return it;
   };
   walk.at.start(num_m, num_n);
+  const bool draws = GROUPED && p.draw != nullptr;
+  // The tile behind this cluster's nth.  Every reader of a drawn one (a whole warp, or the other CTA's producer) says so; >= num_tiles: there is none.
+  auto tile_after = [&](int tile, uint32_t nth) {
+    if (!draws) return tile + n_cta;
+    const uint32_t slot = nth % GP_DRAWN;
+    mbar_wait_cluster(&tile_full[slot], (nth / GP_DRAWN) & 1);
+    const int next = (int)*(volatile uint32_t*)&drawn_s[slot];
+    return next;
+  };
+  auto tile_read = [&](uint32_t nth) { mbar_arrive_cluster(cluster_first(&tile_empty[nth % GP_DRAWN])); };
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < stages; ++i) {
@@ -161,6 +216,11 @@ __device__ __forceinline__ void pair_gemm_body(const CUtensorMap& map_a, const C
       mbar_init(&tmem_empty[i], 2 * GP_EPI_WARPS);  // one arrive per epilogue warp of both CTAs
     }
     mbar_init(cut_full, 1);
+    if (GROUPED)
+      for (int i = 0; i < GP_DRAWN; ++i) {
+        mbar_init(&tile_full[i], 1);
+        mbar_init(&tile_empty[i], 2 + 2 * GP_EPI_WARPS);  // the issuing warp, the other CTA's producer, the epilogue warps
+      }
     *cut_lost = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
@@ -176,39 +236,68 @@ __device__ __forceinline__ void pair_gemm_body(const CUtensorMap& map_a, const C
   if (!GROUPED) pdl_wait();  // barriers, tensor memory and the cluster's meeting are behind the predecessor's end
 
   if (warp == 0) {
-    // ================= TMA producer =================
-    if (lane == 0) {
-      uint32_t s = 0, par = 0, it = 0, nth = 0;
-      uint8_t* st = smem;
-      for (int tile = cta; tile < num_tiles; tile += n_cta, ++nth) {
-        const Item w = next_item(tile);
-        shape_s[nth & (GP_SHAPES - 1)] = (uint32_t)(w.width / 32) << 24 | (uint32_t)(w.kb1 - w.kb0);  // for the MMA thread; more slots than stages: the one it still reads is not overwritten
-        const int expert = GROUPED ? item_expert[w.mu] : 0;
-        const bool packed = GROUPED && (p.w_n | p.w_k) != 0;
-        const CUtensorMap* wmap = map_w_base + (packed ? 0 : expert);
-        const int wr = w.n0 + rank * TG_BM + (packed ? expert * p.w_n : 0), wc = packed ? expert * p.w_k : 0;
-        const int t0 = w.t0 + rank * (w.width / 2);
-        for (int kb = w.kb0; kb < w.kb1; ++kb, ++it) {
+    // ================= TMA producer (one thread, elected by the warp, which walks as a whole) =================
+    const uint32_t full_first = cluster_first(full);
+    uint32_t s = 0, par = 0, it = 0, nth = 0;
+    for (int tile = cta; tile < num_tiles; ++nth) {
+      const Item w = next_item(tile);
+      const uint32_t shape = (uint32_t)(w.width / 32) << 24 | (uint32_t)(w.kb1 - w.kb0);
+      const int expert = GROUPED ? item_expert[w.mu] : 0;
+      const bool packed = GROUPED && (p.w_n | p.w_k) != 0;
+      const CUtensorMap* wmap = map_w_base + (packed ? 0 : expert);
+      const int wr = w.n0 + rank * TG_BM + (packed ? expert * p.w_n : 0), wc = packed ? expert * p.w_k : 0;
+      const int t0 = w.t0 + rank * (w.width / 2);
+      if (elect_one()) shape_s[nth & (GP_SHAPES - 1)] = shape;  // for the MMA warp; more slots than stages: the one it still reads is not overwritten
+      auto copy = [&](int kb0, int kb1) {
+        for (int kb = kb0; kb < kb1; ++kb, ++it) {
           mbar_wait(&empty[s], par ^ 1, 11, it);
-          // the pair's four tiles count on the first CTA's barrier (the other CTA's may land before it is armed: the count goes negative)
-          if (rank == 0) mbar_arrive_expect_tx(&full[s], arriving);
-          const uint32_t bar = cluster_first(&full[s]);
-          tma_load_2d_pair(st, wmap, bar, wc + kb * TG_BK, wr);
-          tma_load_2d_pair(st + GP_W_BYTES, &map_a, bar, kb * TG_BK, t0);
-          st += stage_bytes;
+          if (elect_one()) {
+            // the pair's four tiles count on the first CTA's barrier (the other CTA's may land before it is armed: the count goes negative)
+            if (rank == 0) mbar_arrive_expect_tx(&full[s], arriving);
+            uint8_t* const st = smem + s * stage_bytes;
+            const uint32_t bar = full_first + s * 8u;
+            tma_load_2d_pair(st, wmap, bar, wc + kb * TG_BK, wr);
+            tma_load_2d_pair(st + GP_W_BYTES, &map_a, bar, kb * TG_BK, t0);
+          }
+          __syncwarp();
           if (++s == (uint32_t)stages) {
             s = 0;
             par ^= 1;
-            st = smem;
           }
         }
+      };
+      if (!draws) {
+        copy(w.kb0, w.kb1);
+        tile += n_cta;
+      } else if (rank == 0) {  // every cluster that had a tile draws once in vain, so there are num_tiles draws: the last puts the counter back
+        const uint32_t slot = nth % GP_DRAWN;
+        const int draw_at = max(w.kb1 - GP_DRAW_AHEAD, w.kb0), hand_at = max(w.kb1 - GP_HAND_AHEAD, w.kb0);
+        unsigned drawn = 0;
+        copy(w.kb0, draw_at);
+        if (lane == 0) drawn = atomicAdd(p.draw, 1u);
+        copy(draw_at, hand_at);
+        tile = n_cta + (int)__shfl_sync(0xffffffffu, drawn, 0);
+        mbar_wait(&tile_empty[slot], ((nth / GP_DRAWN) & 1) ^ 1, 16, nth);
+        if (lane == 0) {
+          hand_tile(&drawn_s[slot], &tile_full[slot], (uint32_t)tile);
+          if (drawn == (unsigned)num_tiles - 1u) *(volatile unsigned*)p.draw = 0u;
+        }
+        __syncwarp();
+        copy(hand_at, w.kb1);
+      } else {
+        copy(w.kb0, w.kb1);
+        tile = tile_after(tile, nth);
+        __syncwarp();
+        if (lane == 0) tile_read(nth);
       }
     }
   } else if (warp == 1) {
     // ================= MMA issuer (one thread, for both CTAs) =================
-    if (lane == 0 && rank == 0) {
+    // The warp walks as a whole and elects a lane to issue, so that descriptors and counters are uniform.
+    if (rank == 0) {
+      const uint32_t ring = umma_desc_lo(smem_u32(smem));
       uint32_t s = 0, par = 0, it = 0, acc_it = 0;
-      for (int tile = cta; tile < num_tiles; tile += n_cta, ++acc_it) {
+      for (int tile = cta; tile < num_tiles; ++acc_it) {
         const uint32_t acc = acc_it & 1, acc_par = (acc_it >> 1) & 1;
         mbar_wait(&tmem_empty[acc], acc_par ^ 1, 12, acc_it);  // the epilogue has drained this accumulator buffer
         mbar_wait(&full[s], par, 13, it);
@@ -221,12 +310,15 @@ __device__ __forceinline__ void pair_gemm_body(const CUtensorMap& map_a, const C
           for (int kb = 0; kb < n_kb; ++kb, ++it) {
             if (kb > 0) mbar_wait(&full[s], par, 13, it);
             tc_fence_after();
-            const uint32_t addr = smem_u32(smem) + s * stage_bytes;
-            const uint64_t wdesc = umma_desc_sw128(addr), tdesc = umma_desc_sw128(addr + GP_W_BYTES);
+            const uint32_t wdesc = ring + s * (stage_bytes >> 4), tdesc = wdesc + (GP_W_BYTES >> 4);
+            if (elect_one()) {
+              umma_bf16_pair(d_tmem, wdesc, tdesc, idesc, kb > 0 ? 1u : 0u);
 #pragma unroll
-            for (int k = 0; k < TG_BK / 16; ++k)  // +32 bytes (= 2 in 16-byte units) per K = 16 step inside the 128-byte swizzled row
-              umma_bf16_pair(d_tmem, wdesc + (uint64_t)(2 * k), tdesc + (uint64_t)(2 * k), idesc, (kb > 0 || k) ? 1u : 0u);
-            umma_commit_pair(&empty[s]);  // frees the stage in both CTAs when these MMAs have read it
+              for (int k = 1; k < TG_BK / 16; ++k)  // +32 bytes (= 2 in 16-byte units) per K = 16 step inside the 128-byte swizzled row
+                umma_bf16_pair(d_tmem, wdesc + 2 * k, tdesc + 2 * k, idesc, 1u);
+              umma_commit_pair(&empty[s]);  // frees the stage in both CTAs when these MMAs have read it
+            }
+            __syncwarp();
             if (++s == (uint32_t)stages) {
               s = 0;
               par ^= 1;
@@ -243,14 +335,23 @@ __device__ __forceinline__ void pair_gemm_body(const CUtensorMap& map_a, const C
           case 7: k_blocks(std::integral_constant<uint32_t, 7>()); break;
           default: k_blocks(std::integral_constant<uint32_t, 8>()); break;
         }
-        umma_commit_pair(&tmem_full[acc]);  // accumulator complete, in both CTAs
+        if (elect_one()) umma_commit_pair(&tmem_full[acc]);  // accumulator complete, in both CTAs
+        tile = tile_after(tile, acc_it);
+        __syncwarp();
+        if (draws && lane == 0) tile_read(acc_it);
       }
     }
   } else {
     // ========== epilogue warps 2..9: TMEM lanes (features) 32 * (warp % 4) .. + 31, every second block of 32 columns (tokens) ==========
     const int lane_base = (warp & 3) * 32, row = lane_base + lane, first = (warp - 2) >> 2;
     uint32_t acc_it = 0;
-    for (int tile = cta; tile < num_tiles; tile += n_cta, ++acc_it) {
+    auto after = [&](int tile) {
+      const int next = tile_after(tile, acc_it);
+      __syncwarp();
+      if (draws && lane == 0) tile_read(acc_it);
+      return next;
+    };
+    for (int tile = cta; tile < num_tiles; tile = after(tile), ++acc_it) {
       const Item w = next_item(tile);
       const int n = w.n0 + rank * TG_BM + lane_base;  // this warp's 32 features
       const int chunks = w.width / 32;

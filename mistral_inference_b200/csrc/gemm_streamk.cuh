@@ -110,10 +110,13 @@ __device__ __forceinline__ void sk_gemm_body(const CUtensorMap& map_a, const CUt
 
   if (warp == 0) {
     // ================= TMA producer =================
+    // One thread: of the experts' form elected by the warp, which walks as a whole (8 tokens through eight experts of 14336: 583 us, 560 with it), of the dense one lane 0 (the Nemo shape's
+    // step of 32 tokens: 1624 us, 1666 with an elected one).
     // Iteration `it` handles unit u_begin + it.  Weights are never written by any kernel: the W tiles of the first ring are
     // requested BEFORE the programmatic-dependent-launch wait (they stream in while the previous kernel drains); the A tiles of
     // those stages, which the previous kernel produced, follow after it.
-    if (lane == 0) {
+    if (GROUPED || lane == 0) {
+      auto mine = [&]() { return !GROUPED || elect_one(); };
       const uint32_t n_it = (uint32_t)(u_end - u_begin);
       auto issue = [&](uint32_t it, bool do_a, bool do_w) {
         const uint32_t u = (uint32_t)u_begin + it;
@@ -129,23 +132,27 @@ __device__ __forceinline__ void sk_gemm_body(const CUtensorMap& map_a, const CUt
       };
       const uint32_t head = GROUPED ? 0u : (n_it < (uint32_t)STAGES ? n_it : (uint32_t)STAGES);  // (grouped: the tile list itself is the previous kernel's output)
       for (uint32_t it = 0; it < head; ++it) {
-        mbar_arrive_expect_tx(&full[it % STAGES], STAGE_BYTES);  // first lap: every slot is free
+        mbar_arrive_expect_tx(&full[it % STAGES], STAGE_BYTES);  // first lap: every slot is free (head is 0 in the experts' form)
         issue(it, false, true);
       }
       pdl_wait();
-      SK_STAMP(1);  // predecessor complete: A tiles may be requested
+      if (lane == 0) SK_STAMP(1);  // predecessor complete: A tiles may be requested
       for (uint32_t it = 0; it < head; ++it) issue(it, true, false);
       for (uint32_t it = head; it < n_it; ++it) {
         const uint32_t s = it % STAGES, par = (it / STAGES) & 1;
         mbar_wait(&empty[s], par ^ 1, 21, it);
-        mbar_arrive_expect_tx(&full[s], STAGE_BYTES);
-        issue(it, true, true);
+        if (mine()) {
+          mbar_arrive_expect_tx(&full[s], STAGE_BYTES);
+          issue(it, true, true);
+        }
+        if (GROUPED) __syncwarp();
       }
-      SK_STAMP(3);  // last tile requested
+      if (lane == 0) SK_STAMP(3);  // last tile requested
     }
   } else if (warp == 1) {
-    // ================= MMA issuer (one thread) =================
-    if (lane == 0) {
+    // ================= MMA issuer (one thread, elected by the warp) =================
+    {
+      const uint32_t ring = umma_desc_lo(smem_u32(smem));
       uint32_t it = 0, seg = 0;
       for (long long u = u_begin; u < u_end; ++seg) {
         const int kb0 = (int)(u % num_k);
@@ -158,19 +165,22 @@ __device__ __forceinline__ void sk_gemm_body(const CUtensorMap& map_a, const CUt
           const uint32_t s = it % STAGES, par = (it / STAGES) & 1;
           mbar_wait(&full[s], par, 23, it);
 #ifdef MB200_SK_TRACE
-          if (it == 0) SK_STAMP(2);  // first stage landed: first MMA
+          if (it == 0 && lane == 0) SK_STAMP(2);  // first stage landed: first MMA
 #endif
           tc_fence_after();
-          const uint32_t a_addr = smem_u32(smem + s * STAGE_BYTES);
-          const uint64_t adesc = umma_desc_sw128(a_addr), bdesc = umma_desc_sw128(a_addr + A_BYTES);
+          const uint32_t adesc = ring + s * (STAGE_BYTES >> 4), bdesc = adesc + (A_BYTES >> 4);
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < TG_BK / 16; ++k) umma_bf16(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), kIdesc, (kb > kb0 || k) ? 1u : 0u);
-          umma_commit(&empty[s]);
+            for (int k = 0; k < TG_BK / 16; ++k) umma_bf16(d_tmem, adesc + 2 * k, bdesc + 2 * k, kIdesc, (kb > kb0 || k) ? 1u : 0u);
+            umma_commit(&empty[s]);
+          }
+          __syncwarp();
         }
-        umma_commit(&tmem_full[acc]);
+        if (elect_one()) umma_commit(&tmem_full[acc]);
+        __syncwarp();
         u += kb1 - kb0;
       }
-      SK_STAMP(4);  // last MMA issued
+      if (lane == 0) SK_STAMP(4);  // last MMA issued
     }
   } else {
     // ================= epilogue warps 2..5: TMEM lanes 32 * (warp % 4) .. + 31 =================

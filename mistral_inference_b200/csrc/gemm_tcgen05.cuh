@@ -135,27 +135,52 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// D[tmem] (+)= A[smem] * B[smem], bf16 inputs, fp32 accumulate
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+// Shared-memory matrix descriptor of a K-major, 128B-swizzled tile whose rows are 64 bf16 = 128 bytes:
+// 8-row swizzle atoms of 1024 B (SBO), version 1 (sm_100), layout type 2 (SWIZZLE_128B).  (cute::UMMA::SmemDescriptor)
+// The upper word is one constant, the lower holds the address: an instruction's operands take one addition each.
+constexpr uint32_t UMMA_DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t umma_desc_lo(uint32_t smem_addr) { return ((smem_addr & 0x3ffff) >> 4) | (1u << 16); }
+// D[tmem] (+)= A[smem] * B[smem], bf16 inputs, fp32 accumulate.  a, b: lower words of the tiles' descriptors.
+// The warp that issues walks as a whole and elects a lane (elect_one): descriptors and counters are then uniform.  From a divergent lane an instruction took some 100 clocks to issue,
+// more than it runs on a narrow tile: a k-block of a pair's tile w wide cost 256 + w clocks, and now 2 w and little more (4096 x 28672 from 600 tokens: 132 us, now 112; from 1102: 196, 169).
+__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n"
       ".reg .pred p;\n"
+      ".reg .b64 da, db;\n"
+      "mov.b64 da, {%1, %5};\n"
+      "mov.b64 db, {%2, %5};\n"
       "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n"
       "}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      "r"(a), "r"(b), "r"(idesc), "r"(accumulate), "n"(UMMA_DESC_HI)
       : "memory");
 }
-// the same by a pair of CTAs (issued by the first): its A and B tiles are the rows of both CTAs' shared memories at these offsets, D its rows' halves
-__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+// the same by a pair of CTAs (issued by the first): its A and B tiles are the rows of both CTAs' shared memories at these offsets, D its rows' halves.
+__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n"
       ".reg .pred p;\n"
+      ".reg .b64 da, db;\n"
+      "mov.b64 da, {%1, %5};\n"
+      "mov.b64 db, {%2, %5};\n"
       "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %3, p;\n"
       "}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      "r"(a), "r"(b), "r"(idesc), "r"(accumulate), "n"(UMMA_DESC_HI)
       : "memory");
+}
+// one lane of a warp that runs as a whole (the same one every time)
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "elect.sync _|p, 0xffffffff;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(one));
+  return one != 0u;
 }
 // arrive on an mbarrier once every previously issued tcgen05.mma of this thread has completed
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
@@ -190,12 +215,6 @@ __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.
 __device__ __forceinline__ void tmem_ld_32x32b_x32(uint32_t taddr, uint32_t (&v)[32]) {
   tmem_ld_32x32b_x32_nowait(taddr, v);
   tmem_wait_ld();
-}
-
-// Shared-memory matrix descriptor of a K-major, 128B-swizzled tile whose rows are 64 bf16 = 128 bytes:
-// 8-row swizzle atoms of 1024 B (SBO), version 1 (sm_100), layout type 2 (SWIZZLE_128B).  (cute::UMMA::SmemDescriptor)
-__device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
-  return (uint64_t)((smem_addr & 0x3ffff) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
 
 // Tile order.  The persistent CTAs (pairs) take tiles t = cta, cta + n_cta, ...: at any moment ~n_cta consecutive tile ids are in flight,
@@ -293,8 +312,8 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
   const uint32_t tmem_base = *tmem_base_slot;
 
   if (warp == 0) {
-    // ================= TMA producer =================
-    if (lane == 0) {
+    // ================= TMA producer (one thread, elected by the warp) =================
+    {
       uint32_t it = 0;
       for (int tile = cta; tile < num_tiles; tile += n_cta) {
         int mu, nt;
@@ -307,16 +326,20 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
         for (int kb = 0; kb < num_k; ++kb, ++it) {
           const uint32_t s = it % TG_STAGES, par = (it / TG_STAGES) & 1;
           mbar_wait(&empty[s], par ^ 1, 11, it);
-          uint8_t* sa = smem + s * TG_STAGE_BYTES;
-          mbar_arrive_expect_tx(&full[s], TG_STAGE_BYTES);
-          tma_load_2d(sa, &map_a, &full[s], kb * TG_BK, m0);
-          tma_load_2d(sa + TG_A_BYTES, wmap, &full[s], wc + kb * TG_BK, wr);
+          if (elect_one()) {
+            uint8_t* sa = smem + s * TG_STAGE_BYTES;
+            mbar_arrive_expect_tx(&full[s], TG_STAGE_BYTES);
+            tma_load_2d(sa, &map_a, &full[s], kb * TG_BK, m0);
+            tma_load_2d(sa + TG_A_BYTES, wmap, &full[s], wc + kb * TG_BK, wr);
+          }
+          __syncwarp();
         }
       }
     }
   } else if (warp == 1) {
-    // ================= MMA issuer (one thread) =================
-    if (lane == 0) {
+    // ================= MMA issuer (one thread, elected by the warp) =================
+    {
+      const uint32_t ring = umma_desc_lo(smem_u32(smem));
       uint32_t it = 0, acc_it = 0;
       for (int tile = cta; tile < num_tiles; tile += n_cta, ++acc_it) {
         const uint32_t acc = acc_it & 1, acc_par = (acc_it >> 1) & 1;
@@ -327,14 +350,17 @@ __device__ __forceinline__ void tc_gemm_body(const CUtensorMap& map_a, const CUt
           const uint32_t s = it % TG_STAGES, par = (it / TG_STAGES) & 1;
           mbar_wait(&full[s], par, 13, it);
           tc_fence_after();
-          const uint32_t a_addr = smem_u32(smem + s * TG_STAGE_BYTES);
-          const uint64_t adesc = umma_desc_sw128(a_addr), bdesc = umma_desc_sw128(a_addr + TG_A_BYTES);
+          const uint32_t adesc = ring + s * (TG_STAGE_BYTES >> 4), bdesc = adesc + (TG_A_BYTES >> 4);
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < TG_BK / 16; ++k)  // +32 bytes (= 2 in 16-byte units) per K = 16 step inside the 128-byte swizzled row
-            umma_bf16(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), kUmmaIdesc, (kb > 0 || k) ? 1u : 0u);
-          umma_commit(&empty[s]);
+            for (int k = 0; k < TG_BK / 16; ++k)  // +32 bytes (= 2 in 16-byte units) per K = 16 step inside the 128-byte swizzled row
+              umma_bf16(d_tmem, adesc + 2 * k, bdesc + 2 * k, kUmmaIdesc, (kb > 0 || k) ? 1u : 0u);
+            umma_commit(&empty[s]);
+          }
+          __syncwarp();
         }
-        umma_commit(&tmem_full[acc]);
+        if (elect_one()) umma_commit(&tmem_full[acc]);
+        __syncwarp();
       }
     }
   } else {

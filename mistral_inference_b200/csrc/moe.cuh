@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(256) moe_route_kernel(const bf16* hn, const bf
 
 // ---- plan: one CTA ---------------------------------------------------------------------------------------------------------
 // plan layout (int32): [0] m tiles owned by this rank, [1] padded rows in total, [2] tile capacity, [3] (token, expert) pairs, [4]/[5] statistics, [6] token tiles for
-// pairs of CTAs, [8 + e] start of expert e's segment (e = 0..E), then from word MOE_PLAN_HEADER four lists of `capacity` words: tile_expert, tile_row0 (m tiles),
+// pairs of CTAs, [7] tiles that these have drawn (zero between launches), [8 + e] start of expert e's segment (e = 0..E), then from word MOE_PLAN_HEADER four lists of `capacity` words: tile_expert, tile_row0 (m tiles),
 // pair_expert, pair_info (token tiles: first row | width / 32).
 constexpr int MP_THREADS = 1024, MP_ROW = MP_THREADS + MP_THREADS / 32;
 inline size_t moe_plan_smem(int64_t E) { return ((size_t)E * MP_ROW + 2 * E + 1) * sizeof(int32_t); }
@@ -244,6 +244,7 @@ __global__ void __launch_bounds__(MP_THREADS) moe_plan_kernel(const int32_t* sel
       plan[4] += touched;  // statistics (never reset by the kernel): experts with at least one row, summed over calls ...
       plan[5] += 1;        // ... and the number of calls: the measured "distinct experts per layer" of bench.py
       plan[6] = min(np, tile_cap);
+      plan[7] = 0;
       seg[E] = rows;
       plan[8 + E] = rows;
     }
@@ -428,6 +429,7 @@ int launch_grouped_pair(const CUtensorMap& map_a, const MoeWeightMaps& maps, int
   p.w_n = (int)w_n;
   p.w_k = (int)w_k;
   p.units = sms / 2;
+  if (K >= GP_DRAW_MIN_K) p.draw = reinterpret_cast<unsigned*>(const_cast<int32_t*>(plan) + 7);
   return launch_pairs(gemm_pair_grouped_kernel<MODE>, p.units, stream, map_a, maps, p, plan);
 }
 
