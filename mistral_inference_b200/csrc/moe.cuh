@@ -13,7 +13,7 @@
 //   grouped GEMM x2     g = silu(xs W1_e^T) * (xs W3_e^T);  yw = bf16(w * bf16(g W2_e^T)), the second one storing every row on ALL
 //                       ranks of the group (peer stores over NVLink) -- the exchange step of expert parallelism is the epilogue of
 //                       the down projection, an all-gather of rows with no reduction.  gemm_streamk.cuh for few tokens,
-//                       gemm_tcgen05.cuh, and from ~512 rows an expert gemm_pair.cuh.
+//                       gemm_tcgen05.cuh, and from ~128 rows an expert gemm_pair.cuh.
 //   moe_combine_kernel  (expert parallel: signal the peers / wait for theirs) out[t] = bf16(h[t] + sum_j yw[slot(t, j)]) with the
 //                       sum taken in ascending expert index, each step rounded to bf16 like `results +=`: the reference's
 //                       order for any k and any number of ranks.  (The rows themselves are the same on any number of ranks but for
@@ -472,9 +472,9 @@ int launch_grouped(const void* a, int64_t rows_cap, int64_t K, int64_t N, const 
     return launch_grouped_streamk<MODE, 64>(a, rows_cap, K, N, w_host, E, plan, epi, workspace, workspace_bytes, header, sms, stream);
   }
   if (tile_rows == 128) {
-    // From about 384 rows an expert.  The layer of eight experts of 4096 x 14336 with the GEMMs below and with pairs, us: 300 tokens (75 rows an expert) 529, 562, 600 691, 598,
-    // 1000 836, 775, 1300 970, 1004, 1536 1182, 1079, 2048 1496, 1411.  (The line dates from tiles of 128-row pairs, half of which such segments left empty.)
-    if (N % 128 == 0 && tcgen05_cluster_enabled() && rows_cap >= (int64_t)E * 512) {
+    // From about 128 rows an expert, where the GEMMs below begin to need two tiles of tokens for one.  The layer of eight experts of 4096 x 14336 with the GEMMs below and with pairs, us:
+    // 300 tokens (75 rows an expert) 527, 550, 450 530, 562, 600 681, 594, 800 695, 631, 1000 829, 781, 1300 948, 938; of 6144 x 16384: 400 872, 876, 800 1192, 1018, 1200 1678, 1584.
+    if (N % 128 == 0 && tcgen05_cluster_enabled() && rows_cap >= (int64_t)E * 256) {
       CUtensorMap map_a;
       MoeWeightMaps maps;
       int rc = make_tensor_map_2d(&map_a, a, rows_cap, K, TG_BM);
@@ -594,9 +594,9 @@ inline int launch_grouped_packed(const void* a, int64_t rows_cap, int64_t K, int
   rc = make_tensor_map_2d(&maps.m[0], w, w_rows, w_cols, TG_BM);
   if (rc) return rc;
   for (int e = 1; e < MOE_MAX_EXPERTS; ++e) maps.m[e] = maps.m[0];
-  // As in launch_grouped.  16 experts of 1408, width 2048, with the GEMM below and with pairs, us: 400 tokens 108, 107, 800 146, 127, 1200 168, 148, 1800 225, 180; eight of
-  // 14336, width 4096: 600 tokens 855, 595, 1300 1356, 1075, 2500 2333, 1800.  (The plan of up to 512 rows lists no token tiles of pairs.)
-  if (tcgen05_cluster_enabled() && pairs >= 384 * E && pairs > 512)
+  // Wherever the plan lists token tiles of pairs (more than 512 rows in all).  16 experts of 1408, width 2048, with the GEMM below and with pairs, us: 130 tokens 117, 114, 250 102, 97,
+  // 450 104, 103, 800 135, 123, 1300 162, 143; eight of 14336, width 4096: 300 tokens 539, 523, 600 772, 580, 1000 923, 776, 1300 1126, 998.
+  if (tcgen05_cluster_enabled() && pairs > 512)
     return launch_grouped_pair<EPI_LAYER>(map_a, maps, rows_cap, K, N, w_n, w_k, plan, epi, sms, stream);
   using Cfg = TgCfg<128, 128, kEpiSmem<EPI_LAYER>>;
   TcGemmParams p;
