@@ -20,10 +20,11 @@
 // Linear); accumulation is fp32 in both modes.
 //
 // Kernels: `linear_tiled_mma` (bf16), `linear_f32_pair` (fp32, hybrid_linear_f32.cuh) and `linear_tiled_fma` (fp32, K < 16) for prompts, any shape; `linear_skinny` (M <= 8 rows, FMA,
-// one warp per pair of weight rows) and `linear_skinny_mma` (bf16, up to 16 rows, tensor cores) for decode: every weight byte is read
-// once with 16-byte loads; `linear_decay_mma` for decays from a low rank.  The large aligned bf16 Linears of prompts go to the main
+// one warp per pair of weight rows) and `stream_linear_kernel` (bf16, up to 16 rows, tensor cores) for decode: every weight byte is read
+// once; `linear_decay_mma` for decays from a low rank.  The large aligned bf16 Linears of prompts go to the main
 // library's tcgen05 GEMMs, with these steps in their epilogue (see _abi_hybrid.linear).
 #pragma once
+#include "../stream_linear.cuh"
 #include "hybrid_common.cuh"
 
 namespace mbh {
@@ -381,83 +382,29 @@ __global__ void __launch_bounds__(SK_WARPS * 32) linear_skinny(LinearArgs a) {
         }
 }
 
-// ------------------------------------------------------------------------------------------------ skinny on tensor cores (bf16, 1..16 rows)
-// y^T = W x^T: the 16 weight rows of a CTA are the M side of m16n8k16 tiles, the (up to 8 NT) tokens the N side, so a decode batch
-// costs one tensor-core instruction per 16 x 16 weights instead of 8 FMAs per weight.  The CTA's warps split K; every lane
-// loads 16 contiguous bytes of two weight rows and of a token's activations per step -- the k order inside a step is
-// permuted identically for both operands, which a dot product does not notice.  Needs K % 8 == 0 and 16-byte aligned rows.
-// Bound by memory latency more than by bandwidth (a CTA has 8 to 32 steps of 8 KB): the weights of the first SKM_AHEAD steps -- all of them up to
-// K = 2048 -- are requested before the wait for the predecessor's output, later ones as their registers come free.
-constexpr int SKM_WARPS = 8, SKM_AHEAD = 8, SKM_MAX_M = 16;
+// ------------------------------------------------------------------------------------------------ decode on tensor cores (bf16, 1..16 rows): ../stream_linear.cuh
+constexpr int SM_MAX_M = 16;
 
-__device__ __forceinline__ uint4 load_weights(const bf16* p) {  // read once: not kept in L1
-    uint4 r;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
-    return r;
-}
-
-template <int NT>
-__global__ void __launch_bounds__(SKM_WARPS * 32, 2) linear_skinny_mma(LinearArgs a) {
-    __shared__ float part[SKM_WARPS][16][8 * NT + 1];
-    const bf16* X = static_cast<const bf16*>(a.x);
-    const bf16* W = static_cast<const bf16*>(a.w);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
-    const int n0 = blockIdx.x * 16, k0 = warp * 32 + tig * 8;
-    constexpr int STEP = SKM_WARPS * 32;
-    const bf16* wa = W + (size_t)min(n0 + gid, a.N - 1) * a.K + k0;
-    const bf16* wb = W + (size_t)min(n0 + gid + 8, a.N - 1) * a.K + k0;
-    uint4 va[SKM_AHEAD], vb[SKM_AHEAD];
-    const uint4 zero = make_uint4(0, 0, 0, 0);
-#pragma unroll
-    for (int u = 0; u < SKM_AHEAD; ++u) {
-        const bool ok = k0 + u * STEP < a.K;
-        va[u] = ok ? load_weights(wa + u * STEP) : zero;
-        vb[u] = ok ? load_weights(wb + u * STEP) : zero;
+struct StreamEpi {
+    LinearArgs a;  // (bias: added here)
+    const void* bias;
+    struct Ahead { float b0, b1, o0, o1; };
+    __device__ __forceinline__ bool adds() const { return a.epi == EPI_RESIDUAL || a.epi == EPI_RESIDUAL_SCALED; }
+    __device__ __forceinline__ Ahead fetch(int m, int n, bool two) const {
+        Ahead r = {0.f, 0.f, 0.f, 0.f};
+        if (bias) { r.b0 = to_f(static_cast<const bf16*>(bias)[n]); if (two) r.b1 = to_f(static_cast<const bf16*>(bias)[n + 1]); }
+        if (adds()) { r.o0 = a.out32[(size_t)m * a.N + n]; if (two) r.o1 = a.out32[(size_t)m * a.N + n + 1]; }
+        return r;
     }
-    pdl_trigger();
-    pdl_wait();
-    float c[NT][4];
-    const bf16* xr[NT];
-#pragma unroll
-    for (int t = 0; t < NT; ++t) {
-        c[t][0] = c[t][1] = c[t][2] = c[t][3] = 0.f;
-        xr[t] = X + (size_t)min(t * 8 + gid, a.M - 1) * a.x_pitch() + k0;  // rows past the end repeat the last one: their sums go nowhere
+    __device__ __forceinline__ void finish(int m, int n, float v0, float v1, bool two, const Ahead& r) const {
+        v0 += r.b0;
+        v1 += r.b1;
+        if (!adds()) return epilogue_pair<bf16>(a, m, n, v0, v1, two);
+        const float f = a.epi == EPI_RESIDUAL ? 1.f : a.alpha;
+        a.out32[(size_t)m * a.N + n] = r.o0 + f * rnd<bf16>(v0);
+        if (two) a.out32[(size_t)m * a.N + n + 1] = r.o1 + f * rnd<bf16>(v1);
     }
-    const int steps = (a.K + STEP - 1) / STEP;
-    for (int i = 0; i < steps; i += SKM_AHEAD) {
-#pragma unroll
-        for (int u = 0; u < SKM_AHEAD; ++u) {
-            const int k = (i + u) * STEP;
-            uint4 vx[NT];
-#pragma unroll
-            for (int t = 0; t < NT; ++t) vx[t] = k0 + k < a.K ? *reinterpret_cast<const uint4*>(xr[t] + k) : zero;
-            const uint32_t a0[4] = {va[u].x, vb[u].x, va[u].y, vb[u].y}, a1[4] = {va[u].z, vb[u].z, va[u].w, vb[u].w};
-#pragma unroll
-            for (int t = 0; t < NT; ++t) {
-                mma_bf16(c[t], a0, vx[t].x, vx[t].y);
-                mma_bf16(c[t], a1, vx[t].z, vx[t].w);
-            }
-            const bool more = k0 + k + SKM_AHEAD * STEP < a.K;
-            va[u] = more ? load_weights(wa + k + SKM_AHEAD * STEP) : zero;
-            vb[u] = more ? load_weights(wb + k + SKM_AHEAD * STEP) : zero;
-        }
-    }
-#pragma unroll
-    for (int t = 0; t < NT; ++t) {
-        part[warp][gid][t * 8 + tig * 2] = c[t][0]; part[warp][gid][t * 8 + tig * 2 + 1] = c[t][1];
-        part[warp][gid + 8][t * 8 + tig * 2] = c[t][2]; part[warp][gid + 8][t * 8 + tig * 2 + 1] = c[t][3];
-    }
-    __syncthreads();
-    if (threadIdx.x < 64 * NT) {
-        const int m = threadIdx.x % (8 * NT), r = threadIdx.x / (8 * NT) * 2, n = n0 + r;
-        if (m < a.M && n < a.N) {
-            float s0 = 0.f, s1 = 0.f;
-#pragma unroll
-            for (int w = 0; w < SKM_WARPS; ++w) { s0 += part[w][r][m]; s1 += part[w][r + 1][m]; }
-            epilogue_pair<bf16>(a, m, n, s0, s1, n + 1 < a.N);
-        }
-    }
-}
+};
 
 }  // namespace mbh
 
@@ -470,9 +417,11 @@ template <typename T>
 inline cudaError_t launch_linear(const LinearArgs& a, cudaStream_t st, void* scratch = nullptr, int64_t scratch_bytes = 0) {
     if (a.M <= 0 || a.N <= 0) return cudaSuccess;
     if constexpr (sizeof(T) == 2) {
-        if (a.M <= SKM_MAX_M && a.K % 8 == 0 && a.x_pitch() % 8 == 0 && (reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.w)) % 16 == 0) {
-            const dim3 grid((a.N + 15) / 16);
-            return a.M <= 8 ? launch_pdl(linear_skinny_mma<1>, grid, dim3(SKM_WARPS * 32), 0, st, a) : launch_pdl(linear_skinny_mma<2>, grid, dim3(SKM_WARPS * 32), 0, st, a);
+        if (a.M <= SM_MAX_M && a.K % 8 == 0 && a.x_pitch() % 8 == 0 && (reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.w)) % 16 == 0) {
+            cudaError_t e = cudaSuccess;
+            StreamEpi epi{a, a.bias};
+            epi.a.bias = nullptr;
+            if (a.M <= 8 ? stream_linear::launch<1>(a.x, a.x_pitch(), a.w, a.M, a.N, a.K, epi, st, e) : stream_linear::launch<2>(a.x, a.x_pitch(), a.w, a.M, a.N, a.K, epi, st, e)) return e;
         }
     }
     if (a.M <= SK_MAX_M) {

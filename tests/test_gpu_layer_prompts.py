@@ -751,3 +751,25 @@ def test_fp32_linear_of_more_rows_than_a_launch_takes():
     assert rel(got, (x.double() @ w.double().T).clamp(min=0) ** 2 * rs.double().repeat_interleave(8, 1)) < 2 ** -21
     assert h.lib().mbh_linear_relu2(x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, rs.data_ptr(), 5, 8, 1, torch.cuda.current_stream().cuda_stream) == 0
     assert torch.equal(out, got)
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 16])
+@pytest.mark.parametrize("N,K,pad", [(1, 8, 0), (130, 72, 8), (1024, 64, 0), (1186, 192, 64), (3072, 2048, 0), (2049, 1416, 0), (8192, 448, 16), (18961, 128, 0), (38000, 320, 0)])
+def test_decode_linear_streams_whole_rows(M, N, K, pad):
+    """Rows of 8 to 128 a CTA, one and several units of them, the last ones short, k-blocks that end inside a stage and inside a block, x in a wider matrix: a bf16 Linear is within its
+    rounding (2^-8) of float64, what stays fp32 within 2 K 2^-24 of the products' sizes."""
+    from mistral_inference_b200 import _abi_hybrid as h
+
+    g = torch.Generator(device=DEV).manual_seed(M + N + K)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV)  # noqa: E731
+    x, w, b, base = rnd(M, K + pad).bfloat16()[:, :K], (rnd(N, K) / K ** 0.5).bfloat16(), rnd(N).bfloat16(), rnd(M, N)
+    ref = x.double() @ w.double().T
+    size = x.double().abs() @ w.double().abs().T * (2 * K * 2.0 ** -24)
+    assert ((h.linear(x, w, b).double() - ref - b.double()).abs() <= 2 ** -8 * (ref + b.double()).abs() + size + 1e-30).all()
+    assert ((h.linear(x, w, None, epi=h.EPI_F32).double() - ref).abs() <= size + 1e-30).all()
+    assert ((h.linear(x, w, b, epi=h.EPI_RESIDUAL, residual=base.clone()).double() - base.double() - ref - b.double()).abs()
+            <= 2 ** -8 * (ref + b.double()).abs() + size + 2 ** -23 * (base.double().abs() + (ref + b.double()).abs())).all()
+    if N % 2 == 0:
+        y, F = ref.bfloat16().double(), torch.nn.functional
+        got = h.linear_swiglu(x.contiguous(), w, None)
+        assert rel(got, F.silu(y[:, 0::2]) * y[:, 1::2]) < 2 ** -7
