@@ -53,7 +53,7 @@ static int run_linear(const void* x, const void* norm_w, const void* w, const Ep
   p.K = (int)K;
   p.eps = eps;
   p.epi = epi;
-  if ((T <= MB200_SKINNY_MAX_T && !skinny_mma_better(T, K, norm_w != nullptr)) || (T <= MB200_SKINNY_MAX_T && norm_w && !room))
+  if (T == 1 || (T <= MB200_SKINNY_MAX_T && norm_w && !room))
     return norm_w ? launch_skinny<MODE, true>(p, (int)T, st) : launch_skinny<MODE, false>(p, (int)T, st);
   const void* a = x;
   if (norm_w) {
@@ -63,10 +63,11 @@ static int run_linear(const void* x, const void* norm_w, const void* w, const Ep
     if (rc) return rc;
     a = normed;
   }
-  if (T <= MB200_SKINNY_MAX_T) {
-    p.x = a;
-    return launch_skinny_mma<MODE>(p, (int)T, st);
-  }
+  p.x = a;
+  p.norm_w = nullptr;
+  int rc = MB200_OK;
+  if (launch_stream<MODE>(p, (int)T, st, rc)) return rc;
+  if (T <= MB200_SKINNY_MAX_T) return launch_skinny<MODE, false>(p, (int)T, st);
   GemmParams g;
   g.a = a;
   g.w = w;

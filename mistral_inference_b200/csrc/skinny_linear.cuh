@@ -1,19 +1,13 @@
 // Weight-streaming linears for a decode step's few tokens:  y[t, n] = sum_k x[t, k] * W[n, k]
 //
-// skinny_mma_kernel (2 to 4 tokens, rows above 4096; 4 with the norm in front).  y^T = W x^T on mma.sync: 16 weight rows of a CTA are the M side of m16n8k16 tiles, the
-// tokens the N side; the CTA's 8 warps split K, a lane takes 16 contiguous bytes of two weight rows and of a token per step (the k order inside a
-// step is permuted alike on both sides).  The weights of the first eight steps are requested BEFORE the programmatic-dependent-launch wait -- no
-// kernel writes weights -- so they stream in while the predecessor finishes.  HBM-bound like skinny_linear_kernel, whose FMAs and staging of
-// T * K * 2 bytes per CTA bind first there; figures at skinny_mma_better.  At 8 tokens the stream-K kernel is ahead (637 us a step of 4 layers
-// against 753: it reads the tokens once per 128 weight rows, not per 16).
-//
-// skinny_linear_kernel (1 token, other rows up to 4096; up to 4 tokens where there is no workspace for the normed rows), FMA:
+// skinny_linear_kernel (1 token; up to 4 where there is no workspace for the normed rows), FMA:
 // Roofline: HBM.  Algorithmic bytes = N*K*2 (every weight read exactly once); the activations
 // (T*K*2 bytes) are re-read by every CTA from L2.  Each warp owns 2 adjacent weight rows (one RoPE pair /
 // one gate-up pair) and streams them with 16-byte no-allocate loads, 4 in flight per row per lane; x lives in
 // shared memory (optionally RMS-normalised in place by every CTA -- 8..28 KB, cheaper than a kernel boundary).
 #pragma once
 #include "epilogue.cuh"
+#include "stream_linear.cuh"
 
 namespace mb200 {
 
@@ -155,81 +149,59 @@ __global__ void __launch_bounds__(kSkinnyThreads) skinny_linear_kernel(const Ski
     if (lane == t) epi_pair<MODE>(p.epi, t, n0, acc[0][t], acc[1][t]);
 }
 
-// ---- tensor cores ------------------------------------------------------------------------------------------------------------------
-constexpr int SM_WARPS = 8, SM_AHEAD = 8;
-
-// Which of the two takes 2 to 4 tokens: what an FMA CTA stages and multiplies grows with T * K.  Steps of 4 layers (K = 4096 and 14336 in the 7B
-// shape; 4096, 5120 and 14336 in the Nemo shape), FMAs alone / this rule / tensor cores alone, us: 2 tokens 612 / 548 / 665 and 842 / 729 / -;
-// 3 tokens 666 / 596 / 682 and 1051 / 745 / 927; 4 tokens 780 / 492 / 664 and 1283 / 765 / 969.  Four tokens with the norm in front take tensor
-// cores at any K (7B: 704 without that); the Linear behind the attention (K = 4096, no norm) is the one that loses by them.
-inline bool skinny_mma_better(int64_t T, int64_t K, bool norm) { return (T >= 2 && K > 4096) || (T == 4 && norm); }
-
-__device__ __forceinline__ void skinny_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
+// ---- 2 tokens and more: ../stream_linear.cuh -------------------------------------------------------------------------------------------
+constexpr int STREAM_MAX_T = 32;
 
 template <int MODE>
-__global__ void __launch_bounds__(SM_WARPS * 32, 2) skinny_mma_kernel(const SkinnyParams p, int T) {
-  __shared__ float part[SM_WARPS][16][9];
-  const bf16* X = reinterpret_cast<const bf16*>(p.x);
-  const bf16* W = reinterpret_cast<const bf16*>(p.w);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
-  const int n0 = blockIdx.x * 16, k0 = warp * 32 + tig * 8;
-  constexpr int STEP = SM_WARPS * 32;
-  const bf16* wa = W + (int64_t)min(n0 + gid, p.N - 1) * p.K + k0;
-  const bf16* wb = W + (int64_t)min(n0 + gid + 8, p.N - 1) * p.K + k0;
-  uint4 va[SM_AHEAD], vb[SM_AHEAD];
-  const uint4 zero = make_uint4(0, 0, 0, 0);
-#pragma unroll
-  for (int u = 0; u < SM_AHEAD; ++u) {
-    const bool ok = k0 + u * STEP < p.K;
-    va[u] = ok ? ldg_stream16(wa + u * STEP) : zero;
-    vb[u] = ok ? ldg_stream16(wb + u * STEP) : zero;
+struct DecodeEpi {
+  EpiParams p;
+  struct Ahead {  // residual: a pair of features; QKV: the rotation and the ring's row
+    uint32_t r;
+    float2 cs;
+    int row;
+  };
+  __device__ __forceinline__ Ahead fetch(int t, int n, bool) const {
+    Ahead a = {0u, make_float2(1.f, 0.f), -1};
+    if constexpr (MODE == EPI_RESIDUAL) a.r = *reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint16_t*>(p.residual) + (int64_t)t * p.ld_out + n);
+    if constexpr (MODE == EPI_QKV_ROPE) {
+      if (n < p.q_dim + p.kv_dim) a.cs = *reinterpret_cast<const float2*>(p.rope + ((int64_t)p.positions[t] * (kHeadDim / 2) + ((n & (kHeadDim - 1)) >> 1)) * 2);
+      if (n >= p.q_dim && p.cache_rows != nullptr) a.row = p.cache_rows[t];
+    }
+    return a;
   }
-  pdl_trigger();
-  pdl_wait();
-  float c[4] = {0.f, 0.f, 0.f, 0.f};
-  const bf16* xr = X + (int64_t)min(gid, T - 1) * p.K + k0;  // rows past the end repeat the last one: their sums go nowhere
-  const int steps = (p.K + STEP - 1) / STEP;
-  for (int i = 0; i < steps; i += SM_AHEAD) {
-#pragma unroll
-    for (int u = 0; u < SM_AHEAD; ++u) {
-      const int k = (i + u) * STEP;
-      const uint4 vx = k0 + k < p.K ? *reinterpret_cast<const uint4*>(xr + k) : zero;
-      skinny_mma(c, va[u].x, vb[u].x, va[u].y, vb[u].y, vx.x, vx.y);
-      skinny_mma(c, va[u].z, vb[u].z, va[u].w, vb[u].w, vx.z, vx.w);
-      const bool more = k0 + k + SM_AHEAD * STEP < p.K;
-      va[u] = more ? ldg_stream16(wa + k + SM_AHEAD * STEP) : zero;
-      vb[u] = more ? ldg_stream16(wb + k + SM_AHEAD * STEP) : zero;
+  __device__ __forceinline__ void finish(int t, int n, float v0, float v1, bool, const Ahead& a) const {  // as epi_pair
+    const float y0 = round_bf16(v0), y1 = round_bf16(v1);
+    if constexpr (MODE == EPI_RESIDUAL) {
+      *reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(p.out) + (int64_t)t * p.ld_out + n) = pack_bf16x2(y0 + bf16lo(a.r), y1 + bf16hi(a.r));
+    } else if constexpr (MODE == EPI_QKV_ROPE) {
+      float re = y0, im = y1;
+      if (n < p.q_dim + p.kv_dim) ref_cmul(y0, y1, a.cs.x, a.cs.y, re, im);
+      const uint32_t packed = pack_bf16x2(re, im);
+      const int c = n < p.q_dim ? n : n < p.q_dim + p.kv_dim ? n - p.q_dim : n - p.q_dim - p.kv_dim;
+      void* const to = n < p.q_dim ? p.q_out : n < p.q_dim + p.kv_dim ? p.k_out : p.v_out;
+      *reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(to) + (int64_t)t * (n < p.q_dim ? p.q_dim : p.kv_dim) + c) = packed;
+      if (a.row >= 0) *reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(n < p.q_dim + p.kv_dim ? p.cache_k : p.cache_v) + (int64_t)a.row * p.kv_dim + c) = packed;
+    } else {
+      epi_pair<MODE>(p, t, n, v0, v1);
     }
   }
-  part[warp][gid][tig * 2] = c[0];
-  part[warp][gid][tig * 2 + 1] = c[1];
-  part[warp][gid + 8][tig * 2] = c[2];
-  part[warp][gid + 8][tig * 2 + 1] = c[3];
-  __syncthreads();
-  if (threadIdx.x < 64) {
-    const int t = threadIdx.x & 7, r = (threadIdx.x >> 3) * 2, n = n0 + r;
-    if (t < T && n < p.N) {
-      float s0 = 0.f, s1 = 0.f;
-#pragma unroll
-      for (int w = 0; w < SM_WARPS; ++w) {
-        s0 += part[w][r][t];
-        s1 += part[w][r + 1][t];
-      }
-      epi_pair<MODE>(p.epi, t, n, s0, s1);
-    }
-  }
-}
+};
 
+// false: not launched (an address off the 16-byte grid, odd sizes)
 template <int MODE>
-int launch_skinny_mma(const SkinnyParams& p, int T, cudaStream_t stream) {
-  MB_CHECK_ARG(p.K % 8 == 0 && p.N % 2 == 0, "skinny linear: K=%d must be a multiple of 8, N=%d even", p.K, p.N);
-  MB_CHECK_ARG((size_t)T * p.K * 2 <= 200 * 1024, "skinny linear: T*K too large (%d x %d)", T, p.K);  // the limit of both kernels
-  MB_CHECK_CUDA(launch_pdl(skinny_mma_kernel<MODE>, dim3((unsigned)ceil_div(p.N, 16)), dim3(SM_WARPS * 32), 0, stream, p, T));
-  return MB200_OK;
+bool launch_stream(const SkinnyParams& p, int T, cudaStream_t stream, int& rc) {
+  if (T > STREAM_MAX_T || p.K % 8 != 0 || p.N % 2 != 0 || (reinterpret_cast<uintptr_t>(p.x) | reinterpret_cast<uintptr_t>(p.w)) % 16 != 0) return false;
+  const DecodeEpi<MODE> epi{p.epi};
+  cudaError_t e = cudaSuccess;
+  bool done = false;
+  switch ((T + 7) / 8) {
+    case 1: done = stream_linear::launch<1>(p.x, p.K, p.w, T, p.N, p.K, epi, stream, e); break;
+    case 2: done = stream_linear::launch<2>(p.x, p.K, p.w, T, p.N, p.K, epi, stream, e); break;
+    case 3: done = stream_linear::launch<3>(p.x, p.K, p.w, T, p.N, p.K, epi, stream, e); break;
+    default: done = stream_linear::launch<4>(p.x, p.K, p.w, T, p.N, p.K, epi, stream, e); break;
+  }
+  rc = e == cudaSuccess ? MB200_OK : fail(MB200_E_CUDA, "stream linear: %s", cudaGetErrorString(e));
+  return done;
 }
 
 template <int MODE, bool NORM>

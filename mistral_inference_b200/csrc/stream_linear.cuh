@@ -3,13 +3,15 @@
 //
 // A CTA (one per SM) owns whole rows of W -- `rows` of them, a multiple of 8 with N / rows close to the number of SMs -- for all of K, so no sum crosses a CTA: there is
 // nothing to exchange and nobody to wait for at the end.  A producer thread keeps a ring of stages full by TMA: [rows x 64] blocks of W (128B-swizzled), `blocks` of them
-// along k so that a stage is 14 to 30 KB whatever `rows` is, and the same columns of x.  The weights of the whole first ring are requested before the wait for the predecessor (nobody writes
+// along k so that a stage is 14 to 32 KB whatever `rows` is (47 from 17 tokens on), and the same columns of x.  The weights of the whole first ring are requested before the wait for the predecessor (nobody writes
 // weights), x after it.  Two teams of eight warps take the stages in turn (one stage's latencies lie under the other's) and multiply on mma.sync (m16n8k16: 16 rows of W x 8 tokens):
 // warp w of a team takes row tile w % tiles and every (8 / tiles)-th pair of slices of 16 columns; the sums meet in shared memory, in a fixed order.
 //
 // Why not tiles of 128 rows cut along k (gemm_streamk.cuh): with N / 128 = 16 .. 48 tiles for 148 SMs three or four CTAs finish a tile together, and the exchange through
 // memory is 6 to 10 us at the end of every launch.  Why not the weights straight into registers (a CTA per 16 rows, which this replaces in layered decoders): a fragment's lanes read 64
 // bytes of each of 8 rows, 8 tag lookups an instruction, 4 to 5 TB/s, and x came out of L2 in every step.
+// What bounds it from 17 tokens on is mma.sync itself (7 tiles x 4 slices x 4 groups of tokens of a 13 KB stage take some 700 clocks, memory 600): 32 tokens 28672 x 5120 57 us, 24 tokens
+// 57, 8 tokens of that shape 49.  More warps or two row tiles a warp made it slower.
 // us a Linear in a chain of them, stored / added to the fp32 stream, that kernel and this one: 8 tokens 16384 x 2048 14.1 / 17.1, 12.9 / 12.8; 2048 x 8192 9.5 / 10.1, 8.4 / 8.2; 32768 x 2048
 // 24.9 / 30.1, 24.1 / 24.0 (5.6 TB/s); 2048 x 2048 2.7 / 3.2, 3.9 / 3.7; 16 tokens 28672 x 4096 57 / 155, 44 / 44.  Behind other kernels, whose ends its first ring covers, it gains more: a
 // step of 8 layers of width 2048, 8 sequences, 698 and 529.  With one team of warps 28672 x 4096 took 47.6 us instead of 40, with a ring of 100 KB 43.
@@ -24,7 +26,7 @@ namespace stream_linear {
 constexpr int TEAM = 8, TEAMS = 2, WARPS = TEAM * TEAMS, THREADS = 32 * (WARPS + 1), MAX_ROWS = 16 * TEAM, SUM_PITCH = 16 * WARPS + 4 /* a warp's stores meet no bank twice */;
 constexpr int MAX_STAGES = 24;
 static_assert(MAX_STAGES % TEAMS == 0, "a slot is always the same team's");
-constexpr int RING_BYTES = 190 * 1024, STAGE_BYTES = 30 * 1024;  // of W in a stage at most, unless one block is more
+constexpr int RING_BYTES = 180 * 1024;
 
 struct Shape {
     int M, N, K;
@@ -221,7 +223,7 @@ inline Shape shape_of(int M, int N, int K, int64_t pitch, int sms) {
     while (s.tiles * 16 < s.rows) s.tiles *= 2;
     const int kbs = (K + 63) / 64;
     s.blocks = 1;
-    while (!s.flat && s.blocks + 2 <= kbs && s.blocks < 7 && (s.blocks + 2) * s.rows * 128 <= STAGE_BYTES) s.blocks += 2;
+    while (!s.flat && s.blocks + 2 <= kbs && s.blocks < 7 && (s.blocks + 2) * (s.rows + 8 * NT) * 128 <= (NT > 2 ? 47 : 32) * 1024) s.blocks += 2;
     s.stages = RING_BYTES / ((s.rows + 8 * NT) * 128 * s.blocks);
     if (s.stages > MAX_STAGES) s.stages = MAX_STAGES;
     s.stages = s.stages / TEAMS * TEAMS;  // a slot is always the same team's: its waits follow every phase of the slot's barriers

@@ -773,3 +773,39 @@ def test_decode_linear_streams_whole_rows(M, N, K, pad):
         y, F = ref.bfloat16().double(), torch.nn.functional
         got = h.linear_swiglu(x.contiguous(), w, None)
         assert rel(got, F.silu(y[:, 0::2]) * y[:, 1::2]) < 2 ** -7
+
+
+@pytest.mark.parametrize("T", [2, 8, 9, 17, 24, 25, 32, 33])
+def test_decode_steps_linears_against_float64(T):
+    """Every step behind the Linears of a decode batch, at the edges of their token groups and one past the last: rotation and ring of q, k, v, gated unit, residual, logits."""
+    from mistral_inference_b200 import _abi
+
+    g = torch.Generator(device=DEV).manual_seed(T)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV)  # noqa: E731
+    D, H, KV, hd, F, rows = 640, 4, 2, 128, 1152, 40
+    ws = _abi.Workspace(_abi.workspace_bytes(64, D, H, KV, hd, F, D, 64), DEV)
+    x, nw = rnd(T, D).bfloat16(), (1 + rnd(D) / 8).bfloat16()
+    wqkv, w13, w2 = ((rnd(n, k) / k ** 0.5).bfloat16() for n, k in (((H + 2 * KV) * hd, D), (2 * F, D), (D, F)))
+    n = _abi.rmsnorm(x, nw, 1e-5).double()
+    pos = torch.randint(0, 100, (T,), device=DEV, generator=g).int()
+    ring = torch.randperm(rows, device=DEV, generator=g)[:T].int()
+    ring[0] = -1
+    ang = torch.rand(100, hd // 2, device=DEV, generator=g) * 6.28
+    rope = torch.stack((ang.cos(), ang.sin()), -1).contiguous()
+    q, k, v = (torch.empty(T, h * hd, dtype=torch.bfloat16, device=DEV) for h in (H, KV, KV))
+    ck, cv = (torch.zeros(rows, KV * hd, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    _abi.attn_qkv(x, nw, wqkv, rope, pos, q, k, v, ck, cv, ring, H, KV, hd, 1e-5, ws)
+    y = n @ wqkv.double().T
+    c, s = (t.double()[:, None] for t in (rope[pos.long(), :, 0], rope[pos.long(), :, 1]))
+    turn = lambda t: torch.stack((t[..., 0::2] * c - t[..., 1::2] * s, t[..., 0::2] * s + t[..., 1::2] * c), -1).flatten(1)  # noqa: E731
+    assert rel(q, turn(y[:, : H * hd].view(T, H, hd))) < 2 ** -7 and rel(k, turn(y[:, H * hd:(H + KV) * hd].view(T, KV, hd))) < 2 ** -7  # two roundings to bf16
+    assert rel(v, y[:, (H + KV) * hd:]) < 2 ** -8
+    there = ring[1:].long()
+    assert torch.equal(ck[there], k[1:]) and torch.equal(cv[there], v[1:]) and int((ck != 0).any(1).sum()) == T - 1
+    gate = torch.empty(T, F, dtype=torch.bfloat16, device=DEV)
+    _abi.ffn_gateup(x, nw, w13, gate, 1e-5, ws)
+    u = n @ w13.double().T
+    assert rel(gate, torch.nn.functional.silu(u[:, 0::2]) * u[:, 1::2]) < 2 ** -7
+    res, out = rnd(T, D).bfloat16(), torch.empty(T, D, dtype=torch.bfloat16, device=DEV)
+    _abi.linear_residual(gate, w2, res, out, ws)
+    assert rel(out, res.double() + gate.double() @ w2.double().T) < 2 ** -7
