@@ -137,7 +137,8 @@ def rmsnorm_pair(x32: torch.Tensor, w: torch.Tensor, w2: torch.Tensor, eps: floa
 
 
 SKINNY_MAX_ROWS = 8  # of fp32: more rows run on tensor cores
-PROMPT_GEMM_MIN_ROWS = 17  # fewer rows: this library's own kernel, which streams the weights past up to 16 tokens
+PROMPT_GEMM_MIN_ROWS = 17
+STREAM_MAX_ROWS = 32  # so many rows of bf16 run on this library's own kernel, which streams the weights past them: 20 tokens through two layers of width 2048 268 us, 185 with it
 
 
 def _prompt_gemm_ok(x: torch.Tensor, M: int, N: int, K: int) -> bool:
@@ -185,7 +186,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None
         out32 = torch.empty(M, N, dtype=torch.float32, device=x.device)
     else:
         out = torch.empty(M, N // 2 if epi == EPI_GLU else N, dtype=x.dtype, device=x.device)
-    if _prompt_gemm_ok(x, M, N, K) and _aligned(w, bias, out32) and epi in (EPI_STORE, EPI_RESIDUAL, EPI_RESIDUAL_SCALED, EPI_F32, EPI_GLU):
+    if M > STREAM_MAX_ROWS and _prompt_gemm_ok(x, M, N, K) and _aligned(w, bias, out32) and epi in (EPI_STORE, EPI_RESIDUAL, EPI_RESIDUAL_SCALED, EPI_F32, EPI_GLU):
         xc = x.contiguous()
         if _aligned(xc):
             _abi.layer_linear(xc, w, bias, out, out32, epi, n_act, limit, alpha)
@@ -321,7 +322,7 @@ def linear_swiglu(x: torch.Tensor, w: torch.Tensor, rowscale: Optional[torch.Ten
         assert rowscale.dtype == torch.float32 and rowscale.shape[0] == M and group > 0 and (N // 2 + group - 1) // group <= rowscale.shape[1]
         pitch = rowscale.shape[1]
     out = torch.empty(M, N // 2, dtype=x.dtype, device=x.device)
-    if _prompt_gemm_ok(x, M, N, K) and _aligned(x, w):
+    if M > STREAM_MAX_ROWS and _prompt_gemm_ok(x, M, N, K) and _aligned(x, w):
         _abi.layer_linear(x, w, None, out, None, EPI_GEGLU if gelu else EPI_SWIGLU, rowscale=rowscale, group=max(group, 1))
         return out
     if _linear_f32(x, w, None, out, None, EPI_GEGLU if gelu else EPI_SWIGLU, rowscale=rowscale, group=group):
@@ -662,7 +663,7 @@ def linear_glu(x: torch.Tensor, w: torch.Tensor, limit: float, alpha: float, row
         assert rowscale.dtype == torch.float32 and rowscale.shape[0] == M and group > 0 and (N // 2 + group - 1) // group <= rowscale.shape[1]
         pitch = rowscale.shape[1]
     out = torch.empty(M, N // 2, dtype=x.dtype, device=x.device)
-    if _prompt_gemm_ok(x, M, N, K) and _aligned(x, w):
+    if M > STREAM_MAX_ROWS and _prompt_gemm_ok(x, M, N, K) and _aligned(x, w):
         _abi.layer_linear(x, w, None, out, None, EPI_GLU, limit=limit, alpha=alpha, rowscale=rowscale, group=max(group, 1))
         return out
     if _linear_f32(x, w, None, out, None, EPI_GLU, limit=limit, alpha=alpha, rowscale=rowscale, group=group):
@@ -746,7 +747,7 @@ def linear_relu2(x: torch.Tensor, w: torch.Tensor, rowscale: Optional[torch.Tens
         assert rowscale.dtype == torch.float32 and rowscale.shape[0] == M and group > 0 and (N + group - 1) // group <= rowscale.shape[1]
         pitch = rowscale.shape[1]
     out = torch.empty(M, N, dtype=x.dtype, device=x.device)
-    if _prompt_gemm_ok(x, M, N, K) and _aligned(x, w):
+    if M > STREAM_MAX_ROWS and _prompt_gemm_ok(x, M, N, K) and _aligned(x, w):
         _abi.layer_linear(x, w, None, out, None, EPI_RELU2, rowscale=rowscale, group=max(group, 1))
         return out
     if _linear_f32(x, w, None, out, None, EPI_RELU2, rowscale=rowscale, group=group):

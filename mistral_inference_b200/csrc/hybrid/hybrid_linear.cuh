@@ -20,10 +20,12 @@
 // Linear); accumulation is fp32 in both modes.
 //
 // Kernels: `linear_tiled_mma` (bf16), `linear_f32_pair` (fp32, hybrid_linear_f32.cuh) and `linear_tiled_fma` (fp32, K < 16) for prompts, any shape; `linear_skinny` (M <= 8 rows, FMA,
-// one warp per pair of weight rows) and `stream_linear_kernel` (bf16, up to 16 rows, tensor cores) for decode: every weight byte is read
+// one warp per pair of weight rows) and `stream_linear_kernel` (bf16, up to 32 rows, tensor cores) for decode: every weight byte is read
 // once; `linear_decay_mma` for decays from a low rank.  The large aligned bf16 Linears of prompts go to the main
 // library's tcgen05 GEMMs, with these steps in their epilogue (see _abi_hybrid.linear).
 #pragma once
+#include <type_traits>
+
 #include "../stream_linear.cuh"
 #include "hybrid_common.cuh"
 
@@ -382,8 +384,8 @@ __global__ void __launch_bounds__(SK_WARPS * 32) linear_skinny(LinearArgs a) {
         }
 }
 
-// ------------------------------------------------------------------------------------------------ decode on tensor cores (bf16, 1..16 rows): ../stream_linear.cuh
-constexpr int SM_MAX_M = 16;
+// ------------------------------------------------------------------------------------------------ decode on tensor cores (bf16, 1..32 rows): ../stream_linear.cuh
+constexpr int SM_MAX_M = 32;
 
 struct StreamEpi {
     LinearArgs a;  // (bias: added here)
@@ -421,7 +423,9 @@ inline cudaError_t launch_linear(const LinearArgs& a, cudaStream_t st, void* scr
             cudaError_t e = cudaSuccess;
             StreamEpi epi{a, a.bias};
             epi.a.bias = nullptr;
-            if (a.M <= 8 ? stream_linear::launch<1>(a.x, a.x_pitch(), a.w, a.M, a.N, a.K, epi, st, e) : stream_linear::launch<2>(a.x, a.x_pitch(), a.w, a.M, a.N, a.K, epi, st, e)) return e;
+            auto go = [&](auto nt) { return stream_linear::launch<decltype(nt)::value>(a.x, a.x_pitch(), a.w, a.M, a.N, a.K, epi, st, e); };
+            if (a.M <= 8 ? go(std::integral_constant<int, 1>()) : a.M <= 16 ? go(std::integral_constant<int, 2>()) : a.M <= 24 ? go(std::integral_constant<int, 3>())
+                                                                                                                    : go(std::integral_constant<int, 4>())) return e;
         }
     }
     if (a.M <= SK_MAX_M) {
