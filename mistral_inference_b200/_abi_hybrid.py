@@ -552,9 +552,9 @@ def attn_decode_ok(q: torch.Tensor, H: int, G: int, d: int, e: int, maps: int = 
 
 
 def attn_decode_splits(B: int, G: int, W: int, n_sm: int = 148) -> int:
-    """CTAs per (sequence, key/value head) along the keys: two per SM over the batch, at least one round of 64 ring rows each (batch and ring size
-    only, so a captured decode graph stays valid as the context grows)."""
-    return int(max(1, min((2 * n_sm + B * G - 1) // (B * G), (W + 63) // 64, 64)))
+    """CTAs per (sequence, key/value head) along the keys: at most two per SM over the batch -- as many as run at once; a few more would run alone in a second round --, at
+    least one round of 64 ring rows each (batch and ring size only, so a captured decode graph stays valid as the context grows)."""
+    return int(max(1, min(2 * n_sm // (B * G), (W + 63) // 64, 64)))
 
 
 def attn_decode(q, cache_k, cache_v, positions, slots, out, B: int, W: int, H: int, G: int, d: int, e: int, scale: float, window: int, softcap: float = 0.0, sink=None,
