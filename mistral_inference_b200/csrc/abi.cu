@@ -12,6 +12,7 @@
 #include "gemm_mma.cuh"
 #include "gemm_pair.cuh"
 #include "gemm_streamk.cuh"
+#include "stream_tiles.cuh"
 #include "gemm_tcgen05.cuh"
 #include "moe.cuh"
 #include "sampling.cuh"
@@ -28,7 +29,8 @@ constexpr int64_t MB200_ATTN_FIRST_MIN = 128, MB200_ATTN_PORTION_MIN = 16;
 
 constexpr size_t kWsHeader = 64 * 1024;  // persistent, zero-initialised by the caller once: self-resetting counters
 // behind the header: partial sums of the stream-K kernel or of the prompt GEMM's cut tiles (both with their flags in the header)
-constexpr size_t kWsPartial = TG_CUT_BYTES > SK_PARTIAL_BYTES ? TG_CUT_BYTES : SK_PARTIAL_BYTES;
+constexpr size_t kWsPartial = ST_SLOT_BYTES;
+static_assert(kWsPartial >= TG_CUT_BYTES && kWsPartial >= SK_PARTIAL_BYTES, "one region for the partial sums of every kernel");
 static_assert(2 * TG_MAX_CUTS <= SK_MAX_CTAS, "the flags of cut tiles use those of the stream-K kernel");
 inline size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
@@ -37,6 +39,11 @@ static int run_rmsnorm(const void* x, const void* w, void* out, int64_t T, int64
   if (T == 0) return MB200_OK;
   MB_CHECK_CUDA(launch_pdl(rmsnorm_kernel, dim3((unsigned)T), dim3(256), 0, st, (const uint4*)x, (const uint4*)w, (uint4*)out, (int)dim, eps));
   return MB200_OK;
+}
+
+static int sm_count() {
+  int dev = 0, sms = 0;
+  return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess ? sms : 1;
 }
 
 template <int MODE>
@@ -75,6 +82,8 @@ static int run_linear(const void* x, const void* norm_w, const void* w, const Ep
   g.N = (int)N;
   g.K = (int)K;
   g.epi = epi;
+  if (workspace != nullptr && workspace_bytes >= kWsHeader + kWsPartial && stream_tiles_bytes(T, N, K, sm_count()) > 0)
+    return launch_stream_tiles<MODE>(g, sm_count(), (uint8_t*)workspace + kWsHeader, st);
   if (streamk_eligible(T, N, K)) return launch_streamk<MODE>(g, workspace, workspace_bytes, kWsHeader, st);  // decode-sized batches: HBM-bound
   if (tcgen05_gemm_eligible(T, N, K)) {
     const bool cuts = workspace != nullptr && workspace_bytes >= kWsHeader + kWsPartial;
@@ -542,6 +551,7 @@ int mb200_layer_linear(const void* x, const void* w, const void* bias, void* out
   g.K = (int)K;
   g.epi = e;
   unsigned* flags = nullptr;
+  if (scratch != nullptr && stream_tiles_bytes(T, N, K, sm_count()) > 0) return launch_stream_tiles<EPI_LAYER>(g, sm_count(), scratch, (cudaStream_t)stream);
   if (T < TG_BM) {  // few rows: the weight-streaming stream-K kernel, its flags in front of its partial sums
     MB_CHECK_ARG(scratch != nullptr, "layer_linear: fewer than 128 rows need scratch");
     MB_CHECK_CUDA(cudaMemsetAsync((uint8_t*)scratch + SK_FLAGS_OFFSET, 0, SK_MAX_CTAS * sizeof(unsigned), (cudaStream_t)stream));
@@ -555,6 +565,8 @@ int mb200_layer_linear(const void* x, const void* w, const void* bias, void* out
 }
 
 size_t mb200_layer_linear_scratch(int64_t T, int64_t N, int64_t K) {
+  const size_t slots = stream_tiles_bytes(T, N, K, sm_count());
+  if (slots > 0) return slots;
   if (T < TG_BM) return kWsHeader + SK_PARTIAL_BYTES;
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;

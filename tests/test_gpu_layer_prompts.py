@@ -809,3 +809,25 @@ def test_decode_steps_linears_against_float64(T):
     res, out = rnd(T, D).bfloat16(), torch.empty(T, D, dtype=torch.bfloat16, device=DEV)
     _abi.linear_residual(gate, w2, res, out, ws)
     assert rel(out, res.double() + gate.double() @ w2.double().T) < 2 ** -7
+
+
+@pytest.mark.parametrize("T,N,K", [(33, 128, 64), (48, 384, 128), (49, 1024, 640), (64, 6144, 192), (65, 2176, 1024), (112, 640, 2048), (113, 4096, 320), (127, 20480, 128), (128, 256, 8192),
+                                   (129, 1152, 8256), (192, 128, 8192), (193, 1024, 8192), (256, 4096, 8192)])
+def test_linears_over_streamed_tiles(T, N, K):
+    """Fewer and more units than SMs, tiles in one piece and in many, tokens at the edges of the MMA's columns and of the accumulators: against float64, for the dense model's steps (bf16
+    results: 2^-8) and a layered decoder's (fp32 residual and logits); twice the same bits."""
+    from mistral_inference_b200 import _abi, _abi_hybrid as h
+
+    g = torch.Generator(device=DEV).manual_seed(T + N + K)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV)  # noqa: E731
+    x, w, b, res, base = rnd(T, K).bfloat16(), (rnd(N, K) / K ** 0.5).bfloat16(), rnd(N).bfloat16(), rnd(T, N).bfloat16(), rnd(T, N)
+    ref, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T * (2 * K * 2.0 ** -24)
+    ws, out = _abi.Workspace(_abi.workspace_bytes(T, K, 1, 1, 128, N, N, 8), DEV), torch.empty(T, N, dtype=torch.bfloat16, device=DEV)
+    _abi.linear_residual(x, w, res, out, ws)
+    assert ((out.double() - res.double() - ref).abs() <= 2 ** -8 * (ref.abs() + (ref + res.double()).abs()) + size).all()
+    f32 = h.linear(x, w, b, epi=h.EPI_F32)
+    assert ((f32.double() - ref - b.double()).abs() <= size + 2.0 ** -23 * (ref + b.double()).abs()).all() and torch.equal(f32, h.linear(x, w, b, epi=h.EPI_F32))
+    got = h.linear(x, w, None, epi=h.EPI_RESIDUAL, residual=base.clone())
+    assert ((got.double() - base.double() - ref).abs() <= 2 ** -8 * ref.abs() + size + 2.0 ** -23 * (base.double() + ref).abs()).all()
+    y = ref.bfloat16().double()
+    assert rel(h.linear_swiglu(x, w), torch.nn.functional.silu(y[:, 0::2]) * y[:, 1::2]) < 2 ** -7
