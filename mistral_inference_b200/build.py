@@ -72,7 +72,7 @@ def build_hybrid(force: bool = False) -> Path:
     """libmb200_hybrid.so: the kernels of layered decoders (csrc/hybrid/), a separate, small library so that a fresh checkout
     that only serves such a model compiles only them (seconds).  Safe when several processes start at once: the output is
     written under a private name and renamed."""
-    files = sorted(HYBRID_SRC.glob("*.cu")) + sorted(HYBRID_SRC.glob("*.cuh")) + sorted(HYBRID_SRC.glob("*.h")) + [CSRC / "stream_linear.cuh"] + sorted((PKG.parent / "include").glob("mistral_b200_hybrid*.h"))
+    files = sorted(HYBRID_SRC.glob("*.cu")) + sorted(HYBRID_SRC.glob("*.cuh")) + sorted(HYBRID_SRC.glob("*.h")) + [CSRC / "stream_linear.cuh", CSRC / "device_info.cuh"] + sorted((PKG.parent / "include").glob("mistral_b200_hybrid*.h"))
     h = hashlib.sha256()
     for f in files:
         h.update(f.name.encode())

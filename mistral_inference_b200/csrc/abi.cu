@@ -41,10 +41,7 @@ static int run_rmsnorm(const void* x, const void* w, void* out, int64_t T, int64
   return MB200_OK;
 }
 
-static int sm_count() {
-  int dev = 0, sms = 0;
-  return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess ? sms : 1;
-}
+static int sm_count() { return device_info::sm_count(); }
 
 template <int MODE>
 static int run_linear(const void* x, const void* norm_w, const void* w, const EpiParams& epi, int64_t T, int64_t N, int64_t K, float eps,
@@ -278,7 +275,7 @@ int mb200_attn_prefill(const void* q, const void* k_new, const void* v_new, cons
   p.scale_log2 = 0.08838834764831845f * 1.4426950408889634f;
   const int64_t span = causal ? max_seqlen : T;
   const dim3 grid((unsigned)ceil_div(span, AP_BQ), (unsigned)n_heads, (unsigned)(causal ? B : 1));
-  MB_CHECK_CUDA(cudaFuncSetAttribute(attn_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AP_SMEM));
+  MB_CHECK_CUDA(device_info::allow_shared<attn_prefill_kernel>(AP_SMEM));
   attn_prefill_kernel<<<grid, AP_THREADS, AP_SMEM, (cudaStream_t)stream>>>(p);
   MB_CHECK_LAUNCH("attn_prefill_kernel");
   return MB200_OK;
@@ -568,8 +565,7 @@ size_t mb200_layer_linear_scratch(int64_t T, int64_t N, int64_t K) {
   const size_t slots = stream_tiles_bytes(T, N, K, sm_count());
   if (slots > 0) return slots;
   if (T < TG_BM) return kWsHeader + SK_PARTIAL_BYTES;
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+  const int sms = sm_count();
   if (T <= TG_BM || sms < 2 || !pairs_fill(T, N, K, sms / 2, true)) return 0;
   const long long tiles = (long long)pair_token_tiles(T) * ceil_div(N, GP_ROWS);
   return cut_plan(tiles, (int)(K / TG_BK), sms / 2, TG_MAX_CUTS).cut_pairs > 0 ? TG_CUT_BYTES + 2 * TG_MAX_CUTS * sizeof(unsigned) : 0;

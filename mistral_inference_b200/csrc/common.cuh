@@ -9,6 +9,7 @@
 #include <cstdlib>
 
 #include "../../include/mistral_b200.h"
+#include "device_info.cuh"
 
 namespace mb200 {
 

@@ -565,7 +565,6 @@ __global__ void __launch_bounds__(GP_THREADS, 1)
 // ---- host -------------------------------------------------------------------------------------------------------------
 template <class Kernel, class... Args>
 int launch_pairs(Kernel kernel, int clusters, cudaStream_t stream, const Args&... args) {
-  MB_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2u * (unsigned)clusters);
   cfg.blockDim = dim3(GP_THREADS);
@@ -613,6 +612,7 @@ int launch_gemm_pair(const GemmParams& g, int sms, cudaStream_t stream, void* sc
   rc = make_tensor_map_2d(&map_w, g.w, g.N, g.K, TG_BM);
   if (rc) return rc;
   const long long tiles = (long long)p.tok_tiles * ceil_div(g.N, GP_ROWS);
+  MB_CHECK_CUDA(device_info::allow_shared<gemm_pair_kernel<MODE>>(GP_SMEM));
   const bool cut = scratch != nullptr && cut_plan(tiles, g.K / TG_BK, p.units, TG_MAX_CUTS).cut_pairs > 0;
   return launch_pairs(gemm_pair_kernel<MODE>, cut || tiles > p.units ? p.units : (int)tiles, stream, map_a, map_w, p);  // (cut: item s of the last round runs on cluster s, so all of them are there)
 }
@@ -620,9 +620,8 @@ int launch_gemm_pair(const GemmParams& g, int sms, cudaStream_t stream, void* sc
 // T >= TG_BM
 template <int MODE>
 int launch_gemm_tcgen05_prompt(const GemmParams& g, cudaStream_t stream, void* scratch = nullptr, unsigned* flags = nullptr) {
-  int dev = 0, sms = 0;
-  MB_CHECK_CUDA(cudaGetDevice(&dev));
-  MB_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const int sms = device_info::sm_count();
+  if (sms == 0) return fail(MB200_E_CUDA, "no device");
   const int forced = tcgen05_forced_bn();
   const bool pairs = tcgen05_cluster_enabled() && g.N % 128 == 0;
   if ((forced == 128 || forced == 192 || forced == 256) && g.N % forced == 0) {
@@ -639,9 +638,8 @@ int launch_gemm_tcgen05_prompt(const GemmParams& g, cudaStream_t stream, void* s
 template <int MODE>
 int launch_gemm_tcgen05(const GemmParams& g, cudaStream_t stream, void* scratch, unsigned* flags) {
   if (g.T >= TG_BM) return launch_gemm_tcgen05_prompt<MODE>(g, stream, scratch, flags);
-  int dev = 0, sms = 0;
-  MB_CHECK_CUDA(cudaGetDevice(&dev));
-  MB_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const int sms = device_info::sm_count();
+  if (sms == 0) return fail(MB200_E_CUDA, "no device");
   return launch_gemm_tcgen05_small<MODE>(g, sms, stream);
 }
 

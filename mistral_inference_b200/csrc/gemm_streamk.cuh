@@ -351,9 +351,8 @@ inline bool streamk_eligible(int64_t T, int64_t N, int64_t K) {
 template <int MODE, int TA>
 int launch_streamk_ta(const GemmParams& g, void* workspace, size_t workspace_bytes, size_t header, cudaStream_t stream) {
   using Cfg = TgCfg<SK_BN, TA>;
-  int dev = 0, sms = 0;
-  MB_CHECK_CUDA(cudaGetDevice(&dev));
-  MB_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  int sms = device_info::sm_count();
+  if (sms == 0) return fail(MB200_E_CUDA, "no device");
   if (sms > SK_MAX_CTAS) sms = SK_MAX_CTAS;
   if (workspace == nullptr || workspace_bytes < header + SK_PARTIAL_BYTES) return fail(MB200_E_WORKSPACE, "stream-K gemm: workspace %zu < %zu", workspace_bytes, header + SK_PARTIAL_BYTES);
   CUtensorMap map_a, map_w;
@@ -370,7 +369,7 @@ int launch_streamk_ta(const GemmParams& g, void* workspace, size_t workspace_byt
   p.flags = reinterpret_cast<unsigned*>((uint8_t*)workspace + SK_FLAGS_OFFSET);
   const long long units = (long long)(g.N / SK_BN) * (g.K / TG_BK);
   const int grid = (int)(units < sms ? units : sms);
-  MB_CHECK_CUDA(cudaFuncSetAttribute(gemm_streamk_kernel<MODE, TA>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
+  MB_CHECK_CUDA((device_info::allow_shared<gemm_streamk_kernel<MODE, TA>>(Cfg::kSmem)));
   MB_CHECK_CUDA(launch_pdl(gemm_streamk_kernel<MODE, TA>, dim3((unsigned)grid), dim3(TG_THREADS), (size_t)Cfg::kSmem, stream, map_a, map_w, p));
   return MB200_OK;
 }

@@ -519,7 +519,7 @@ int launch_gemm_tcgen05_bn(const GemmParams& g, int sms, cudaStream_t stream) {
   p.K = g.K;
   p.epi = g.epi;
   const int tiles = ceil_div(g.T, TG_BM) * (g.N / BN);
-  MB_CHECK_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<MODE, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+  MB_CHECK_CUDA((device_info::allow_shared<gemm_tcgen05_kernel<MODE, BN>>(kSmem)));
   gemm_tcgen05_kernel<MODE, BN><<<tiles < sms ? tiles : sms, TG_THREADS, kSmem, stream>>>(map_a, map_w, p);
   MB_CHECK_LAUNCH("gemm_tcgen05_kernel");
   return MB200_OK;
@@ -562,7 +562,7 @@ int launch_gemm_tcgen05_small_bn(const GemmParams& g, int sms, cudaStream_t stre
   p.K = g.K;
   p.epi = g.epi;
   const int tiles = g.N / BN;
-  MB_CHECK_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<MODE, BN, TA>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
+  MB_CHECK_CUDA((device_info::allow_shared<gemm_tcgen05_kernel<MODE, BN, TA>>(Cfg::kSmem)));
   gemm_tcgen05_kernel<MODE, BN, TA><<<tiles < sms ? tiles : sms, TG_THREADS, Cfg::kSmem, stream>>>(map_a, map_w, p);
   MB_CHECK_LAUNCH("gemm_tcgen05_kernel<small batch>");
   return MB200_OK;

@@ -609,8 +609,8 @@ inline FtEncode ft_encode() {  // the driver's entry point through the runtime: 
     return fn;
 }
 inline int ft_units() {  // pairs of SMs
-    int dev = 0, sms = 0;
-    return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms >= 2 ? sms / 2 : 1;
+    const int sms = device_info::sm_count();
+    return sms >= 2 ? sms / 2 : 1;
 }
 
 // scratch: counters, slots, the parts of x
@@ -652,7 +652,7 @@ inline cudaError_t launch_f32_tokens(const LinearArgs& a, const F32Plan& p, int 
                                a.x_pitch(), a.M, a.K, s.kp, parts, args.counters, (int)s.counters);
     if (e) return e;
     auto kernel = vec ? linear_f32_pair<true> : linear_f32_pair<false>;
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FT_SMEM);
+    e = vec ? device_info::allow_shared<linear_f32_pair<true>>(FT_SMEM) : device_info::allow_shared<linear_f32_pair<false>>(FT_SMEM);
     if (e) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2u * (unsigned)p.clusters);

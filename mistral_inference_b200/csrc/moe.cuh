@@ -409,7 +409,7 @@ int launch_grouped_bn(const void* a, int64_t rows_cap, int64_t K, int64_t N, con
   p.N = (int)N;
   p.K = (int)K;
   p.epi = epi;
-  MB_CHECK_CUDA(cudaFuncSetAttribute(gemm_tcgen05_grouped_kernel<MODE, BN, TA>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
+  MB_CHECK_CUDA((device_info::allow_shared<gemm_tcgen05_grouped_kernel<MODE, BN, TA>>(Cfg::kSmem)));
   gemm_tcgen05_grouped_kernel<MODE, BN, TA><<<sms, TG_THREADS, Cfg::kSmem, stream>>>(map_a, maps, p, plan);
   MB_CHECK_LAUNCH("gemm_tcgen05_grouped_kernel");
   return MB200_OK;
@@ -430,6 +430,7 @@ int launch_grouped_pair(const CUtensorMap& map_a, const MoeWeightMaps& maps, int
   p.w_k = (int)w_k;
   p.units = sms / 2;
   if (K >= GP_DRAW_MIN_K) p.draw = reinterpret_cast<unsigned*>(const_cast<int32_t*>(plan) + 7);
+  MB_CHECK_CUDA(device_info::allow_shared<gemm_pair_grouped_kernel<MODE>>(GP_SMEM));
   return launch_pairs(gemm_pair_grouped_kernel<MODE>, p.units, stream, map_a, maps, p, plan);
 }
 
@@ -455,7 +456,7 @@ int launch_grouped_streamk(const void* a, int64_t rows_cap, int64_t K, int64_t N
   p.epi = epi;
   p.partials = reinterpret_cast<float*>((uint8_t*)workspace + header);
   p.flags = reinterpret_cast<unsigned*>((uint8_t*)workspace + SK_FLAGS_OFFSET);
-  MB_CHECK_CUDA(cudaFuncSetAttribute(gemm_streamk_grouped_kernel<MODE, TA>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
+  MB_CHECK_CUDA((device_info::allow_shared<gemm_streamk_grouped_kernel<MODE, TA>>(Cfg::kSmem)));
   MB_CHECK_CUDA(launch_pdl(gemm_streamk_grouped_kernel<MODE, TA>, dim3((unsigned)sms), dim3(TG_THREADS), (size_t)Cfg::kSmem, stream, map_a, maps, p, plan));
   return MB200_OK;
 }
@@ -463,9 +464,8 @@ int launch_grouped_streamk(const void* a, int64_t rows_cap, int64_t K, int64_t N
 template <int MODE>
 int launch_grouped(const void* a, int64_t rows_cap, int64_t K, int64_t N, const void* const* w_host, int E, int est_mtiles, int tile_rows,
                    const int32_t* plan, const EpiParams& epi, void* workspace, size_t workspace_bytes, size_t header, cudaStream_t stream) {
-  int dev = 0, sms = 0;
-  MB_CHECK_CUDA(cudaGetDevice(&dev));
-  MB_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const int sms = device_info::sm_count();
+  if (sms == 0) return fail(MB200_E_CUDA, "no device");
   MB_CHECK_ARG(K % TG_BK == 0 && N % 32 == 0, "grouped gemm: K=%lld must be a multiple of 64, N=%lld of 32", (long long)K, (long long)N);
   if (tile_rows < 128 && streamk_eligible(tile_rows, N, K)) {
     if (tile_rows == 32) return launch_grouped_streamk<MODE, 32>(a, rows_cap, K, N, w_host, E, plan, epi, workspace, workspace_bytes, header, sms, stream);
@@ -584,9 +584,8 @@ __global__ void __launch_bounds__(256) layer_moe_combine_kernel(const float4* ro
 // w: rows x cols, expert e at row e * w_n, column e * w_k.  N % 128 == 0, K % 64 == 0.
 inline int launch_grouped_packed(const void* a, int64_t rows_cap, int64_t K, int64_t N, const void* w, int64_t w_rows, int64_t w_cols, int64_t w_n, int64_t w_k,
                                  int64_t pairs, int64_t E, const int32_t* plan, const EpiParams& epi, cudaStream_t stream) {
-  int dev = 0, sms = 0;
-  MB_CHECK_CUDA(cudaGetDevice(&dev));
-  MB_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const int sms = device_info::sm_count();
+  if (sms == 0) return fail(MB200_E_CUDA, "no device");
   CUtensorMap map_a;
   MoeWeightMaps maps;
   int rc = make_tensor_map_2d(&map_a, a, rows_cap, K, TG_BM);
@@ -606,7 +605,7 @@ inline int launch_grouped_packed(const void* a, int64_t rows_cap, int64_t K, int
   p.epi = epi;
   p.w_n = (int)w_n;
   p.w_k = (int)w_k;
-  MB_CHECK_CUDA(cudaFuncSetAttribute(gemm_tcgen05_grouped_kernel<EPI_LAYER, 128, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
+  MB_CHECK_CUDA((device_info::allow_shared<gemm_tcgen05_grouped_kernel<EPI_LAYER, 128, 128>>(Cfg::kSmem)));
   gemm_tcgen05_grouped_kernel<EPI_LAYER, 128, 128><<<sms, TG_THREADS, Cfg::kSmem, stream>>>(map_a, maps, p, plan);
   MB_CHECK_LAUNCH("gemm_tcgen05_grouped_kernel<layer>");
   return MB200_OK;

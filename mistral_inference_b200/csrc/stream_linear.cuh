@@ -21,6 +21,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "device_info.cuh"
+
 namespace stream_linear {
 
 constexpr int TEAM = 8, TEAMS = 2, WARPS = TEAM * TEAMS, THREADS = 32 * (WARPS + 1), MAX_ROWS = 16 * TEAM, SUM_PITCH = 16 * WARPS + 4 /* a warp's stores meet no bank twice */;
@@ -233,11 +235,9 @@ inline Shape shape_of(int M, int N, int K, int64_t pitch, int sms) {
 // x rows `pitch` elements apart; K % 8 == 0, pitch % 8 == 0, both 16-byte aligned.  false: no tensor maps here
 template <int NT, class Epi>
 inline bool launch(const void* x, int64_t pitch, const void* w, int M, int N, int K, const Epi& epi, cudaStream_t st, cudaError_t& e) {
-    int dev = 0, sms = 0;
-    e = cudaGetDevice(&dev);
-    if (!e) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e) return true;
-    if (!encode()) return false;
+    e = cudaSuccess;
+    const int sms = device_info::sm_count();
+    if (sms == 0 || !encode()) return false;
     const Shape s = shape_of<NT>(M, N, K, pitch, sms);
     CUtensorMap map_x, map_w;
     if (!make_map(&map_x, x, M, K, pitch, 8 * NT, s.blocks, s.flat) || !make_map(&map_w, w, N, K, K, s.rows, s.blocks, s.flat)) return false;
@@ -245,7 +245,7 @@ inline bool launch(const void* x, int64_t pitch, const void* w, int M, int N, in
     // (a fragment of the last tile may reach past the stage's rows of W, into what follows them: its sums go nowhere)
     const size_t smem = 1024 + (size_t)s.stages * (s.rows + 8 * NT) * 128 * s.blocks + sizeof(float) * 8 * NT * SUM_PITCH;
     auto kernel = stream_linear_kernel<NT, Epi>;
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = device_info::allow_shared<stream_linear_kernel<NT, Epi>>(RING_BYTES + 1024 + (int)sizeof(float) * 8 * NT * SUM_PITCH);
     if (e) return true;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(units < sms ? units : sms));

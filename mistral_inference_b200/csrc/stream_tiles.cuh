@@ -185,7 +185,7 @@ inline bool stream_tiles_better(int64_t T, int64_t N, int64_t K) { return T < TG
 // bytes of slots, 0: not for this kernel
 inline size_t stream_tiles_bytes(int64_t T, int64_t N, int64_t K, int sms) {
   const char* e = getenv("MB200_STREAMK");
-  if ((e != nullptr && e[0] == '0') || T < 1 || !stream_tiles_better(T, N, K) || N % ST_ROWS != 0 || K % TG_BK != 0) return 0;
+  if (sms < 1 || (e != nullptr && e[0] == '0') || T < 1 || !stream_tiles_better(T, N, K) || N % ST_ROWS != 0 || K % TG_BK != 0) return 0;
   const int64_t tiles = N / ST_ROWS, units = tiles * (K / TG_BK), grid = units < sms ? units : sms;
   const size_t bytes = (size_t)(grid + tiles - 1) * st_piece(T) * sizeof(float);
   return bytes <= ST_SLOT_BYTES ? bytes : 0;
@@ -211,7 +211,7 @@ int launch_stream_tiles(const GemmParams& g, int sms, void* slots, cudaStream_t 
   rc = make_tensor_map_2d(&map_w, g.w, g.N, g.K, ST_ROWS);
   if (rc) return rc;
   const size_t smem = (size_t)p.stages * stage_bytes + 1024;
-  MB_CHECK_CUDA(cudaFuncSetAttribute(stream_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  MB_CHECK_CUDA(device_info::allow_shared<stream_tiles_kernel>(ST_RING + 1024));
   MB_CHECK_CUDA(launch_pdl(stream_tiles_kernel, dim3((unsigned)p.grid), dim3(ST_THREADS), smem, stream, map_a, map_w, p));
   const long long threads = (long long)(g.N / 32) * g.T;
   MB_CHECK_CUDA(launch_pdl(stream_tiles_combine_kernel<MODE>, dim3((unsigned)((threads + SC_THREADS - 1) / SC_THREADS)), dim3(SC_THREADS), 0, stream, p));
