@@ -26,8 +26,6 @@ _SIGNATURES = {
     "mbh_rmsnorm": (c_int, [P, P, P, P, P, I, I, F, F, c_int, P]),
     "mbh_linear_decay": (c_int, [P, I, P, P, P, I, P, I, I, I, c_int, P]),
     "mbh_linear": (c_int, [P, I, P, P, P, P, I, I, I, c_int, I, F, F, c_int, P]),
-    "mbh_linear_scratch": (I, [I, I, I, c_int]),
-    "mbh_linear_any": (c_int, [P, I, P, P, P, P, I, I, I, c_int, I, F, F, P, I, I, P, P, I, c_int, P]),
     "mbh_attn_prep": (c_int, [P, P, P, P, P, P, P, P, P, P, c_int, I, I, I, I, I, F, F, I, c_int, P]),
     "mbh_attn_bias": (c_int, [P, P, P, P, I, P, P, P, P, I, I, I, I, I, I, I, F, I, I, P, c_int, P]),
     "mbh_lightning_scan": (c_int, [P, P, P, P, P, P, P, I, I, I, I, c_int, P]),
@@ -69,6 +67,10 @@ _SIGNATURES = {
     "mbh_delta_step": (c_int, [P, I, I, I, P, I, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, F, c_int, P]),
     "mbh_rows_axpy": (c_int, [P, P, P, I, I, I, I, c_int, P]),
 }
+_LINEAR_SIGNATURES = {  # mistral_b200_hybrid_linear.h
+    "mbh_linear_scratch": (I, [I, I, I, c_int]),
+    "mbh_linear_any": (c_int, [P, I, P, P, P, P, I, I, I, c_int, I, F, F, P, I, I, P, P, I, c_int, P]),
+}
 
 
 def lib() -> ctypes.CDLL:
@@ -76,7 +78,7 @@ def lib() -> ctypes.CDLL:
     if _lib is None:
         path = build.build_hybrid()
         handle = ctypes.CDLL(str(path))
-        for name, (restype, argtypes) in _SIGNATURES.items():
+        for name, (restype, argtypes) in {**_SIGNATURES, **_LINEAR_SIGNATURES}.items():
             fn = getattr(handle, name)
             fn.restype, fn.argtypes = restype, argtypes
         if handle.mbh_abi_version() != ABI_VERSION:
@@ -143,7 +145,7 @@ STREAM_MAX_ROWS = 32  # so many rows of bf16 run on this library's own kernel, w
 
 def _prompt_gemm_ok(x: torch.Tensor, M: int, N: int, K: int) -> bool:
     """Large bf16 Linears of prompts go to the main library's tcgen05 GEMMs (`_abi.layer_linear`: the step after the Linear is the
-    epilogue; below 128 rows the stream-K kernel, above the persistent one) when it is built and the shape fits their tiles (K % 64 == 0,
+    epilogue; up to 128 rows tiles streamed in one range a CTA, above the persistent kernels) when it is built and the shape fits their tiles (K % 64 == 0,
     N % 128 == 0); everything else runs on this library's own kernels.  A checkout that has only libmb200_hybrid.so never builds the main
     library for this."""
     return (x.dtype == torch.bfloat16 and M >= PROMPT_GEMM_MIN_ROWS and K % 64 == 0 and N % 128 == 0 and os.environ.get("MB200_HYBRID_GEMM", "1") != "0"
