@@ -28,7 +28,7 @@ static unsigned long long* g_mk_prof_bar = nullptr;  // debug: decode megakernel
 constexpr int64_t MB200_ATTN_FIRST_MIN = 128, MB200_ATTN_PORTION_MIN = 16;
 
 constexpr size_t kWsHeader = 64 * 1024;  // persistent, zero-initialised by the caller once: self-resetting counters
-// behind the header: partial sums of the stream-K kernel or of the prompt GEMM's cut tiles (both with their flags in the header)
+// behind the header: the slots of streamed tiles, or partial sums of the stream-K kernel or of the prompt GEMM's cut tiles (these two with their flags in the header)
 constexpr size_t kWsPartial = ST_SLOT_BYTES;
 static_assert(kWsPartial >= TG_CUT_BYTES && kWsPartial >= SK_PARTIAL_BYTES, "one region for the partial sums of every kernel");
 static_assert(2 * TG_MAX_CUTS <= SK_MAX_CTAS, "the flags of cut tiles use those of the stream-K kernel");
@@ -549,7 +549,7 @@ int mb200_layer_linear(const void* x, const void* w, const void* bias, void* out
   g.epi = e;
   unsigned* flags = nullptr;
   if (scratch != nullptr && stream_tiles_bytes(T, N, K, sm_count()) > 0) return launch_stream_tiles<EPI_LAYER>(g, sm_count(), scratch, (cudaStream_t)stream);
-  if (T < TG_BM) {  // few rows: the weight-streaming stream-K kernel, its flags in front of its partial sums
+  if (T < TG_BM) {  // few rows whose slots would take too much: the stream-K kernel, its flags in front of its partial sums
     MB_CHECK_ARG(scratch != nullptr, "layer_linear: fewer than 128 rows need scratch");
     MB_CHECK_CUDA(cudaMemsetAsync((uint8_t*)scratch + SK_FLAGS_OFFSET, 0, SK_MAX_CTAS * sizeof(unsigned), (cudaStream_t)stream));
     return launch_streamk<EPI_LAYER>(g, scratch, kWsHeader + SK_PARTIAL_BYTES, kWsHeader, (cudaStream_t)stream);

@@ -1,11 +1,11 @@
-// Weight-streaming GEMM for decode-sized batches (5 <= T <= 128 tokens):  C[T, N] = A[T, K] * W[N, K]^T, bound by HBM.
+// Weight-streaming GEMM for decode-sized batches (T <= 128 tokens):  C[T, N] = A[T, K] * W[N, K]^T, bound by HBM: the experts of a mixture's decode step, and dense matrices whose sums
+// have no room in the slots of stream_tiles.cuh (a head of 131072 rows from 48 tokens on).  Up to 32 tokens dense Linears run on stream_linear.cuh.
 //
 // At these sizes the step reads every weight byte once and does ~2T flop per byte: the kernel's only job is to keep all 148 SMs
 // pulling their share of W at the HBM rate.  Two measured facts shape it (B200, Nemo-12B shapes, batch 32):
 //   * tile width: a W stage of [128 rows x 64] = 16 KB streams at the full HBM rate (lm head: 1.34 GB in 205 us), [64 x 64] gets
 //     ~40 % and [32 x 64] ~26 %: per stage the one-thread TMA producer and the one-thread MMA issuer each spend a few hundred
 //     cycles, so a stage must carry >= 16 KB.  Tiles are therefore always 128 wide;
-//   * N / 128 tiles do not divide over 148 SMs (wo of Nemo: 40 tiles; gate/up: 224 = 1.5 rounds), so the work is cut stream-K
 //   * N / 128 tiles do not divide over 148 SMs: the (tile, k-block) units of the whole problem are one sequence, and CTA c takes the c-th contiguous 1/G of
 //     it -- every SM streams the same number of bytes (+- one 16 KB stage) in one pass, whatever N and K are.
 // CTAs are counted from the launch's last block (split_schedule.cuh).  A CTA's range covers the tail of one tile, some whole tiles and the head of another (or, when tiles are longer than ranges,
