@@ -145,6 +145,71 @@ struct AttnPrepArgs {
     float eps, temp_coef; int temp_every;  // temperature 1 + coef * ln(floor((p + 1) / every) + 1); every == 0: none
 };
 
+// Heads of up to 128 entries on eight lanes, in pieces of four entries (8 or 16 bytes a load and store): four heads a warp.  Issuing instructions is what
+// bounds it: a head costs a warp some 40 where 32 lanes, an entry each at a time, spent some 150.  4096 tokens of 32 + 8 + 8 heads of 128 (100 MB): 72 us
+// entry by entry, 48 with a warp a head and four entries a lane, 32 so (fp32: 70 and 39); 171 tokens 8.8 and 4.7; 8 tokens 3.8 and 2.6.
+constexpr int PREP_LANES = 8, PREP_PIECES = 4, PREP_MAX_DIM = PREP_LANES * PREP_PIECES * 4;
+template <typename T>
+__global__ void attn_prep_fours_kernel(AttnPrepArgs a) {
+    pdl_trigger();
+    pdl_wait();
+    const int t = blockIdx.x, at = threadIdx.x % PREP_LANES * 4, teams = blockDim.x / PREP_LANES;
+    const int Nq = a.H * a.d, Nk = a.G * a.d, Nv = a.G * a.e;
+    const T* row = static_cast<const T*>(a.qkv) + (size_t)t * (Nq + Nk + Nv);
+    const int pos = a.positions[t], crow = a.cache_rows ? a.cache_rows[t] : -1;
+    const float temp = a.temp_every > 0 ? 1.f + a.temp_coef * logf((float)((pos + 1) / a.temp_every + 1)) : 1.f;
+    for (int base = 0; base < a.H + a.G; base += teams) {  // every lane of a warp takes every turn: the sums are shuffles
+        const int h = base + threadIdx.x / PREP_LANES;
+        const bool is_q = h < a.H, mine = h < a.H + a.G;
+        const T* src = row + (size_t)h * a.d;  // the keys' heads follow the queries'
+        const T* nwgt = static_cast<const T*>(is_q ? a.qnorm : a.knorm);
+        float x[PREP_PIECES][4], w[PREP_PIECES][4], ss = 0.f;
+#pragma unroll
+        for (int k = 0; k < PREP_PIECES; ++k) {
+            const int i = k * PREP_LANES * 4 + at;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) { x[k][c] = 0.f; w[k][c] = 1.f; }
+            if (mine && i < a.d) {
+                load4(src + i, x[k]);
+                if (nwgt) load4(nwgt + i, w[k]);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < PREP_PIECES; ++k)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) ss = fmaf(x[k][c], x[k][c], ss);
+#pragma unroll
+        for (int o = PREP_LANES / 2; o; o /= 2) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        const float inv = nwgt ? 1.f / sqrtf(ss / (float)a.d + a.eps) : 1.f;
+        T* dst = is_q ? static_cast<T*>(a.q_out) + (size_t)t * Nq + h * a.d : static_cast<T*>(a.cache_k) + (size_t)crow * Nk + (h - a.H) * a.d;
+#pragma unroll
+        for (int k = 0; k < PREP_PIECES; ++k) {
+            const int i = k * PREP_LANES * 4 + at;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                x[k][c] = x[k][c] * inv * w[k][c];
+                if (is_q) x[k][c] = rnd<T>(x[k][c]) * temp;
+            }
+            if (mine && i < a.d && (is_q || crow >= 0)) store4<T>(dst + i, x[k]);
+        }
+    }
+    const T* vsrc = row + Nq + Nk;
+    T* vf = static_cast<T*>(a.v_first) + (size_t)t * Nv;
+    const float lam = a.vmix_mode == 2 ? to_f(*static_cast<const T*>(a.vmix)) : 0.f;
+    for (int c = threadIdx.x * 4; c < Nv; c += blockDim.x * 4) {
+        float v[4], f[4];
+        load4(vsrc + c, v);
+        if (a.vmix_mode == 1) store4<T>(vf + c, v);
+        else if (a.vmix_mode == 2) {
+            load4(vf + c, f);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) v[k] = (1.f - lam) * v[k] + lam * f[k];
+        }
+        if (crow >= 0) store4<T>(static_cast<T*>(a.cache_v) + (size_t)crow * Nv + c, v);
+    }
+}
+
+// heads of more entries, of no whole number of pieces, or not on a piece's boundary
 template <typename T>
 __global__ void attn_prep_kernel(AttnPrepArgs a) {
     pdl_trigger();

@@ -831,3 +831,44 @@ def test_linears_over_streamed_tiles(T, N, K):
     assert ((got.double() - base.double() - ref).abs() <= 2 ** -8 * ref.abs() + size + 2.0 ** -23 * (base.double() + ref).abs()).all()
     y = ref.bfloat16().double()
     assert rel(h.linear_swiglu(x, w), torch.nn.functional.silu(y[:, 0::2]) * y[:, 1::2]) < 2 ** -7
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("mode", [0, 1, 2])
+@pytest.mark.parametrize("norm", [True, False])
+@pytest.mark.parametrize("T,H,G,d,e", [(1, 1, 1, 4, 4), (9, 5, 2, 128, 96), (1100, 7, 1, 64, 132), (33, 3, 2, 132, 4), (33, 3, 1, 100, 6), (17, 2, 2, 30, 32)])
+def test_heads_prepared_four_entries_a_lane(T, H, G, d, e, norm, mode, dt):
+    """Heads of up to 128 entries in fours; larger ones, odd ones and values of an odd count entry by entry.  A stored number is one rounding of dt from its
+    exact value, a query two (it is rounded before its temperature), on top of a few of fp32; lost tokens leave the ring alone."""
+    from mistral_inference_b200 import _abi_hybrid as h
+
+    g = torch.Generator().manual_seed(T + d)
+    rnd = lambda *s: torch.randn(*s, generator=g).to(dt).to(DEV)
+    qkv, qn, kn, first, lam = rnd(T, H * d + G * (d + e)), rnd(d), rnd(d), rnd(T, G * e), rnd(1)
+    pos = torch.randint(0, 5000, (T,), generator=g).int().to(DEV)
+    rows = torch.randperm(T + 5, generator=g)[:T].int()
+    if T > 1:
+        rows[T // 2] = -1
+    rows = rows.to(DEV)
+    q = torch.empty(T, H * d, dtype=dt, device=DEV)
+    ck, cv = torch.full((T + 5, G * d), 7.0, dtype=dt, device=DEV), torch.full((T + 5, G * e), 7.0, dtype=dt, device=DEV)
+    before = first.clone()
+    h.attn_prep(qkv, qn if norm else None, kn if norm else None, pos, rows, q, ck, cv, first, lam, mode, H, G, d, e, 1e-5, 0.1, 64)
+    xq, xk, xv = (t.double() for t in qkv.split([H * d, G * d, G * e], 1))
+    unit = lambda x, n, w: (x.view(T, n, d) / (x.view(T, n, d).square().mean(-1, keepdim=True) + 1e-5).sqrt() * w.double()).reshape(T, -1) if norm else x
+    xq = unit(xq, H, qn) * (1 + 0.1 * torch.log((pos.double() + 1).div(64).floor() + 1))[:, None]
+    xk = unit(xk, G, kn)
+    if mode == 2:
+        xv = (1 - lam.double()) * xv + lam.double() * before.double()
+    assert torch.equal(first, qkv[:, -G * e:] if mode == 1 else before)
+    step = 2.0 ** -8 if dt == torch.bfloat16 else 2.0 ** -24
+    fp32 = 12 * 2.0 ** -23  # the sum of squares, its root and quotient, the logarithm and three products
+    kept = rows >= 0
+    at = rows[kept].long()
+    big = lam.double().abs() * before.double().abs() + (1 + lam.double().abs()) * qkv[:, -G * e:].double().abs()  # what a mixed value's fp32 steps are measured by
+    assert ((q.double() - xq).abs() <= (2 * step + step * step + fp32) * xq.abs()).all()
+    assert ((ck[at].double() - xk[kept]).abs() <= (step + fp32) * xk[kept].abs()).all()
+    assert ((cv[at].double() - xv[kept]).abs() <= step * xv[kept].abs() + (4 * 2.0 ** -24 * big[kept] * (1 + step) if mode == 2 else 0)).all()
+    lost = torch.ones(T + 5, dtype=torch.bool, device=DEV)
+    lost[at] = False
+    assert (ck[lost] == 7).all() and (cv[lost] == 7).all()
