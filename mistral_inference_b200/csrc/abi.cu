@@ -442,7 +442,7 @@ int mb200_moe_grouped_ffn(const void* xs, const void* const* w13_host, const voi
   EpiParams e1;
   e1.out = g;
   e1.ld_out = hidden;
-  int rc = launch_grouped<EPI_SWIGLU>(xs, rows_cap, dim, 2 * hidden, w13_host, (int)n_experts, est, tile_rows, plan, e1, workspace, workspace_bytes, kWsHeader, st);
+  int rc = launch_grouped<EPI_SWIGLU>(xs, rows_cap, dim, 2 * hidden, w13_host, (int)n_experts, pairs, est, tile_rows, plan, e1, workspace, workspace_bytes, kWsHeader, st);
   if (rc) return rc;
   EpiParams e2;
   e2.out = yw;
@@ -453,7 +453,7 @@ int mb200_moe_grouped_ffn(const void* xs, const void* const* w13_host, const voi
     MB_CHECK_ARG(comm->peer_yw[r] != nullptr, "moe_grouped_ffn: peer buffer %d missing", r);
     e2.peer_out[r] = comm->peer_yw[r];
   }
-  rc = launch_grouped<EPI_MOE_SCALE>(g, rows_cap, hidden, dim, w2_host, (int)n_experts, est, tile_rows, plan, e2, workspace, workspace_bytes, kWsHeader, st);
+  rc = launch_grouped<EPI_MOE_SCALE>(g, rows_cap, hidden, dim, w2_host, (int)n_experts, pairs, est, tile_rows, plan, e2, workspace, workspace_bytes, kWsHeader, st);
   if (rc) return rc;
   MoeCombineParams c;
   c.yw = (const uint4*)yw;

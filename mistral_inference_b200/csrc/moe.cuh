@@ -121,6 +121,9 @@ __global__ void __launch_bounds__(256) moe_route_kernel(const bf16* hn, const bf
 // pairs of CTAs, [7] tiles that these have drawn (zero between launches), [8 + e] start of expert e's segment (e = 0..E), then from word MOE_PLAN_HEADER four lists of `capacity` words: tile_expert, tile_row0 (m tiles),
 // pair_expert, pair_info (token tiles: first row | width / 32).
 constexpr int MP_THREADS = 1024, MP_ROW = MP_THREADS + MP_THREADS / 32;
+// A plan of up to this many (token, expert) pairs lists no token tiles for pairs of CTAs: whoever launches on them asks here first.
+constexpr int MOE_SHORT_PLAN = 512;
+MB_HD bool moe_plan_lists_pairs(int64_t pairs) { return pairs > MOE_SHORT_PLAN; }
 inline size_t moe_plan_smem(int64_t E) { return ((size_t)E * MP_ROW + 2 * E + 1) * sizeof(int32_t); }
 __global__ void __launch_bounds__(MP_THREADS) moe_plan_kernel(const int32_t* sel, int pairs, int E, int tile_rows, int shard_rank,
                                                               int shard_world, int tile_cap, int32_t* __restrict__ slot, int32_t* __restrict__ plan) {
@@ -131,7 +134,7 @@ __global__ void __launch_bounds__(MP_THREADS) moe_plan_kernel(const int32_t* sel
   int32_t* seg = sm + E * MP_ROW;
   int32_t* total = seg + E + 1;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (pairs <= 512) {
+  if (!moe_plan_lists_pairs(pairs)) {
     // decode-sized batch: thread e walks the whole (short) pair list for expert e -- same deterministic plan, a few hundred cycles
     if (tid < E) {
       int n = 0;
@@ -161,7 +164,8 @@ __global__ void __launch_bounds__(MP_THREADS) moe_plan_kernel(const int32_t* sel
       plan[3] = pairs;
       plan[4] += touched;
       plan[5] += 1;
-      plan[6] = 0;  // calls this small never run on pairs of CTAs
+      plan[6] = 0;
+      plan[7] = 0;
     }
     __syncthreads();
     for (int i = tid; i < pairs; i += MP_THREADS) slot[i] = sel[i] < E ? slot[i] + seg[sel[i]] : -1;
@@ -462,7 +466,7 @@ int launch_grouped_streamk(const void* a, int64_t rows_cap, int64_t K, int64_t N
 }
 
 template <int MODE>
-int launch_grouped(const void* a, int64_t rows_cap, int64_t K, int64_t N, const void* const* w_host, int E, int est_mtiles, int tile_rows,
+int launch_grouped(const void* a, int64_t rows_cap, int64_t K, int64_t N, const void* const* w_host, int E, int64_t pairs, int est_mtiles, int tile_rows,
                    const int32_t* plan, const EpiParams& epi, void* workspace, size_t workspace_bytes, size_t header, cudaStream_t stream) {
   const int sms = device_info::sm_count();
   if (sms == 0) return fail(MB200_E_CUDA, "no device");
@@ -474,7 +478,7 @@ int launch_grouped(const void* a, int64_t rows_cap, int64_t K, int64_t N, const 
   if (tile_rows == 128) {
     // From about 128 rows an expert, where the GEMMs below begin to need two tiles of tokens for one.  The layer of eight experts of 4096 x 14336 with the GEMMs below and with pairs, us:
     // 300 tokens (75 rows an expert) 527, 550, 450 530, 562, 600 681, 594, 800 695, 631, 1000 829, 781, 1300 948, 938; of 6144 x 16384: 400 872, 876, 800 1192, 1018, 1200 1678, 1584.
-    if (N % 128 == 0 && tcgen05_cluster_enabled() && rows_cap >= (int64_t)E * 256) {
+    if (N % 128 == 0 && tcgen05_cluster_enabled() && moe_plan_lists_pairs(pairs) && rows_cap >= (int64_t)E * 256) {
       CUtensorMap map_a;
       MoeWeightMaps maps;
       int rc = make_tensor_map_2d(&map_a, a, rows_cap, K, TG_BM);
@@ -595,7 +599,7 @@ inline int launch_grouped_packed(const void* a, int64_t rows_cap, int64_t K, int
   for (int e = 1; e < MOE_MAX_EXPERTS; ++e) maps.m[e] = maps.m[0];
   // Wherever the plan lists token tiles of pairs (more than 512 rows in all).  16 experts of 1408, width 2048, with the GEMM below and with pairs, us: 130 tokens 117, 114, 250 102, 97,
   // 450 104, 103, 800 135, 123, 1300 162, 143; eight of 14336, width 4096: 300 tokens 539, 523, 600 772, 580, 1000 923, 776, 1300 1126, 998.
-  if (tcgen05_cluster_enabled() && pairs > 512)
+  if (tcgen05_cluster_enabled() && moe_plan_lists_pairs(pairs))
     return launch_grouped_pair<EPI_LAYER>(map_a, maps, rows_cap, K, N, w_n, w_k, plan, epi, sms, stream);
   using Cfg = TgCfg<128, 128, kEpiSmem<EPI_LAYER>>;
   TcGemmParams p;

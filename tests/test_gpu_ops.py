@@ -514,22 +514,29 @@ def _moe_case(T, dim, hid, E, seed):
 
 def _router_margin_ulps(x, gate_w, k):
     logits = F.linear(x, gate_w).float()
+    if k == logits.shape[-1]:
+        return torch.full((x.shape[0],), float("inf"))  # every expert is chosen
     top = logits.topk(k + 1, dim=-1).values
     ulp = torch.pow(2.0, torch.floor(torch.log2(top[:, k - 1].abs().clamp_min(1e-30))) - 7)
     return (top[:, k - 1] - top[:, k]) / ulp
 
 
-@pytest.mark.parametrize("T,dim,hid,k", [(5, 256, 256, 2), (37, 256, 256, 3), (200, 256, 512, 2), (16, 4096, 14336, 2), (300, 4096, 14336, 2),
-                                         (2500, 256, 512, 2), (2100, 1152, 1024, 2)])  # last two: enough rows per expert for the grouped GEMM on pairs
-def test_moe_route_grouped_ffn_vs_oracle(T, dim, hid, k):
+_FEW = [(E, T, 256, 256, k) for E, k, Ts in [(2, 1, (128, 129, 512, 513)), (2, 2, (64, 65, 200, 256, 257)), (4, 1, (385, 512, 513)), (4, 2, (65, 193, 256, 257)), (4, 3, (129, 170, 171)),
+                                             (4, 4, (97, 128, 129)), (16, 4, (128, 129))] for T in Ts]
+
+
+@pytest.mark.parametrize("E,T,dim,hid,k", [(8, 5, 256, 256, 2), (8, 37, 256, 256, 3), (8, 200, 256, 512, 2), (8, 16, 4096, 14336, 2), (8, 300, 4096, 14336, 2),
+                                           (8, 2500, 256, 512, 2), (8, 2100, 1152, 1024, 2),  # enough rows per expert for the grouped GEMM on pairs
+                                           (8, 1300, 3072, 3200, 2), (4, 257, 3136, 4224, 2)]  # ... whose tiles are drawn (K >= 3072) in both GEMMs, in several turns and in one
+                         + _FEW)  # few experts around 512 rows in all, where the plan begins to list tiles of pairs
+def test_moe_route_grouped_ffn_vs_oracle(E, T, dim, hid, k):
     """mb200_moe_route + mb200_moe_grouped_ffn against the oracle's MoE (moe.py:24-32) + residual: routing decisions and weights
     exactly (tokens whose k-th / (k+1)-th router logits are within 2 ulps excepted), the deterministic row plan exactly, the
-    output within 2 bf16 ulps."""
+    output within 2 bf16 ulps, the same bits from the same plan again, whose counter of drawn tiles is back at zero."""
     from mistral_inference_b200.moe import MoeBuffers
 
     from .util import moe_plan_host, moe_route_host
 
-    E = 8
     x, gate_w, experts = _moe_case(T, dim, hid, E, seed=90)
     h = rnd(T, dim, seed=89)
     want = h + R.moe_forward(x, gate_w, experts, k)
@@ -563,10 +570,15 @@ def test_moe_route_grouped_ffn_vs_oracle(T, dim, hid, k):
         keep += [packed, down]
         w13[e], w2[e] = packed.data_ptr(), down.data_ptr()
     out = torch.empty(T, dim, dtype=torch.bfloat16, device=DEV)
+    first = None
     for _ in range(2):  # twice: stream-K flags and plan buffers must be reusable
         out.zero_()
+        b.yw.fill_(1000.0)  # what no expert writes would show
         _abi.moe_grouped_ffn(b, w13, w2, h.to(DEV), out, T, dim, hid, E, k, None, ws)
         torch.cuda.synchronize()
+        assert b.plan[7].item() == 0
+        assert first is None or torch.equal(first, out)
+        first = out.clone()
         rows = safe & (sel == sel_ref).all(-1)
         assert rows.float().mean() > 0.8
         assert_bf16_close(out.cpu()[rows], want[rows], max_ulp=2, min_exact=0.9, atol=2 * 2 ** -8 * want.abs().max().item(), what="moe layer")
