@@ -152,6 +152,7 @@ __device__ __forceinline__ void sk_gemm_body(const CUtensorMap& map_a, const CUt
   } else if (warp == 1) {
     // ================= MMA issuer (one thread, elected by the warp) =================
     {
+      if (!GROUPED) pdl_wait();  // (the tokens come behind it: the waits' limits count from there)
       const uint32_t ring = umma_desc_lo(smem_u32(smem));
       uint32_t it = 0, seg = 0;
       for (long long u = u_begin; u < u_end; ++seg) {

@@ -49,7 +49,8 @@ __device__ __forceinline__ uint32_t ft_smem(const void* p) { return (uint32_t)__
 __device__ __forceinline__ void ft_bar_init(uint64_t* b, uint32_t count) { asm volatile("mbarrier.init.shared.b64 [%0], %1;" ::"r"(ft_smem(b)), "r"(count) : "memory"); }
 __device__ __forceinline__ void ft_bar_arrive(uint32_t b) { asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(b) : "memory"); }  // b: ft_first_cta
 __device__ __forceinline__ void ft_bar_expect(uint64_t* b, uint32_t bytes) { asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" ::"r"(ft_smem(b)), "r"(bytes) : "memory"); }
-// Waits a bounded time.  false: gave up (the caller marks the CTA dead and goes on to the end without waiting again).
+// Waits a bounded time.  false: gave up: the caller marks its CTA (`lost`), whose sums from then on are NaN, goes on to the end without waiting again, and says nothing more that
+// would let the other CTA of the pair take what is not there (no arrival, no copy, no commit): that one gives up too.
 __device__ __forceinline__ bool ft_bar_wait(uint64_t* b, uint32_t parity) {
     for (int i = 0; i < (1 << 22); ++i) {
         uint32_t ok;
@@ -153,17 +154,18 @@ __device__ __forceinline__ void ft_cluster_sync() {
 }
 
 // Up to 128 rows of x times a CTA's features with FMAs in the order of k, through shared memory (the stages: the parts are not needed any more).  A thread takes four
-// columns of every 16th row.  About the time the whole tile takes with FMAs, once per tile that holds an infinity or a NaN.
+// columns of every 16th row.  About the time the whole tile takes with FMAs, once per tile that holds an infinity or a NaN.  lost: copies may still be on their way to
+// the stages; NaN in place of the sums.
 template <bool VEC>
-__device__ __noinline__ void ft_fma_rows(const LinearArgs& a, const float* X, const float* W, float* sm, int m0, int n0, int rows, int cols) {
+__device__ __noinline__ void ft_fma_rows(const LinearArgs& a, const float* X, const float* W, float* sm, int m0, int n0, int rows, int cols, bool lost) {
     constexpr int KB = 64, XP = KB + 4, WP = FT_BN + 4, share = 128;
     float *xs = sm, *ws = sm + share * XP;  // [share][XP], [KB][WP]
     static_assert((share * XP + KB * WP) * 4 <= 2 * FT_STAGE, "both blocks fit in the stages");
     const int tid = threadIdx.x, c4 = (tid & 31) * 4, r0 = tid >> 5, nr = (rows + 15) / 16;
     float acc[8][4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
-    for (int k0 = 0; k0 < a.K; k0 += KB) {
+    for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = lost ? __int_as_float(0x7fffffff) : 0.f;
+    for (int k0 = 0; k0 < a.K && !lost; k0 += KB) {
         __syncthreads();
         for (int i = tid; i < (share + FT_BN) * (KB / 4); i += FT_THREADS) {
             const int r = i / (KB / 4), kc = (i % (KB / 4)) * 4, k = k0 + kc, n = r - share;
@@ -323,6 +325,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) linear_f32_pair(const __grid_co
     __shared__ uint64_t full[2], done[2], taken[2];  // a stage is there; its MMAs have completed; their sums have been added (full and taken: the first CTA's)
     __shared__ uint32_t tmem_slot;
     __shared__ unsigned redo[FT_REDO_WORDS];
+    __shared__ volatile int lost;  // a wait of this CTA ran out
     const LinearArgs& a = args.a;
     const F32Plan& p = args.p;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -346,6 +349,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) linear_f32_pair(const __grid_co
     };
 
     if (tid == 0) {
+        lost = 0;
         for (int i = 0; i < 2; ++i) { ft_bar_init(&full[i], 2 * FT_SPLIT_WARPS + 1); ft_bar_init(&done[i], 1); ft_bar_init(&taken[i], 2 * FT_SUM_WARPS); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&parts) : "memory");
@@ -418,7 +422,8 @@ __global__ void __launch_bounds__(FT_THREADS, 1) linear_f32_pair(const __grid_co
         }
         bool alive = true;
         for (int it = 0; it < total; ++it) {
-            if (it >= 2 && alive && !ft_bar_wait(&done[it & 1], ((it >> 1) - 1) & 1)) alive = false;
+            if (it == 2) pdl_wait();  // nothing is multiplied before the predecessor's end: the wait's limit counts from there
+            if (it >= 2 && alive && !ft_bar_wait(&done[it & 1], ((it >> 1) - 1) & 1)) { alive = false; lost = 1; }
             unsigned char* st = at + (it & 1) * FT_STAGE;
 #pragma unroll
             for (int i = 0; i < NF; ++i) {
@@ -429,7 +434,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) linear_f32_pair(const __grid_co
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
-            if (lane == 0) ft_bar_arrive(full_at[it & 1]);
+            if (lane == 0 && alive) ft_bar_arrive(full_at[it & 1]);
             if (kb < 0) start();
             next();  // (behind the arrival, which would wait for the loads)
         }
@@ -453,7 +458,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) linear_f32_pair(const __grid_co
 #pragma unroll
                 for (int j = 0; j < 16; ++j) acc[q][j] = 0.f;
             for (int kb = c.kb0; kb < c.kb1; ++kb, ++it) {
-                if (alive && !ft_bar_wait(&done[it & 1], (it >> 1) & 1)) alive = false;
+                if (alive && !ft_bar_wait(&done[it & 1], (it >> 1) & 1)) { alive = false; lost = 1; }
                 __syncwarp();
                 ft_fence_after();
                 const uint32_t from = mine + (it & 1) * 256;
@@ -474,10 +479,11 @@ __global__ void __launch_bounds__(FT_THREADS, 1) linear_f32_pair(const __grid_co
                 }
                 ft_fence_before();
                 __syncwarp();
-                if (lane == 0) ft_bar_arrive(taken_at[it & 1]);
+                if (lane == 0 && alive) ft_bar_arrive(taken_at[it & 1]);
             }
             // The tile's sums.  An operand that is not finite makes a part that is NaN (inf - inf), so every sum it enters is NaN: found here, once.
             int strange = 0;
+            if (lost) alive = false;
 #pragma unroll
             for (int q = 0; q < FT_CHUNKS; ++q)
 #pragma unroll
@@ -532,7 +538,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) linear_f32_pair(const __grid_co
             for (int i = cluster; i < p.items; i += p.clusters) {
                 const Item c = item_of(i);
                 for (int kb = c.kb0; kb < c.kb1; ++kb, ++it) {
-                    if (it >= 2 && alive && !ft_bar_wait(&done[it & 1], ((it >> 1) - 1) & 1)) alive = false;
+                    if (it >= 2 && alive && !ft_bar_wait(&done[it & 1], ((it >> 1) - 1) & 1)) { alive = false; lost = 1; }
                     if (!alive) continue;
                     // the pair's copies count on the first CTA's barrier (the other CTA's may land before it is armed)
                     if (rank == 0) ft_bar_expect(&full[it & 1], 2u * 3u * (uint32_t)half * 128u);
@@ -546,6 +552,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) linear_f32_pair(const __grid_co
         if (warp == FT_SPLIT_WARPS + FT_SUM_WARPS + 1 && rank == 0) {
             // (the whole warp walks, one thread of it issues: so the operands are uniform.  In a thread's own registers the 24 instructions of a k-block took longer to
             // issue than to run)
+            pdl_wait();  // (the copies begin behind it: the waits' limits count from there)
             bool alive = true;
             int it = 0;
             const uint32_t idesc = FT_IDESC | (uint32_t)(p.w >> 3) << 17, x_part = (uint32_t)(p.w / 2) * 128u >> 4, first = ft_desc_lo(ft_smem(sm));
@@ -554,7 +561,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) linear_f32_pair(const __grid_co
                 for (int kb = c.kb0; kb < c.kb1; ++kb, ++it) {
                     if (it >= 2 && alive && !ft_bar_wait(&taken[it & 1], ((it >> 1) - 1) & 1)) alive = false;
                     if (alive && !ft_bar_wait(&full[it & 1], (it >> 1) & 1)) alive = false;
-                    if (!__all_sync(0xffffffffu, alive)) { alive = false; continue; }
+                    if (!__all_sync(0xffffffffu, alive)) { alive = false; lost = 1; continue; }
                     ft_fence_after();
                     const uint32_t w0 = first + (it & 1) * (FT_STAGE >> 4), w1 = w0 + (FT_TILE >> 4), w2 = w1 + (FT_TILE >> 4), d = tmem + (it & 1) * 256;
                     const uint32_t x0 = w2 + (FT_TILE >> 4), x1 = x0 + x_part, x2 = x1 + x_part;  // parts: 0 hi, 1 mid, 2 lo
@@ -594,7 +601,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) linear_f32_pair(const __grid_co
         const int end = min(a.M, c.t0 + p.w);
         for (int m = c.t0; m < end; m += 128)
             ft_fma_rows<VEC>(a, static_cast<const float*>(a.x) + (size_t)m * a.x_pitch(), W + (size_t)c.n0 * a.K, reinterpret_cast<float*>(sm), m, c.n0, min(128, end - m),
-                             min(FT_BN, a.N - c.n0));
+                             min(FT_BN, a.N - c.n0), lost);
     }
 }
 

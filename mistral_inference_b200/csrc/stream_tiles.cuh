@@ -91,6 +91,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stream_tiles_kernel(const __gri
     }
   } else if (warp == 1) {
     // ================= MMA issuer (one thread, elected by the warp) =================
+    pdl_wait();  // (the tokens come behind it: the waits' limits count from there)
     const uint32_t ring = umma_desc_lo(smem_u32(smem)), idesc = (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t)(p.cols >> 3) << 17 | (uint32_t)(ST_ROWS >> 4) << 24;
     int s = 0, par = 0;
     uint32_t seg = 0;

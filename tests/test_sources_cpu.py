@@ -30,3 +30,18 @@ def test_what_a_predecessor_writes_is_no_read_only_parameter(files):
     assert len(launched) >= 9, launched
     read_only = {k: set(re.findall(r"const\s+[\w:]+\s*\*\s*__restrict__\s+(\w+)", params[k])) - WEIGHTS for k in launched}
     assert not {k: v for k, v in read_only.items() if v}
+
+
+@pytest.mark.parametrize("name,start,wait", [("hybrid/hybrid_linear_f32.cuh", "linear_f32_pair(const", "ft_bar_wait("), ("stream_linear.cuh", "stream_linear_kernel(const", "bar_wait("),
+                                             ("stream_tiles.cuh", "stream_tiles_kernel(const", "mbar_wait("), ("gemm_streamk.cuh", "void sk_gemm_body(const", "mbar_wait(")])
+def test_limits_of_waits_count_from_the_predecessors_end(name, start, wait):
+    """A kernel launched programmatically may be resident for as long as its predecessors run.  Its waits are bounded, and none of its barriers completes before the predecessor has
+    ended, so every role waits for that end before its first barrier: else a long predecessor uses the limit up."""
+    text = re.sub(r"//[^\n]*", "", (CSRC / name).read_text())
+    body = text[text.index(start):]
+    body = body[:body.index("\n}\n")]
+    roles = [r for r in re.split(r'\n {2,4}(?:if \(warp|\} else|\}\n(?= +asm volatile\("griddepcontrol\.wait))', body) if wait in r]
+    assert len(roles) >= 2
+    for role in roles:
+        ends = [i for i in (role.find("pdl_wait()"), role.find("griddepcontrol.wait")) if i >= 0]
+        assert ends and min(ends) < role.index(wait), role[:300]
