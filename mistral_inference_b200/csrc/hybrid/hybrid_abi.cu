@@ -194,7 +194,7 @@ int mbh_rmsnorm(const void* x32, const void* w, const void* w2, void* y, void* y
 }
 
 int64_t mbh_linear_scratch(int64_t M, int64_t N, int64_t K, int dt) {
-    if (dt != 1 || M <= SK_MAX_M || N <= 0 || K < FT_MIN_K) return 0;
+    if (dt != 1 || M <= SK_MAX_M || N <= 0 || K < FT_MIN_K || f32_few_features((int)M, (int)N, (int)K)) return 0;
     return f32_scratch_bytes((int)M, (int)N, (int)K, FT_TO_SLOTS);
 }
 

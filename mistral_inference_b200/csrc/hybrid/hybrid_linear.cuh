@@ -19,7 +19,7 @@
 // In bf16 mode the Linear's own output is rounded to bf16 before the epilogue's arithmetic (the rounding point of a bf16
 // Linear); accumulation is fp32 in both modes.
 //
-// Kernels: `linear_tiled_mma` (bf16), `linear_f32_pair` (fp32, hybrid_linear_f32.cuh) and `linear_tiled_fma` (fp32, K < 16) for prompts, any shape; `linear_skinny` (M <= 8 rows, FMA,
+// Kernels: `linear_tiled_mma` (bf16), `linear_f32_pair` and `linear_f32_parts` (fp32, hybrid_linear_f32.cuh, hybrid_linear_f32_cta.cuh) and `linear_tiled_fma` (fp32, K < 16) for prompts, any shape; `linear_skinny` (M <= 8 rows, FMA,
 // one warp per pair of weight rows) and `stream_linear_kernel` (bf16, up to 32 rows, tensor cores) for decode: every weight byte is read
 // once; `linear_decay_mma` for decays from a low rank.  The large aligned bf16 Linears of prompts go to the main
 // library's tcgen05 GEMMs, with these steps in their epilogue (see _abi_hybrid.linear).
@@ -410,7 +410,7 @@ struct StreamEpi {
 
 }  // namespace mbh
 
-#include "hybrid_linear_f32.cuh"
+#include "hybrid_linear_f32_cta.cuh"
 
 namespace mbh {
 
@@ -439,7 +439,7 @@ inline cudaError_t launch_linear(const LinearArgs& a, cudaStream_t st, void* scr
         linear_tiled_mma<<<grid, MM_THREADS, 0, st>>>(a);
     } else {
         cudaError_t e = cudaSuccess;
-        if (a.K >= FT_MIN_K && launch_linear_f32_pair(a, scratch, scratch_bytes, st, e)) return e;
+        if (a.K >= FT_MIN_K) return launch_linear_f32_pair(a, scratch, scratch_bytes, st, e) ? e : launch_linear_f32_parts(a, st);
         linear_tiled_fma<<<dim3((a.N + LT_BN - 1) / LT_BN, (a.M + LT_BM - 1) / LT_BM), LT_THREADS, 0, st>>>(a);
     }
     return cudaGetLastError();

@@ -25,7 +25,9 @@
 // Two stages, two accumulators.  Clusters are persistent; a last round that is not full is cut along k, and f32_combine_kernel adds the parts in the order of k, so nobody waits for another
 // cluster and the result is the same every time.
 //
-// An infinity or a NaN in the operands of a tile, or a number from 2^120 on (256 x is formed): its outputs are computed again with FMAs (ft_fma_rows).
+// An infinity or a NaN in the operands of a tile, or a number from 2^120 on (256 x is formed): its outputs are computed again with FMAs (ft_fma_rows; one NaN among 804 x 16384 x 2048: 2046 us).
+//
+// Where x is the larger operand hybrid_linear_f32_cta.cuh runs.
 #pragma once
 #include <cuda.h>
 
@@ -43,7 +45,6 @@ static_assert(2 * FT_SPLIT_REGS + 2 * FT_SUM_REGS + FT_REST_REGS <= 5 * FT_REGS,
 constexpr int FT_TILE = FT_BN * FT_BK * 2, FT_STAGE = 3 * FT_TILE + 3 * (FT_MAX_W / 2) * FT_BK * 2;  // a part of W: 128 rows of 128 bytes; a stage: three of W, three of half the tile's tokens
 constexpr int FT_SMEM = 2 * FT_STAGE + 1024;
 constexpr int FT_REDO_WORDS = 512;  // a bit per tile of a cluster
-constexpr int FT_MAX_TOKENS = 4096;  // of a launch: the slots of a longer prompt would take as much memory as its result
 
 __device__ __forceinline__ uint32_t ft_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void ft_bar_init(uint64_t* b, uint32_t count) { asm volatile("mbarrier.init.shared.b64 [%0], %1;" ::"r"(ft_smem(b)), "r"(count) : "memory"); }
@@ -156,7 +157,7 @@ __device__ __forceinline__ void ft_cluster_sync() {
 // Up to 128 rows of x times a CTA's features with FMAs in the order of k, through shared memory (the stages: the parts are not needed any more).  A thread takes four
 // columns of every 16th row.  About the time the whole tile takes with FMAs, once per tile that holds an infinity or a NaN.  lost: copies may still be on their way to
 // the stages; NaN in place of the sums.
-template <bool VEC>
+template <bool VEC, int THREADS>
 __device__ __noinline__ void ft_fma_rows(const LinearArgs& a, const float* X, const float* W, float* sm, int m0, int n0, int rows, int cols, bool lost) {
     constexpr int KB = 64, XP = KB + 4, WP = FT_BN + 4, share = 128;
     float *xs = sm, *ws = sm + share * XP;  // [share][XP], [KB][WP]
@@ -167,7 +168,7 @@ __device__ __noinline__ void ft_fma_rows(const LinearArgs& a, const float* X, co
     for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = lost ? __int_as_float(0x7fffffff) : 0.f;
     for (int k0 = 0; k0 < a.K && !lost; k0 += KB) {
         __syncthreads();
-        for (int i = tid; i < (share + FT_BN) * (KB / 4); i += FT_THREADS) {
+        for (int i = tid; i < (share + FT_BN) * (KB / 4); i += THREADS) {
             const int r = i / (KB / 4), kc = (i % (KB / 4)) * 4, k = k0 + kc, n = r - share;
             const bool is_x = r < share, ok = is_x ? r < rows : n < cols;
             const float* src = is_x ? X + (size_t)r * a.x_pitch() + k : W + (size_t)n * a.K + k;
@@ -253,7 +254,7 @@ inline F32Plan f32_plan(int M, int N, int K, int units) {
         const int rest = (int)(tiles % units);
         int cut = rest ? units / rest : 1;
         if (cut > 8) cut = 8;
-        while (cut > 1 && nkb < 2 * cut) --cut;
+        while (cut > 1 && nkb < 4 * cut) --cut;  // (parts of fewer k-blocks cost more in slots than they save: 300 x 1024 x 1024 20.8 us with two, 17.2; 2000 x 1024 x 256 21.8, 15.9)
         p.cut = cut;
         p.whole = (int)(cut > 1 ? tiles - rest : tiles);
         p.items = (int)(p.whole + (tiles - p.whole) * cut);
@@ -600,7 +601,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) linear_f32_pair(const __grid_co
         const Item c = item_of(i);
         const int end = min(a.M, c.t0 + p.w);
         for (int m = c.t0; m < end; m += 128)
-            ft_fma_rows<VEC>(a, static_cast<const float*>(a.x) + (size_t)m * a.x_pitch(), W + (size_t)c.n0 * a.K, reinterpret_cast<float*>(sm), m, c.n0, min(128, end - m),
+            ft_fma_rows<VEC, FT_THREADS>(a, static_cast<const float*>(a.x) + (size_t)m * a.x_pitch(), W + (size_t)c.n0 * a.K, reinterpret_cast<float*>(sm), m, c.n0, min(128, end - m),
                              min(FT_BN, a.N - c.n0), lost);
     }
 }
@@ -635,9 +636,16 @@ inline F32Scratch f32_scratch(int M, int K, const F32Plan& p, int step) {
     s.bytes = s.parts + 3 * (int64_t)M * s.kp * 2;
     return s;
 }
-// of a Linear of M rows, whatever its step: launches of at most FT_MAX_TOKENS
+// Rows of a launch: 4096, because the slots of a longer prompt would take as much memory as its result, and more only where slots and parts stay below 128 MB; equal shares, since a launch
+// of a few rows takes as long as one of a few hundred (5000 x 384 x 128 in 4096 + 904 rows 25 us, 15.1 so).
+inline int f32_launch_rows(int M, int N, int K) {
+    const int64_t room = ((int64_t)128 << 20) / (4 * (int64_t)N + 6 * (int64_t)K), most = room < 4096 ? 4096 : room > 16384 ? 16384 : room;
+    const int launches = (int)((M + most - 1) / most);
+    return ((M + launches - 1) / launches + 15) / 16 * 16;
+}
+// of a Linear of M rows
 inline int64_t f32_scratch_bytes(int M, int N, int K, int step) {
-    const int m = M < FT_MAX_TOKENS ? M : FT_MAX_TOKENS, rest = M > m ? M % m : 0;
+    const int rows = f32_launch_rows(M, N, K), m = M < rows ? M : rows, rest = M > m ? M % m : 0;
     const int64_t bytes = f32_scratch(m, K, f32_plan(m, N, K, ft_units()), step).bytes, more = rest ? f32_scratch(rest, K, f32_plan(rest, N, K, ft_units()), step).bytes : 0;
     return bytes > more ? bytes : more;
 }
@@ -679,13 +687,21 @@ inline cudaError_t launch_f32_tokens(const LinearArgs& a, const F32Plan& p, int 
     return e ? e : cudaGetLastError();
 }
 
-// false: not for this kernel (no memory, more tiles a cluster than `redo` has bits): linear_tiled_fma takes it
+// Few features over many tokens: hybrid_linear_f32_cta.cuh, which reads x once or a few times and writes nothing of it.  us there and here: 4096 x 8 x 2048 21, 39; 4096 x 128 x 4096 43, 73;
+// 804 x 32 x 2048 16, 19; 300 x 32 x 4096 21.5, 22.7; 2000 x 128 x 1024 19, 23; but 300 x 128 x 2048 20, 17.5, 2000 x 32 x 2048 29, 25 (its clusters of eight CTAs fill a second round),
+// 4096 x 256 x 2048 43, 43.  Up to 384 features where its tiles fill the SMs once and K is short: 3000 x 384 x 512 20, 24; 2000 x 256 x 1024 20, 22; 1200 x 384 x 1024 20, 22.5.
+inline bool f32_few_features(int M, int N, int K) {
+    if (N <= 128) return M > 4096 || (K >= 512 && (M > 2048 || (M > 1024 && K <= 1024) || (N <= 64 && M >= 256 && M <= 1024 && K >= 1024)));
+    return N <= 384 && M > 1024 && K >= 512 && K <= 1024 && ((M + 127) / 128) * ((N + 127) / 128) <= ft_units();
+}
+// false: not for this kernel (no memory, few features, more tiles a cluster than `redo` has bits)
 inline bool launch_linear_f32_pair(const LinearArgs& a, void* scratch, int64_t scratch_bytes, cudaStream_t st, cudaError_t& e) {
-    const int step = f32_step_of(a);
+    const int step = f32_step_of(a), rows = f32_launch_rows(a.M, a.N, a.K);
     const int64_t need = f32_scratch_bytes(a.M, a.N, a.K, step);
+    if (f32_few_features(a.M, a.N, a.K) || !ft_encode()) return false;
     {
-        const F32Plan p = f32_plan(a.M < FT_MAX_TOKENS ? a.M : FT_MAX_TOKENS, a.N, a.K, ft_units());
-        if (p.items / p.clusters >= 32 * FT_REDO_WORDS || !ft_encode()) return false;
+        const F32Plan p = f32_plan(a.M < rows ? a.M : rows, a.N, a.K, ft_units());
+        if (p.items / p.clusters >= 32 * FT_REDO_WORDS) return false;
     }
     if (!scratch || scratch_bytes < need || reinterpret_cast<uintptr_t>(scratch) % 16) {
         void* own = nullptr;
@@ -698,9 +714,9 @@ inline bool launch_linear_f32_pair(const LinearArgs& a, void* scratch, int64_t s
         if (!e) e = f;
         return taken;
     }
-    for (int m = 0; m < a.M; m += FT_MAX_TOKENS) {  // (rows of everything that a row of x makes)
+    for (int m = 0; m < a.M; m += rows) {  // (rows of everything that a row of x makes)
         LinearArgs b = a;
-        b.M = a.M - m < FT_MAX_TOKENS ? a.M - m : FT_MAX_TOKENS;
+        b.M = a.M - m < rows ? a.M - m : rows;
         b.ldx = a.x_pitch();
         const bool half = a.epi == EPI_GLU || a.epi == EPI_SWIGLU || a.epi == EPI_GEGLU;
         b.x = static_cast<const float*>(a.x) + (size_t)m * a.x_pitch();

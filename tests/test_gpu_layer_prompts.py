@@ -872,3 +872,15 @@ def test_heads_prepared_four_entries_a_lane(T, H, G, d, e, norm, mode, dt):
     lost = torch.ones(T + 5, dtype=torch.bool, device=DEV)
     lost[at] = False
     assert (ck[lost] == 7).all() and (cv[lost] == 7).all()
+
+
+@pytest.mark.parametrize("M,N,K", [(255, 64, 1024), (256, 64, 1024), (1024, 33, 1040), (1025, 65, 1024), (2049, 128, 512), (2049, 129, 512), (1153, 384, 1024), (3200, 384, 512), (4097, 128, 16), (4097, 300, 40), (8197, 8200, 32), (16385, 130, 24)])
+def test_fp32_linears_of_few_features_and_of_several_launches(M, N, K):
+    """Both sides of the lines at which x is no longer split ahead, and prompts of one row more than a launch takes."""
+    from mistral_inference_b200 import _abi_hybrid as h
+
+    g = torch.Generator(device=DEV).manual_seed(M)
+    x, w, rs = torch.randn(M, K, generator=g, device=DEV), torch.randn(N, K, generator=g, device=DEV) / K ** 0.5, torch.rand(M, (N + 7) // 8, generator=g, device=DEV)
+    got = h.linear_relu2(x, w, rs, 8)
+    assert rel(got, (x.double() @ w.double().T).clamp(min=0) ** 2 * rs.double().repeat_interleave(8, 1)[:, :N]) < 2 ** -21
+    assert torch.equal(got[-5:], h.linear_relu2(x, w, rs, 8)[-5:])
