@@ -158,15 +158,19 @@ def _aligned(*tensors: Optional[torch.Tensor]) -> bool:
 
 
 def _linear_f32(x, w, bias, out, out32, epi: int, n_act: int = 0, limit: float = 0.0, alpha: float = 0.0, rowscale=None, group: int = 0, a_log=None) -> bool:
-    """fp32 prompts: the call with room for the parts of x from the caching allocator.  False: a call that needs none."""
+    """fp32 prompts: the call with room for the parts of x from the caching allocator.  False: the caller's own call, which needs none: another kernel, slower for matrices of more than
+    a few features, that also runs where the room is not to be had (another order of sums)."""
     M, K, N = x.shape[0], x.shape[1], w.shape[0]
     if x.dtype != torch.float32 or M <= SKINNY_MAX_ROWS:
         return False
     need = lib().mbh_linear_scratch(M, N, K, 1)
     if not need:
         return False
+    try:
+        scratch = torch.empty(need, dtype=torch.uint8, device=x.device)
+    except torch.OutOfMemoryError:
+        return False
     xp, ldx = _rows(x)
-    scratch = torch.empty(need, dtype=torch.uint8, device=x.device)
     _check(lib().mbh_linear_any(xp, ldx, _ptr(w), _ptr(bias), _ptr(out), _ptr(out32), M, N, K, epi, n_act, limit, alpha, _ptr(rowscale), rowscale.shape[1] if rowscale is not None else 0,
                                 group, _ptr(a_log), _ptr(scratch), need, 1, _stream()), "mbh_linear_any")
     return True

@@ -27,7 +27,7 @@
 //
 // An infinity or a NaN in the operands of a tile, or a number from 2^120 on (256 x is formed): its outputs are computed again with FMAs (ft_fma_rows; one NaN among 804 x 16384 x 2048: 2046 us).
 //
-// Where x is the larger operand hybrid_linear_f32_cta.cuh runs.
+// The parts of x and the slots are room that the caller brings; without it, and where x is the larger operand, hybrid_linear_f32_cta.cuh runs.
 #pragma once
 #include <cuda.h>
 
@@ -694,25 +694,13 @@ inline bool f32_few_features(int M, int N, int K) {
     if (N <= 128) return M > 4096 || (K >= 512 && (M > 2048 || (M > 1024 && K <= 1024) || (N <= 64 && M >= 256 && M <= 1024 && K >= 1024)));
     return N <= 384 && M > 1024 && K >= 512 && K <= 1024 && ((M + 127) / 128) * ((N + 127) / 128) <= ft_units();
 }
-// false: not for this kernel (no memory, few features, more tiles a cluster than `redo` has bits)
+// false: not for this kernel (no room, few features, more tiles a cluster than `redo` has bits)
 inline bool launch_linear_f32_pair(const LinearArgs& a, void* scratch, int64_t scratch_bytes, cudaStream_t st, cudaError_t& e) {
     const int step = f32_step_of(a), rows = f32_launch_rows(a.M, a.N, a.K);
-    const int64_t need = f32_scratch_bytes(a.M, a.N, a.K, step);
-    if (f32_few_features(a.M, a.N, a.K) || !ft_encode()) return false;
+    if (f32_few_features(a.M, a.N, a.K) || !scratch || scratch_bytes < f32_scratch_bytes(a.M, a.N, a.K, step) || reinterpret_cast<uintptr_t>(scratch) % 16 || !ft_encode()) return false;
     {
         const F32Plan p = f32_plan(a.M < rows ? a.M : rows, a.N, a.K, ft_units());
         if (p.items / p.clusters >= 32 * FT_REDO_WORDS) return false;
-    }
-    if (!scratch || scratch_bytes < need || reinterpret_cast<uintptr_t>(scratch) % 16) {
-        void* own = nullptr;
-        if (cudaMallocAsync(&own, (size_t)need, st) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
-        const bool taken = launch_linear_f32_pair(a, own, need, st, e);
-        const cudaError_t f = cudaFreeAsync(own, st);
-        if (!e) e = f;
-        return taken;
     }
     for (int m = 0; m < a.M; m += rows) {  // (rows of everything that a row of x makes)
         LinearArgs b = a;

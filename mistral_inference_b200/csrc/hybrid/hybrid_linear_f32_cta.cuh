@@ -1,6 +1,7 @@
 // fp32 Linears of prompts by single CTAs, with no memory beside their operands: the arithmetic of hybrid_linear_f32.cuh, both operands split where they are used.
 //
-// For matrices of few features, where x is the larger operand and its parts, written out ahead and read back, cost more than splitting it once or twice here (f32_few_features).
+// For calls that bring no room for the parts of x (the entries of mistral_b200_hybrid.h allocate nothing) and for matrices of few features, where
+// x is the larger operand and its parts, written out ahead and read back, cost more than splitting it once or twice here (f32_few_features).
 //
 // CTA = 128 tokens x 128 features, or one of `splits` parts of their k range (a cluster; the parts are added through distributed shared memory in
 // rank order, so a small problem fills the chip and the result is the same every time).  17 warps: sixteen load fp32 from global memory

@@ -874,6 +874,68 @@ def test_heads_prepared_four_entries_a_lane(T, H, G, d, e, norm, mode, dt):
     assert (ck[lost] == 7).all() and (cv[lost] == 7).all()
 
 
+@pytest.mark.parametrize("M,N,K", [(9, 300, 64), (300, 2048, 1024), (130, 258, 132)])
+def test_fp32_entries_without_room_allocate_nothing(M, N, K):
+    """The entries of mistral_b200_hybrid.h bring no room for the parts of x and take none from the device: their results are fp32 numbers all the same, under capture too."""
+    from cuda.bindings import runtime as rt
+
+    from mistral_inference_b200 import _abi_hybrid as h
+
+    g = torch.Generator().manual_seed(M)
+    x, w, b = torch.randn(M, K, generator=g).to(DEV), (torch.randn(N, K, generator=g) / K ** 0.5).to(DEV), torch.randn(N, generator=g).to(DEV)
+    rs, a_log = torch.rand(M, (N + 7) // 8, generator=g).to(DEV), torch.linspace(-1, 1, N // 2, device=DEV)
+    y, F = x.double() @ w.double().T, torch.nn.functional
+    out = {k: torch.empty(M, N // 2 if k in ("glu", "swiglu") else N, device=DEV) for k in ("store", "glu", "swiglu", "relu2", "decay")}
+    lib, p = h.lib(), {k: v.data_ptr() for k, v in out.items()}
+
+    def calls(st):
+        X, Wp, B, R = x.data_ptr(), w.data_ptr(), b.data_ptr(), rs.data_ptr()
+        return [lib.mbh_linear(X, K, Wp, B, p["store"], None, M, N, K, 0, 0, 0.0, 0.0, 1, st), lib.mbh_linear_glu(X, Wp, p["glu"], M, N, K, 2.0, 1.7, R, rs.shape[1], 8, 1, st),
+                lib.mbh_linear_swiglu(X, Wp, p["swiglu"], M, N, K, R, rs.shape[1], 8, 0, 1, st), lib.mbh_linear_relu2(X, Wp, p["relu2"], M, N, K, R, rs.shape[1], 8, 1, st),
+                lib.mbh_linear_decay(X, K, Wp, B, a_log.data_ptr(), 2, p["decay"], M, N, K, 1, st)]
+
+    def check():
+        r = rs.double().repeat_interleave(8, 1)
+        gate, up = (y[:, i::2] * r[:, : N // 2] for i in (0, 1))
+        ref = {"store": y + b.double(), "glu": gate.clamp(max=2) * torch.sigmoid(1.7 * gate.clamp(max=2)) * (up.clamp(-2, 2) + 1), "swiglu": F.silu(y[:, 0::2]) * y[:, 1::2] * r[:, : N // 2],
+               "relu2": y.clamp(min=0) ** 2 * r[:, :N], "decay": torch.exp(-torch.exp(a_log.double().repeat_interleave(2)) * F.softplus(y + b.double()))}
+        for k, v in ref.items():
+            assert rel(out[k], v) < 2 ** -21, k
+
+    attr = rt.cudaMemPoolAttr.cudaMemPoolAttrUsedMemHigh
+    err, pool = rt.cudaDeviceGetDefaultMemPool(torch.cuda.current_device())
+    from cuda.bindings import driver
+
+    torch.cuda.synchronize()
+    rt.cudaMemPoolSetAttribute(pool, attr, driver.cuuint64_t(0))
+    assert calls(torch.cuda.current_stream().cuda_stream) == [0] * 5
+    torch.cuda.synchronize()
+    assert int(rt.cudaMemPoolGetAttribute(pool, attr)[1]) == 0
+    check()
+    for o in out.values():
+        o.fill_(7)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        assert calls(torch.cuda.current_stream().cuda_stream) == [0] * 5
+    graph.replay()
+    check()
+
+
+def test_fp32_linear_runs_where_its_room_is_not_to_be_had(monkeypatch):
+    from mistral_inference_b200 import _abi_hybrid as h
+
+    x, w, base, empty = torch.randn(300, 512, device=DEV), torch.randn(1024, 512, device=DEV) / 512 ** 0.5, torch.randn(300, 1024, device=DEV), torch.empty
+
+    def full(*a, **k):
+        if k.get("dtype") == torch.uint8:
+            raise torch.OutOfMemoryError("no room")
+        return empty(*a, **k)
+
+    monkeypatch.setattr(torch, "empty", full)
+    got = h.linear(x, w, None, epi=h.EPI_RESIDUAL, residual=base.clone())
+    assert rel(got, base.double() + x.double() @ w.double().T) < 2 ** -21
+
+
 @pytest.mark.parametrize("M,N,K", [(255, 64, 1024), (256, 64, 1024), (1024, 33, 1040), (1025, 65, 1024), (2049, 128, 512), (2049, 129, 512), (1153, 384, 1024), (3200, 384, 512), (4097, 128, 16), (4097, 300, 40), (8197, 8200, 32), (16385, 130, 24)])
 def test_fp32_linears_of_few_features_and_of_several_launches(M, N, K):
     """Both sides of the lines at which x is no longer split ahead, and prompts of one row more than a launch takes."""
