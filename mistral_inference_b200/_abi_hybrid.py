@@ -69,6 +69,7 @@ _SIGNATURES = {
 }
 _LINEAR_SIGNATURES = {  # mistral_b200_hybrid_linear.h
     "mbh_linear_scratch": (I, [I, I, I, c_int]),
+    "mbh_linear_any_scratch": (I, [I, I, I, c_int, I, F, F, c_int]),
     "mbh_linear_any": (c_int, [P, I, P, P, P, P, I, I, I, c_int, I, F, F, P, I, I, P, P, I, c_int, P]),
 }
 
@@ -163,7 +164,7 @@ def _linear_f32(x, w, bias, out, out32, epi: int, n_act: int = 0, limit: float =
     M, K, N = x.shape[0], x.shape[1], w.shape[0]
     if x.dtype != torch.float32 or M <= SKINNY_MAX_ROWS:
         return False
-    need = lib().mbh_linear_scratch(M, N, K, 1)
+    need = lib().mbh_linear_any_scratch(M, N, K, epi, n_act, limit, alpha, 1)
     if not need:
         return False
     try:

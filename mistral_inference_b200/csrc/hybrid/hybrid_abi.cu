@@ -194,8 +194,14 @@ int mbh_rmsnorm(const void* x32, const void* w, const void* w2, void* y, void* y
 }
 
 int64_t mbh_linear_scratch(int64_t M, int64_t N, int64_t K, int dt) {
-    if (dt != 1 || M <= SK_MAX_M || N <= 0 || K < FT_MIN_K || f32_few_features((int)M, (int)N, (int)K)) return 0;
+    if (dt != 1 || M <= SK_MAX_M || N <= 0 || K < FT_MIN_K) return 0;
     return f32_scratch_bytes((int)M, (int)N, (int)K, FT_TO_SLOTS);
+}
+
+int64_t mbh_linear_any_scratch(int64_t M, int64_t N, int64_t K, int epi, int64_t n_act, float limit, float alpha, int dt) {
+    if (dt != 1 || M <= SK_MAX_M || N <= 0 || K < FT_MIN_K || f32_few_features((int)M, (int)N, (int)K)) return 0;
+    const LinearArgs a{nullptr, nullptr, nullptr, nullptr, nullptr, (int)M, (int)N, (int)K, epi, (int)n_act, limit, alpha};
+    return f32_scratch_bytes((int)M, (int)N, (int)K, f32_step_of(a));
 }
 
 int mbh_linear_any(const void* x, int64_t ldx, const void* w, const void* bias, void* out, void* out32, int64_t M, int64_t N, int64_t K, int epi, int64_t n_act, float limit,

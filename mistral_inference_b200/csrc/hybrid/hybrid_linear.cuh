@@ -414,7 +414,7 @@ struct StreamEpi {
 
 namespace mbh {
 
-// scratch: fp32 prompts, of mbh_linear_scratch bytes; null or less: single CTAs, which need none
+// scratch: fp32 prompts, of mbh_linear_any_scratch bytes; null or less: single CTAs, which need none
 template <typename T>
 inline cudaError_t launch_linear(const LinearArgs& a, cudaStream_t st, void* scratch = nullptr, int64_t scratch_bytes = 0) {
     if (a.M <= 0 || a.N <= 0) return cudaSuccess;

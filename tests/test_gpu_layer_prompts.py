@@ -936,6 +936,28 @@ def test_fp32_linear_runs_where_its_room_is_not_to_be_had(monkeypatch):
     assert rel(got, base.double() + x.double() @ w.double().T) < 2 ** -21
 
 
+@pytest.mark.parametrize("kind,epi,kw", [("plain", 0, {}), ("logits", 3, dict(limit=5.0, alpha=2.0)), ("scaled add", 5, dict(alpha=0.3))])
+@pytest.mark.parametrize("M,N,K", [(9, 300, 64), (804, 2048, 1024), (449, 20480, 192)])
+def test_fp32_room_is_what_the_step_needs(M, N, K, kind, epi, kw):
+    """Room for the parts of x and for the slots of the tiles that have any: a plain store keeps none for whole tiles.  So many bytes are enough, nothing behind them is touched,
+    and the result is that of the Python call."""
+    from mistral_inference_b200 import _abi_hybrid as h
+
+    g = torch.Generator().manual_seed(M)
+    rnd = lambda *s: torch.randn(*s, generator=g).to(DEV)  # noqa: E731
+    x, w, b, base = rnd(M, K), rnd(N, K) / K ** 0.5, rnd(N), rnd(M, N)
+    want, _ = _f32_step(h, kind, x, w, b, None, base)
+    limit, alpha = kw.get("limit", 0.0), kw.get("alpha", 0.0)
+    need, every = h.lib().mbh_linear_any_scratch(M, N, K, epi, 0, limit, alpha, 1), h.lib().mbh_linear_scratch(M, N, K, 1)
+    assert 6 * M * K <= need <= every and (kind != "plain" or N < 20000 or need < every - M * N * 2)  # (the small ones are all cut)
+    room = torch.full((need + 4096,), 0x5a, dtype=torch.uint8, device=DEV)
+    out = torch.empty(M, N, device=DEV) if kind != "scaled add" else base.clone()
+    bias = None if kind == "logits" else b.data_ptr()
+    assert h.lib().mbh_linear_any(x.data_ptr(), K, w.data_ptr(), bias, out.data_ptr(), out.data_ptr(), M, N, K, epi, 0, limit, alpha, None, 0, 0, None, room.data_ptr(), need, 1,
+                                  torch.cuda.current_stream().cuda_stream) == 0
+    assert torch.equal(out, want) and (room[need:] == 0x5a).all()
+
+
 @pytest.mark.parametrize("M,N,K", [(255, 64, 1024), (256, 64, 1024), (1024, 33, 1040), (1025, 65, 1024), (2049, 128, 512), (2049, 129, 512), (1153, 384, 1024), (3200, 384, 512), (4097, 128, 16), (4097, 300, 40), (8197, 8200, 32), (16385, 130, 24)])
 def test_fp32_linears_of_few_features_and_of_several_launches(M, N, K):
     """Both sides of the lines at which x is no longer split ahead, and prompts of one row more than a launch takes."""
