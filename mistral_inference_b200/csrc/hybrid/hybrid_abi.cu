@@ -210,6 +210,8 @@ int mbh_linear_any(const void* x, int64_t ldx, const void* w, const void* bias, 
     if (epi < 0 || epi > EPI_DECAY) return bad("mbh_linear_any: unknown epilogue");
     if ((epi == EPI_GLU || epi == EPI_SWIGLU || epi == EPI_GEGLU) && (N & 1)) return bad("mbh_linear_any: the gated epilogues need interleaved (even) rows");
     if ((rowscale && rs_group <= 0) || (epi == EPI_DECAY && (!a_log || rs_group <= 0 || N % rs_group))) return bad("mbh_linear_any: groups of outputs");
+    const bool to32 = epi == EPI_RESIDUAL || epi == EPI_RESIDUAL_SCALED || epi == EPI_F32 || epi == EPI_DECAY;
+    if (M > 0 && N > 0 && (!x || !w || !(to32 ? out32 : out))) return bad("mbh_linear_any: null pointer");
     LinearArgs a{x, w, bias, out, (float*)out32, (int)M, (int)N, (int)K, epi, (int)n_act, limit, alpha, (const float*)rowscale, (int)rs_pitch, (int)rs_group};
     a.a_log = a_log;
     a.ldx = (int)ldx;

@@ -94,3 +94,14 @@ def test_the_stream_where_torch_has_no_raw_getter(monkeypatch):
     module = importlib.util.module_from_spec(spec)
     spec.loader.exec_module(module)
     assert module._stream() == 77
+
+
+@pytest.mark.parametrize("epi,missing", [(0, "x"), (1, "w"), (0, "out"), (2, "out"), (1, "out32"), (3, "out32"), (8, "out32")])
+def test_linears_without_an_operand_are_refused(epi, missing):
+    from mistral_inference_b200 import _abi_hybrid as h
+
+    p = {k: 4096 for k in ("x", "w", "out", "out32", "a_log")}  # never read: the call is refused before any launch
+    p[missing] = None
+    for dt in (0, 1):
+        assert h.lib().mbh_linear_any(p["x"], 64, p["w"], None, p["out"], p["out32"], 32, 64, 64, epi, 0, 0.0, 0.0, None, 0, 8, p["a_log"], None, 0, dt, None) != 0
+        assert "null pointer" in h.lib().mbh_last_error().decode()
