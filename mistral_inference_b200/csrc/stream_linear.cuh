@@ -3,17 +3,17 @@
 //
 // A CTA (one per SM) owns whole rows of W -- `rows` of them, a multiple of 8 with N / rows close to the number of SMs -- for all of K, so no sum crosses a CTA: there is
 // nothing to exchange and nobody to wait for at the end.  A producer thread keeps a ring of stages full by TMA: [rows x 64] blocks of W (128B-swizzled), `blocks` of them
-// along k so that a stage is 14 to 32 KB whatever `rows` is (47 from 17 tokens on), and the same columns of x.  The weights of the whole first ring are requested before the wait for the predecessor (nobody writes
+// along k so that a stage is 14 to 32 KB whatever `rows` is (47 from 17 tokens on; less where K has not so many, and one block where K is no multiple of 64), and the same columns of x.  The weights of the whole first ring are requested before the wait for the predecessor (nobody writes
 // weights), x after it.  Two teams of eight warps take the stages in turn (one stage's latencies lie under the other's) and multiply on mma.sync (m16n8k16: 16 rows of W x 8 tokens):
 // warp w of a team takes row tile w % tiles and every (8 / tiles)-th pair of slices of 16 columns; the sums meet in shared memory, in a fixed order.
 //
 // Why not tiles of 128 rows cut along k (gemm_streamk.cuh): with N / 128 = 16 .. 48 tiles for 148 SMs three or four CTAs finish a tile together, and the exchange through
-// memory is 6 to 10 us at the end of every launch.  Why not the weights straight into registers (a CTA per 16 rows, which this replaces in layered decoders): a fragment's lanes read 64
-// bytes of each of 8 rows, 8 tag lookups an instruction, 4 to 5 TB/s, and x came out of L2 in every step.
+// memory is 6 to 10 us at the end of every launch.  Why not the weights straight into registers (row_linear_kernel below, which small matrices keep): a fragment's lanes read 64
+// bytes of each of 8 rows, 8 tag lookups an instruction, 4 to 5 TB/s, and x comes out of L2 in every step.
 // What bounds it from 17 tokens on is mma.sync itself (7 tiles x 4 slices x 4 groups of tokens of a 13 KB stage take some 700 clocks, memory 600): 32 tokens 28672 x 5120 57 us, 24 tokens
 // 57, 8 tokens of that shape 49.  More warps or two row tiles a warp made it slower.
-// us a Linear in a chain of them, stored / added to the fp32 stream, that kernel and this one: 8 tokens 16384 x 2048 14.1 / 17.1, 12.9 / 12.8; 2048 x 8192 9.5 / 10.1, 8.4 / 8.2; 32768 x 2048
-// 24.9 / 30.1, 24.1 / 24.0 (5.6 TB/s); 2048 x 2048 2.7 / 3.2, 3.9 / 3.7; 16 tokens 28672 x 4096 57 / 155, 44 / 44.  Behind other kernels, whose ends its first ring covers, it gains more: a
+// us a Linear in a chain of them, stored / added to the fp32 stream, that kernel and this one: 8 tokens 16384 x 2048 17.0 / 16.4, 13.7 / 13.4; 2048 x 8192 10.3 / 10.1, 8.7 / 8.5;
+// 16 tokens 28672 x 4096 61 / 57, 45 / 44.  Behind other kernels, whose ends its first ring covers, it gains more: a
 // step of 8 layers of width 2048, 8 sequences, 698 and 529.  With one team of warps 28672 x 4096 took 47.6 us instead of 40, with a ring of 100 KB 43.
 #pragma once
 #include <cuda.h>
@@ -194,6 +194,83 @@ __global__ void __launch_bounds__(THREADS, 1) stream_linear_kernel(const __grid_
     }
 }
 
+// The same for matrices of few rows, the weights straight into registers: a CTA of eight warps per 16 rows of W, which split K; a lane takes 16 contiguous bytes of two rows and of
+// a token's x per step (the k order inside a step is permuted alike for both, which a dot product does not notice).  The weights of the first AHEAD steps -- all of them up to K = 2048 -- are
+// requested before the wait for the predecessor, and two CTAs fit an SM beside the predecessor's: there is no ring to fill, and a launch's head and tail
+// are shorter.  Needs K % 8 == 0 and 16-byte aligned rows.
+constexpr int ROWS_WARPS = 8, ROWS_AHEAD = 8;
+__device__ __forceinline__ uint4 load_weights(const __nv_bfloat16* p) {  // read once: not kept in L1
+    uint4 r;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
+    return r;
+}
+template <int NT, class Epi>
+__global__ void __launch_bounds__(ROWS_WARPS * 32, 2) row_linear_kernel(const __nv_bfloat16* X, int64_t pitch, const __nv_bfloat16* W, int M, int N, int K, const Epi epi) {
+    __shared__ float part[ROWS_WARPS][16][8 * NT + 1];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
+    const int n0 = blockIdx.x * 16, k0 = warp * 32 + tig * 8;
+    constexpr int STEP = ROWS_WARPS * 32;
+    const __nv_bfloat16* wa = W + (size_t)min(n0 + gid, N - 1) * K + k0;
+    const __nv_bfloat16* wb = W + (size_t)min(n0 + gid + 8, N - 1) * K + k0;
+    uint4 va[ROWS_AHEAD], vb[ROWS_AHEAD];
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int u = 0; u < ROWS_AHEAD; ++u) {
+        const bool ok = k0 + u * STEP < K;
+        va[u] = ok ? load_weights(wa + u * STEP) : zero;
+        vb[u] = ok ? load_weights(wb + u * STEP) : zero;
+    }
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int em = threadIdx.x % (8 * NT), er = threadIdx.x / (8 * NT) * 2, en = n0 + er;  // this thread's pair of results
+    const bool ends = threadIdx.x < 64 * NT && em < M && en < N;
+    typename Epi::Ahead ahead;
+    if (ends) ahead = epi.fetch(em, en, en + 1 < N);
+    float c[NT][4];
+    const __nv_bfloat16* xr[NT];
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+        c[t][0] = c[t][1] = c[t][2] = c[t][3] = 0.f;
+        xr[t] = X + (size_t)min(t * 8 + gid, M - 1) * pitch + k0;  // rows past the end repeat the last one: their sums go nowhere
+    }
+    const int steps = (K + STEP - 1) / STEP;
+    for (int i = 0; i < steps; i += ROWS_AHEAD) {
+#pragma unroll
+        for (int u = 0; u < ROWS_AHEAD; ++u) {
+            const int k = (i + u) * STEP;
+            uint4 vx[NT];
+#pragma unroll
+            for (int t = 0; t < NT; ++t) vx[t] = k0 + k < K ? *reinterpret_cast<const uint4*>(xr[t] + k) : zero;
+            const uint32_t a0[4] = {va[u].x, vb[u].x, va[u].y, vb[u].y}, a1[4] = {va[u].z, vb[u].z, va[u].w, vb[u].w};
+#pragma unroll
+            for (int t = 0; t < NT; ++t) {
+                mma(c[t], a0, vx[t].x, vx[t].y);
+                mma(c[t], a1, vx[t].z, vx[t].w);
+            }
+            const bool more = k0 + k + ROWS_AHEAD * STEP < K;
+            va[u] = more ? load_weights(wa + k + ROWS_AHEAD * STEP) : zero;
+            vb[u] = more ? load_weights(wb + k + ROWS_AHEAD * STEP) : zero;
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+        part[warp][gid][t * 8 + tig * 2] = c[t][0];
+        part[warp][gid][t * 8 + tig * 2 + 1] = c[t][1];
+        part[warp][gid + 8][t * 8 + tig * 2] = c[t][2];
+        part[warp][gid + 8][t * 8 + tig * 2 + 1] = c[t][3];
+    }
+    __syncthreads();
+    if (ends) {
+        float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+        for (int w = 0; w < ROWS_WARPS; ++w) {
+            s0 += part[w][er][em];
+            s1 += part[w][er + 1][em];
+        }
+        epi.finish(em, en, s0, s1, en + 1 < N, ahead);
+    }
+}
+
 // ---- host ----
 typedef CUresult (*Encode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                            CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -211,6 +288,31 @@ inline bool make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t K
     const cuuint32_t box[3] = {64u, (cuuint32_t)blocks, (cuuint32_t)box_rows}, unit[3] = {1u, 1u, 1u};
     return encode()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, unit, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// a launch that may begin before its predecessor in the stream has ended
+template <class Kernel, class... Args>
+inline cudaError_t launch_serial(Kernel kernel, int ctas, int threads, size_t smem, cudaStream_t st, const Args&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)ctas);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+// Which of the two, up to 16 rows of x: the one without a ring where the ring would take k-blocks one by one, and for small matrices.  us in a chain of Linears / behind a row norm, 8 rows of x, here
+// and there: K = 1000 and 4096 rows 3.0 / 4.7, 5.7 / 6.7; 8192 5.7 / 7.7, 7.1 / 8.3; 16384 10.5, 9.3; 1024 x 64 1.7 / 3.4, 2.6 / 3.5; 1024 x 1024 2.2 / 3.8, 3.2 / 4.3; 2048 x 2048 3.0 / 4.9, 4.0 / 5.6.  Larger ones
+// gain in such a chain (4096 x 4096 8.1, 8.5) and lose in a model's step, where the ring fills while other kernels end (two layers of the 7B shape, 8 sequences 283, 272;
+// with 4096 x 14336 here too 335; eight layers of width 2048, 2048 x 2048 and 3072 x 2048 here: one sequence 431, 442, eight 502, 495).  From 9 rows of x on: behind a norm 2048 x 256 4.6, 3.9.
+inline bool rows_better(int M, int N, int K, int64_t pitch) {
+    if (K % 64 != 0 || pitch % 64 != 0) return N <= (M <= 8 && K >= 512 ? 8192 : 4096);
+    return M <= 8 && N <= 4096 && K <= (M <= 4 ? 2048 : 1024);
 }
 
 template <int NT>
@@ -237,6 +339,11 @@ template <int NT, class Epi>
 inline bool launch(const void* x, int64_t pitch, const void* w, int M, int N, int K, const Epi& epi, cudaStream_t st, cudaError_t& e) {
     e = cudaSuccess;
     const int sms = device_info::sm_count();
+    if constexpr (NT <= 2)
+        if (rows_better(M, N, K, pitch)) {
+            e = launch_serial(row_linear_kernel<NT, Epi>, (N + 15) / 16, ROWS_WARPS * 32, 0, st, static_cast<const __nv_bfloat16*>(x), pitch, static_cast<const __nv_bfloat16*>(w), M, N, K, epi);
+            return true;
+        }
     if (sms == 0 || !encode()) return false;
     const Shape s = shape_of<NT>(M, N, K, pitch, sms);
     CUtensorMap map_x, map_w;
@@ -247,17 +354,7 @@ inline bool launch(const void* x, int64_t pitch, const void* w, int M, int N, in
     auto kernel = stream_linear_kernel<NT, Epi>;
     e = device_info::allow_shared<stream_linear_kernel<NT, Epi>>(RING_BYTES + 1024 + (int)sizeof(float) * 8 * NT * SUM_PITCH);
     if (e) return true;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(units < sms ? units : sms));
-    cfg.blockDim = dim3(THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, kernel, map_x, map_w, s, epi);
+    e = launch_serial(kernel, units < sms ? units : sms, THREADS, smem, st, map_x, map_w, s, epi);
     return true;
 }
 

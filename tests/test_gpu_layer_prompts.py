@@ -754,9 +754,11 @@ def test_fp32_linear_of_more_rows_than_a_launch_takes():
 
 
 @pytest.mark.parametrize("M", [1, 8, 9, 16])
-@pytest.mark.parametrize("N,K,pad", [(1, 8, 0), (130, 72, 8), (1024, 64, 0), (1186, 192, 64), (3072, 2048, 0), (2049, 1416, 0), (8192, 448, 16), (18961, 128, 0), (38000, 320, 0)])
+@pytest.mark.parametrize("N,K,pad", [(1, 8, 0), (130, 72, 8), (1024, 64, 0), (1186, 192, 64), (3072, 2048, 0), (2049, 1416, 0), (8192, 448, 16), (18961, 128, 0), (38000, 320, 0),
+                                     (4096, 2112, 0), (4097, 2048, 0), (1184, 4096, 0), (3071, 4160, 0), (3072, 4160, 0), (8192, 1000, 0), (8200, 1000, 0), (40, 264, 0)])
 def test_decode_linear_streams_whole_rows(M, N, K, pad):
-    """Rows of 8 to 128 a CTA, one and several units of them, the last ones short, k-blocks that end inside a stage and inside a block, x in a wider matrix: a bf16 Linear is within its
+    """Rows of 8 to 128 a CTA, one and several units of them, the last ones short, k-blocks that end inside a stage and inside a block, x in a wider matrix; matrices of few rows, 16 a CTA, on
+    both sides of that line: a bf16 Linear is within its
     rounding (2^-8) of float64, what stays fp32 within 2 K 2^-24 of the products' sizes."""
     from mistral_inference_b200 import _abi_hybrid as h
 
