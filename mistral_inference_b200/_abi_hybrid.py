@@ -153,6 +153,15 @@ def _prompt_gemm_ok(x: torch.Tensor, M: int, N: int, K: int) -> bool:
             and _abi.library_path().exists())
 
 
+COPIED_ROWS_FROM = 17  # fewer rows run on registers or FMAs from wherever they lie
+
+
+def _streamed_as_it_lies(x: torch.Tensor) -> bool:
+    """Rows of a wider matrix that the streaming kernel reads as fast as rows of their own: 16-byte addresses, pitches of whole k-blocks where K is one.  Others are copied first: 32 rows of
+    2048 columns, pitch 2056, times 1024 features: 12.2 us as they lie, 8.7 copied; pitch 2052, which only mma.sync tiles read, 173 and 8.7."""
+    return x.data_ptr() % 16 == 0 and x.stride(0) % (64 if x.shape[1] % 64 == 0 else 8) == 0
+
+
 def _aligned(*tensors: Optional[torch.Tensor]) -> bool:
     """16-byte aligned starts: what the tensor-core GEMM's copies and vector accesses need."""
     return all(t is None or t.data_ptr() % 16 == 0 for t in tensors)
@@ -200,6 +209,8 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None
             return out if out is not None else out32
     if _linear_f32(x, w, bias, out, out32, epi, n_act, limit, alpha):
         return out if out is not None else out32
+    if x.dtype == torch.bfloat16 and COPIED_ROWS_FROM <= M <= STREAM_MAX_ROWS and not _streamed_as_it_lies(x):
+        x = x.contiguous()
     xp, ldx = _rows(x)
     _check(lib().mbh_linear(xp, ldx, _ptr(w), _ptr(bias), _ptr(out), _ptr(out32), M, N, K, epi, n_act, limit, alpha, dt_of(x.dtype), _stream()),
            "mbh_linear")

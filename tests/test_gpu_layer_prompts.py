@@ -970,3 +970,18 @@ def test_fp32_linears_of_few_features_and_of_several_launches(M, N, K):
     got = h.linear_relu2(x, w, rs, 8)
     assert rel(got, (x.double() @ w.double().T).clamp(min=0) ** 2 * rs.double().repeat_interleave(8, 1)[:, :N]) < 2 ** -21
     assert torch.equal(got[-5:], h.linear_relu2(x, w, rs, 8)[-5:])
+
+
+@pytest.mark.parametrize("M", [9, 16, 17, 24, 32])
+@pytest.mark.parametrize("K,first,pitch", [(512, 0, 516), (512, 0, 520), (512, 4, 576), (520, 0, 524), (520, 1, 528), (512, 64, 640)])
+def test_decode_rows_of_a_wider_matrix(M, K, first, pitch):
+    """Rows that start, or follow one another, off the 16-byte grid or off the k-blocks: from 17 on the same bits as rows of their own, which stream (they ran on mma.sync tiles, 25 times
+    as long); fewer are read as they lie."""
+    from mistral_inference_b200 import _abi_hybrid as h
+
+    g = torch.Generator(device=DEV).manual_seed(M + K)
+    x = torch.randn(M, pitch + 8, generator=g, device=DEV).bfloat16().flatten()[: M * pitch].view(M, pitch)[:, first:first + K]
+    w = (torch.randn(1024, K, generator=g, device=DEV) / K ** 0.5).bfloat16()
+    got, own = (h.linear(t, w, None, epi=h.EPI_F32) for t in (x, x.contiguous()))
+    assert rel(got, x.double() @ w.double().T) < 2 * K * 2.0 ** -24
+    assert M < 17 or torch.equal(got, own)
