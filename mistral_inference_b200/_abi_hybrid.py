@@ -140,17 +140,22 @@ def rmsnorm_pair(x32: torch.Tensor, w: torch.Tensor, w2: torch.Tensor, eps: floa
 
 
 SKINNY_MAX_ROWS = 8  # of fp32: more rows run on tensor cores
-PROMPT_GEMM_MIN_ROWS = 17
 STREAM_MAX_ROWS = 32  # so many rows of bf16 run on this library's own kernel, which streams the weights past them: 20 tokens through two layers of width 2048 268 us, 185 with it
 
 
 def _prompt_gemm_ok(x: torch.Tensor, M: int, N: int, K: int) -> bool:
-    """Large bf16 Linears of prompts go to the main library's tcgen05 GEMMs (`_abi.layer_linear`: the step after the Linear is the
-    epilogue; up to 128 rows tiles streamed in one range a CTA, above the persistent kernels) when it is built and the shape fits their tiles (K % 64 == 0,
-    N % 128 == 0); everything else runs on this library's own kernels.  A checkout that has only libmb200_hybrid.so never builds the main
+    """Whether the main library's tcgen05 GEMMs (`_abi.layer_linear`: the step after the Linear is the epilogue; up to 128 rows tiles streamed in one range a CTA, above the
+    persistent kernels) take this Linear: it is built and the shape fits their tiles (K % 64 == 0, N % 128 == 0).  A checkout that has only libmb200_hybrid.so never builds the main
     library for this."""
-    return (x.dtype == torch.bfloat16 and M >= PROMPT_GEMM_MIN_ROWS and K % 64 == 0 and N % 128 == 0 and os.environ.get("MB200_HYBRID_GEMM", "1") != "0"
-            and _abi.library_path().exists())
+    return (x.dtype == torch.bfloat16 and K % 64 == 0 and N % 128 == 0 and os.environ.get("MB200_HYBRID_GEMM", "1") != "0"
+            and build.LIB.exists())
+
+
+def _prompt_gemm(x: torch.Tensor, M: int, N: int, K: int) -> bool:
+    """Whether a bf16 Linear goes there: from 33 rows on, and fewer times a matrix so wide that mma.sync bounds the streaming kernel.  us there and on streamed tiles: 32 rows 16384 x 1024
+    14.1, 11.6; 28672 x 4096 67, 46; 17 rows 52, 44; but 24 rows 16384 x 4096 30.9, 30.0; 32 rows 8192 x 4096 18.8, 18.2.  Everything else runs on this library's own kernels."""
+    wide = K >= 1024 and (N >= 16384 if M > 24 else M > 16 and N >= 24576)
+    return (M > STREAM_MAX_ROWS or wide) and _prompt_gemm_ok(x, M, N, K)
 
 
 COPIED_ROWS_FROM = 17  # fewer rows run on registers or FMAs from wherever they lie
@@ -202,7 +207,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None
         out32 = torch.empty(M, N, dtype=torch.float32, device=x.device)
     else:
         out = torch.empty(M, N // 2 if epi == EPI_GLU else N, dtype=x.dtype, device=x.device)
-    if M > STREAM_MAX_ROWS and _prompt_gemm_ok(x, M, N, K) and _aligned(w, bias, out32) and epi in (EPI_STORE, EPI_RESIDUAL, EPI_RESIDUAL_SCALED, EPI_F32, EPI_GLU):
+    if _prompt_gemm(x, M, N, K) and _aligned(w, bias, out32) and epi in (EPI_STORE, EPI_RESIDUAL, EPI_RESIDUAL_SCALED, EPI_F32, EPI_GLU):
         xc = x.contiguous()
         if _aligned(xc):
             _abi.layer_linear(xc, w, bias, out, out32, epi, n_act, limit, alpha)
@@ -340,7 +345,7 @@ def linear_swiglu(x: torch.Tensor, w: torch.Tensor, rowscale: Optional[torch.Ten
         assert rowscale.dtype == torch.float32 and rowscale.shape[0] == M and group > 0 and (N // 2 + group - 1) // group <= rowscale.shape[1]
         pitch = rowscale.shape[1]
     out = torch.empty(M, N // 2, dtype=x.dtype, device=x.device)
-    if M > STREAM_MAX_ROWS and _prompt_gemm_ok(x, M, N, K) and _aligned(x, w):
+    if _prompt_gemm(x, M, N, K) and _aligned(x, w):
         _abi.layer_linear(x, w, None, out, None, EPI_GEGLU if gelu else EPI_SWIGLU, rowscale=rowscale, group=max(group, 1))
         return out
     if _linear_f32(x, w, None, out, None, EPI_GEGLU if gelu else EPI_SWIGLU, rowscale=rowscale, group=group):
@@ -681,7 +686,7 @@ def linear_glu(x: torch.Tensor, w: torch.Tensor, limit: float, alpha: float, row
         assert rowscale.dtype == torch.float32 and rowscale.shape[0] == M and group > 0 and (N // 2 + group - 1) // group <= rowscale.shape[1]
         pitch = rowscale.shape[1]
     out = torch.empty(M, N // 2, dtype=x.dtype, device=x.device)
-    if M > STREAM_MAX_ROWS and _prompt_gemm_ok(x, M, N, K) and _aligned(x, w):
+    if _prompt_gemm(x, M, N, K) and _aligned(x, w):
         _abi.layer_linear(x, w, None, out, None, EPI_GLU, limit=limit, alpha=alpha, rowscale=rowscale, group=max(group, 1))
         return out
     if _linear_f32(x, w, None, out, None, EPI_GLU, limit=limit, alpha=alpha, rowscale=rowscale, group=group):
@@ -765,7 +770,7 @@ def linear_relu2(x: torch.Tensor, w: torch.Tensor, rowscale: Optional[torch.Tens
         assert rowscale.dtype == torch.float32 and rowscale.shape[0] == M and group > 0 and (N + group - 1) // group <= rowscale.shape[1]
         pitch = rowscale.shape[1]
     out = torch.empty(M, N, dtype=x.dtype, device=x.device)
-    if M > STREAM_MAX_ROWS and _prompt_gemm_ok(x, M, N, K) and _aligned(x, w):
+    if _prompt_gemm(x, M, N, K) and _aligned(x, w):
         _abi.layer_linear(x, w, None, out, None, EPI_RELU2, rowscale=rowscale, group=max(group, 1))
         return out
     if _linear_f32(x, w, None, out, None, EPI_RELU2, rowscale=rowscale, group=group):

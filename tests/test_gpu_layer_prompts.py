@@ -633,10 +633,10 @@ def test_scoring_counts_logits_that_are_no_numbers(T, cols, value):
     assert (got - ref)[ok].abs().max() <= 1e-5 * 10 + (2 * step if T == 128 else 0.0) if ok.any() else True
 
 
-@pytest.mark.parametrize("T", [17, 32, 33, 64, 65, 127, 128, 171, 600])
-@pytest.mark.parametrize("N,K", [(256, 128), (4096, 8192), (4224, 128)])  # the last: at 600 rows pairs, half a tile of weights at the end
+@pytest.mark.parametrize("T", [16, 17, 24, 25, 32, 33, 64, 65, 127, 128, 171, 600])
+@pytest.mark.parametrize("N,K", [(256, 128), (4096, 8192), (4224, 128), (16384, 1024), (24576, 1024)])  # the third: at 600 rows pairs, half a tile of weights at the end
 def test_prompt_linear_steps_by_rows(T, N, K):
-    """The steps behind a prompt's Linear at every change of kernel over the rows (stream-K boxes, single tiles, pairs cut along k): bf16 results
+    """The steps behind a prompt's Linear at every change of kernel over the rows (whole rows streamed, tiles streamed, single tiles, pairs cut along k): bf16 results
     within a rounding (2^-8) of float64, fp32 ones within 2^-8 of the sum's scale for the rounded sum that is added."""
     from mistral_inference_b200 import _abi_hybrid as h
 
@@ -645,7 +645,7 @@ def test_prompt_linear_steps_by_rows(T, N, K):
     b, base, rs = torch.randn(N, device=DEV, generator=g).bfloat16(), torch.randn(T, N, device=DEV, generator=g), torch.rand(T, 2, device=DEV, generator=g)
     z = x.double() @ w.double().T
     zb = z + b.double()
-    assert h._prompt_gemm_ok(x, T, N, K)
+    assert h._prompt_gemm_ok(x, T, N, K) and h._prompt_gemm(x, T, N, K) == (T > 32 or (T > 24 and N >= 16384) or (T > 16 and N >= 24576))
     assert rel(h.linear(x, w, b, n_act=N // 2), torch.cat((torch.nn.functional.silu(zb[:, : N // 2]), zb[:, N // 2:]), 1)) < 2 ** -8
     assert rel(h.linear(x, w, b, epi=h.EPI_F32, alpha=0.5), 0.5 * zb) < 1e-5
     assert rel(h.linear(x, w, epi=h.EPI_RESIDUAL, residual=base.clone()) - base, z) < 2 ** -8
