@@ -574,17 +574,28 @@ def attn_decode_ok(q: torch.Tensor, H: int, G: int, d: int, e: int, maps: int = 
     return q.dtype == torch.bfloat16 and H // G <= DECODE_MAX_GROUP and (d, e) in DECODE_SIZES[maps] and os.environ.get("MB200_ATTN_DECODE", "1") != "0"
 
 
-def attn_decode_splits(B: int, G: int, W: int, n_sm: int = 148) -> int:
-    """CTAs per (sequence, key/value head) along the keys: at most two per SM over the batch -- as many as run at once; a few more would run alone in a second round --, at
-    least one round of 64 ring rows each (batch and ring size only, so a captured decode graph stays valid as the context grows)."""
-    return int(max(1, min(2 * n_sm // (B * G), (W + 63) // 64, 64)))
+def attn_decode_splits(B: int, G: int, W: int, n_sm: int = 148, per_sm: int = 2) -> int:
+    """CTAs per (sequence, key/value head) along the keys: at most `per_sm` per SM over the batch -- as many as run at once; a few more would run alone in a second round --, at
+    least one round of 64 ring rows each (batch and ring size only, so a captured decode graph stays valid as the context grows).  Two where one would leave a quarter of those
+    places empty: 200 pairs of 3000 tokens, two maps 102 us with one, 88; groups of 16 heads of 128 94, 84."""
+    pairs, places = B * G, per_sm * n_sm
+    splits = places // pairs
+    if splits == 1 and 4 * pairs < 3 * places:
+        splits = 2
+    return int(max(1, min(splits, (W + 63) // 64, 64)))
+
+
+def _decode_ctas(B: int, H: int, G: int, d: int, e: int, maps: int) -> int:
+    """CTAs of a decode step's attention that an SM holds: of groups of more than 8 heads four where keys and values are small; few pairs gain nothing by it (us for 64 pairs of
+    3000 tokens, 16 heads of 64, with two 23.1, 20.2 with four; 37 15.8, 13.8; 20 11.8, 13.6)."""
+    return 4 if H // G > 8 and maps * d + e <= 128 and B * G >= 32 else 2
 
 
 def attn_decode(q, cache_k, cache_v, positions, slots, out, B: int, W: int, H: int, G: int, d: int, e: int, scale: float, window: int, softcap: float = 0.0, sink=None,
                 chunked: bool = False, gate=None, gate_entry: bool = False, lam=None, out_scale: float = 1.0, norm_eps: float = 0.0, splits: int = 0) -> None:
     """`attn_window` for one token per sequence on tensor cores (attn_decode_ok says when)."""
     maps = 1 if lam is None else 2
-    splits = splits or attn_decode_splits(B, G, W)
+    splits = splits or attn_decode_splits(B, G, W, per_sm=_decode_ctas(B, H, G, d, e, maps))
     scratch = torch.empty(B * H * maps * splits * (2 + e), dtype=torch.float32, device=q.device)
     gp, g_pitch = _rows(gate) if gate is not None else (None, 0)
     assert gate is None or (gate.dtype == q.dtype and gate.shape == (B, H * e if gate_entry else H))
@@ -606,7 +617,7 @@ def attn_bias_decode_ok(q: torch.Tensor, cache_k: torch.Tensor, cache_v: torch.T
 def attn_bias_decode(q, cache_k, cache_v, bias_tab, positions, slots, out, B: int, W: int, H: int, G: int, d: int, e: int, scale: float) -> None:
     """`attn_bias` for one token per sequence on tensor cores (attn_bias_decode_ok says when)."""
     _check_bias_table(bias_tab, H)
-    splits = attn_decode_splits(B, G, W)
+    splits = attn_decode_splits(B, G, W, per_sm=_decode_ctas(B, H, G, d, e, 1))
     scratch = torch.empty(B * H * splits * (2 + e), dtype=torch.float32, device=q.device)
     _check(lib().mbh_attn_bias_decode(_ptr(q), _ptr(cache_k), _ptr(cache_v), _ptr(bias_tab), bias_tab.shape[0], _ptr(positions), _ptr(slots), _ptr(out), B, W, H, G, d, e,
                                       scale, splits, _ptr(scratch), _stream()), "mbh_attn_bias_decode")

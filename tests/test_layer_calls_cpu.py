@@ -105,3 +105,14 @@ def test_linears_without_an_operand_are_refused(epi, missing):
     for dt in (0, 1):
         assert h.lib().mbh_linear_any(p["x"], 64, p["w"], None, p["out"], p["out32"], 32, 64, 64, epi, 0, 0.0, 0.0, None, 0, 8, p["a_log"], None, 0, dt, None) != 0
         assert "null pointer" in h.lib().mbh_last_error().decode()
+
+
+@pytest.mark.parametrize("B,H,G,d,W,splits", [(1, 8, 8, 128, 4096, 37), (148, 8, 1, 128, 4096, 2), (149, 8, 1, 128, 4096, 2), (221, 8, 1, 128, 4096, 2), (222, 8, 1, 128, 4096, 1), (600, 8, 1, 128, 4096, 1),
+                                              (64, 16, 1, 128, 4096, 4), (64, 16, 1, 64, 4096, 9), (64, 8, 1, 64, 4096, 4), (31, 16, 1, 64, 4096, 9), (32, 16, 1, 64, 4096, 18), (443, 16, 1, 64, 4096, 2),
+                                              (444, 16, 1, 64, 4096, 1), (1, 8, 1, 128, 64, 1), (1, 8, 1, 128, 65, 2), (1, 1, 1, 64, 100000, 64)])
+def test_decode_attention_fills_the_places_there_are(B, H, G, d, W, splits):
+    from mistral_inference_b200 import _abi_hybrid as h
+
+    got = h.attn_decode_splits(B, G, W, per_sm=h._decode_ctas(B, H, G, d, d, 1))
+    assert got == splits and 1 <= got <= 64
+    assert got <= 2 or got * B * G <= 148 * h._decode_ctas(B, H, G, d, d, 1)
