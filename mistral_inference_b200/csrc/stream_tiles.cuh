@@ -183,11 +183,18 @@ __global__ void __launch_bounds__(SC_THREADS) stream_tiles_combine_kernel(const 
 // (128 tokens, which run on no pairs: 5120 x 5120 31, 30, 5120 x 14336 66, 50, but 6144 x 4096 29, 30.)
 inline bool stream_tiles_better(int64_t T, int64_t N, int64_t K) { return T < TG_BM || (T == TG_BM && K >= 5120) || (T <= ST_MAX_T && K >= 8192 && N <= 4096); }
 
+// CTAs: every SM, but at most twelve a tile where tiles are few: a tile's pieces are added one after another.  us with all SMs and with twelve a tile: 128 tokens 256 x 8192 58, 16; 128 x 5120
+// 54, 14; 1024 x 8192 21, 20; with more than 128 tokens from seven tiles on the pieces' own length counts for more: 160 tokens 768 x 8192 26, 18.5; 1024 x 14336 23.6, 24.9.
+inline int stream_tiles_grid(int64_t T, int64_t N, int64_t K, int sms) {
+  const int64_t tiles = N / ST_ROWS, units = tiles * (K / TG_BK), most = T <= TG_BM || tiles <= 6 ? 12 * tiles : sms;
+  return (int)(units < sms ? (units < most ? units : most) : most < sms ? most : sms);
+}
+
 // bytes of slots, 0: not for this kernel
 inline size_t stream_tiles_bytes(int64_t T, int64_t N, int64_t K, int sms) {
   const char* e = getenv("MB200_STREAMK");
   if (sms < 1 || (e != nullptr && e[0] == '0') || T < 1 || !stream_tiles_better(T, N, K) || N % ST_ROWS != 0 || K % TG_BK != 0) return 0;
-  const int64_t tiles = N / ST_ROWS, units = tiles * (K / TG_BK), grid = units < sms ? units : sms;
+  const int64_t tiles = N / ST_ROWS, grid = stream_tiles_grid(T, N, K, sms);
   const size_t bytes = (size_t)(grid + tiles - 1) * st_piece(T) * sizeof(float);
   return bytes <= ST_SLOT_BYTES ? bytes : 0;
 }
@@ -202,8 +209,7 @@ int launch_stream_tiles(const GemmParams& g, int sms, void* slots, cudaStream_t 
   if (p.cols == 128 || p.cols == 192) p.cols += 16;  // measured: 128 tokens 5120 x 14336 56 us at 128 columns, 50 at 144; 192 60, (224: 56).  The stages are then 16-KB multiples; why that costs is not known
   const int stage_bytes = ST_W_BYTES + p.cols * TG_BK * 2;
   p.stages = ST_RING / stage_bytes < ST_MAX_STAGES ? ST_RING / stage_bytes : ST_MAX_STAGES;
-  const long long units = (long long)(g.N / ST_ROWS) * (g.K / TG_BK);
-  p.grid = (int)(units < sms ? units : sms);
+  p.grid = stream_tiles_grid(g.T, g.N, g.K, sms);
   p.epi = g.epi;
   p.slots = reinterpret_cast<float*>(slots);
   CUtensorMap map_a, map_w;

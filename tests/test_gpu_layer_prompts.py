@@ -814,9 +814,9 @@ def test_decode_steps_linears_against_float64(T):
 
 
 @pytest.mark.parametrize("T,N,K", [(33, 128, 64), (48, 384, 128), (49, 1024, 640), (64, 6144, 192), (65, 2176, 1024), (112, 640, 2048), (113, 4096, 320), (127, 20480, 128), (128, 256, 8192),
-                                   (129, 1152, 8256), (192, 128, 8192), (193, 1024, 8192), (256, 4096, 8192)])
+                                   (129, 1152, 8256), (192, 128, 8192), (193, 1024, 8192), (256, 4096, 8192), (128, 128, 5120), (33, 128, 768), (100, 1664, 832), (129, 768, 8192), (256, 896, 8256), (64, 1536, 704)])
 def test_linears_over_streamed_tiles(T, N, K):
-    """Fewer and more units than SMs, tiles in one piece and in many, tokens at the edges of the MMA's columns and of the accumulators: against float64, for the dense model's steps (bf16
+    """Fewer and more units than SMs and than twelve a tile, tiles in one piece and in many, tokens at the edges of the MMA's columns and of the accumulators: against float64, for the dense model's steps (bf16
     results: 2^-8) and a layered decoder's (fp32 residual and logits); twice the same bits."""
     from mistral_inference_b200 import _abi, _abi_hybrid as h
 
