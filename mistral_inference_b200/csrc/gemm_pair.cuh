@@ -22,8 +22,9 @@
 // GROUPED: the mixtures' form, token tiles from the plan of moe.cuh (pair_expert, pair_info), weights by expert; nothing is cut.  Token tiles there are 32 to 256 wide, and a tile's time
 // follows its width: clusters that take every n_cta-th tile drift apart by rounds, and the two or three that share an expert's weight tile no longer meet in L2 (2048 tokens, eight
 // experts of 4096 x 14336: 5.4 GB read from memory, 3.9 with the draw).  So a cluster takes the next tile that nobody has: the first CTA's producer draws it from a counter shortly before
-// it needs it and hands it to the warps of both CTAs (tile_full, tile_empty): 1545 us without, 1470 with.  Short tiles are dealt, their hand-over costs more (16 experts of 2048 x 1408,
-// 2500 tokens: 232 us dealt, 244 drawn); the line (GP_DRAW_MIN_K) lies between K = 2048 and 4096.
+// it needs it and hands it to the warps of both CTAs (tile_full, tile_empty): 1545 us without, 1470 with.  Short tiles are dealt, their hand-over costs more (both GEMMs of a layer,
+// dealt and drawn, us: 16 experts of 2048 x 1408, 2500 tokens 195, 207; 3072 x 1408 278, 287; eight of 2560 x 5120 349, 361; 3072 x 8192 640, 643; 3584 x 10240 901, 901; 4096 x 14336 1459, 1428): the line
+// is GP_DRAW_MIN_K.
 #pragma once
 #include <type_traits>
 
@@ -35,7 +36,7 @@ constexpr int GP_ROWS = 256;                         // features a tile
 constexpr int GP_EPI_WARPS = 8, GP_THREADS = 64 + 32 * GP_EPI_WARPS;
 constexpr int GP_W_BYTES = TG_BM * TG_BK * 2;        // a CTA's half of the weight tile, per stage
 constexpr int GP_MAX_STAGES = 7, GP_SHAPES = 16, GP_INFO = 32, GP_DRAWN = 4;
-constexpr int GP_DRAW_MIN_K = 3072;
+constexpr int GP_DRAW_MIN_K = 4096;
 constexpr int GP_DRAW_AHEAD = 24, GP_HAND_AHEAD = 14;  // k-blocks before a tile's last: the draw's way to memory and back, and the hand-over's to the other CTA, lie under copies
 static_assert(GP_SHAPES > GP_MAX_STAGES + 1, "see shape_s");
 template <int MODE>

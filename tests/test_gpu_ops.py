@@ -527,7 +527,7 @@ _FEW = [(E, T, 256, 256, k) for E, k, Ts in [(2, 1, (128, 129, 512, 513)), (2, 2
 
 @pytest.mark.parametrize("E,T,dim,hid,k", [(8, 5, 256, 256, 2), (8, 37, 256, 256, 3), (8, 200, 256, 512, 2), (8, 16, 4096, 14336, 2), (8, 300, 4096, 14336, 2),
                                            (8, 2500, 256, 512, 2), (8, 2100, 1152, 1024, 2),  # enough rows per expert for the grouped GEMM on pairs
-                                           (8, 1300, 3072, 3200, 2), (4, 257, 3136, 4224, 2)]  # ... whose tiles are drawn (K >= 3072) in both GEMMs, in several turns and in one
+                                           (8, 1300, 4096, 4224, 2), (4, 257, 4160, 4096, 2), (8, 700, 4032, 4096, 2)]  # ... whose tiles are drawn (K >= 4096) in both GEMMs, in several turns and in few, and in one
                          + _FEW)  # few experts around 512 rows in all, where the plan begins to list tiles of pairs
 def test_moe_route_grouped_ffn_vs_oracle(E, T, dim, hid, k):
     """mb200_moe_route + mb200_moe_grouped_ffn against the oracle's MoE (moe.py:24-32) + residual: routing decisions and weights
