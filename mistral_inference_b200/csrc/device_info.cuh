@@ -1,7 +1,9 @@
 // What a launch asks the runtime about the current device, asked once per device: a Linear of a short prompt is 3 us of GPU time, and its queries took as long on the host.
+// And whether kernels may be launched programmatically, for both libraries.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <stdlib.h>
 
 #include <atomic>
 
@@ -33,6 +35,15 @@ inline cudaError_t allow_shared(int bytes) {
     const cudaError_t e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_relaxed);
     return e;
+}
+
+// MB200_PDL=0: no kernel begins before its predecessor in the stream has ended
+inline bool pdl_enabled() {
+    static const bool on = [] {
+        const char* e = getenv("MB200_PDL");
+        return !(e != nullptr && e[0] == '0');
+    }();
+    return on;
 }
 
 }  // namespace device_info

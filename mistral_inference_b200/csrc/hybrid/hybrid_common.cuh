@@ -9,6 +9,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "../device_info.cuh"
+
 namespace mbh {
 
 using bf16 = __nv_bfloat16;
@@ -102,7 +104,7 @@ __device__ __forceinline__ float softcap_fast(float x, float cap, float two_over
 
 // Programmatic dependent launch: a kernel launched through launch_pdl may start while its predecessor in the stream still runs; up to pdl_wait() it
 // touches nothing that an earlier kernel writes (weights only).  pdl_wait() returns when the predecessor has completed and its writes are
-// visible.  Both are no-ops in a kernel launched the ordinary way.  A decode step is some 80 short kernels: their launches and first loads
+// visible.  Both are no-ops in a kernel launched the ordinary way (MB200_PDL=0: all of them).  A decode step is some 80 short kernels: their launches and first loads
 // otherwise stand in the open.
 // What a predecessor writes is never a `const __restrict__` parameter of such a kernel: the qualifier promises that nobody writes it while the grid
 // lives, so its loads may take the read-only path and move above pdl_wait().  (Weights may be.)
@@ -119,7 +121,7 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = device_info::pdl_enabled() ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
 

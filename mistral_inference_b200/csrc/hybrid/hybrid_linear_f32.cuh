@@ -681,7 +681,7 @@ inline cudaError_t launch_f32_tokens(const LinearArgs& a, const F32Plan& p, int 
     at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 2;
+    cfg.numAttrs = device_info::pdl_enabled() ? 2 : 1;
     e = cudaLaunchKernelEx(&cfg, kernel, map, args);
     if (!e && s.counters) e = launch_pdl(f32_combine_kernel, dim3((unsigned)s.counters * (unsigned)((p.w + FC_TOKENS - 1) / FC_TOKENS)), dim3(FC_THREADS), 0, st, args);
     return e ? e : cudaGetLastError();

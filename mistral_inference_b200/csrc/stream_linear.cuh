@@ -290,7 +290,7 @@ inline bool make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t K
                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// a launch that may begin before its predecessor in the stream has ended
+// a launch that may begin before its predecessor in the stream has ended (MB200_PDL)
 template <class Kernel, class... Args>
 inline cudaError_t launch_serial(Kernel kernel, int ctas, int threads, size_t smem, cudaStream_t st, const Args&... args) {
     cudaLaunchConfig_t cfg = {};
@@ -302,7 +302,7 @@ inline cudaError_t launch_serial(Kernel kernel, int ctas, int threads, size_t sm
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = device_info::pdl_enabled() ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 

@@ -985,3 +985,40 @@ def test_decode_rows_of_a_wider_matrix(M, K, first, pitch):
     got, own = (h.linear(t, w, None, epi=h.EPI_F32) for t in (x, x.contiguous()))
     assert rel(got, x.double() @ w.double().T) < 2 * K * 2.0 ** -24
     assert M < 17 or torch.equal(got, own)
+
+
+_LAUNCHES = """
+import torch
+from cuda.bindings import runtime as rt
+from mistral_inference_b200 import _abi, _abi_hybrid as h
+ws = _abi.Workspace(_abi.workspace_bytes(128, 640, 1, 1, 128, 1024, 1024, 8), torch.device("cuda"))
+w, wf = torch.randn(1024, 640, device="cuda").bfloat16(), torch.randn(1024, 640, device="cuda")
+rows = {m: torch.randn(m, 640, device="cuda").bfloat16() for m in (4, 20, 100)}
+fp32, out = torch.randn(300, 640, device="cuda"), {m: torch.empty(m, 1024, device="cuda").bfloat16() for m in rows}
+def run():
+    for m, x in rows.items():
+        h.linear(x, w)
+        _abi.linear_residual(x, w, out[m], out[m], ws)
+    h.linear(fp32, wf)
+run()
+graph = torch.cuda.CUDAGraph(keep_graph=True)
+with torch.cuda.graph(graph):
+    run()
+err, *_, count = rt.cudaGraphGetEdges_v2(graph.raw_cuda_graph())
+err, _, _, data, count = rt.cudaGraphGetEdges_v2(graph.raw_cuda_graph(), count)
+print(count, sum(int(e.type) == int(rt.cudaGraphDependencyType.cudaGraphDependencyTypeProgrammatic) for e in data[:count]))
+"""
+
+
+@pytest.mark.parametrize("pdl", ["0", "1"])
+def test_programmatic_launches_can_be_switched_off(pdl):
+    """MB200_PDL=0 launches everything the ordinary way, in both libraries: no edge of a captured graph is a programmatic one."""
+    import os
+    import subprocess
+    import sys
+    from pathlib import Path
+
+    r = subprocess.run([sys.executable, "-c", _LAUNCHES], capture_output=True, text=True, cwd=Path(__file__).resolve().parents[1], env={**os.environ, "MB200_PDL": pdl}, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    edges, programmatic = (int(v) for v in r.stdout.split())
+    assert edges >= 9 and (programmatic == 0 if pdl == "0" else programmatic >= 5)
