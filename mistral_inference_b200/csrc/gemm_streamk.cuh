@@ -31,24 +31,6 @@ constexpr int SK_MAX_CTAS = 160;
 constexpr size_t SK_PARTIAL_BYTES = (size_t)SK_MAX_CTAS * 128 * SK_BN * sizeof(float);  // one [128 x 128] fp32 slot per CTA
 constexpr size_t SK_FLAGS_OFFSET = 24576;  // inside the zero-initialised workspace header: uint32 flags[SK_MAX_CTAS]
 
-// -DMB200_SK_TRACE: every CTA of the dense kernel stamps %globaltimer / %clock64 at eight points of its life into a device ring
-// (scripts/trace_streamk.py reads it through mb200_debug_sk_trace) -- how the microseconds between dependent launches are spent.
-#ifdef MB200_SK_TRACE
-constexpr int SK_TRACE_LAUNCHES = 64, SK_TRACE_POINTS = 8;
-__device__ unsigned long long sk_trace_buf[SK_TRACE_LAUNCHES][SK_MAX_CTAS][SK_TRACE_POINTS][2];
-__device__ unsigned sk_trace_count;
-__device__ __forceinline__ void sk_stamp(unsigned launch, int point) {
-  unsigned long long g, c;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(g));
-  asm volatile("mov.u64 %0, %%clock64;" : "=l"(c));
-  sk_trace_buf[launch % SK_TRACE_LAUNCHES][blockIdx.x][point][0] = g;
-  sk_trace_buf[launch % SK_TRACE_LAUNCHES][blockIdx.x][point][1] = c;
-}
-#define SK_STAMP(point) sk_stamp(*trace_launch, point)
-#else
-#define SK_STAMP(point) ((void)0)
-#endif
-
 struct SkParams {
   int T, N, K;
   EpiParams epi;
@@ -94,17 +76,11 @@ __device__ __forceinline__ void sk_gemm_body(const CUtensorMap& map_a, const CUt
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
   }
   if (warp == 1) tmem_alloc(tmem_base_slot, TMEM_COLS);
-#ifdef MB200_SK_TRACE
-  __shared__ unsigned trace_launch_slot;
-  if (threadIdx.x == 96) trace_launch_slot = atomicAdd(&sk_trace_count, 1u) / gridDim.x;  // all CTAs of a launch start before any of the next
-  volatile unsigned* trace_launch = &trace_launch_slot;
-#endif
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_base_slot;
   if (threadIdx.x == 0) {
-    SK_STAMP(0);  // CTA set up
     pdl_trigger();
   }
 
@@ -136,7 +112,6 @@ __device__ __forceinline__ void sk_gemm_body(const CUtensorMap& map_a, const CUt
         issue(it, false, true);
       }
       pdl_wait();
-      if (lane == 0) SK_STAMP(1);  // predecessor complete: A tiles may be requested
       for (uint32_t it = 0; it < head; ++it) issue(it, true, false);
       for (uint32_t it = head; it < n_it; ++it) {
         const uint32_t s = it % STAGES, par = (it / STAGES) & 1;
@@ -147,7 +122,6 @@ __device__ __forceinline__ void sk_gemm_body(const CUtensorMap& map_a, const CUt
         }
         if (GROUPED) __syncwarp();
       }
-      if (lane == 0) SK_STAMP(3);  // last tile requested
     }
   } else if (warp == 1) {
     // ================= MMA issuer (one thread, elected by the warp) =================
@@ -165,9 +139,6 @@ __device__ __forceinline__ void sk_gemm_body(const CUtensorMap& map_a, const CUt
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const uint32_t s = it % STAGES, par = (it / STAGES) & 1;
           mbar_wait(&full[s], par, 23, it);
-#ifdef MB200_SK_TRACE
-          if (it == 0 && lane == 0) SK_STAMP(2);  // first stage landed: first MMA
-#endif
           tc_fence_after();
           const uint32_t adesc = ring + s * (STAGE_BYTES >> 4), bdesc = adesc + (A_BYTES >> 4);
           if (elect_one()) {
@@ -181,7 +152,6 @@ __device__ __forceinline__ void sk_gemm_body(const CUtensorMap& map_a, const CUt
         __syncwarp();
         u += kb1 - kb0;
       }
-      if (lane == 0) SK_STAMP(4);  // last MMA issued
     }
   } else {
     // ================= epilogue warps 2..5: TMEM lanes 32 * (warp % 4) .. + 31 =================
@@ -250,9 +220,6 @@ __device__ __forceinline__ void sk_gemm_body(const CUtensorMap& map_a, const CUt
       const int t = row_ok ? m0 + lane_base + lane : 0x7fffffff;
       if (kb0 == 0 && t < p.T) epi_prefetch128<MODE>(p.epi, t, n0);  // this segment ends in an epilogue: its operands, while the MMAs run
       mbar_wait(&tmem_full[acc], acc_par, 24, seg);
-#ifdef MB200_SK_TRACE
-      if (threadIdx.x == 64 && u + (kb1 - kb0) >= u_end) SK_STAMP(5);  // last accumulator complete
-#endif
       tc_fence_after();
       const uint32_t trow = tmem_base + ((uint32_t)lane_base << 16) + acc * SK_BN;
       uint32_t v[32];
@@ -317,16 +284,10 @@ __device__ __forceinline__ void sk_gemm_body(const CUtensorMap& map_a, const CUt
       if (lane == 0) mbar_arrive(&tmem_empty[acc]);
       u += kb1 - kb0;
     }
-#ifdef MB200_SK_TRACE
-    if (threadIdx.x == 64) SK_STAMP(6);  // epilogues done
-#endif
   }
   tc_fence_before();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
-#ifdef MB200_SK_TRACE
-  if (threadIdx.x == 0) SK_STAMP(7);  // exit
-#endif
 }
 
 template <int MODE, int TA>
@@ -377,7 +338,6 @@ int launch_streamk_ta(const GemmParams& g, void* workspace, size_t workspace_byt
 
 template <int MODE>
 int launch_streamk(const GemmParams& g, void* workspace, size_t workspace_bytes, size_t header, cudaStream_t stream) {
-  if (g.T <= 32) return launch_streamk_ta<MODE, 32>(g, workspace, workspace_bytes, header, stream);
   if (g.T <= 64) return launch_streamk_ta<MODE, 64>(g, workspace, workspace_bytes, header, stream);
   return launch_streamk_ta<MODE, 128>(g, workspace, workspace_bytes, header, stream);
 }

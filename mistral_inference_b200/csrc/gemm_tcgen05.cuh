@@ -581,7 +581,6 @@ int launch_gemm_tcgen05_small_ta(const GemmParams& g, int sms, cudaStream_t stre
 
 template <int MODE>
 int launch_gemm_tcgen05_small(const GemmParams& g, int sms, cudaStream_t stream) {
-  if (g.T <= 32) return launch_gemm_tcgen05_small_ta<MODE, 32>(g, sms, stream);
   if (g.T <= 64) return launch_gemm_tcgen05_small_ta<MODE, 64>(g, sms, stream);
   return launch_gemm_tcgen05_small_ta<MODE, 128>(g, sms, stream);
 }

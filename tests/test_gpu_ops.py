@@ -326,9 +326,8 @@ def test_kv_ring_write():
                                  (5120, 14336),     # Nemo down projection, K = 14336: 224 k-blocks through the deep ring
                                  (1024, 6144)])     # fewer tiles than half the SMs: narrow tiles
 def test_small_batch_gemm_vs_oracle(T, N, K, ws):
-    """5 <= T < 128 runs gemm_tcgen05_kernel with 32/64-row A boxes (the MMA's upper rows read past the box; rows >= T are never
-    stored) and a tile width chosen per N: plain store and residual epilogues against the CPU oracle, and every legal tile width
-    against each other (bit-identical: same k order)."""
+    """A decode batch's Linears, up to 32 tokens on streamed rows of W and above on streamed tiles: plain store and residual epilogues against the CPU oracle, rows >= T never
+    stored."""
     if K == 14336 and T not in (16, 33, 127):
         pytest.skip("long K: representative T only")
     x, w, res = rnd(T, K, seed=50), rnd(N, K, seed=51, scale=K ** -0.5), rnd(T, N, seed=52)
@@ -340,10 +339,12 @@ def test_small_batch_gemm_vs_oracle(T, N, K, ws):
     assert_bf16_close(out[:T], F.linear(x, w), what="small-batch gemm")
 
 
-def test_small_batch_gemm_tile_widths_agree(ws, monkeypatch, rope):
-    """All tile widths of the small-batch kernel give the same bits through the QKV+RoPE+ring-scatter and SiLU*mul epilogues."""
-    monkeypatch.setenv("MB200_STREAMK", "0")  # the fallback for N not a multiple of 128: narrow tiles, one m tile
-    T, dim, H, KV, hd, hid = 24, 1024, 8, 2, 128, 1024
+@pytest.mark.parametrize("T", [33, 40, 64, 65, 127])
+def test_small_batch_gemm_tile_widths_agree(T, ws, monkeypatch, rope):
+    """All tile widths of the small-batch kernel, which takes 33 to 127 tokens where streamed tiles are off or N is no multiple of 128, give the same bits through the
+    QKV+RoPE+ring-scatter and SiLU*mul epilogues; a width that does not divide N is not taken."""
+    monkeypatch.setenv("MB200_STREAMK", "0")  # one m tile, narrow tiles
+    dim, H, KV, hd, hid = 1024, 8, 2, 128, 1024
     x = rnd(T, dim, seed=60).to(DEV)
     nw = (1 + 0.2 * rnd(dim, seed=61).float()).to(torch.bfloat16).to(DEV)
     wqkv = rnd((H + 2 * KV) * hd, dim, seed=62, scale=dim ** -0.5).to(DEV)
@@ -362,8 +363,17 @@ def test_small_batch_gemm_tile_widths_agree(ws, monkeypatch, rope):
         _abi.attn_qkv(x, nw, wqkv, table_dev, positions, q, k, v, ck, cv, rows, H, KV, hd, 1e-5, ws)
         g = torch.empty(T, hid, dtype=torch.bfloat16, device=DEV)
         _abi.ffn_gateup(x, nw, w13, g, 1e-5, ws)
+        w2 = rnd(480, hid, seed=64, scale=hid ** -0.5).to(DEV)  # 480: only the tiles of 32
+        odd = torch.empty(T, 480, dtype=torch.bfloat16, device=DEV)
+        monkeypatch.setenv("MB200_STREAMK", "1")
+        _abi.linear_residual(x, w2, None, odd, ws)
+        monkeypatch.setenv("MB200_STREAMK", "0")
         torch.cuda.synchronize()
+        assert_bf16_close(odd, F.linear(x.cpu(), w2.cpu()), what="480 features")
         outs[bn] = (q, k, v, ck, cv, g)
+    y = F.linear(x.float() * torch.rsqrt(x.float().square().mean(-1, keepdim=True) + 1e-5) * nw.float(), w13.float())
+    want = F.silu(y[:, 0::2]) * y[:, 1::2]
+    assert ((outs["32"][-1].float() - want).norm() / want.norm()).item() < 2 ** -6  # three roundings to bf16: the norm's, gate's and up's
     for bn in ("64", "128", "256"):
         for a, b, what in zip(outs["32"], outs[bn], ("q", "k", "v", "cache_k", "cache_v", "g")):
             assert torch.equal(a, b), f"{what}: tile width {bn} differs from 32"
