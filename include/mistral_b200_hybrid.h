@@ -3,7 +3,8 @@
  *
  * Conventions: pointers are device pointers; `dt` = 0 (bf16) or 1 (fp32) is the storage type of every `void*` activation
  * and weight operand; index tensors are int32 unless said otherwise; `stream` is a cudaStream_t.  Every call returns 0 or
- * an error code and leaves the text in mbh_last_error().  No call synchronises or allocates.
+ * an error code and leaves the text in mbh_last_error().  No call synchronises or allocates.  Kernels that wait on barriers of their own wait a bounded time; one whose
+ * wait runs out ends and leaves NaN where sums are missing.
  */
 #ifndef MISTRAL_B200_HYBRID_H
 #define MISTRAL_B200_HYBRID_H
@@ -32,7 +33,8 @@ int mbh_rmsnorm(const void* x32, const void* w, const void* w2, void* y, void* y
  *                              out = g * sigmoid(alpha * g) * (u + 1)
  *   3  out32[M, N] = .         fp32 result (logits); with limit > 0: limit * tanh(. / limit); with alpha != 0 times alpha
  *   5  out32[M, N] += alpha * .  the residual add of epilogue 1 with a fixed weight
- * Any M, N, K.  M <= 8 runs the weight-streaming kernel, larger M the tiled one (tensor cores for bf16). */
+ * Any M, N, K.  Up to 32 rows of bf16 (K % 8 == 0, ldx % 8 == 0, 16-byte addresses) and up to 8 of fp32 run kernels that stream the weights past them, larger M tiled ones on tensor
+ * cores (fp32: as products of bf16 parts, K >= 16). */
 int mbh_linear(const void* x, int64_t ldx, const void* w, const void* bias, void* out, void* out32, int64_t M, int64_t N, int64_t K, int epi, int64_t n_act,
                float limit, float alpha, int dt, void* stream);
 

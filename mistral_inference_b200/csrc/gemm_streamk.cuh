@@ -1,5 +1,5 @@
 // Weight-streaming GEMM for decode-sized batches (T <= 128 tokens):  C[T, N] = A[T, K] * W[N, K]^T, bound by HBM: the experts of a mixture's decode step, and dense matrices whose sums
-// have no room in the slots of stream_tiles.cuh (a head of 131072 rows from 48 tokens on).  Up to 32 tokens dense Linears run on stream_linear.cuh.
+// have no room in the slots of stream_tiles.cuh (a head of 131072 rows from 46 tokens on).  Up to 32 tokens dense Linears run on stream_linear.cuh.
 //
 // At these sizes the step reads every weight byte once and does ~2T flop per byte: the kernel's only job is to keep all 148 SMs
 // pulling their share of W at the HBM rate.  Two measured facts shape it (B200, Nemo-12B shapes, batch 32):

@@ -259,7 +259,7 @@ __device__ __forceinline__ void tile_mn(int tile, int num_m, int num_n, int& mu,
 // GROUPED = true (mixture of experts, csrc/moe.cuh): the A rows are the (token, expert) pairs sorted by expert, every expert's
 // segment padded to a multiple of TA rows; m tile i covers rows plan.tile_row0[i] .. + TA of expert plan.tile_expert[i], whose
 // weight matrix has its own tensor map (map_w[expert]).  The number of m tiles is DEVICE data (no host sync after routing).
-constexpr int MOE_PLAN_HEADER = 64;  // int32 words: [0] m tiles of this rank, [1] padded rows in total, [2] tile capacity, [6] token tiles of pairs of CTAs, [8..] segment starts
+constexpr int MOE_PLAN_HEADER = 64;  // int32 words: [0] m tiles of this rank, [1] padded rows in total, [2] tile capacity, [6] token tiles of pairs of CTAs, [7] tiles that these have drawn, [8..] segment starts
 // after the header: tile_expert[cap], tile_row0[cap], pair_expert[cap], pair_info[cap] (cap = plan[2]).  The last two list the token tiles of
 // gemm_pair.cuh: info = first row (a multiple of 32) | width / 32.
 constexpr int MOE_MAX_EXPERTS = 16;  // tensor maps travel as kernel parameters (128 B each)

@@ -20,7 +20,7 @@
 // Linear); accumulation is fp32 in both modes.
 //
 // Kernels: `linear_tiled_mma` (bf16), `linear_f32_pair` and `linear_f32_parts` (fp32, hybrid_linear_f32.cuh, hybrid_linear_f32_cta.cuh) and `linear_tiled_fma` (fp32, K < 16) for prompts, any shape; `linear_skinny` (M <= 8 rows, FMA,
-// one warp per pair of weight rows) and `stream_linear_kernel` (bf16, up to 32 rows, tensor cores) for decode: every weight byte is read
+// one warp per pair of weight rows) and `stream_linear_kernel` / `row_linear_kernel` (bf16, up to 32 / 16 rows, tensor cores) for decode: every weight byte is read
 // once; `linear_decay_mma` for decays from a low rank.  The large aligned bf16 Linears of prompts go to the main
 // library's tcgen05 GEMMs, with these steps in their epilogue (see _abi_hybrid.linear).
 #pragma once

@@ -1,7 +1,7 @@
 #!/usr/bin/env python
 """Summarise an .ncu-rep (ncu --set full) into the text kept under profiles/.
 
-usage: python scripts/ncu_summary.py prof_x.ncu-rep "header line" > profiles/r01_ncu_x.txt
+usage: python scripts/ncu_summary.py prof_x.ncu-rep "header line" > profiles/ncu_x.txt
 """
 import csv
 import io
