@@ -103,7 +103,7 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 def _rows(x: torch.Tensor):
     """(pointer, elements between rows) of a matrix whose rows are contiguous: columns of a wider one are taken as they are."""
-    assert x.is_cuda and x.dim() == 2 and x.stride(1) == 1, "rows of contiguous elements"
+    assert x.is_cuda and x.dim() == 2 and x.stride(1) == 1 and (x.shape[0] <= 1 or x.stride(0) >= x.shape[1]), "rows of contiguous elements that do not overlap"
     return x.data_ptr(), max(x.stride(0), x.shape[1])
 
 
@@ -162,9 +162,11 @@ COPIED_ROWS_FROM = 17  # fewer rows run on registers or FMAs from wherever they 
 
 
 def _streamed_as_it_lies(x: torch.Tensor) -> bool:
-    """Rows of a wider matrix that the streaming kernel reads as fast as rows of their own: 16-byte addresses, pitches of whole k-blocks where K is one.  Others are copied first: 32 rows of
+    """Rows of a wider matrix that the streaming kernel reads as fast as rows of their own: 16-byte addresses, pitches of whole k-blocks where K is one.  Others (columns of a transposed matrix and
+    rows that overlap among them) are copied first: 32 rows of
     2048 columns, pitch 2056, times 1024 features: 12.2 us as they lie, 8.7 copied; pitch 2052, which only mma.sync tiles read, 173 and 8.7."""
-    return x.data_ptr() % 16 == 0 and x.stride(0) % (64 if x.shape[1] % 64 == 0 else 8) == 0
+    return (x.stride(1) == 1 and x.stride(0) >= x.shape[1] and x.data_ptr() % 16 == 0
+            and x.stride(0) % (64 if x.shape[1] % 64 == 0 else 8) == 0)
 
 
 def _aligned(*tensors: Optional[torch.Tensor]) -> bool:

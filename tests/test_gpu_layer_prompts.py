@@ -1022,3 +1022,21 @@ def test_programmatic_launches_can_be_switched_off(pdl):
     assert r.returncode == 0, r.stderr[-2000:]
     edges, programmatic = (int(v) for v in r.stdout.split())
     assert edges >= 9 and (programmatic == 0 if pdl == "0" else programmatic >= 5)
+
+
+@pytest.mark.parametrize("M", [9, 16, 17, 32, 33, 128])
+def test_rows_of_other_orders_are_copied_or_refused(M):
+    """A transposed matrix, one row for all and rows that overlap: from 17 bf16 rows on the bits of a copy, below (and in fp32) refused, never read where they do not lie."""
+    from mistral_inference_b200 import _abi_hybrid as h
+
+    g = torch.Generator(device=DEV).manual_seed(M)
+    w = (torch.randn(256, 512, generator=g, device=DEV) / 512 ** 0.5).bfloat16()
+    flat = torch.randn(512 * M + 512, generator=g, device=DEV).bfloat16()
+    for x in (flat[: 512 * M].view(512, M).T, flat[:512].expand(M, 512), flat.as_strided((M, 512), (64, 1))):
+        if M >= 17:
+            assert torch.equal(h.linear(x, w, None, epi=h.EPI_F32), h.linear(x.contiguous(), w, None, epi=h.EPI_F32))
+        else:
+            with pytest.raises(AssertionError):
+                h.linear(x, w)
+        with pytest.raises(AssertionError):
+            h.linear(x.float() if x.stride(0) != 0 and x.stride(1) != 1 else flat.float().as_strided(x.shape, x.stride()), w.float())
