@@ -1,7 +1,7 @@
 """Generate tests/golden/*.safetensors from the UNMODIFIED reference modules
 (TEST INFRASTRUCTURE -- see oracle/__init__.py).
 
-Run in the build container (where /root/reference exists):   python -m oracle.make_golden
+Run where the reference's source tree exists:   python -m oracle.make_golden
 The reference cannot travel to the GPU box, so its outputs on small seeded cases are committed as
 fixtures.  Each fixture holds the outputs of the reference's own `Transformer.forward` /
 `generate` (mistral_inference/transformer.py:221-242, generate.py:43-148) imported behind

@@ -1,15 +1,15 @@
-"""Import shims that let the UNMODIFIED reference modules run on CPU in this container
+"""Import shims that let the UNMODIFIED reference modules run on CPU
 (TEST INFRASTRUCTURE -- see oracle/__init__.py).
 
-The reference (`/root/reference/src/mistral_inference`) imports two packages that are not
-installed and cannot be installed (no network): `xformers` (transformer_layers.py:6-7,
+The reference (`src/mistral_inference`) imports two packages that are not
+installed: `xformers` (transformer_layers.py:6-7,
 cache.py:5-10, vision_encoder.py) and `simple_parsing` (args.py:4, moe.py:6, lora.py:9).
 `install()` registers minimal stand-ins in `sys.modules` and puts the reference's `src/` on
 `sys.path`; after that `import mistral_inference.transformer` etc. work unmodified.
 
-Only usable where `/root/reference` exists (this container, not the GPU box): used by
+Only usable where the reference's source tree exists (MISTRAL_REFERENCE_SRC): used by
 `oracle/make_golden.py` to produce tests/golden/ and by tests/test_oracle_vs_reference.py to pin
-the restatement.  Mask semantics: SURVEY.md Appendix B.
+the restatement.  Mask semantics: the reference's cache.py.
 """
 import dataclasses
 import os

@@ -1,5 +1,5 @@
 """Pins the oracle restatement bit-exactly against the reference's own modules (run unmodified
-behind oracle/ref_shims.py).  Needs /root/reference, so it runs in the build container only."""
+behind oracle/ref_shims.py).  Runs only where the reference's source tree exists."""
 import pytest
 import torch
 
